@@ -21,15 +21,53 @@
 using namespace oa;
 
 namespace {
+// Scratch of one call (partials, plans, tables) comes from a stream-ordered pool of this library's own, one per device, made at the first use:
+// cudaMalloc and cudaFree stop the whole device and cost 0.1 ms to several ms a call, more than most kernels here (paged attention of 6 x 3000
+// tokens: 10 us of kernels in a call of 0.7 ms and more; from the pool 0.05 ms).  An allocation is ordered on the call's stream, so calls on
+// several streams and threads never share a block; what the pool keeps between calls is bounded, the rest goes back to the device when a call
+// synchronises.
+constexpr uint64_t SCRATCH_KEEP_BYTES = 64ull << 20;
+cudaMemPool_t scratch_pool() {
+    static std::mutex mu;
+    static std::map<int, cudaMemPool_t> pools;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+    std::lock_guard<std::mutex> lk(mu);
+    cudaMemPool_t& pool = pools[dev];
+    if (!pool) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned; props.handleTypes = cudaMemHandleTypeNone;
+        props.location.type = cudaMemLocationTypeDevice; props.location.id = dev;
+        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) { pool = nullptr; return nullptr; }
+        uint64_t keep = SCRATCH_KEEP_BYTES;
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    }
+    return pool;
+}
 struct DevBuf {
     void* p = nullptr;
-    explicit DevBuf(size_t n) { if (cudaMalloc(&p, n ? n : 16) != cudaSuccess) p = nullptr; }
-    ~DevBuf() { if (p) cudaFree(p); }
+    cudaStream_t s;
+    DevBuf(size_t n, cudaStream_t stream) : s(stream) {
+        cudaMemPool_t pool = scratch_pool();
+        if (!pool || cudaMallocFromPoolAsync(&p, n ? n : 16, pool, s) != cudaSuccess) p = nullptr;
+    }
+    DevBuf(const DevBuf&) = delete;
+    ~DevBuf() { if (p) cudaFreeAsync(p, s); }
+};
+// Host arrays of one call, packed so that ONE copy brings them to the device (each on a 16-byte boundary)
+struct Packed {
+    std::vector<uint8_t> bytes;
+    size_t add(const void* src, size_t n) {
+        const size_t at = (bytes.size() + 15) & ~size_t(15);
+        bytes.resize(at + n);
+        if (n) std::memcpy(bytes.data() + at, src, n);
+        return at;
+    }
 };
 int rc_of(cudaError_t e) { return e == cudaSuccess ? OA_OK : OA_ERR_INTERNAL; }
 }  // namespace
 
-// test-only: materialise the deterministic fixed-order sum of stream-K partials as fp32 [M,N]
+// materialise the deterministic fixed-order sum of stream-K partials as fp32 [M,N]
 __global__ void sk_reduce_f32_kernel(const StreamK sk, float* __restrict__ out, int M, int N) {
     const int row = blockIdx.x;
     for (int col = threadIdx.x; col < N; col += blockDim.x) {
@@ -49,7 +87,7 @@ int oa_k_gemm_streamk(const void* A, const void* B, int32_t M, int32_t N, int32_
     CUtensorMap tmA, tmB;
     if (make_tmap_bf16_2d(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)K, 128, 64) != 0) return OA_ERR_INTERNAL;
     if (make_tmap_bf16_2d(&tmB, B, (uint64_t)N, (uint64_t)K, (uint64_t)K, (uint32_t)block_n, 64) != 0) return OA_ERR_INTERNAL;
-    DevBuf ws(streamk_ws_bytes(N, block_n, n_ctas, M));
+    DevBuf ws(streamk_ws_bytes(N, block_n, n_ctas, M), s);
     if (!ws.p) return OA_ERR_INTERNAL;
     StreamK sk = make_streamk((float*)ws.p, N, K, block_n, n_ctas, M);
     cudaError_t e = launch_gemm_streamk(&tmA, &tmB, M, N, K, sk, s);
@@ -77,7 +115,7 @@ int oa_k_gemm(const void* A, const void* B, int32_t M, int32_t N, int32_t K, int
     p.bias = bias; p.resid = resid; p.ldr = N; p.logits = logits; p.ldl = N;
     if (epilogue == EPI_LOGITS) {
         const int nt = gemm_n_tiles(N, block_n);
-        DevBuf av((size_t)M * nt * 4), ai((size_t)M * nt * 4);
+        DevBuf av((size_t)M * nt * 4, s), ai((size_t)M * nt * 4, s);
         if (!av.p || !ai.p) return OA_ERR_INTERNAL;
         p.amax_val = (float*)av.p; p.amax_idx = (int*)ai.p;
         cudaError_t e = launch_gemm(&tmA, &tmB, p, epilogue, block_n, s);
@@ -88,9 +126,9 @@ int oa_k_gemm(const void* A, const void* B, int32_t M, int32_t N, int32_t K, int
     return rc_of(launch_gemm(&tmA, &tmB, p, epilogue, block_n, s));
 }
 
-int oa_k_paged_attention(const void* q, void* out, const void* kv_cache, int32_t num_pages, const int32_t* block_tables,
-                         int32_t max_pages_per_seq, const int32_t* ctx_lens, const int32_t* q_lens, int32_t n_seqs,
-                         int32_t n_heads, int32_t n_kv, int32_t head_dim, int32_t force_splits, void* stream) {
+static int paged_attention(const void* q, void* out, const void* kv_cache, int32_t num_pages, const int32_t* block_tables,
+                           int32_t max_pages_per_seq, const int32_t* ctx_lens, const int32_t* q_lens, int32_t n_seqs,
+                           int32_t n_heads, int32_t n_kv, int32_t head_dim, int32_t force_splits, void* stream) {
     cudaStream_t s = (cudaStream_t)stream;
     KvLayout kv{}; kv.base = const_cast<void*>(kv_cache); kv.page_size = 64; kv.n_kv = n_kv; kv.head_dim = head_dim; kv.num_pages = num_pages;
     kv.kv_stride_rows = (int64_t)num_pages * n_kv * 64; kv.layer_stride_rows = 2 * kv.kv_stride_rows;
@@ -100,26 +138,25 @@ int oa_k_paged_attention(const void* q, void* out, const void* kv_cache, int32_t
     const int grp = n_heads / n_kv;
     bool decode = true; int total_q = 0;
     for (int i = 0; i < n_seqs; ++i) { if (q_lens && q_lens[i] != 1) decode = false; total_q += q_lens ? q_lens[i] : 1; }
-    DevBuf d_bt((size_t)n_seqs * max_pages_per_seq * 4), d_ctx((size_t)n_seqs * 4);
-    if (!d_bt.p || !d_ctx.p) return OA_ERR_INTERNAL;
-    cudaMemcpyAsync(d_bt.p, block_tables, (size_t)n_seqs * max_pages_per_seq * 4, cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(d_ctx.p, ctx_lens, (size_t)n_seqs * 4, cudaMemcpyHostToDevice, s);
+    Packed host;
+    const size_t o_bt = host.add(block_tables, (size_t)n_seqs * max_pages_per_seq * 4), o_ctx = host.add(ctx_lens, (size_t)n_seqs * 4);
     cudaError_t e;
     if (decode) {
         DecodePlan plan;
         build_decode_plan(ctx_lens, n_seqs, n_kv, 2 * 148, force_splits, plan);
-        DevBuf d_segs(plan.segs.size() * sizeof(DecodeSeg)), d_ptr(plan.cta_ptr.size() * 4), d_merge(plan.merges.size() * sizeof(MergeItem));
-        DevBuf d_po((size_t)(plan.n_slots + 1) * grp * head_dim * 4), d_pml((size_t)(plan.n_slots + 1) * grp * 2 * 4);
-        if (!d_segs.p || !d_ptr.p || !d_merge.p || !d_po.p || !d_pml.p) return OA_ERR_INTERNAL;
-        cudaMemcpyAsync(d_segs.p, plan.segs.data(), plan.segs.size() * sizeof(DecodeSeg), cudaMemcpyHostToDevice, s);
-        cudaMemcpyAsync(d_ptr.p, plan.cta_ptr.data(), plan.cta_ptr.size() * 4, cudaMemcpyHostToDevice, s);
-        cudaMemcpyAsync(d_merge.p, plan.merges.data(), plan.merges.size() * sizeof(MergeItem), cudaMemcpyHostToDevice, s);
-        DecodeAttnParams a{}; a.q = q; a.out = out; a.block_tables = (const int32_t*)d_bt.p; a.ctx_lens = (const int32_t*)d_ctx.p;
-        a.max_pages_per_seq = max_pages_per_seq; a.segs = (const DecodeSeg*)d_segs.p; a.cta_seg_ptr = (const int32_t*)d_ptr.p;
+        const size_t o_segs = host.add(plan.segs.data(), plan.segs.size() * sizeof(DecodeSeg)), o_ptr = host.add(plan.cta_ptr.data(), plan.cta_ptr.size() * 4);
+        const size_t o_merge = host.add(plan.merges.data(), plan.merges.size() * sizeof(MergeItem));
+        DevBuf d_meta(host.bytes.size(), s);
+        DevBuf d_po((size_t)(plan.n_slots + 1) * grp * head_dim * 4, s), d_pml((size_t)(plan.n_slots + 1) * grp * 2 * 4, s);
+        if (!d_meta.p || !d_po.p || !d_pml.p) return OA_ERR_INTERNAL;
+        cudaMemcpyAsync(d_meta.p, host.bytes.data(), host.bytes.size(), cudaMemcpyHostToDevice, s);
+        const char* meta = (const char*)d_meta.p;
+        DecodeAttnParams a{}; a.q = q; a.out = out; a.block_tables = (const int32_t*)(meta + o_bt); a.ctx_lens = (const int32_t*)(meta + o_ctx);
+        a.max_pages_per_seq = max_pages_per_seq; a.segs = (const DecodeSeg*)(meta + o_segs); a.cta_seg_ptr = (const int32_t*)(meta + o_ptr);
         a.n_ctas = (int)plan.cta_ptr.size() - 1; a.part_o = (float*)d_po.p; a.part_ml = (float*)d_pml.p; a.layer = 0;
         a.n_heads = n_heads; a.n_kv = n_kv; a.scale_log2e = scale_log2e;
         e = launch_decode_attention(&tm, kv, a, s);
-        if (e == cudaSuccess) e = launch_decode_merge((const MergeItem*)d_merge.p, (int)plan.merges.size(), a.part_o, a.part_ml, out, n_heads, n_kv, head_dim, s);
+        if (e == cudaSuccess) e = launch_decode_merge((const MergeItem*)(meta + o_merge), (int)plan.merges.size(), a.part_o, a.part_ml, out, n_heads, n_kv, head_dim, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         return rc_of(e);
     }
@@ -129,11 +166,13 @@ int oa_k_paged_attention(const void* q, void* out, const void* kv_cache, int32_t
         for (int r = 0; r < ql; r += PREFILL_TILE_ROWS) tiles.push_back(PrefillTile{i, row + r, p0 + r, std::min(PREFILL_TILE_ROWS, ql - r)});
         row += ql;
     }
-    DevBuf d_tiles(tiles.size() * sizeof(PrefillTile));
-    if (!d_tiles.p) return OA_ERR_INTERNAL;
-    cudaMemcpyAsync(d_tiles.p, tiles.data(), tiles.size() * sizeof(PrefillTile), cudaMemcpyHostToDevice, s);
-    PrefillAttnParams a{}; a.q = q; a.out = out; a.block_tables = (const int32_t*)d_bt.p; a.max_pages_per_seq = max_pages_per_seq;
-    a.tiles = (const PrefillTile*)d_tiles.p; a.n_tiles = (int)tiles.size(); a.layer = 0; a.n_heads = n_heads; a.n_kv = n_kv; a.scale_log2e = scale_log2e;
+    const size_t o_tiles = host.add(tiles.data(), tiles.size() * sizeof(PrefillTile));
+    DevBuf d_meta(host.bytes.size(), s);
+    if (!d_meta.p) return OA_ERR_INTERNAL;
+    cudaMemcpyAsync(d_meta.p, host.bytes.data(), host.bytes.size(), cudaMemcpyHostToDevice, s);
+    const char* meta = (const char*)d_meta.p;
+    PrefillAttnParams a{}; a.q = q; a.out = out; a.block_tables = (const int32_t*)(meta + o_bt); a.max_pages_per_seq = max_pages_per_seq;
+    a.tiles = (const PrefillTile*)(meta + o_tiles); a.n_tiles = (int)tiles.size(); a.layer = 0; a.n_heads = n_heads; a.n_kv = n_kv; a.scale_log2e = scale_log2e;
     const char* leg = std::getenv("OA_PREFILL_ATTN");
     if (leg && std::string(leg) == "legacy") e = launch_prefill_attention(&tm, kv, a, s);
     else {
@@ -143,6 +182,13 @@ int oa_k_paged_attention(const void* q, void* out, const void* kv_cache, int32_t
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     return rc_of(e);
+}
+int oa_k_paged_attention(const void* q, void* out, const void* kv_cache, int32_t num_pages, const int32_t* block_tables,
+                         int32_t max_pages_per_seq, const int32_t* ctx_lens, const int32_t* q_lens, int32_t n_seqs,
+                         int32_t n_heads, int32_t n_kv, int32_t head_dim, int32_t force_splits, void* stream) {
+    try {      // the host arrays are packed into vectors: no exception may cross the C boundary
+        return paged_attention(q, out, kv_cache, num_pages, block_tables, max_pages_per_seq, ctx_lens, q_lens, n_seqs, n_heads, n_kv, head_dim, force_splits, stream);
+    } catch (const std::exception&) { return OA_ERR_INTERNAL; }
 }
 
 
