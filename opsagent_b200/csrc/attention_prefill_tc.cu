@@ -19,7 +19,6 @@
 
 namespace oa {
 
-static constexpr int PTC_MAX_THREADS = 64 + 2 * 128;
 static constexpr int KV_TILE = 128;
 
 template <int D>
@@ -272,6 +271,292 @@ __global__ void __launch_bounds__(64 + 128 * NWG, 1) prefill_attention_tc_kernel
     if (warp == 1) { tcgen05_fence_after(); tmem_dealloc<Cfg::TMEM_COLS>(tmem_base); }
 }
 
+// ---------------------------------------------------------------------------------------------
+// Two heads of one key/value group per CTA, for batches that fill the chip.
+//
+// One query tile's chain per KV tile — S, maximum, 128 exponentials a row, P, P·V — keeps either the tensor pipe or the softmax warps waiting
+// (30 % of the tensor pipe at prompts of 1.5 thousand tokens).  Here a CTA carries the SAME 128 query rows of TWO heads that read the same keys
+// and values, each with a softmax warpgroup of its own: while warpgroup A works on S_A, the tensor core runs P_B·V and the next S_B.  The heads
+// see the same keys, so both take the same number of KV tiles, and a K / V tile is fetched once for both.  P goes back into TMEM over its own S
+// (bf16, columns 0..63 of the 128) and is the A operand of P·V from there: no shared-memory round trip, and shared memory holds Q of both heads
+// and two K and two V tiles.  tcgen05.mma of one thread run in order, so S_X(j+1) may be issued right behind P_X(j)·V: it overwrites P_X(j)
+// after that has been read, and its completion says that O_X has landed, which is all that rescaling O_X needs.
+// Persistent: one CTA per SM walks (row tile, head pair) items, heaviest first, every second round in reverse; the ring keeps loading across
+// items and one warpgroup's output is written under the other's last products.
+//   warp 0    : TMA (K, Q, V)        warp 1 : tcgen05.mma        warps 4-7 / 8-11 : softmax and output of head A / B, one query row per thread
+// A group with an odd number of heads leaves its last one alone in an item (warpgroup B idles).
+// Measured against the kernel above: 4096 rows behind 12288 cached ones, 64 / 8 heads of 128: 1967 -> 1544 us (1.25 PFLOP/s; the tensor and the
+// special-function pipe are each busy 60 % of the time and the clock is down to 1.63 GHz under the 1000 W cap); five prompts of 1.4 thousand rows,
+// 32 / 8 heads: 184 -> 121 us.  Handing P over in two or three parts, taking exponentials from a reference that may still rise, moving an eighth
+// or a quarter of them to the FMA pipe and two threads per row were each 3 to 12 % slower.
+// ---------------------------------------------------------------------------------------------
+template <int D>
+struct PtpCfg {
+    static constexpr int HALVES = D / 64;
+    static constexpr int HALF_BYTES = 128 * 128;
+    static constexpr int TILE_BYTES = HALVES * HALF_BYTES;       // Q of one head, K or V of one 128-token tile
+    static constexpr int STAGES = 2;
+    static constexpr int SMEM_BYTES = (2 + 2 * STAGES) * TILE_BYTES + 256;
+    static constexpr uint32_t TMEM_COLS = 512;
+    static constexpr uint32_t S_COL = 0, O_COL = 256;            // S_A, S_B (P over them), then O_A, O_B: 128 columns each
+    static constexpr int THREADS = 3 * 128;
+};
+
+struct PtpItem { PrefillTile tile; int head, two, n_kvt; };
+// item of this CTA in round r: rounds alternate direction, so that no CTA gets the heaviest item of every round
+OA_DEVINL bool ptp_item(const PrefillAttnParams& p, int pairs_per_group, int round, PtpItem& it) {
+    const int G = (int)gridDim.x, n_items = p.n_tiles * p.n_kv * pairs_per_group;
+    const int idx = round * G + ((round & 1) ? G - 1 - (int)blockIdx.x : (int)blockIdx.x);
+    if (idx >= n_items) return false;
+    const int per_tile = p.n_kv * pairs_per_group, ti = idx / per_tile, hp = idx - ti * per_tile;
+    const int kvh = hp / pairs_per_group, pr = hp - kvh * pairs_per_group, grp = p.n_heads / p.n_kv;
+    it.tile = p.tiles[ti];
+    it.head = kvh * grp + 2 * pr;
+    it.two = 2 * pr + 1 < grp;
+    it.n_kvt = (it.tile.pos0 + it.tile.n_rows + KV_TILE - 1) / KV_TILE;
+    return true;
+}
+
+template <int D>
+__global__ void __launch_bounds__(PtpCfg<D>::THREADS, 1) prefill_attention_pair_kernel(const __grid_constant__ CUtensorMap tm_q,
+                                                                                       const __grid_constant__ CUtensorMap tm_kv,
+                                                                                       const PrefillAttnParams p, const int64_t layer_row0,
+                                                                                       const int64_t kv_stride_rows) {
+    using Cfg = PtpCfg<D>;
+    constexpr int HALVES = Cfg::HALVES, STAGES = Cfg::STAGES;
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t* q_s = smem_raw;                                     // [2 heads]
+    uint8_t* k_s = q_s + 2 * Cfg::TILE_BYTES;                    // [STAGES]
+    uint8_t* v_s = k_s + STAGES * Cfg::TILE_BYTES;               // [STAGES]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(v_s + STAGES * Cfg::TILE_BYTES);
+    uint64_t* q_full = bars;                  // 1
+    uint64_t* q_empty = bars + 1;             // 1
+    uint64_t* k_full = bars + 2;              // [STAGES]
+    uint64_t* k_empty = k_full + STAGES;
+    uint64_t* v_full = k_empty + STAGES;
+    uint64_t* v_empty = v_full + STAGES;
+    uint64_t* s_full = v_empty + STAGES;      // [2 heads]
+    uint64_t* p_full = s_full + 2;
+    uint64_t* o_full = p_full + 2;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 2);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int grp = p.n_heads / p.n_kv, ppg = (grp + 1) / 2;
+    PtpItem it;
+
+    if (warp == 0 && lane == 0) {
+        tma_prefetch_desc(&tm_q); tma_prefetch_desc(&tm_kv);
+        mbar_init(q_full, 1); mbar_init(q_empty, 1);
+        for (int i = 0; i < STAGES; ++i) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
+        for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 4); mbar_init(&o_full[i], 1); }
+        fence_barrier_init();
+    }
+    if (warp == 1) tmem_alloc<Cfg::TMEM_COLS>(tmem_slot);
+    tcgen05_fence_before();
+    __syncthreads();
+    tcgen05_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    griddep_launch();
+
+    // registers: 384 x 168 at launch = 128 x (88 + 208 + 208)
+    if (warp < 4) {
+        reg_dec<88>();
+        if (warp == 0 && lane == 0) {
+            griddep_wait();
+            uint32_t kc = 0;
+            for (int r = 0; ptp_item(p, ppg, r, it); ++r) {
+                const int32_t* bt = p.block_tables + (size_t)it.tile.seq * p.max_pages_per_seq;
+                const int kvh = it.head / grp;
+                auto page_row = [&](int pi, int fallback) { return layer_row0 + ((int64_t)bt[pi < p.max_pages_per_seq ? pi : fallback] * p.n_kv + kvh) * 64; };   // a missing second page is fully masked anyway
+                auto load = [&](uint8_t* dst, uint64_t* bar, int64_t r0, int64_t r1) {
+                    mbar_expect_tx(bar, Cfg::TILE_BYTES);
+#pragma unroll
+                    for (int h = 0; h < HALVES; ++h) {
+                        tma_load_2d(dst + h * Cfg::HALF_BYTES, &tm_kv, bar, h * 64, (int32_t)r0, kEvictLast);
+                        tma_load_2d(dst + h * Cfg::HALF_BYTES + 8192, &tm_kv, bar, h * 64, (int32_t)r1, kEvictLast);
+                    }
+                };
+                int64_t r0 = page_row(0, 0), r1 = page_row(1, 0);
+                for (int j = 0; j < it.n_kvt; ++j, ++kc) {
+                    const uint32_t st = kc % STAGES, ph = (kc / STAGES) & 1;
+                    mbar_wait(&k_empty[st], ph ^ 1);
+                    load(k_s + st * Cfg::TILE_BYTES, &k_full[st], r0, r1);
+                    if (j == 0) {
+                        mbar_wait(q_empty, ((uint32_t)r & 1) ^ 1);
+                        mbar_expect_tx(q_full, (it.two ? 2 : 1) * Cfg::TILE_BYTES);
+                        for (int x = 0; x <= it.two; ++x)
+#pragma unroll
+                            for (int h = 0; h < HALVES; ++h)
+                                tma_load_2d(q_s + x * Cfg::TILE_BYTES + h * Cfg::HALF_BYTES, &tm_q, q_full, (it.head + x) * D + h * 64, it.tile.q_row0, kEvictFirst);
+                    }
+                    int64_t n0 = r0, n1 = r1;                                  // the next tile's pages are looked up while this one's slot is waited for
+                    if (j + 1 < it.n_kvt) { n0 = page_row(2 * j + 2, 0); n1 = page_row(2 * j + 3, 2 * j + 2); }
+                    mbar_wait(&v_empty[st], ph ^ 1);
+                    load(v_s + st * Cfg::TILE_BYTES, &v_full[st], r0 + kv_stride_rows, r1 + kv_stride_rows);
+                    r0 = n0; r1 = n1;
+                }
+            }
+        } else if (warp == 1 && lane == 0) {
+            constexpr uint32_t idesc_s = umma_idesc_bf16(128, KV_TILE), idesc_o = umma_idesc_bf16_bmn(128, D);
+            const uint32_t q_addr = smem_u32(q_s), k_addr0 = smem_u32(k_s), v_addr0 = smem_u32(v_s);
+            uint32_t kc = 0, vc = 0, pc[2] = {0, 0};                           // K / V tiles taken, P tiles taken per head
+            auto issue_s = [&](int x) {                                        // S_x = Q_x K^T with K tile kc
+                const uint32_t a = q_addr + x * Cfg::TILE_BYTES, b = k_addr0 + (kc % STAGES) * Cfg::TILE_BYTES;
+#pragma unroll
+                for (int ks = 0; ks < D / 16; ++ks) {
+                    const uint32_t off = (uint32_t)((ks >> 2) * Cfg::HALF_BYTES + (ks & 3) * 32);
+                    umma_bf16(tmem_base + Cfg::S_COL + x * 128, umma_desc_sw128(a + off), umma_desc_sw128(b + off), idesc_s, ks > 0 ? 1u : 0u);
+                }
+                umma_commit(&s_full[x]);
+            };
+            auto issue_o = [&](int x, bool first) {                            // O_x (+)= P_x V with V tile vc
+                mbar_wait(&p_full[x], pc[x] & 1); ++pc[x];
+                tcgen05_fence_after();
+                const uint32_t b = v_addr0 + (vc % STAGES) * Cfg::TILE_BYTES;
+#pragma unroll
+                for (int ks = 0; ks < KV_TILE / 16; ++ks)
+                    umma_bf16_ta(tmem_base + Cfg::O_COL + x * 128, tmem_base + Cfg::S_COL + x * 128 + ks * 8, umma_desc_sw128_mn(b + (uint32_t)(ks * 2048), (uint32_t)Cfg::HALF_BYTES, 1024u),
+                                 idesc_o, (!first || ks > 0) ? 1u : 0u);
+            };
+            for (int r = 0; ptp_item(p, ppg, r, it); ++r) {
+                mbar_wait(q_full, (uint32_t)r & 1);
+                mbar_wait(&k_full[kc % STAGES], (kc / STAGES) & 1);
+                tcgen05_fence_after();
+                for (int x = 0; x <= it.two; ++x) issue_s(x);
+                umma_commit(&k_empty[kc % STAGES]); ++kc;
+                if (it.n_kvt == 1) umma_commit(q_empty);
+                for (int j = 0; j < it.n_kvt; ++j) {
+                    const bool last = j + 1 == it.n_kvt;
+                    mbar_wait(&v_full[vc % STAGES], (vc / STAGES) & 1);
+                    if (!last) mbar_wait(&k_full[kc % STAGES], (kc / STAGES) & 1);
+                    for (int x = 0; x <= it.two; ++x) {
+                        issue_o(x, j == 0);
+                        if (last) umma_commit(&o_full[x]); else issue_s(x);
+                    }
+                    umma_commit(&v_empty[vc % STAGES]); ++vc;
+                    if (!last) {
+                        umma_commit(&k_empty[kc % STAGES]); ++kc;
+                        if (j + 2 == it.n_kvt) umma_commit(q_empty);           // the item's last S: the next item's Q may come
+                    }
+                }
+            }
+        }
+    } else {
+        reg_inc<208>();
+        const int q = warp & 3, x = (warp - 4) >> 2;                // TMEM lanes 32 q ..; head A or B of the item
+        const int row = q * 32 + lane;
+        const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
+        const uint32_t s_addr = tmem_base + lane_addr + Cfg::S_COL + x * 128, o_addr = tmem_base + lane_addr + Cfg::O_COL + x * 128;
+        constexpr float kRescaleThreshold = 8.0f;                   // log2 units: p may reach 2^8 before O is rescaled
+        const uint64_t scale2 = pack_f32x2(p.scale_log2e, p.scale_log2e);
+        griddep_wait();                                             // the output may still be read by a predecessor
+        uint32_t sc = 0, oc = 0;                                    // S tiles and items this warpgroup has taken
+        for (int r = 0; ptp_item(p, ppg, r, it); ++r) {
+            if (x > it.two) continue;
+            const int qpos = it.tile.pos0 + row;
+            float m_ref = -INFINITY, l_run = 0.f;
+            for (int j = 0; j < it.n_kvt; ++j, ++sc) {
+                mbar_wait(&s_full[x], sc & 1);
+                tcgen05_fence_after();
+                uint32_t v[4][32];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) tmem_ld_32x32b_x32(s_addr + (uint32_t)(c * 32), v[c]);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) tmem_ld_wait_for(v[c]);
+                if (j * KV_TILE + KV_TILE - 1 > it.tile.pos0) {                     // some (row, key) pairs of this tile are masked
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) if (j * KV_TILE + c * 32 + i > qpos) v[c][i] = 0xff800000u;
+                }
+                float m[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    m[k] = __uint_as_float(v[0][k]);
+#pragma unroll
+                    for (int i = 4; i < 124; i += 8) m[k] = fmax3_nan(m[k], __uint_as_float(v[(i + k) / 32][(i + k) % 32]), __uint_as_float(v[(i + k + 4) / 32][(i + k + 4) % 32]));
+                    m[k] = fmax_nan(m[k], __uint_as_float(v[3][28 + k]));
+                }
+                const float mx = fmax_nan(fmax3_nan(m[0], m[1], m[2]), m[3]) * p.scale_log2e;       // the scale is positive
+                // always true on tile 0 (key 0 is visible to every row); also where a score is NaN: then m_ref, every p and the row's result are
+                const bool raise = !(mx <= m_ref + kRescaleThreshold);
+                if (__any_sync(0xffffffffu, raise)) {
+                    if (j > 0) {                                    // S_j has completed, so P_{j-1} V has: O holds every tile before this one
+                        const float alpha = raise ? exp2f(m_ref - mx) : 1.0f;
+#pragma unroll 1
+                        for (int c = 0; c < D; c += 16) {
+                            uint32_t o[16];
+                            tmem_ld_32x32b_x16(o_addr + (uint32_t)c, o);
+                            tmem_ld_wait();
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                            tmem_st_32x32b_x16(o_addr + (uint32_t)c, o);
+                        }
+                        l_run *= alpha;
+                    }
+                    if (raise) m_ref = mx;
+                }
+                const uint64_t nref2 = pack_f32x2(-m_ref, -m_ref);
+                uint64_t sum2[2] = {0ull, 0ull};
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {                       // 32 scores of the row -> 16 columns of P: p = 2^(s * scale - m_ref)
+                    uint32_t pw[16];
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        float a, b;
+                        unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(v[c][2 * i]), __uint_as_float(v[c][2 * i + 1])), scale2, nref2), a, b);
+                        a = ex2_approx(a); b = ex2_approx(b);
+                        sum2[i & 1] = add_f32x2(sum2[i & 1], pack_f32x2(a, b));
+                        pw[i] = pack_bf16x2(a, b);
+                    }
+                    tmem_st_32x32b_x16(s_addr + (uint32_t)(c * 16), pw);
+                }
+                tmem_st_wait();
+                tcgen05_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&p_full[x]);
+                float a, b;
+                unpack_f32x2(add_f32x2(sum2[0], sum2[1]), a, b);
+                l_run += a + b;
+            }
+            mbar_wait(&o_full[x], oc & 1); ++oc;
+            tcgen05_fence_after();
+            const float inv = 1.0f / l_run;
+            uint16_t* orow = reinterpret_cast<uint16_t*>(p.out) + (size_t)(it.tile.q_row0 + row) * p.n_heads * D + (size_t)(it.head + x) * D;
+#pragma unroll 1
+            for (int c = 0; c < D; c += 32) {
+                uint32_t o[32];
+                tmem_ld_32x32b_x32(o_addr + (uint32_t)c, o);
+                tmem_ld_wait();
+                if (row < it.tile.n_rows) {
+#pragma unroll
+                    for (int i = 0; i < 32; i += 8) {
+                        uint4 w4;
+                        w4.x = pack_bf16x2(__uint_as_float(o[i]) * inv, __uint_as_float(o[i + 1]) * inv);
+                        w4.y = pack_bf16x2(__uint_as_float(o[i + 2]) * inv, __uint_as_float(o[i + 3]) * inv);
+                        w4.z = pack_bf16x2(__uint_as_float(o[i + 4]) * inv, __uint_as_float(o[i + 5]) * inv);
+                        w4.w = pack_bf16x2(__uint_as_float(o[i + 6]) * inv, __uint_as_float(o[i + 7]) * inv);
+                        *reinterpret_cast<uint4*>(orow + c + i) = w4;
+                    }
+                }
+            }
+            tcgen05_fence_before();                                 // O has been read before this warp's next p_full lets P·V overwrite it
+        }
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+    if (warp == 1) { tcgen05_fence_after(); tmem_dealloc<Cfg::TMEM_COLS>(tmem_base); }
+}
+
+template <int D>
+static cudaError_t launch_ptp(const CUtensorMap* tm_q, const CUtensorMap* tm_kv, const KvLayout& kv, const PrefillAttnParams& p, int items, int sms, cudaStream_t s) {
+    auto kern = prefill_attention_pair_kernel<D>;
+    static bool attr_done[16] = {};
+    { cudaError_t e = ensure_dynamic_smem(kern, PtpCfg<D>::SMEM_BYTES, attr_done); if (e != cudaSuccess) return e; }
+    return launch_k(kern, dim3(items < sms ? items : sms), dim3(PtpCfg<D>::THREADS), PtpCfg<D>::SMEM_BYTES, s, *tm_q, *tm_kv, p,
+                    (int64_t)p.layer * kv.layer_stride_rows, kv.kv_stride_rows);
+}
+
 template <int D, int NWG>
 static cudaError_t launch_ptc(const CUtensorMap* tm_q, const CUtensorMap* tm_kv, const KvLayout& kv, const PrefillAttnParams& p, cudaStream_t s) {
     auto kern = prefill_attention_tc_kernel<D, NWG>;
@@ -281,10 +566,24 @@ static cudaError_t launch_ptc(const CUtensorMap* tm_q, const CUtensorMap* tm_kv,
                     (int64_t)p.layer * kv.layer_stride_rows, kv.kv_stride_rows);
 }
 
+static int prefill_sm_count() {
+    static const int n = [] { int dev = 0, v = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev); return v > 0 ? v : 148; }();
+    return n;
+}
+
 cudaError_t launch_prefill_attention_tc(const CUtensorMap* tm_q, const CUtensorMap* tm_kv, const KvLayout& kv, const PrefillAttnParams& p, cudaStream_t s) {
     if (p.n_tiles <= 0) return cudaSuccess;
     if (kv.page_size != 64 || p.n_heads % p.n_kv != 0) return cudaErrorInvalidValue;
     static const int nwg = [] { const char* e = std::getenv("OA_PREFILL_WG"); return (e && e[0] == '1') ? 1 : 2; }();      // OA_PREFILL_WG=1: the one-warpgroup kernel of round 1 (A/B)
+    const int grp = p.n_heads / p.n_kv, items = p.n_tiles * p.n_kv * ((grp + 1) / 2);
+    const int sms = prefill_sm_count();
+    // Up to half as many items as SMs, twice as many single-head CTAs are all resident at once and each is done sooner (32 / 8 heads, 400 rows
+    // behind 6000, 64 items: 97 us against 130 in pairs); above that the pairs win (700 rows behind 4000, 96 items: 125 -> 107 us; 614 rows,
+    // 80 items: 47 -> 46; 1536 rows, 192 items: 76 -> 62).
+    if (grp > 1 && items > sms / 2) {
+        if (kv.head_dim == 128) return launch_ptp<128>(tm_q, tm_kv, kv, p, items, sms, s);
+        if (kv.head_dim == 64) return launch_ptp<64>(tm_q, tm_kv, kv, p, items, sms, s);
+    }
     if (kv.head_dim == 128) return nwg == 2 ? launch_ptc<128, 2>(tm_q, tm_kv, kv, p, s) : launch_ptc<128, 1>(tm_q, tm_kv, kv, p, s);
     if (kv.head_dim == 64) return nwg == 2 ? launch_ptc<64, 2>(tm_q, tm_kv, kv, p, s) : launch_ptc<64, 1>(tm_q, tm_kv, kv, p, s);
     return cudaErrorInvalidValue;

@@ -166,6 +166,8 @@ static int paged_attention(const void* q, void* out, const void* kv_cache, int32
         for (int r = 0; r < ql; r += PREFILL_TILE_ROWS) tiles.push_back(PrefillTile{i, row + r, p0 + r, std::min(PREFILL_TILE_ROWS, ql - r)});
         row += ql;
     }
+    // the tiles with most keys first, as the engine has them: the causal triangle otherwise ends in a tail of heavy tiles
+    std::stable_sort(tiles.begin(), tiles.end(), [](const PrefillTile& x, const PrefillTile& y) { return x.pos0 + x.n_rows > y.pos0 + y.n_rows; });
     const size_t o_tiles = host.add(tiles.data(), tiles.size() * sizeof(PrefillTile));
     DevBuf d_meta(host.bytes.size(), s);
     if (!d_meta.p) return OA_ERR_INTERNAL;

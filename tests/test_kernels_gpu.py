@@ -280,3 +280,33 @@ def test_paged_prefill_attention(L, nh, nkv, D):
     assert torch.isfinite(out.float()).all()
     err = (out.float() - ref).abs().max().item()
     assert err < 2e-2, err
+
+
+# batches that fill the chip take the two-heads-per-CTA kernel: an even and an odd number of heads per group (the last head of an odd group is
+# alone), portions behind a cached prefix, tiles of one row, key tiles whose second page is missing, and more items than CTAs
+@pytest.mark.parametrize("nh,nkv,D", [(32, 8, 128), (20, 4, 128), (32, 8, 64), (15, 3, 64), (16, 2, 128)])
+def test_paged_prefill_attention_two_heads_per_cta(L, nh, nkv, D):
+    cases = [(64, 64), (130, 130), (200, 37), (1, 1), (700, 513), (128, 128), (65, 65), (449, 1), (333, 300), (1000, 129)] * 2
+    ctx = [c for c, _ in cases]; qlens = [q for _, q in cases]
+    n = len(ctx); maxp = 16; num_pages = 140
+    kv = _mk_cache(num_pages, nkv, D, 3)
+    g = torch.Generator(device="cpu").manual_seed(9)
+    perm = torch.randperm(num_pages, generator=g)
+    bt = torch.zeros(n, maxp, dtype=torch.int32); k = 0
+    for i, c in enumerate(ctx):
+        npg = (c + 63) // 64; bt[i, :npg] = perm[k:k + npg].to(torch.int32); k += npg
+    T = sum(qlens)
+    q = torch.randn(T, nh, D, generator=g)
+    q[::7] *= 12                                     # scores that raise a row's maximum by more than 2^8 in a later tile
+    q[5, 0, 3] = float("nan")                        # a query with a NaN: its own result, and nothing else, is NaN
+    q = q.to(torch.bfloat16).to(dev())
+    out = torch.full((T, nh, D), 7.0, dtype=torch.bfloat16, device=dev())
+    ctx_a = np.array(ctx, np.int32); ql = np.array(qlens, np.int32); bt_np = np.ascontiguousarray(bt.numpy())
+    rc = L.oa_k_paged_attention(ptr(q), ptr(out), ptr(kv), num_pages, bt_np.ctypes.data, maxp, ctx_a.ctypes.data, ql.ctypes.data, n,
+                                nh, nkv, D, 0, None)
+    assert rc == 0, _lib.last_error()
+    ref = _attn_ref(q, kv[0], kv[1], bt.to(dev()).long(), ctx, qlens, nh, nkv, D)
+    assert torch.equal(torch.isnan(out), torch.isnan(ref)) and torch.isnan(out).sum().item() == D
+    # probabilities and result are rounded to bf16 (2^-9 relative each); |values| stay below 5
+    err = (out.float() - ref).nan_to_num().abs().max().item()
+    assert err < 2 * 5 * 2.0 ** -8, err
