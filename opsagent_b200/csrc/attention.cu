@@ -12,7 +12,7 @@
 //                 group's heads in the M rows), online softmax in registers, O += P·V; per-warp (m, l, O)
 //                 states are merged once per segment through 12 KB of shared memory.
 //   Long or ragged contexts are cut into segments by a host-made plan; partial (m, l, O) go to a workspace and
-//   decode_merge_kernel combines them (flash-decoding).
+//   the CTA that finishes an item's last piece combines them (flash-decoding).
 // The 16-row mma.sync tile is the right tool here: with <= 8 real rows per tile even the legacy tensor path
 // is > 10x faster than the HBM stream it has to keep up with, and tcgen05's 128-row minimum cannot be filled.
 //
@@ -34,7 +34,7 @@ struct AttCfg {
     static constexpr int STAGE_BYTES = 2 * KV_BYTES;
     static constexpr int STAGES = (D == 128) ? 3 : 4;
     static constexpr int SCRATCH_BYTES = 3 * (D / 4) * 32 * 4;   // 3 warps x (D/8 tiles x 2 regs) x 32 lanes fp32
-    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + SCRATCH_BYTES + 4 * 8 * 2 * 4 + 2 * STAGES * 8 + 1024;
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + SCRATCH_BYTES + 4 * 8 * 2 * 4 + 2 * STAGES * 8 + 16 + 1024;
 };
 
 // byte offset of the 16-byte chunk holding (row r, columns d..d+7) inside one K or V stage buffer
@@ -62,6 +62,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) decode_attention_kernel(const 
     float* ml_s = scratch + Cfg::SCRATCH_BYTES / 4;          // [4 warps][8 rows][2]
     uint64_t* full_bar = reinterpret_cast<uint64_t*>(ml_s + 64);
     uint64_t* empty_bar = full_bar + STAGES;
+    volatile int* merge_s = reinterpret_cast<volatile int*>(empty_bar + STAGES);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int grp = p.n_heads / p.n_kv;
@@ -235,68 +236,53 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) decode_attention_kernel(const 
                     }
                 }
             }
-            if (sg.partial_slot >= 0 && p.merge_counters) {
+            if (sg.partial_slot >= 0) {
                 // flash-decoding merge without a second kernel: the CTA that finishes an item's LAST piece combines all pieces.
                 // Counters advance by n_pieces per layer and start each step at zero, so "last" is a multiple of n_pieces.
                 __threadfence();
                 __syncwarp();
-                int last = 0;
-                if (lane == 0) last = ((atomicAdd(p.merge_counters + sg.item, 1) + 1) % sg.n_pieces) == 0;
-                last = __shfl_sync(0xffffffffu, last, 0);
-                if (last) {
+                if (lane == 0) {
+                    const int last = ((atomicAdd(p.merge_counters + sg.item, 1) + 1) % sg.n_pieces) == 0;
                     __threadfence();
-                    if (g < grp) {
-                        float m_all = -INFINITY;
-                        for (int i = 0; i < sg.n_pieces; ++i) m_all = fmaxf(m_all, __ldcg(p.part_ml + ((size_t)(sg.slot_begin + i) * grp + g) * 2));
-                        float l_all = 0.f;
-#pragma unroll
-                        for (int j = 0; j < NT; ++j) { oacc[j][0] = 0.f; oacc[j][1] = 0.f; }
-                        for (int i = 0; i < sg.n_pieces; ++i) {                       // slot order: deterministic
-                            const size_t sl = (size_t)(sg.slot_begin + i) * grp + g;
-                            const float f = exp2f(__ldcg(p.part_ml + sl * 2) - m_all);
-                            l_all += f * __ldcg(p.part_ml + sl * 2 + 1);
-                            const float* pi = p.part_o + sl * D;
-#pragma unroll
-                            for (int j = 0; j < NT; ++j) { const float2 v2 = __ldcg(reinterpret_cast<const float2*>(pi + j * 8 + 2 * t)); oacc[j][0] += f * v2.x; oacc[j][1] += f * v2.y; }
-                        }
-                        const float inv = 1.0f / l_all;
-                        uint16_t* orow = reinterpret_cast<uint16_t*>(p.out) + (size_t)sg.seq * p.n_heads * D + (size_t)(sg.kvh * grp + g) * D;
-#pragma unroll
-                        for (int j = 0; j < NT; ++j)
-                            *reinterpret_cast<uint32_t*>(orow + j * 8 + 2 * t) = pack_bf16x2(oacc[j][0] * inv, oacc[j][1] * inv);
-                    }
+                    *merge_s = last;
                 }
             }
         }
-        named_bar_sync(1, 128);   // scratch free for the next segment
-    }
-}
-
-// out[seq, head, :] = sum_i 2^(m_i - m) o_i / sum_i 2^(m_i - m) l_i over the item's partial slots
-__global__ void decode_merge_kernel(const MergeItem* __restrict__ items, const float* __restrict__ part_o,
-                                    const float* __restrict__ part_ml, uint16_t* __restrict__ out, int n_heads, int n_kv, int D) {
-    griddep_launch(); griddep_wait();
-    const MergeItem it = items[blockIdx.x];
-    const int grp = n_heads / n_kv;
-    for (int idx = threadIdx.x; idx < grp * D; idx += blockDim.x) {
-        const int g = idx / D, d = idx - g * D;
-        float m_tot = -INFINITY;
-        for (int i = 0; i < it.n_slots; ++i) m_tot = fmaxf(m_tot, part_ml[((size_t)(it.slot_begin + i) * grp + g) * 2]);
-        float o = 0.f, l = 0.f;
-        for (int i = 0; i < it.n_slots; ++i) {
-            const size_t sl = (size_t)(it.slot_begin + i) * grp + g;
-            const float f = exp2f(part_ml[sl * 2] - m_tot);
-            o += f * part_o[sl * D + d];
-            l += f * part_ml[sl * 2 + 1];
+        named_bar_sync(1, 128);   // scratch free for the next segment; merge_s says whether this CTA merges the item
+        if (sg.partial_slot >= 0) {
+            if (*merge_s) {
+                // The four warps take a quarter of the columns each (lane: head g, NC consecutive columns from t * NC of the quarter), pieces in
+                // slot order (deterministic), four pieces' loads in flight: a context cut over the whole chip has up to 37 pieces per item, and
+                // one warp reading them one after the other was as long as the attention itself
+                constexpr int NC = D / 16;                               // columns per lane: 8 (D = 128) or 4
+                if (g < grp) {
+                    const float* ml = p.part_ml + ((size_t)sg.slot_begin * grp + g) * 2;
+                    const float* po = p.part_o + ((size_t)sg.slot_begin * grp + g) * D + warp * (D / 4) + t * NC;
+                    float m_all = -INFINITY;
+                    for (int i = 0; i < sg.n_pieces; ++i) m_all = fmaxf(m_all, __ldcg(ml + (size_t)i * grp * 2));
+                    float l_all = 0.f, o[NC];
+#pragma unroll
+                    for (int k = 0; k < NC; ++k) o[k] = 0.f;
+#pragma unroll 4
+                    for (int i = 0; i < sg.n_pieces; ++i) {
+                        const float2 st = __ldcg(reinterpret_cast<const float2*>(ml + (size_t)i * grp * 2));
+                        float4 u[NC / 4];
+#pragma unroll
+                        for (int k = 0; k < NC / 4; ++k) u[k] = __ldcg(reinterpret_cast<const float4*>(po + (size_t)i * grp * D) + k);
+                        const float f = exp2f(st.x - m_all);
+                        l_all += f * st.y;
+#pragma unroll
+                        for (int k = 0; k < NC / 4; ++k) { o[4 * k] += f * u[k].x; o[4 * k + 1] += f * u[k].y; o[4 * k + 2] += f * u[k].z; o[4 * k + 3] += f * u[k].w; }
+                    }
+                    const float inv = 1.0f / l_all;
+                    uint32_t* orow = reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(p.out) + (size_t)sg.seq * p.n_heads * D + (size_t)(sg.kvh * grp + g) * D + warp * (D / 4) + t * NC);
+#pragma unroll
+                    for (int k = 0; k < NC / 2; ++k) orow[k] = pack_bf16x2(o[2 * k] * inv, o[2 * k + 1] * inv);
+                }
+            }
+            named_bar_sync(1, 128);   // merge_s has been read
         }
-        out[(size_t)it.seq * n_heads * D + (size_t)(it.kvh * grp + g) * D + d] = f32_to_bf16_bits(o / l);
     }
-}
-
-cudaError_t launch_decode_merge(const MergeItem* items, int n_items, const float* part_o, const float* part_ml, void* out,
-                                int n_heads, int n_kv, int head_dim, cudaStream_t s) {
-    if (n_items <= 0) return cudaSuccess;
-    return launch_k(decode_merge_kernel, dim3(n_items), dim3(128), 0, s, items, part_o, part_ml, reinterpret_cast<uint16_t*>(out), n_heads, n_kv, head_dim);
 }
 
 template <int D>
@@ -309,7 +295,7 @@ static cudaError_t launch_decode_d(const CUtensorMap* tm_kv, const KvLayout& kv,
 
 cudaError_t launch_decode_attention(const CUtensorMap* tm_kv, const KvLayout& kv, const DecodeAttnParams& p, cudaStream_t s) {
     if (p.n_ctas <= 0) return cudaSuccess;
-    if (kv.page_size != PAGE || p.n_heads % p.n_kv != 0 || p.n_heads / p.n_kv > 8) return cudaErrorInvalidValue;
+    if (kv.page_size != PAGE || p.n_heads % p.n_kv != 0 || p.n_heads / p.n_kv > 8 || !p.merge_counters) return cudaErrorInvalidValue;
     if (kv.head_dim == 128) return launch_decode_d<128>(tm_kv, kv, p, s);
     if (kv.head_dim == 64) return launch_decode_d<64>(tm_kv, kv, p, s);
     return cudaErrorInvalidValue;

@@ -16,6 +16,7 @@
 #include "token_mask.hpp"
 #include "tokenizer.hpp"
 #include "model.hpp"
+#include "sk_consumers.cuh"
 #include "tokenizer.hpp"
 
 using namespace oa;
@@ -67,16 +68,21 @@ struct Packed {
 int rc_of(cudaError_t e) { return e == cudaSuccess ? OA_OK : OA_ERR_INTERNAL; }
 }  // namespace
 
-// materialise the deterministic fixed-order sum of stream-K partials as fp32 [M,N]
-__global__ void sk_reduce_f32_kernel(const StreamK sk, float* __restrict__ out, int M, int N) {
-    const int row = blockIdx.x;
-    for (int col = threadIdx.x; col < N; col += blockDim.x) {
-        const uint32_t tile = (uint32_t)col / (uint32_t)sk.bn, cc = (uint32_t)col - tile * (uint32_t)sk.bn;
-        uint32_t c_first, c_last;
-        sk_tile_ctas(sk, tile, c_first, c_last);
-        float acc = 0.f;
-        for (uint32_t c = c_first; c <= c_last; ++c) acc += sk.ws[((size_t)(c + tile) * sk.rows + row) * sk.bn + cc];
-        out[(size_t)row * N + col] = acc;
+// materialise the deterministic fixed-order sum of stream-K partials as fp32 [M,N]: 8 columns of a row per thread, every partial's loads in
+// flight together (a row per CTA with one column and one load at a time was latency-bound: 23 us for 32 x 6144, more than the product itself)
+__global__ void sk_reduce_f32_kernel(const StreamK sk, float* __restrict__ out, int N, int aligned) {
+    griddep_launch(); griddep_wait();
+    const int row = blockIdx.y, col = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
+    if (col >= N) return;
+    float acc[8];
+    sk_sum8(sk, row, col, acc);
+    float* o = out + (size_t)row * N + col;
+    if (aligned) {
+        reinterpret_cast<float4*>(o)[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+        reinterpret_cast<float4*>(o)[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) o[i] = acc[i];
     }
 }
 
@@ -91,7 +97,7 @@ int oa_k_gemm_streamk(const void* A, const void* B, int32_t M, int32_t N, int32_
     if (!ws.p) return OA_ERR_INTERNAL;
     StreamK sk = make_streamk((float*)ws.p, N, K, block_n, n_ctas, M);
     cudaError_t e = launch_gemm_streamk(&tmA, &tmB, M, N, K, sk, s);
-    if (e == cudaSuccess) { sk_reduce_f32_kernel<<<M, 256, 0, s>>>(sk, out_f32, M, N); e = cudaGetLastError(); }
+    if (e == cudaSuccess) e = launch_k(sk_reduce_f32_kernel, dim3((N / 8 + 127) / 128, M), dim3(128), 0, s, sk, out_f32, N, (int)(((uintptr_t)out_f32 & 15) == 0));
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     return rc_of(e);
 }
@@ -145,18 +151,19 @@ static int paged_attention(const void* q, void* out, const void* kv_cache, int32
         DecodePlan plan;
         build_decode_plan(ctx_lens, n_seqs, n_kv, 2 * 148, force_splits, plan);
         const size_t o_segs = host.add(plan.segs.data(), plan.segs.size() * sizeof(DecodeSeg)), o_ptr = host.add(plan.cta_ptr.data(), plan.cta_ptr.size() * 4);
-        const size_t o_merge = host.add(plan.merges.data(), plan.merges.size() * sizeof(MergeItem));
-        DevBuf d_meta(host.bytes.size(), s);
-        DevBuf d_po((size_t)(plan.n_slots + 1) * grp * head_dim * 4, s), d_pml((size_t)(plan.n_slots + 1) * grp * 2 * 4, s);
-        if (!d_meta.p || !d_po.p || !d_pml.p) return OA_ERR_INTERNAL;
+        const std::vector<int32_t> zeros(plan.merges.size() + 1, 0);
+        const size_t o_count = host.add(zeros.data(), zeros.size() * 4);         // merge counters: the CTA with an item's last piece merges it
+        const size_t o_po = (host.bytes.size() + 255) & ~size_t(255), o_pml = o_po + (size_t)(plan.n_slots + 1) * grp * head_dim * 4;
+        DevBuf d_meta(o_pml + (size_t)(plan.n_slots + 1) * grp * 2 * 4, s);       // [tables, plan, counters | partial outputs | partial maxima and sums]
+        if (!d_meta.p) return OA_ERR_INTERNAL;
         cudaMemcpyAsync(d_meta.p, host.bytes.data(), host.bytes.size(), cudaMemcpyHostToDevice, s);
         const char* meta = (const char*)d_meta.p;
         DecodeAttnParams a{}; a.q = q; a.out = out; a.block_tables = (const int32_t*)(meta + o_bt); a.ctx_lens = (const int32_t*)(meta + o_ctx);
         a.max_pages_per_seq = max_pages_per_seq; a.segs = (const DecodeSeg*)(meta + o_segs); a.cta_seg_ptr = (const int32_t*)(meta + o_ptr);
-        a.n_ctas = (int)plan.cta_ptr.size() - 1; a.part_o = (float*)d_po.p; a.part_ml = (float*)d_pml.p; a.layer = 0;
+        a.n_ctas = (int)plan.cta_ptr.size() - 1; a.part_o = (float*)(meta + o_po); a.part_ml = (float*)(meta + o_pml); a.layer = 0;
         a.n_heads = n_heads; a.n_kv = n_kv; a.scale_log2e = scale_log2e;
+        a.merge_counters = (int32_t*)((char*)d_meta.p + o_count);
         e = launch_decode_attention(&tm, kv, a, s);
-        if (e == cudaSuccess) e = launch_decode_merge((const MergeItem*)(meta + o_merge), (int)plan.merges.size(), a.part_o, a.part_ml, out, n_heads, n_kv, head_dim, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         return rc_of(e);
     }

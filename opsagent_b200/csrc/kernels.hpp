@@ -152,14 +152,12 @@ struct DecodeAttnParams {
     int32_t max_pages_per_seq;
     const DecodeSeg* segs; const int32_t* cta_seg_ptr; int32_t n_ctas;   // CTA c runs segs[ptr[c] .. ptr[c+1])
     float* part_o; float* part_ml; // partial workspace: [slots, group, D] fp32 and [slots, group, 2]
-    int32_t* merge_counters;       // [items], zero at the start of a step; the CTA that completes an item's last piece merges it (null: separate merge kernel)
+    int32_t* merge_counters;       // [items], zero at the start of a step; the CTA that completes an item's last piece merges it
     int32_t layer, n_heads, n_kv;
     float scale_log2e;             // (1/sqrt(D)) * log2(e)
 };
 cudaError_t launch_decode_attention(const CUtensorMap* tm_kv, const KvLayout& kv, const DecodeAttnParams& p, cudaStream_t s);
 struct MergeItem { int32_t seq, kvh, slot_begin, n_slots; };
-cudaError_t launch_decode_merge(const MergeItem* items, int n_items, const float* part_o, const float* part_ml, void* out,
-                                int n_heads, int n_kv, int head_dim, cudaStream_t s);
 
 constexpr int PREFILL_TILE_ROWS = 128;                     // query rows of one (tile, head) CTA
 struct PrefillTile { int32_t seq, q_row0, pos0, n_rows; };  // <= PREFILL_TILE_ROWS rows of one sequence; q_row0 = row in the token batch

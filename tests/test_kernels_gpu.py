@@ -310,3 +310,34 @@ def test_paged_prefill_attention_two_heads_per_cta(L, nh, nkv, D):
     # probabilities and result are rounded to bf16 (2^-9 relative each); |values| stay below 5
     err = (out.float() - ref).nan_to_num().abs().max().item()
     assert err < 2 * 5 * 2.0 ** -8, err
+
+
+# few long contexts: an item is cut over up to 37 CTAs and the last of them merges the pieces (one, two, several, more than four at a time)
+@pytest.mark.parametrize("ctx,nh,nkv,D", [([9000], 32, 8, 128), ([9001, 5, 70], 16, 2, 128), ([5000, 64], 32, 8, 64), ([700], 5, 1, 64), ([3333, 3334, 129], 40, 8, 128)])
+def test_paged_decode_attention_merges_many_pieces(L, ctx, nh, nkv, D):
+    n = len(ctx); maxp = (max(ctx) + 63) // 64; num_pages = sum((c + 63) // 64 for c in ctx)
+    kv = _mk_cache(num_pages, nkv, D, 17)
+    g = torch.Generator(device="cpu").manual_seed(6)
+    perm = torch.randperm(num_pages, generator=g)
+    bt = torch.zeros(n, maxp, dtype=torch.int32); k = 0
+    for i, c in enumerate(ctx):
+        npg = (c + 63) // 64; bt[i, :npg] = perm[k:k + npg].to(torch.int32); k += npg
+    q = (torch.randn(n, nh, D, generator=g) * 2).to(torch.bfloat16).to(dev())
+    out = torch.full((n, nh, D), float("nan"), dtype=torch.bfloat16, device=dev())
+    ctx_a = np.array(ctx, np.int32); bt_np = np.ascontiguousarray(bt.numpy())
+    for _ in range(2):
+        assert L.oa_k_paged_attention(ptr(q), ptr(out), ptr(kv), num_pages, bt_np.ctypes.data, maxp, ctx_a.ctypes.data, None, n, nh, nkv, D, 0, None) == 0, _lib.last_error()
+    ref = _attn_ref(q, kv[0], kv[1], bt.to(dev()).long(), ctx, [1] * n, nh, nkv, D)
+    # probabilities and result are rounded to bf16 (2^-9 relative each); |values| stay below 3
+    assert (out.float() - ref).abs().max().item() < 2 * 3 * 2.0 ** -8
+
+
+def test_streamk_result_on_any_float_boundary(L):
+    M, N, K = 37, 1000, 320
+    g = torch.Generator(device="cpu").manual_seed(1)
+    A = (torch.randn(M, K, generator=g) * 0.5).to(torch.bfloat16).to(dev()); B = (torch.randn(N, K, generator=g) * 0.5).to(torch.bfloat16).to(dev())
+    whole = torch.empty(M * N + 1, dtype=torch.float32, device=dev())
+    out = torch.empty(M, N, dtype=torch.float32, device=dev())
+    assert L.oa_k_gemm_streamk(ptr(A), ptr(B), M, N, K, 128, 148, ptr(out), None) == 0
+    assert L.oa_k_gemm_streamk(ptr(A), ptr(B), M, N, K, 128, 148, ptr(whole[1:]), None) == 0
+    assert torch.equal(whole[1:].view(M, N), out)
