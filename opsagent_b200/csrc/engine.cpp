@@ -202,6 +202,13 @@ public:
             const int V = model_.cfg.vocab;
             StepInput in; in.decode = false; in.want_logits = true;
             std::vector<std::shared_ptr<Seq>> batch; std::vector<int> take_of;
+            // Entries of one token are decoding rows: as in the scheduler's mixed steps they come first and go to the decode attention kernel, which
+            // reads a page once for all heads of its group and cuts long contexts over the chip (32 requests of 100 cached tokens, 32 / 8 heads of
+            // 128: 42 us a layer as query tiles of one row, 6 us as decoding rows).  Only where that kernel and its plan's buffers are made for it.
+            const ModelConfig& mc = model_.cfg;
+            int singles = 0;
+            for (int e = 0; e < n_entries; ++e) singles += n_tokens[e] == 1;
+            const bool decode_rows = !mc.hybrid && opt_.tp == 1 && (mc.head_dim == 64 || mc.head_dim == 128) && mc.n_heads / mc.n_kv_heads <= 8 && singles <= opt_.max_batch;
             {
                 std::lock_guard<std::mutex> lk(mu_);
                 if (fatal_) return fail(OA_ERR_INTERNAL, "engine is in a failed state: " + fatal_msg_);
@@ -223,16 +230,29 @@ public:
                     if ((int)s->tokens.size() > opt_.max_seq_len) return fail(OA_ERR_BAD_REQUEST, "request longer than max_seq_len");
                     const int need = ((int)s->tokens.size() + 63) / 64 - (int)s->pages.size();
                     if (need > 0 && !alloc_pages_locked(s->pages, need)) return fail(OA_ERR_OVERLOADED, "no free cache pages");
-                    const int row0 = (int)in.tokens.size();
-                    const int sidx = append_rows_locked(in, *s, s->n_cached, take);
-                    for (int r = 0; r < take; r += PREFILL_TILE_ROWS) in.tiles.push_back(PrefillTile{sidx, row0 + r, s->n_cached + r, std::min(PREFILL_TILE_ROWS, take - r)});
                     for (int k = 0; k < n_want[e]; ++k) {
                         const int wpos = want[want_at + k];
                         if (wpos < 0 || wpos >= take) return fail(OA_ERR_BAD_REQUEST, "wanted place outside the entry's tokens");
-                        in.sample_rows.push_back(row0 + wpos);
                     }
                     want_at += (size_t)n_want[e];
                     batch.push_back(s); take_of.push_back(take);
+                }
+                std::vector<int> row0_of(batch.size());
+                for (int pass = decode_rows ? 0 : 1; pass < 2; ++pass) {      // decoding rows, then the rest
+                    for (size_t b = 0; b < batch.size(); ++b) {
+                        Seq& s = *batch[b];
+                        const int take = take_of[b], row0 = (int)in.tokens.size();
+                        if (decode_rows && (take == 1) != (pass == 0)) continue;
+                        row0_of[b] = row0;
+                        const int sidx = append_rows_locked(in, s, s.n_cached, take);
+                        if (pass == 0) { in.n_decode = in.n_seqs; continue; }
+                        for (int r = 0; r < take; r += PREFILL_TILE_ROWS) in.tiles.push_back(PrefillTile{sidx, row0 + r, s.n_cached + r, std::min(PREFILL_TILE_ROWS, take - r)});
+                    }
+                }
+                want_at = 0;
+                for (size_t b = 0; b < batch.size(); ++b) {
+                    for (int k = 0; k < n_want[b]; ++k) in.sample_rows.push_back(row0_of[b] + want[want_at + k]);
+                    want_at += (size_t)n_want[b];
                 }
             }
             const size_t n_rows = in.sample_rows.size();

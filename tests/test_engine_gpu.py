@@ -756,3 +756,26 @@ def test_native_front_cancels_completions_of_clients_that_hang_up():
     es = eng.stats()
     assert es["running"] == 0 and es["waiting"] == 0 and es["pages_free"] >= es["pages_total"] - 16      # only prefix-cache pages of short prompts stay held
     front.shutdown(); eng.close()
+
+
+# trace_step: entries of one token are decoding rows wherever they stand among the entries of a step, and keep their place in the result
+@pytest.mark.parametrize("preset", ["tiny-llama-d128", "tiny-llama"])
+def test_trace_step_mixes_single_tokens_and_portions(preset):
+    spec = O.PRESETS[preset]
+    rng = np.random.default_rng(3)
+    seqs = [rng.integers(0, spec.vocab, n).tolist() for n in (150, 70, 1, 131)]
+    with Engine(spec.engine_json(num_pages=32, max_seq_len=256, max_batch=8, max_step_tokens=512)) as eng:
+        ref = [eng.debug_prefill_logits(s) for s in seqs]
+        got = [[] for _ in seqs]
+        at = [0] * 4
+        for takes in ([64, 1, 0, 130], [1, 68, 1, 1], [85, 1, 0, 0]):          # singles before, between and after portions; a request of one token
+            live = [i for i in range(4) if takes[i]]
+            end = [i for i in live if at[i] + takes[i] == len(seqs[i])]
+            out = eng.trace_step([(i, seqs[i][at[i]:at[i] + takes[i]], list(range(takes[i]))) for i in live], end)
+            k = 0
+            for i in live:
+                got[i].append(out[k:k + takes[i]]); k += takes[i]; at[i] += takes[i]
+        for i in range(4):
+            g = np.concatenate(got[i])
+            assert g.shape == ref[i].shape
+            assert np.abs(g - ref[i]).max() < 2.5e-2          # two kernels' roundings, as between the engine and the oracle
