@@ -49,8 +49,9 @@ struct DevBuf {
     void* p = nullptr;
     cudaStream_t s;
     DevBuf(size_t n, cudaStream_t stream) : s(stream) {
+        if (n == 0) return;
         cudaMemPool_t pool = scratch_pool();
-        if (!pool || cudaMallocFromPoolAsync(&p, n ? n : 16, pool, s) != cudaSuccess) p = nullptr;
+        if (!pool || cudaMallocFromPoolAsync(&p, n, pool, s) != cudaSuccess) p = nullptr;
     }
     DevBuf(const DevBuf&) = delete;
     ~DevBuf() { if (p) cudaFreeAsync(p, s); }
@@ -115,10 +116,17 @@ int oa_k_gemm(const void* A, const void* B, int32_t M, int32_t N, int32_t K, int
               const void* bias, const void* resid, float* logits, int32_t* argmax_out, void* stream) {
     cudaStream_t s = (cudaStream_t)stream;
     CUtensorMap tmA, tmB;
-    if (make_tmap_bf16_2d(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)K, 128, 64) != 0) return OA_ERR_INTERNAL;
-    if (make_tmap_bf16_2d(&tmB, B, (uint64_t)N, (uint64_t)K, (uint64_t)K, (uint32_t)block_n, 64) != 0) return OA_ERR_INTERNAL;
     GemmParams p{}; p.M = M; p.N = N; p.K = K; p.out = out; p.ldo = epilogue == EPI_SWIGLU ? N / 2 : N;
     p.bias = bias; p.resid = resid; p.ldr = N; p.logits = logits; p.ldl = N;
+    if (make_tmap_bf16_2d(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)K, 128, 64) != 0) return OA_ERR_INTERNAL;
+    // room for cut tiles, where this product has any
+    const bool cut = gemm_may_split(p, epilogue, block_n);
+    DevBuf ws(cut ? GEMM_SPLIT_WS_BYTES + GEMM_SPLIT_COUNTERS * 4 : 0, s);
+    if (cut && ws.p) {
+        p.split_ws = (float*)ws.p; p.split_count = (unsigned int*)((char*)ws.p + GEMM_SPLIT_WS_BYTES);
+        if (cudaMemsetAsync(p.split_count, 0, GEMM_SPLIT_COUNTERS * 4, s) != cudaSuccess) return OA_ERR_INTERNAL;
+    }
+    if (make_tmap_bf16_2d(&tmB, B, (uint64_t)N, (uint64_t)K, (uint64_t)K, (uint32_t)gemm_b_box(p, epilogue, block_n), 64) != 0) return OA_ERR_INTERNAL;
     if (epilogue == EPI_LOGITS) {
         const int nt = gemm_n_tiles(N, block_n);
         DevBuf av((size_t)M * nt * 4, s), ai((size_t)M * nt * 4, s);

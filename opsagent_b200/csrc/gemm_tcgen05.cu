@@ -17,6 +17,7 @@
 #include <cstdlib>
 
 #include "common.cuh"
+#include "gemm_epilogue.cuh"
 #include "kernels.hpp"
 #include "sk_consumers.cuh"
 
@@ -26,13 +27,6 @@ static constexpr int BLOCK_M = 128;
 static constexpr int BLOCK_K = 64;     // 64 bf16 = 128 B = one swizzle row
 static constexpr int UMMA_K = 16;
 static constexpr int GEMM_THREADS = 192;
-static constexpr int RASTER_GROUP_M = 16;
-
-OA_DEVINL float glu_row_scale(const GemmParams& p, int row) {
-    if (!p.row_scale) return 1.0f;
-    const int i = p.row_scale_idx[row];
-    return i >= 0 ? p.row_scale[i] : 0.0f;
-}
 
 template <int BN>
 struct GemmCfg {
@@ -317,12 +311,39 @@ static long long persistent_min_tiles();
 template <int EPI>
 static cudaError_t launch_persistent(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, cudaStream_t stream);
 
+// CTA-pair kernel or one of the kernels here, and whether the last round's tiles are cut: the least estimate of rounds x k blocks x time of a k block
+// plus what a launch costs besides.  Constants in us fitted to a sweep of 200 .. 8192 rows over the projections of the four model sizes: a k block
+// takes 0.345 in a pair (0.39 once more than two rounds run against the power cap), 0.42 in a 128 x 256 tile and 0.26 in a narrower one; outside the
+// k loop 11 and 8; cutting adds 16 (publishing and adding the pieces; 5 of it is the counters' memset of a single call).  E.g. 200 x 4096 x 4096: 64
+// tiles of 128 x 64 24 us, 16 pair tiles 32; 400 rows: 44 and 32.  Up to 128 rows half of a pair's rows would be padding.
+struct GemmChoice { bool pair; int split; };
+static GemmChoice gemm_choose(const GemmParams& p, int epilogue, int block_n, bool room) {
+    GemmChoice best{false, 1};
+    const int sms = sm_count_cached(), pairs = sms / 2;
+    if (epilogue == EPI_LOGITS || p.m_tile_group || p.M <= BLOCK_M || pairs < 1) return best;
+    auto up = [](long long a, long long b) { return (a + b - 1) / b; };
+    const double kb = (double)up(p.K, BLOCK_K);
+    double least = (double)up(up(p.N, block_n) * up(p.M, BLOCK_M), sms) * kb * (block_n >= 256 ? 0.42 : 0.26) + 8.0;
+    const long long tiles = up(p.N, 256) * up(p.M, 256), rest = tiles % pairs;
+    for (int s = 1; s <= (room ? 3 : 1); ++s) {
+        if (s > 1 && (rest == 0 || rest * s > GEMM_SPLIT_SLOTS || kb < 4 * s)) continue;
+        const double rounds = s == 1 ? (double)up(tiles, pairs) : (double)(tiles / pairs) + (double)up(rest * s, pairs) / s;
+        const double est = rounds * kb * (rounds > 2 ? 0.39 : 0.345) + 11.0 + (s > 1 ? 16.0 : 0.0);
+        if (est < least) { least = est; best = GemmChoice{true, s}; }
+    }
+    return best;
+}
+int gemm_b_box(const GemmParams& p, int epilogue, int block_n) { return gemm_choose(p, epilogue, block_n, p.split_ws && p.split_count).pair ? 128 : block_n; }
+bool gemm_may_split(const GemmParams& p, int epilogue, int block_n) { return gemm_choose(p, epilogue, block_n, true).split > 1; }
+
 cudaError_t launch_gemm(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epilogue, int block_n,
                         cudaStream_t stream) {
     if (p.M <= 0 || p.N <= 0 || p.K <= 0 || (p.N % 8) != 0 || (p.K % 8) != 0) return cudaErrorInvalidValue;
     if (epilogue == EPI_SWIGLU && (p.N % 32) != 0) return cudaErrorInvalidValue;
     // large-M (prefill) shapes with the widest tile go to the persistent kernel (epilogue overlapped with the next tile)
     if (epilogue == EPI_F32 && ((p.ldf % 4) != 0 || !p.f32_out)) return cudaErrorInvalidValue;
+    const GemmChoice choice = gemm_choose(p, epilogue, block_n, p.split_ws && p.split_count);
+    if (choice.pair) return launch_gemm_pair(tmA, tmB, p, epilogue, choice.split, sm_count_cached(), stream);
     if (block_n == 256 && epilogue != EPI_LOGITS && !persistent_disabled() &&
         (long long)((p.N + 255) / 256) * ((p.M + BLOCK_M - 1) / BLOCK_M) >= persistent_min_tiles()) {
         switch (epilogue) {
@@ -350,18 +371,9 @@ struct PersistCfg {
     static constexpr int BN = 256;
     static constexpr int A_BYTES = BLOCK_M * BLOCK_K * 2, B_BYTES = BN * BLOCK_K * 2, STAGE_BYTES = A_BYTES + B_BYTES;
     static constexpr int STAGES = 4;
-    static constexpr int EPI_ROW_FLOATS = 36, EPI_WARP_BYTES = 32 * EPI_ROW_FLOATS * 4;
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 4 * EPI_WARP_BYTES + 1024 + 256;
     static constexpr uint32_t TMEM_COLS = 512;
 };
-
-OA_DEVINL void raster_tile(int idx, int m_tiles, int n_tiles, int& m_blk, int& n_blk) {
-    const int per_band = RASTER_GROUP_M * n_tiles;
-    const int band = idx / per_band, within = idx - band * per_band;
-    const int m0 = band * RASTER_GROUP_M;
-    const int rows = (m_tiles - m0) < RASTER_GROUP_M ? (m_tiles - m0) : RASTER_GROUP_M;
-    m_blk = m0 + within % rows; n_blk = within / rows;
-}
 
 template <int EPI>
 __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_persistent_kernel(const __grid_constant__ CUtensorMap tmA,
@@ -372,7 +384,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_persistent_kernel(const 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     float* epi_smem = reinterpret_cast<float*>(smem + STAGES * Cfg::STAGE_BYTES);
-    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * Cfg::STAGE_BYTES + 4 * Cfg::EPI_WARP_BYTES);
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * Cfg::STAGE_BYTES + 4 * EPI_WARP_BYTES);
     uint64_t* empty_bar = full_bar + STAGES;
     uint64_t* acc_full = empty_bar + STAGES;
     uint64_t* acc_empty = acc_full + 2;
@@ -444,7 +456,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_persistent_kernel(const 
         }
     } else {
         const int q = warp & 3;
-        float* stage = epi_smem + (warp - 2) * (Cfg::EPI_WARP_BYTES / 4);
+        float* stage = epi_smem + (warp - 2) * (EPI_WARP_BYTES / 4);
         griddep_wait();
         int it = 0;
         for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++it) {
@@ -456,96 +468,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_persistent_kernel(const 
                 for (int i2 = 0; i2 < 2; ++i2) if (row_base + i2 * 16 + (lane >> 1) < p.M) glu_sc[i2] = glu_row_scale(p, row_base + i2 * 16 + (lane >> 1));
             mbar_wait(&acc_full[as], ((uint32_t)it >> 1) & 1);
             tcgen05_fence_after();
-#pragma unroll 1
-            for (int cc = 0; cc < BN; cc += 32) {
-                uint32_t v[32];
-                tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * BN + cc), v);
-                tmem_ld_wait();
-                const int col0 = n_blk * BN + cc;
-#pragma unroll
-                for (int j = 0; j < 32; j += 4)
-                    *reinterpret_cast<float4*>(stage + lane * Cfg::EPI_ROW_FLOATS + j) =
-                        make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
-                __syncwarp();
-                if (EPI == EPI_SWIGLU) {
-                    // chunk = 16 gate + 16 up columns -> 16 output features; lane = (row, 8-feature half)
-                    const int h = lane & 1;
-#pragma unroll
-                    for (int i2 = 0; i2 < 2; ++i2) {
-                        const int r = i2 * 16 + (lane >> 1), row = row_base + r;
-                        const float* sp = stage + r * Cfg::EPI_ROW_FLOATS + h * 8;
-                        const float4 g0 = *reinterpret_cast<const float4*>(sp), g1 = *reinterpret_cast<const float4*>(sp + 4);
-                        const float4 u0 = *reinterpret_cast<const float4*>(sp + 16), u1 = *reinterpret_cast<const float4*>(sp + 20);
-                        const float gg[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-                        const float uu[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
-                        float f[8];
-                        if (p.glu_limit > 0.f) {
-#pragma unroll
-                            for (int k = 0; k < 8; ++k) f[k] = clamped_glu_f32(gg[k] * glu_sc[i2], uu[k] * glu_sc[i2], p.glu_limit, p.glu_slope);
-                        } else if (p.glu_gelu) {
-#pragma unroll
-                            for (int k = 0; k < 8; ++k) f[k] = gelu_tanh_fast_f32(gg[k]) * uu[k];
-                        } else
-#pragma unroll
-                        for (int k = 0; k < 8; ++k) f[k] = __fdividef(gg[k], 1.0f + __expf(-gg[k])) * uu[k];
-                        if (row < p.M && col0 < p.N) {
-                            uint4 o; o.x = pack_bf16x2(f[0], f[1]); o.y = pack_bf16x2(f[2], f[3]); o.z = pack_bf16x2(f[4], f[5]); o.w = pack_bf16x2(f[6], f[7]);
-                            *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out) + (size_t)row * p.ldo + (col0 >> 1) + h * 8) = o;
-                        }
-                    }
-                } else {
-                    // lane = (row, 8-column group): 8 rows x 64 B per store instruction
-                    const int c8 = (lane & 3) * 8, col = col0 + c8;
-#pragma unroll
-                    for (int i4 = 0; i4 < 4; ++i4) {
-                        const int r = i4 * 8 + (lane >> 2), row = row_base + r;
-                        const float* sp = stage + r * Cfg::EPI_ROW_FLOATS + c8;
-                        const float4 a0 = *reinterpret_cast<const float4*>(sp), a1 = *reinterpret_cast<const float4*>(sp + 4);
-                        float f[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-                        if (EPI == EPI_F32) {
-                            if (row < p.M && col < p.N) {
-                                const float al = p.alpha == 0.f ? 1.f : p.alpha;
-                                float* op = p.f32_out + (size_t)row * p.ldf + col;
-                                float4 o0 = make_float4(f[0] * al, f[1] * al, f[2] * al, f[3] * al), o1 = make_float4(f[4] * al, f[5] * al, f[6] * al, f[7] * al);
-                                if (p.bias_f32) {
-                                    const float4 b0 = *reinterpret_cast<const float4*>(p.bias_f32 + col), b1 = *reinterpret_cast<const float4*>(p.bias_f32 + col + 4);
-                                    o0.x += b0.x; o0.y += b0.y; o0.z += b0.z; o0.w += b0.w; o1.x += b1.x; o1.y += b1.y; o1.z += b1.z; o1.w += b1.w;
-                                }
-                                if (p.f32_accumulate) {
-                                    const float4 r0 = *reinterpret_cast<const float4*>(op), r1 = *reinterpret_cast<const float4*>(op + 4);
-                                    o0.x += r0.x; o0.y += r0.y; o0.z += r0.z; o0.w += r0.w; o1.x += r1.x; o1.y += r1.y; o1.z += r1.z; o1.w += r1.w;
-                                }
-                                *reinterpret_cast<float4*>(op) = o0; *reinterpret_cast<float4*>(op + 4) = o1;
-                            }
-                        } else if (row < p.M && col < p.N) {
-                            if (EPI == EPI_STORE) {
-                                if (p.bias) {
-                                    const uint4 bb = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.bias) + col);
-                                    f[0] += bf16lo(bb.x); f[1] += bf16hi(bb.x); f[2] += bf16lo(bb.y); f[3] += bf16hi(bb.y);
-                                    f[4] += bf16lo(bb.z); f[5] += bf16hi(bb.z); f[6] += bf16lo(bb.w); f[7] += bf16hi(bb.w);
-                                }
-                                if (p.store_act == 1) {
-#pragma unroll
-                                    for (int k = 0; k < 8; ++k) { const float r = fmaxf(f[k], 0.f); f[k] = r * r; }
-                                } else if (p.store_act == 2) {
-#pragma unroll
-                                    for (int k = 0; k < 8; ++k) f[k] = gelu_tanh_f32(f[k]);
-                                } else if (p.store_act == 3 && col >= p.act_col0 && col < p.act_col1) {
-#pragma unroll
-                                    for (int k = 0; k < 8; ++k) f[k] = silu_fast_f32(f[k]);
-                                }
-                            } else {
-                                const uint4 rr = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.resid) + (size_t)row * p.ldr + col);
-                                f[0] += bf16lo(rr.x); f[1] += bf16hi(rr.x); f[2] += bf16lo(rr.y); f[3] += bf16hi(rr.y);
-                                f[4] += bf16lo(rr.z); f[5] += bf16hi(rr.z); f[6] += bf16lo(rr.w); f[7] += bf16hi(rr.w);
-                            }
-                            uint4 o; o.x = pack_bf16x2(f[0], f[1]); o.y = pack_bf16x2(f[2], f[3]); o.z = pack_bf16x2(f[4], f[5]); o.w = pack_bf16x2(f[6], f[7]);
-                            *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out) + (size_t)row * p.ldo + col) = o;
-                        }
-                    }
-                }
-                __syncwarp();
-            }
+            persist_epilogue<EPI>(p, stage, tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * BN), row_base, n_blk * BN, BN, lane, glu_sc, SplitTile{nullptr, 1, 0, 0});
             tcgen05_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&acc_empty[as]);

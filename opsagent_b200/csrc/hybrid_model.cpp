@@ -518,6 +518,7 @@ HybridModel::HybridModel(const ModelConfig& c, const EngineOptions& o) : ModelBa
         ld_gates_ = max_gates; gates_ = (float*)dmalloc(MR * ld_gates_ * 4);
         gin_ = (float*)dmalloc(MR * max_h * 4); floor_ = (float*)dmalloc(MR * max_h * 4); ndot_ = (float*)dmalloc(MR * max_h * 4);
     }
+    if (!f32_ && opt.hy_tensor_core) { gemm_split_ws_ = (float*)dmalloc(GEMM_SPLIT_WS_BYTES); gemm_split_count_ = (unsigned int*)dmalloc(GEMM_SPLIT_COUNTERS * 4); }
     hs_ = dmalloc((size_t)MS_ * Wld_ * es_); d_out_ids_ = (int32_t*)dmalloc((size_t)MS_ * 4);
     logits_ = (float*)dmalloc((size_t)opt.max_batch * V * 4);      // own logits: sampling steps only (one row per sequence)
     cuda_check(cudaMallocHost(&h_out_ids, (size_t)MS_ * 4), "cudaMallocHost");
@@ -598,11 +599,12 @@ void HybridModel::gemm(int mode, const void* A, int lda, const Mat& B, void* C, 
     CUtensorMap tmA;
     if (tc && make_tmap_bf16_2d(&tmA, A, (uint64_t)M, (uint64_t)B.ld, (uint64_t)lda, 128, 64) != 0) tc = false;
     if (!tc) { cuda_check(hy_gemm(f32_, mode, A, lda, B.p, B.ld, C, ldc, M, B.N, B.K, bias, alpha, 1, 0, 0, 0, stream, act), "gemm"); return; }
-    GemmParams g{}; g.M = M; g.N = up8(B.N); g.K = B.ld;
+    GemmParams g{}; g.M = M; g.N = up8(B.N); g.K = B.ld; g.split_ws = gemm_split_ws_; g.split_count = gemm_split_count_;
+    auto map = [&](int epi, int bn) { const int box = gemm_b_box(g, epi, bn); return &B.tm[box == 32 ? 0 : box == 64 ? 1 : box == 128 ? 2 : 3]; };
     const int bn = pick_tile_n(M, g.N, sm_count);
-    if (mode == HY_STORE) { g.out = C; g.ldo = ldc; g.bias = bias ? bias_act : nullptr; g.store_act = act.kind; g.act_col0 = act.col0; g.act_col1 = act.col1; cuda_check(launch_gemm(&tmA, &B.tm[bn == 32 ? 0 : bn == 64 ? 1 : bn == 128 ? 2 : 3], g, EPI_STORE, bn, stream), "gemm (tcgen05)"); return; }
+    if (mode == HY_STORE) { g.out = C; g.ldo = ldc; g.bias = bias ? bias_act : nullptr; g.store_act = act.kind; g.act_col0 = act.col0; g.act_col1 = act.col1; cuda_check(launch_gemm(&tmA, map(EPI_STORE, bn), g, EPI_STORE, bn, stream), "gemm (tcgen05)"); return; }
     g.f32_out = reinterpret_cast<float*>(C); g.ldf = ldc; g.f32_accumulate = mode == HY_ACC_F32; g.alpha = alpha; g.bias_f32 = bias;
-    cuda_check(launch_gemm(&tmA, &B.tm[bn == 32 ? 0 : bn == 64 ? 1 : bn == 128 ? 2 : 3], g, EPI_F32, bn, stream), "gemm (tcgen05, fp32 out)");
+    cuda_check(launch_gemm(&tmA, map(EPI_F32, bn), g, EPI_F32, bn, stream), "gemm (tcgen05, fp32 out)");
 }
 
 bool HybridModel::moe(const LayerW& w, const HyLayer& l, const void* h_in, const HyRows& r, const std::function<void(int)>& MARK, const int32_t* tokens, float beta) {
@@ -613,9 +615,9 @@ bool HybridModel::moe(const LayerW& w, const HyLayer& l, const void* h_in, const
     if (m.dense && m.act == HY_EXPERT_GELU_GLU) {        // gated: both halves in one product, gelu(gate) * up in its epilogue
         CUtensorMap tmA;
         if (w.up.tc && make_tmap_bf16_2d(&tmA, h_in, (uint64_t)T, (uint64_t)w.up.ld, (uint64_t)Wld_, 128, 64) == 0) {
-            GemmParams g{}; g.M = T; g.N = w.up.N; g.K = w.up.ld; g.out = act_; g.ldo = w.ffp; g.glu_gelu = 1;
-            const int bn = pick_tile_n(T, g.N, sm_count);
-            cuda_check(launch_gemm(&tmA, &w.up.tm[bn == 32 ? 0 : bn == 64 ? 1 : bn == 128 ? 2 : 3], g, EPI_SWIGLU, bn, stream), "gated feed-forward (tcgen05)");
+            GemmParams g{}; g.M = T; g.N = w.up.N; g.K = w.up.ld; g.out = act_; g.ldo = w.ffp; g.glu_gelu = 1; g.split_ws = gemm_split_ws_; g.split_count = gemm_split_count_;
+            const int bn = pick_tile_n(T, g.N, sm_count), box = gemm_b_box(g, EPI_SWIGLU, bn);
+            cuda_check(launch_gemm(&tmA, &w.up.tm[box == 32 ? 0 : box == 64 ? 1 : box == 128 ? 2 : 3], g, EPI_SWIGLU, bn, stream), "gated feed-forward (tcgen05)");
         } else {
             if (!glu_) throw std::runtime_error("tensor map for the feed-forward's input failed");
             gemm(HY_STORE, h_in, Wld_, w.up, glu_, ld_glu_, T, nullptr, 1.f);

@@ -41,12 +41,22 @@ struct GemmParams {
     // EPI_SWIGLU with glu_limit > 0: out = g sigmoid(glu_slope g) (u + 1), g = min(s gate, limit), u = clamp(s up, -limit, limit), where row r's s is
     // row_scale[row_scale_idx[r]] (0 for a negative index: a padding row of a grouped product) — the router's weight on an expert's input, exact in fp32
     float glu_limit, glu_slope; const float* row_scale; const int32_t* row_scale_idx;
+    // room for the fp32 partials of tiles whose k range is cut (GEMM_SPLIT_WS_BYTES) and their counters (GEMM_SPLIT_COUNTERS, zero between launches: the
+    // kernel re-arms them); null: tiles are never cut
+    float* split_ws; unsigned int* split_count;
     int glu_gelu;                   // EPI_SWIGLU: the gate passes the tanh form of GELU instead of SiLU
 };
-// tmA: box {64, 128} over A[M,K]; tmB: box {64, block_n} over B[N,K].  block_n in {32,64,128,256}.
+// tmA: box {64, 128} over A[M,K]; tmB: box {64, gemm_b_box(p, epilogue, block_n)} over B[N,K].  block_n in {32,64,128,256}.
 cudaError_t launch_gemm(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epilogue, int block_n,
                         cudaStream_t stream);
 int gemm_n_tiles(int N, int block_n);
+// rows of the B tensor map's box that launch_gemm(.., block_n, ..) reads for this product: block_n, or what the CTA-pair kernel takes where that runs
+int gemm_b_box(const GemmParams& p, int epilogue, int block_n);
+bool gemm_may_split(const GemmParams& p, int epilogue, int block_n);      // the product has tiles worth cutting if GemmParams::split_ws gives room
+// CTA-pair kernel (gemm_pair.cu): tiles of 256 x 256; tmB: box {64, 128}; split > 1: the last round's tiles are cut into that many ranges of k (2 or 3)
+cudaError_t launch_gemm_pair(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epilogue, int split, int sms, cudaStream_t stream);
+constexpr int GEMM_SPLIT_SLOTS = 148, GEMM_SPLIT_COUNTERS = GEMM_SPLIT_SLOTS * 8;      // pieces of cut tiles per launch; counters: one per tile, CTA and warp
+constexpr size_t GEMM_SPLIT_WS_BYTES = (size_t)GEMM_SPLIT_SLOTS * 256 * 256 * 4;
 // ---- stream-K variant for decode (M <= 128): persistent, one CTA per SM; work unit = (n_tile, 64-wide k block),
 // units dealt out contiguously so every SM streams the same number of weight bytes.  Each CTA writes the fp32
 // partial of every tile segment it owns to ws[slot = cta + tile][128][BN]; consumers (sk_* kernels) add a tile's

@@ -341,3 +341,40 @@ def test_streamk_result_on_any_float_boundary(L):
     assert L.oa_k_gemm_streamk(ptr(A), ptr(B), M, N, K, 128, 148, ptr(out), None) == 0
     assert L.oa_k_gemm_streamk(ptr(A), ptr(B), M, N, K, 128, 148, ptr(whole[1:]), None) == 0
     assert torch.equal(whole[1:].view(M, N), out)
+
+
+# CTA-pair kernel: whole tiles, tiles cut in two and in three (alone and behind a whole round), ragged last rows and columns, one CTA's rows all
+# beyond the last; every epilogue.  M, N, K chosen so that the rule takes each (2 or 3 pieces need a k range of some length).
+PAIR_CASES = [(300, 3072, 1024), (257, 6152, 320), (400, 2048, 8192), (614, 4096, 14336), (1337, 4096, 14336), (1000, 5120, 4160), (384, 296, 27648), (2000, 1000, 8192), (513, 2304, 72)]
+
+
+@pytest.mark.parametrize("M,N,K", PAIR_CASES)
+def test_gemm_cta_pairs(L, M, N, K):
+    g = torch.Generator(device=dev()).manual_seed(M + N + K)
+    A = torch.randn(M, K, generator=g, device=dev()).to(torch.bfloat16)
+    B = (torch.randn(N, K, generator=g, device=dev()) * 0.05).to(torch.bfloat16)
+    ref = A.double() @ B.double().T
+    bias = torch.randn(N, generator=g, device=dev()).to(torch.bfloat16)
+    # bf16 result: half an ulp (2^-9 relative) of the rounded value plus what fp32 sums of K products may be off by
+    def close(got, want, extra=0.0):
+        s = 0.05 * K ** 0.5 * K * 2.0 ** -24
+        assert torch.isfinite(got.float()).all()
+        assert ((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + s + extra + 1e-6).all(), float((got.double() - want).abs().max())
+    outs = []
+    for _ in range(2):                               # twice: counters must be zero again, and the order of summation is fixed
+        out = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=dev())
+        assert L.oa_k_gemm(ptr(A), ptr(B), M, N, K, EPI_STORE, 256, ptr(out), ptr(bias), None, None, None, None) == 0
+        torch.cuda.synchronize(); outs.append(out)
+    assert torch.equal(outs[0], outs[1])
+    close(outs[0], ref + bias.double())
+    x = torch.randn(M, N, generator=g, device=dev()).to(torch.bfloat16)
+    want = ref + x.double()
+    assert L.oa_k_gemm(ptr(A), ptr(B), M, N, K, EPI_RESID, 256, ptr(x), None, ptr(x), None, None, None) == 0       # in place
+    torch.cuda.synchronize()
+    close(x, want)
+    if N % 32 == 0:
+        y = torch.full((M, N // 2), float("nan"), dtype=torch.bfloat16, device=dev())
+        assert L.oa_k_gemm(ptr(A), ptr(B), M, N, K, EPI_SWIGLU, 256, ptr(y), None, None, None, None, None) == 0
+        torch.cuda.synchronize()
+        v = ref.view(M, N // 32, 2, 16)
+        close(y, (torch.nn.functional.silu(v[:, :, 0]) * v[:, :, 1]).reshape(M, N // 2), 2e-5 * float(v.abs().max()) ** 2)
