@@ -316,9 +316,24 @@ static cudaError_t launch_persistent(const CUtensorMap* tmA, const CUtensorMap* 
 // takes 0.345 in a pair (0.39 once more than two rounds run against the power cap), 0.42 in a 128 x 256 tile and 0.26 in a narrower one; outside the
 // k loop 11 and 8; cutting adds 16 (publishing and adding the pieces; 5 of it is the counters' memset of a single call).  E.g. 200 x 4096 x 4096: 64
 // tiles of 128 x 64 24 us, 16 pair tiles 32; 400 rows: 44 and 32.  Up to 128 rows half of a pair's rows would be padding.
-struct GemmChoice { bool pair; int split; };
+// Cluster size of the few-row kernel for this product, or 0: one of the kernels here takes it.  The largest that keeps the CTAs within 7/4 of the SMs
+// (two are resident on one; measured 16 .. 224 tiles of 128 weight rows).  Every row costs its exchange, S CTAs' worth, so with more rows it takes
+// more of a k range per CTA to pay: up to 16 rows always (28672 x 4096: 41 us against 42; 8192 x 2048: 9 against 17), up to 32 with four CTAs a
+// tile (6208 x 2048: 10.3 against 12.1; with two 12.6), up to 64 with eight, or with four from K = 4096 (6208 x 2048: 12.2 against 12.3; 6144 x 4096:
+// 17 against 21), up to 128 with four of K >= 4096 (4096 x 14336: 36 against 62; 2048 x 2048: 13 against 11).
+static int gemm_rows_split(const GemmParams& p, int epilogue) {
+    if (!p.few_rows_ok || epilogue == EPI_LOGITS || p.m_tile_group || gemm_rows_box(p.M) == 0) return 0;
+    const int tiles = (p.N + 127) / 128, kb = (p.K + BLOCK_K - 1) / BLOCK_K;
+    int s = p.M > 64 ? 4 : 8;
+    while (s > 1 && (tiles * s > sm_count_cached() * 7 / 4 || kb < 2 * s)) s >>= 1;
+    const bool pays = p.M <= 16 || (p.M <= 32 && s >= 4) || (p.M <= 64 && (s == 8 || (s == 4 && kb >= 64))) || (s == 4 && kb >= 64);
+    return pays ? s : 0;
+}
+struct GemmChoice { bool pair; int split, rows; };
 static GemmChoice gemm_choose(const GemmParams& p, int epilogue, int block_n, bool room) {
-    GemmChoice best{false, 1};
+    GemmChoice best{false, 1, 0};
+    best.rows = gemm_rows_split(p, epilogue);
+    if (best.rows) return best;
     const int sms = sm_count_cached(), pairs = sms / 2;
     if (epilogue == EPI_LOGITS || p.m_tile_group || p.M <= BLOCK_M || pairs < 1) return best;
     auto up = [](long long a, long long b) { return (a + b - 1) / b; };
@@ -329,11 +344,15 @@ static GemmChoice gemm_choose(const GemmParams& p, int epilogue, int block_n, bo
         if (s > 1 && (rest == 0 || rest * s > GEMM_SPLIT_SLOTS || kb < 4 * s)) continue;
         const double rounds = s == 1 ? (double)up(tiles, pairs) : (double)(tiles / pairs) + (double)up(rest * s, pairs) / s;
         const double est = rounds * kb * (rounds > 2 ? 0.39 : 0.345) + 11.0 + (s > 1 ? 16.0 : 0.0);
-        if (est < least) { least = est; best = GemmChoice{true, s}; }
+        if (est < least) { least = est; best = GemmChoice{true, s, 0}; }
     }
     return best;
 }
-int gemm_b_box(const GemmParams& p, int epilogue, int block_n) { return gemm_choose(p, epilogue, block_n, p.split_ws && p.split_count).pair ? 128 : block_n; }
+int gemm_b_box(const GemmParams& p, int epilogue, int block_n) {
+    const GemmChoice c = gemm_choose(p, epilogue, block_n, p.split_ws && p.split_count);
+    return c.pair || c.rows ? 128 : block_n;
+}
+int gemm_a_box(const GemmParams& p, int epilogue, int block_n) { return gemm_choose(p, epilogue, block_n, false).rows ? gemm_rows_box(p.M) : 128; }
 bool gemm_may_split(const GemmParams& p, int epilogue, int block_n) { return gemm_choose(p, epilogue, block_n, true).split > 1; }
 
 cudaError_t launch_gemm(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epilogue, int block_n,
@@ -343,6 +362,7 @@ cudaError_t launch_gemm(const CUtensorMap* tmA, const CUtensorMap* tmB, const Ge
     // large-M (prefill) shapes with the widest tile go to the persistent kernel (epilogue overlapped with the next tile)
     if (epilogue == EPI_F32 && ((p.ldf % 4) != 0 || !p.f32_out)) return cudaErrorInvalidValue;
     const GemmChoice choice = gemm_choose(p, epilogue, block_n, p.split_ws && p.split_count);
+    if (choice.rows) return launch_gemm_rows(tmA, tmB, p, epilogue, choice.rows, stream);
     if (choice.pair) return launch_gemm_pair(tmA, tmB, p, epilogue, choice.split, sm_count_cached(), stream);
     if (block_n == 256 && epilogue != EPI_LOGITS && !persistent_disabled() &&
         (long long)((p.N + 255) / 256) * ((p.M + BLOCK_M - 1) / BLOCK_M) >= persistent_min_tiles()) {

@@ -44,15 +44,22 @@ struct GemmParams {
     // room for the fp32 partials of tiles whose k range is cut (GEMM_SPLIT_WS_BYTES) and their counters (GEMM_SPLIT_COUNTERS, zero between launches: the
     // kernel re-arms them); null: tiles are never cut
     float* split_ws; unsigned int* split_count;
+    int few_rows_ok;                // the caller's A map has the box gemm_a_box() asks for (else 128 rows)
     int glu_gelu;                   // EPI_SWIGLU: the gate passes the tanh form of GELU instead of SiLU
 };
-// tmA: box {64, 128} over A[M,K]; tmB: box {64, gemm_b_box(p, epilogue, block_n)} over B[N,K].  block_n in {32,64,128,256}.
+// tmA: box {64, 128} over A[M,K] (few_rows_ok: {64, gemm_a_box(p, epilogue, block_n)}); tmB: box {64, gemm_b_box(p, epilogue, block_n)} over B[N,K].  block_n in {32,64,128,256}.
 cudaError_t launch_gemm(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epilogue, int block_n,
                         cudaStream_t stream);
 int gemm_n_tiles(int N, int block_n);
 // rows of the B tensor map's box that launch_gemm(.., block_n, ..) reads for this product: block_n, or what the CTA-pair kernel takes where that runs
 int gemm_b_box(const GemmParams& p, int epilogue, int block_n);
 bool gemm_may_split(const GemmParams& p, int epilogue, int block_n);      // the product has tiles worth cutting if GemmParams::split_ws gives room
+// rows of the A tensor map's box that launch_gemm reads for this product: 128, or what the few-row kernel takes where that runs (only with few_rows_ok)
+int gemm_a_box(const GemmParams& p, int epilogue, int block_n);
+// few-row kernel (gemm_rows.cu), M <= 128: weights in the tensor core's rows, a cluster of S = 1, 2, 4 or 8 CTAs per 128 weight rows; tmA: box {64,
+// gemm_rows_box(M)}, tmB: box {64, 128}
+inline int gemm_rows_box(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 0; }
+cudaError_t launch_gemm_rows(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epilogue, int S, cudaStream_t stream);
 // CTA-pair kernel (gemm_pair.cu): tiles of 256 x 256; tmB: box {64, 128}; split > 1: the last round's tiles are cut into that many ranges of k (2 or 3)
 cudaError_t launch_gemm_pair(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epilogue, int split, int sms, cudaStream_t stream);
 constexpr int GEMM_SPLIT_SLOTS = 148, GEMM_SPLIT_COUNTERS = GEMM_SPLIT_SLOTS * 8;      // pieces of cut tiles per launch; counters: one per tile, CTA and warp

@@ -378,3 +378,39 @@ def test_gemm_cta_pairs(L, M, N, K):
         torch.cuda.synchronize()
         v = ref.view(M, N // 32, 2, 16)
         close(y, (torch.nn.functional.silu(v[:, :, 0]) * v[:, :, 1]).reshape(M, N // 2), 2e-5 * float(v.abs().max()) ** 2)
+
+
+# few-row kernel: every row tile, clusters of 1, 2, 4 and 8 CTAs, ragged rows and columns, k ranges that do not divide evenly; every epilogue
+ROWS_CASES = [(1, 1024, 1088), (3, 2048, 4096), (16, 28672, 320), (17, 4096, 2056), (16, 9000, 1024), (32, 6144, 4160), (33, 2048, 1024), (64, 1000, 8192), (50, 6208, 4096), (65, 2048, 4096), (128, 4096, 4160), (100, 296, 14336)]
+
+
+@pytest.mark.parametrize("M,N,K", ROWS_CASES)
+def test_gemm_few_rows(L, M, N, K):
+    g = torch.Generator(device=dev()).manual_seed(M + N + K)
+    A = torch.randn(M, K, generator=g, device=dev()).to(torch.bfloat16)
+    B = (torch.randn(N, K, generator=g, device=dev()) * 0.05).to(torch.bfloat16)
+    ref = A.double() @ B.double().T
+    bias = torch.randn(N, generator=g, device=dev()).to(torch.bfloat16)
+    # bf16 result: half an ulp (2^-9 relative) of the rounded value plus what fp32 sums of K products may be off by
+    def close(got, want, extra=0.0):
+        s = 0.05 * K ** 0.5 * K * 2.0 ** -24
+        assert torch.isfinite(got.float()).all()
+        assert ((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + s + extra + 1e-6).all(), float((got.double() - want).abs().max())
+    outs = []
+    for use_bias in (True, True, False):
+        out = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=dev())
+        assert L.oa_k_gemm(ptr(A), ptr(B), M, N, K, EPI_STORE, 128, ptr(out), ptr(bias) if use_bias else None, None, None, None, None) == 0
+        torch.cuda.synchronize(); outs.append(out)
+    assert torch.equal(outs[0], outs[1])             # a fixed order of summation
+    close(outs[0], ref + bias.double()); close(outs[2], ref)
+    x = torch.randn(M, N, generator=g, device=dev()).to(torch.bfloat16)
+    want = ref + x.double()
+    assert L.oa_k_gemm(ptr(A), ptr(B), M, N, K, EPI_RESID, 128, ptr(x), None, ptr(x), None, None, None) == 0
+    torch.cuda.synchronize()
+    close(x, want)
+    if N % 32 == 0:
+        y = torch.full((M, N // 2), float("nan"), dtype=torch.bfloat16, device=dev())
+        assert L.oa_k_gemm(ptr(A), ptr(B), M, N, K, EPI_SWIGLU, 128, ptr(y), None, None, None, None, None) == 0
+        torch.cuda.synchronize()
+        v = ref.view(M, N // 32, 2, 16)
+        close(y, (torch.nn.functional.silu(v[:, :, 0]) * v[:, :, 1]).reshape(M, N // 2), 2e-5 * float(v.abs().max()) ** 2)
