@@ -397,6 +397,167 @@ __global__ void __launch_bounds__(128) hy_mla_attention_mma_kernel(HyLatentAttn 
 }
 
 // joins the parts of a decoding row: out = sum_p 2^(m_p - M) O_p / sum_p 2^(m_p - M) l_p, parts in order
+// ---------------------------------------------------------------------------------------------------------------------------------
+// the same for ONE row of a sequence with at most 16 heads (a decoding row): its queries fill one warp's 16 mma rows, so the four warps take
+// turns at groups of 16 cache rows instead, each with an online softmax and accumulators of its own, joined once at the end.  Cache rows come
+// by one bulk copy each into a ring per warp: no warp waits for another before the join.  What bounds it is the chain of a warp's groups.
+// 16 rows of 170 cached tokens, 16 heads of a 512 + 64 wide latent: 60 -> 18 us against the 64-query tile, of which three warps idled.
+// ---------------------------------------------------------------------------------------------------------------------------------
+constexpr int MLA_DQ = 16;
+static size_t mla_decode_smem(int E, int nvb, int stages) {
+    const size_t ring = (size_t)4 * stages * 16 * (E + 8) * 2, join = (size_t)4 * 16 * nvb * 8 * 4;
+    return (size_t)MLA_DQ * (E + 8) * 2 + std::max(ring, join) + 4 * 16 * 2 * 4 + 4 * 2 * 8;
+}
+template <int NVB, int STAGES>
+__global__ void __launch_bounds__(128) hy_mla_decode_mma_kernel(HyLatentAttn a, const float* __restrict__ q_abs, const __nv_bfloat16* __restrict__ cache,
+                                                                __nv_bfloat16* __restrict__ lat_out, HyRows r, const int32_t* __restrict__ tile_seq, HyMlaSplit sp) {
+    HY_PDL();
+    extern __shared__ __align__(16) uint8_t mla_smem[];
+    const int R = a.kv_rank, E = R + a.rot_dim, EP = E + 8, H = a.heads;
+    __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(mla_smem);      // [16][EP]
+    __nv_bfloat16* ring = Qs + MLA_DQ * EP;                              // [4 warps][STAGES][16][EP]
+    float* join = reinterpret_cast<float*>(ring);                        // after the last group: [4 warps][16][NVB * 8]
+    const size_t ring_b = (size_t)4 * STAGES * 16 * EP * 2, join_b = (size_t)4 * 16 * NVB * 8 * 4;
+    float* ml = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(ring) + (ring_b > join_b ? ring_b : join_b));      // [4 warps][16][2]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(ml + 4 * 16 * 2);       // [4 warps][2]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int seq = tile_seq[blockIdx.x], vbase = blockIdx.y * NVB * 8, row = r.seq_row0[seq], pos = r.positions[row];
+    const int k0 = sp.tile_k0 ? sp.tile_k0[blockIdx.x] : 0, k1 = sp.tile_k0 ? sp.tile_k1[blockIdx.x] : 0, slot = sp.tile_k0 ? sp.tile_slot[blockIdx.x] : -1;
+    const int win = a.window > 0 ? a.window : 0x40000000;
+    const int last = k1 > 0 ? min(pos, k1 - 1) : pos, first = max(max(k0, pos - win + 1), 0);      // the cache rows this CTA walks
+    const int g_begin = first / 16 + warp, g_end = last / 16 + 1;
+    const int32_t* bt = r.block_tables + (long long)seq * r.max_pages_per_seq;
+    __nv_bfloat16* my = ring + (size_t)warp * STAGES * 16 * EP;
+    uint64_t* bar = bars + warp * 2;
+    if (lane == 0) { for (int s = 0; s < STAGES; ++s) mbar_init(&bar[s], 1); fence_barrier_init(); }
+    __syncwarp();
+    auto issue = [&](int g, int st) {               // group g into stage st: rows behind the last are zeroed (their weights are zero, stale bits need not be finite)
+        const int n = min(16, last - g * 16 + 1);
+        if (lane == 0) mbar_expect_tx(&bar[st], (uint32_t)(n * E * 2));
+        __syncwarp();
+        __nv_bfloat16* dst = my + st * 16 * EP;
+        if (lane < n)
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                         ::"r"(smem_u32(dst + lane * EP)), "l"(cache + ((long long)bt[g >> 2] * 64 + (g & 3) * 16 + lane) * E), "r"((uint32_t)(E * 2)), "r"(smem_u32(&bar[st])) : "memory");
+        for (int j = n; j < 16; ++j) for (int c = lane; c < E / 8; c += 32) *reinterpret_cast<uint4*>(dst + j * EP + c * 8) = make_uint4(0, 0, 0, 0);
+        __syncwarp();
+    };
+    for (int s = 0; s < STAGES; ++s) if (g_begin + 4 * s < g_end) issue(g_begin + 4 * s, s);
+    const float qscale = a.scale * 1.4426950408889634f;
+    const int e4 = E / 4;
+#pragma unroll 6
+    for (int idx = tid; idx < MLA_DQ * e4; idx += 128) {
+        const int qi = idx / e4, e = (idx - qi * e4) * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (qi < H) v = *reinterpret_cast<const float4*>(q_abs + ((long long)row * H + qi) * E + e);
+        *reinterpret_cast<uint2*>(Qs + qi * EP + e) = make_uint2(pack_bf16x2(v.x * qscale, v.y * qscale), pack_bf16x2(v.z * qscale, v.w * qscale));
+    }
+    __syncthreads();
+    float o[NVB][4];
+#pragma unroll
+    for (int i = 0; i < NVB; ++i) { o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f; }
+    float m_lo = -INFINITY, m_hi = -INFINITY, l_lo = 0.f, l_hi = 0.f;
+    int st = 0; uint32_t ph = 0;
+    for (int g = g_begin; g < g_end; g += 4) {
+        mbar_wait(&bar[st], ph);
+        const __nv_bfloat16* Kb = my + st * 16 * EP;
+        float s[2][2][4];                           // even and odd k steps apart: two chains
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) { s[i][j][0] = s[i][j][1] = s[i][j][2] = s[i][j][3] = 0.f; }
+        const uint32_t qa = smem_u32(Qs + (lane & 15) * EP + (lane >> 4) * 8);
+        const uint32_t ka = smem_u32(Kb + ((lane >> 4) * 8 + (lane & 7)) * EP + ((lane >> 3) & 1) * 8);
+#pragma unroll 4
+        for (int ks = 0; ks < E / 16; ++ks) {
+            uint32_t a0, a1, a2, a3, b0, b1, b2, b3;
+            ldmatrix_x4(qa + ks * 32, a0, a1, a2, a3);
+            ldmatrix_x4(ka + ks * 32, b0, b1, b2, b3);
+            if (ks & 1) { mma_bf16_16816(s[1][0], a0, a1, a2, a3, b0, b1); mma_bf16_16816(s[1][1], a0, a1, a2, a3, b2, b3); }
+            else { mma_bf16_16816(s[0][0], a0, a1, a2, a3, b0, b1); mma_bf16_16816(s[0][1], a0, a1, a2, a3, b2, b3); }
+        }
+        float mx_lo = -INFINITY, mx_hi = -INFINITY;
+#pragma unroll
+        for (int nb = 0; nb < 2; ++nb)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int key = g * 16 + nb * 8 + (lane & 3) * 2 + (c & 1);
+                s[0][nb][c] = key > last || key < first ? -INFINITY : s[0][nb][c] + s[1][nb][c];
+                if (c < 2) mx_lo = fmaxf(mx_lo, s[0][nb][c]); else mx_hi = fmaxf(mx_hi, s[0][nb][c]);
+            }
+        mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 1)); mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 2));
+        mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 1)); mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 2));
+        const float t_lo = fmaxf(m_lo, mx_lo), t_hi = fmaxf(m_hi, mx_hi);
+        const float n_lo = t_lo == -INFINITY ? 0.f : t_lo, n_hi = t_hi == -INFINITY ? 0.f : t_hi;
+        const float c_lo = exp2f(m_lo - n_lo), c_hi = exp2f(m_hi - n_hi);
+        m_lo = t_lo; m_hi = t_hi;
+        float sum_lo = 0.f, sum_hi = 0.f;
+#pragma unroll
+        for (int nb = 0; nb < 2; ++nb) {
+            s[0][nb][0] = exp2f(s[0][nb][0] - n_lo); s[0][nb][1] = exp2f(s[0][nb][1] - n_lo); s[0][nb][2] = exp2f(s[0][nb][2] - n_hi); s[0][nb][3] = exp2f(s[0][nb][3] - n_hi);
+            sum_lo += s[0][nb][0] + s[0][nb][1]; sum_hi += s[0][nb][2] + s[0][nb][3];
+        }
+        l_lo = l_lo * c_lo + sum_lo; l_hi = l_hi * c_hi + sum_hi;
+        const uint32_t p0 = pack_bf16x2(s[0][0][0], s[0][0][1]), p1 = pack_bf16x2(s[0][0][2], s[0][0][3]), p2 = pack_bf16x2(s[0][1][0], s[0][1][1]), p3 = pack_bf16x2(s[0][1][2], s[0][1][3]);
+        const uint32_t va = smem_u32(Kb + (((lane >> 3) & 1) * 8 + (lane & 7)) * EP + vbase + (lane >> 4) * 8);
+#pragma unroll
+        for (int np = 0; np < NVB / 2; ++np) {
+            uint32_t b0, b1, b2, b3;
+            ldmatrix_x4_trans(va + np * 32, b0, b1, b2, b3);
+            o[2 * np][0] *= c_lo; o[2 * np][1] *= c_lo; o[2 * np][2] *= c_hi; o[2 * np][3] *= c_hi;
+            o[2 * np + 1][0] *= c_lo; o[2 * np + 1][1] *= c_lo; o[2 * np + 1][2] *= c_hi; o[2 * np + 1][3] *= c_hi;
+            mma_bf16_16816(o[2 * np], p0, p1, p2, p3, b0, b1); mma_bf16_16816(o[2 * np + 1], p0, p1, p2, p3, b2, b3);
+        }
+        __syncwarp();                               // every lane is done with the stage
+        if (g + 4 * STAGES < g_end) issue(g + 4 * STAGES, st);
+        if (++st == STAGES) { st = 0; ph ^= 1; }
+    }
+    l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 1); l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 2);
+    l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 1); l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 2);
+    __syncthreads();                                // the rings are free
+    {
+        const int q_lo = lane >> 2;
+        float* dst = join + ((size_t)warp * 16 + q_lo) * (NVB * 8) + (lane & 3) * 2;
+#pragma unroll
+        for (int nb = 0; nb < NVB; ++nb) {
+            *reinterpret_cast<float2*>(dst + nb * 8) = make_float2(o[nb][0], o[nb][1]);
+            *reinterpret_cast<float2*>(dst + 8 * NVB * 8 + nb * 8) = make_float2(o[nb][2], o[nb][3]);
+        }
+        if ((lane & 3) == 0) {
+            ml[(warp * 16 + q_lo) * 2] = m_lo; ml[(warp * 16 + q_lo) * 2 + 1] = l_lo;
+            ml[(warp * 16 + q_lo + 8) * 2] = m_hi; ml[(warp * 16 + q_lo + 8) * 2 + 1] = l_hi;
+        }
+    }
+    __syncthreads();
+    for (int idx = tid; idx < H * NVB * 2; idx += 128) {        // four channels of one head
+        const int h = idx / (NVB * 2), c = (idx - h * (NVB * 2)) * 4;
+        float M = -INFINITY, l = 0.f;
+#pragma unroll
+        for (int w = 0; w < 4; ++w) M = fmaxf(M, ml[(w * 16 + h) * 2]);
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {                            // warp order: a fixed order of summation
+            const float mw = ml[(w * 16 + h) * 2], f = mw == -INFINITY ? 0.f : exp2f(mw - M);
+            const float4 u = *reinterpret_cast<const float4*>(join + ((size_t)w * 16 + h) * (NVB * 8) + c);
+            l += f * ml[(w * 16 + h) * 2 + 1];
+            v.x += f * u.x; v.y += f * u.y; v.z += f * u.z; v.w += f * u.w;
+        }
+        if (slot >= 0) {                                         // partial of a row whose cache rows are cut into parts
+            *reinterpret_cast<float4*>(sp.ws_o + ((long long)slot * H + h) * R + vbase + c) = v;
+            if (blockIdx.y == 0 && c == 0) { sp.ws_ml[((long long)slot * H + h) * 2] = M; sp.ws_ml[((long long)slot * H + h) * 2 + 1] = l; }
+            continue;
+        }
+        float up = 1.f;
+        if (a.sink) {                                            // the sink joins the denominator (scores are kept in base-2 units)
+            const float s2 = a.sink[h] * 1.4426950408889634f, T = fmaxf(M, s2);
+            up = M == -INFINITY ? 0.f : exp2f(M - T); l = l * up + exp2f(s2 - T);
+        }
+        float inv = l > 0.f ? up / l : 0.f;
+        if (a.head_gate) inv *= sigmoidf_(ldf(reinterpret_cast<const __nv_bfloat16*>(a.head_gate) + (long long)row * a.ldg + h));
+        *reinterpret_cast<uint2*>(lat_out + ((long long)row * H + h) * R + vbase + c) = make_uint2(pack_bf16x2(v.x * inv, v.y * inv), pack_bf16x2(v.z * inv, v.w * inv));
+    }
+}
+
 __global__ void __launch_bounds__(128) hy_mla_merge_kernel(const int32_t* item_row, const int32_t* item_slot0, const int32_t* item_parts, const float* ws_o,
                                                            const float* ws_ml, __nv_bfloat16* lat_out, int H, int R, const float* sink,
                                                            const __nv_bfloat16* head_gate, int ldg) {
@@ -1331,6 +1492,31 @@ static cudaError_t mla_mma_launch(const HyLatentAttn& a, const float* q_abs, con
     return launch_plain(hy_mla_attention_mma_kernel<NVB, KT>, grid, dim3(128), mla_mma_smem(a.kv_rank + a.rot_dim, KT), s, a, q_abs, (const bf*)cache, (bf*)lat_out, r,
                         tile_seq, tile_q0, sp);
 }
+// rows of one token with up to 16 heads, where the four warps' rings fit an SM (two stages, else one)
+static int mla_decode_stages(const HyLatentAttn& a) {
+    const int nvb = mla_mma_nvb(a), E = a.kv_rank + a.rot_dim;
+    if (!nvb || a.heads > MLA_DQ) return 0;
+    return mla_decode_smem(E, nvb, 2) <= 200 * 1024 ? 2 : mla_decode_smem(E, nvb, 1) <= 200 * 1024 ? 1 : 0;
+}
+bool hy_mla_decode_supported(const HyLatentAttn& a) { return mla_decode_stages(a) != 0; }
+template <int NVB, int STAGES>
+static cudaError_t mla_decode_launch(const HyLatentAttn& a, const float* q_abs, const void* cache, void* lat_out, const HyRows& r, const int32_t* tile_seq, int n_tiles,
+                                     const HyMlaSplit& sp, cudaStream_t s) {
+    static bool done[16] = {};
+    cudaError_t e = ensure_dynamic_smem(hy_mla_decode_mma_kernel<NVB, STAGES>, 200 * 1024, done);      // set once per device: the most any size asks for
+    if (e != cudaSuccess) return e;
+    return launch_plain(hy_mla_decode_mma_kernel<NVB, STAGES>, dim3(n_tiles, a.kv_rank / (NVB * 8)), dim3(128), mla_decode_smem(a.kv_rank + a.rot_dim, NVB, STAGES), s, a, q_abs,
+                        (const bf*)cache, (bf*)lat_out, r, tile_seq, sp);
+}
+cudaError_t hy_mla_decode_mma(const HyLatentAttn& a, const float* q_abs, const void* cache, void* lat_out, const HyRows& r, const int32_t* tile_seq, int n_tiles,
+                              const HyMlaSplit& sp, cudaStream_t s) {
+    if (n_tiles <= 0) return cudaSuccess;
+    const int nvb = mla_mma_nvb(a), stages = mla_decode_stages(a);
+    if (!stages) return cudaErrorInvalidValue;
+#define HY_MLD(NVB) (stages == 2 ? mla_decode_launch<NVB, 2>(a, q_abs, cache, lat_out, r, tile_seq, n_tiles, sp, s) : mla_decode_launch<NVB, 1>(a, q_abs, cache, lat_out, r, tile_seq, n_tiles, sp, s))
+    return nvb == 32 ? HY_MLD(32) : nvb == 16 ? HY_MLD(16) : HY_MLD(8);
+#undef HY_MLD
+}
 cudaError_t hy_mla_merge(const int32_t* item_row, const int32_t* item_slot0, const int32_t* item_parts, int n_items, const float* ws_o, const float* ws_ml, void* lat_out,
                          int heads, int kv_rank, cudaStream_t s, const float* sink, const void* head_gate, int ldg) {
     if (n_items <= 0) return cudaSuccess;
@@ -1339,6 +1525,7 @@ cudaError_t hy_mla_merge(const int32_t* item_row, const int32_t* item_slot0, con
 cudaError_t hy_mla_attention_mma(const HyLatentAttn& a, const float* q_abs, const void* cache, void* lat_out, const HyRows& r, const int32_t* tile_seq,
                                  const int32_t* tile_q0, int n_tiles, const HyMlaSplit& sp, cudaStream_t s) {
     const int nvb = mla_mma_nvb(a), E = a.kv_rank + a.rot_dim;
+    if (n_tiles <= 0) return cudaSuccess;
     if (!nvb) return cudaErrorInvalidValue;
     // 32-row tiles when two CTAs (8 warps) still fit an SM's shared memory or nothing smaller would make them fit; else 16-row tiles
     // (a step with few tiles — decoding — is a latency chain per CTA: the larger tile halves its length)

@@ -147,6 +147,10 @@ struct HyMlaSplit { const int32_t* tile_k0; const int32_t* tile_k1; const int32_
 bool hy_mla_mma_supported(const HyLatentAttn& a);
 cudaError_t hy_mla_attention_mma(const HyLatentAttn& a, const float* q_abs, const void* cache, void* lat_out, const HyRows& r, const int32_t* tile_seq,
                                  const int32_t* tile_q0, int n_tiles, const HyMlaSplit& sp, cudaStream_t s);
+// rows of one token (tile_seq: their sequences), up to 16 heads, sizes whose rings fit: four warps split a row's cache rows
+bool hy_mla_decode_supported(const HyLatentAttn& a);
+cudaError_t hy_mla_decode_mma(const HyLatentAttn& a, const float* q_abs, const void* cache, void* lat_out, const HyRows& r, const int32_t* tile_seq, int n_tiles,
+                              const HyMlaSplit& sp, cudaStream_t s);
 cudaError_t hy_mla_merge(const int32_t* item_row, const int32_t* item_slot0, const int32_t* item_parts, int n_items, const float* ws_o, const float* ws_ml, void* lat_out,
                          int heads, int kv_rank, cudaStream_t s, const float* sink = nullptr, const void* head_gate = nullptr, int ldg = 0);
 

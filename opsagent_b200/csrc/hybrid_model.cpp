@@ -817,7 +817,10 @@ void HybridModel::latent_mixer(const HyRun& run, const HyLayer& l, const LayerW&
         if (tl.mma) {
             HyMlaSplit sp{nullptr, nullptr, nullptr, split_o_, split_ml_};
             if (tl.n_merge > 0) { sp.tile_k0 = d_meta_ + tl.o_k0; sp.tile_k1 = d_meta_ + tl.o_k1; sp.tile_slot = d_meta_ + tl.o_slot; }
-            cuda_check(hy_mla_attention_mma(a, q_abs_, caches_[run.cache_idx], lat_, r, d_meta_ + tl.o_seq, d_meta_ + tl.o_q0, tl.n, sp, stream), "latent attention (mma)");
+            cuda_check(hy_mla_decode_mma(a, q_abs_, caches_[run.cache_idx], lat_, r, d_meta_ + tl.o_seq, tl.n_one, sp, stream), "latent attention (mma, decoding rows)");
+            HyMlaSplit rest = sp;
+            if (rest.tile_k0) { rest.tile_k0 += tl.n_one; rest.tile_k1 += tl.n_one; rest.tile_slot += tl.n_one; }
+            cuda_check(hy_mla_attention_mma(a, q_abs_, caches_[run.cache_idx], lat_, r, d_meta_ + tl.o_seq + tl.n_one, d_meta_ + tl.o_q0 + tl.n_one, tl.n - tl.n_one, rest, stream), "latent attention (mma)");
             cuda_check(hy_mla_merge(d_meta_ + tl.o_mrow, d_meta_ + tl.o_mslot, d_meta_ + tl.o_mparts, tl.n_merge, split_o_, split_ml_, lat_, l.heads, l.kv_rank, stream, a.sink, a.head_gate, a.ldg), "latent attention (join)");
         } else cuda_check(hy_mla_attention(f32_, a, q_abs_, caches_[run.cache_idx], lat_, r, stream), "latent attention");
         MARK(5);
@@ -1003,6 +1006,18 @@ void HybridModel::forward(const StepInput& in, float* logits_out) {
                 continue;
             }
             for (int q0 = 0; q0 < nq; q0 += HY_MLA_TILE_QUERIES) { tile_seq_.push_back(sq); tile_q0_.push_back(q0); tile_k0_.push_back(0); tile_k1_.push_back(0); tile_slot_.push_back(-1); }
+        }
+        if (tl.mma && hy_mla_decode_supported(latent_params(l, lw_[li]))) {      // tiles of decoding rows first
+            const size_t n = tile_seq_.size();
+            std::vector<size_t> order(n);
+            for (size_t i = 0; i < n; ++i) order[i] = i;
+            auto one = [&](size_t i) { return in.seq_row0[tile_seq_[i] + 1] - in.seq_row0[tile_seq_[i]] == 1; };
+            tl.n_one = (int)(std::stable_partition(order.begin(), order.end(), one) - order.begin());
+            if (tl.n_one > 0 && tl.n_one < (int)n)
+                for (std::vector<int32_t>* v : {&tile_seq_, &tile_q0_, &tile_k0_, &tile_k1_, &tile_slot_}) {
+                    const std::vector<int32_t> old = *v;
+                    for (size_t i = 0; i < n; ++i) (*v)[i] = old[order[i]];
+                }
         }
         tl.n = (int)tile_seq_.size(); tl.n_merge = (int)merge_row_.size(); tl.n_ptiles = (int)ptile_seq_.size();
         tl.o_seq = put(tile_seq_.data(), tile_seq_.size()); tl.o_q0 = put(tile_q0_.data(), tile_q0_.size());

@@ -322,3 +322,30 @@ def test_greedy_generation_through_the_scheduler(tmp_path):
                 assert top2[1] - top2[0] < 1e-3, "greedy token differs from the oracle's outside a near tie"
                 break
             seq.append(tok)
+
+
+@pytest.mark.parametrize("heads,rank,rot,window", [(16, 64, 16, None), (1, 128, 16, 45), (5, 256, 32, 33), (16, 512, 64, 130), (8, 192, 16, 20)])
+def test_decoding_rows_of_latent_attention_split_their_keys_over_warps(tmp_path, heads, rank, rot, window):
+    """one row, up to 16 heads: groups of 16 cache rows per warp — contexts around 16, 64 and the parts' edges, windows that begin inside a group,
+    every split of the latent's channels; a portion and a decoding row in one step; one stage per warp for the wide latent"""
+    layers = [G.latent_layer(heads=heads, dim=32, rot_dim=rot, vdim=32, kv_rank=rank, q_rank=48, window=window, base=10000.0, mlp=64)]
+    cfg = G.make_config(layers, width=64, vocab=72, streams=2)
+    W = checkpoint(tmp_path, cfg, 31)
+    a, b = tokens_of(cfg, 290, 1), tokens_of(cfg, 80, 2)
+    ref_a, ref_b = G.forward(cfg, W, a), G.forward(cfg, W, b)
+    with engine(tmp_path, "bfloat16", pages=12) as eng:
+        got = [eng.trace_step([(1, a[:13], list(range(13)))])]
+        for i in range(13, 72):
+            got.append(eng.trace_step([(1, [a[i]], [0])]))
+        got.append(eng.trace_step([(1, a[72:252], list(range(180)))]))
+        for i in range(252, 262):
+            got.append(eng.trace_step([(1, [a[i]], [0])]))
+        rows_b = []
+        for i in range(262, 266):                                   # a decoding row beside a portion of another request
+            k = i - 262
+            out = eng.trace_step([(2, b[20 * k:20 * k + 20], list(range(20))), (1, [a[i]], [0])])
+            rows_b.append(out[:20]); got.append(out[20:])
+        for i in range(266, 290):
+            got.append(eng.trace_step([(1, [a[i]], [0])], [1] if i == 289 else []))
+    check(np.concatenate(got), ref_a, "bfloat16")
+    check(np.concatenate(rows_b), ref_b, "bfloat16")
