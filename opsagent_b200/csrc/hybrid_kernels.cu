@@ -71,40 +71,48 @@ __global__ void __launch_bounds__(256) hy_gemm_kernel(const TA* __restrict__ A, 
     }
 }
 
-// The same product for a handful of rows (decoding steps), bf16 operands with K in aligned groups of 8: one warp per output column keeps
-// its row of B in registers (K <= 1024: four 16-byte pieces per lane) and walks the M rows of A; a lane sums its pieces in order, then the
-// warp joins by a butterfly, so a row's result does not depend on the other rows.  The tile kernel above leaves most of a 64-row tile empty
-// at these sizes and runs K / 16 barrier-separated slices on a few CTAs.
+// The same product for a handful of rows (decoding steps), bf16 operands with K in aligned groups of 8: a warp owns 8 columns and 16 rows as
+// mma.sync m16n8k16 products straight from global memory.  The order of k inside a product is free as long as A and B agree, so lane t of a
+// quad takes eight consecutive values of its rows in one 16-byte load — two products' worth — and nothing goes through shared memory.  Four
+// blocks of 32 k are in flight; sums run in ascending blocks, so a row's result does not depend on the other rows.  What bounds it is that load
+// latency: 16 rows x 16 heads x 512 x 128 27 us -> about 5 as one warp per column that walked the rows, each with a butterfly of its own.
 template <int MODE>
-__global__ void __launch_bounds__(256) hy_gemm_fewrows_kernel(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bfloat16* __restrict__ B, int ldb, void* Cv, int ldc, int M, int N,
+__global__ void __launch_bounds__(128) hy_gemm_fewrows_kernel(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bfloat16* __restrict__ B, int ldb, void* Cv, int ldc, int M, int N,
                                                               int K, const float* __restrict__ bias, float alpha, long long sA, long long sB, long long sC, HyGemmAct act) {
     HY_PDL();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n = blockIdx.x * 8 + warp;
-    if (n >= N) return;
-    A += (long long)blockIdx.y * sA; B += (long long)blockIdx.y * sB;
-    uint4 b[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) { const int k = (lane + 32 * i) * 8; b[i] = k < K ? *reinterpret_cast<const uint4*>(B + (long long)n * ldb + k) : make_uint4(0, 0, 0, 0); }
-    for (int m = 0; m < M; ++m) {
-        float acc = 0.f;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int n0 = (blockIdx.x * 4 + warp) * 8, m0 = blockIdx.z * 16;
+    if (n0 >= N) return;
+    const __nv_bfloat16* a_lo = A + (long long)blockIdx.y * sA + (long long)(m0 + g) * lda;
+    const __nv_bfloat16* a_hi = a_lo + (long long)8 * lda;
+    const __nv_bfloat16* b_n = B + (long long)blockIdx.y * sB + (long long)(n0 + g) * ldb;
+    const bool lo = m0 + g < M, hi = m0 + g + 8 < M, col = n0 + g < N;
+    float d[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int kb = 0; kb < K; kb += 128) {
+        uint4 x[4], y[4], w[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const int k = (lane + 32 * i) * 8;
-            if (k < K) {
-                const uint4 a = *reinterpret_cast<const uint4*>(A + (long long)m * lda + k);
-                acc = fmaf(bf16lo(a.x), bf16lo(b[i].x), acc); acc = fmaf(bf16hi(a.x), bf16hi(b[i].x), acc); acc = fmaf(bf16lo(a.y), bf16lo(b[i].y), acc); acc = fmaf(bf16hi(a.y), bf16hi(b[i].y), acc);
-                acc = fmaf(bf16lo(a.z), bf16lo(b[i].z), acc); acc = fmaf(bf16hi(a.z), bf16hi(b[i].z), acc); acc = fmaf(bf16lo(a.w), bf16lo(b[i].w), acc); acc = fmaf(bf16hi(a.w), bf16hi(b[i].w), acc);
-            }
+            const int k = kb + i * 32 + t * 8;
+            x[i] = lo && k < K ? *reinterpret_cast<const uint4*>(a_lo + k) : make_uint4(0, 0, 0, 0);
+            y[i] = hi && k < K ? *reinterpret_cast<const uint4*>(a_hi + k) : make_uint4(0, 0, 0, 0);
+            w[i] = col && k < K ? *reinterpret_cast<const uint4*>(b_n + k) : make_uint4(0, 0, 0, 0);
         }
-        acc = warp_sum(acc);
-        if (lane == 0) {
-            float v = acc * alpha + (bias ? bias[n] : 0.f);
-            v = gemm_act(act, v, n);
-            const long long at = (long long)blockIdx.y * sC + (long long)m * ldc + n;
-            if (MODE == HY_STORE) reinterpret_cast<__nv_bfloat16*>(Cv)[at] = __float2bfloat16_rn(v);
-            else if (MODE == HY_STORE_F32) reinterpret_cast<float*>(Cv)[at] = v;
-            else reinterpret_cast<float*>(Cv)[at] += v;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            mma_bf16_16816(d, x[i].x, y[i].x, x[i].y, y[i].y, w[i].x, w[i].y);
+            mma_bf16_16816(d, x[i].z, y[i].z, x[i].w, y[i].w, w[i].z, w[i].w);
         }
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const int m = m0 + g + (c >= 2 ? 8 : 0), n = n0 + 2 * t + (c & 1);
+        if (m >= M || n >= N) continue;
+        float v = d[c] * alpha + (bias ? bias[n] : 0.f);
+        v = gemm_act(act, v, n);
+        const long long at = (long long)blockIdx.y * sC + (long long)m * ldc + n;
+        if (MODE == HY_STORE) reinterpret_cast<__nv_bfloat16*>(Cv)[at] = __float2bfloat16_rn(v);
+        else if (MODE == HY_STORE_F32) reinterpret_cast<float*>(Cv)[at] = v;
+        else reinterpret_cast<float*>(Cv)[at] += v;
     }
 }
 
@@ -1437,11 +1445,11 @@ cudaError_t hy_gemm(bool f32, int mode, const void* A, int lda, const void* B, i
     if (M <= 0 || N <= 0 || K <= 0 || batch <= 0) return cudaSuccess;
     auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
     if (!f32 && M <= HY_GEMM_FEW_ROWS && K % 8 == 0 && K <= 1024 && lda % 8 == 0 && ldb % 8 == 0 && sA % 8 == 0 && sB % 8 == 0 && al16(A) && al16(B)) {
-        const dim3 grid((N + 7) / 8, batch);
+        const dim3 grid((N + 31) / 32, batch, (M + 15) / 16);
         switch (mode) {
-            case HY_STORE: return launch_plain(hy_gemm_fewrows_kernel<HY_STORE>, grid, dim3(256), 0, s, (const bf*)A, lda, (const bf*)B, ldb, C, ldc, M, N, K, bias, alpha, sA, sB, sC, act);
-            case HY_STORE_F32: return launch_plain(hy_gemm_fewrows_kernel<HY_STORE_F32>, grid, dim3(256), 0, s, (const bf*)A, lda, (const bf*)B, ldb, C, ldc, M, N, K, bias, alpha, sA, sB, sC, act);
-            default: return launch_plain(hy_gemm_fewrows_kernel<HY_ACC_F32>, grid, dim3(256), 0, s, (const bf*)A, lda, (const bf*)B, ldb, C, ldc, M, N, K, bias, alpha, sA, sB, sC, act);
+            case HY_STORE: return launch_plain(hy_gemm_fewrows_kernel<HY_STORE>, grid, dim3(128), 0, s, (const bf*)A, lda, (const bf*)B, ldb, C, ldc, M, N, K, bias, alpha, sA, sB, sC, act);
+            case HY_STORE_F32: return launch_plain(hy_gemm_fewrows_kernel<HY_STORE_F32>, grid, dim3(128), 0, s, (const bf*)A, lda, (const bf*)B, ldb, C, ldc, M, N, K, bias, alpha, sA, sB, sC, act);
+            default: return launch_plain(hy_gemm_fewrows_kernel<HY_ACC_F32>, grid, dim3(128), 0, s, (const bf*)A, lda, (const bf*)B, ldb, C, ldc, M, N, K, bias, alpha, sA, sB, sC, act);
         }
     }
     return f32 ? gemm_t<float>(mode, A, lda, B, ldb, C, ldc, M, N, K, bias, alpha, batch, sA, sB, sC, s, act)
