@@ -118,6 +118,7 @@ int oa_k_gemm(const void* A, const void* B, int32_t M, int32_t N, int32_t K, int
     CUtensorMap tmA, tmB;
     GemmParams p{}; p.M = M; p.N = N; p.K = K; p.out = out; p.ldo = epilogue == EPI_SWIGLU ? N / 2 : N;
     p.bias = bias; p.resid = resid; p.ldr = N; p.logits = logits; p.ldl = N;
+    if (epilogue == EPI_LOGITS) block_n = gemm_logits_bn(M, N, block_n);
     p.few_rows_ok = 1;
     if (make_tmap_bf16_2d(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)K, (uint32_t)gemm_a_box(p, epilogue, block_n), 64) != 0) return OA_ERR_INTERNAL;
     // room for cut tiles, where this product has any

@@ -40,6 +40,42 @@ struct GemmCfg {
     static constexpr uint32_t TMEM_COLS = BN < 32 ? 32 : BN;
 };
 
+// 32 columns of one row of the vocabulary head: the row's running arg-max (ties: lowest column) and, where wanted, the logits
+OA_DEVINL const uint32_t* logits_mask(const GemmParams& p, int row) {
+    const int ms = p.mask_slot ? p.mask_slot[row] : -1;
+    return ms >= 0 ? p.mask_table + (size_t)ms * p.mask_words : nullptr;
+}
+OA_DEVINL void logits_chunk(const GemmParams& p, int row, const uint32_t (&v)[32], int col0, const uint32_t* mask_row, float& best_v, int& best_i) {
+    if (mask_row) {
+        // grammar-constrained row: only token ids allowed in this sequence's automaton state compete.  The 32 columns of
+        // this chunk are 32 consecutive global ids: at most two words of the bitset.
+        const uint32_t g0 = (uint32_t)(p.col_offset + col0);
+        const uint32_t w0 = (g0 >> 5) < (uint32_t)p.mask_words ? __ldg(mask_row + (g0 >> 5)) : 0u;
+        const uint32_t w1 = ((g0 & 31u) && (g0 >> 5) + 1 < (uint32_t)p.mask_words) ? __ldg(mask_row + (g0 >> 5) + 1) : 0u;
+        const uint32_t bits = (g0 & 31u) ? __funnelshift_r(w0, w1, g0 & 31u) : w0;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            float f = __uint_as_float(v[j]);
+            if (((bits >> j) & 1u) && col0 + j < p.N && f > best_v) { best_v = f; best_i = col0 + j; }
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            float f = __uint_as_float(v[j]);
+            if (col0 + j < p.N && f > best_v) { best_v = f; best_i = col0 + j; }
+        }
+    }
+    if (p.logits) {
+        float* lrow = p.logits + (size_t)row * p.ldl;
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) {
+            if (col0 + j < p.N)
+                *reinterpret_cast<float4*>(lrow + col0 + j) =
+                    make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
+        }
+    }
+}
+
 template <int BN, int EPI>
 __global__ void __launch_bounds__(GEMM_THREADS) gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
                                                                       const __grid_constant__ CUtensorMap tmB,
@@ -140,7 +176,7 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_tcgen05_kernel(const __grid
         tcgen05_fence_after();
         float best_v = -INFINITY; int best_i = 0x7fffffff;
         const uint32_t* mask_row = nullptr;
-        if (EPI == EPI_LOGITS && row_ok && p.mask_slot) { const int ms = p.mask_slot[row]; if (ms >= 0) mask_row = p.mask_table + (size_t)ms * p.mask_words; }
+        if (EPI == EPI_LOGITS && row_ok) mask_row = logits_mask(p, row);
 #pragma unroll 1
         for (int c = 0; c < BN; c += 32) {
             uint32_t v[32];
@@ -235,36 +271,7 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_tcgen05_kernel(const __grid
                     }
                 }
             } else {  // EPI_LOGITS
-                if (row_ok) {
-                    if (mask_row) {
-                        // grammar-constrained row: only token ids allowed in this sequence's automaton state compete.  The 32 columns of
-                        // this chunk are 32 consecutive global ids: at most two words of the bitset.
-                        const uint32_t g0 = (uint32_t)(p.col_offset + col0);
-                        const uint32_t w0 = (g0 >> 5) < (uint32_t)p.mask_words ? __ldg(mask_row + (g0 >> 5)) : 0u;
-                        const uint32_t w1 = ((g0 & 31u) && (g0 >> 5) + 1 < (uint32_t)p.mask_words) ? __ldg(mask_row + (g0 >> 5) + 1) : 0u;
-                        const uint32_t bits = (g0 & 31u) ? __funnelshift_r(w0, w1, g0 & 31u) : w0;
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) {
-                            float f = __uint_as_float(v[j]);
-                            if (((bits >> j) & 1u) && col0 + j < p.N && f > best_v) { best_v = f; best_i = col0 + j; }
-                        }
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) {
-                            float f = __uint_as_float(v[j]);
-                            if (col0 + j < p.N && f > best_v) { best_v = f; best_i = col0 + j; }
-                        }
-                    }
-                    if (p.logits) {
-                        float* lrow = p.logits + (size_t)row * p.ldl;
-#pragma unroll
-                        for (int j = 0; j < 32; j += 4) {
-                            if (col0 + j < p.N)
-                                *reinterpret_cast<float4*>(lrow + col0 + j) =
-                                    make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
-                        }
-                    }
-                }
+                if (row_ok) logits_chunk(p, row, v, col0, mask_row, best_v, best_i);
             }
         }
         if (EPI == EPI_LOGITS && row_ok) {
@@ -306,6 +313,9 @@ static cudaError_t launch_bn(const CUtensorMap* tmA, const CUtensorMap* tmB, con
 }
 
 static bool persistent_disabled();
+static bool head_persistent(int M, int N);
+static cudaError_t launch_head(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, cudaStream_t stream);
+static constexpr int HEAD_BN = 128;
 static int sm_count_cached();
 static long long persistent_min_tiles();
 template <int EPI>
@@ -373,6 +383,7 @@ cudaError_t launch_gemm(const CUtensorMap* tmA, const CUtensorMap* tmB, const Ge
             case EPI_F32: return launch_persistent<EPI_F32>(tmA, tmB, p, stream);
         }
     }
+    if (epilogue == EPI_LOGITS && block_n == HEAD_BN && head_persistent(p.M, p.N)) return launch_head(tmA, tmB, p, stream);
     switch (block_n) {
         case 32: return launch_bn<32>(tmA, tmB, p, epilogue, stream);
         case 64: return launch_bn<64>(tmA, tmB, p, epilogue, stream);
@@ -498,6 +509,131 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_persistent_kernel(const 
     __syncthreads();
     if (warp == 1) { tcgen05_fence_after(); tmem_dealloc<Cfg::TMEM_COLS>(tmem_base); }
 }
+
+// =============================================================================================
+// vocabulary head: persistent 128 x 128 tiles, one CTA per SM, two accumulators.  The head streams its weights once (1 GB for 128 thousand tokens of
+// width 4096) and is bound by that.  One CTA per 128 x 256 tile left the last of 3.4 rounds mostly empty and paid each tile's epilogue (logits,
+// arg-max) behind its products; here 1002 tiles make 6.8 rounds and the epilogue runs under the next tile's.  128 rows, with logits: 205 -> 180 us.
+// =============================================================================================
+struct HeadCfg {
+    static constexpr int BN = HEAD_BN, STAGES = 6, A_BYTES = BLOCK_M * BLOCK_K * 2, B_BYTES = BN * BLOCK_K * 2, STAGE_BYTES = A_BYTES + B_BYTES;
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
+    static constexpr uint32_t TMEM_COLS = 2 * BN;
+};
+__global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_head_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
+    using Cfg = HeadCfg;
+    constexpr int BN = Cfg::BN, STAGES = Cfg::STAGES;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * Cfg::STAGE_BYTES);
+    uint64_t* empty_bar = full_bar + STAGES;
+    uint64_t* acc_full = empty_bar + STAGES;
+    uint64_t* acc_empty = acc_full + 2;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n_tiles = (p.N + BN - 1) / BN, m_tiles = (p.M + BLOCK_M - 1) / BLOCK_M, total_tiles = n_tiles * m_tiles;
+    const int num_kb = (p.K + BLOCK_K - 1) / BLOCK_K;
+
+    if (warp == 0 && lane == 0) {
+        tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmB);
+        for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+        for (int s = 0; s < 2; ++s) { mbar_init(&acc_full[s], 1); mbar_init(&acc_empty[s], 4); }
+        fence_barrier_init();
+    }
+    if (warp == 1) tmem_alloc<Cfg::TMEM_COLS>(tmem_slot);
+    tcgen05_fence_before();
+    __syncthreads();
+    tcgen05_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    griddep_launch();
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int s = 0; uint32_t ph = 0;
+            const int pre = num_kb < STAGES ? num_kb : STAGES;      // the first tile's weights before the wait: no predecessor writes them
+            for (int t = blockIdx.x, first = 1; t < total_tiles; t += gridDim.x, first = 0) {
+                int m_blk, n_blk; raster_tile(t, m_tiles, n_tiles, m_blk, n_blk);
+                if (first) {
+                    for (int kb = 0; kb < pre; ++kb) {
+                        mbar_expect_tx(&full_bar[kb], Cfg::STAGE_BYTES);
+                        tma_load_2d(smem + kb * Cfg::STAGE_BYTES + Cfg::A_BYTES, &tmB, &full_bar[kb], kb * BLOCK_K, n_blk * BN, kEvictFirst);
+                    }
+                    griddep_wait();
+                }
+                for (int kb = 0; kb < num_kb; ++kb) {
+                    uint8_t* a_dst = smem + s * Cfg::STAGE_BYTES;
+                    if (!first || kb >= pre) {
+                        mbar_wait(&empty_bar[s], ph ^ 1);
+                        mbar_expect_tx(&full_bar[s], Cfg::STAGE_BYTES);
+                        tma_load_2d(a_dst + Cfg::A_BYTES, &tmB, &full_bar[s], kb * BLOCK_K, n_blk * BN, m_tiles > 1 ? kEvictNormal : kEvictFirst);
+                    }
+                    tma_load_2d(a_dst, &tmA, &full_bar[s], kb * BLOCK_K, m_blk * BLOCK_M, kEvictLast);
+                    if (++s == STAGES) { s = 0; ph ^= 1; }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            constexpr uint32_t idesc = umma_idesc_bf16(BLOCK_M, BN);
+            int s = 0; uint32_t ph = 0; int it = 0;
+            for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++it) {
+                const int as = it & 1;
+                mbar_wait(&acc_empty[as], (((uint32_t)it >> 1) & 1) ^ 1);
+                tcgen05_fence_after();
+                const uint32_t tmem_d = tmem_base + (uint32_t)(as * BN);
+                for (int kb = 0; kb < num_kb; ++kb) {
+                    mbar_wait(&full_bar[s], ph);
+                    tcgen05_fence_after();
+                    const uint32_t a_addr = smem_u32(smem + s * Cfg::STAGE_BYTES);
+                    const uint64_t a_desc = umma_desc_sw128(a_addr), b_desc = umma_desc_sw128(a_addr + Cfg::A_BYTES);
+#pragma unroll
+                    for (int k = 0; k < BLOCK_K / UMMA_K; ++k)
+                        umma_bf16(tmem_d, a_desc + (uint64_t)(k * 2), b_desc + (uint64_t)(k * 2), idesc, (kb | k) != 0);
+                    umma_commit(&empty_bar[s]);
+                    if (++s == STAGES) { s = 0; ph ^= 1; }
+                }
+                umma_commit(&acc_full[as]);
+            }
+        }
+    } else {
+        const int q = warp & 3;
+        griddep_wait();
+        int it = 0;
+        for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++it) {
+            int m_blk, n_blk; raster_tile(t, m_tiles, n_tiles, m_blk, n_blk);
+            const int as = it & 1, row = m_blk * BLOCK_M + q * 32 + lane;
+            const bool row_ok = row < p.M;
+            const uint32_t* mask_row = row_ok ? logits_mask(p, row) : nullptr;
+            float best_v = -INFINITY; int best_i = 0x7fffffff;
+            mbar_wait(&acc_full[as], ((uint32_t)it >> 1) & 1);
+            tcgen05_fence_after();
+#pragma unroll 1
+            for (int c = 0; c < BN; c += 32) {
+                uint32_t v[32];
+                tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * BN + c), v);
+                tmem_ld_wait();
+                if (row_ok) logits_chunk(p, row, v, n_blk * BN + c, mask_row, best_v, best_i);
+            }
+            if (row_ok) { p.amax_val[(size_t)row * n_tiles + n_blk] = best_v; p.amax_idx[(size_t)row * n_tiles + n_blk] = best_i; }
+            tcgen05_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty[as]);
+        }
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+    if (warp == 1) { tcgen05_fence_after(); tmem_dealloc<Cfg::TMEM_COLS>(tmem_base); }
+}
+static cudaError_t launch_head(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, cudaStream_t stream) {
+    static bool attr_done[16] = {};
+    { cudaError_t e = ensure_dynamic_smem(gemm_head_kernel, HeadCfg::SMEM_BYTES, attr_done); if (e != cudaSuccess) return e; }
+    const int tiles = gemm_n_tiles(p.N, HeadCfg::BN) * ((p.M + BLOCK_M - 1) / BLOCK_M);
+    return launch_k(gemm_head_kernel, dim3(std::min(tiles, sm_count_cached())), dim3(GEMM_THREADS), HeadCfg::SMEM_BYTES, stream, *tmA, *tmB, p);
+}
+// the persistent kernel from two rounds of its tiles on; the narrow tiles of a small vocabulary fill the SMs better one CTA each
+static bool head_persistent(int M, int N) { return (long long)gemm_n_tiles(N, HeadCfg::BN) * ((M + BLOCK_M - 1) / BLOCK_M) >= 2LL * sm_count_cached(); }
+int gemm_logits_bn(int M, int N, int block_n) { return block_n >= HeadCfg::BN && head_persistent(M, N) ? HeadCfg::BN : block_n; }
 
 static bool persistent_disabled() { static const bool off = [] { const char* e = std::getenv("OA_GEMM_PERSISTENT"); return e && e[0] == '0'; }(); return off; }
 // tests lower the threshold (OA_GEMM_PERSISTENT_MIN_TILES=1) to drive tiny shapes through the persistent kernel

@@ -51,6 +51,7 @@ struct GemmParams {
 cudaError_t launch_gemm(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epilogue, int block_n,
                         cudaStream_t stream);
 int gemm_n_tiles(int N, int block_n);
+int gemm_logits_bn(int M, int N, int block_n);      // EPI_LOGITS: the tile width to ask launch_gemm for (and to count the arg-max partials by) where block_n would do
 // rows of the B tensor map's box that launch_gemm(.., block_n, ..) reads for this product: block_n, or what the CTA-pair kernel takes where that runs
 int gemm_b_box(const GemmParams& p, int epilogue, int block_n);
 bool gemm_may_split(const GemmParams& p, int epilogue, int block_n);      // the product has tiles worth cutting if GemmParams::split_ws gives room

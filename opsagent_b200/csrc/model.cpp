@@ -623,7 +623,7 @@ void DeviceModel::forward(const StepInput& in, float* logits_out) {
             cuda_check(launch_rmsnorm(xs_, final_norm, xsn_, S, H, cfg.rms_eps, stream), "final norm");
         }
         MARK(11);
-        const int bn_lm = pick_bn(S, V, opt.bn_lm, false);
+        const int bn_lm = opt.bn_lm ? pick_bn(S, V, opt.bn_lm, false) : gemm_logits_bn(S, V, pick_bn(S, V, 0, false));
         const int n_tiles = gemm_n_tiles(V, bn_lm);
         GemmParams gl{}; gl.M = S; gl.N = V; gl.K = H; gl.logits = logits_out; gl.ldl = V; gl.amax_val = amax_val_; gl.amax_idx = amax_idx_;
         if (!in.mask_slots.empty()) {          // constrained rows: the arg-max runs over their state's allowed tokens, on every vocabulary shard

@@ -414,3 +414,22 @@ def test_gemm_few_rows(L, M, N, K):
         torch.cuda.synchronize()
         v = ref.view(M, N // 32, 2, 16)
         close(y, (torch.nn.functional.silu(v[:, :, 0]) * v[:, :, 1]).reshape(M, N // 2), 2e-5 * float(v.abs().max()) ** 2)
+
+
+# persistent vocabulary head: fewer k blocks than ring stages and more, one and several row tiles, a ragged last tile, the largest in the last column
+@pytest.mark.parametrize("M,N,K", [(1, 128256, 64), (128, 38016, 200), (3, 128256, 1024), (129, 40008, 512), (64, 152064, 448)])
+def test_persistent_vocabulary_head(L, M, N, K):
+    g = torch.Generator(device=dev()).manual_seed(N + K)
+    A = torch.randn(M, K, generator=g, device=dev()).to(torch.bfloat16)
+    B = (torch.randn(N, K, generator=g, device=dev()) * 0.1).to(torch.bfloat16)
+    B[N - 1] = (A[0].float() * 0.5).to(torch.bfloat16)
+    logits = torch.full((M, N), float("nan"), dtype=torch.float32, device=dev())
+    ids = torch.empty(M, dtype=torch.int32, device=dev()); ids2 = torch.empty_like(ids)
+    assert L.oa_k_gemm(ptr(A), ptr(B), M, N, K, EPI_LOGITS, 256, None, None, None, ptr(logits), ptr(ids), None) == 0
+    assert L.oa_k_gemm(ptr(A), ptr(B), M, N, K, EPI_LOGITS, 128, None, None, None, None, ptr(ids2), None) == 0
+    ref = A.double() @ B.double().T
+    # fp32 sums of K products of size about 0.1 |a|
+    assert ((logits.double() - ref).abs() <= 0.1 * 4 * K * 2.0 ** -23 + 1e-5 * ref.abs()).all()
+    mx = logits.max(dim=1, keepdim=True).values
+    first = torch.where(logits == mx, torch.arange(N, device=dev())[None, :], N).min(dim=1).values
+    assert (ids.long() == first).all() and (ids2 == ids).all() and ids[0].item() == N - 1
