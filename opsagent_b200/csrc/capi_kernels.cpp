@@ -92,11 +92,11 @@ extern "C" {
 int oa_k_gemm_streamk(const void* A, const void* B, int32_t M, int32_t N, int32_t K, int32_t block_n, int32_t n_ctas, float* out_f32, void* stream) {
     cudaStream_t s = (cudaStream_t)stream;
     CUtensorMap tmA, tmB;
-    if (make_tmap_bf16_2d(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)K, 128, 64) != 0) return OA_ERR_INTERNAL;
+    if (make_tmap_bf16_2d(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)K, (uint32_t)streamk_a_rows(M), 64) != 0) return OA_ERR_INTERNAL;
     if (make_tmap_bf16_2d(&tmB, B, (uint64_t)N, (uint64_t)K, (uint64_t)K, (uint32_t)block_n, 64) != 0) return OA_ERR_INTERNAL;
     DevBuf ws(streamk_ws_bytes(N, block_n, n_ctas, M), s);
     if (!ws.p) return OA_ERR_INTERNAL;
-    StreamK sk = make_streamk((float*)ws.p, N, K, block_n, n_ctas, M);
+    StreamK sk = make_streamk((float*)ws.p, N, K, block_n, n_ctas, M, streamk_a_rows(M));
     cudaError_t e = launch_gemm_streamk(&tmA, &tmB, M, N, K, sk, s);
     if (e == cudaSuccess) e = launch_k(sk_reduce_f32_kernel, dim3((N / 8 + 127) / 128, M), dim3(128), 0, s, sk, out_f32, N, (int)(((uintptr_t)out_f32 & 15) == 0));
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);

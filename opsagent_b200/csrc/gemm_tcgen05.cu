@@ -700,6 +700,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, OCC) gemm_streamk_kernel(const _
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long c = blockIdx.x, G = gridDim.x;
     const long long u0 = c * sk.total / G, u1 = (c + 1) * sk.total / G;
+    const uint32_t stage_tx = (uint32_t)(MT * sk.a_rows * BLOCK_K * 2 + Cfg::B_BYTES);      // few rows: only they are loaded (the rest of the tile is stale, and its products are never read)
 
     if (warp == 0 && lane == 0) {
         tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmB);
@@ -721,7 +722,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, OCC) gemm_streamk_kernel(const _
             for (int i = 0; i < pre; ++i) {
                 const long long u = u0 + i;
                 const int tile = (int)(u / sk.kb), kblk = (int)(u - (long long)tile * sk.kb);
-                mbar_expect_tx(&full_bar[i], Cfg::STAGE_BYTES);
+                mbar_expect_tx(&full_bar[i], stage_tx);
                 tma_load_2d(smem + i * Cfg::STAGE_BYTES + Cfg::A_BYTES, &tmB, &full_bar[i], kblk * BLOCK_K, tile * BN, kEvictFirst);
             }
             // ... and pull the next weight tiles into L2 while the (L2-bound) predecessor still runs and HBM is idle
@@ -745,7 +746,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, OCC) gemm_streamk_kernel(const _
                 const int tile = (int)(u / sk.kb), kblk = (int)(u - (long long)tile * sk.kb);
                 mbar_wait(&empty_bar[s], ph ^ 1);
                 uint8_t* a_dst = smem + s * Cfg::STAGE_BYTES;
-                mbar_expect_tx(&full_bar[s], Cfg::STAGE_BYTES);
+                mbar_expect_tx(&full_bar[s], stage_tx);
 #pragma unroll
                 for (int m = 0; m < MT; ++m)
                     tma_load_2d(a_dst + m * Cfg::A_TILE_BYTES, &tmA, &full_bar[s], kblk * BLOCK_K, m * BLOCK_M, kEvictLast);
@@ -1037,8 +1038,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, OCC) gemm_streamk_kernel(const _
     if (warp == 1) { tcgen05_fence_after(); tmem_dealloc<Cfg::TMEM_COLS>(tmem_base); }
 }
 
-StreamK make_streamk(float* ws, int N, int K, int bn, int G, int rows) {
-    StreamK sk{}; sk.ws = ws; sk.bn = bn; sk.rows = rows > 128 ? 256 : 128; sk.kb = (K + BLOCK_K - 1) / BLOCK_K; sk.n_tiles = (N + bn - 1) / bn;
+StreamK make_streamk(float* ws, int N, int K, int bn, int G, int rows, int a_rows) {
+    StreamK sk{}; sk.a_rows = rows > 128 ? 128 : a_rows; sk.ws = ws; sk.bn = bn; sk.rows = rows > 128 ? 256 : 128; sk.kb = (K + BLOCK_K - 1) / BLOCK_K; sk.n_tiles = (N + bn - 1) / bn;
     sk.total = (long long)sk.n_tiles * sk.kb; sk.G = (int)std::min<long long>(G, sk.total);
     sk.l2_prefetch_units = 0;
     return sk;
@@ -1054,28 +1055,28 @@ static cudaError_t launch_sk(const CUtensorMap* tmA, const CUtensorMap* tmB, int
 }
 cudaError_t launch_gemm_streamk_swiglu(const CUtensorMap* tmA, const CUtensorMap* tmB, int M, int F, int K, const StreamK& sk, void* act,
                                        unsigned int* tile_flags, cudaStream_t stream) {
-    if (M <= 0 || M > BLOCK_M || sk.rows != 128 || sk.bn != 128 || (F % 16) != 0 || (K % 8) != 0 || !act || !tile_flags) return cudaErrorInvalidValue;
+    if (M <= 0 || M > BLOCK_M || M > sk.a_rows || sk.rows != 128 || sk.bn != 128 || (F % 16) != 0 || (K % 8) != 0 || !act || !tile_flags) return cudaErrorInvalidValue;
     if (sk.G > sm_count_cached()) return cudaErrorInvalidValue;      // finishing CTAs wait for publishing CTAs: all must be resident
     SkFuse fz{}; fz.act = reinterpret_cast<uint16_t*>(act); fz.F = F; fz.tile_flags = tile_flags;
     return launch_sk<128, 1, 1, 1>(tmA, tmB, M, sk, stream, fz);
 }
 cudaError_t launch_gemm_streamk_resid(const CUtensorMap* tmA, const CUtensorMap* tmB, int M, int N, int K, const StreamK& sk, void* x, int ldx,
                                       unsigned int* tile_flags, cudaStream_t stream) {
-    if (M <= 0 || M > BLOCK_M || sk.rows != 128 || sk.bn != 128 || (N % 32) != 0 || (K % 8) != 0 || !x || !tile_flags || (ldx % 8) != 0) return cudaErrorInvalidValue;
+    if (M <= 0 || M > BLOCK_M || M > sk.a_rows || sk.rows != 128 || sk.bn != 128 || (N % 32) != 0 || (K % 8) != 0 || !x || !tile_flags || (ldx % 8) != 0) return cudaErrorInvalidValue;
     if (sk.G > sm_count_cached()) return cudaErrorInvalidValue;      // finishing CTAs wait for publishing CTAs: all must be resident
     SkFuse fz{}; fz.tile_flags = tile_flags; fz.x = reinterpret_cast<uint16_t*>(x); fz.ldx = ldx; fz.N = N;
     return launch_sk<128, 1, 1, 2>(tmA, tmB, M, sk, stream, fz);
 }
 cudaError_t launch_gemm_streamk_rope(const CUtensorMap* tmA, const CUtensorMap* tmB, int M, int N, int K, const StreamK& sk, const SkRopeArgs& rope,
                                      unsigned int* tile_flags, cudaStream_t stream) {
-    if (M <= 0 || M > BLOCK_M || sk.rows != 128 || sk.bn != 128 || (K % 8) != 0 || !tile_flags) return cudaErrorInvalidValue;
+    if (M <= 0 || M > BLOCK_M || M > sk.a_rows || sk.rows != 128 || sk.bn != 128 || (K % 8) != 0 || !tile_flags) return cudaErrorInvalidValue;
     if ((rope.D != 64 && rope.D != 128) || N != (rope.nh + 2 * rope.nkv) * rope.D) return cudaErrorInvalidValue;      // BN must be a multiple of D; chunks of 32 never straddle a head
     if (sk.G > sm_count_cached()) return cudaErrorInvalidValue;
     SkFuse fz{}; fz.tile_flags = tile_flags; fz.N = N; fz.rope = rope;
     return launch_sk<128, 1, 1, 3>(tmA, tmB, M, sk, stream, fz);
 }
 cudaError_t launch_gemm_streamk(const CUtensorMap* tmA, const CUtensorMap* tmB, int M, int N, int K, const StreamK& sk, cudaStream_t stream) {
-    if (M <= 0 || M > sk.rows || (N % 8) != 0 || (K % 8) != 0) return cudaErrorInvalidValue;
+    if (M <= 0 || (sk.rows == 128 && M > sk.a_rows) || M > sk.rows || (N % 8) != 0 || (K % 8) != 0) return cudaErrorInvalidValue;
     if (sk.rows == 256) return sk.bn == 128 ? launch_sk<128, 2>(tmA, tmB, M, sk, stream) : cudaErrorInvalidValue;
     if (sk.bn == 256) return launch_sk<256, 1>(tmA, tmB, M, sk, stream);
     if (sk.bn == 128) return sk.G > sm_count_cached() ? launch_sk<128, 1, 2>(tmA, tmB, M, sk, stream) : launch_sk<128, 1, 1>(tmA, tmB, M, sk, stream);

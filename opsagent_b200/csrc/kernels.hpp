@@ -72,9 +72,11 @@ constexpr size_t GEMM_SPLIT_WS_BYTES = (size_t)GEMM_SPLIT_SLOTS * 256 * 256 * 4;
 // RMSNorm / RoPE / SwiGLU while they are at it.
 struct StreamK {
     float* ws; int bn, kb, n_tiles, G, rows; long long total;  // rows = 128 or 256 accumulator rows per slot      // kb = k blocks per tile, total = n_tiles * kb, G = CTAs
+    int a_rows;                                               // rows of A a stage loads: the box of tmA (16, 32, 64 or 128; all M rows, the tile's others are not looked at)
     int l2_prefetch_units;                                    // weight tiles each CTA prefetches into L2 before griddepcontrol.wait
 };
-StreamK make_streamk(float* ws, int N, int K, int bn, int G, int rows = 128);
+StreamK make_streamk(float* ws, int N, int K, int bn, int G, int rows = 128, int a_rows = 128);
+inline int streamk_a_rows(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128; }
 // CTA c owns units [c*total/G, (c+1)*total/G), so unit u lives in CTA floor(((u+1)*G - 1) / total): the CTAs holding the first and the
 // last k-block of `tile`.  One definition for the kernels, the consumers and the host plan (32-bit products: host-checked per model).
 #ifdef __CUDACC__
