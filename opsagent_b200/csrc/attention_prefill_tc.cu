@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(64 + 128 * NWG, 1) prefill_attention_tc_kernel
 // A group with an odd number of heads leaves its last one alone in an item (warpgroup B idles).
 // Measured against the kernel above: 4096 rows behind 12288 cached ones, 64 / 8 heads of 128: 1967 -> 1544 us (1.25 PFLOP/s; the tensor and the
 // special-function pipe are each busy 60 % of the time and the clock is down to 1.63 GHz under the 1000 W cap); five prompts of 1.4 thousand rows,
-// 32 / 8 heads: 184 -> 121 us.  Handing P over in two or three parts, taking exponentials from a reference that may still rise, moving an eighth
+// 32 / 8 heads: 184 -> 118 us.  Handing P over in two or three parts, taking exponentials from a reference that may still rise, moving an eighth
 // or a quarter of them to the FMA pipe and two threads per row were each 3 to 12 % slower.
 // ---------------------------------------------------------------------------------------------
 template <int D>

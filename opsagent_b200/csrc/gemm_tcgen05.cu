@@ -513,7 +513,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_persistent_kernel(const 
 // =============================================================================================
 // vocabulary head: persistent 128 x 128 tiles, one CTA per SM, two accumulators.  The head streams its weights once (1 GB for 128 thousand tokens of
 // width 4096) and is bound by that.  One CTA per 128 x 256 tile left the last of 3.4 rounds mostly empty and paid each tile's epilogue (logits,
-// arg-max) behind its products; here 1002 tiles make 6.8 rounds and the epilogue runs under the next tile's.  128 rows, with logits: 205 -> 180 us.
+// arg-max) behind its products; here 1002 tiles make 6.8 rounds and the epilogue runs under the next tile's.  128 rows, with logits: 205 -> 183 us.
 // =============================================================================================
 struct HeadCfg {
     static constexpr int BN = HEAD_BN, STAGES = 6, A_BYTES = BLOCK_M * BLOCK_K * 2, B_BYTES = BN * BLOCK_K * 2, STAGE_BYTES = A_BYTES + B_BYTES;

@@ -76,23 +76,26 @@ __global__ void __launch_bounds__(256) hy_gemm_kernel(const TA* __restrict__ A, 
 // quad takes eight consecutive values of its rows in one 16-byte load — two products' worth — and nothing goes through shared memory.  Four
 // blocks of 32 k are in flight; sums run in ascending blocks, so a row's result does not depend on the other rows.  What bounds it is that load
 // latency: 16 rows x 16 heads x 512 x 128 27 us -> about 5 as one warp per column that walked the rows, each with a butterfly of its own.
-template <int MODE>
+// SPLIT (K of 256 and more): the four warps of a block share eight columns, each every fourth block of 32 k, and join in warp order; otherwise each
+// warp has eight columns of its own.
+template <int MODE, bool SPLIT>
 __global__ void __launch_bounds__(128) hy_gemm_fewrows_kernel(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bfloat16* __restrict__ B, int ldb, void* Cv, int ldc, int M, int N,
                                                               int K, const float* __restrict__ bias, float alpha, long long sA, long long sB, long long sC, HyGemmAct act) {
     HY_PDL();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int n0 = (blockIdx.x * 4 + warp) * 8, m0 = blockIdx.z * 16;
+    const int n0 = (SPLIT ? blockIdx.x : blockIdx.x * 4 + warp) * 8, m0 = blockIdx.z * 16;
     if (n0 >= N) return;
     const __nv_bfloat16* a_lo = A + (long long)blockIdx.y * sA + (long long)(m0 + g) * lda;
     const __nv_bfloat16* a_hi = a_lo + (long long)8 * lda;
     const __nv_bfloat16* b_n = B + (long long)blockIdx.y * sB + (long long)(n0 + g) * ldb;
     const bool lo = m0 + g < M, hi = m0 + g + 8 < M, col = n0 + g < N;
+    constexpr int STEP = SPLIT ? 128 : 32;                   // from one of a warp's blocks of 32 k to its next
     float d[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int kb = 0; kb < K; kb += 128) {
+    for (int kb = SPLIT ? warp * 32 : 0; kb < K; kb += 4 * STEP) {
         uint4 x[4], y[4], w[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const int k = kb + i * 32 + t * 8;
+            const int k = kb + i * STEP + t * 8;
             x[i] = lo && k < K ? *reinterpret_cast<const uint4*>(a_lo + k) : make_uint4(0, 0, 0, 0);
             y[i] = hi && k < K ? *reinterpret_cast<const uint4*>(a_hi + k) : make_uint4(0, 0, 0, 0);
             w[i] = col && k < K ? *reinterpret_cast<const uint4*>(b_n + k) : make_uint4(0, 0, 0, 0);
@@ -102,6 +105,14 @@ __global__ void __launch_bounds__(128) hy_gemm_fewrows_kernel(const __nv_bfloat1
             mma_bf16_16816(d, x[i].x, y[i].x, x[i].y, y[i].y, w[i].x, w[i].y);
             mma_bf16_16816(d, x[i].z, y[i].z, x[i].w, y[i].w, w[i].z, w[i].w);
         }
+    }
+    if constexpr (SPLIT) {
+        __shared__ float4 part[3][32];
+        if (warp > 0) part[warp - 1][lane] = make_float4(d[0], d[1], d[2], d[3]);
+        __syncthreads();
+        if (warp > 0) return;
+#pragma unroll
+        for (int w = 0; w < 3; ++w) { const float4 u = part[w][lane]; d[0] += u.x; d[1] += u.y; d[2] += u.z; d[3] += u.w; }
     }
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
@@ -409,7 +420,7 @@ __global__ void __launch_bounds__(128) hy_mla_attention_mma_kernel(HyLatentAttn 
 // the same for ONE row of a sequence with at most 16 heads (a decoding row): its queries fill one warp's 16 mma rows, so the four warps take
 // turns at groups of 16 cache rows instead, each with an online softmax and accumulators of its own, joined once at the end.  Cache rows come
 // by one bulk copy each into a ring per warp: no warp waits for another before the join.  What bounds it is the chain of a warp's groups.
-// 16 rows of 170 cached tokens, 16 heads of a 512 + 64 wide latent: 60 -> 18 us against the 64-query tile, of which three warps idled.
+// 16 rows of 170 cached tokens, 16 heads of a 512 + 64 wide latent: 60 -> 20 us against the 64-query tile, of which three warps idled.
 // ---------------------------------------------------------------------------------------------------------------------------------
 constexpr int MLA_DQ = 16;
 static size_t mla_decode_smem(int E, int nvb, int stages) {
@@ -1391,22 +1402,43 @@ __global__ void hy_gather_rows_f32_kernel(const float* x, const int32_t* rows, f
     const int i = blockIdx.x;
     for (int c = threadIdx.x; c < W; c += blockDim.x) out[(long long)i * W + c] = x[(long long)rows[i] * W + c];
 }
-__global__ void __launch_bounds__(256) hy_argmax_rows_kernel(float* logits, int V, float softcap, int32_t* out_ids) {
+// One CTA per row; 16-byte loads, four in flight per thread, where rows start on 16 bytes (V a multiple of 4).  Latency-bound: four rows of 32
+// thousand logits 62 -> 9 us against one 4-byte load at a time on 256 threads.
+__global__ void __launch_bounds__(1024) hy_argmax_rows_kernel(float* logits, int V, float softcap, int32_t* out_ids) {
     HY_PDL();
-    __shared__ float bv[8]; __shared__ int bi[8];
+    __shared__ float bv[32]; __shared__ int bi[32];
     float* lr = logits + (long long)blockIdx.x * V;
     float v = -INFINITY; int i = 0x7fffffff;
-    for (int c = threadIdx.x; c < V; c += blockDim.x) {
-        float f = lr[c];
-        if (softcap > 0.f) { f = softcap * tanhf(f / softcap); lr[c] = f; }
-        if (f > v || (f == v && c < i)) { v = f; i = c; }
+    auto take = [&](float f, int c) { if (f > v || (f == v && c < i)) { v = f; i = c; } };
+    auto cap = [&](float f) { return softcap * tanhf(f / softcap); };
+    if ((V & 3) == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0) {
+        const int V4 = V / 4;
+        for (int c0 = threadIdx.x; c0 < V4; c0 += 4 * blockDim.x) {
+            float4 f[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) { const int c = c0 + k * blockDim.x; if (c < V4) f[k] = reinterpret_cast<const float4*>(lr)[c]; }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int c = c0 + k * blockDim.x;
+                if (c >= V4) break;
+                if (softcap > 0.f) { f[k] = make_float4(cap(f[k].x), cap(f[k].y), cap(f[k].z), cap(f[k].w)); reinterpret_cast<float4*>(lr)[c] = f[k]; }
+                take(f[k].x, 4 * c); take(f[k].y, 4 * c + 1); take(f[k].z, 4 * c + 2); take(f[k].w, 4 * c + 3);
+            }
+        }
+    } else {
+        for (int c = threadIdx.x; c < V; c += blockDim.x) {
+            float f = lr[c];
+            if (softcap > 0.f) { f = cap(f); lr[c] = f; }
+            take(f, c);
+        }
     }
     warp_argmax(v, i);
     if ((threadIdx.x & 31) == 0) { bv[threadIdx.x >> 5] = v; bi[threadIdx.x >> 5] = i; }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < 8; ++w) if (bv[w] > v || (bv[w] == v && bi[w] < i)) { v = bv[w]; i = bi[w]; }
-        out_ids[blockIdx.x] = i < V ? i : 0;
+    if (threadIdx.x < 32) {
+        v = bv[threadIdx.x]; i = bi[threadIdx.x];
+        warp_argmax(v, i);
+        if (threadIdx.x == 0) out_ids[blockIdx.x] = i < V ? i : 0;
     }
 }
 // gate / up products side by side in blocks of 16 -> gelu_tanh(gate) * up
@@ -1445,12 +1477,12 @@ cudaError_t hy_gemm(bool f32, int mode, const void* A, int lda, const void* B, i
     if (M <= 0 || N <= 0 || K <= 0 || batch <= 0) return cudaSuccess;
     auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
     if (!f32 && M <= HY_GEMM_FEW_ROWS && K % 8 == 0 && K <= 1024 && lda % 8 == 0 && ldb % 8 == 0 && sA % 8 == 0 && sB % 8 == 0 && al16(A) && al16(B)) {
-        const dim3 grid((N + 31) / 32, batch, (M + 15) / 16);
-        switch (mode) {
-            case HY_STORE: return launch_plain(hy_gemm_fewrows_kernel<HY_STORE>, grid, dim3(128), 0, s, (const bf*)A, lda, (const bf*)B, ldb, C, ldc, M, N, K, bias, alpha, sA, sB, sC, act);
-            case HY_STORE_F32: return launch_plain(hy_gemm_fewrows_kernel<HY_STORE_F32>, grid, dim3(128), 0, s, (const bf*)A, lda, (const bf*)B, ldb, C, ldc, M, N, K, bias, alpha, sA, sB, sC, act);
-            default: return launch_plain(hy_gemm_fewrows_kernel<HY_ACC_F32>, grid, dim3(128), 0, s, (const bf*)A, lda, (const bf*)B, ldb, C, ldc, M, N, K, bias, alpha, sA, sB, sC, act);
-        }
+        const bool split = K >= 256;
+        const dim3 grid(split ? (N + 7) / 8 : (N + 31) / 32, batch, (M + 15) / 16);
+#define HY_FEW(MODE) (split ? launch_plain(hy_gemm_fewrows_kernel<MODE, true>, grid, dim3(128), 0, s, (const bf*)A, lda, (const bf*)B, ldb, C, ldc, M, N, K, bias, alpha, sA, sB, sC, act) \
+                            : launch_plain(hy_gemm_fewrows_kernel<MODE, false>, grid, dim3(128), 0, s, (const bf*)A, lda, (const bf*)B, ldb, C, ldc, M, N, K, bias, alpha, sA, sB, sC, act))
+        return mode == HY_STORE ? HY_FEW(HY_STORE) : mode == HY_STORE_F32 ? HY_FEW(HY_STORE_F32) : HY_FEW(HY_ACC_F32);
+#undef HY_FEW
     }
     return f32 ? gemm_t<float>(mode, A, lda, B, ldb, C, ldc, M, N, K, bias, alpha, batch, sA, sB, sC, s, act)
                : gemm_t<bf>(mode, A, lda, B, ldb, C, ldc, M, N, K, bias, alpha, batch, sA, sB, sC, s, act);
@@ -1710,7 +1742,7 @@ cudaError_t hy_gather_rows_f32(const float* x, const int32_t* rows, float* out, 
 }
 cudaError_t hy_argmax_rows(float* logits, int n, int V, float softcap, int32_t* out_ids, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    return launch_plain(hy_argmax_rows_kernel, dim3(n), dim3(256), 0, s, logits, V, softcap, out_ids);
+    return launch_plain(hy_argmax_rows_kernel, dim3(n), dim3(1024), 0, s, logits, V, softcap, out_ids);
 }
 cudaError_t hy_gelu_glu(bool f32, const void* gu, int ld, void* out, int ldo, int ff, int T, cudaStream_t s) {
     const dim3 grid((ff + 255) / 256, T);
