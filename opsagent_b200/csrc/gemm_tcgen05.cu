@@ -342,10 +342,11 @@ static int gemm_rows_split(const GemmParams& p, int epilogue) {
 struct GemmChoice { bool pair; int split, rows; };
 static GemmChoice gemm_choose(const GemmParams& p, int epilogue, int block_n, bool room) {
     GemmChoice best{false, 1, 0};
+    if ((block_n != 32 && block_n != 64 && block_n != 128 && block_n != 256) || p.M <= 0 || p.N <= 0 || p.K <= 0) return best;      // refused by launch_gemm
     best.rows = gemm_rows_split(p, epilogue);
     if (best.rows) return best;
     const int sms = sm_count_cached(), pairs = sms / 2;
-    if (epilogue == EPI_LOGITS || p.m_tile_group || p.M <= BLOCK_M || pairs < 1) return best;
+    if (epilogue == EPI_LOGITS || p.m_tile_group || p.M <= BLOCK_M || pairs < 1 || std::getenv("OA_GEMM_PERSISTENT_MIN_TILES")) return best;      // (tests that drive the 128 x 256 kernel set it)
     auto up = [](long long a, long long b) { return (a + b - 1) / b; };
     const double kb = (double)up(p.K, BLOCK_K);
     double least = (double)up(up(p.N, block_n) * up(p.M, BLOCK_M), sms) * kb * (block_n >= 256 ? 0.42 : 0.26) + 8.0;
@@ -394,7 +395,7 @@ cudaError_t launch_gemm(const CUtensorMap* tmA, const CUtensorMap* tmB, const Ge
 }
 
 // =============================================================================================
-// persistent tile GEMM (prefill, M > 128): one CTA per SM loops over 128 x 256 tiles in grouped raster order; TMEM holds
+// persistent tile GEMM (grouped products, and prefill shapes that gemm_choose leaves here): one CTA per SM loops over 128 x 256 tiles in grouped raster order; TMEM holds
 // TWO accumulators so the epilogue of tile i (tcgen05.ld -> smem transpose -> coalesced bf16 stores, fused bias /
 // residual / SwiGLU) overlaps the tcgen05.mma main loop of tile i+1.
 // =============================================================================================
@@ -633,7 +634,7 @@ static cudaError_t launch_head(const CUtensorMap* tmA, const CUtensorMap* tmB, c
 }
 // the persistent kernel from two rounds of its tiles on; the narrow tiles of a small vocabulary fill the SMs better one CTA each
 static bool head_persistent(int M, int N) { return (long long)gemm_n_tiles(N, HeadCfg::BN) * ((M + BLOCK_M - 1) / BLOCK_M) >= 2LL * sm_count_cached(); }
-int gemm_logits_bn(int M, int N, int block_n) { return block_n >= HeadCfg::BN && head_persistent(M, N) ? HeadCfg::BN : block_n; }
+int gemm_logits_bn(int M, int N, int block_n) { return (block_n == 128 || block_n == 256) && head_persistent(M, N) ? HeadCfg::BN : block_n; }
 
 static bool persistent_disabled() { static const bool off = [] { const char* e = std::getenv("OA_GEMM_PERSISTENT"); return e && e[0] == '0'; }(); return off; }
 // tests lower the threshold (OA_GEMM_PERSISTENT_MIN_TILES=1) to drive tiny shapes through the persistent kernel

@@ -433,3 +433,15 @@ def test_persistent_vocabulary_head(L, M, N, K):
     mx = logits.max(dim=1, keepdim=True).values
     first = torch.where(logits == mx, torch.arange(N, device=dev())[None, :], N).min(dim=1).values
     assert (ids.long() == first).all() and (ids2 == ids).all() and ids[0].item() == N - 1
+
+
+@pytest.mark.parametrize("M", [5, 100, 700])
+@pytest.mark.parametrize("epi", [EPI_STORE, EPI_SWIGLU, EPI_LOGITS])
+@pytest.mark.parametrize("bn", [0, 16, 96, 192, 512, -64])
+def test_gemm_refuses_tile_widths_it_has_no_kernel_for(L, M, epi, bn):
+    """whatever kernel the shape would take: a width that is refused for one shape is refused for all"""
+    N, K = 40960, 64
+    A = torch.zeros(M, K, dtype=torch.bfloat16, device=dev()); B = torch.zeros(N, K, dtype=torch.bfloat16, device=dev())
+    out = torch.zeros(M, N, dtype=torch.bfloat16, device=dev()); ids = torch.zeros(M, dtype=torch.int32, device=dev())
+    assert L.oa_k_gemm(ptr(A), ptr(B), M, N, K, epi, bn, ptr(out), None, None, None, ptr(ids), None) != 0
+    torch.cuda.synchronize()
