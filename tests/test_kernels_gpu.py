@@ -445,3 +445,22 @@ def test_gemm_refuses_tile_widths_it_has_no_kernel_for(L, M, epi, bn):
     out = torch.zeros(M, N, dtype=torch.bfloat16, device=dev()); ids = torch.zeros(M, dtype=torch.int32, device=dev())
     assert L.oa_k_gemm(ptr(A), ptr(B), M, N, K, epi, bn, ptr(out), None, None, None, ptr(ids), None) != 0
     torch.cuda.synchronize()
+
+
+def test_gemm_with_cut_tiles_under_stream_capture(L):
+    """a product whose last round is cut takes scratch from the pool: captured, it replays to the same bits"""
+    M, N, K = 614, 4096, 14336
+    g = torch.Generator(device=dev()).manual_seed(5)
+    A = torch.randn(M, K, generator=g, device=dev()).to(torch.bfloat16); B = (torch.randn(N, K, generator=g, device=dev()) * 0.05).to(torch.bfloat16)
+    want = torch.empty(M, N, dtype=torch.bfloat16, device=dev()); got = torch.zeros_like(want)
+    assert L.oa_k_gemm(ptr(A), ptr(B), M, N, K, EPI_STORE, 256, ptr(want), None, None, None, None, None) == 0
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        rc = L.oa_k_gemm(ptr(A), ptr(B), M, N, K, EPI_STORE, 256, ptr(got), None, None, None, None, C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    for _ in range(3):
+        got.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(got, want)
