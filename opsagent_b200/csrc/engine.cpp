@@ -204,7 +204,7 @@ public:
             std::vector<std::shared_ptr<Seq>> batch; std::vector<int> take_of;
             // Entries of one token are decoding rows: as in the scheduler's mixed steps they come first and go to the decode attention kernel, which
             // reads a page once for all heads of its group and cuts long contexts over the chip (32 requests of 100 cached tokens, 32 / 8 heads of
-            // 128: 42 us a layer as query tiles of one row, 6 us as decoding rows).  Only where that kernel and its plan's buffers are made for it.
+            // 128: 42 us a layer as query tiles of one row, 13 us as decoding rows).  Only where that kernel and its plan's buffers are made for it.
             const ModelConfig& mc = model_.cfg;
             int singles = 0;
             for (int e = 0; e < n_entries; ++e) singles += n_tokens[e] == 1;
