@@ -1,9 +1,9 @@
-"""Host-side race / memory-error detection (SURVEY.md 5.2): the native HTTP front under TSAN and ASAN+UBSAN with a stub engine, and the parsers of
+"""Host-side race / memory-error detection: the native HTTP front under TSAN and ASAN+UBSAN with a stub engine, and the parsers of
 untrusted bytes (BPE, tokenizer.json, config JSON, safetensors headers, the ToolPrompt automaton + token masks) under ASAN+UBSAN.  The device side is
-covered by compute-sanitizer on the GPU box: tools/sanitize_gpu.sh, results in profiles/r02j_sanitizers.md."""
+covered by compute-sanitizer runs; results in profiles/r02j_sanitizers.md."""
 import pytest
 
-# ---- race / memory-error detection on the host side (SURVEY.md 5.2) -----------------------------------------------------------------------
+# ---- race / memory-error detection on the host side -----------------------------------------------------------------------
 import os
 import subprocess
 import sys
