@@ -121,13 +121,6 @@ int oa_k_gemm(const void* A, const void* B, int32_t M, int32_t N, int32_t K, int
     if (epilogue == EPI_LOGITS) block_n = gemm_logits_bn(M, N, block_n);
     p.few_rows_ok = 1;
     if (make_tmap_bf16_2d(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)K, (uint32_t)gemm_a_box(p, epilogue, block_n), 64) != 0) return OA_ERR_INTERNAL;
-    // room for cut tiles, where this product has any
-    const bool cut = gemm_may_split(p, epilogue, block_n);
-    DevBuf ws(cut ? GEMM_SPLIT_WS_BYTES + GEMM_SPLIT_COUNTERS * 4 : 0, s);
-    if (cut && ws.p) {
-        p.split_ws = (float*)ws.p; p.split_count = (unsigned int*)((char*)ws.p + GEMM_SPLIT_WS_BYTES);
-        if (cudaMemsetAsync(p.split_count, 0, GEMM_SPLIT_COUNTERS * 4, s) != cudaSuccess) return OA_ERR_INTERNAL;
-    }
     if (make_tmap_bf16_2d(&tmB, B, (uint64_t)N, (uint64_t)K, (uint64_t)K, (uint32_t)gemm_b_box(p, epilogue, block_n), 64) != 0) return OA_ERR_INTERNAL;
     if (epilogue == EPI_LOGITS) {
         const int nt = gemm_n_tiles(N, block_n);

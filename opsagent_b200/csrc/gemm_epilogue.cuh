@@ -23,28 +23,10 @@ OA_DEVINL void raster_tile(int idx, int m_tiles, int n_tiles, int& m_blk, int& n
     m_blk = m0 + within % rows; n_blk = within / rows;
 }
 
-// A tile whose k range two or three CTAs took: piece i's fp32 partial of this lane's row, columns 4 g .. 4 g + 3, is at part[i * stride + g * 512] (so
-// a warp's 16-byte accesses are contiguous); `own` is the piece in tensor memory.  n == 1: not cut.
-struct SplitTile { const float* part; int n, own; size_t stride; };
-// the other pieces' values of 32 columns, all loads in flight together
-OA_DEVINL void split_load(const SplitTile& cut, int col, float4 (&t)[2][8]) {
-#pragma unroll
-    for (int o = 0; o < 2; ++o) {
-        if (o + 1 >= cut.n) return;
-        const float* pc = cut.part + (size_t)(o < cut.own ? o : o + 1) * cut.stride + (size_t)col * 128;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) t[o][j] = __ldcg(reinterpret_cast<const float4*>(pc + j * 512));
-    }
-}
-OA_DEVINL void split_add(float (&a)[32], const float4 (&t)[8]) {
-#pragma unroll
-    for (int j = 0; j < 8; ++j) { a[4 * j] += t[j].x; a[4 * j + 1] += t[j].y; a[4 * j + 2] += t[j].z; a[4 * j + 3] += t[j].w; }
-}
-
 // One warp: rows row_base .. row_base + 31 (TMEM lanes of `acc`), columns n0 .. n0 + bn - 1 of the product.  glu_sc: scales of the two rows this
 // lane stores in a clamped gated activation.
 template <int EPI>
-OA_DEVINL void persist_epilogue(const GemmParams& p, float* stage, uint32_t acc, int row_base, int n0, int bn, int lane, const float (&glu_sc)[2], const SplitTile& cut) {
+OA_DEVINL void persist_epilogue(const GemmParams& p, float* stage, uint32_t acc, int row_base, int n0, int bn, int lane, const float (&glu_sc)[2]) {
     // residual of the columns at hand and, on their way meanwhile, of the next ones (each lane reads and writes its own places: out may be resid)
     uint4 res[4], res_next[4];
     auto load_res = [&](int cc, uint4 (&rr)[4]) {
@@ -55,32 +37,11 @@ OA_DEVINL void persist_epilogue(const GemmParams& p, float* stage, uint32_t acc,
         }
     };
     if (EPI == EPI_RESID) load_res(0, res_next);
-    float4 part[2][8];
-    if (cut.n > 1) split_load(cut, 0, part);
 #pragma unroll 1
     for (int cc = 0; cc < bn; cc += 32) {
         uint32_t v[32];
         tmem_ld_32x32b_x32(acc + (uint32_t)cc, v);
         tmem_ld_wait();
-        if (cut.n > 1) {                       // the pieces in k order, whichever CTA came last: a fixed order of summation
-            float4 next[2][8];                 // the next columns' values are on their way during this sum
-            if (cc + 32 < bn) split_load(cut, cc + 32, next);
-            float a[32];
-#pragma unroll
-            for (int j = 0; j < 32; ++j) a[j] = 0.f;
-            if (cut.own > 0) split_add(a, part[0]);
-            if (cut.own > 1) split_add(a, part[1]);
-#pragma unroll
-            for (int j = 0; j < 32; ++j) a[j] += __uint_as_float(v[j]);
-            if (cut.own == 0) split_add(a, part[0]);
-            if (cut.n == 3 && cut.own <= 1) split_add(a, part[1]);
-#pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(a[j]);
-#pragma unroll
-            for (int o = 0; o < 2; ++o)
-#pragma unroll
-                for (int j = 0; j < 8; ++j) part[o][j] = next[o][j];
-        }
         const int col0 = n0 + cc;
         if (EPI == EPI_RESID) {
 #pragma unroll

@@ -9,9 +9,9 @@
 //   warp 0   : TMA producer of this CTA's A rows and B half; both CTAs' bytes are counted on the EVEN CTA's `full` barrier
 //   warp 1   : allocates TMEM (both CTAs); in the even CTA one thread issues the products; commits release the ring slot in both CTAs
 //   warps 2-5: epilogue of this CTA's 128 rows while the next tile is multiplied (two accumulators of 256 columns)
-// Persistent over tiles in grouped raster order.  Where the tiles do not fill the last round, its tiles' k ranges are cut in two or three and the fp32
-// pieces added in a fixed order by whichever warp comes last (1337 x 4096 x 14336 residual, 96 tiles on 74 pairs: 152 -> 132 us; 400 x 4096 x 14336,
-// 32 tiles: 81 -> 62).
+// Persistent over tiles in grouped raster order.  Every tile sums its k blocks in ascending order in one accumulator, as the single-CTA kernels do: a
+// row's bits depend neither on how many rows share the product nor on its place among them.  (The last round's tiles cut along k filled idle pairs,
+// 16 to 20 us of a product whose tiles fill half a round, and gave that up: 1337 x 4096 x 14336 residual 156 -> 172, against 192 in single-CTA tiles.)
 #include <algorithm>
 
 #include "common.cuh"
@@ -66,7 +66,7 @@ OA_DEVINL void gp_wait(uint64_t* bar, uint32_t parity) {
 
 template <int EPI>
 __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                                                                  const GemmParams p, const int split) {
+                                                                  const GemmParams p) {
     extern __shared__ __align__(1024) uint8_t smem[];
     float* epi_smem = reinterpret_cast<float*>(smem + GP_STAGES * GP_STAGE_BYTES);
     uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + GP_STAGES * GP_STAGE_BYTES + 4 * EPI_WARP_BYTES);
@@ -79,14 +79,6 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
     const uint32_t rank = gp_rank();
     const int n_tiles = (p.N + GP_BN - 1) / GP_BN, m_tiles = (p.M + 255) / 256, tiles = n_tiles * m_tiles;
     const int num_kb = (p.K + GP_BK - 1) / GP_BK, pair = (int)blockIdx.x >> 1, pairs = (int)gridDim.x >> 1;
-    // Units of work: whole tiles while every pair gets one, then the pieces of the remaining tiles, `split` ranges of k blocks each
-    const int whole = split > 1 ? tiles / pairs * pairs : tiles, units = whole + (tiles - whole) * split;
-    struct Unit { int tile, piece, kb0, kb1; };
-    auto unit = [&](int u) {
-        if (u < whole) return Unit{u, -1, 0, num_kb};
-        const int j = u - whole, t = j / split, s = j - t * split;
-        return Unit{whole + t, j, (int)((long long)s * num_kb / split), (int)((long long)(s + 1) * num_kb / split)};
-    };
 
     if (warp == 0 && lane == 0) {
         tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmB);
@@ -109,11 +101,10 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
         if (lane == 0) {
             griddep_wait();
             int s = 0; uint32_t ph = 0;
-            for (int u = pair; u < units; u += pairs) {
-                const Unit w = unit(u);
-                int m_blk, n_blk; raster_tile(w.tile, m_tiles, n_tiles, m_blk, n_blk, GP_GROUP_M);
+            for (int t = pair; t < tiles; t += pairs) {
+                int m_blk, n_blk; raster_tile(t, m_tiles, n_tiles, m_blk, n_blk, GP_GROUP_M);
                 const int a_row = m_blk * 256 + (int)rank * 128, b_row = n_blk * GP_BN + (int)rank * 128;
-                for (int kb = w.kb0; kb < w.kb1; ++kb) {
+                for (int kb = 0; kb < num_kb; ++kb) {
                     gp_wait(&empty_bar[s], ph ^ 1);
                     uint8_t* dst = smem + s * GP_STAGE_BYTES;
                     if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * GP_STAGE_BYTES);      // both CTAs' A rows and B halves
@@ -132,19 +123,18 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
         if (rank == 0 && lane == 0) {
             constexpr uint32_t idesc = umma_idesc_bf16(256, GP_BN);
             int s = 0; uint32_t ph = 0; int it = 0;
-            for (int u = pair; u < units; u += pairs, ++it) {
-                const Unit w = unit(u);
+            for (int t = pair; t < tiles; t += pairs, ++it) {
                 const int as = it & 1;
                 gp_wait(&acc_empty[as], (((uint32_t)it >> 1) & 1) ^ 1);
                 tcgen05_fence_after();
                 const uint32_t tmem_d = tmem_base + (uint32_t)(as * GP_BN);
-                for (int kb = w.kb0; kb < w.kb1; ++kb) {
+                for (int kb = 0; kb < num_kb; ++kb) {
                     gp_wait(&full_bar[s], ph);
                     tcgen05_fence_after();
                     const uint32_t a_addr = smem_u32(smem + s * GP_STAGE_BYTES);
                     const uint64_t a_desc = umma_desc_sw128(a_addr), b_desc = umma_desc_sw128(a_addr + GP_A_BYTES);
 #pragma unroll
-                    for (int k = 0; k < GP_BK / 16; ++k) gp_umma(tmem_d, a_desc + (uint64_t)(k * 2), b_desc + (uint64_t)(k * 2), idesc, (kb > w.kb0 || k > 0) ? 1u : 0u);
+                    for (int k = 0; k < GP_BK / 16; ++k) gp_umma(tmem_d, a_desc + (uint64_t)(k * 2), b_desc + (uint64_t)(k * 2), idesc, (kb | k) != 0 ? 1u : 0u);
                     gp_commit(&empty_bar[s]);
                     if (++s == GP_STAGES) { s = 0; ph ^= 1; }
                 }
@@ -156,9 +146,8 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
         float* stage = epi_smem + (warp - 2) * (EPI_WARP_BYTES / 4);
         griddep_wait();
         int it = 0;
-        for (int u = pair; u < units; u += pairs, ++it) {
-            const Unit w = unit(u);
-            int m_blk, n_blk; raster_tile(w.tile, m_tiles, n_tiles, m_blk, n_blk, GP_GROUP_M);
+        for (int t = pair; t < tiles; t += pairs, ++it) {
+            int m_blk, n_blk; raster_tile(t, m_tiles, n_tiles, m_blk, n_blk, GP_GROUP_M);
             const int as = it & 1, row_base = m_blk * 256 + (int)rank * 128 + q * 32;
             const uint32_t acc = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * GP_BN);
             float glu_sc[2] = {0.f, 0.f};          // scales of the two rows this lane stores (clamped gated activation), read while the tile is still being multiplied
@@ -166,37 +155,7 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
                 for (int i2 = 0; i2 < 2; ++i2) if (row_base + i2 * 16 + (lane >> 1) < p.M) glu_sc[i2] = glu_row_scale(p, row_base + i2 * 16 + (lane >> 1));
             gp_wait(&acc_full[as], ((uint32_t)it >> 1) & 1);
             tcgen05_fence_after();
-            if (row_base < p.M) {
-                SplitTile cut{nullptr, 1, 0, 0};
-                bool finish = true;
-                if (w.piece >= 0) {
-                    // Publish this warp's rows of the piece, [column / 4][row][4]: contiguous 16-byte stores.  Whichever warp comes last for its rows of
-                    // the tile adds all pieces up and finishes them: nobody waits.
-                    const size_t stride = (size_t)2 * 128 * 256;
-                    const int t = w.tile - whole, own = w.piece - t * split;
-                    float* mine = p.split_ws + ((size_t)w.piece * 2 + rank) * (128 * 256) + (q * 32 + lane) * 4;
-#pragma unroll 1
-                    for (int c = 0; c < GP_BN; c += 32) {
-                        uint32_t v[32];
-                        tmem_ld_32x32b_x32(acc + (uint32_t)c, v);
-                        tmem_ld_wait();
-#pragma unroll
-                        for (int j = 0; j < 8; ++j)
-                            *reinterpret_cast<float4*>(mine + (c * 128 + j * 512)) = make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]), __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
-                    }
-                    __threadfence();
-                    __syncwarp();
-                    unsigned int* count = p.split_count + (t * 2 + (int)rank) * 4 + q;
-                    int last = 0;
-                    if (lane == 0) {
-                        last = atomicAdd(count, 1u) == (unsigned int)(split - 1);
-                        if (last) { *count = 0u; __threadfence(); }
-                    }
-                    finish = __shfl_sync(0xffffffffu, last, 0) != 0;
-                    cut = SplitTile{mine - (size_t)own * stride, split, own, stride};
-                }
-                if (finish) persist_epilogue<EPI>(p, stage, acc, row_base, n_blk * GP_BN, GP_BN, lane, glu_sc, cut);
-            }
+            if (row_base < p.M) persist_epilogue<EPI>(p, stage, acc, row_base, n_blk * GP_BN, GP_BN, lane, glu_sc);
             tcgen05_fence_before();
             __syncwarp();
             if (lane == 0) gp_arrive_remote(gp_mapa(&acc_empty[as], 0));
@@ -212,31 +171,28 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
 }
 
 template <int EPI>
-static cudaError_t launch_gp(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int split, int sms, cudaStream_t stream) {
+static cudaError_t launch_gp(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int sms, cudaStream_t stream) {
     auto kern = gemm_pair_kernel<EPI>;
     static bool attr_done[16] = {};
     { cudaError_t e = ensure_dynamic_smem(kern, GP_SMEM_BYTES, attr_done); if (e != cudaSuccess) return e; }
-    const int tiles = ((p.N + GP_BN - 1) / GP_BN) * ((p.M + 255) / 256), rest = tiles % (sms / 2);
-    if (split < 1 || split > (p.K + GP_BK - 1) / GP_BK) return cudaErrorInvalidValue;
-    if (split > 1 && (!p.split_ws || !p.split_count || split > 3 || rest * split > GEMM_SPLIT_SLOTS)) return cudaErrorInvalidValue;
-    const int units = split > 1 ? tiles - rest + rest * split : tiles;
+    const int tiles = ((p.N + GP_BN - 1) / GP_BN) * ((p.M + 255) / 256);
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * std::min(units, sms / 2)); cfg.blockDim = dim3(GP_THREADS); cfg.dynamicSmemBytes = GP_SMEM_BYTES; cfg.stream = stream;
+    cfg.gridDim = dim3(2 * std::min(tiles, sms / 2)); cfg.blockDim = dim3(GP_THREADS); cfg.dynamicSmemBytes = GP_SMEM_BYTES; cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension; attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr; cfg.numAttrs = pdl_enabled() ? 2 : 1;
     count_launch();
-    return cudaLaunchKernelEx(&cfg, kern, *tmA, *tmB, p, split);
+    return cudaLaunchKernelEx(&cfg, kern, *tmA, *tmB, p);
 }
 
-cudaError_t launch_gemm_pair(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epilogue, int split, int sms, cudaStream_t stream) {
+cudaError_t launch_gemm_pair(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epilogue, int sms, cudaStream_t stream) {
     if (p.m_tile_group || sms < 2) return cudaErrorInvalidValue;
     switch (epilogue) {
-        case EPI_STORE: return launch_gp<EPI_STORE>(tmA, tmB, p, split, sms, stream);
-        case EPI_RESID: return launch_gp<EPI_RESID>(tmA, tmB, p, split, sms, stream);
-        case EPI_SWIGLU: return launch_gp<EPI_SWIGLU>(tmA, tmB, p, split, sms, stream);
-        case EPI_F32: return launch_gp<EPI_F32>(tmA, tmB, p, split, sms, stream);
+        case EPI_STORE: return launch_gp<EPI_STORE>(tmA, tmB, p, sms, stream);
+        case EPI_RESID: return launch_gp<EPI_RESID>(tmA, tmB, p, sms, stream);
+        case EPI_SWIGLU: return launch_gp<EPI_SWIGLU>(tmA, tmB, p, sms, stream);
+        case EPI_F32: return launch_gp<EPI_F32>(tmA, tmB, p, sms, stream);
     }
     return cudaErrorInvalidValue;
 }

@@ -321,11 +321,6 @@ static long long persistent_min_tiles();
 template <int EPI>
 static cudaError_t launch_persistent(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, cudaStream_t stream);
 
-// CTA-pair kernel or one of the kernels here, and whether the last round's tiles are cut: the least estimate of rounds x k blocks x time of a k block
-// plus what a launch costs besides.  Constants in us fitted to a sweep of 200 .. 8192 rows over the projections of the four model sizes: a k block
-// takes 0.345 in a pair (0.39 once more than two rounds run against the power cap), 0.42 in a 128 x 256 tile and 0.26 in a narrower one; outside the
-// k loop 11 and 8; cutting adds 16 (publishing and adding the pieces; 5 of it is the counters' memset of a single call).  E.g. 200 x 4096 x 4096: 64
-// tiles of 128 x 64 24 us, 16 pair tiles 32; 400 rows: 44 and 32.  Up to 128 rows half of a pair's rows would be padding.
 // Cluster size of the few-row kernel for this product, or 0: one of the kernels here takes it.  The largest that keeps the CTAs within 7/4 of the SMs
 // (two are resident on one; measured 16 .. 224 tiles of 128 weight rows).  Every row costs its exchange, S CTAs' worth, so with more rows it takes
 // more of a k range per CTA to pay: up to 16 rows always (28672 x 4096: 41 us against 42; 8192 x 2048: 9 against 17), up to 32 with four CTAs a
@@ -339,9 +334,13 @@ static int gemm_rows_split(const GemmParams& p, int epilogue) {
     const bool pays = p.M <= 16 || (p.M <= 32 && s >= 4) || (p.M <= 64 && (s == 8 || (s == 4 && kb >= 64))) || (s == 4 && kb >= 64);
     return pays ? s : 0;
 }
-struct GemmChoice { bool pair; int split, rows; };
-static GemmChoice gemm_choose(const GemmParams& p, int epilogue, int block_n, bool room) {
-    GemmChoice best{false, 1, 0};
+// CTA-pair kernel or one of the kernels here: the least estimate of rounds x k blocks x time of a k block plus what a launch costs besides.  Constants in
+// us fitted to a sweep of 200 .. 8192 rows over the projections of the four model sizes: a k block takes 0.345 in a pair (0.39 once more than two rounds
+// run against the power cap), 0.42 in a 128 x 256 tile and 0.26 in a narrower one; outside the k loop 11 and 8.  E.g. 200 x 4096 x 4096: 64 tiles of 128
+// x 64 24 us, 16 pair tiles 32.  Up to 128 rows half of a pair's rows would be padding.  These kernels sum k in the same order: the choice moves no bit.
+struct GemmChoice { bool pair; int rows; };
+static GemmChoice gemm_choose(const GemmParams& p, int epilogue, int block_n) {
+    GemmChoice best{false, 0};
     if ((block_n != 32 && block_n != 64 && block_n != 128 && block_n != 256) || p.M <= 0 || p.N <= 0 || p.K <= 0) return best;      // refused by launch_gemm
     best.rows = gemm_rows_split(p, epilogue);
     if (best.rows) return best;
@@ -349,22 +348,16 @@ static GemmChoice gemm_choose(const GemmParams& p, int epilogue, int block_n, bo
     if (epilogue == EPI_LOGITS || p.m_tile_group || p.M <= BLOCK_M || pairs < 1 || std::getenv("OA_GEMM_PERSISTENT_MIN_TILES")) return best;      // (tests that drive the 128 x 256 kernel set it)
     auto up = [](long long a, long long b) { return (a + b - 1) / b; };
     const double kb = (double)up(p.K, BLOCK_K);
-    double least = (double)up(up(p.N, block_n) * up(p.M, BLOCK_M), sms) * kb * (block_n >= 256 ? 0.42 : 0.26) + 8.0;
-    const long long tiles = up(p.N, 256) * up(p.M, 256), rest = tiles % pairs;
-    for (int s = 1; s <= (room ? 3 : 1); ++s) {
-        if (s > 1 && (rest == 0 || rest * s > GEMM_SPLIT_SLOTS || kb < 4 * s)) continue;
-        const double rounds = s == 1 ? (double)up(tiles, pairs) : (double)(tiles / pairs) + (double)up(rest * s, pairs) / s;
-        const double est = rounds * kb * (rounds > 2 ? 0.39 : 0.345) + 11.0 + (s > 1 ? 16.0 : 0.0);
-        if (est < least) { least = est; best = GemmChoice{true, s, 0}; }
-    }
+    const double single = (double)up(up(p.N, block_n) * up(p.M, BLOCK_M), sms) * kb * (block_n >= 256 ? 0.42 : 0.26) + 8.0;
+    const double rounds = (double)up(up(p.N, 256) * up(p.M, 256), pairs), pair = rounds * kb * (rounds > 2 ? 0.39 : 0.345) + 11.0;
+    best.pair = pair < single;
     return best;
 }
 int gemm_b_box(const GemmParams& p, int epilogue, int block_n) {
-    const GemmChoice c = gemm_choose(p, epilogue, block_n, p.split_ws && p.split_count);
+    const GemmChoice c = gemm_choose(p, epilogue, block_n);
     return c.pair || c.rows ? 128 : block_n;
 }
-int gemm_a_box(const GemmParams& p, int epilogue, int block_n) { return gemm_choose(p, epilogue, block_n, false).rows ? gemm_rows_box(p.M) : 128; }
-bool gemm_may_split(const GemmParams& p, int epilogue, int block_n) { return gemm_choose(p, epilogue, block_n, true).split > 1; }
+int gemm_a_box(const GemmParams& p, int epilogue, int block_n) { return gemm_choose(p, epilogue, block_n).rows ? gemm_rows_box(p.M) : 128; }
 
 cudaError_t launch_gemm(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epilogue, int block_n,
                         cudaStream_t stream) {
@@ -372,9 +365,9 @@ cudaError_t launch_gemm(const CUtensorMap* tmA, const CUtensorMap* tmB, const Ge
     if (epilogue == EPI_SWIGLU && (p.N % 32) != 0) return cudaErrorInvalidValue;
     // large-M (prefill) shapes with the widest tile go to the persistent kernel (epilogue overlapped with the next tile)
     if (epilogue == EPI_F32 && ((p.ldf % 4) != 0 || !p.f32_out)) return cudaErrorInvalidValue;
-    const GemmChoice choice = gemm_choose(p, epilogue, block_n, p.split_ws && p.split_count);
+    const GemmChoice choice = gemm_choose(p, epilogue, block_n);
     if (choice.rows) return launch_gemm_rows(tmA, tmB, p, epilogue, choice.rows, stream);
-    if (choice.pair) return launch_gemm_pair(tmA, tmB, p, epilogue, choice.split, sm_count_cached(), stream);
+    if (choice.pair) return launch_gemm_pair(tmA, tmB, p, epilogue, sm_count_cached(), stream);
     if (block_n == 256 && epilogue != EPI_LOGITS && !persistent_disabled() &&
         (long long)((p.N + 255) / 256) * ((p.M + BLOCK_M - 1) / BLOCK_M) >= persistent_min_tiles()) {
         switch (epilogue) {
@@ -500,7 +493,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_persistent_kernel(const 
                 for (int i2 = 0; i2 < 2; ++i2) if (row_base + i2 * 16 + (lane >> 1) < p.M) glu_sc[i2] = glu_row_scale(p, row_base + i2 * 16 + (lane >> 1));
             mbar_wait(&acc_full[as], ((uint32_t)it >> 1) & 1);
             tcgen05_fence_after();
-            persist_epilogue<EPI>(p, stage, tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * BN), row_base, n_blk * BN, BN, lane, glu_sc, SplitTile{nullptr, 1, 0, 0});
+            persist_epilogue<EPI>(p, stage, tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * BN), row_base, n_blk * BN, BN, lane, glu_sc);
             tcgen05_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&acc_empty[as]);

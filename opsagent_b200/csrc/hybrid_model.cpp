@@ -518,7 +518,6 @@ HybridModel::HybridModel(const ModelConfig& c, const EngineOptions& o) : ModelBa
         ld_gates_ = max_gates; gates_ = (float*)dmalloc(MR * ld_gates_ * 4);
         gin_ = (float*)dmalloc(MR * max_h * 4); floor_ = (float*)dmalloc(MR * max_h * 4); ndot_ = (float*)dmalloc(MR * max_h * 4);
     }
-    if (!f32_ && opt.hy_tensor_core) { gemm_split_ws_ = (float*)dmalloc(GEMM_SPLIT_WS_BYTES); gemm_split_count_ = (unsigned int*)dmalloc(GEMM_SPLIT_COUNTERS * 4); }
     hs_ = dmalloc((size_t)MS_ * Wld_ * es_); d_out_ids_ = (int32_t*)dmalloc((size_t)MS_ * 4);
     logits_ = (float*)dmalloc((size_t)opt.max_batch * V * 4);      // own logits: sampling steps only (one row per sequence)
     cuda_check(cudaMallocHost(&h_out_ids, (size_t)MS_ * 4), "cudaMallocHost");
@@ -596,7 +595,7 @@ void HybridModel::gemm(int mode, const void* A, int lda, const Mat& B, void* C, 
     bool tc = B.tc && !f32_ && lda % 8 == 0 && aligned16(A) && lda >= B.ld;
     if (mode == HY_STORE) tc = tc && ldc % 8 == 0 && aligned16(C) && (!bias || (bias_act && aligned16(bias_act))) && alpha == 1.f;     // a bias in the activation type, padded to N rounded up to 8
     else tc = tc && B.N % 8 == 0 && ldc % 4 == 0 && aligned16(C) && (!bias || aligned16(bias)) && act.kind == 0;
-    GemmParams g{}; g.M = M; g.N = up8(B.N); g.K = B.ld; g.split_ws = gemm_split_ws_; g.split_count = gemm_split_count_; g.few_rows_ok = 1;
+    GemmParams g{}; g.M = M; g.N = up8(B.N); g.K = B.ld; g.few_rows_ok = 1;
     const int bn = pick_tile_n(M, g.N, sm_count), epi = mode == HY_STORE ? EPI_STORE : EPI_F32;
     CUtensorMap tmA;
     if (tc && make_tmap_bf16_2d(&tmA, A, (uint64_t)M, (uint64_t)B.ld, (uint64_t)lda, (uint32_t)gemm_a_box(g, epi, bn), 64) != 0) tc = false;
@@ -614,7 +613,7 @@ bool HybridModel::moe(const LayerW& w, const HyLayer& l, const void* h_in, const
     if (hc_.sequential) { out = y_; beta = 0.f; }        // the residual is closed by whoever opens the next sublayer
     const bool relu2 = m.act == HY_EXPERT_RELU2; const int rows1 = relu2 ? w.ffp : 2 * w.ffp;
     if (m.dense && m.act == HY_EXPERT_GELU_GLU) {        // gated: both halves in one product, gelu(gate) * up in its epilogue
-        GemmParams g{}; g.M = T; g.N = w.up.N; g.K = w.up.ld; g.out = act_; g.ldo = w.ffp; g.glu_gelu = 1; g.split_ws = gemm_split_ws_; g.split_count = gemm_split_count_; g.few_rows_ok = 1;
+        GemmParams g{}; g.M = T; g.N = w.up.N; g.K = w.up.ld; g.out = act_; g.ldo = w.ffp; g.glu_gelu = 1; g.few_rows_ok = 1;
         const int bn = pick_tile_n(T, g.N, sm_count), box = gemm_b_box(g, EPI_SWIGLU, bn);
         CUtensorMap tmA;
         if (w.up.tc && make_tmap_bf16_2d(&tmA, h_in, (uint64_t)T, (uint64_t)w.up.ld, (uint64_t)Wld_, (uint32_t)gemm_a_box(g, EPI_SWIGLU, bn), 64) == 0) {

@@ -124,7 +124,6 @@ private:
     std::vector<int32_t> ptile_seq_, ptile_head_, ptile_row0_, seq_base_;
     void *lat_ctx_ = nullptr, *kv_ctx_ = nullptr; int ld_kv_ = 0, ctx_cap_ = 0;    // prefill form of attention: gathered cache rows of whole contexts and their keys / values
     float *split_o_ = nullptr, *split_ml_ = nullptr; int split_slots_ = 0;       // partials of decoding rows whose cache rows are cut into parts
-    float* gemm_split_ws_ = nullptr; unsigned int* gemm_split_count_ = nullptr;  // pieces and counters of cut GEMM tiles (self-resetting)
 };
 
 }  // namespace oa

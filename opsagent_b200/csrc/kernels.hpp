@@ -41,9 +41,6 @@ struct GemmParams {
     // EPI_SWIGLU with glu_limit > 0: out = g sigmoid(glu_slope g) (u + 1), g = min(s gate, limit), u = clamp(s up, -limit, limit), where row r's s is
     // row_scale[row_scale_idx[r]] (0 for a negative index: a padding row of a grouped product) — the router's weight on an expert's input, exact in fp32
     float glu_limit, glu_slope; const float* row_scale; const int32_t* row_scale_idx;
-    // room for the fp32 partials of tiles whose k range is cut (GEMM_SPLIT_WS_BYTES) and their counters (GEMM_SPLIT_COUNTERS, zero between launches: the
-    // kernel re-arms them); null: tiles are never cut
-    float* split_ws; unsigned int* split_count;
     int few_rows_ok;                // the caller's A map has the box gemm_a_box() asks for (else 128 rows)
     int glu_gelu;                   // EPI_SWIGLU: the gate passes the tanh form of GELU instead of SiLU
 };
@@ -54,17 +51,14 @@ int gemm_n_tiles(int N, int block_n);
 int gemm_logits_bn(int M, int N, int block_n);      // EPI_LOGITS: the tile width to ask launch_gemm for (and to count the arg-max partials by) where block_n would do
 // rows of the B tensor map's box that launch_gemm(.., block_n, ..) reads for this product: block_n, or what the CTA-pair kernel takes where that runs
 int gemm_b_box(const GemmParams& p, int epilogue, int block_n);
-bool gemm_may_split(const GemmParams& p, int epilogue, int block_n);      // the product has tiles worth cutting if GemmParams::split_ws gives room
 // rows of the A tensor map's box that launch_gemm reads for this product: 128, or what the few-row kernel takes where that runs (only with few_rows_ok)
 int gemm_a_box(const GemmParams& p, int epilogue, int block_n);
 // few-row kernel (gemm_rows.cu), M <= 128: weights in the tensor core's rows, a cluster of S = 1, 2, 4 or 8 CTAs per 128 weight rows; tmA: box {64,
 // gemm_rows_box(M)}, tmB: box {64, 128}
 inline int gemm_rows_box(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 0; }
 cudaError_t launch_gemm_rows(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epilogue, int S, cudaStream_t stream);
-// CTA-pair kernel (gemm_pair.cu): tiles of 256 x 256; tmB: box {64, 128}; split > 1: the last round's tiles are cut into that many ranges of k (2 or 3)
-cudaError_t launch_gemm_pair(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epilogue, int split, int sms, cudaStream_t stream);
-constexpr int GEMM_SPLIT_SLOTS = 148, GEMM_SPLIT_COUNTERS = GEMM_SPLIT_SLOTS * 8;      // pieces of cut tiles per launch; counters: one per tile, CTA and warp
-constexpr size_t GEMM_SPLIT_WS_BYTES = (size_t)GEMM_SPLIT_SLOTS * 256 * 256 * 4;
+// CTA-pair kernel (gemm_pair.cu): tiles of 256 x 256; tmB: box {64, 128}
+cudaError_t launch_gemm_pair(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epilogue, int sms, cudaStream_t stream);
 // ---- stream-K variant for decode (M <= 128): persistent, one CTA per SM; work unit = (n_tile, 64-wide k block),
 // units dealt out contiguously so every SM streams the same number of weight bytes.  Each CTA writes the fp32
 // partial of every tile segment it owns to ws[slot = cta + tile][128][BN]; consumers (sk_* kernels) add a tile's

@@ -208,9 +208,6 @@ DeviceModel::DeviceModel(const ModelConfig& c, const EngineOptions& o) : ModelBa
         sk_ws_ = reinterpret_cast<float*>(dmalloc(wsb));
         tile_flags_ = reinterpret_cast<unsigned int*>(dmalloc((size_t)4 * SK_MAX_FLAG_TILES * 4));
         cuda_check(cudaMemset(tile_flags_, 0, (size_t)4 * SK_MAX_FLAG_TILES * 4), "stream-K tile flags memset");
-        split_ws_ = reinterpret_cast<float*>(dmalloc(GEMM_SPLIT_WS_BYTES));
-        split_count_ = reinterpret_cast<unsigned int*>(dmalloc(GEMM_SPLIT_COUNTERS * 4));
-        cuda_check(cudaMemset(split_count_, 0, GEMM_SPLIT_COUNTERS * 4), "split counters memset");
         // 32-bit index arithmetic in the consumers: (units of the largest shape + kb) * G must stay below 2^32
         const double worst = ((double)((2 * F + sk_bn_ - 1) / sk_bn_) * ((std::max(H, F) + 63) / 64) + (std::max(H, F) + 63) / 64) * sk_G_;
         if (worst >= 4.0e9) throw std::runtime_error("stream-K index range exceeds 32 bits for this model");
@@ -590,31 +587,31 @@ void DeviceModel::forward(const StepInput& in, float* logits_out) {
         for (int l = 0; l < L; ++l) {
             const Layer& ly = layers[l];
             cuda_check(launch_rmsnorm(x_, ly.ln1, xn_, T, H, cfg.rms_eps, stream), "rmsnorm1"); MARK(1);
-            GemmParams g{}; g.M = T; g.N = qkvd; g.split_ws = split_ws_; g.split_count = split_count_; g.K = H; g.out = qkv_; g.ldo = qkvd; g.bias = ly.bqkv;
+            GemmParams g{}; g.M = T; g.N = qkvd; g.K = H; g.out = qkv_; g.ldo = qkvd; g.bias = ly.bqkv;
             cuda_check(launch_gemm(&tm_xn_, ly.qkv.map(gemm_b_box(g, EPI_STORE, bn_qkv)), g, EPI_STORE, bn_qkv, stream), "qkv gemm"); MARK(2);
             cuda_check(launch_rope_kv_write(qkv_, d_pos, d_slot, rope_cos, rope_sin, q_, kv, l, T, nh, stream), "rope"); MARK(3);
             attention(l);
             if (use_tp) {      // bf16 partial -> symmetric buffer, barrier, x += sum over ranks (rank order)
                 const int b = comm->next_buffer();
-                GemmParams go{}; go.M = T; go.split_ws = split_ws_; go.split_count = split_count_; go.N = H; go.K = qd; go.out = comm->sym(b); go.ldo = H;
+                GemmParams go{}; go.M = T; go.N = H; go.K = qd; go.out = comm->sym(b); go.ldo = H;
                 cuda_check(launch_gemm(&tm_attn_, ly.o.map(gemm_b_box(go, EPI_STORE, bn_o)), go, EPI_STORE, bn_o, stream), "o gemm"); MARK(6);
                 cuda_check(comm->barrier(stream), "xgpu barrier");
                 allreduce_resid_bf16(b);
             } else {
-                GemmParams go{}; go.M = T; go.split_ws = split_ws_; go.split_count = split_count_; go.N = H; go.K = qd; go.out = x_; go.ldo = H; go.resid = x_; go.ldr = H;
+                GemmParams go{}; go.M = T; go.N = H; go.K = qd; go.out = x_; go.ldo = H; go.resid = x_; go.ldr = H;
                 cuda_check(launch_gemm(&tm_attn_, ly.o.map(gemm_b_box(go, EPI_RESID, bn_o)), go, EPI_RESID, bn_o, stream), "o gemm"); MARK(6);
             }
             cuda_check(launch_rmsnorm(x_, ly.ln2, xn_, T, H, cfg.rms_eps, stream), "rmsnorm2"); MARK(1);
-            GemmParams gg{}; gg.M = T; gg.split_ws = split_ws_; gg.split_count = split_count_; gg.N = 2 * F; gg.K = H; gg.out = act_; gg.ldo = F;
+            GemmParams gg{}; gg.M = T; gg.N = 2 * F; gg.K = H; gg.out = act_; gg.ldo = F;
             cuda_check(launch_gemm(&tm_xn_, ly.gu.map(gemm_b_box(gg, EPI_SWIGLU, bn_gu)), gg, EPI_SWIGLU, bn_gu, stream), "gate_up gemm"); MARK(8);
             if (use_tp) {
                 const int b = comm->next_buffer();
-                GemmParams gd{}; gd.M = T; gd.split_ws = split_ws_; gd.split_count = split_count_; gd.N = H; gd.K = F; gd.out = comm->sym(b); gd.ldo = H;
+                GemmParams gd{}; gd.M = T; gd.N = H; gd.K = F; gd.out = comm->sym(b); gd.ldo = H;
                 cuda_check(launch_gemm(&tm_act_, ly.down.map(gemm_b_box(gd, EPI_STORE, bn_down)), gd, EPI_STORE, bn_down, stream), "down gemm"); MARK(10);
                 cuda_check(comm->barrier(stream), "xgpu barrier");
                 allreduce_resid_bf16(b);
             } else {
-                GemmParams gd{}; gd.M = T; gd.split_ws = split_ws_; gd.split_count = split_count_; gd.N = H; gd.K = F; gd.out = x_; gd.ldo = H; gd.resid = x_; gd.ldr = H;
+                GemmParams gd{}; gd.M = T; gd.N = H; gd.K = F; gd.out = x_; gd.ldo = H; gd.resid = x_; gd.ldr = H;
                 cuda_check(launch_gemm(&tm_act_, ly.down.map(gemm_b_box(gd, EPI_RESID, bn_down)), gd, EPI_RESID, bn_down, stream), "down gemm"); MARK(10);
             }
         }

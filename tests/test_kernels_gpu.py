@@ -464,3 +464,36 @@ def test_gemm_with_cut_tiles_under_stream_capture(L):
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(got, want)
+
+
+# A row of a product has the same bits whatever shares the product with it: every kernel and tile width sums k in ascending order in one accumulator.
+# Rows alone or among others, at another place of the batch, on both sides of every kernel's and tile width's border.
+def _products(L, A, B, x, widths):
+    """every epilogue's result over these rows, per tile width"""
+    (M, K), N = A.shape, B.shape[0]
+    outs = []
+    for bn in widths:
+        y = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=dev()); r = x[:M].clone(); h = torch.full((M, N // 2), float("nan"), dtype=torch.bfloat16, device=dev())
+        assert L.oa_k_gemm(ptr(A), ptr(B), M, N, K, EPI_STORE, bn, ptr(y), ptr(B[0, :1].expand(N).contiguous()), None, None, None, None) == 0
+        assert L.oa_k_gemm(ptr(A), ptr(B), M, N, K, EPI_RESID, bn, ptr(r), None, ptr(r), None, None, None) == 0
+        assert L.oa_k_gemm(ptr(A), ptr(B), M, N, K, EPI_SWIGLU, bn, ptr(h), None, None, None, None, None) == 0
+        torch.cuda.synchronize()
+        outs.append((y, r, h))
+    return outs
+
+
+def _bits_follow_the_row(L, N, K, total, spans, widths):
+    g = torch.Generator(device=dev()).manual_seed(N + K)
+    A = torch.randn(total, K, generator=g, device=dev()).to(torch.bfloat16)
+    B = (torch.randn(N, K, generator=g, device=dev()) * 0.05).to(torch.bfloat16)
+    x = torch.randn(1, N, generator=g, device=dev()).to(torch.bfloat16).expand(total, N).contiguous()
+    whole = _products(L, A, B, x, widths[:1])[0]
+    for r0, r1 in spans:
+        for bn, got in zip(widths, _products(L, A[r0:r1].contiguous(), B, x, widths)):
+            for name, w, v in zip(("store", "residual", "gated"), whole, got):
+                assert torch.equal(v, w[r0:r1]), (r0, r1, bn, name, int((v != w[r0:r1]).sum()))
+
+
+@pytest.mark.parametrize("N,K", [(4096, 14336), (4096, 4096), (6144, 4096), (2048, 2048), (1024, 328)])
+def test_prefill_rows_keep_their_bits_beside_others(L, N, K):
+    _bits_follow_the_row(L, N, K, 1337, [(0, 1337), (0, 129), (0, 200), (100, 357), (0, 400), (700, 1314), (313, 1337)], (256, 128, 64))
