@@ -40,6 +40,20 @@ struct GemmCfg {
     static constexpr uint32_t TMEM_COLS = BN < 32 ? 32 : BN;
 };
 
+// FEW: a product of up to 64 rows loads only the 16, 32 or 64 of them (the box of tmA) and keeps more stages of the narrower ring in flight.  Its
+// products, their order and so every bit are those of the plain form: a decoding row must not feel how many requests share its step.  (Sharing a tile's k
+// range over a cluster is faster, 7.0 against 12.6 us for 16 x 2048 x 4096, and gives that up.)  What bounds it is the chain of one tile's k blocks, 0.16
+// us each at a width of 32; us, 128 rows loaded -> here: 16 x 2048 x 4096 18.6 -> 12.6, 16 x 4096 x 14336 62 -> 42, 64 x 6144 x 4096 20.8 -> 15.6.
+struct FewRing { int a_rows, stages; };
+static constexpr int FEW_MAX_ROWS = 64, FEW_BAR_BYTES = 512;
+static int few_box(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : 64; }
+static FewRing few_ring(int M, int N, int bn, int sms) {
+    // 130 KB in flight a CTA; with more tiles than SMs 96 KB, so that two CTAs fit one (16 x 8192 x 2048 in 256 tiles: 17.3 us alone on an SM, 10.3 in
+    // twos).  A hybrid model's step with 100, 130, 160 and 200 KB: 4517, 4390, 4401 and 4426 us a pass.
+    const int a_rows = few_box(M), stage = (a_rows + bn) * BLOCK_K * 2;
+    return FewRing{a_rows, std::max(4, std::min(28, ((N + bn - 1) / bn > sms ? 96 : 130) * 1024 / stage))};
+}
+
 // 32 columns of one row of the vocabulary head: the row's running arg-max (ties: lowest column) and, where wanted, the logits
 OA_DEVINL const uint32_t* logits_mask(const GemmParams& p, int row) {
     const int ms = p.mask_slot ? p.mask_slot[row] : -1;
@@ -76,20 +90,23 @@ OA_DEVINL void logits_chunk(const GemmParams& p, int row, const uint32_t (&v)[32
     }
 }
 
-template <int BN, int EPI>
+template <int BN, int EPI, bool FEW>
 __global__ void __launch_bounds__(GEMM_THREADS) gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
                                                                       const __grid_constant__ CUtensorMap tmB,
-                                                                      const GemmParams p) {
+                                                                      const GemmParams p, const FewRing few) {
     using Cfg = GemmCfg<BN>;
-    constexpr int STAGES = Cfg::STAGES;
+    // ring: [stage][A | B]; FEW: [stage][A], then [stage][B], A stages of the rows there are
+    const int STAGES = FEW ? few.stages : Cfg::STAGES, A_BYTES = FEW ? few.a_rows * BLOCK_K * 2 : Cfg::A_BYTES;
+    const int A_STRIDE = FEW ? A_BYTES : Cfg::STAGE_BYTES, B_STRIDE = FEW ? Cfg::B_BYTES : Cfg::STAGE_BYTES, B_AT = FEW ? STAGES * A_BYTES : Cfg::A_BYTES;
+    const uint32_t STAGE_TX = (uint32_t)(A_BYTES + Cfg::B_BYTES);
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * Cfg::STAGE_BYTES);
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * (int)STAGE_TX);
     uint64_t* empty_bar = full_bar + STAGES;
     uint64_t* acc_bar = empty_bar + STAGES;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_bar + 1);
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);      // warp-uniform, and known to be
     const int lane = threadIdx.x & 31;
     // Grouped rasterisation: CTAs walk bands of RASTER_GROUP_M row tiles, M fastest inside a band, so a band of A
     // (16 x 128 rows) stays L2-resident while each B tile is streamed from HBM once per band instead of once per row tile.
@@ -121,51 +138,52 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_tcgen05_kernel(const __grid
     tcgen05_fence_before();
     __syncthreads();
     tcgen05_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     griddep_launch();
 
     if (warp == 0) {
-        if (lane == 0) {
-            // weights (B) are written by no kernel of the chain: fill the ring with them BEFORE waiting for the predecessor
-            const int pre = num_kb < STAGES ? num_kb : STAGES;
-            for (int kb = 0; kb < pre; ++kb) {
-                mbar_expect_tx(&full_bar[kb], Cfg::STAGE_BYTES);
-                tma_load_2d(smem + kb * Cfg::STAGE_BYTES + Cfg::A_BYTES, &tmB, &full_bar[kb], kb * BLOCK_K, b_row0, kEvictFirst);
+        // weights (B) are written by no kernel of the chain: fill the ring with them BEFORE waiting for the predecessor
+        const int pre = num_kb < STAGES ? num_kb : STAGES;
+        for (int kb = 0; kb < pre; ++kb)
+            if (elect_one()) {
+                mbar_expect_tx(&full_bar[kb], STAGE_TX);
+                tma_load_2d(smem + B_AT + kb * B_STRIDE, &tmB, &full_bar[kb], kb * BLOCK_K, b_row0, kEvictFirst);
             }
-            griddep_wait();
-            for (int kb = 0; kb < pre; ++kb)
-                tma_load_2d(smem + kb * Cfg::STAGE_BYTES, &tmA, &full_bar[kb], kb * BLOCK_K, m_blk * BLOCK_M, kEvictLast);
-            int s = pre == STAGES ? 0 : pre; uint32_t ph = pre == STAGES ? 1 : 0;
-            for (int kb = pre; kb < num_kb; ++kb) {
-                mbar_wait(&empty_bar[s], ph ^ 1);
-                uint8_t* a_dst = smem + s * Cfg::STAGE_BYTES;
-                uint8_t* b_dst = a_dst + Cfg::A_BYTES;
-                mbar_expect_tx(&full_bar[s], Cfg::STAGE_BYTES);
-                tma_load_2d(a_dst, &tmA, &full_bar[s], kb * BLOCK_K, m_blk * BLOCK_M, kEvictLast);
-                tma_load_2d(b_dst, &tmB, &full_bar[s], kb * BLOCK_K, b_row0, kEvictFirst);
-                if (++s == STAGES) { s = 0; ph ^= 1; }
+        griddep_wait();
+        for (int kb = 0; kb < pre; ++kb)
+            if (elect_one()) tma_load_2d(smem + kb * A_STRIDE, &tmA, &full_bar[kb], kb * BLOCK_K, m_blk * BLOCK_M, kEvictLast);
+        int s = pre == STAGES ? 0 : pre; uint32_t ph = pre == STAGES ? 1 : 0;
+        for (int kb = pre; kb < num_kb; ++kb) {
+            mbar_wait(&empty_bar[s], ph ^ 1);
+            if (elect_one()) {
+                mbar_expect_tx(&full_bar[s], STAGE_TX);
+                tma_load_2d(smem + s * A_STRIDE, &tmA, &full_bar[s], kb * BLOCK_K, m_blk * BLOCK_M, kEvictLast);
+                tma_load_2d(smem + B_AT + s * B_STRIDE, &tmB, &full_bar[s], kb * BLOCK_K, b_row0, kEvictFirst);
             }
+            __syncwarp();
+            if (++s == STAGES) { s = 0; ph ^= 1; }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = umma_idesc_bf16(BLOCK_M, BN);
-            int s = 0; uint32_t ph = 0;
-            for (int kb = 0; kb < num_kb; ++kb) {
-                mbar_wait(&full_bar[s], ph);
-                tcgen05_fence_after();
-                const uint32_t a_addr = smem_u32(smem + s * Cfg::STAGE_BYTES);
-                const uint64_t a_desc = umma_desc_sw128(a_addr);
-                const uint64_t b_desc = umma_desc_sw128(a_addr + Cfg::A_BYTES);
+        constexpr uint32_t idesc = umma_idesc_bf16(BLOCK_M, BN);
+        int s = 0; uint32_t ph = 0;
+        for (int kb = 0; kb < num_kb; ++kb) {
+            mbar_wait(&full_bar[s], ph);
+            tcgen05_fence_after();
+            // FEW: the product reads 128 rows from the start of its A stage, the rows beyond those loaded being whatever lies behind it in the ring
+            // (inside the block's shared memory: at least four B stages follow).  They are rows of the result that nobody looks at.
+            const uint64_t a_desc = umma_desc_sw128(smem_u32(smem + s * A_STRIDE));
+            const uint64_t b_desc = umma_desc_sw128(smem_u32(smem + B_AT + s * B_STRIDE));
+            if (elect_one()) {
 #pragma unroll
-                for (int k = 0; k < BLOCK_K / UMMA_K; ++k) {
-                    // advance 16 bf16 = 32 B inside the 128 B swizzle row: +2 in the (>>4) address field
+                for (int k = 0; k < BLOCK_K / UMMA_K; ++k)      // 16 bf16 = 32 B further inside the 128 B swizzle row: +2 in the (>>4) address field
                     umma_bf16(tmem_base, a_desc + (uint64_t)(k * 2), b_desc + (uint64_t)(k * 2), idesc, (kb | k) != 0);
-                }
-                umma_commit(&empty_bar[s]);   // slot reusable once these MMAs have read it
-                if (++s == STAGES) { s = 0; ph ^= 1; }
+                umma_commit(&empty_bar[s]);       // slot reusable once these MMAs have read it
             }
-            umma_commit(acc_bar);             // accumulator complete
+            __syncwarp();
+            if (++s == STAGES) { s = 0; ph ^= 1; }
         }
+        if (elect_one()) umma_commit(acc_bar);    // accumulator complete
+        __syncwarp();
     } else {
         // ---------------- epilogue: warps 2..5, TMEM lane group = warp % 4 ----------------
         const int q = warp & 3;
@@ -290,14 +308,36 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_tcgen05_kernel(const __grid
 
 int gemm_n_tiles(int N, int block_n) { return (N + block_n - 1) / block_n; }
 
+static int sm_count_cached();
+// few rows (tmA: a box of few_box(M) rows)
+template <int BN, int EPI>
+static cudaError_t launch_few(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, cudaStream_t stream) {
+    auto kern = gemm_tcgen05_kernel<BN, EPI, true>;
+    const FewRing few = few_ring(p.M, p.N, BN, sm_count_cached());
+    const int smem = few.stages * (few.a_rows + BN) * BLOCK_K * 2 + 1024 + FEW_BAR_BYTES;
+    static bool attr_done[16] = {};
+    { cudaError_t e = ensure_dynamic_smem(kern, 227 * 1024, attr_done); if (e != cudaSuccess) return e; }
+    return launch_k(kern, dim3((p.N + BN - 1) / BN), dim3(GEMM_THREADS), smem, stream, *tmA, *tmB, p, few);
+}
+template <int BN>
+static cudaError_t launch_few_bn(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epi, cudaStream_t s) {
+    switch (epi) {
+        case EPI_STORE: return launch_few<BN, EPI_STORE>(tmA, tmB, p, s);
+        case EPI_RESID: return launch_few<BN, EPI_RESID>(tmA, tmB, p, s);
+        case EPI_SWIGLU: return launch_few<BN, EPI_SWIGLU>(tmA, tmB, p, s);
+        case EPI_F32: return launch_few<BN, EPI_F32>(tmA, tmB, p, s);
+    }
+    return cudaErrorInvalidValue;
+}
+
 template <int BN, int EPI>
 static cudaError_t launch_one(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, cudaStream_t stream) {
     using Cfg = GemmCfg<BN>;
-    auto kern = gemm_tcgen05_kernel<BN, EPI>;
+    auto kern = gemm_tcgen05_kernel<BN, EPI, false>;
     static bool attr_done[16] = {};
     { cudaError_t e = ensure_dynamic_smem(kern, Cfg::SMEM_BYTES, attr_done); if (e != cudaSuccess) return e; }
     dim3 grid(((p.N + BN - 1) / BN) * ((p.M + BLOCK_M - 1) / BLOCK_M), 1, 1);
-    return launch_k(kern, grid, dim3(GEMM_THREADS), Cfg::SMEM_BYTES, stream, *tmA, *tmB, p);
+    return launch_k(kern, grid, dim3(GEMM_THREADS), Cfg::SMEM_BYTES, stream, *tmA, *tmB, p, FewRing{});
 }
 
 template <int BN>
@@ -321,29 +361,15 @@ static long long persistent_min_tiles();
 template <int EPI>
 static cudaError_t launch_persistent(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, cudaStream_t stream);
 
-// Cluster size of the few-row kernel for this product, or 0: one of the kernels here takes it.  The largest that keeps the CTAs within 7/4 of the SMs
-// (two are resident on one; measured 16 .. 224 tiles of 128 weight rows).  Every row costs its exchange, S CTAs' worth, so with more rows it takes
-// more of a k range per CTA to pay: up to 16 rows always (28672 x 4096: 41 us against 42; 8192 x 2048: 9 against 17), up to 32 with four CTAs a
-// tile (6208 x 2048: 10.3 against 12.1; with two 12.6), up to 64 with eight, or with four from K = 4096 (6208 x 2048: 12.2 against 12.3; 6144 x 4096:
-// 17 against 21), up to 128 with four of K >= 4096 (4096 x 14336: 36 against 62; 2048 x 2048: 13 against 11).
-static int gemm_rows_split(const GemmParams& p, int epilogue) {
-    if (!p.few_rows_ok || epilogue == EPI_LOGITS || p.m_tile_group || gemm_rows_box(p.M) == 0) return 0;
-    const int tiles = (p.N + 127) / 128, kb = (p.K + BLOCK_K - 1) / BLOCK_K;
-    int s = p.M > 64 ? 4 : 8;
-    while (s > 1 && (tiles * s > sm_count_cached() * 7 / 4 || kb < 2 * s)) s >>= 1;
-    const bool pays = p.M <= 16 || (p.M <= 32 && s >= 4) || (p.M <= 64 && (s == 8 || (s == 4 && kb >= 64))) || (s == 4 && kb >= 64);
-    return pays ? s : 0;
-}
 // CTA-pair kernel or one of the kernels here: the least estimate of rounds x k blocks x time of a k block plus what a launch costs besides.  Constants in
 // us fitted to a sweep of 200 .. 8192 rows over the projections of the four model sizes: a k block takes 0.345 in a pair (0.39 once more than two rounds
 // run against the power cap), 0.42 in a 128 x 256 tile and 0.26 in a narrower one; outside the k loop 11 and 8.  E.g. 200 x 4096 x 4096: 64 tiles of 128
-// x 64 24 us, 16 pair tiles 32.  Up to 128 rows half of a pair's rows would be padding.  These kernels sum k in the same order: the choice moves no bit.
-struct GemmChoice { bool pair; int rows; };
+// x 64 24 us, 16 pair tiles 32.  Up to 128 rows half of a pair's rows would be padding.  Every kernel sums k in the same order: the choice moves no bit.
+struct GemmChoice { bool pair, few; };
 static GemmChoice gemm_choose(const GemmParams& p, int epilogue, int block_n) {
-    GemmChoice best{false, 0};
+    GemmChoice best{false, false};
     if ((block_n != 32 && block_n != 64 && block_n != 128 && block_n != 256) || p.M <= 0 || p.N <= 0 || p.K <= 0) return best;      // refused by launch_gemm
-    best.rows = gemm_rows_split(p, epilogue);
-    if (best.rows) return best;
+    best.few = p.few_rows_ok && p.M <= FEW_MAX_ROWS && epilogue != EPI_LOGITS && !p.m_tile_group;
     const int sms = sm_count_cached(), pairs = sms / 2;
     if (epilogue == EPI_LOGITS || p.m_tile_group || p.M <= BLOCK_M || pairs < 1 || std::getenv("OA_GEMM_PERSISTENT_MIN_TILES")) return best;      // (tests that drive the 128 x 256 kernel set it)
     auto up = [](long long a, long long b) { return (a + b - 1) / b; };
@@ -354,10 +380,9 @@ static GemmChoice gemm_choose(const GemmParams& p, int epilogue, int block_n) {
     return best;
 }
 int gemm_b_box(const GemmParams& p, int epilogue, int block_n) {
-    const GemmChoice c = gemm_choose(p, epilogue, block_n);
-    return c.pair || c.rows ? 128 : block_n;
+    return gemm_choose(p, epilogue, block_n).pair ? 128 : block_n;
 }
-int gemm_a_box(const GemmParams& p, int epilogue, int block_n) { return gemm_choose(p, epilogue, block_n).rows ? gemm_rows_box(p.M) : 128; }
+int gemm_a_box(const GemmParams& p, int epilogue, int block_n) { return gemm_choose(p, epilogue, block_n).few ? few_box(p.M) : 128; }
 
 cudaError_t launch_gemm(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epilogue, int block_n,
                         cudaStream_t stream) {
@@ -366,7 +391,14 @@ cudaError_t launch_gemm(const CUtensorMap* tmA, const CUtensorMap* tmB, const Ge
     // large-M (prefill) shapes with the widest tile go to the persistent kernel (epilogue overlapped with the next tile)
     if (epilogue == EPI_F32 && ((p.ldf % 4) != 0 || !p.f32_out)) return cudaErrorInvalidValue;
     const GemmChoice choice = gemm_choose(p, epilogue, block_n);
-    if (choice.rows) return launch_gemm_rows(tmA, tmB, p, epilogue, choice.rows, stream);
+    if (choice.few) {
+        switch (block_n) {
+            case 32: return launch_few_bn<32>(tmA, tmB, p, epilogue, stream);
+            case 64: return launch_few_bn<64>(tmA, tmB, p, epilogue, stream);
+            case 128: return launch_few_bn<128>(tmA, tmB, p, epilogue, stream);
+            case 256: return launch_few_bn<256>(tmA, tmB, p, epilogue, stream);
+        }
+    }
     if (choice.pair) return launch_gemm_pair(tmA, tmB, p, epilogue, sm_count_cached(), stream);
     if (block_n == 256 && epilogue != EPI_LOGITS && !persistent_disabled() &&
         (long long)((p.N + 255) / 256) * ((p.M + BLOCK_M - 1) / BLOCK_M) >= persistent_min_tiles()) {

@@ -51,12 +51,8 @@ int gemm_n_tiles(int N, int block_n);
 int gemm_logits_bn(int M, int N, int block_n);      // EPI_LOGITS: the tile width to ask launch_gemm for (and to count the arg-max partials by) where block_n would do
 // rows of the B tensor map's box that launch_gemm(.., block_n, ..) reads for this product: block_n, or what the CTA-pair kernel takes where that runs
 int gemm_b_box(const GemmParams& p, int epilogue, int block_n);
-// rows of the A tensor map's box that launch_gemm reads for this product: 128, or what the few-row kernel takes where that runs (only with few_rows_ok)
+// rows of the A tensor map's box that launch_gemm reads for this product: 128, or 16, 32 or 64 for a product of that few rows (only with few_rows_ok)
 int gemm_a_box(const GemmParams& p, int epilogue, int block_n);
-// few-row kernel (gemm_rows.cu), M <= 128: weights in the tensor core's rows, a cluster of S = 1, 2, 4 or 8 CTAs per 128 weight rows; tmA: box {64,
-// gemm_rows_box(M)}, tmB: box {64, 128}
-inline int gemm_rows_box(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 0; }
-cudaError_t launch_gemm_rows(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epilogue, int S, cudaStream_t stream);
 // CTA-pair kernel (gemm_pair.cu): tiles of 256 x 256; tmB: box {64, 128}
 cudaError_t launch_gemm_pair(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epilogue, int sms, cudaStream_t stream);
 // ---- stream-K variant for decode (M <= 128): persistent, one CTA per SM; work unit = (n_tile, 64-wide k block),

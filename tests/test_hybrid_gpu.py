@@ -144,6 +144,27 @@ def test_unequal_requests_in_one_batch_and_reused_pages_and_slots(tmp_path, dtyp
         check(np.concatenate(got[r]), want[r], dtype)
 
 
+def test_bf16_rows_keep_their_bits_whole_in_portions_and_beside_others(tmp_path):
+    """A row's bits follow from its own tokens alone, also on the tensor cores: a prompt whole, in portions on both sides of every kernel's row count,
+    token by token, and beside other requests.  (Latent attention has two forms that round at different places, and routed experts take another kernel
+    for steps of a few rows; neither is here.)  Matrices wide enough that a product's k would be worth sharing."""
+    cfg = O.make_config([O.delta_layer(heads=8, kv_heads=4, dim=64, vdim=64), O.mamba_layer(heads=16, vdim=64, state=32, norm_groups=2)], width=1024, vocab=96)
+    checkpoint(tmp_path, cfg, seed=23)
+    a, b = tokens_of(cfg, 260, 1), tokens_of(cfg, 260, 2)
+    with engine(tmp_path, "bfloat16", pages=16) as eng:
+        whole_a, whole_b = replay(eng, 1, a, [260]), replay(eng, 2, b, [260])
+        for rid, cuts in ((3, [1, 15, 16, 17, 32, 33, 64, 65, 5]), (4, [129, 127]), (5, [200])):
+            got = replay(eng, rid, a, cuts)
+            assert np.array_equal(got, whole_a), (cuts, int((got != whole_a).any(axis=1).sum()))
+        rows_a, rows_b, at_a, at_b = [], [], 0, 0
+        for na, nb in ((1, 16), (16, 1), (1, 1), (33, 31), (60, 68), (2, 126), (140, 1), (7, 16)):
+            na, nb = min(na, 260 - at_a), min(nb, 260 - at_b)
+            out = eng.trace_step([(6, a[at_a:at_a + na], list(range(na))), (7, b[at_b:at_b + nb], list(range(nb)))])
+            rows_a.append(out[:na]); rows_b.append(out[na:]); at_a += na; at_b += nb
+        assert at_a == at_b == 260
+    assert np.array_equal(np.concatenate(rows_a), whole_a) and np.array_equal(np.concatenate(rows_b), whole_b)
+
+
 def test_a_far_key_decides_and_is_found_through_pages_and_decoding(tmp_path):
     """Sharp attention: single keys dominate, also hundreds of tokens back.  The oracle itself shows the sensitivity (without the first page
     the answer changes by far more than the tolerance), and the engine must agree with it in prompts and in decoding."""

@@ -497,3 +497,8 @@ def _bits_follow_the_row(L, N, K, total, spans, widths):
 @pytest.mark.parametrize("N,K", [(4096, 14336), (4096, 4096), (6144, 4096), (2048, 2048), (1024, 328)])
 def test_prefill_rows_keep_their_bits_beside_others(L, N, K):
     _bits_follow_the_row(L, N, K, 1337, [(0, 1337), (0, 129), (0, 200), (100, 357), (0, 400), (700, 1314), (313, 1337)], (256, 128, 64))
+
+
+@pytest.mark.parametrize("N,K", [(4096, 14336), (2048, 4096), (6144, 2056), (2048, 2048), (1024, 72), (28672, 1024)])
+def test_decoding_rows_keep_their_bits_beside_others(L, N, K):
+    _bits_follow_the_row(L, N, K, 300, [(0, 300), (0, 1), (17, 18), (0, 16), (3, 20), (0, 32), (7, 40), (0, 64), (30, 95), (0, 128), (50, 179), (299, 300)], (32, 64, 128, 256))
