@@ -285,9 +285,11 @@ __global__ void __launch_bounds__(64 + 128 * NWG, 1) prefill_attention_tc_kernel
 // items and one warpgroup's output is written under the other's last products.
 //   warp 0    : TMA (K, Q, V)        warp 1 : tcgen05.mma        warps 4-7 / 8-11 : softmax and output of head A / B, one query row per thread
 // A group with an odd number of heads leaves its last one alone in an item (warpgroup B idles).
-// Measured against the kernel above: 4096 rows behind 12288 cached ones, 64 / 8 heads of 128: 1967 -> 1544 us (1.25 PFLOP/s; the tensor and the
+// A row's scores, reference maxima, probabilities and sums are those of the kernel above, in its order: which of the two a batch takes moves no bit.
+// (Four sums per row instead of two are 3 % faster, and moved the last one.)
+// Measured against the kernel above: 4096 rows behind 12288 cached ones, 64 / 8 heads of 128: 1963 -> 1560 us in a burst (the tensor and the
 // special-function pipe are each busy 60 % of the time and the clock is down to 1.63 GHz under the 1000 W cap); five prompts of 1.4 thousand rows,
-// 32 / 8 heads: 184 -> 118 us.  Handing P over in two or three parts, taking exponentials from a reference that may still rise, moving an eighth
+// 32 / 8 heads: 184 -> 121 us.  Handing P over in two or three parts, taking exponentials from a reference that may still rise, moving an eighth
 // or a quarter of them to the FMA pipe and two threads per row were each 3 to 12 % slower.
 // ---------------------------------------------------------------------------------------------
 template <int D>
@@ -454,7 +456,7 @@ __global__ void __launch_bounds__(PtpCfg<D>::THREADS, 1) prefill_attention_pair_
         for (int r = 0; ptp_item(p, ppg, r, it); ++r) {
             if (x > it.two) continue;
             const int qpos = it.tile.pos0 + row;
-            float m_ref = -INFINITY, l_run = 0.f;
+            float m_ref = -INFINITY, l_lo = 0.f, l_hi = 0.f;        // row sums of the tiles' lower and upper 64 keys: the order of the kernel above
             for (int j = 0; j < it.n_kvt; ++j, ++sc) {
                 mbar_wait(&s_full[x], sc & 1);
                 tcgen05_fence_after();
@@ -492,36 +494,41 @@ __global__ void __launch_bounds__(PtpCfg<D>::THREADS, 1) prefill_attention_pair_
                             for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
                             tmem_st_32x32b_x16(o_addr + (uint32_t)c, o);
                         }
-                        l_run *= alpha;
+                        l_lo *= alpha; l_hi *= alpha;
                     }
                     if (raise) m_ref = mx;
                 }
                 const uint64_t nref2 = pack_f32x2(-m_ref, -m_ref);
-                uint64_t sum2[2] = {0ull, 0ull};
+                uint64_t sum2 = 0ull;                               // the two halves' sums, each in ascending keys
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {                       // 32 scores of the row -> 16 columns of P: p = 2^(s * scale - m_ref)
-                    uint32_t pw[16];
+                for (int c = 0; c < 2; ++c) {                       // 32 scores of either half -> 16 columns of P each: p = 2^(s * scale - m_ref)
+                    uint32_t pw[2][16];
 #pragma unroll
                     for (int i = 0; i < 16; ++i) {
-                        float a, b;
-                        unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(v[c][2 * i]), __uint_as_float(v[c][2 * i + 1])), scale2, nref2), a, b);
-                        a = ex2_approx(a); b = ex2_approx(b);
-                        sum2[i & 1] = add_f32x2(sum2[i & 1], pack_f32x2(a, b));
-                        pw[i] = pack_bf16x2(a, b);
+                        float p0[2], p1[2];
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(v[c + 2 * h][2 * i]), __uint_as_float(v[c + 2 * h][2 * i + 1])), scale2, nref2), p0[h], p1[h]);
+                            p0[h] = ex2_approx(p0[h]); p1[h] = ex2_approx(p1[h]);
+                            pw[h][i] = pack_bf16x2(p0[h], p1[h]);
+                        }
+                        sum2 = add_f32x2(sum2, pack_f32x2(p0[0], p0[1]));
+                        sum2 = add_f32x2(sum2, pack_f32x2(p1[0], p1[1]));
                     }
-                    tmem_st_32x32b_x16(s_addr + (uint32_t)(c * 16), pw);
+                    tmem_st_32x32b_x16(s_addr + (uint32_t)(c * 16), pw[0]);
+                    tmem_st_32x32b_x16(s_addr + (uint32_t)((c + 2) * 16), pw[1]);
                 }
                 tmem_st_wait();
                 tcgen05_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&p_full[x]);
                 float a, b;
-                unpack_f32x2(add_f32x2(sum2[0], sum2[1]), a, b);
-                l_run += a + b;
+                unpack_f32x2(sum2, a, b);
+                l_lo += a; l_hi += b;
             }
             mbar_wait(&o_full[x], oc & 1); ++oc;
             tcgen05_fence_after();
-            const float inv = 1.0f / l_run;
+            const float inv = 1.0f / (l_lo + l_hi);
             uint16_t* orow = reinterpret_cast<uint16_t*>(p.out) + (size_t)(it.tile.q_row0 + row) * p.n_heads * D + (size_t)(it.head + x) * D;
 #pragma unroll 1
             for (int c = 0; c < D; c += 32) {

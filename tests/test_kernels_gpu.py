@@ -502,3 +502,42 @@ def test_prefill_rows_keep_their_bits_beside_others(L, N, K):
 @pytest.mark.parametrize("N,K", [(4096, 14336), (2048, 4096), (6144, 2056), (2048, 2048), (1024, 72), (28672, 1024)])
 def test_decoding_rows_keep_their_bits_beside_others(L, N, K):
     _bits_follow_the_row(L, N, K, 300, [(0, 300), (0, 1), (17, 18), (0, 16), (3, 20), (0, 32), (7, 40), (0, 64), (30, 95), (0, 128), (50, 179), (299, 300)], (32, 64, 128, 256))
+
+
+# A prompt's attention has the same bits alone (few items: one head per CTA) and beside others (the two-heads-per-CTA kernel): both take the same keys per
+# tile, raise a row's reference maximum at the same scores and sum its exponentials in the same order.
+@pytest.mark.parametrize("nh,nkv,D", [(32, 8, 128), (20, 4, 128), (32, 8, 64), (15, 3, 64), (16, 2, 128)])
+def test_prefill_attention_keeps_its_bits_beside_others(L, nh, nkv, D):
+    pairs = nkv * ((nh // nkv + 1) // 2)
+    half = torch.cuda.get_device_properties(0).multi_processor_count // 2
+    few = half // pairs                                  # row tiles of a lone prompt that stay on the one-head kernel
+    cases = [(c, min(q, 128 * few)) for c, q in [(64, 64), (130, 130), (700, 200), (513, 513), (1, 1), (999, 385), (2000, 129)]] * 2
+    ctx = [c for c, _ in cases]; qlens = [q for _, q in cases]
+    assert sum((q + 127) // 128 for q in qlens) * pairs > half and all((q + 127) // 128 * pairs <= half for q in qlens)
+    n = len(ctx); maxp = 32; num_pages = sum((c + 63) // 64 for c in ctx)
+    kv = _mk_cache(num_pages, nkv, D, 21)
+    g = torch.Generator(device="cpu").manual_seed(4)
+    perm = torch.randperm(num_pages, generator=g)
+    bt = torch.zeros(n, maxp, dtype=torch.int32); k = 0
+    for i, c in enumerate(ctx):
+        npg = (c + 63) // 64; bt[i, :npg] = perm[k:k + npg].to(torch.int32); k += npg
+    T = sum(qlens)
+    q = torch.randn(T, nh, D, generator=g)
+    q[::5] *= 9                                          # scores that raise a row's reference maximum in later tiles
+    q = q.to(torch.bfloat16).to(dev())
+
+    def attend(seqs, rows):
+        out = torch.full((len(rows), nh, D), float("nan"), dtype=torch.bfloat16, device=dev())
+        qq = q[rows].contiguous()
+        ca = np.array([ctx[i] for i in seqs], np.int32); qa = np.array([qlens[i] for i in seqs], np.int32); b = np.ascontiguousarray(bt[seqs].numpy())
+        assert L.oa_k_paged_attention(ptr(qq), ptr(out), ptr(kv), num_pages, b.ctypes.data, maxp, ca.ctypes.data, qa.ctypes.data, len(seqs), nh, nkv, D, 0, None) == 0
+        return out
+
+    whole = attend(list(range(n)), list(range(T)))
+    row0 = 0
+    for i in range(n):
+        if qlens[i] > 1:                                 # (a lone row is a decoding row: another kernel)
+            rows = list(range(row0, row0 + qlens[i]))
+            alone = attend([i], rows)
+            assert torch.equal(alone, whole[row0:row0 + qlens[i]]), (i, int((alone != whole[row0:row0 + qlens[i]]).sum()))
+        row0 += qlens[i]
