@@ -144,6 +144,9 @@ OA_API int oa_k_gemm(const void* A, const void* B, int32_t M, int32_t N, int32_t
               const void* bias, const void* resid, float* logits, int32_t* argmax_out, void* stream);
 /* persistent stream-K GEMM (M <= 128) followed by the fixed-order partial sum: out_f32[M,N] */
 OA_API int oa_k_gemm_streamk(const void* A, const void* B, int32_t M, int32_t N, int32_t K, int32_t block_n, int32_t n_ctas, float* out_f32, void* stream);
+/* the hybrid models' plain products (bf16 operands, fp32 FMA): C[b] = alpha A[b] . B[b]^T; mode 0: bf16 result, 1: fp32, 2: added to fp32 */
+OA_API int oa_k_hybrid_gemm(int32_t mode, const void* A, int32_t lda, const void* B, int32_t ldb, void* C, int32_t ldc, int32_t M, int32_t N, int32_t K, float alpha,
+                            int32_t batch, int64_t stride_a, int64_t stride_b, int64_t stride_c, void* stream);
 OA_API int oa_k_init_weight(void* dst, uint64_t seed, uint64_t tensor_id, int64_t tensor_id_b, int64_t rows, int64_t cols, float std,
                      float mean, void* stream);
 /* paged attention on a caller-provided cache [2(K,V)][num_pages][n_kv][64][D] (one layer): decode when q has one

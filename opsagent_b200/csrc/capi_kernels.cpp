@@ -16,6 +16,7 @@
 #include "token_mask.hpp"
 #include "tokenizer.hpp"
 #include "model.hpp"
+#include "hybrid_kernels.hpp"
 #include "sk_consumers.cuh"
 #include "tokenizer.hpp"
 
@@ -133,6 +134,12 @@ int oa_k_gemm(const void* A, const void* B, int32_t M, int32_t N, int32_t K, int
         return rc_of(e);
     }
     return rc_of(launch_gemm(&tmA, &tmB, p, epilogue, block_n, s));
+}
+
+int oa_k_hybrid_gemm(int32_t mode, const void* A, int32_t lda, const void* B, int32_t ldb, void* C, int32_t ldc, int32_t M, int32_t N, int32_t K, float alpha,
+                     int32_t batch, int64_t stride_a, int64_t stride_b, int64_t stride_c, void* stream) {
+    if (mode != HY_STORE && mode != HY_STORE_F32 && mode != HY_ACC_F32) return OA_ERR_BAD_REQUEST;
+    return rc_of(hy_gemm(false, mode, A, lda, B, ldb, C, ldc, M, N, K, nullptr, alpha, batch, stride_a, stride_b, stride_c, (cudaStream_t)stream));
 }
 
 static int paged_attention(const void* q, void* out, const void* kv_cache, int32_t num_pages, const int32_t* block_tables,

@@ -71,54 +71,76 @@ __global__ void __launch_bounds__(256) hy_gemm_kernel(const TA* __restrict__ A, 
     }
 }
 
-// The same product for a handful of rows (decoding steps), bf16 operands with K in aligned groups of 8: a warp owns 8 columns and 16 rows as
-// mma.sync m16n8k16 products straight from global memory.  The order of k inside a product is free as long as A and B agree, so lane t of a
-// quad takes eight consecutive values of its rows in one 16-byte load — two products' worth — and nothing goes through shared memory.  Four
-// blocks of 32 k are in flight; sums run in ascending blocks, so a row's result does not depend on the other rows.  What bounds it is that load
-// latency: 16 rows x 16 heads x 512 x 128 27 us -> about 5 as one warp per column that walked the rows, each with a butterfly of its own.
-// SPLIT (K of 256 and more): the four warps of a block share eight columns, each every fourth block of 32 k, and join in warp order; otherwise each
-// warp has eight columns of its own.
-template <int MODE, bool SPLIT>
+// The same product for a handful of rows (decoding steps), bf16 operands with K <= 1024 in aligned groups of 8, on fp32 FMA: G lanes (a half warp up to
+// K = 128, else a warp) share two columns and eight rows.  A lane sums its pieces of eight k in ascending order and the lanes join by a butterfly, so a
+// row's result does not depend on the other rows.  The butterfly runs over the eight rows at once: a lane hands half of its rows on at each distance and
+// keeps the other half (9 shuffles for eight rows and a warp where one row at a time takes 40), the same sums in the same order.  What bounds it is the
+// latency of the loads, ten 16-byte ones in flight a lane.
+// us, 16 heads at 16 rows: 512 x 128 with fp32 results 4.5, 128 x 512 5.1 (a warp per column that walks the rows: 27).  mma.sync takes 2.6 and 2.9, but
+// its sums are 1.2e-7 off the 64-bit result where these are 4.8e-8, and hy_tensor_core = 0 promises plain FMA.
+template <int MODE, int G>
 __global__ void __launch_bounds__(128) hy_gemm_fewrows_kernel(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bfloat16* __restrict__ B, int ldb, void* Cv, int ldc, int M, int N,
                                                               int K, const float* __restrict__ bias, float alpha, long long sA, long long sB, long long sC, HyGemmAct act) {
     HY_PDL();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int n0 = (SPLIT ? blockIdx.x : blockIdx.x * 4 + warp) * 8, m0 = blockIdx.z * 16;
-    if (n0 >= N) return;
-    const __nv_bfloat16* a_lo = A + (long long)blockIdx.y * sA + (long long)(m0 + g) * lda;
-    const __nv_bfloat16* a_hi = a_lo + (long long)8 * lda;
-    const __nv_bfloat16* b_n = B + (long long)blockIdx.y * sB + (long long)(n0 + g) * ldb;
-    const bool lo = m0 + g < M, hi = m0 + g + 8 < M, col = n0 + g < N;
-    constexpr int STEP = SPLIT ? 128 : 32;                   // from one of a warp's blocks of 32 k to its next
-    float d[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int kb = SPLIT ? warp * 32 : 0; kb < K; kb += 4 * STEP) {
-        uint4 x[4], y[4], w[4];
+    constexpr int ROWS = 8, COLS = 2;
+    const int l = threadIdx.x & (G - 1), n0 = (blockIdx.x * (128 / G) + threadIdx.x / G) * COLS, m0 = blockIdx.z * ROWS;
+    A += (long long)blockIdx.y * sA + (long long)m0 * lda; B += (long long)blockIdx.y * sB;
+    float acc[COLS][ROWS];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int k = kb + i * STEP + t * 8;
-            x[i] = lo && k < K ? *reinterpret_cast<const uint4*>(a_lo + k) : make_uint4(0, 0, 0, 0);
-            y[i] = hi && k < K ? *reinterpret_cast<const uint4*>(a_hi + k) : make_uint4(0, 0, 0, 0);
-            w[i] = col && k < K ? *reinterpret_cast<const uint4*>(b_n + k) : make_uint4(0, 0, 0, 0);
+    for (int c = 0; c < COLS; ++c)
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) acc[c][r] = 0.f;
+    for (int k = l * 8; k < K; k += G * 8) {
+        uint4 a[ROWS], b[COLS];
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) b[c] = n0 + c < N ? *reinterpret_cast<const uint4*>(B + (long long)(n0 + c) * ldb + k) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) a[r] = m0 + r < M ? *reinterpret_cast<const uint4*>(A + (long long)r * lda + k) : make_uint4(0, 0, 0, 0);
+        float bf[COLS][8];
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) {
+            bf[c][0] = bf16lo(b[c].x); bf[c][1] = bf16hi(b[c].x); bf[c][2] = bf16lo(b[c].y); bf[c][3] = bf16hi(b[c].y);
+            bf[c][4] = bf16lo(b[c].z); bf[c][5] = bf16hi(b[c].z); bf[c][6] = bf16lo(b[c].w); bf[c][7] = bf16hi(b[c].w);
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            mma_bf16_16816(d, x[i].x, y[i].x, x[i].y, y[i].y, w[i].x, w[i].y);
-            mma_bf16_16816(d, x[i].z, y[i].z, x[i].w, y[i].w, w[i].z, w[i].w);
+        for (int r = 0; r < ROWS; ++r) {
+            const float af[8] = {bf16lo(a[r].x), bf16hi(a[r].x), bf16lo(a[r].y), bf16hi(a[r].y), bf16lo(a[r].z), bf16hi(a[r].z), bf16lo(a[r].w), bf16hi(a[r].w)};
+#pragma unroll
+            for (int c = 0; c < COLS; ++c)
+#pragma unroll
+                for (int e = 0; e < 8; ++e) acc[c][r] = fmaf(af[e], bf[c][e], acc[c][r]);
         }
     }
-    if constexpr (SPLIT) {
-        __shared__ float4 part[3][32];
-        if (warp > 0) part[warp - 1][lane] = make_float4(d[0], d[1], d[2], d[3]);
-        __syncthreads();
-        if (warp > 0) return;
+    // butterfly from the widest distance down; up to three of its steps also halve a lane's rows, the last ones join what is left
+    constexpr int FIRST = G / 2;
+    int row = 0;                                             // the row this lane ends up with
 #pragma unroll
-        for (int w = 0; w < 3; ++w) { const float4 u = part[w][lane]; d[0] += u.x; d[1] += u.y; d[2] += u.z; d[3] += u.w; }
+    for (int c = 0; c < COLS; ++c) {
+        if (G == 16) {                                       // the half warp that would hold k >= 128 adds its zero
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r) acc[c][r] += 0.f;
+        }
+#pragma unroll
+        for (int h = ROWS / 2, o = FIRST; h > 0; h >>= 1, o >>= 1) {
+            const bool up = (l & o) != 0;
+#pragma unroll
+            for (int r = 0; r < ROWS / 2; ++r) {
+                if (r >= h) break;
+                const float mine = up ? acc[c][r + h] : acc[c][r], give = up ? acc[c][r] : acc[c][r + h];
+                acc[c][r] = mine + __shfl_xor_sync(0xffffffffu, give, o);
+            }
+            if (c == 0) row += up ? h : 0;
+        }
+#pragma unroll
+        for (int o = FIRST / ROWS; o > 0; o >>= 1) acc[c][0] += __shfl_xor_sync(0xffffffffu, acc[c][0], o);
     }
+    // distances FIRST, FIRST / 2, FIRST / 4 chose the row; of the lanes left with it, the first COLS write a column each
+    const int rest = l & (2 * FIRST / ROWS - 1), m = m0 + row;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        const int m = m0 + g + (c >= 2 ? 8 : 0), n = n0 + 2 * t + (c & 1);
-        if (m >= M || n >= N) continue;
-        float v = d[c] * alpha + (bias ? bias[n] : 0.f);
+    for (int c = 0; c < COLS; ++c) {
+        const int n = n0 + c;
+        if (rest != c || m >= M || n >= N) continue;
+        float v = acc[c][0] * alpha + (bias ? bias[n] : 0.f);
         v = gemm_act(act, v, n);
         const long long at = (long long)blockIdx.y * sC + (long long)m * ldc + n;
         if (MODE == HY_STORE) reinterpret_cast<__nv_bfloat16*>(Cv)[at] = __float2bfloat16_rn(v);
@@ -1477,10 +1499,10 @@ cudaError_t hy_gemm(bool f32, int mode, const void* A, int lda, const void* B, i
     if (M <= 0 || N <= 0 || K <= 0 || batch <= 0) return cudaSuccess;
     auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
     if (!f32 && M <= HY_GEMM_FEW_ROWS && K % 8 == 0 && K <= 1024 && lda % 8 == 0 && ldb % 8 == 0 && sA % 8 == 0 && sB % 8 == 0 && al16(A) && al16(B)) {
-        const bool split = K >= 256;
-        const dim3 grid(split ? (N + 7) / 8 : (N + 31) / 32, batch, (M + 15) / 16);
-#define HY_FEW(MODE) (split ? launch_plain(hy_gemm_fewrows_kernel<MODE, true>, grid, dim3(128), 0, s, (const bf*)A, lda, (const bf*)B, ldb, C, ldc, M, N, K, bias, alpha, sA, sB, sC, act) \
-                            : launch_plain(hy_gemm_fewrows_kernel<MODE, false>, grid, dim3(128), 0, s, (const bf*)A, lda, (const bf*)B, ldb, C, ldc, M, N, K, bias, alpha, sA, sB, sC, act))
+        const bool half = K <= 128;
+        const dim3 grid(half ? (N + 15) / 16 : (N + 7) / 8, batch, (M + 7) / 8);
+#define HY_FEW(MODE) (half ? launch_plain(hy_gemm_fewrows_kernel<MODE, 16>, grid, dim3(128), 0, s, (const bf*)A, lda, (const bf*)B, ldb, C, ldc, M, N, K, bias, alpha, sA, sB, sC, act) \
+                           : launch_plain(hy_gemm_fewrows_kernel<MODE, 32>, grid, dim3(128), 0, s, (const bf*)A, lda, (const bf*)B, ldb, C, ldc, M, N, K, bias, alpha, sA, sB, sC, act))
         return mode == HY_STORE ? HY_FEW(HY_STORE) : mode == HY_STORE_F32 ? HY_FEW(HY_STORE_F32) : HY_FEW(HY_ACC_F32);
 #undef HY_FEW
     }

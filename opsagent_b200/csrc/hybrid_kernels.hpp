@@ -38,7 +38,7 @@ enum HyGemmMode : int { HY_STORE = 0, HY_STORE_F32 = 1, HY_ACC_F32 = 2 };
 // accumulation for any sizes: the fp32 mode's matrix product, and the bf16 mode's fallback where a shape does not fit the tensor-core tiles.
 // act.kind = 1: the stored value is relu(.)^2, 2: the tanh form of GELU, 3: SiLU on columns col0 .. col1 - 1 (HY_STORE / HY_STORE_F32)
 struct HyGemmAct { int kind = 0, col0 = 0, col1 = 0; };
-// bf16 steps of at most HY_GEMM_FEW_ROWS rows with K <= 1024 in aligned groups of 8 take mma.sync products straight from global memory instead of the tile kernel
+// bf16 steps of at most HY_GEMM_FEW_ROWS rows with K <= 1024 in aligned groups of 8 take a kernel of a few rows on fp32 FMA instead of the tile kernel
 constexpr int HY_GEMM_FEW_ROWS = 32;
 cudaError_t hy_gemm(bool f32, int mode, const void* A, int lda, const void* B, int ldb, void* C, int ldc, int M, int N, int K, const float* bias,
                     float alpha, int batch, long long sA, long long sB, long long sC, cudaStream_t s, HyGemmAct act = HyGemmAct());

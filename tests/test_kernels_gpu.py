@@ -541,3 +541,29 @@ def test_prefill_attention_keeps_its_bits_beside_others(L, nh, nkv, D):
             alone = attend([i], rows)
             assert torch.equal(alone, whole[row0:row0 + qlens[i]]), (i, int((alone != whole[row0:row0 + qlens[i]]).sum()))
         row0 += qlens[i]
+
+
+# Plain FMA kernel of a few rows (hybrid models: absorbed products of decoding rows; every product of a few rows with hy_tensor_core = 0): the fp32 chain it
+# promises, bit for bit.  A lane sums its pieces of eight k in ascending order with one rounding per product, then a butterfly from distance 16 down.
+@pytest.mark.parametrize("M,N,K,batch", [(1, 24, 8, 1), (5, 41, 128, 3), (16, 512, 128, 4), (17, 33, 136, 2), (32, 64, 512, 2), (9, 17, 1000, 1), (8, 130, 1024, 2), (3, 7, 120, 5)])
+def test_few_row_products_are_an_fp32_chain(L, M, N, K, batch):
+    g = torch.Generator(device="cpu").manual_seed(M * N + K)
+    A = torch.randn(batch, M, K, generator=g).to(torch.bfloat16); B = torch.randn(batch, N, K, generator=g).to(torch.bfloat16)
+    a, b = A.double().numpy(), B.double().numpy()
+    lanes = np.zeros((batch, M, N, 32), np.float32)
+    for piece in range(0, K, 256):
+        for e in range(8):
+            k = piece + np.arange(32) * 8 + e
+            ok = k < K
+            prod = a[:, :, None, k[ok]] * b[:, None, :, k[ok]]                                      # exact in 64 bits
+            lanes[..., ok] = (lanes[..., ok].astype(np.float64) + prod).astype(np.float32)          # one rounding, as a fused multiply-add
+    for o in (16, 8, 4, 2, 1):
+        lanes = lanes + lanes[..., np.arange(32) ^ o]
+    want = lanes[..., 0]
+    Ad, Bd = A.to(dev()), B.to(dev())
+    out = torch.full((batch, M, N), float("nan"), dtype=torch.float32, device=dev()); out16 = out.to(torch.bfloat16)
+    for mode, o in ((1, out), (0, out16)):
+        assert L.oa_k_hybrid_gemm(mode, ptr(Ad), K, ptr(Bd), K, ptr(o), N, M, N, K, 1.0, batch, M * K, N * K, M * N, None) == 0
+    torch.cuda.synchronize()
+    assert (out.cpu().numpy() == want).all(), int((out.cpu().numpy() != want).sum())
+    assert torch.equal(out16, out.to(torch.bfloat16))
