@@ -12,7 +12,6 @@
 //               2^8 (lazy rescaling), so the common tile costs one TMEM read, 128 exp2 and 16 shared-memory stores per thread and
 //               overlaps the tensor-core work of its neighbours (S and P are double-buffered).
 // Row sums use the unrounded p, P·V the bf16-rounded p — the rounding points the oracle mirrors.  TMEM: 2x128 (S) + D (O).
-#include <cstdlib>
 
 #include "common.cuh"
 #include "kernels.hpp"
@@ -36,11 +35,12 @@ struct PtcCfg {
     static constexpr uint32_t T_COL = 256;                       // S[0] at 0, S[1] at 128, T at 256
 };
 
-// NWG = softmax warpgroups.  With one, each SM sub-partition holds a single softmax warp and the 128 exp2 + pack + store chain of a tile
-// (~1.1 us) is longer than its two MMAs (~0.75 us): the tensor pipe idles 70 % of the time (profiles/r01f).  With two, the warps w and w+4
+// NWG = 2 softmax warpgroups: with one, each SM sub-partition holds a single softmax warp and the 128 exp2 + pack + store chain of a tile
+// (~1.1 us) is longer than its two MMAs (~0.75 us), and the tensor pipe idles 70 % of the time.  The warps w and w+4
 // share the same 32 query rows (same TMEM lanes) and split every S tile by KEY columns — 64 scores, 64 exp2, 8 P stores per thread, two
 // warps per sub-partition to hide latencies; the halves' row maxima meet through shared memory once per tile, the row sums once at the end.
-template <int D, int NWG>
+static constexpr int NWG = 2;
+template <int D>
 __global__ void __launch_bounds__(64 + 128 * NWG, 1) prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap tm_q,
                                                                               const __grid_constant__ CUtensorMap tm_kv,
                                                                               const PrefillAttnParams p, const int64_t layer_row0,
@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(64 + 128 * NWG, 1) prefill_attention_tc_kernel
             for (int c = 0; c < CH; ++c)
 #pragma unroll
                 for (int i = 0; i < 32; ++i) mraw = fmaxf(mraw, __uint_as_float(v[c][i]));
-            if constexpr (NWG == 2) {                                           // the row's other half lives in the partner warpgroup
+            {                                                                   // the row's other half lives in the partner warpgroup
                 xch[(sb * 2 + wg) * 128 + row] = mraw;
                 asm volatile("bar.sync 2, 256;" ::: "memory");
                 mraw = fmaxf(mraw, xch[(sb * 2 + (wg ^ 1)) * 128 + row]);
@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(64 + 128 * NWG, 1) prefill_attention_tc_kernel
         }
         mbar_wait(t_full, (uint32_t)(n_kvt - 1) & 1);
         tcgen05_fence_after();
-        if constexpr (NWG == 2) {                                   // row sum = the two key halves' sums (fixed order: half 0 + half 1)
+        {                                                           // row sum = the two key halves' sums (fixed order: half 0 + half 1)
             const int xb = n_kvt & 1;                               // the buffer the last tile did not use
             xch[(xb * 2 + wg) * 128 + row] = l_run;
             asm volatile("bar.sync 2, 256;" ::: "memory");
@@ -287,9 +287,9 @@ __global__ void __launch_bounds__(64 + 128 * NWG, 1) prefill_attention_tc_kernel
 // A group with an odd number of heads leaves its last one alone in an item (warpgroup B idles).
 // A row's scores, reference maxima, probabilities and sums are those of the kernel above, in its order: which of the two a batch takes moves no bit.
 // (Four sums per row instead of two are 3 % faster, and moved the last one.)
-// Measured against the kernel above: 4096 rows behind 12288 cached ones, 64 / 8 heads of 128: 1963 -> 1560 us in a burst (the tensor and the
+// Measured against the kernel above: 4096 rows behind 12288 cached ones, 64 / 8 heads of 128: 1963 -> 1590 us in a burst (the tensor and the
 // special-function pipe are each busy 60 % of the time and the clock is down to 1.63 GHz under the 1000 W cap); five prompts of 1.4 thousand rows,
-// 32 / 8 heads: 184 -> 121 us.  Handing P over in two or three parts, taking exponentials from a reference that may still rise, moving an eighth
+// 32 / 8 heads: 184 -> 122 us.  Handing P over in two or three parts, taking exponentials from a reference that may still rise, moving an eighth
 // or a quarter of them to the FMA pipe and two threads per row were each 3 to 12 % slower.
 // ---------------------------------------------------------------------------------------------
 template <int D>
@@ -564,9 +564,9 @@ static cudaError_t launch_ptp(const CUtensorMap* tm_q, const CUtensorMap* tm_kv,
                     (int64_t)p.layer * kv.layer_stride_rows, kv.kv_stride_rows);
 }
 
-template <int D, int NWG>
+template <int D>
 static cudaError_t launch_ptc(const CUtensorMap* tm_q, const CUtensorMap* tm_kv, const KvLayout& kv, const PrefillAttnParams& p, cudaStream_t s) {
-    auto kern = prefill_attention_tc_kernel<D, NWG>;
+    auto kern = prefill_attention_tc_kernel<D>;
     static bool attr_done[16] = {};
     { cudaError_t e = ensure_dynamic_smem(kern, PtcCfg<D>::SMEM_BYTES, attr_done); if (e != cudaSuccess) return e; }
     return launch_k(kern, dim3(p.n_tiles, p.n_heads), dim3(64 + 128 * NWG), PtcCfg<D>::SMEM_BYTES, s, *tm_q, *tm_kv, p,
@@ -581,7 +581,6 @@ static int prefill_sm_count() {
 cudaError_t launch_prefill_attention_tc(const CUtensorMap* tm_q, const CUtensorMap* tm_kv, const KvLayout& kv, const PrefillAttnParams& p, cudaStream_t s) {
     if (p.n_tiles <= 0) return cudaSuccess;
     if (kv.page_size != 64 || p.n_heads % p.n_kv != 0) return cudaErrorInvalidValue;
-    static const int nwg = [] { const char* e = std::getenv("OA_PREFILL_WG"); return (e && e[0] == '1') ? 1 : 2; }();      // OA_PREFILL_WG=1: the one-warpgroup kernel of round 1 (A/B)
     const int grp = p.n_heads / p.n_kv, items = p.n_tiles * p.n_kv * ((grp + 1) / 2);
     const int sms = prefill_sm_count();
     // Up to half as many items as SMs, twice as many single-head CTAs are all resident at once and each is done sooner (32 / 8 heads, 400 rows
@@ -591,8 +590,8 @@ cudaError_t launch_prefill_attention_tc(const CUtensorMap* tm_q, const CUtensorM
         if (kv.head_dim == 128) return launch_ptp<128>(tm_q, tm_kv, kv, p, items, sms, s);
         if (kv.head_dim == 64) return launch_ptp<64>(tm_q, tm_kv, kv, p, items, sms, s);
     }
-    if (kv.head_dim == 128) return nwg == 2 ? launch_ptc<128, 2>(tm_q, tm_kv, kv, p, s) : launch_ptc<128, 1>(tm_q, tm_kv, kv, p, s);
-    if (kv.head_dim == 64) return nwg == 2 ? launch_ptc<64, 2>(tm_q, tm_kv, kv, p, s) : launch_ptc<64, 1>(tm_q, tm_kv, kv, p, s);
+    if (kv.head_dim == 128) return launch_ptc<128>(tm_q, tm_kv, kv, p, s);
+    if (kv.head_dim == 64) return launch_ptc<64>(tm_q, tm_kv, kv, p, s);
     return cudaErrorInvalidValue;
 }
 
