@@ -142,6 +142,11 @@ OA_API int oa_debug_kernel_times(oa_engine*, char* buf, size_t n, int32_t reset)
 OA_API int oa_k_rmsnorm(const void* x, const void* gain, void* y, int32_t T, int32_t H, float eps, void* stream);
 OA_API int oa_k_gemm(const void* A, const void* B, int32_t M, int32_t N, int32_t K, int32_t epilogue, int32_t block_n, void* out,
               const void* bias, const void* resid, float* logits, int32_t* argmax_out, void* stream);
+/* the same products with what the hybrid models ask of their epilogues.  epilogue 0: bf16, out = act(A . B^T + bias), act 1 relu^2, 2 tanh GELU, 3 SiLU on
+ * columns act_col0 .. act_col1 - 1; 2: bf16 [M, N / 2], act(gate) * up, act 0 SiLU, 2 tanh GELU; 4: fp32, out = alpha A . B^T + bias (fp32), added to out
+ * where accumulate != 0 (alpha 0 counts as 1) */
+OA_API int oa_k_gemm_ext(const void* A, const void* B, int32_t M, int32_t N, int32_t K, int32_t epilogue, int32_t block_n, void* out, const void* bias, int32_t act,
+                         int32_t act_col0, int32_t act_col1, float alpha, int32_t accumulate, void* stream);
 /* persistent stream-K GEMM (M <= 128) followed by the fixed-order partial sum: out_f32[M,N] */
 OA_API int oa_k_gemm_streamk(const void* A, const void* B, int32_t M, int32_t N, int32_t K, int32_t block_n, int32_t n_ctas, float* out_f32, void* stream);
 /* the hybrid models' plain products (bf16 operands, fp32 FMA): C[b] = alpha A[b] . B[b]^T; mode 0: bf16 result, 1: fp32, 2: added to fp32 */
@@ -170,6 +175,10 @@ OA_API int oa_host_decode_plan(const int32_t* ctx_lens, int32_t n_seqs, int32_t 
 OA_API int oa_host_streamk_plan(int32_t N, int32_t K, int32_t block_n, int32_t n_ctas, int64_t* cta_unit0_out, int32_t cap_ctas,
                          int32_t* tile_first_out, int32_t* tile_last_out, int32_t cap_tiles, int32_t* n_ctas_out, int32_t* n_tiles_out,
                          int32_t* kb_out);
+/* which kernel a product runs: -1 refused, 0 a tile per CTA, 1 the same of up to 64 loaded rows, 2 persistent 128 x 256 tiles, 3 CTA pairs, 4 the persistent
+ * vocabulary head.  few_rows: the caller's A map may have the narrower box (the entry points above and the hybrid models); grouped: a row tile's weights
+ * come from a table */
+OA_API int oa_host_gemm_kernel(int32_t M, int32_t N, int32_t K, int32_t epilogue, int32_t block_n, int32_t few_rows, int32_t grouped);
 /* byte-level BPE tokenizer read from a Hugging Face tokenizer.json (Llama-3 / Qwen2.5 format), host only: what the engine uses
  * for text when its config names one ("tokenizer": path) instead of the synthetic byte-level vocabulary.  Loaded files are cached
  * by path.  encode: *n_out = number of ids (written up to cap; OA_ERR_BAD_REQUEST if cap is too small or the file is unsupported);

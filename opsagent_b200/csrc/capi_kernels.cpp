@@ -1,5 +1,6 @@
-// capi_kernels.cpp — kernel-level C entry points on raw device pointers (parity tests drive these with
-// torch-allocated memory; nothing here is on the serving path).
+// capi_kernels.cpp — kernel-level C entry points on raw device pointers: the launchers that the models' forwards call, one product or one attention a
+// call, for programs that bring their own memory (tests and measurements bring torch's).  The engine calls the launchers, not these entries: what a call
+// adds here (scratch, tables, a synchronisation) is not part of a serving step.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -140,6 +141,27 @@ int oa_k_hybrid_gemm(int32_t mode, const void* A, int32_t lda, const void* B, in
                      int32_t batch, int64_t stride_a, int64_t stride_b, int64_t stride_c, void* stream) {
     if (mode != HY_STORE && mode != HY_STORE_F32 && mode != HY_ACC_F32) return OA_ERR_BAD_REQUEST;
     return rc_of(hy_gemm(false, mode, A, lda, B, ldb, C, ldc, M, N, K, nullptr, alpha, batch, stride_a, stride_b, stride_c, (cudaStream_t)stream));
+}
+
+int oa_k_gemm_ext(const void* A, const void* B, int32_t M, int32_t N, int32_t K, int32_t epilogue, int32_t block_n, void* out, const void* bias, int32_t act, int32_t act_col0,
+                  int32_t act_col1, float alpha, int32_t accumulate, void* stream) {
+    if (epilogue != EPI_STORE && epilogue != EPI_SWIGLU && epilogue != EPI_F32) return OA_ERR_BAD_REQUEST;
+    if (act < 0 || act > 3 || (epilogue == EPI_F32 && act != 0) || (epilogue == EPI_SWIGLU && act != 0 && act != 2)) return OA_ERR_BAD_REQUEST;
+    CUtensorMap tmA, tmB;
+    GemmParams p{}; p.M = M; p.N = N; p.K = K; p.few_rows_ok = 1;
+    if (epilogue == EPI_F32) { p.f32_out = (float*)out; p.ldf = N; p.bias_f32 = (const float*)bias; p.alpha = alpha; p.f32_accumulate = accumulate; }
+    else { p.out = out; p.ldo = epilogue == EPI_SWIGLU ? N / 2 : N; p.bias = epilogue == EPI_STORE ? bias : nullptr; }
+    if (epilogue == EPI_STORE) { p.store_act = act; p.act_col0 = act_col0; p.act_col1 = act_col1; } else p.glu_gelu = act == 2;
+    if (make_tmap_bf16_2d(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)K, (uint32_t)gemm_a_box(p, epilogue, block_n), 64) != 0) return OA_ERR_INTERNAL;
+    if (make_tmap_bf16_2d(&tmB, B, (uint64_t)N, (uint64_t)K, (uint64_t)K, (uint32_t)gemm_b_box(p, epilogue, block_n), 64) != 0) return OA_ERR_INTERNAL;
+    return rc_of(launch_gemm(&tmA, &tmB, p, epilogue, block_n, (cudaStream_t)stream));
+}
+
+int oa_host_gemm_kernel(int32_t M, int32_t N, int32_t K, int32_t epilogue, int32_t block_n, int32_t few_rows, int32_t grouped) {
+    GemmParams p{}; p.M = M; p.N = N; p.K = K; p.few_rows_ok = few_rows;
+    static const int32_t group = 0;
+    if (grouped) p.m_tile_group = &group;
+    return (int)gemm_kernel_of(p, epilogue, block_n);
 }
 
 static int paged_attention(const void* q, void* out, const void* kv_cache, int32_t num_pages, const int32_t* block_tables,

@@ -25,7 +25,7 @@ OA_DEVINL void raster_tile(int idx, int m_tiles, int n_tiles, int& m_blk, int& n
 
 // One warp: rows row_base .. row_base + 31 (TMEM lanes of `acc`), columns n0 .. n0 + bn - 1 of the product.  glu_sc: scales of the two rows this
 // lane stores in a clamped gated activation.
-template <int EPI>
+template <int EPI, bool CLAMPED = true>      // CLAMPED: the product may ask for the clamped gated activation (only grouped ones do)
 OA_DEVINL void persist_epilogue(const GemmParams& p, float* stage, uint32_t acc, int row_base, int n0, int bn, int lane, const float (&glu_sc)[2]) {
     // residual of the columns at hand and, on their way meanwhile, of the next ones (each lane reads and writes its own places: out may be resid)
     uint4 res[4], res_next[4];
@@ -65,7 +65,7 @@ OA_DEVINL void persist_epilogue(const GemmParams& p, float* stage, uint32_t acc,
                 const float gg[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
                 const float uu[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
                 float f[8];
-                if (p.glu_limit > 0.f) {
+                if (CLAMPED && p.glu_limit > 0.f) {
 #pragma unroll
                     for (int k = 0; k < 8; ++k) f[k] = clamped_glu_f32(gg[k] * glu_sc[i2], uu[k] * glu_sc[i2], p.glu_limit, p.glu_slope);
                 } else if (p.glu_gelu) {

@@ -144,18 +144,16 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
     } else {
         const int q = warp & 3;
         float* stage = epi_smem + (warp - 2) * (EPI_WARP_BYTES / 4);
+        const float no_scale[2] = {0.f, 0.f};
         griddep_wait();
         int it = 0;
         for (int t = pair; t < tiles; t += pairs, ++it) {
             int m_blk, n_blk; raster_tile(t, m_tiles, n_tiles, m_blk, n_blk, GP_GROUP_M);
             const int as = it & 1, row_base = m_blk * 256 + (int)rank * 128 + q * 32;
             const uint32_t acc = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * GP_BN);
-            float glu_sc[2] = {0.f, 0.f};          // scales of the two rows this lane stores (clamped gated activation), read while the tile is still being multiplied
-            if (EPI == EPI_SWIGLU && p.glu_limit > 0.f)
-                for (int i2 = 0; i2 < 2; ++i2) if (row_base + i2 * 16 + (lane >> 1) < p.M) glu_sc[i2] = glu_row_scale(p, row_base + i2 * 16 + (lane >> 1));
             gp_wait(&acc_full[as], ((uint32_t)it >> 1) & 1);
             tcgen05_fence_after();
-            if (row_base < p.M) persist_epilogue<EPI>(p, stage, acc, row_base, n_blk * GP_BN, GP_BN, lane, glu_sc);
+            if (row_base < p.M) persist_epilogue<EPI, false>(p, stage, acc, row_base, n_blk * GP_BN, GP_BN, lane, no_scale);
             tcgen05_fence_before();
             __syncwarp();
             if (lane == 0) gp_arrive_remote(gp_mapa(&acc_empty[as], 0));
@@ -187,7 +185,7 @@ static cudaError_t launch_gp(const CUtensorMap* tmA, const CUtensorMap* tmB, con
 }
 
 cudaError_t launch_gemm_pair(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epilogue, int sms, cudaStream_t stream) {
-    if (p.m_tile_group || sms < 2) return cudaErrorInvalidValue;
+    if (p.m_tile_group || p.glu_limit > 0.f || sms < 2) return cudaErrorInvalidValue;
     switch (epilogue) {
         case EPI_STORE: return launch_gp<EPI_STORE>(tmA, tmB, p, sms, stream);
         case EPI_RESID: return launch_gp<EPI_RESID>(tmA, tmB, p, sms, stream);

@@ -357,7 +357,6 @@ static bool head_persistent(int M, int N);
 static cudaError_t launch_head(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, cudaStream_t stream);
 static constexpr int HEAD_BN = 128;
 static int sm_count_cached();
-static long long persistent_min_tiles();
 template <int EPI>
 static cudaError_t launch_persistent(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, cudaStream_t stream);
 
@@ -365,62 +364,59 @@ static cudaError_t launch_persistent(const CUtensorMap* tmA, const CUtensorMap* 
 // us fitted to a sweep of 200 .. 8192 rows over the projections of the four model sizes: a k block takes 0.345 in a pair (0.39 once more than two rounds
 // run against the power cap), 0.42 in a 128 x 256 tile and 0.26 in a narrower one; outside the k loop 11 and 8.  E.g. 200 x 4096 x 4096: 64 tiles of 128
 // x 64 24 us, 16 pair tiles 32.  Up to 128 rows half of a pair's rows would be padding.  Every kernel sums k in the same order: the choice moves no bit.
-struct GemmChoice { bool pair, few; };
-static GemmChoice gemm_choose(const GemmParams& p, int epilogue, int block_n) {
-    GemmChoice best{false, false};
-    if ((block_n != 32 && block_n != 64 && block_n != 128 && block_n != 256) || p.M <= 0 || p.N <= 0 || p.K <= 0) return best;      // refused by launch_gemm
-    best.few = p.few_rows_ok && p.M <= FEW_MAX_ROWS && epilogue != EPI_LOGITS && !p.m_tile_group;
-    const int sms = sm_count_cached(), pairs = sms / 2;
-    if (epilogue == EPI_LOGITS || p.m_tile_group || p.M <= BLOCK_M || pairs < 1 || std::getenv("OA_GEMM_PERSISTENT_MIN_TILES")) return best;      // (tests that drive the 128 x 256 kernel set it)
+GemmKernel gemm_kernel_of(const GemmParams& p, int epilogue, int block_n) {
+    if (block_n != 32 && block_n != 64 && block_n != 128 && block_n != 256) return GEMM_NONE;
+    if (p.M <= 0 || p.N <= 0 || p.K <= 0 || (p.N % 8) != 0 || (p.K % 8) != 0) return GEMM_NONE;
+    if (epilogue == EPI_SWIGLU && (p.N % 32) != 0) return GEMM_NONE;
     auto up = [](long long a, long long b) { return (a + b - 1) / b; };
-    const double kb = (double)up(p.K, BLOCK_K);
-    const double single = (double)up(up(p.N, block_n) * up(p.M, BLOCK_M), sms) * kb * (block_n >= 256 ? 0.42 : 0.26) + 8.0;
-    const double rounds = (double)up(up(p.N, 256) * up(p.M, 256), pairs), pair = rounds * kb * (rounds > 2 ? 0.39 : 0.345) + 11.0;
-    best.pair = pair < single;
-    return best;
+    const int sms = sm_count_cached(), pairs = sms / 2;
+    if (epilogue == EPI_LOGITS) return block_n == HEAD_BN && head_persistent(p.M, p.N) ? GEMM_HEAD : GEMM_TILE;
+    // the threshold of the 128 x 256 kernel, where it is set: that kernel and plain tiles are all there is then
+    const char* forced = std::getenv("OA_GEMM_PERSISTENT_MIN_TILES");
+    if (!forced && p.few_rows_ok && p.M <= FEW_MAX_ROWS && !p.m_tile_group) return GEMM_FEW;
+    if (persistent_disabled()) return GEMM_TILE;
+    if (!forced && !p.m_tile_group && p.glu_limit <= 0.f && p.M > BLOCK_M && pairs > 0) {
+        const double kb = (double)up(p.K, BLOCK_K);
+        const double single = (double)up(up(p.N, block_n) * up(p.M, BLOCK_M), sms) * kb * (block_n >= 256 ? 0.42 : 0.26) + 8.0;
+        const double rounds = (double)up(up(p.N, 256) * up(p.M, 256), pairs), pair = rounds * kb * (rounds > 2 ? 0.39 : 0.345) + 11.0;
+        if (pair < single) return GEMM_PAIR;
+    }
+    return block_n == 256 && up(p.N, 256) * up(p.M, BLOCK_M) >= (forced ? std::atoll(forced) : 2LL * sms) ? GEMM_PERSISTENT : GEMM_TILE;
 }
-int gemm_b_box(const GemmParams& p, int epilogue, int block_n) {
-    return gemm_choose(p, epilogue, block_n).pair ? 128 : block_n;
-}
-int gemm_a_box(const GemmParams& p, int epilogue, int block_n) { return gemm_choose(p, epilogue, block_n).few ? few_box(p.M) : 128; }
+int gemm_b_box(const GemmParams& p, int epilogue, int block_n) { return gemm_kernel_of(p, epilogue, block_n) == GEMM_PAIR ? 128 : block_n; }
+int gemm_a_box(const GemmParams& p, int epilogue, int block_n) { return gemm_kernel_of(p, epilogue, block_n) == GEMM_FEW ? few_box(p.M) : 128; }
 
 cudaError_t launch_gemm(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epilogue, int block_n,
                         cudaStream_t stream) {
-    if (p.M <= 0 || p.N <= 0 || p.K <= 0 || (p.N % 8) != 0 || (p.K % 8) != 0) return cudaErrorInvalidValue;
-    if (epilogue == EPI_SWIGLU && (p.N % 32) != 0) return cudaErrorInvalidValue;
-    // large-M (prefill) shapes with the widest tile go to the persistent kernel (epilogue overlapped with the next tile)
     if (epilogue == EPI_F32 && ((p.ldf % 4) != 0 || !p.f32_out)) return cudaErrorInvalidValue;
-    const GemmChoice choice = gemm_choose(p, epilogue, block_n);
-    if (choice.few) {
-        switch (block_n) {
-            case 32: return launch_few_bn<32>(tmA, tmB, p, epilogue, stream);
-            case 64: return launch_few_bn<64>(tmA, tmB, p, epilogue, stream);
-            case 128: return launch_few_bn<128>(tmA, tmB, p, epilogue, stream);
-            case 256: return launch_few_bn<256>(tmA, tmB, p, epilogue, stream);
-        }
+    const GemmKernel kernel = gemm_kernel_of(p, epilogue, block_n);
+    switch (kernel) {
+        case GEMM_NONE: return cudaErrorInvalidValue;
+        case GEMM_HEAD: return launch_head(tmA, tmB, p, stream);
+        case GEMM_PAIR: return launch_gemm_pair(tmA, tmB, p, epilogue, sm_count_cached(), stream);
+        case GEMM_PERSISTENT:      // the widest tile over many rows: the epilogue overlaps the next tile
+            switch (epilogue) {
+                case EPI_STORE: return launch_persistent<EPI_STORE>(tmA, tmB, p, stream);
+                case EPI_RESID: return launch_persistent<EPI_RESID>(tmA, tmB, p, stream);
+                case EPI_SWIGLU: return launch_persistent<EPI_SWIGLU>(tmA, tmB, p, stream);
+                case EPI_F32: return launch_persistent<EPI_F32>(tmA, tmB, p, stream);
+            }
+            return cudaErrorInvalidValue;
+        case GEMM_FEW:
+        case GEMM_TILE: break;
     }
-    if (choice.pair) return launch_gemm_pair(tmA, tmB, p, epilogue, sm_count_cached(), stream);
-    if (block_n == 256 && epilogue != EPI_LOGITS && !persistent_disabled() &&
-        (long long)((p.N + 255) / 256) * ((p.M + BLOCK_M - 1) / BLOCK_M) >= persistent_min_tiles()) {
-        switch (epilogue) {
-            case EPI_STORE: return launch_persistent<EPI_STORE>(tmA, tmB, p, stream);
-            case EPI_RESID: return launch_persistent<EPI_RESID>(tmA, tmB, p, stream);
-            case EPI_SWIGLU: return launch_persistent<EPI_SWIGLU>(tmA, tmB, p, stream);
-            case EPI_F32: return launch_persistent<EPI_F32>(tmA, tmB, p, stream);
-        }
-    }
-    if (epilogue == EPI_LOGITS && block_n == HEAD_BN && head_persistent(p.M, p.N)) return launch_head(tmA, tmB, p, stream);
+    const bool few = kernel == GEMM_FEW;
     switch (block_n) {
-        case 32: return launch_bn<32>(tmA, tmB, p, epilogue, stream);
-        case 64: return launch_bn<64>(tmA, tmB, p, epilogue, stream);
-        case 128: return launch_bn<128>(tmA, tmB, p, epilogue, stream);
-        case 256: return launch_bn<256>(tmA, tmB, p, epilogue, stream);
+        case 32: return few ? launch_few_bn<32>(tmA, tmB, p, epilogue, stream) : launch_bn<32>(tmA, tmB, p, epilogue, stream);
+        case 64: return few ? launch_few_bn<64>(tmA, tmB, p, epilogue, stream) : launch_bn<64>(tmA, tmB, p, epilogue, stream);
+        case 128: return few ? launch_few_bn<128>(tmA, tmB, p, epilogue, stream) : launch_bn<128>(tmA, tmB, p, epilogue, stream);
+        case 256: return few ? launch_few_bn<256>(tmA, tmB, p, epilogue, stream) : launch_bn<256>(tmA, tmB, p, epilogue, stream);
     }
     return cudaErrorInvalidValue;
 }
 
 // =============================================================================================
-// persistent tile GEMM (grouped products, and prefill shapes that gemm_choose leaves here): one CTA per SM loops over 128 x 256 tiles in grouped raster order; TMEM holds
+// persistent tile GEMM (grouped products, and prefill shapes that gemm_kernel_of leaves here): one CTA per SM loops over 128 x 256 tiles in grouped raster order; TMEM holds
 // TWO accumulators so the epilogue of tile i (tcgen05.ld -> smem transpose -> coalesced bf16 stores, fused bias /
 // residual / SwiGLU) overlaps the tcgen05.mma main loop of tile i+1.
 // =============================================================================================
@@ -662,8 +658,6 @@ static bool head_persistent(int M, int N) { return (long long)gemm_n_tiles(N, He
 int gemm_logits_bn(int M, int N, int block_n) { return (block_n == 128 || block_n == 256) && head_persistent(M, N) ? HeadCfg::BN : block_n; }
 
 static bool persistent_disabled() { static const bool off = [] { const char* e = std::getenv("OA_GEMM_PERSISTENT"); return e && e[0] == '0'; }(); return off; }
-// tests lower the threshold (OA_GEMM_PERSISTENT_MIN_TILES=1) to drive tiny shapes through the persistent kernel
-static long long persistent_min_tiles() { const char* e = std::getenv("OA_GEMM_PERSISTENT_MIN_TILES"); return e ? std::atoll(e) : 2LL * sm_count_cached(); }
 static int sm_count_cached() {
     static int n = 0;
     if (n == 0) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev); if (n <= 0) n = 148; }

@@ -48,6 +48,10 @@ struct GemmParams {
 cudaError_t launch_gemm(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epilogue, int block_n,
                         cudaStream_t stream);
 int gemm_n_tiles(int N, int block_n);
+// which kernel launch_gemm runs for a product: a 128 x block_n tile per CTA (FEW: of up to 64 loaded rows), the persistent 128 x 256 tiles, CTA pairs, the
+// persistent vocabulary head; NONE: refused.  All sum k in ascending order in one accumulator: the choice moves no bit.
+enum GemmKernel : int { GEMM_NONE = -1, GEMM_TILE = 0, GEMM_FEW = 1, GEMM_PERSISTENT = 2, GEMM_PAIR = 3, GEMM_HEAD = 4 };
+GemmKernel gemm_kernel_of(const GemmParams& p, int epilogue, int block_n);
 int gemm_logits_bn(int M, int N, int block_n);      // EPI_LOGITS: the tile width to ask launch_gemm for (and to count the arg-max partials by) where block_n would do
 // rows of the B tensor map's box that launch_gemm(.., block_n, ..) reads for this product: block_n, or what the CTA-pair kernel takes where that runs
 int gemm_b_box(const GemmParams& p, int epilogue, int block_n);
@@ -167,6 +171,7 @@ struct DecodeAttnParams {
     float scale_log2e;             // (1/sqrt(D)) * log2(e)
 };
 cudaError_t launch_decode_attention(const CUtensorMap* tm_kv, const KvLayout& kv, const DecodeAttnParams& p, cudaStream_t s);
+
 struct MergeItem { int32_t seq, kvh, slot_begin, n_slots; };
 
 constexpr int PREFILL_TILE_ROWS = 128;                     // query rows of one (tile, head) CTA

@@ -2,6 +2,9 @@
 invariants, model presets, Chat() retry semantics of the Python mirror (reference pkg/llms/openai.go:69-104)."""
 import ctypes as C
 import json
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -707,3 +710,27 @@ def test_get_token_limits_and_constrict_messages_follow_the_reference():
     assert [m.Content[0] for m in got] == ["s", "c"]                                                       # system prompt + the newest that fit
     with pytest.raises(IndexError):
         ConstrictMessages([M("system", "s" * 1000)], "m", 100, count, engine_limit=600)                   # the reference panics here
+
+
+def test_which_kernel_a_product_takes(monkeypatch):
+    """host rule of the products (148 SMs): few rows, CTA pairs, persistent tiles, the vocabulary head; refused sizes; the debug switches"""
+    L = _lib.load()
+    TILE, FEW, PERSISTENT, PAIR, HEAD = 0, 1, 2, 3, 4
+    k = L.oa_host_gemm_kernel
+    for epi in (0, 1, 2, 4):
+        assert k(64, 4096, 4096, epi, 64, 1, 0) == FEW and k(64, 4096, 4096, epi, 64, 0, 0) == TILE and k(65, 4096, 4096, epi, 64, 1, 0) == TILE
+        assert k(8192, 28672, 4096, epi, 256, 1, 0) == PAIR and k(8192, 28672, 4096, epi, 256, 0, 1) == PERSISTENT and k(16, 4096, 4096, epi, 256, 1, 1) == TILE
+        assert k(200, 4096, 4096, epi, 64, 1, 0) == TILE              # 64 narrow tiles finish before 16 pairs do
+    assert k(128, 128256, 4096, 3, 128, 1, 0) == HEAD and k(128, 32000, 4096, 3, 128, 1, 0) == TILE and k(128, 128256, 4096, 3, 64, 1, 0) == TILE
+    for bad in ((0, 64, 64, 0, 64), (8, 60, 64, 0, 64), (8, 64, 60, 0, 64), (8, 48, 64, 2, 64), (8, 64, 64, 0, 96), (700, 64, 64, 0, 0)):
+        assert k(*bad, 1, 0) == -1
+    monkeypatch.setenv("OA_GEMM_PERSISTENT_MIN_TILES", "1")
+    assert k(64, 4096, 4096, 0, 256, 1, 0) == PERSISTENT and k(8192, 28672, 4096, 0, 256, 1, 0) == PERSISTENT and k(300, 1024, 512, 0, 128, 1, 0) == TILE
+
+
+@pytest.mark.parametrize("value,kernel", [("0", 0), ("1", 3)])
+def test_the_switch_that_turns_persistent_products_off(value, kernel):
+    """OA_GEMM_PERSISTENT=0: one CTA per tile for every product, also for those that CTA pairs would take"""
+    code = "from opsagent_b200 import _lib; print(_lib.load().oa_host_gemm_kernel(8192, 28672, 4096, 0, 256, 0, 0))"
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))), env=dict(os.environ, OA_GEMM_PERSISTENT=value))
+    assert r.returncode == 0 and int(r.stdout) == kernel, (r.stdout, r.stderr[-500:])

@@ -343,13 +343,19 @@ def test_streamk_result_on_any_float_boundary(L):
     assert torch.equal(whole[1:].view(M, N), out)
 
 
-# CTA-pair kernel: whole tiles, tiles cut in two and in three (alone and behind a whole round), ragged last rows and columns, one CTA's rows all
-# beyond the last; every epilogue.  M, N, K chosen so that the rule takes each (2 or 3 pieces need a k range of some length).
-PAIR_CASES = [(300, 3072, 1024), (257, 6152, 320), (400, 2048, 8192), (614, 4096, 14336), (1337, 4096, 14336), (1000, 5120, 4160), (384, 296, 27648), (2000, 1000, 8192), (513, 2304, 72)]
+TILE, FEW, PERSISTENT, PAIR, HEAD = 0, 1, 2, 3, 4                  # oa_host_gemm_kernel
+
+
+# CTA-pair kernel: one round of tiles and several, ragged last rows and columns, one CTA's rows all beyond the last, and k ranges shorter than the ring
+# over many tiles (ring phases run across tiles, accumulators change hands every block or two); store, residual and gated.  Which kernel a product takes is
+# asserted: a rule that moves must not empty a case.
+PAIR_CASES = [(614, 6144, 4096), (257, 6152, 4096), (700, 6152, 2056), (400, 2048, 8192), (614, 4096, 14336), (1337, 4096, 14336), (1000, 5120, 4160), (384, 296, 27648), (2000, 1000, 8192),
+              (7900, 14336, 320), (8192, 24576, 192)]
 
 
 @pytest.mark.parametrize("M,N,K", PAIR_CASES)
 def test_gemm_cta_pairs(L, M, N, K):
+    assert L.oa_host_gemm_kernel(M, N, K, EPI_STORE, 256, 1, 0) == PAIR
     g = torch.Generator(device=dev()).manual_seed(M + N + K)
     A = torch.randn(M, K, generator=g, device=dev()).to(torch.bfloat16)
     B = (torch.randn(N, K, generator=g, device=dev()) * 0.05).to(torch.bfloat16)
@@ -361,7 +367,7 @@ def test_gemm_cta_pairs(L, M, N, K):
         assert torch.isfinite(got.float()).all()
         assert ((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + s + extra + 1e-6).all(), float((got.double() - want).abs().max())
     outs = []
-    for _ in range(2):                               # twice: counters must be zero again, and the order of summation is fixed
+    for _ in range(2):                               # the order of summation is fixed
         out = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=dev())
         assert L.oa_k_gemm(ptr(A), ptr(B), M, N, K, EPI_STORE, 256, ptr(out), ptr(bias), None, None, None, None) == 0
         torch.cuda.synchronize(); outs.append(out)
@@ -380,12 +386,14 @@ def test_gemm_cta_pairs(L, M, N, K):
         close(y, (torch.nn.functional.silu(v[:, :, 0]) * v[:, :, 1]).reshape(M, N // 2), 2e-5 * float(v.abs().max()) ** 2)
 
 
-# few-row kernel: every row tile, clusters of 1, 2, 4 and 8 CTAs, ragged rows and columns, k ranges that do not divide evenly; every epilogue
+# products of a few rows: every box of loaded rows and the plain tile behind the last, fewer k blocks than ring stages and more, ragged rows and columns,
+# tiles for one CTA per SM and for two; store, residual and gated
 ROWS_CASES = [(1, 1024, 1088), (3, 2048, 4096), (16, 28672, 320), (17, 4096, 2056), (16, 9000, 1024), (32, 6144, 4160), (33, 2048, 1024), (64, 1000, 8192), (50, 6208, 4096), (65, 2048, 4096), (128, 4096, 4160), (100, 296, 14336)]
 
 
 @pytest.mark.parametrize("M,N,K", ROWS_CASES)
 def test_gemm_few_rows(L, M, N, K):
+    assert L.oa_host_gemm_kernel(M, N, K, EPI_STORE, 128, 1, 0) == (FEW if M <= 64 else TILE)
     g = torch.Generator(device=dev()).manual_seed(M + N + K)
     A = torch.randn(M, K, generator=g, device=dev()).to(torch.bfloat16)
     B = (torch.randn(N, K, generator=g, device=dev()) * 0.05).to(torch.bfloat16)
@@ -419,6 +427,7 @@ def test_gemm_few_rows(L, M, N, K):
 # persistent vocabulary head: fewer k blocks than ring stages and more, one and several row tiles, a ragged last tile, the largest in the last column
 @pytest.mark.parametrize("M,N,K", [(1, 128256, 64), (128, 38016, 200), (3, 128256, 1024), (129, 40008, 512), (64, 152064, 448)])
 def test_persistent_vocabulary_head(L, M, N, K):
+    assert L.oa_host_gemm_kernel(M, N, K, EPI_LOGITS, 128, 1, 0) == HEAD
     g = torch.Generator(device=dev()).manual_seed(N + K)
     A = torch.randn(M, K, generator=g, device=dev()).to(torch.bfloat16)
     B = (torch.randn(N, K, generator=g, device=dev()) * 0.1).to(torch.bfloat16)
@@ -447,8 +456,8 @@ def test_gemm_refuses_tile_widths_it_has_no_kernel_for(L, M, epi, bn):
     torch.cuda.synchronize()
 
 
-def test_gemm_with_cut_tiles_under_stream_capture(L):
-    """a product whose last round is cut takes scratch from the pool: captured, it replays to the same bits"""
+def test_gemm_with_a_partial_last_round_under_stream_capture(L):
+    """a product on CTA pairs whose tiles do not fill the last round: captured, it replays to the same bits"""
     M, N, K = 614, 4096, 14336
     g = torch.Generator(device=dev()).manual_seed(5)
     A = torch.randn(M, K, generator=g, device=dev()).to(torch.bfloat16); B = (torch.randn(N, K, generator=g, device=dev()) * 0.05).to(torch.bfloat16)
@@ -567,3 +576,50 @@ def test_few_row_products_are_an_fp32_chain(L, M, N, K, batch):
     torch.cuda.synchronize()
     assert (out.cpu().numpy() == want).all(), int((out.cpu().numpy() != want).sum())
     assert torch.equal(out16, out.to(torch.bfloat16))
+
+
+# What the hybrid models ask of the epilogues, on every kernel that has them: fp32 results with alpha, bias and accumulation, activations on a store, the
+# gated form of GELU; ragged rows and columns, whole and partial tiles.
+EXT_CASES = [(1, 2048, 1024, 32, FEW), (17, 1000, 328, 64, FEW), (64, 4104, 2056, 128, FEW), (40, 512, 64, 256, FEW), (100, 1032, 520, 64, TILE), (200, 1024, 512, 64, TILE),
+             (1337, 4096, 4096, 256, PAIR), (1100, 6152, 2056, 256, PAIR), (7900, 14336, 320, 256, PAIR), (9000, 2560, 128, 256, PERSISTENT)]
+
+
+@pytest.mark.parametrize("M,N,K,bn,kernel", EXT_CASES)
+def test_gemm_epilogues_of_the_hybrid_models(L, M, N, K, bn, kernel, monkeypatch):
+    if kernel == PERSISTENT:
+        monkeypatch.setenv("OA_GEMM_PERSISTENT_MIN_TILES", "1")       # leaves the pairs out
+    for epi in (0, 4) + ((2,) if N % 32 == 0 else ()):
+        assert L.oa_host_gemm_kernel(M, N, K, epi, bn, 1, 0) == kernel
+    g = torch.Generator(device=dev()).manual_seed(M + N + K)
+    A = torch.randn(M, K, generator=g, device=dev()).to(torch.bfloat16)
+    B = (torch.randn(N, K, generator=g, device=dev()) * K ** -0.5).to(torch.bfloat16)
+    ref = A.double() @ B.double().T
+    s = 4 * K ** 0.5 * 2.0 ** -23                                     # fp32 sums of K products of unit variance in all
+    bias32 = torch.randn(N, generator=g, device=dev())
+    for alpha, use_bias, acc in ((1.0, True, 0), (-0.375, True, 1), (0.0, False, 1), (1.7, False, 0)):
+        start = torch.randn(M, N, generator=g, device=dev())
+        out = start.clone() if acc else torch.full((M, N), float("nan"), device=dev())
+        assert L.oa_k_gemm_ext(ptr(A), ptr(B), M, N, K, 4, bn, ptr(out), ptr(bias32) if use_bias else None, 0, 0, 0, alpha, acc, None) == 0
+        torch.cuda.synchronize()
+        want = ref * (alpha if alpha != 0 else 1.0) + (bias32.double() if use_bias else 0) + (start.double() if acc else 0)
+        assert ((out.double() - want).abs() <= 2 * s + want.abs() * 2.0 ** -22).all(), float((out.double() - want).abs().max())
+    bias = torch.randn(N, generator=g, device=dev()).to(torch.bfloat16)
+    v = ref + bias.double()
+    c0, c1 = N // 4 // 8 * 8, N // 2 // 8 * 8
+    cols = torch.arange(N, device=dev())
+    silu = torch.where((cols >= c0) & (cols < c1), torch.nn.functional.silu(v), v)
+    for act, want in ((0, v), (1, torch.relu(v) ** 2), (2, torch.nn.functional.gelu(v, approximate="tanh")), (3, silu)):
+        out = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=dev())
+        assert L.oa_k_gemm_ext(ptr(A), ptr(B), M, N, K, 0, bn, ptr(out), ptr(bias), act, c0, c1, 0.0, 0, None) == 0
+        torch.cuda.synchronize()
+        # half an ulp of bf16, and fp32 arithmetic of the activation: relative 2^-16 of the arguments it is made of, whose slope stays under 2 |v| + 2
+        assert ((out.double() - want).abs() <= want.abs() * 2.0 ** -8 + (2 * v.abs() + 2) * (s + v.abs() * 2.0 ** -16) + 1e-6).all(), (act, float((out.double() - want).abs().max()))
+    if N % 32 == 0:
+        gate, up = ref.view(M, N // 32, 2, 16)[:, :, 0], ref.view(M, N // 32, 2, 16)[:, :, 1]
+        for act, f in ((0, torch.nn.functional.silu(gate)), (2, torch.nn.functional.gelu(gate, approximate="tanh"))):
+            out = torch.full((M, N // 2), float("nan"), dtype=torch.bfloat16, device=dev())
+            assert L.oa_k_gemm_ext(ptr(A), ptr(B), M, N, K, 2, bn, ptr(out), None, act, 0, 0, 0.0, 0, None) == 0
+            torch.cuda.synchronize()
+            want = (f * up).reshape(M, N // 2)
+            room = ((gate.abs() + 1) * (up.abs() + 1)).reshape(M, N // 2)
+            assert ((out.double() - want).abs() <= want.abs() * 2.0 ** -8 + room * (4 * s + 2.0 ** -15) + 1e-6).all(), (act, float((out.double() - want).abs().max()))
