@@ -183,7 +183,7 @@ static int paged_attention(const void* q, void* out, const void* kv_cache, int32
         DecodePlan plan;
         build_decode_plan(ctx_lens, n_seqs, n_kv, 2 * 148, force_splits, plan);
         const size_t o_segs = host.add(plan.segs.data(), plan.segs.size() * sizeof(DecodeSeg)), o_ptr = host.add(plan.cta_ptr.data(), plan.cta_ptr.size() * 4);
-        const std::vector<int32_t> zeros(plan.merges.size() + 1, 0);
+        const std::vector<int32_t> zeros(plan.n_cut + 1, 0);
         const size_t o_count = host.add(zeros.data(), zeros.size() * 4);         // merge counters: the CTA with an item's last piece merges it
         const size_t o_po = (host.bytes.size() + 255) & ~size_t(255), o_pml = o_po + (size_t)(plan.n_slots + 1) * grp * head_dim * 4;
         DevBuf d_meta(o_pml + (size_t)(plan.n_slots + 1) * grp * 2 * 4, s);       // [tables, plan, counters | partial outputs | partial maxima and sums]

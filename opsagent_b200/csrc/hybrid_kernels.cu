@@ -437,7 +437,6 @@ __global__ void __launch_bounds__(128) hy_mla_attention_mma_kernel(HyLatentAttn 
     }
 }
 
-// joins the parts of a decoding row: out = sum_p 2^(m_p - M) O_p / sum_p 2^(m_p - M) l_p, parts in order
 // ---------------------------------------------------------------------------------------------------------------------------------
 // the same for ONE row of a sequence with at most 16 heads (a decoding row): its queries fill one warp's 16 mma rows, so the four warps take
 // turns at groups of 16 cache rows instead, each with an online softmax and accumulators of its own, joined once at the end.  Cache rows come
@@ -599,6 +598,7 @@ __global__ void __launch_bounds__(128) hy_mla_decode_mma_kernel(HyLatentAttn a, 
     }
 }
 
+// joins the parts of a decoding row: out = sum_p 2^(m_p - M) O_p / sum_p 2^(m_p - M) l_p, parts in order
 __global__ void __launch_bounds__(128) hy_mla_merge_kernel(const int32_t* item_row, const int32_t* item_slot0, const int32_t* item_parts, const float* ws_o,
                                                            const float* ws_ml, __nv_bfloat16* lat_out, int H, int R, const float* sink,
                                                            const __nv_bfloat16* head_gate, int ldg) {

@@ -172,8 +172,6 @@ struct DecodeAttnParams {
 };
 cudaError_t launch_decode_attention(const CUtensorMap* tm_kv, const KvLayout& kv, const DecodeAttnParams& p, cudaStream_t s);
 
-struct MergeItem { int32_t seq, kvh, slot_begin, n_slots; };
-
 constexpr int PREFILL_TILE_ROWS = 128;                     // query rows of one (tile, head) CTA
 struct PrefillTile { int32_t seq, q_row0, pos0, n_rows; };  // <= PREFILL_TILE_ROWS rows of one sequence; q_row0 = row in the token batch
 struct PrefillAttnParams {

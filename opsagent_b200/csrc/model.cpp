@@ -332,7 +332,7 @@ int DeviceModel::pick_bn(int M, int N, int override_bn, bool swiglu) const {
 }
 
 void build_decode_plan(const int32_t* ctx_lens, int n_seqs, int n_kv, int n_ctas_target, int force_splits, DecodePlan& out) {
-    out.segs.clear(); out.cta_ptr.clear(); out.merges.clear(); out.n_slots = 0;
+    out.segs.clear(); out.cta_ptr.clear(); out.n_slots = 0; out.n_cut = 0;
     long long total = 0;
     for (int i = 0; i < n_seqs; ++i) total += (long long)((ctx_lens[i] + 63) / 64) * n_kv;
     if (total <= 0) { out.cta_ptr.push_back(0); return; }
@@ -343,13 +343,12 @@ void build_decode_plan(const int32_t* ctx_lens, int n_seqs, int n_kv, int n_ctas
             const int nch = (ctx_lens[s] + 63) / 64; if (nch == 0) continue;
             const int pieces = std::min(force_splits, nch), per = (nch + pieces - 1) / pieces;
             const int real = (nch + per - 1) / per;
-            MergeItem mi{s, h, out.n_slots, real};
-            const int slot0 = out.n_slots, item = (int)out.merges.size();
+            const int slot0 = out.n_slots, item = out.n_cut;
             for (int pz = 0; pz < real; ++pz) {
                 DecodeSeg sg{s, h, pz * per, std::min(nch, (pz + 1) * per), real > 1 ? out.n_slots++ : -1, slot0, real, item};
                 out.segs.push_back(sg); out.cta_ptr.push_back((int32_t)out.segs.size());
             }
-            if (real > 1) out.merges.push_back(mi);
+            out.n_cut += real > 1;
         }
         return;
     }
@@ -364,14 +363,13 @@ void build_decode_plan(const int32_t* ctx_lens, int n_seqs, int n_kv, int n_ctas
         const long long g0 = gpos, g1 = gpos + nch;
         const long long c_first = g0 / per, c_last = (g1 - 1) / per;
         const int pieces = (int)(c_last - c_first + 1);
-        MergeItem mi{s, h, out.n_slots, pieces};
-        const int slot0 = out.n_slots, item = (int)out.merges.size();
+        const int slot0 = out.n_slots, item = out.n_cut;
         for (long long c = c_first; c <= c_last; ++c) {
             const long long a = std::max(g0, c * per), b = std::min(g1, (c + 1) * per);
             DecodeSeg sg{s, h, (int32_t)(a - g0), (int32_t)(b - g0), pieces > 1 ? out.n_slots++ : -1, slot0, pieces, item};
             out.segs.push_back(sg); cta_of_seg.push_back((int)c);
         }
-        if (pieces > 1) out.merges.push_back(mi);
+        out.n_cut += pieces > 1;
         gpos = g1;
     }
     // segs are already ordered by CTA; build the CSR pointer
@@ -420,7 +418,7 @@ void DeviceModel::forward(const StepInput& in, float* logits_out) {
         if (plan_.n_slots > max_part_slots_) throw std::runtime_error("forward: partial workspace overflow");
         o_segs = put(plan_.segs.data(), plan_.segs.size() * 8);
         o_ptr = put(plan_.cta_ptr.data(), plan_.cta_ptr.size());
-        zero_counters_.assign(plan_.merges.size() + 1, 0);
+        zero_counters_.assign(plan_.n_cut + 1, 0);
         o_cnt = put(zero_counters_.data(), zero_counters_.size());     // merge counters start every step at zero
     }
     if (!in.decode) {

@@ -37,7 +37,7 @@ struct StepInput {
 };
 
 struct DecodePlan {
-    std::vector<DecodeSeg> segs; std::vector<int32_t> cta_ptr; std::vector<MergeItem> merges; int n_slots = 0;
+    std::vector<DecodeSeg> segs; std::vector<int32_t> cta_ptr; int n_slots = 0, n_cut = 0;      // n_cut: items cut into pieces (DecodeSeg::item counts them)
 };
 // contiguous, balanced partition of all (sequence, kv head) page lists over n_ctas CTAs
 void build_decode_plan(const int32_t* ctx_lens, int n_seqs, int n_kv, int n_ctas_target, int force_splits, DecodePlan& out);
