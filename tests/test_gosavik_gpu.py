@@ -324,10 +324,10 @@ def test_greedy_generation_through_the_scheduler(tmp_path):
             seq.append(tok)
 
 
-@pytest.mark.parametrize("heads,rank,rot,window", [(16, 64, 16, None), (1, 128, 16, 45), (5, 256, 32, 33), (16, 512, 64, 130), (8, 192, 16, 20)])
+@pytest.mark.parametrize("heads,rank,rot,window", [(16, 64, 16, None), (1, 128, 16, 45), (5, 256, 32, 33), (16, 512, 64, 130), (8, 192, 16, 20), (16, 768, 16, None), (16, 768, 64, 77), (16, 1024, 32, 100)])
 def test_decoding_rows_of_latent_attention_split_their_keys_over_warps(tmp_path, heads, rank, rot, window):
     """one row, up to 16 heads: groups of 16 cache rows per warp — contexts around 16, 64 and the parts' edges, windows that begin inside a group,
-    every split of the latent's channels; a portion and a decoding row in one step; one stage per warp for the wide latent"""
+    every split of the latent's channels; a portion and a decoding row in one step; rings of two stages a warp and, from 768 channels on, of one"""
     layers = [G.latent_layer(heads=heads, dim=32, rot_dim=rot, vdim=32, kv_rank=rank, q_rank=48, window=window, base=10000.0, mlp=64)]
     cfg = G.make_config(layers, width=64, vocab=72, streams=2)
     W = checkpoint(tmp_path, cfg, 31)
@@ -349,3 +349,21 @@ def test_decoding_rows_of_latent_attention_split_their_keys_over_warps(tmp_path,
             got.append(eng.trace_step([(1, [a[i]], [0])], [1] if i == 289 else []))
     check(np.concatenate(got), ref_a, "bfloat16")
     check(np.concatenate(rows_b), ref_b, "bfloat16")
+
+
+@pytest.mark.parametrize("heads,rank,rot,window", [(16, 768, 16, None), (16, 768, 64, 300), (12, 128, 16, None), (16, 512, 64, 530)])
+def test_decoding_rows_of_latent_attention_cut_into_parts(tmp_path, heads, rank, rot, window):
+    """contexts of 512 rows and more are cut into parts, one CTA each, joined afterwards: both ring depths, windows that leave parts empty or begin inside one"""
+    layers = [G.latent_layer(heads=heads, dim=32, rot_dim=rot, vdim=32, kv_rank=rank, q_rank=48, window=window, base=10000.0, mlp=64)]
+    cfg = G.make_config(layers, width=64, vocab=72, streams=2)
+    W = checkpoint(tmp_path, cfg, 37)
+    a = tokens_of(cfg, 800, 3)
+    ref = G.forward(cfg, W, a)
+    got = []
+    with engine(tmp_path, "bfloat16", pages=14) as eng:
+        for r0, r1 in ((500, 530), (760, 800)):
+            at = len(got) and 530
+            eng.trace_step([(1, a[at:r0], [])])
+            for i in range(r0, r1):
+                got.append(eng.trace_step([(1, [a[i]], [0])], [1] if i == 799 else []))
+    check(np.concatenate(got), np.concatenate([ref[500:530], ref[760:800]]), "bfloat16")
