@@ -4,14 +4,14 @@
 // memory, and one thread of the even CTA issues 256 x 256 x 16 products that read both halves.  Against a 128 x 256 tile per SM that is 2/3 of the
 // shared-memory reads and of the L2 traffic per product, and six k blocks of 32 KB in flight instead of four of 48 KB.  Large products run against the
 // 1000 W cap here (85 % of the tensor peak at a clock that is down to 1.25 GHz), so what counts is the energy per product.  Against 128 x 256 tiles,
-// us in a sustained loop: 8192 x 28672 x 4096 gated 1472 -> 1413, 8192 x 7168 x 5120 485 -> 459, 8192 x 4096 x 14336 residual 788 -> 751; for a single
-// prompt, where a k block costs 0.35 us a tile whatever its width: 614 x 6144 x 4096 47 -> 32, 1337 x 4096 x 4096 residual 72 -> 53.
+// us a call in a loop: 8192 x 28672 x 4096 gated 1505 -> 1445, 8192 x 7168 x 5120 499 -> 471; for a single prompt, where the rounds of tiles count: 614 x
+// 6144 x 4096 47 -> 32, 1337 x 4096 x 4096 residual 72 -> 53.
 //   warp 0   : TMA producer of this CTA's A rows and B half; both CTAs' bytes are counted on the EVEN CTA's `full` barrier
 //   warp 1   : allocates TMEM (both CTAs); in the even CTA one thread issues the products; commits release the ring slot in both CTAs
 //   warps 2-5: epilogue of this CTA's 128 rows while the next tile is multiplied (two accumulators of 256 columns)
 // Persistent over tiles in grouped raster order.  Every tile sums its k blocks in ascending order in one accumulator, as the single-CTA kernels do: a
 // row's bits depend neither on how many rows share the product nor on its place among them.  (The last round's tiles cut along k filled idle pairs,
-// 16 to 20 us of a product whose tiles fill half a round, and gave that up: 1337 x 4096 x 14336 residual 156 -> 172, against 192 in single-CTA tiles.)
+// 16 to 20 us of a product whose tiles fill half a round, and gave that up: 1337 x 4096 x 14336 residual 153 -> 170, against 191 in single-CTA tiles.)
 #include <algorithm>
 
 #include "common.cuh"
