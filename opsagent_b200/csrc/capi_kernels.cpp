@@ -32,9 +32,9 @@ namespace {
 constexpr uint64_t SCRATCH_KEEP_BYTES = 64ull << 20;
 cudaMemPool_t scratch_pool() {
     static std::mutex mu;
-    static std::map<int, cudaMemPool_t> pools;
+    static cudaMemPool_t pools[64] = {};         // by device; nothing here may throw through the C boundary
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
     std::lock_guard<std::mutex> lk(mu);
     cudaMemPool_t& pool = pools[dev];
     if (!pool) {
