@@ -1,7 +1,7 @@
 #!/usr/bin/env python
-"""bench.py — the reference's headline metric on BASELINE.json configs[1]:
+"""bench.py — the reference's headline metric:
 Llama-3-8B bf16, 1xB200, batch=128 concurrent `analyze` ReAct steps over synthetic Pod YAML
-(P=1536 prompt tokens, G=256 generated tokens, mean decode context 1664; SURVEY.md §8d config 2).
+(P=1536 prompt tokens, G=256 generated tokens, mean decode context 1664).
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
 
@@ -14,10 +14,10 @@ A "step" is one decode forward of the whole batch (128 sequences, one new token 
   roofline: dominant kernel = paged decode attention; achieved = algorithmic KV bytes per launch / mean launch time
            (CUDA events on the engine stream) against the measured HBM copy bandwidth.
   cpu_baseline: the CPU oracle (a port — the reference has no model arithmetic of its own) on the host cores.
-N>1 = data-parallel replicas (BASELINE configs[2]): one engine per GPU, no data-path collective, weak scaling.
+N>1 = data-parallel replicas: one engine per GPU, no data-path collective, weak scaling.
 N>=2 additionally runs, AFTER the headline (metric/value unchanged), the tensor-parallel path at t = N over the same N ranks:
   tp.parity : tests/tp_worker.py at t=N against the CPU oracle (t=4: Qwen2.5-32B TP=4's per-rank head layout, t=8: Llama-3-70B TP=8's)
-  tp.*      : BASELINE configs[3] (Qwen2.5-32B TP=4, B=256, ctx 2048) at N=4, configs[4] (Llama-3-70B TP=8, B=64, ctx 16.9k incl. its
+  tp.*      : Qwen2.5-32B TP=4 (B=256, ctx 2048) at N=4, Llama-3-70B TP=8 (B=64, ctx 16.9k incl. its
               1.08M-token prefill) at N=8, Llama-3-8B TP=2 at N=2 — decode ms/step, tokens/s per group and per GPU, fraction of the per-GPU
               HBM roofline, the all-reduce chain (in-situ us per all-reduce x count per step).
 `--impl reference` times the CPU port alone (rank 0 only), same JSON line shape.
@@ -94,7 +94,7 @@ KVB = {"qwen2.5-32b": 262144, "llama-3-70b": 327680, "llama-3-8b": 131072}
 
 
 def run_tp_block(args, rank, world, nonce, log):
-    """Tensor parallelism at t = world over the same ranks: parity first (checker: the CPU oracle on rank 0), then the BASELINE TP
+    """Tensor parallelism at t = world over the same ranks: parity first (checker: the CPU oracle on rank 0), then the TP
     config for this N.  Rank 0 returns the "tp" block, followers return None.  Own NVLink peer-memory all-reduce, no NCCL on the data path."""
     import importlib.util
     from opsagent_b200 import Engine
@@ -448,8 +448,8 @@ def run_ours(args, rank, world, local_rank):
                          "frac": round(r["algorithmic_bytes_per_step"] / (ms_step * 1e-3) / 1e9 / peak, 4)}}
     # ------------------------------------------------------------------ e2e: public chat API, host buffers
     # The reference's own request shapes with its system prompts VERBATIM (opsagent_b200/workloads.py <- tests/golden/prompts/), tokenised
-    # by the engine's byte-level BPE.  N=1: BASELINE configs[1], 128 analyze requests padded with synthetic Pod YAML to P=1536 tokens.
-    # N>=2: configs[2]'s mix per replica: 40 % analyze (P=1536) / 30 % diagnose / 30 % execute (zh prompt); diagnose and execute carry no
+    # by the engine's byte-level BPE.  N=1: 128 analyze requests padded with synthetic Pod YAML to P=1536 tokens.
+    # N>=2: the mix per replica: 40 % analyze (P=1536) / 30 % diagnose / 30 % execute (zh prompt); diagnose and execute carry no
     # bulk payload in the reference, so their prompt length is what the verbatim prompt + question tokenise to.
     from opsagent_b200 import workloads as WL
     cli = LocalCUDAClient(eng)

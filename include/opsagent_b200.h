@@ -73,7 +73,7 @@ typedef struct {
 } oa_chat_resp;
 
 /* config_json: {"model":"llama-3-8b"|"llama-3.2-1b"|"qwen2.5-32b"|"llama-3-70b"|custom dims..., "seed":1234,
- *  "device":0, "kv_gb":100, "max_batch":128, "max_seq_len":4096, "max_step_tokens":8192, ...} — see DESIGN.md */
+ *  "device":0, "kv_gb":100, "max_batch":128, "max_seq_len":4096, "max_step_tokens":8192, ...} */
 OA_API int oa_engine_create(const char* config_json, oa_engine** out);
 OA_API void oa_engine_destroy(oa_engine*);
 /* tensor-parallel groups (config "tp": t, "tp_rank": r, "tp_shm": name; one process per GPU): rank 0 is the engine callers talk
@@ -108,7 +108,7 @@ OA_API int oa_model_info(oa_engine*, char* buf, size_t n);   /* JSON: resolved a
 /* ---- native OpenAI-compatible HTTP front (csrc/http_server.cpp): what the UNMODIFIED reference binary is pointed at (`baseUrl` of POST /api/execute,
  * pkg/handlers/execute.go:21,205; OPENAI_API_BASE for the swarm flows, pkg/workflows/swarm.go:83).  POST /v1/chat/completions in go-openai's wire
  * format (openai.go:70-82) incl. `tools` -> grammar-forced `tool_calls`, GET /v1/models, GET /api/perf/stats.  One OS thread per connection; with
- * n_engines > 1 (data-parallel replicas, BASELINE configs[2]) conversations stick to the replica holding their prefix pages, new ones go to the
+ * n_engines > 1 (data-parallel replicas) conversations stick to the replica holding their prefix pages, new ones go to the
  * least-loaded replica, a replica over `max_inflight` answers 429 (openai.go:91-94 backs off).
  * options_json (flat): {"host":"127.0.0.1","port":0,"require_key":1,"api_key":"","tool_steps":3,"max_inflight":256,"max_connections":8192,"max_body_bytes":67108864,"idle_timeout_s":120} */
 typedef struct oa_http oa_http;

@@ -9,7 +9,7 @@
       Chat again; reply with final_answer -> return it; unparsable reply -> "Summarize all the chat history…" Chat (simple.go:515-600)
 
 Used by bench/tests to drive multi-step tool-calling loops through the engine; `tools` is injectable because the reference's
-pkg/tools shell out to kubectl/trivy (out of scope: SURVEY.md §2 #6)."""
+pkg/tools shell out to kubectl/trivy (out of scope here)."""
 from __future__ import annotations
 
 import json

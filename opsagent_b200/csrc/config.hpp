@@ -78,13 +78,13 @@ struct ModelConfig {
     int kv_dim() const { return n_kv_heads * head_dim; }
     int qkv_dim() const { return q_dim() + 2 * kv_dim(); }
     size_t kv_bytes_per_token() const { return (size_t)2 * n_layers * kv_dim() * 2; }
-    double decode_weight_bytes() const {   // W_dec of SURVEY.md §8d: all layers + final norm + lm_head
+    double decode_weight_bytes() const {   // all layers + final norm + lm_head
         double per = (double)qkv_dim() * hidden + (double)hidden * q_dim() + 3.0 * ffn * hidden + 2.0 * hidden + (qkv_bias ? qkv_dim() : 0);
         return 2.0 * (per * n_layers + hidden + (double)vocab * hidden);
     }
 };
 
-// public architectures (SURVEY.md §8d); oracle/oracle.py PRESETS is the test-side copy
+// public architectures; oracle/oracle.py PRESETS is the test-side copy
 inline bool preset_model(const std::string& n, ModelConfig& c) {
     c.name = n;
     if (n == "llama-3.2-1b") { c.hidden = 2048; c.n_layers = 16; c.n_heads = 32; c.n_kv_heads = 8; c.head_dim = 64; c.ffn = 8192; c.vocab = 128256; c.tie_embeddings = 1; c.rope_scaling = 1; return true; }

@@ -367,9 +367,9 @@ public:
             const double mean_ctx = ctx_sum / steps;
             out[0] = bracket_ms / steps; if (n_out > 6) out[6] = total_ms / steps; out[1] = prefill_ms; out[2] = (double)(launches1 - launches0) / steps; out[3] = mean_ctx;
             out[4] = model_.profile_attn ? model_.attn_ms_accum / steps : 0.0;
-            // W_dec + sum ctx*KVB + B*KVB (the new token's KV write)
+            // weights + sum ctx*KVB + B*KVB (the new token's KV write)
             out[5] = (model_.cfg.decode_weight_bytes() + (double)batch * mean_ctx * (double)model_.cfg.kv_bytes_per_token() +
-                      (double)batch * (double)model_.cfg.kv_bytes_per_token()) / opt_.tp;      // per GPU (W_dec/t + ctx*KVB/t)
+                      (double)batch * (double)model_.cfg.kv_bytes_per_token()) / opt_.tp;      // per GPU
         } catch (const std::exception& ex) { return fail(OA_ERR_INTERNAL, ex.what()); }
         return OA_OK;
     }

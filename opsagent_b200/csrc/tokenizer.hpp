@@ -1,6 +1,6 @@
 // tokenizer.hpp — synthetic byte-level tokenizer and chat templates.
 //
-// No tokenizer files exist offline (SURVEY.md §0-5), so text maps to ids 0..255 (one per UTF-8 byte) and
+// No tokenizer files exist offline, so text maps to ids 0..255 (one per UTF-8 byte) and
 // the chat-format control tokens keep their real ids inside the real vocabulary size.  Decode is
 // many-to-one: a non-control id t renders as byte (t & 0xFF).  With config "tokenizer": "<tokenizer.json>" text goes through the
 // checkpoint's own byte-level BPE instead (bpe.hpp) and the control ids come from its added_tokens.  The message order/roles templated here are

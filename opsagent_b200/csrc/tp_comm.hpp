@@ -1,4 +1,4 @@
-// tp_comm.hpp — tensor-parallel plumbing for models that do not fit one GPU (BASELINE configs[3,4]).
+// tp_comm.hpp — tensor-parallel plumbing for models that do not fit one GPU (Qwen2.5-32B over 4, Llama-3-70B over 8).
 //
 // One process per GPU on one NVSwitch node.  No NCCL: ranks exchange CUDA-IPC handles of *symmetric* buffers through a
 // POSIX shared-memory segment, map each other's buffers, and the row-parallel projections are all-reduced by the

@@ -8,7 +8,7 @@
 //     llms.NumTokensFromMessages / llms.ConstrictPrompt                                                   reference pkg/llms/tokens.go:60, 128-144
 // The reference is Go (no toolchain in this image), so — like localcuda_client.hpp for the seam itself — the host side above the C ABI is written in
 // C++ with the same names, argument meaning and error behaviour.  The LLM call and the tools are injected (`ChatFn`, `Tool`): the reference's
-// pkg/tools shell out to kubectl / trivy (out of scope) and its client is built from apiKey/baseUrl on every call (simple.go:316),
+// pkg/tools shell out to kubectl / trivy (out of scope here) and its client is built from apiKey/baseUrl on every call (simple.go:316),
 // which here is LocalCUDAClient::Chat bound to the process-wide engine.  opsagent_b200/assistants.py is the same loop in Python;
 // tests/test_host_cpp.py runs both on the same scripted scenarios and demands identical results and histories.
 #pragma once

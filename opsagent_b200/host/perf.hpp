@@ -1,7 +1,7 @@
 // perf.hpp — C++ host-side mirror of the reference's PerfStats (reference pkg/utils/perf.go): StartTimer / StopTimer accumulate per-operation
 // durations and call counts (perf.go:64-121), TraceFunc returns the closer (perf.go:288), GetStats returns {"timers", "callCounts", "lastResetTime"}
 // (perf.go:296-320), Reset clears them (perf.go:323-335), GetPerfStats() is the process-wide instance (perf.go:38-47).  Two deliberate differences
-// (same as opsagent_b200/perf.py): running timers are keyed per (thread, operation), so concurrent requests do not overwrite each
+// (as opsagent_b200/perf.py): running timers are keyed per (thread, operation), so concurrent requests do not overwrite each
 // other's start time (the reference keeps ONE start time per operation name), and durations are integer nanoseconds — what Go's time.Duration
 // marshals to in the /api/perf/stats JSON (pkg/handlers/perf.go:12-25).
 #pragma once

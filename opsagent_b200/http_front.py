@@ -1,4 +1,4 @@
-"""http_front — OpenAI-compatible /v1/chat/completions in front of the engine (SURVEY.md §8f-1).
+"""http_front — OpenAI-compatible /v1/chat/completions in front of the engine.
 
 Lets the UNMODIFIED reference binary use the engine through its existing knobs: `baseUrl` in POST /api/execute
 (reference pkg/handlers/execute.go:21,205) or OPENAI_API_BASE for the swarm flows (pkg/workflows/swarm.go:83).
@@ -154,9 +154,9 @@ def make_handler(engine, require_key: bool = True, tool_steps: int = 3, api_key:
 
 def serve(engine, host: str = "127.0.0.1", port: int = 8000, require_key: bool = True, tool_steps: int = 3, api_key: str | None = None):
     """-> (server, thread).  One OS thread per in-flight request, each blocking in the engine — the same concurrency shape as
-    gin's goroutine-per-request (SURVEY.md §8b); batching happens inside the engine."""
+    gin's goroutine-per-request; batching happens inside the engine."""
     class Server(ThreadingHTTPServer):
-        request_queue_size = 4096          # hundreds of agents connect at once (BASELINE configs[2]: 1024 concurrent requests); the default backlog is 5
+        request_queue_size = 4096          # hundreds of agents connect at once (1024 concurrent requests over eight replicas); the default backlog is 5
     srv = Server((host, port), make_handler(engine, require_key, tool_steps, api_key))
     srv.daemon_threads = True
     th = threading.Thread(target=srv.serve_forever, daemon=True)

@@ -1,5 +1,5 @@
 """native_front — the C++ OpenAI-compatible HTTP front (csrc/http_server.cpp) from Python: `NativeFront(engines, ...)` starts it on the engines of
-this process (one: a single GPU; several: the data-parallel router of BASELINE configs[2] — sticky least-loaded routing inside the server) and
+this process (one: a single GPU; several: the data-parallel router — sticky least-loaded routing inside the server) and
 `.port` / `.stats()` / `.shutdown()` manage it.  Same wire behaviour as http_front.py, no interpreter between the socket and the engines."""
 from __future__ import annotations
 

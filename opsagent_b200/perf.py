@@ -1,8 +1,8 @@
-"""perf — the reference's PerfStats surface for the local engine (SURVEY.md §8f-4).
+"""perf — the reference's PerfStats surface for the local engine.
 
 Mirrors reference pkg/utils/perf.go: StartTimer/StopTimer accumulate per-operation durations and call counts
 (perf.go:64-121), TraceFunc returns the closer (perf.go:288), GetStats returns {"timers", "callCounts", "lastResetTime"}
-(perf.go:296-320) and Reset clears them (perf.go:323-335).  Two deliberate differences, both called out in SURVEY.md §5.1:
+(perf.go:296-320) and Reset clears them (perf.go:323-335).  Two deliberate differences, both deliberate:
 timers are keyed per (thread, operation) while running, so concurrent requests do not overwrite each other's start time
 (the reference keeps ONE start time per operation name: perf.go:64-80), and durations are integer nanoseconds — what Go's
 time.Duration marshals to in the /api/perf/stats JSON (pkg/handlers/perf.go:12-25)."""

@@ -1,7 +1,7 @@
 """router — the data-parallel front: ONE process that owns N engines (one per GPU) and routes live requests to them.
 
 The reference serves every request from one process (pkg/api/router.go:95 — gin, one goroutine per request); with the model replicated
-on N GPUs (BASELINE configs[2]) that one front has to spread independent requests over N engines with no data-path collective:
+on N GPUs that one front has to spread independent requests over N engines with no data-path collective:
 
   * sticky per conversation — the ReAct loop resends its whole history on every step (pkg/assistants/simple.go:498-501), so a
     conversation is keyed by its first two messages (system prompt + first user turn) and always goes to the replica that already holds

@@ -5,7 +5,7 @@
         --devices 0,1,2,3 --port 8000 --json-mode
     python -m opsagent_b200.serve --model-dir /ckpt/zurevik-small --tokenizer /ckpt/.../tokenizer.json      # a hybrid-family checkpoint folder
 
-One engine per device (data-parallel replicas behind one endpoint, BASELINE configs[2]); `--engine '{"kv_gb": 100, ...}'` passes any other engine
+One engine per device (data-parallel replicas behind one endpoint); `--engine '{"kv_gb": 100, ...}'` passes any other engine
 option.  Fails loudly if the CUDA library or a GPU is missing — there is no CPU path."""
 from __future__ import annotations
 

@@ -1,5 +1,5 @@
 """synthetic — seeded stand-ins for what the reference shells out to (kubectl/trivy via bash, pkg/tools/*.go) so that ReAct loops can
-run on-box without a cluster: BASELINE.json configs describe 'synthetic Pod YAML', 'kubectl tool-calls' and 'synthetic trivy-scan
+run on-box without a cluster: the benchmarked workloads describe 'synthetic Pod YAML', 'kubectl tool-calls' and 'synthetic trivy-scan
 observations'.  Not on the hot path; used by bench.py / tests as the `tools` argument of assistants.AssistantWithConfig."""
 from __future__ import annotations
 

@@ -13,7 +13,7 @@ message = `System`, user message = `Instructions` followed by the step inputs as
 reference's, the joining punctuation is ours.
 
 Synthetic payloads (Pod manifests, kubectl tables, trivy reports) are seeded and process-independent; `fit_to_tokens` pads or trims a
-payload so that a request has an exact prompt-token count under the ENGINE's tokenizer (BASELINE configs quote P per class)."""
+payload so that a request has an exact prompt-token count under the ENGINE's tokenizer (the workloads quote P per class)."""
 from __future__ import annotations
 
 import os
@@ -120,7 +120,7 @@ def fit_to_tokens(build, payload: str, target: int, count_tokens, filler: str = 
 
 
 def mixed_request(i: int, count_tokens, p_analyze: int = 1536, p_diagnose: int = 0, p_execute: int = 0, seed: int = 42):
-    """request i of BASELINE configs[2]'s mix: 40 % analyze / 30 % diagnose / 30 % execute.  -> (kind, messages).
+    """request i of the data-parallel mix: 40 % analyze / 30 % diagnose / 30 % execute.  -> (kind, messages).
     analyze requests are padded with Pod YAML to p_analyze tokens; diagnose / execute carry no bulk payload in the reference, so their
     prompt length is whatever the verbatim prompt + the question tokenises to (p_* = 0), or padded with a trailing comment if p_* > 0."""
     r = random.Random(seed * 7919 + i)

@@ -7,7 +7,7 @@
  * PARITY UNPINNED BY THE REFERENCE: myysophia/OpsAgent contains no model arithmetic at all.  Its
  * "LLM path" is llms.OpenAIClient.Chat (reference pkg/llms/openai.go:69-104), an HTTP call to
  * whichever OpenAI-compatible server the operator runs; no test, fixture or golden vector in the
- * reference constrains logits or token ids (SURVEY.md §8c).  The arithmetic restated here is
+ * reference constrains logits or token ids.  The arithmetic restated here is
  * therefore the published Llama-3 / Qwen2.5 decoder definition, and it is pinned against an
  * independent implementation instead: HF transformers 5.5 LlamaForCausalLM / Qwen2ForCausalLM in
  * fp32 on CPU (tests/golden/gen_golden_hf.py writes the fixtures, tests/test_oracle_golden.py

@@ -91,7 +91,7 @@ def lib():
 
 
 # ------------------------------------------------------------------------------------------------
-# Model presets — public architectures (SURVEY.md §8d).  The engine's csrc/model_config.cpp holds
+# Model presets — public architectures.  The engine's csrc/model_config.cpp holds
 # the same table; tests/test_host_logic.py checks they agree through oa_model_info().
 # ------------------------------------------------------------------------------------------------
 @dataclass
@@ -237,7 +237,7 @@ class Oracle:
 
 # ------------------------------------------------------------------------------------------------
 # Synthetic byte-level tokenizer + chat templates (restated; the product's is csrc/tokenizer.cpp).
-# No tokenizer files exist offline (SURVEY.md §0-5), so text maps to ids 0..255 (one per UTF-8
+# No tokenizer files exist offline, so text maps to ids 0..255 (one per UTF-8
 # byte) and the chat-format control tokens keep their real ids inside the real vocab size.
 # ------------------------------------------------------------------------------------------------
 LLAMA3_SPECIALS = {"<|begin_of_text|>": 128000, "<|end_of_text|>": 128001, "<|start_header_id|>": 128006,

@@ -4,7 +4,7 @@ ByteLevel pre-tokenizer, ignore_merges, the five control tokens) with an 8,192-e
 OpsAgent actually sends — the reference's system prompts (tests/golden/prompts/*.txt), synthetic Pod manifests, kubectl tables, trivy
 reports and ToolPrompt JSON.  No checkpoint tokenizer exists offline; with this one the verbatim prompts cost about as many tokens as
 they would with a real Llama-3 vocabulary (analysisPrompt ~450, executeSystemPrompt_cn ~1,100 — the byte-level synthetic vocabulary
-needs 1,965 / 3,233), so BASELINE's prompt lengths (P = 1536 / 1024 / 1280) hold the reference's real text.
+needs 1,965 / 3,233), so the workloads' prompt lengths (P = 1536 / 1024 / 1280) hold the reference's real text.
 
     python tests/golden/gen_k8s_bpe.py     ->  tests/golden/bpe_k8s_8k.json   (needs the `tokenizers` library; the engine itself reads
                                                the JSON with its own C++ implementation, opsagent_b200/csrc/bpe.hpp)"""

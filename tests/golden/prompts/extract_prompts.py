@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Extracts the reference's system prompts VERBATIM into fixtures (contract text, SURVEY.md §8c: "the system prompts verbatim").
+"""Extracts the reference's system prompts VERBATIM into fixtures (contract text: "the system prompts verbatim").
 
 These strings are the bytes the reference feeds the Chat seam on every request, so tests and bench.py must tokenise exactly
 them, not a paraphrase.  Run in the build container (reads /root/reference, which does not exist on the GPU box):

@@ -1,4 +1,4 @@
-// Race / memory-error harness for the native HTTP front (SURVEY.md 5.2): csrc/http_server.cpp compiled together with a STUB engine (no CUDA) under
+// Race / memory-error harness for the native HTTP front: csrc/http_server.cpp compiled together with a STUB engine (no CUDA) under
 // -fsanitize=thread or -fsanitize=address,undefined, hammered by concurrent in-process HTTP clients — well-formed chats, function calls, bad JSON,
 // clients that hang up mid-request — then stopped while connections are still open.  tests/test_native_front.py builds and runs it; exit 0 = the
 // wire checks passed and the sanitizer reported nothing (TSAN exits 66, ASAN aborts).

@@ -1,4 +1,4 @@
-// ASAN + UBSAN pass over the host-only pieces of the engine that parse UNTRUSTED bytes (SURVEY.md 5.2): request text -> BPE, tokenizer.json and
+// ASAN + UBSAN pass over the host-only pieces of the engine that parse UNTRUSTED bytes: request text -> BPE, tokenizer.json and
 // config JSON readers, the safetensors header reader, the ToolPrompt byte automaton and its token masks.  Seeded mutations of valid inputs; every
 // input must end in a result or a C++ exception, never in a sanitizer report.  argv: <tokenizer.json> <scratch dir> [iterations]
 #include <cstdio>

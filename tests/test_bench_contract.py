@@ -24,7 +24,7 @@ def check_base(line):
     for k, t in BASE_KEYS.items():
         assert k in line, k
         assert isinstance(line[k], t), (k, type(line[k]))
-    assert "vs_baseline" in line and line["vs_baseline"] is None          # BASELINE.md publishes no number for this metric
+    assert "vs_baseline" in line and line["vs_baseline"] is None          # the reference publishes no number for this metric
     assert "workload" in line["config"] and "model" not in line["config"]
     for k in ("value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step"):
         assert k in line["e2e"], k
@@ -39,7 +39,7 @@ def test_our_arm_line(name):
     if "dp" in name:
         line["cpu_baseline"] = load("r01h_bench.json")["cpu_baseline"]   # the CPU leg runs at N=1 only
     if name.startswith("r02"):
-        # round 2: the reference's own request shapes, the multi-step loop and (N >= 2) the served mix + tensor parallelism are inside the contract
+        # the reference's own request shapes, the multi-step loop and (N >= 2) the served mix + tensor parallelism are inside the contract
         assert "verbatim" in line["e2e"]["prompts"] and set(line["e2e"]["prompt_tokens_by_kind"]) <= {"analyze", "diagnose", "execute"}
         r = line["react"]
         assert r["conversations_with_final_answer"] == r["conversations"] and 0 < r["prefix_hit_rate"] < 1 and r["react_steps_per_sec"] > 0

@@ -335,7 +335,7 @@ def test_prefix_cache_reuses_history_pages_without_changing_results():
     eng.close(); orc.close()
 
 
-# ---- full-size parity: the models BASELINE.json names, same seeded weights on both sides --------------------------------------
+# ---- full-size parity: the benchmarked models, same seeded weights on both sides --------------------------------------
 def _bpe_template_ids(tokenizer_json, msgs):
     """llama3 chat template over a byte-level BPE, built with the Hugging Face `tokenizers` library itself (independent of csrc/bpe.hpp)"""
     tokenizers = pytest.importorskip("tokenizers")
@@ -406,7 +406,7 @@ K8S_BPE = os.path.join(os.path.dirname(os.path.abspath(__file__)), "golden", "bp
 
 
 def test_full_size_llama_3_2_1b_execute_prompt_matches_oracle():
-    """BASELINE configs[0]: the single `execute` question of the reference's README (README.md:247) exactly as POST /api/execute builds it
+    """the single `execute` question of the reference's README (README.md:247) exactly as POST /api/execute builds it
     (pkg/handlers/execute.go:190-199: system = executeSystemPrompt_cn VERBATIM, user = the cleaned instructions) on Llama-3.2-1B (tied
     embeddings, llama3 RoPE scaling, head_dim 64), tokenised by a real byte-level BPE; logits of every prompt position and 32 greedy tokens."""
     from opsagent_b200 import workloads as WL
@@ -416,9 +416,9 @@ def test_full_size_llama_3_2_1b_execute_prompt_matches_oracle():
 
 
 def test_full_size_llama_3_8b_matches_oracle():
-    """the bench model itself (BASELINE configs[1]) on the bench's own request: the analyze flow's verbatim prompt + a synthetic Pod
+    """the bench model itself on the bench's own request: the analyze flow's verbatim prompt + a synthetic Pod
     manifest padded to P = 1536 tokens; fp32 logits at early, middle and the last prompt positions (RoPE phase and pages past position
-    1,500) and 32 greedy tokens vs the CPU oracle.  Short prompt first (every position), as in round 1."""
+    1,500) and 32 greedy tokens vs the CPU oracle.  Short prompt first (every position)."""
     from opsagent_b200 import workloads as WL
     msgs = [("user", "why is pod web-0 in CrashLoopBackOff?")]
     short = _full_size_parity("llama-3-8b", msgs, 6, 64)

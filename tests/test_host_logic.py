@@ -58,7 +58,7 @@ def test_real_special_token_ids():
 
 @pytest.mark.parametrize("name", ["llama-3.2-1b", "llama-3-8b", "qwen2.5-32b", "llama-3-70b"])
 def test_presets_agree_with_survey_table(name):
-    """SURVEY.md §8d model constants: W_dec GB and KV bytes/token"""
+    """model constants: W_dec GB and KV bytes/token"""
     L = _lib.load()
     buf = C.create_string_buffer(2048)
     assert L.oa_host_model_info(json.dumps({"model": name}).encode(), buf, 2048) == 0
@@ -388,7 +388,7 @@ def test_http_front_speaks_the_wire_format_go_openai_expects():
     srv.shutdown()
 
 
-# ---- PerfStats mirror + /api/perf/stats bridge (reference pkg/utils/perf.go, pkg/handlers/perf.go; SURVEY.md §8f-4) ----
+# ---- PerfStats mirror + /api/perf/stats bridge (reference pkg/utils/perf.go, pkg/handlers/perf.go) ----
 def test_perf_stats_mirror_accumulates_counts_and_is_request_safe():
     import threading
     from opsagent_b200.perf import PerfStats
@@ -502,7 +502,7 @@ PROMPTS_DIR = os.path.join(os.path.dirname(os.path.abspath(__file__)), "golden",
 
 
 def test_prompt_fixtures_are_the_reference_constants_verbatim():
-    """byte lengths are the ones SURVEY.md §8a measured (3,233 / 3,109 / 1,965 / 2,164 B); sha256 pins every byte; when the reference
+    """byte lengths are the reference's (3,233 / 3,109 / 1,965 / 2,164 B); sha256 pins every byte; when the reference
     tree is present (build container) the fixtures are re-extracted and compared"""
     idx = json.load(open(os.path.join(PROMPTS_DIR, "index.json")))
     want = {"executeSystemPrompt_cn": 3233, "diagnoseSystemPrompt": 3109, "analysisPrompt": 1965, "auditPrompt": 2164}

@@ -1,6 +1,6 @@
 """Pins the CPU oracle (oracle/llama_ref.c) against the committed HF-transformers fp32 fixtures
 (tests/golden/hf_*.npz, written by tests/golden/gen_golden_hf.py).  The reference holds no golden
-vectors for this path (SURVEY.md §8c) — these are the pin."""
+vectors for this path — these are the pin."""
 import os
 
 import numpy as np

@@ -1,4 +1,4 @@
-"""ReAct-loop benchmark (BASELINE configs[1]/[2] style, multi-step): N concurrent agent conversations, each driven by the mirror of the
+"""ReAct-loop benchmark (multi-step): N concurrent agent conversations, each driven by the mirror of the
 reference's loop (opsagent_b200.assistants.AssistantWithConfig <-> pkg/assistants/simple.go:292) through LocalCUDAClient.Chat, with the
 engine in json_mode (grammar-forced tools.ToolPrompt output) so that every reply parses and the loop really iterates:
 `tool_steps` tool calls answered by a synthetic kubectl, then a final answer.  Reports ReAct steps/s = completed Chat calls per second.

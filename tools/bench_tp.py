@@ -1,5 +1,5 @@
-"""Tensor-parallel decode benchmark for BASELINE configs[3] (Qwen2.5-32B TP=4, B=256, ctx 2048) and configs[4]
-(Llama-3-70B TP=8, B=64, ctx ~16.9k).  Run under torchrun with --nproc-per-node T; rank 0 prints one JSON line.
+"""Tensor-parallel decode benchmark: Qwen2.5-32B TP=4 (B=256, ctx 2048) and Llama-3-70B
+TP=8 (B=64, ctx ~16.9k).  Run under torchrun with --nproc-per-node T; rank 0 prints one JSON line.
     python -m torch.distributed.run --nproc-per-node 4 tools/bench_tp.py --model qwen2.5-32b --batch 256 --ctx 2048
 """
 import argparse

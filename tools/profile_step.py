@@ -1,4 +1,4 @@
-"""Runs the BASELINE configs[1] decode workload (Llama-3-8B, B=128, ctx~1664) for a few steps so that ncu can
+"""Runs decode steps of Llama-3-8B (B=128, ctx~1664) for a few steps so that ncu can
 capture exactly the timed decode steps:  OA_CUDA_PROFILER=1 ncu --profile-from-start off ... python tools/profile_step.py"""
 import argparse
 import json

@@ -20,7 +20,7 @@ def launches(src, dst, n_steps=2, cmd=None):
         a = agg.setdefault(key, [0, 0.0]); a[0] += 1; a[1] += v
     tot = sum(v[1] for v in agg.values())
     with open(dst, "w") as f:
-        f.write(f"# ncu launch list — decode steps of BASELINE configs[1] (Llama-3-8B, B=128, ctx~1664), {n_steps} steps\n\n")
+        f.write(f"# ncu launch list — decode steps of Llama-3-8B, B=128, ctx~1664, {n_steps} steps\n\n")
         f.write("`" + (cmd or "OA_CUDA_PROFILER=1 ncu --profile-from-start off --metrics gpu__time_duration.sum --clock-control none python tools/profile_step.py --steps 2") + "`\n\n")
         f.write(f"Per-launch times are cold-cache and serialised (compare SHARES).  Sum = {tot / n_steps / 1e3:.3f} ms per step.\n\n")
         f.write("| kernel | grid | launches/step | avg us | share |\n|---|---|---:|---:|---:|\n")
@@ -42,7 +42,7 @@ def report(src, dst):
     hdr, units = rows[0], rows[1]
     idx = {h: i for i, h in enumerate(hdr)}
     with open(dst, "w") as f:
-        f.write(f"# ncu --set full captures ({src.split('/')[-1]}; decode step of BASELINE configs[1])\n\n")
+        f.write(f"# ncu --set full captures ({src.split('/')[-1]}; Llama-3-8B decode step, B=128)\n\n")
         for r in rows[2:]:
             name = re.sub(r"\(.*", "", r[idx["Kernel Name"]]).replace("void ", "")
             f.write(f"## `{name}`  grid {r[idx['Grid Size']]} block {r[idx['Block Size']]}\n\n| metric | value | unit |\n|---|---:|---|\n")
