@@ -179,6 +179,8 @@ OA_API int oa_host_streamk_plan(int32_t N, int32_t K, int32_t block_n, int32_t n
  * vocabulary head.  few_rows: the caller's A map may have the narrower box (the entry points above and the hybrid models); grouped: a row tile's weights
  * come from a table */
 OA_API int oa_host_gemm_kernel(int32_t M, int32_t N, int32_t K, int32_t epilogue, int32_t block_n, int32_t few_rows, int32_t grouped);
+/* columns of the tiles the CTA-pair kernel takes for that product (128, 160, .. 256), 0 where another kernel runs it */
+OA_API int oa_host_gemm_pair_width(int32_t M, int32_t N, int32_t K, int32_t epilogue, int32_t block_n);
 /* byte-level BPE tokenizer read from a Hugging Face tokenizer.json (Llama-3 / Qwen2.5 format), host only: what the engine uses
  * for text when its config names one ("tokenizer": path) instead of the synthetic byte-level vocabulary.  Loaded files are cached
  * by path.  encode: *n_out = number of ids (written up to cap; OA_ERR_BAD_REQUEST if cap is too small or the file is unsupported);

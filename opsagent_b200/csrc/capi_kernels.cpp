@@ -164,6 +164,11 @@ int oa_host_gemm_kernel(int32_t M, int32_t N, int32_t K, int32_t epilogue, int32
     return (int)gemm_kernel_of(p, epilogue, block_n);
 }
 
+int oa_host_gemm_pair_width(int32_t M, int32_t N, int32_t K, int32_t epilogue, int32_t block_n) {
+    GemmParams p{}; p.M = M; p.N = N; p.K = K;
+    return gemm_kernel_of(p, epilogue, block_n) == GEMM_PAIR ? 2 * gemm_b_box(p, epilogue, block_n) : 0;
+}
+
 static int paged_attention(const void* q, void* out, const void* kv_cache, int32_t num_pages, const int32_t* block_tables,
                            int32_t max_pages_per_seq, const int32_t* ctx_lens, const int32_t* q_lens, int32_t n_seqs,
                            int32_t n_heads, int32_t n_kv, int32_t head_dim, int32_t force_splits, void* stream) {

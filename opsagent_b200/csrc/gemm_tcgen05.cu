@@ -360,30 +360,44 @@ static int sm_count_cached();
 template <int EPI>
 static cudaError_t launch_persistent(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, cudaStream_t stream);
 
-// CTA-pair kernel or one of the kernels here: the least estimate of rounds x k blocks x time of a k block plus what a launch costs besides.  Constants in
-// us fitted to a sweep of 200 .. 8192 rows over the projections of the four model sizes: a k block takes 0.345 in a pair (0.39 once more than two rounds
-// run against the power cap), 0.42 in a 128 x 256 tile and 0.26 in a narrower one; outside the k loop 11 and 8.  E.g. 200 x 4096 x 4096: 64 tiles of 128
-// x 64 24 us, 16 pair tiles 32.  Up to 128 rows half of a pair's rows would be padding.  Every kernel sums k in the same order: the choice moves no bit.
+// CTA pairs (and how wide a tile) or one of the kernels here: the least estimate of rounds x k blocks x time of a k block plus what a launch costs
+// besides.  A k block of a pair's 256 x bn tile takes bn / 256 x (0.28 + 0.14 x busy) + 0.02 us, busy the share of the pairs' rounds that have a tile: the
+// more of the chip multiplies, the lower the clock the 1000 W cap leaves.  Fitted to 21 products of 142 .. 7204 rows over the projections of the four model
+// sizes, timed in loops at all five widths: the rule takes the fastest of the eight forms timed but for 1 to 2 % (widths in us, 256 224 192 160 128): 372 x 4096 x 14336
+// 76 71 67 62 57, 1334 x 5120 x 27648 363 347 401 372 412, 2029 x 7168 x 5120 132 126 128 123 132, 5968 x 28672 x 4096 1070 1077 1094 1110 1161.  A tile of one CTA:
+// 128 x 256 0.22 + 0.27 x busy (354 x 57344 x 8192: 353 us, three row tiles instead of two of 256 rows: 384 on pairs), 128 x 128 0.17 + 0.13 x busy, narrower
+// 0.15 + 0.07 x busy.  Up to 128 rows half of a pair's rows would be padding.  Every kernel sums k in the same order: the choice moves no bit.
+struct PairWidth { int bn; double us; };
+static long long ceil_div(long long a, long long b) { return (a + b - 1) / b; }
+static PairWidth gemm_pair_width(const GemmParams& p, int sms) {
+    const long long pairs = sms / 2, kb = ceil_div(p.K, BLOCK_K);
+    PairWidth best{0, 0.0};
+    for (int bn = 256; bn >= 128; bn -= 32) {
+        const long long tiles = ceil_div(p.N, bn) * ceil_div(p.M, 256), rounds = ceil_div(tiles, pairs);
+        const double us = (double)(rounds * kb) * (bn / 256.0 * (0.28 + 0.14 * (double)tiles / (double)(rounds * pairs)) + 0.02) + 8.5;
+        if (!best.bn || us < best.us) best = PairWidth{bn, us};
+    }
+    return best;
+}
 GemmKernel gemm_kernel_of(const GemmParams& p, int epilogue, int block_n) {
     if (block_n != 32 && block_n != 64 && block_n != 128 && block_n != 256) return GEMM_NONE;
     if (p.M <= 0 || p.N <= 0 || p.K <= 0 || (p.N % 8) != 0 || (p.K % 8) != 0) return GEMM_NONE;
     if (epilogue == EPI_SWIGLU && (p.N % 32) != 0) return GEMM_NONE;
-    auto up = [](long long a, long long b) { return (a + b - 1) / b; };
-    const int sms = sm_count_cached(), pairs = sms / 2;
+    const int sms = sm_count_cached();
     if (epilogue == EPI_LOGITS) return block_n == HEAD_BN && head_persistent(p.M, p.N) ? GEMM_HEAD : GEMM_TILE;
     // the threshold of the 128 x 256 kernel, where it is set: that kernel and plain tiles are all there is then
     const char* forced = std::getenv("OA_GEMM_PERSISTENT_MIN_TILES");
     if (!forced && p.few_rows_ok && p.M <= FEW_MAX_ROWS && !p.m_tile_group) return GEMM_FEW;
     if (persistent_disabled()) return GEMM_TILE;
-    if (!forced && !p.m_tile_group && p.glu_limit <= 0.f && p.M > BLOCK_M && pairs > 0) {
-        const double kb = (double)up(p.K, BLOCK_K);
-        const double single = (double)up(up(p.N, block_n) * up(p.M, BLOCK_M), sms) * kb * (block_n >= 256 ? 0.42 : 0.26) + 8.0;
-        const double rounds = (double)up(up(p.N, 256) * up(p.M, 256), pairs), pair = rounds * kb * (rounds > 2 ? 0.39 : 0.345) + 11.0;
-        if (pair < single) return GEMM_PAIR;
+    if (!forced && !p.m_tile_group && p.glu_limit <= 0.f && p.M > BLOCK_M && sms >= 2) {
+        const long long tiles = ceil_div(p.N, block_n) * ceil_div(p.M, BLOCK_M), rounds = ceil_div(tiles, sms);
+        const double busy = (double)tiles / (double)(rounds * sms);
+        const double per_kb = block_n >= 256 ? 0.22 + 0.27 * busy : block_n == 128 ? 0.17 + 0.13 * busy : 0.15 + 0.07 * busy;
+        if (gemm_pair_width(p, sms).us < (double)(rounds * ceil_div(p.K, BLOCK_K)) * per_kb + (block_n >= 256 ? 10.0 : 7.0)) return GEMM_PAIR;
     }
-    return block_n == 256 && up(p.N, 256) * up(p.M, BLOCK_M) >= (forced ? std::atoll(forced) : 2LL * sms) ? GEMM_PERSISTENT : GEMM_TILE;
+    return block_n == 256 && ceil_div(p.N, 256) * ceil_div(p.M, BLOCK_M) >= (forced ? std::atoll(forced) : 2LL * sms) ? GEMM_PERSISTENT : GEMM_TILE;
 }
-int gemm_b_box(const GemmParams& p, int epilogue, int block_n) { return gemm_kernel_of(p, epilogue, block_n) == GEMM_PAIR ? 128 : block_n; }
+int gemm_b_box(const GemmParams& p, int epilogue, int block_n) { return gemm_kernel_of(p, epilogue, block_n) == GEMM_PAIR ? gemm_pair_width(p, sm_count_cached()).bn / 2 : block_n; }
 int gemm_a_box(const GemmParams& p, int epilogue, int block_n) { return gemm_kernel_of(p, epilogue, block_n) == GEMM_FEW ? few_box(p.M) : 128; }
 
 cudaError_t launch_gemm(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epilogue, int block_n,
@@ -393,7 +407,7 @@ cudaError_t launch_gemm(const CUtensorMap* tmA, const CUtensorMap* tmB, const Ge
     switch (kernel) {
         case GEMM_NONE: return cudaErrorInvalidValue;
         case GEMM_HEAD: return launch_head(tmA, tmB, p, stream);
-        case GEMM_PAIR: return launch_gemm_pair(tmA, tmB, p, epilogue, sm_count_cached(), stream);
+        case GEMM_PAIR: return launch_gemm_pair(tmA, tmB, p, epilogue, gemm_pair_width(p, sm_count_cached()).bn, sm_count_cached(), stream);
         case GEMM_PERSISTENT:      // the widest tile over many rows: the epilogue overlaps the next tile
             switch (epilogue) {
                 case EPI_STORE: return launch_persistent<EPI_STORE>(tmA, tmB, p, stream);

@@ -54,9 +54,9 @@ HybridModel::Mat HybridModel::upload_mat(const HostMat& m) {
     for (int r = 0; r < m.N; ++r) std::memcpy(&padded[(size_t)r * d.ld], &m.v[(size_t)r * m.K], (size_t)m.K * 4);
     d.p = upload_act(padded);
     if (!f32_ && opt.hy_tensor_core) {
-        const int bns[4] = {32, 64, 128, 256}; d.tc = true;
-        for (int i = 0; i < 4; ++i)
-            if (make_tmap_bf16_2d(&d.tm[i], d.p, (uint64_t)up8(m.N), (uint64_t)d.ld, (uint64_t)d.ld, (uint32_t)bns[i], 64) != 0) d.tc = false;
+        d.tc = true;
+        for (int i = 0; i < GEMM_N_B_BOXES; ++i)
+            if (make_tmap_bf16_2d(&d.tm[i], d.p, (uint64_t)up8(m.N), (uint64_t)d.ld, (uint64_t)d.ld, (uint32_t)GEMM_B_BOXES[i], 64) != 0) d.tc = false;
     }
     return d;
 }
@@ -352,13 +352,13 @@ HybridModel::HybridModel(const ModelConfig& c, const EngineOptions& o) : ModelBa
             }
             w.o = upload_mat(tensor(mx + "o", W, l.heads * l.vdim));
             if (!f32_ && opt.hy_tensor_core && l.dim % 8 == 0 && l.rot_dim % 8 == 0 && l.kv_rank % 8 == 0 && l.vdim % 8 == 0) {
-                const int bns[4] = {32, 64, 128, 256}; bool all = true;
+                bool all = true;
                 for (int h = 0; h < l.heads && all; ++h) {
                     Mat a; a.p = reinterpret_cast<char*>(w.uk_t) + (size_t)h * l.kv_rank * l.dim * 2; a.N = l.kv_rank; a.K = a.ld = l.dim; a.tc = true;
                     Mat b; b.p = reinterpret_cast<char*>(w.uv) + (size_t)h * l.vdim * l.kv_rank * 2; b.N = l.vdim; b.K = b.ld = l.kv_rank; b.tc = true;
-                    for (int i = 0; i < 4; ++i)
-                        all = all && make_tmap_bf16_2d(&a.tm[i], a.p, (uint64_t)a.N, (uint64_t)a.ld, (uint64_t)a.ld, (uint32_t)bns[i], 64) == 0 &&
-                              make_tmap_bf16_2d(&b.tm[i], b.p, (uint64_t)b.N, (uint64_t)b.ld, (uint64_t)b.ld, (uint32_t)bns[i], 64) == 0;
+                    for (int i = 0; i < GEMM_N_B_BOXES; ++i)
+                        all = all && make_tmap_bf16_2d(&a.tm[i], a.p, (uint64_t)a.N, (uint64_t)a.ld, (uint64_t)a.ld, (uint32_t)GEMM_B_BOXES[i], 64) == 0 &&
+                              make_tmap_bf16_2d(&b.tm[i], b.p, (uint64_t)b.N, (uint64_t)b.ld, (uint64_t)b.ld, (uint32_t)GEMM_B_BOXES[i], 64) == 0;
                     w.uk_heads.push_back(a); w.uv_heads.push_back(b);
                 }
                 if (!all) { w.uk_heads.clear(); w.uv_heads.clear(); }
@@ -601,7 +601,7 @@ void HybridModel::gemm(int mode, const void* A, int lda, const Mat& B, void* C, 
     if (tc && make_tmap_bf16_2d(&tmA, A, (uint64_t)M, (uint64_t)B.ld, (uint64_t)lda, (uint32_t)gemm_a_box(g, epi, bn), 64) != 0) tc = false;
     if (!tc) { cuda_check(hy_gemm(f32_, mode, A, lda, B.p, B.ld, C, ldc, M, B.N, B.K, bias, alpha, 1, 0, 0, 0, stream, act), "gemm"); return; }
     const int box = gemm_b_box(g, epi, bn);
-    const CUtensorMap* tmB = &B.tm[box == 32 ? 0 : box == 64 ? 1 : box == 128 ? 2 : 3];
+    const CUtensorMap* tmB = &B.tm[gemm_b_box_index(box)];
     if (mode == HY_STORE) { g.out = C; g.ldo = ldc; g.bias = bias ? bias_act : nullptr; g.store_act = act.kind; g.act_col0 = act.col0; g.act_col1 = act.col1; cuda_check(launch_gemm(&tmA, tmB, g, EPI_STORE, bn, stream), "gemm (tcgen05)"); return; }
     g.f32_out = reinterpret_cast<float*>(C); g.ldf = ldc; g.f32_accumulate = mode == HY_ACC_F32; g.alpha = alpha; g.bias_f32 = bias;
     cuda_check(launch_gemm(&tmA, tmB, g, EPI_F32, bn, stream), "gemm (tcgen05, fp32 out)");
@@ -617,7 +617,7 @@ bool HybridModel::moe(const LayerW& w, const HyLayer& l, const void* h_in, const
         const int bn = pick_tile_n(T, g.N, sm_count), box = gemm_b_box(g, EPI_SWIGLU, bn);
         CUtensorMap tmA;
         if (w.up.tc && make_tmap_bf16_2d(&tmA, h_in, (uint64_t)T, (uint64_t)w.up.ld, (uint64_t)Wld_, (uint32_t)gemm_a_box(g, EPI_SWIGLU, bn), 64) == 0) {
-            cuda_check(launch_gemm(&tmA, &w.up.tm[box == 32 ? 0 : box == 64 ? 1 : box == 128 ? 2 : 3], g, EPI_SWIGLU, bn, stream), "gated feed-forward (tcgen05)");
+            cuda_check(launch_gemm(&tmA, &w.up.tm[gemm_b_box_index(box)], g, EPI_SWIGLU, bn, stream), "gated feed-forward (tcgen05)");
         } else {
             if (!glu_) throw std::runtime_error("tensor map for the feed-forward's input failed");
             gemm(HY_STORE, h_in, Wld_, w.up, glu_, ld_glu_, T, nullptr, 1.f);

@@ -29,7 +29,7 @@ public:
 private:
     struct Mat {                    // [N, ld] matrix in the activation type, ld = K rounded up to 8 (zero padded); B operand of C = A . B^T
         void* p = nullptr; int N = 0, K = 0, ld = 0;
-        bool tc = false; CUtensorMap tm[4];           // tensor-core path (bf16): B-operand maps for BLOCK_N = 32, 64, 128, 256
+        bool tc = false; CUtensorMap tm[GEMM_N_B_BOXES];      // tensor-core path (bf16): B-operand maps, boxes of GEMM_B_BOXES rows
     };
     struct HostMat { int N = 0, K = 0; std::vector<float> v; };
     struct LayerW {

@@ -57,8 +57,11 @@ int gemm_logits_bn(int M, int N, int block_n);      // EPI_LOGITS: the tile widt
 int gemm_b_box(const GemmParams& p, int epilogue, int block_n);
 // rows of the A tensor map's box that launch_gemm reads for this product: 128, or 16, 32 or 64 for a product of that few rows (only with few_rows_ok)
 int gemm_a_box(const GemmParams& p, int epilogue, int block_n);
-// CTA-pair kernel (gemm_pair.cu): tiles of 256 x 256; tmB: box {64, 128}
-cudaError_t launch_gemm_pair(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epilogue, int sms, cudaStream_t stream);
+// CTA-pair kernel (gemm_pair.cu): tiles of 256 x bn, bn = 128, 160, .. 256; tmB: box {64, bn / 2}
+cudaError_t launch_gemm_pair(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epilogue, int bn, int sms, cudaStream_t stream);
+// the box heights gemm_b_box can ask for: a weight matrix keeps one map of each
+constexpr int GEMM_B_BOXES[] = {32, 64, 80, 96, 112, 128, 256}, GEMM_N_B_BOXES = 7;
+constexpr int gemm_b_box_index(int box) { int i = 0; while (i + 1 < GEMM_N_B_BOXES && GEMM_B_BOXES[i] != box) ++i; return i; }
 // ---- stream-K variant for decode (M <= 128): persistent, one CTA per SM; work unit = (n_tile, 64-wide k block),
 // units dealt out contiguously so every SM streams the same number of weight bytes.  Each CTA writes the fp32
 // partial of every tile segment it owns to ws[slot = cta + tile][128][BN]; consumers (sk_* kernels) add a tile's

@@ -28,9 +28,8 @@ void* DeviceModel::dmalloc(size_t bytes) {
 }
 
 void DeviceModel::make_weight_maps(WeightMat& w) {
-    const int bns[4] = {32, 64, 128, 256};
-    for (int i = 0; i < 4; ++i) {
-        int r = make_tmap_bf16_2d(&w.tm[i], w.ptr, (uint64_t)w.N, (uint64_t)w.K, (uint64_t)w.K, (uint32_t)bns[i], 64);
+    for (int i = 0; i < GEMM_N_B_BOXES; ++i) {
+        int r = make_tmap_bf16_2d(&w.tm[i], w.ptr, (uint64_t)w.N, (uint64_t)w.K, (uint64_t)w.K, (uint32_t)GEMM_B_BOXES[i], 64);
         if (r != 0) throw std::runtime_error("cuTensorMapEncodeTiled failed for a weight matrix (code " + std::to_string(r) + ")");
     }
 }

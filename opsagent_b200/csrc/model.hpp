@@ -13,8 +13,8 @@ namespace oa {
 
 struct WeightMat {
     void* ptr = nullptr; int N = 0, K = 0;
-    CUtensorMap tm[4];            // B-operand maps for BLOCK_N = 32, 64, 128, 256
-    const CUtensorMap* map(int bn) const { return &tm[bn == 32 ? 0 : bn == 64 ? 1 : bn == 128 ? 2 : 3]; }
+    CUtensorMap tm[GEMM_N_B_BOXES];            // B-operand maps, boxes of GEMM_B_BOXES rows
+    const CUtensorMap* map(int box) const { return &tm[gemm_b_box_index(box)]; }
 };
 
 struct StepInput {

@@ -508,6 +508,38 @@ def test_prefill_rows_keep_their_bits_beside_others(L, N, K):
     _bits_follow_the_row(L, N, K, 1337, [(0, 1337), (0, 129), (0, 200), (100, 357), (0, 400), (700, 1314), (313, 1337)], (256, 128, 64))
 
 
+# Every width of a pair's tile: one round and several, ragged last rows and columns (N no multiple of the width, and where the gated form runs, of 64), a k
+# range shorter than the ring; the bits of one-CTA tiles.  The width a case is for is asserted.
+@pytest.mark.parametrize("M,N,K,width", [(257, 264, 2056, 128), (129, 9000, 1032, 128), (300, 5120, 4096, 160), (700, 3080, 1032, 160), (1000, 6152, 2056, 192), (513, 8192, 1032, 192),
+                                         (640, 5120, 4096, 224), (2000, 8192, 320, 224), (1000, 9000, 2056, 256), (2000, 2048, 4096, 256)])
+def test_pair_tiles_of_every_width(L, M, N, K, width):
+    assert L.oa_host_gemm_pair_width(M, N, K, EPI_STORE, 256) == width
+    g = torch.Generator(device=dev()).manual_seed(M + N + K)
+    A = torch.randn(M, K, generator=g, device=dev()).to(torch.bfloat16)
+    B = (torch.randn(N, K, generator=g, device=dev()) * 0.05).to(torch.bfloat16)
+    bias, resid = torch.randn(N, generator=g, device=dev()).to(torch.bfloat16), torch.randn(M, N, generator=g, device=dev()).to(torch.bfloat16)
+    ref = A.double() @ B.double().T
+    room = 0.05 * K ** 1.5 * 2.0 ** -24              # fp32 sums of K products; the rounding to bf16 besides
+
+    def products(a, add, bn):
+        rows = a.shape[0]
+        outs = [torch.full((rows, N), float("nan"), dtype=torch.bfloat16, device=dev()) for _ in range(2)] + [torch.full((rows, N // 2), float("nan"), dtype=torch.bfloat16, device=dev())]
+        assert L.oa_k_gemm(ptr(a), ptr(B), rows, N, K, EPI_STORE, bn, ptr(outs[0]), ptr(bias), None, None, None, None) == 0
+        assert L.oa_k_gemm(ptr(a), ptr(B), rows, N, K, EPI_RESID, bn, ptr(outs[1]), None, ptr(add), None, None, None) == 0
+        if N % 32 == 0:
+            assert L.oa_k_gemm(ptr(a), ptr(B), rows, N, K, EPI_SWIGLU, bn, ptr(outs[2]), None, None, None, None, None) == 0
+        torch.cuda.synchronize()
+        return outs[:3 if N % 32 == 0 else 2]
+
+    got = products(A, resid, 256)
+    for o, want in ((got[0], ref + bias.double()), (got[1], ref + resid.double())):
+        assert ((o.double() - want).abs() <= want.abs() * 2.0 ** -8 + room + 1e-6).all(), float((o.double() - want).abs().max())
+    for r0 in range(0, M, 128):                      # up to 128 rows take one-CTA tiles
+        part = products(A[r0:r0 + 128].contiguous(), resid[r0:r0 + 128].contiguous(), 64)
+        for o, q in zip(got, part):
+            assert torch.equal(o[r0:r0 + 128], q)
+
+
 @pytest.mark.parametrize("N,K", [(4096, 14336), (2048, 4096), (6144, 2056), (2048, 2048), (1024, 72), (28672, 1024)])
 def test_decoding_rows_keep_their_bits_beside_others(L, N, K):
     _bits_follow_the_row(L, N, K, 300, [(0, 300), (0, 1), (17, 18), (0, 16), (3, 20), (0, 32), (7, 40), (0, 64), (30, 95), (0, 128), (50, 179), (299, 300)], (32, 64, 128, 256))
