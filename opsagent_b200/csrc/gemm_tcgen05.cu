@@ -40,18 +40,21 @@ struct GemmCfg {
     static constexpr uint32_t TMEM_COLS = BN < 32 ? 32 : BN;
 };
 
-// FEW: a product of up to 64 rows loads only the 16, 32 or 64 of them (the box of tmA) and keeps more stages of the narrower ring in flight.  Its
-// products, their order and so every bit are those of the plain form: a decoding row must not feel how many requests share its step.  (Sharing a tile's k
-// range over a cluster is faster, 7.0 against 12.6 us for 16 x 2048 x 4096, and gives that up.)  What bounds it is the chain of one tile's k blocks, 0.16
-// us each at a width of 32; us, 128 rows loaded -> here: 16 x 2048 x 4096 18.6 -> 12.6, 16 x 4096 x 14336 62 -> 42, 64 x 6144 x 4096 20.8 -> 15.6.
-struct FewRing { int a_rows, stages; };
-static constexpr int FEW_MAX_ROWS = 64, FEW_BAR_BYTES = 512;
+// FEW: a product of up to 64 rows loads only the 16, 32 or 64 of them (the box of tmA) and multiplies 64-row tiles.  Its products, their order and so
+// every bit are those of the plain form: a decoding row must not feel how many requests share its step.  (Sharing a tile's k range over a cluster gives
+// that up.)  What bounds it is the chain of one tile's k blocks: a barrier's wait, arming and release take 240 cycles in the producer whatever it loads
+// (a load only 17 more), and a 128 x 32 x 16 product 40, of which 32 read A.  So a stage holds several k blocks under one barrier (98 cycles a k block
+// with four) and the tile has 64 rows (26 a product).  us, a k block a stage and 128-row tiles -> here: 16 x 2048 x 4096 12.7 -> 7.4, 16 x 4096 x 14336
+// 42 -> 24, 64 x 6144 x 4096 15.8 -> 13.8, 16 x 8192 x 2048 10.2 -> 7.8.
+struct FewRing { int a_rows, stages, kq; };       // kq: k blocks of a stage
+static constexpr int FEW_MAX_ROWS = 64, FEW_BAR_BYTES = 512, FEW_M = 64;
 static int few_box(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : 64; }
 static FewRing few_ring(int M, int N, int bn, int sms) {
-    // 130 KB in flight a CTA; with more tiles than SMs 96 KB, so that two CTAs fit one (16 x 8192 x 2048 in 256 tiles: 17.3 us alone on an SM, 10.3 in
-    // twos).  A hybrid model's step with 100, 130, 160 and 200 KB: 4517, 4390, 4401 and 4426 us a pass.
-    const int a_rows = few_box(M), stage = (a_rows + bn) * BLOCK_K * 2;
-    return FewRing{a_rows, std::max(4, std::min(28, ((N + bn - 1) / bn > sms ? 96 : 130) * 1024 / stage))};
+    // 160 KB in flight a CTA; with more tiles than SMs 96 KB, so that two CTAs fit one.  A hybrid model's pass with 64, 96, 130, 160 and 200 KB: 4100, 3929,
+    // 3871, 3835 and 3829 us; the other figure at 48, 64, 80, 96 and 104 KB: 3879, 3892, 3863, 3846 and 3912.
+    const int a_rows = few_box(M), block = (a_rows + bn) * BLOCK_K * 2, room = ((N + bn - 1) / bn > sms ? 96 : 160) * 1024;
+    const int kq = block * 4 <= 32 * 1024 ? 4 : block * 2 <= 32 * 1024 ? 2 : 1;
+    return FewRing{a_rows, std::max(kq > 1 ? 3 : 4, std::min(28, room / (block * kq))), kq};
 }
 
 // 32 columns of one row of the vocabulary head: the row's running arg-max (ties: lowest column) and, where wanted, the logits
@@ -90,18 +93,19 @@ OA_DEVINL void logits_chunk(const GemmParams& p, int row, const uint32_t (&v)[32
     }
 }
 
-template <int BN, int EPI, bool FEW>
+template <int BN, int EPI, int FEW>      // FEW: 0, or the k blocks of a stage of the few-row form
 __global__ void __launch_bounds__(GEMM_THREADS) gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
                                                                       const __grid_constant__ CUtensorMap tmB,
                                                                       const GemmParams p, const FewRing few) {
     using Cfg = GemmCfg<BN>;
-    // ring: [stage][A | B]; FEW: [stage][A], then [stage][B], A stages of the rows there are
+    // ring: [stage][A | B], a k block a stage; FEW: [stage][k block][A], then [stage][k block][B], A blocks of the rows there are
+    constexpr int KQ = FEW ? FEW : 1;
     const int STAGES = FEW ? few.stages : Cfg::STAGES, A_BYTES = FEW ? few.a_rows * BLOCK_K * 2 : Cfg::A_BYTES;
-    const int A_STRIDE = FEW ? A_BYTES : Cfg::STAGE_BYTES, B_STRIDE = FEW ? Cfg::B_BYTES : Cfg::STAGE_BYTES, B_AT = FEW ? STAGES * A_BYTES : Cfg::A_BYTES;
-    const uint32_t STAGE_TX = (uint32_t)(A_BYTES + Cfg::B_BYTES);
+    const int A_STRIDE = FEW ? KQ * A_BYTES : Cfg::STAGE_BYTES, B_STRIDE = FEW ? KQ * Cfg::B_BYTES : Cfg::STAGE_BYTES, B_AT = FEW ? STAGES * A_STRIDE : Cfg::A_BYTES;
+    const uint32_t BLOCK_TX = (uint32_t)(A_BYTES + Cfg::B_BYTES);
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * (int)STAGE_TX);
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * KQ * (int)BLOCK_TX);
     uint64_t* empty_bar = full_bar + STAGES;
     uint64_t* acc_bar = empty_bar + STAGES;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_bar + 1);
@@ -143,40 +147,54 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_tcgen05_kernel(const __grid
 
     if (warp == 0) {
         // weights (B) are written by no kernel of the chain: fill the ring with them BEFORE waiting for the predecessor
-        const int pre = num_kb < STAGES ? num_kb : STAGES;
-        for (int kb = 0; kb < pre; ++kb)
+        const int n_st = (num_kb + KQ - 1) / KQ, pre = n_st < STAGES ? n_st : STAGES;      // stages of the whole k range; the last may hold fewer blocks
+        for (int st = 0; st < pre; ++st)
             if (elect_one()) {
-                mbar_expect_tx(&full_bar[kb], STAGE_TX);
-                tma_load_2d(smem + B_AT + kb * B_STRIDE, &tmB, &full_bar[kb], kb * BLOCK_K, b_row0, kEvictFirst);
+                const int kb0 = st * KQ, n = num_kb - kb0 < KQ ? num_kb - kb0 : KQ;
+                mbar_expect_tx(&full_bar[st], n * BLOCK_TX);
+                for (int j = 0; j < KQ; ++j) if (j < n) tma_load_2d(smem + B_AT + st * B_STRIDE + j * Cfg::B_BYTES, &tmB, &full_bar[st], (kb0 + j) * BLOCK_K, b_row0, kEvictFirst);
             }
         griddep_wait();
-        for (int kb = 0; kb < pre; ++kb)
-            if (elect_one()) tma_load_2d(smem + kb * A_STRIDE, &tmA, &full_bar[kb], kb * BLOCK_K, m_blk * BLOCK_M, kEvictLast);
+        for (int st = 0; st < pre; ++st)
+            if (elect_one()) {
+                const int kb0 = st * KQ, n = num_kb - kb0 < KQ ? num_kb - kb0 : KQ;
+                for (int j = 0; j < KQ; ++j) if (j < n) tma_load_2d(smem + st * A_STRIDE + j * A_BYTES, &tmA, &full_bar[st], (kb0 + j) * BLOCK_K, m_blk * BLOCK_M, kEvictLast);
+            }
         int s = pre == STAGES ? 0 : pre; uint32_t ph = pre == STAGES ? 1 : 0;
-        for (int kb = pre; kb < num_kb; ++kb) {
+        for (int st = pre; st < n_st; ++st) {
             mbar_wait(&empty_bar[s], ph ^ 1);
             if (elect_one()) {
-                mbar_expect_tx(&full_bar[s], STAGE_TX);
-                tma_load_2d(smem + s * A_STRIDE, &tmA, &full_bar[s], kb * BLOCK_K, m_blk * BLOCK_M, kEvictLast);
-                tma_load_2d(smem + B_AT + s * B_STRIDE, &tmB, &full_bar[s], kb * BLOCK_K, b_row0, kEvictFirst);
+                const int kb0 = st * KQ, n = num_kb - kb0 < KQ ? num_kb - kb0 : KQ;
+                mbar_expect_tx(&full_bar[s], n * BLOCK_TX);
+#pragma unroll
+                for (int j = 0; j < KQ; ++j) {
+                    if (j >= n) break;
+                    tma_load_2d(smem + s * A_STRIDE + j * A_BYTES, &tmA, &full_bar[s], (kb0 + j) * BLOCK_K, m_blk * BLOCK_M, kEvictLast);
+                    tma_load_2d(smem + B_AT + s * B_STRIDE + j * Cfg::B_BYTES, &tmB, &full_bar[s], (kb0 + j) * BLOCK_K, b_row0, kEvictFirst);
+                }
             }
             __syncwarp();
             if (++s == STAGES) { s = 0; ph ^= 1; }
         }
     } else if (warp == 1) {
-        constexpr uint32_t idesc = umma_idesc_bf16(BLOCK_M, BN);
+        constexpr uint32_t idesc = umma_idesc_bf16(FEW ? FEW_M : BLOCK_M, BN);
         int s = 0; uint32_t ph = 0;
-        for (int kb = 0; kb < num_kb; ++kb) {
+        for (int kb0 = 0; kb0 < num_kb; kb0 += KQ) {
             mbar_wait(&full_bar[s], ph);
             tcgen05_fence_after();
-            // FEW: the product reads 128 rows from the start of its A stage, the rows beyond those loaded being whatever lies behind it in the ring
-            // (inside the block's shared memory: at least four B stages follow).  They are rows of the result that nobody looks at.
+            // FEW: the product reads 64 rows from the start of its A block, the rows beyond those loaded being whatever lies behind it in the ring
+            // (inside the block's shared memory: at least two B stages follow, 8 KB and more).  They are rows of the result that nobody looks at.
             const uint64_t a_desc = umma_desc_sw128(smem_u32(smem + s * A_STRIDE));
             const uint64_t b_desc = umma_desc_sw128(smem_u32(smem + B_AT + s * B_STRIDE));
             if (elect_one()) {
 #pragma unroll
-                for (int k = 0; k < BLOCK_K / UMMA_K; ++k)      // 16 bf16 = 32 B further inside the 128 B swizzle row: +2 in the (>>4) address field
-                    umma_bf16(tmem_base, a_desc + (uint64_t)(k * 2), b_desc + (uint64_t)(k * 2), idesc, (kb | k) != 0);
+                for (int j = 0; j < KQ; ++j) {
+                    if (j > 0 && kb0 + j >= num_kb) break;
+                    const uint64_t aj = a_desc + (uint64_t)(j * (A_BYTES >> 4)), bj = b_desc + (uint64_t)(j * (Cfg::B_BYTES >> 4));
+#pragma unroll
+                    for (int k = 0; k < BLOCK_K / UMMA_K; ++k)      // 16 bf16 = 32 B further inside the 128 B swizzle row: +2 in the (>>4) address field
+                        umma_bf16(tmem_base, aj + (uint64_t)(k * 2), bj + (uint64_t)(k * 2), idesc, (kb0 | j | k) != 0);
+                }
                 umma_commit(&empty_bar[s]);       // slot reusable once these MMAs have read it
             }
             __syncwarp();
@@ -187,8 +205,9 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_tcgen05_kernel(const __grid
     } else {
         // ---------------- epilogue: warps 2..5, TMEM lane group = warp % 4 ----------------
         const int q = warp & 3;
-        const int row = m_blk * BLOCK_M + q * 32 + lane;
-        const bool row_ok = row < p.M;
+        // a 64-row tile stands in lanes 0 .. 15 of each warp's 32
+        const int row = FEW ? q * 16 + lane : m_blk * BLOCK_M + q * 32 + lane;
+        const bool row_ok = row < p.M && (!FEW || lane < 16);
         griddep_wait();                   // bias/residual reads and every store below come after the predecessor grid
         mbar_wait(acc_bar, 0);
         tcgen05_fence_after();
@@ -310,14 +329,20 @@ int gemm_n_tiles(int N, int block_n) { return (N + block_n - 1) / block_n; }
 
 static int sm_count_cached();
 // few rows (tmA: a box of few_box(M) rows)
-template <int BN, int EPI>
-static cudaError_t launch_few(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, cudaStream_t stream) {
-    auto kern = gemm_tcgen05_kernel<BN, EPI, true>;
-    const FewRing few = few_ring(p.M, p.N, BN, sm_count_cached());
-    const int smem = few.stages * (few.a_rows + BN) * BLOCK_K * 2 + 1024 + FEW_BAR_BYTES;
+template <int BN, int EPI, int KQ>
+static cudaError_t launch_few_kq(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, const FewRing& few, cudaStream_t stream) {
+    auto kern = gemm_tcgen05_kernel<BN, EPI, KQ>;
+    const int smem = few.stages * few.kq * (few.a_rows + BN) * BLOCK_K * 2 + 1024 + FEW_BAR_BYTES;
     static bool attr_done[16] = {};
     { cudaError_t e = ensure_dynamic_smem(kern, 227 * 1024, attr_done); if (e != cudaSuccess) return e; }
     return launch_k(kern, dim3((p.N + BN - 1) / BN), dim3(GEMM_THREADS), smem, stream, *tmA, *tmB, p, few);
+}
+template <int BN, int EPI>
+static cudaError_t launch_few(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, cudaStream_t stream) {
+    const FewRing few = few_ring(p.M, p.N, BN, sm_count_cached());
+    if constexpr (BN <= 32) if (few.kq == 4) return launch_few_kq<BN, EPI, 4>(tmA, tmB, p, few, stream);
+    if constexpr (BN <= 64) if (few.kq == 2) return launch_few_kq<BN, EPI, 2>(tmA, tmB, p, few, stream);
+    return few.kq == 1 ? launch_few_kq<BN, EPI, 1>(tmA, tmB, p, few, stream) : cudaErrorInvalidValue;
 }
 template <int BN>
 static cudaError_t launch_few_bn(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epi, cudaStream_t s) {
@@ -333,7 +358,7 @@ static cudaError_t launch_few_bn(const CUtensorMap* tmA, const CUtensorMap* tmB,
 template <int BN, int EPI>
 static cudaError_t launch_one(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, cudaStream_t stream) {
     using Cfg = GemmCfg<BN>;
-    auto kern = gemm_tcgen05_kernel<BN, EPI, false>;
+    auto kern = gemm_tcgen05_kernel<BN, EPI, 0>;
     static bool attr_done[16] = {};
     { cudaError_t e = ensure_dynamic_smem(kern, Cfg::SMEM_BYTES, attr_done); if (e != cudaSuccess) return e; }
     dim3 grid(((p.N + BN - 1) / BN) * ((p.M + BLOCK_M - 1) / BLOCK_M), 1, 1);
@@ -397,7 +422,19 @@ GemmKernel gemm_kernel_of(const GemmParams& p, int epilogue, int block_n) {
     }
     return block_n == 256 && ceil_div(p.N, 256) * ceil_div(p.M, BLOCK_M) >= (forced ? std::atoll(forced) : 2LL * sms) ? GEMM_PERSISTENT : GEMM_TILE;
 }
-int gemm_b_box(const GemmParams& p, int epilogue, int block_n) { return gemm_kernel_of(p, epilogue, block_n) == GEMM_PAIR ? gemm_pair_width(p, sm_count_cached()).bn / 2 : block_n; }
+// The narrowest tiles give the shortest chain a k block; from more than two tiles an SM on, wider ones (each SM then walks several chains in turn).  us at
+// 32, 64 and 128 columns, 16 rows: 2048 x 4096 7.4 9.9 13.9, 8192 x 2048 7.8 8.7 10.6, 16384 x 2048 15.6 13.5 15.0, 28672 x 4096 45.0 42.3 40.3.
+static int few_width(int N, int sms) {
+    for (int bn : {32, 64}) if (ceil_div(N, bn) <= 2 * sms) return bn;
+    return 128;
+}
+int gemm_b_box(const GemmParams& p, int epilogue, int block_n) {
+    switch (gemm_kernel_of(p, epilogue, block_n)) {
+        case GEMM_PAIR: return gemm_pair_width(p, sm_count_cached()).bn / 2;
+        case GEMM_FEW: return few_width(p.N, sm_count_cached());
+        default: return block_n;
+    }
+}
 int gemm_a_box(const GemmParams& p, int epilogue, int block_n) { return gemm_kernel_of(p, epilogue, block_n) == GEMM_FEW ? few_box(p.M) : 128; }
 
 cudaError_t launch_gemm(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epilogue, int block_n,
@@ -417,14 +454,18 @@ cudaError_t launch_gemm(const CUtensorMap* tmA, const CUtensorMap* tmB, const Ge
             }
             return cudaErrorInvalidValue;
         case GEMM_FEW:
+            switch (few_width(p.N, sm_count_cached())) {
+                case 32: return launch_few_bn<32>(tmA, tmB, p, epilogue, stream);
+                case 64: return launch_few_bn<64>(tmA, tmB, p, epilogue, stream);
+                default: return launch_few_bn<128>(tmA, tmB, p, epilogue, stream);
+            }
         case GEMM_TILE: break;
     }
-    const bool few = kernel == GEMM_FEW;
     switch (block_n) {
-        case 32: return few ? launch_few_bn<32>(tmA, tmB, p, epilogue, stream) : launch_bn<32>(tmA, tmB, p, epilogue, stream);
-        case 64: return few ? launch_few_bn<64>(tmA, tmB, p, epilogue, stream) : launch_bn<64>(tmA, tmB, p, epilogue, stream);
-        case 128: return few ? launch_few_bn<128>(tmA, tmB, p, epilogue, stream) : launch_bn<128>(tmA, tmB, p, epilogue, stream);
-        case 256: return few ? launch_few_bn<256>(tmA, tmB, p, epilogue, stream) : launch_bn<256>(tmA, tmB, p, epilogue, stream);
+        case 32: return launch_bn<32>(tmA, tmB, p, epilogue, stream);
+        case 64: return launch_bn<64>(tmA, tmB, p, epilogue, stream);
+        case 128: return launch_bn<128>(tmA, tmB, p, epilogue, stream);
+        case 256: return launch_bn<256>(tmA, tmB, p, epilogue, stream);
     }
     return cudaErrorInvalidValue;
 }

@@ -424,6 +424,13 @@ def test_gemm_few_rows(L, M, N, K):
         close(y, (torch.nn.functional.silu(v[:, :, 0]) * v[:, :, 1]).reshape(M, N // 2), 2e-5 * float(v.abs().max()) ** 2)
 
 
+# a stage of the few-row form holds four k blocks (32-column tiles of up to 32 rows), two (of 64 rows; 64-column tiles) or one (128): last stages of every
+# remainder, fewer stages than the ring and more, tiles of 32, 64 and 128 columns with a ragged last one
+@pytest.mark.parametrize("M,N,K", [(16, 520, 64), (2, 2048, 4104), (31, 9472, 192), (32, 2056, 8256), (33, 2056, 4160), (64, 9472, 136), (5, 9480, 1088), (64, 12008, 1096), (17, 18944, 64), (64, 18952, 2112), (1, 57344, 264)])
+def test_few_row_stages_of_several_blocks(L, M, N, K):
+    test_gemm_few_rows(L, M, N, K)
+
+
 # persistent vocabulary head: fewer k blocks than ring stages and more, one and several row tiles, a ragged last tile, the largest in the last column
 @pytest.mark.parametrize("M,N,K", [(1, 128256, 64), (128, 38016, 200), (3, 128256, 1024), (129, 40008, 512), (64, 152064, 448)])
 def test_persistent_vocabulary_head(L, M, N, K):
