@@ -62,7 +62,7 @@ OA_DEVINL const uint32_t* logits_mask(const GemmParams& p, int row) {
     const int ms = p.mask_slot ? p.mask_slot[row] : -1;
     return ms >= 0 ? p.mask_table + (size_t)ms * p.mask_words : nullptr;
 }
-OA_DEVINL void logits_chunk(const GemmParams& p, int row, const uint32_t (&v)[32], int col0, const uint32_t* mask_row, float& best_v, int& best_i) {
+OA_DEVINL void logits_chunk(const GemmParams& p, int row, const uint32_t (&v)[32], int col0, const uint32_t* mask_row, float& best_v, int& best_i, bool store = true) {
     if (mask_row) {
         // grammar-constrained row: only token ids allowed in this sequence's automaton state compete.  The 32 columns of
         // this chunk are 32 consecutive global ids: at most two words of the bitset.
@@ -82,7 +82,7 @@ OA_DEVINL void logits_chunk(const GemmParams& p, int row, const uint32_t (&v)[32
             if (col0 + j < p.N && f > best_v) { best_v = f; best_i = col0 + j; }
         }
     }
-    if (p.logits) {
+    if (store && p.logits) {
         float* lrow = p.logits + (size_t)row * p.ldl;
 #pragma unroll
         for (int j = 0; j < 32; j += 4) {
@@ -435,7 +435,10 @@ int gemm_b_box(const GemmParams& p, int epilogue, int block_n) {
         default: return block_n;
     }
 }
-int gemm_a_box(const GemmParams& p, int epilogue, int block_n) { return gemm_kernel_of(p, epilogue, block_n) == GEMM_FEW ? few_box(p.M) : 128; }
+int gemm_a_box(const GemmParams& p, int epilogue, int block_n) {
+    const GemmKernel k = gemm_kernel_of(p, epilogue, block_n);
+    return k == GEMM_FEW || (k == GEMM_HEAD && p.few_rows_ok && p.M <= FEW_MAX_ROWS) ? few_box(p.M) : 128;
+}
 
 cudaError_t launch_gemm(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epilogue, int block_n,
                         cudaStream_t stream) {
@@ -498,7 +501,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_persistent_kernel(const 
     uint64_t* acc_empty = acc_full + 2;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // warp: uniform, and known to be
     const int n_tiles = (p.N + BN - 1) / BN;
     int m_tiles = (p.M + BLOCK_M - 1) / BLOCK_M;
     if (p.m_tile_group) {                 // grouped product: the number of live row tiles comes from the device (possibly from the preceding kernel)
@@ -519,48 +522,51 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_persistent_kernel(const 
     tcgen05_fence_before();
     __syncthreads();
     tcgen05_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     griddep_launch();
 
     if (warp == 0) {
-        if (lane == 0) {
-            griddep_wait();
-            int s = 0; uint32_t ph = 0;
-            for (int t = blockIdx.x; t < total_tiles; t += gridDim.x) {
-                int m_blk, n_blk; raster_tile(t, m_tiles, n_tiles, m_blk, n_blk);
-                const int b_row0 = n_blk * BN + (p.m_tile_group ? p.m_tile_group[m_blk] * p.group_rows : 0);
-                for (int kb = 0; kb < num_kb; ++kb) {
-                    mbar_wait(&empty_bar[s], ph ^ 1);
+        griddep_wait();
+        int s = 0; uint32_t ph = 0;
+        for (int t = blockIdx.x; t < total_tiles; t += gridDim.x) {
+            int m_blk, n_blk; raster_tile(t, m_tiles, n_tiles, m_blk, n_blk);
+            const int b_row0 = n_blk * BN + (p.m_tile_group ? p.m_tile_group[m_blk] * p.group_rows : 0);
+            for (int kb = 0; kb < num_kb; ++kb) {
+                mbar_wait(&empty_bar[s], ph ^ 1);
+                if (elect_one()) {
                     uint8_t* a_dst = smem + s * Cfg::STAGE_BYTES;
                     mbar_expect_tx(&full_bar[s], Cfg::STAGE_BYTES);
                     tma_load_2d(a_dst, &tmA, &full_bar[s], kb * BLOCK_K, m_blk * BLOCK_M, kEvictNormal);
                     tma_load_2d(a_dst + Cfg::A_BYTES, &tmB, &full_bar[s], kb * BLOCK_K, b_row0, kEvictNormal);
-                    if (++s == STAGES) { s = 0; ph ^= 1; }
                 }
+                __syncwarp();
+                if (++s == STAGES) { s = 0; ph ^= 1; }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = umma_idesc_bf16(BLOCK_M, BN);
-            int s = 0; uint32_t ph = 0; int it = 0;
-            for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++it) {
-                const int as = it & 1;
-                mbar_wait(&acc_empty[as], (((uint32_t)it >> 1) & 1) ^ 1);
+        constexpr uint32_t idesc = umma_idesc_bf16(BLOCK_M, BN);
+        int s = 0; uint32_t ph = 0; int it = 0;
+        for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++it) {
+            const int as = it & 1;
+            mbar_wait(&acc_empty[as], (((uint32_t)it >> 1) & 1) ^ 1);
+            tcgen05_fence_after();
+            const uint32_t tmem_d = tmem_base + (uint32_t)(as * BN);
+            for (int kb = 0; kb < num_kb; ++kb) {
+                mbar_wait(&full_bar[s], ph);
                 tcgen05_fence_after();
-                const uint32_t tmem_d = tmem_base + (uint32_t)(as * BN);
-                for (int kb = 0; kb < num_kb; ++kb) {
-                    mbar_wait(&full_bar[s], ph);
-                    tcgen05_fence_after();
-                    const uint32_t a_addr = smem_u32(smem + s * Cfg::STAGE_BYTES);
-                    const uint64_t a_desc = umma_desc_sw128(a_addr), b_desc = umma_desc_sw128(a_addr + Cfg::A_BYTES);
+                const uint32_t a_addr = smem_u32(smem + s * Cfg::STAGE_BYTES);
+                const uint64_t a_desc = umma_desc_sw128(a_addr), b_desc = umma_desc_sw128(a_addr + Cfg::A_BYTES);
+                if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < BLOCK_K / UMMA_K; ++k)
                         umma_bf16(tmem_d, a_desc + (uint64_t)(k * 2), b_desc + (uint64_t)(k * 2), idesc, (kb | k) != 0);
                     umma_commit(&empty_bar[s]);
-                    if (++s == STAGES) { s = 0; ph ^= 1; }
                 }
-                umma_commit(&acc_full[as]);
+                __syncwarp();
+                if (++s == STAGES) { s = 0; ph ^= 1; }
             }
+            if (elect_one()) umma_commit(&acc_full[as]);
+            __syncwarp();
         }
     } else {
         const int q = warp & 3;
@@ -591,24 +597,32 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_persistent_kernel(const 
 // vocabulary head: persistent 128 x 128 tiles, one CTA per SM, two accumulators.  The head streams its weights once (1 GB for 128 thousand tokens of
 // width 4096) and is bound by that.  One CTA per 128 x 256 tile left the last of 3.4 rounds mostly empty and paid each tile's epilogue (logits,
 // arg-max) behind its products; here 1002 tiles make 6.8 rounds and the epilogue runs under the next tile's.  128 rows, with logits: 205 -> 183 us.
+// Of up to 64 rows only those there are are loaded (boxes of 16, 32 or 64 rows, of which most lie in the tensor: a 128-row box over a handful of rows made
+// the head of one conversation slower than that of a hundred), which also leaves room for ten stages instead of six.  us a call with logits at 1, 8, 16, 64 and
+// 128 rows, before the boxes, converged warps and whole-line stores of the logits: 256 245 187 200 216; here: 183 182 184 199 210 (200 x 152064 x 5120: 440, 385).
 // =============================================================================================
 struct HeadCfg {
-    static constexpr int BN = HEAD_BN, STAGES = 6, A_BYTES = BLOCK_M * BLOCK_K * 2, B_BYTES = BN * BLOCK_K * 2, STAGE_BYTES = A_BYTES + B_BYTES;
-    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
+    static constexpr int BN = HEAD_BN, B_BYTES = BN * BLOCK_K * 2, RING_BYTES = 192 * 1024, MAX_STAGES = 10;
+    static constexpr int SMEM_BYTES = RING_BYTES + 4 * EPI_WARP_BYTES + 1024 + 256;
     static constexpr uint32_t TMEM_COLS = 2 * BN;
 };
-__global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_head_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
+__global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_head_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p, const int a_rows) {
     using Cfg = HeadCfg;
-    constexpr int BN = Cfg::BN, STAGES = Cfg::STAGES;
+    constexpr int BN = Cfg::BN;
+    // ring: [stage][A rows loaded], then [stage][B]; a product reads 128 rows from the start of its A block (see the stream-K kernel)
+    const int A_BYTES = a_rows * BLOCK_K * 2, STAGES = min(Cfg::MAX_STAGES, Cfg::RING_BYTES / (A_BYTES + Cfg::B_BYTES));
+    const uint32_t STAGE_TX = (uint32_t)(A_BYTES + Cfg::B_BYTES);
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * Cfg::STAGE_BYTES);
-    uint64_t* empty_bar = full_bar + STAGES;
-    uint64_t* acc_full = empty_bar + STAGES;
+    uint8_t* ring_b = smem + STAGES * A_BYTES;
+    float* epi_smem = reinterpret_cast<float*>(smem + Cfg::RING_BYTES);
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + Cfg::RING_BYTES + 4 * EPI_WARP_BYTES);
+    uint64_t* empty_bar = full_bar + Cfg::MAX_STAGES;
+    uint64_t* acc_full = empty_bar + Cfg::MAX_STAGES;
     uint64_t* acc_empty = acc_full + 2;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // warp: uniform, and known to be
     const int n_tiles = (p.N + BN - 1) / BN, m_tiles = (p.M + BLOCK_M - 1) / BLOCK_M, total_tiles = n_tiles * m_tiles;
     const int num_kb = (p.K + BLOCK_K - 1) / BLOCK_K;
 
@@ -622,59 +636,63 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_head_kernel(const __grid
     tcgen05_fence_before();
     __syncthreads();
     tcgen05_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     griddep_launch();
 
     if (warp == 0) {
-        if (lane == 0) {
-            int s = 0; uint32_t ph = 0;
-            const int pre = num_kb < STAGES ? num_kb : STAGES;      // the first tile's weights before the wait: no predecessor writes them
-            for (int t = blockIdx.x, first = 1; t < total_tiles; t += gridDim.x, first = 0) {
-                int m_blk, n_blk; raster_tile(t, m_tiles, n_tiles, m_blk, n_blk);
-                if (first) {
-                    for (int kb = 0; kb < pre; ++kb) {
-                        mbar_expect_tx(&full_bar[kb], Cfg::STAGE_BYTES);
-                        tma_load_2d(smem + kb * Cfg::STAGE_BYTES + Cfg::A_BYTES, &tmB, &full_bar[kb], kb * BLOCK_K, n_blk * BN, kEvictFirst);
+        int s = 0; uint32_t ph = 0;
+        const int pre = num_kb < STAGES ? num_kb : STAGES;      // the first tile's weights before the wait: no predecessor writes them
+        for (int t = blockIdx.x, first = 1; t < total_tiles; t += gridDim.x, first = 0) {
+            int m_blk, n_blk; raster_tile(t, m_tiles, n_tiles, m_blk, n_blk);
+            if (first) {
+                for (int kb = 0; kb < pre; ++kb)
+                    if (elect_one()) {
+                        mbar_expect_tx(&full_bar[kb], STAGE_TX);
+                        tma_load_2d(ring_b + kb * Cfg::B_BYTES, &tmB, &full_bar[kb], kb * BLOCK_K, n_blk * BN, kEvictFirst);
                     }
-                    griddep_wait();
-                }
-                for (int kb = 0; kb < num_kb; ++kb) {
-                    uint8_t* a_dst = smem + s * Cfg::STAGE_BYTES;
-                    if (!first || kb >= pre) {
-                        mbar_wait(&empty_bar[s], ph ^ 1);
-                        mbar_expect_tx(&full_bar[s], Cfg::STAGE_BYTES);
-                        tma_load_2d(a_dst + Cfg::A_BYTES, &tmB, &full_bar[s], kb * BLOCK_K, n_blk * BN, m_tiles > 1 ? kEvictNormal : kEvictFirst);
+                griddep_wait();
+            }
+            for (int kb = 0; kb < num_kb; ++kb) {
+                const bool fresh = !first || kb >= pre;
+                if (fresh) mbar_wait(&empty_bar[s], ph ^ 1);
+                if (elect_one()) {
+                    if (fresh) {
+                        mbar_expect_tx(&full_bar[s], STAGE_TX);
+                        tma_load_2d(ring_b + s * Cfg::B_BYTES, &tmB, &full_bar[s], kb * BLOCK_K, n_blk * BN, m_tiles > 1 ? kEvictNormal : kEvictFirst);
                     }
-                    tma_load_2d(a_dst, &tmA, &full_bar[s], kb * BLOCK_K, m_blk * BLOCK_M, kEvictLast);
-                    if (++s == STAGES) { s = 0; ph ^= 1; }
+                    tma_load_2d(smem + s * A_BYTES, &tmA, &full_bar[s], kb * BLOCK_K, m_blk * BLOCK_M, kEvictLast);
                 }
+                __syncwarp();
+                if (++s == STAGES) { s = 0; ph ^= 1; }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = umma_idesc_bf16(BLOCK_M, BN);
-            int s = 0; uint32_t ph = 0; int it = 0;
-            for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++it) {
-                const int as = it & 1;
-                mbar_wait(&acc_empty[as], (((uint32_t)it >> 1) & 1) ^ 1);
+        constexpr uint32_t idesc = umma_idesc_bf16(BLOCK_M, BN);
+        int s = 0; uint32_t ph = 0; int it = 0;
+        for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++it) {
+            const int as = it & 1;
+            mbar_wait(&acc_empty[as], (((uint32_t)it >> 1) & 1) ^ 1);
+            tcgen05_fence_after();
+            const uint32_t tmem_d = tmem_base + (uint32_t)(as * BN);
+            for (int kb = 0; kb < num_kb; ++kb) {
+                mbar_wait(&full_bar[s], ph);
                 tcgen05_fence_after();
-                const uint32_t tmem_d = tmem_base + (uint32_t)(as * BN);
-                for (int kb = 0; kb < num_kb; ++kb) {
-                    mbar_wait(&full_bar[s], ph);
-                    tcgen05_fence_after();
-                    const uint32_t a_addr = smem_u32(smem + s * Cfg::STAGE_BYTES);
-                    const uint64_t a_desc = umma_desc_sw128(a_addr), b_desc = umma_desc_sw128(a_addr + Cfg::A_BYTES);
+                const uint64_t a_desc = umma_desc_sw128(smem_u32(smem + s * A_BYTES)), b_desc = umma_desc_sw128(smem_u32(ring_b + s * Cfg::B_BYTES));
+                if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < BLOCK_K / UMMA_K; ++k)
                         umma_bf16(tmem_d, a_desc + (uint64_t)(k * 2), b_desc + (uint64_t)(k * 2), idesc, (kb | k) != 0);
                     umma_commit(&empty_bar[s]);
-                    if (++s == STAGES) { s = 0; ph ^= 1; }
                 }
-                umma_commit(&acc_full[as]);
+                __syncwarp();
+                if (++s == STAGES) { s = 0; ph ^= 1; }
             }
+            if (elect_one()) umma_commit(&acc_full[as]);
+            __syncwarp();
         }
     } else {
         const int q = warp & 3;
+        float* stage = epi_smem + (warp - 2) * (EPI_WARP_BYTES / 4);
         griddep_wait();
         int it = 0;
         for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++it) {
@@ -690,7 +708,22 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_head_kernel(const __grid
                 uint32_t v[32];
                 tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * BN + c), v);
                 tmem_ld_wait();
-                if (row_ok) logits_chunk(p, row, v, n_blk * BN + c, mask_row, best_v, best_i);
+                if (row_ok) logits_chunk(p, row, v, n_blk * BN + c, mask_row, best_v, best_i, false);
+                if (p.logits) {          // through shared memory: four whole 128-byte lines a store instruction
+                    __syncwarp();
+#pragma unroll
+                    for (int j = 0; j < 32; j += 4)
+                        *reinterpret_cast<float4*>(stage + lane * EPI_ROW_FLOATS + j) =
+                            make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
+                    __syncwarp();
+                    const int c4 = (lane & 7) * 4, row0 = m_blk * BLOCK_M + q * 32;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const int r = i * 4 + (lane >> 3);
+                        if (row0 + r < p.M && n_blk * BN + c + c4 < p.N)
+                            *reinterpret_cast<float4*>(p.logits + (size_t)(row0 + r) * p.ldl + n_blk * BN + c + c4) = *reinterpret_cast<const float4*>(stage + r * EPI_ROW_FLOATS + c4);
+                    }
+                }
             }
             if (row_ok) { p.amax_val[(size_t)row * n_tiles + n_blk] = best_v; p.amax_idx[(size_t)row * n_tiles + n_blk] = best_i; }
             tcgen05_fence_before();
@@ -706,7 +739,7 @@ static cudaError_t launch_head(const CUtensorMap* tmA, const CUtensorMap* tmB, c
     static bool attr_done[16] = {};
     { cudaError_t e = ensure_dynamic_smem(gemm_head_kernel, HeadCfg::SMEM_BYTES, attr_done); if (e != cudaSuccess) return e; }
     const int tiles = gemm_n_tiles(p.N, HeadCfg::BN) * ((p.M + BLOCK_M - 1) / BLOCK_M);
-    return launch_k(gemm_head_kernel, dim3(std::min(tiles, sm_count_cached())), dim3(GEMM_THREADS), HeadCfg::SMEM_BYTES, stream, *tmA, *tmB, p);
+    return launch_k(gemm_head_kernel, dim3(std::min(tiles, sm_count_cached())), dim3(GEMM_THREADS), HeadCfg::SMEM_BYTES, stream, *tmA, *tmB, p, gemm_a_box(p, EPI_LOGITS, HEAD_BN));
 }
 // the persistent kernel from two rounds of its tiles on; the narrow tiles of a small vocabulary fill the SMs better one CTA each
 static bool head_persistent(int M, int N) { return (long long)gemm_n_tiles(N, HeadCfg::BN) * ((M + BLOCK_M - 1) / BLOCK_M) >= 2LL * sm_count_cached(); }
@@ -734,14 +767,14 @@ static cudaError_t launch_persistent(const CUtensorMap* tmA, const CUtensorMap* 
 // =============================================================================================
 template <int BN, int MT, int OCC = 1>     // MT = 128-row tiles of A per unit (1: M <= 128, 2: M <= 256); OCC = CTAs per SM the ring is sized for
 struct SkCfg {
-    static constexpr int A_TILE_BYTES = BLOCK_M * BLOCK_K * 2;
-    static constexpr int A_BYTES = MT * A_TILE_BYTES;
     static constexpr int B_BYTES = BN * BLOCK_K * 2;
-    static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-    static constexpr int STAGES = (OCC == 2 ? 92 * 1024 : 200 * 1024) / STAGE_BYTES;   // 6 x 32 KB (BN=128), 4 x 48 KB (BN=256); halved for 2 CTAs/SM
+    static constexpr int RING_BYTES = (OCC == 2 ? 92 : 200) * 1024, MAX_STAGES = 12;
+    // A rows a stage holds (MT tiles of those loaded) and stages that fit: 6 of 32 KB (128 rows, BN = 128), 10 of 20 KB (32 rows); halved for 2 CTAs/SM
+    __host__ __device__ static constexpr int a_tile_bytes(int a_rows) { return a_rows * BLOCK_K * 2; }
+    __host__ __device__ static constexpr int stages(int a_rows) { return RING_BYTES / (MT * a_tile_bytes(a_rows) + B_BYTES) < MAX_STAGES ? RING_BYTES / (MT * a_tile_bytes(a_rows) + B_BYTES) : MAX_STAGES; }
     static constexpr int EPI_ROW_FLOATS = 36;                          // 32 + 4 pad: conflict-free 16-byte smem accesses
     static constexpr int EPI_WARP_BYTES = 32 * EPI_ROW_FLOATS * 4;     // one 32x32 fp32 chunk per epilogue warp
-    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 4 * EPI_WARP_BYTES + 1024 + 256;
+    static constexpr int SMEM_BYTES = RING_BYTES + 4 * EPI_WARP_BYTES + 1024 + 256;
     static constexpr uint32_t TMEM_COLS = 2 * MT * BN;                 // two accumulator stages of MT row tiles
     static_assert(TMEM_COLS * OCC <= 512, "TMEM holds 512 columns per SM");
 };
@@ -757,25 +790,32 @@ struct SkFuse {
     SkRopeArgs rope;                    // FUSE 3
 };
 
+// Loads and products are issued by converged warps that walk (tile, k block) along: behind one lane, with a 64-bit division a unit, a unit took 480 cycles
+// and more of the 700 in which HBM delivers it, and a step's start, where the ring is full and only has to be multiplied, ran at that rate.  A stage
+// holds the rows of A there are, so a step of 32 rows has ten units in flight instead of six.  us a decoding step of four 8B layers, 32 conversations: 489 ->
+// 466; products alone, 64 x 57344 x 8192 175.7 -> 171.2, 64 x 5120 x 27648 67.2 -> 64.4, 32 x 4096 x 14336 42.1 -> 40.6 a call.
 template <int BN, int MT, int OCC, int FUSE = 0>
 __global__ void __launch_bounds__(GEMM_THREADS, OCC) gemm_streamk_kernel(const __grid_constant__ CUtensorMap tmA,
                                                                          const __grid_constant__ CUtensorMap tmB, const int M,
                                                                          const StreamK sk, const SkFuse fz) {
     using Cfg = SkCfg<BN, MT, OCC>;
-    constexpr int STAGES = Cfg::STAGES;
+    // ring: [stage][MT][A rows loaded], then [stage][B].  A product reads 128 rows from the start of its A block, beyond those loaded whatever lies behind
+    // it in the ring (inside it: the B stages follow): rows of the result that nobody looks at.
+    const int A_TILE = Cfg::a_tile_bytes(sk.a_rows), A_STRIDE = MT * A_TILE, STAGES = Cfg::stages(sk.a_rows);
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    float* epi_smem = reinterpret_cast<float*>(smem + STAGES * Cfg::STAGE_BYTES);
-    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * Cfg::STAGE_BYTES + 4 * Cfg::EPI_WARP_BYTES);
-    uint64_t* empty_bar = full_bar + STAGES;
-    uint64_t* acc_full = empty_bar + STAGES;      // [2]
+    uint8_t* ring_b = smem + STAGES * A_STRIDE;
+    float* epi_smem = reinterpret_cast<float*>(smem + Cfg::RING_BYTES);
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + Cfg::RING_BYTES + 4 * Cfg::EPI_WARP_BYTES);
+    uint64_t* empty_bar = full_bar + Cfg::MAX_STAGES;
+    uint64_t* acc_full = empty_bar + Cfg::MAX_STAGES;      // [2]
     uint64_t* acc_empty = acc_full + 2;           // [2]
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // warp: uniform, and known to be
     const long long c = blockIdx.x, G = gridDim.x;
     const long long u0 = c * sk.total / G, u1 = (c + 1) * sk.total / G;
-    const uint32_t stage_tx = (uint32_t)(MT * sk.a_rows * BLOCK_K * 2 + Cfg::B_BYTES);      // few rows: only they are loaded (the rest of the tile is stale, and its products are never read)
+    const uint32_t stage_tx = (uint32_t)(MT * A_TILE + Cfg::B_BYTES);
 
     if (warp == 0 && lane == 0) {
         tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmB);
@@ -787,77 +827,78 @@ __global__ void __launch_bounds__(GEMM_THREADS, OCC) gemm_streamk_kernel(const _
     tcgen05_fence_before();
     __syncthreads();
     tcgen05_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     griddep_launch();
 
     if (warp == 0) {
-        if (lane == 0) {
-            // weights first: they depend on no predecessor, so the HBM stream starts while the previous kernel drains
-            const int pre = (u1 - u0) < STAGES ? (int)(u1 - u0) : STAGES;
-            for (int i = 0; i < pre; ++i) {
-                const long long u = u0 + i;
-                const int tile = (int)(u / sk.kb), kblk = (int)(u - (long long)tile * sk.kb);
+        // (tile, k block) of the next unit, walked along: one division
+        const int n_units = (int)(u1 - u0), tile0 = (int)(u0 / sk.kb), kblk0 = (int)(u0 - (long long)tile0 * sk.kb);
+        int tile = tile0, kblk = kblk0;
+        auto next = [&]() { if (++kblk == sk.kb) { kblk = 0; ++tile; } };
+        // weights first: they depend on no predecessor, so the HBM stream starts while the previous kernel drains
+        const int pre = n_units < STAGES ? n_units : STAGES;
+        for (int i = 0; i < pre; ++i, next())
+            if (elect_one()) {
                 mbar_expect_tx(&full_bar[i], stage_tx);
-                tma_load_2d(smem + i * Cfg::STAGE_BYTES + Cfg::A_BYTES, &tmB, &full_bar[i], kblk * BLOCK_K, tile * BN, kEvictFirst);
+                tma_load_2d(ring_b + i * Cfg::B_BYTES, &tmB, &full_bar[i], kblk * BLOCK_K, tile * BN, kEvictFirst);
             }
-            // ... and pull the next weight tiles into L2 while the (L2-bound) predecessor still runs and HBM is idle
-            {
-                const long long pf_end = (u0 + pre + sk.l2_prefetch_units) < u1 ? (u0 + pre + sk.l2_prefetch_units) : u1;
-                for (long long u = u0 + pre; u < pf_end; ++u) {
-                    const int tile = (int)(u / sk.kb), kblk = (int)(u - (long long)tile * sk.kb);
-                    tma_prefetch_l2_2d(&tmB, kblk * BLOCK_K, tile * BN);
-                }
-            }
-            griddep_wait();
+        if (sk.l2_prefetch_units > 0) {          // ... and pull the next weight tiles into L2 while the (L2-bound) predecessor still runs and HBM is idle
+            const int t1 = tile, k1 = kblk, pf = n_units - pre < sk.l2_prefetch_units ? n_units - pre : sk.l2_prefetch_units;
+            for (int i = 0; i < pf; ++i, next())
+                if (elect_one()) tma_prefetch_l2_2d(&tmB, kblk * BLOCK_K, tile * BN);
+            tile = t1; kblk = k1;
+        }
+        griddep_wait();
+        {
+            int k0 = kblk0;
             for (int i = 0; i < pre; ++i) {
-                const long long u = u0 + i;
-                const int tile = (int)(u / sk.kb), kblk = (int)(u - (long long)tile * sk.kb);
+                if (elect_one()) {
 #pragma unroll
-                for (int m = 0; m < MT; ++m)
-                    tma_load_2d(smem + i * Cfg::STAGE_BYTES + m * Cfg::A_TILE_BYTES, &tmA, &full_bar[i], kblk * BLOCK_K, m * BLOCK_M, kEvictLast);
-            }
-            int s = pre == STAGES ? 0 : pre; uint32_t ph = pre == STAGES ? 1 : 0;
-            for (long long u = u0 + pre; u < u1; ++u) {
-                const int tile = (int)(u / sk.kb), kblk = (int)(u - (long long)tile * sk.kb);
-                mbar_wait(&empty_bar[s], ph ^ 1);
-                uint8_t* a_dst = smem + s * Cfg::STAGE_BYTES;
-                mbar_expect_tx(&full_bar[s], stage_tx);
-#pragma unroll
-                for (int m = 0; m < MT; ++m)
-                    tma_load_2d(a_dst + m * Cfg::A_TILE_BYTES, &tmA, &full_bar[s], kblk * BLOCK_K, m * BLOCK_M, kEvictLast);
-                tma_load_2d(a_dst + Cfg::A_BYTES, &tmB, &full_bar[s], kblk * BLOCK_K, tile * BN, kEvictFirst);
-                if (++s == STAGES) { s = 0; ph ^= 1; }
+                    for (int m = 0; m < MT; ++m) tma_load_2d(smem + i * A_STRIDE + m * A_TILE, &tmA, &full_bar[i], k0 * BLOCK_K, m * BLOCK_M, kEvictLast);
+                }
+                if (++k0 == sk.kb) k0 = 0;
             }
         }
-    } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = umma_idesc_bf16(BLOCK_M, BN);
-            int s = 0; uint32_t ph = 0; int seg = 0;
-            for (long long u = u0; u < u1; ++seg) {
-                const int tile = (int)(u / sk.kb);
-                const long long uend = min(u1, (long long)(tile + 1) * sk.kb);
-                const int as = seg & 1;
-                mbar_wait(&acc_empty[as], (((uint32_t)seg >> 1) & 1) ^ 1);      // epilogue has drained this accumulator
-                tcgen05_fence_after();
-                const uint32_t tmem_d = tmem_base + (uint32_t)(as * MT * BN);
-                for (long long uu = u; uu < uend; ++uu) {
-                    mbar_wait(&full_bar[s], ph);
-                    tcgen05_fence_after();
-                    const uint32_t a_addr = smem_u32(smem + s * Cfg::STAGE_BYTES);
-                    const uint64_t b_desc = umma_desc_sw128(a_addr + Cfg::A_BYTES);
+        int s = pre == STAGES ? 0 : pre; uint32_t ph = pre == STAGES ? 1 : 0;
+        for (int i = pre; i < n_units; ++i, next()) {
+            mbar_wait(&empty_bar[s], ph ^ 1);
+            if (elect_one()) {
+                mbar_expect_tx(&full_bar[s], stage_tx);
+                tma_load_2d(ring_b + s * Cfg::B_BYTES, &tmB, &full_bar[s], kblk * BLOCK_K, tile * BN, kEvictFirst);
 #pragma unroll
-                    for (int m = 0; m < MT; ++m) {
-                        const uint64_t a_desc = umma_desc_sw128(a_addr + m * Cfg::A_TILE_BYTES);
+                for (int m = 0; m < MT; ++m) tma_load_2d(smem + s * A_STRIDE + m * A_TILE, &tmA, &full_bar[s], kblk * BLOCK_K, m * BLOCK_M, kEvictLast);
+            }
+            __syncwarp();
+            if (++s == STAGES) { s = 0; ph ^= 1; }
+        }
+    } else if (warp == 1) {
+        constexpr uint32_t idesc = umma_idesc_bf16(BLOCK_M, BN);
+        int s = 0; uint32_t ph = 0; int seg = 0;
+        int kblk = (int)(u0 - (long long)(int)(u0 / sk.kb) * sk.kb);
+        for (int left = (int)(u1 - u0); left > 0; ++seg) {
+            const int n = left < sk.kb - kblk ? left : sk.kb - kblk;      // this CTA's units of one tile
+            const int as = seg & 1;
+            mbar_wait(&acc_empty[as], (((uint32_t)seg >> 1) & 1) ^ 1);      // epilogue has drained this accumulator
+            tcgen05_fence_after();
+            const uint32_t tmem_d = tmem_base + (uint32_t)(as * MT * BN);
+            for (int i = 0; i < n; ++i) {
+                mbar_wait(&full_bar[s], ph);
+                tcgen05_fence_after();
+                const uint64_t a_desc = umma_desc_sw128(smem_u32(smem + s * A_STRIDE)), b_desc = umma_desc_sw128(smem_u32(ring_b + s * Cfg::B_BYTES));
+                if (elect_one()) {
+#pragma unroll
+                    for (int m = 0; m < MT; ++m)
 #pragma unroll
                         for (int k = 0; k < BLOCK_K / UMMA_K; ++k)
-                            umma_bf16(tmem_d + (uint32_t)(m * BN), a_desc + (uint64_t)(k * 2), b_desc + (uint64_t)(k * 2), idesc, (uu > u || k > 0) ? 1u : 0u);
-                    }
+                            umma_bf16(tmem_d + (uint32_t)(m * BN), a_desc + (uint64_t)(m * (A_TILE >> 4) + k * 2), b_desc + (uint64_t)(k * 2), idesc, (i > 0 || k > 0) ? 1u : 0u);
                     umma_commit(&empty_bar[s]);
-                    if (++s == STAGES) { s = 0; ph ^= 1; }
                 }
-                umma_commit(&acc_full[as]);
-                u = uend;
+                __syncwarp();
+                if (++s == STAGES) { s = 0; ph ^= 1; }
             }
+            if (elect_one()) umma_commit(&acc_full[as]);
+            __syncwarp();
+            left -= n; kblk = 0;
         }
     } else {
         const int q = warp & 3;

@@ -149,6 +149,7 @@ DeviceModel::DeviceModel(const ModelConfig& c, const EngineOptions& o) : ModelBa
     xs_ = dmalloc((size_t)MS * H * 2); xsn_ = dmalloc((size_t)MS * H * 2);
     cuda_check(cudaMemsetAsync(xsn_, 0, (size_t)MS * H * 2, stream), "memset");
     amap(&tm_xsn_, xsn_, MS, H);
+    for (int i = 0; i < 3; ++i) amap(&tm_few_xsn_[i], xsn_, MS, H, 16 << i);
     const int lm_tiles_max = gemm_n_tiles(V_l, 32);
     amax_val_ = reinterpret_cast<float*>(dmalloc((size_t)MS * lm_tiles_max * 4));
     amax_idx_ = reinterpret_cast<int*>(dmalloc((size_t)MS * lm_tiles_max * 4));
@@ -623,7 +624,7 @@ void DeviceModel::forward(const StepInput& in, float* logits_out) {
         MARK(11);
         const int bn_lm = opt.bn_lm ? pick_bn(S, V, opt.bn_lm, false) : gemm_logits_bn(S, V, pick_bn(S, V, 0, false));
         const int n_tiles = gemm_n_tiles(V, bn_lm);
-        GemmParams gl{}; gl.M = S; gl.N = V; gl.K = H; gl.logits = logits_out; gl.ldl = V; gl.amax_val = amax_val_; gl.amax_idx = amax_idx_;
+        GemmParams gl{}; gl.M = S; gl.N = V; gl.K = H; gl.logits = logits_out; gl.ldl = V; gl.amax_val = amax_val_; gl.amax_idx = amax_idx_; gl.few_rows_ok = 1;
         if (!in.mask_slots.empty()) {          // constrained rows: the arg-max runs over their state's allowed tokens, on every vocabulary shard
             gl.mask_table = mask_table_; gl.mask_slot = d_meta_ + o_mslot; gl.mask_words = mask_words; gl.col_offset = tp_rank * V;
         }
@@ -635,7 +636,8 @@ void DeviceModel::forward(const StepInput& in, float* logits_out) {
                 lb = comm->next_buffer(); gl.logits = reinterpret_cast<float*>(comm->sym(lb)); gl.ldl = V;
             }
         }
-        cuda_check(launch_gemm(&tm_xsn_, lm_head.map(bn_lm), gl, EPI_LOGITS, bn_lm, stream), "lm_head gemm"); MARK(12);
+        const int lm_rows = gemm_a_box(gl, EPI_LOGITS, bn_lm);
+        cuda_check(launch_gemm(lm_rows == 128 ? &tm_xsn_ : &tm_few_xsn_[lm_rows >> 5], lm_head.map(bn_lm), gl, EPI_LOGITS, bn_lm, stream), "lm_head gemm"); MARK(12);
         if (use_tp) {
             const int b = comm->next_buffer();
             cuda_check(launch_argmax_reduce_pair(amax_val_, amax_idx_, S, n_tiles, tp_rank * V, comm->arg(b), stream), "argmax (local shard)");

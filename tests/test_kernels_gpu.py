@@ -451,6 +451,28 @@ def test_persistent_vocabulary_head(L, M, N, K):
     assert (ids.long() == first).all() and (ids2 == ids).all() and ids[0].item() == N - 1
 
 
+# rings of 16, 32, 64 and 128 loaded rows (head and stream-K): rows have the bits they have among 128, more k blocks than stages and fewer
+@pytest.mark.parametrize("N,K", [(38016, 1000), (40008, 72), (38400, 136)])
+def test_rings_of_few_rows_keep_the_bits(L, N, K):
+    g = torch.Generator(device=dev()).manual_seed(N + K)
+    A = torch.randn(128, K, generator=g, device=dev()).to(torch.bfloat16)
+    B = (torch.randn(N, K, generator=g, device=dev()) * 0.1).to(torch.bfloat16)
+
+    def products(M):
+        logits, ids, sk = torch.full((M, N), float("nan"), device=dev()), torch.full((M,), -1, dtype=torch.int32, device=dev()), torch.full((M, N), float("nan"), device=dev())
+        assert L.oa_host_gemm_kernel(M, N, K, EPI_LOGITS, 128, 1, 0) == HEAD
+        assert L.oa_k_gemm(ptr(A), ptr(B), M, N, K, EPI_LOGITS, 128, None, None, None, ptr(logits), ptr(ids), None) == 0
+        assert L.oa_k_gemm_streamk(ptr(A), ptr(B), M, N, K, 128, 148, ptr(sk), None) == 0
+        return logits, ids, sk
+
+    whole = products(128)
+    # fp32 sums of K products of size about 0.1 |a| (the bits are compared below)
+    assert ((whole[0].double() - A.double() @ B.double().T).abs() <= 0.1 * 4 * K * 2.0 ** -23 + 1e-6).all()
+    for M in (1, 7, 15, 16, 17, 32, 33, 64, 65, 127):
+        for got, want in zip(products(M), whole):
+            assert torch.equal(got, want[:M]), M
+
+
 @pytest.mark.parametrize("M", [5, 100, 700])
 @pytest.mark.parametrize("epi", [EPI_STORE, EPI_SWIGLU, EPI_LOGITS])
 @pytest.mark.parametrize("bn", [0, 16, 96, 192, 512, -64])
