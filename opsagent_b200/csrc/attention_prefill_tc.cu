@@ -1,7 +1,7 @@
 // attention_prefill_tc.cu — causal prefill attention over the paged KV cache on the 5th-generation tensor cores.
 //
 // One CTA = 128 query rows of one (sequence, head); KV is consumed in tiles of 128 tokens (two 64-token pages):
-//   warp 0    : TMA producers — lane 0: Q tile once, then the K pages of each KV tile; lane 1: the V pages.  K and V have SEPARATE
+//   warp 0    : TMA producer — Q tile once, then the K pages of a KV tile and the V pages of the one before it.  K and V have SEPARATE
 //               2-stage rings: K_j is released as soon as S_j has been computed, V_j only after P_j·V_j, so the K load of tile
 //               j+2 gets a full tile period of slack instead of being exposed behind the second MMA
 //   warp 1    : tcgen05.mma issuer —  S_j = Q · K_j^T   (M=128, N=128, K=D;   A, B K-major)        -> TMEM S[j&1]
@@ -19,6 +19,57 @@
 namespace oa {
 
 static constexpr int KV_TILE = 128;
+
+// One warp: 64 columns of O of its 32 rows (TMEM lanes of `addr`, a row's values scaled by its lane's inv), rounded to bf16.  A lane holds a row, so a store
+// straight from registers is 32 pieces of 16 bytes; through 4 KB of shared memory it is four whole 128-byte lines.
+OA_DEVINL void store_o_64(uint8_t* stage, uint32_t addr, float inv, uint16_t* out, size_t pitch, int lane) {
+#pragma unroll
+    for (int c = 0; c < 64; c += 32) {
+        uint32_t o[32];
+        tmem_ld_32x32b_x32(addr + (uint32_t)c, o);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 32; i += 8) {
+            uint4 w;
+            w.x = pack_bf16x2(__uint_as_float(o[i]) * inv, __uint_as_float(o[i + 1]) * inv);
+            w.y = pack_bf16x2(__uint_as_float(o[i + 2]) * inv, __uint_as_float(o[i + 3]) * inv);
+            w.z = pack_bf16x2(__uint_as_float(o[i + 4]) * inv, __uint_as_float(o[i + 5]) * inv);
+            w.w = pack_bf16x2(__uint_as_float(o[i + 6]) * inv, __uint_as_float(o[i + 7]) * inv);
+            *reinterpret_cast<uint4*>(stage + lane * 128 + ((((c + i) >> 3) ^ (lane & 7)) << 4)) = w;
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int r = i * 4 + (lane >> 3), ch = lane & 7;
+        const uint4 w = *reinterpret_cast<const uint4*>(stage + r * 128 + ((ch ^ (r & 7)) << 4));
+        *reinterpret_cast<uint4*>(out + (size_t)r * pitch + ch * 8) = w;
+    }
+    __syncwarp();
+}
+
+// The same of COLS columns straight from registers, a lane its row: with 64 columns a head a row is one line, and this is the faster way (five prompts of
+// 1400 rows, 32 / 8 heads of 64: 74.7 us a layer against 78.9 through shared memory).  So it is for warps with rows missing.
+template <int COLS>
+OA_DEVINL void store_o_direct(uint32_t addr, float inv, uint16_t* row, bool live) {
+#pragma unroll 1
+    for (int c = 0; c < COLS; c += 32) {
+        uint32_t o[32];
+        tmem_ld_32x32b_x32(addr + (uint32_t)c, o);
+        tmem_ld_wait();
+        if (live) {
+#pragma unroll
+            for (int i = 0; i < 32; i += 8) {
+                uint4 w;
+                w.x = pack_bf16x2(__uint_as_float(o[i]) * inv, __uint_as_float(o[i + 1]) * inv);
+                w.y = pack_bf16x2(__uint_as_float(o[i + 2]) * inv, __uint_as_float(o[i + 3]) * inv);
+                w.z = pack_bf16x2(__uint_as_float(o[i + 4]) * inv, __uint_as_float(o[i + 5]) * inv);
+                w.w = pack_bf16x2(__uint_as_float(o[i + 6]) * inv, __uint_as_float(o[i + 7]) * inv);
+                *reinterpret_cast<uint4*>(row + c + i) = w;
+            }
+        }
+    }
+}
 
 template <int D>
 struct PtcCfg {
@@ -65,11 +116,11 @@ __global__ void __launch_bounds__(64 + 128 * NWG, 1) prefill_attention_tc_kernel
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
     float* xch = reinterpret_cast<float*>(p_s + 2 * Cfg::P_BYTES + 256);       // [2][2][128]
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // warp: uniform, and known to be
     const PrefillTile tile = p.tiles[blockIdx.x];
     const int head = blockIdx.y;
     const int grp = p.n_heads / p.n_kv, kvh = head / grp;
-    const int n_kvt = (tile.pos0 + tile.n_rows + KV_TILE - 1) / KV_TILE;       // KV tiles 0..n_kvt-1 cover every visible key
+    const int n_kvt = __shfl_sync(0xffffffffu, (tile.pos0 + tile.n_rows + KV_TILE - 1) / KV_TILE, 0);       // KV tiles 0..n_kvt-1 cover every visible key
 
     if (warp == 0 && lane == 0) {
         tma_prefetch_desc(&tm_q); tma_prefetch_desc(&tm_kv);
@@ -83,75 +134,88 @@ __global__ void __launch_bounds__(64 + 128 * NWG, 1) prefill_attention_tc_kernel
     tcgen05_fence_before();
     __syncthreads();
     tcgen05_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     griddep_launch();
 
     if (warp == 0) {
-        if (lane < 2) {
-            const bool is_v = lane == 1;
-            griddep_wait();
-            if (!is_v) {
-                mbar_expect_tx(q_full, Cfg::Q_BYTES);
+        griddep_wait();
+        if (elect_one()) {
+            mbar_expect_tx(q_full, Cfg::Q_BYTES);
 #pragma unroll
-                for (int h = 0; h < HALVES; ++h) tma_load_2d(q_s + h * Cfg::HALF_BYTES, &tm_q, q_full, head * D + h * 64, tile.q_row0, kEvictFirst);
+            for (int h = 0; h < HALVES; ++h) tma_load_2d(q_s + h * Cfg::HALF_BYTES, &tm_q, q_full, head * D + h * 64, tile.q_row0, kEvictFirst);
+        }
+        __syncwarp();
+        const int32_t* bt = p.block_tables + (size_t)tile.seq * p.max_pages_per_seq;
+        // K of tile j, then V of the tile before it: K_j's slot is free as soon as S_{j-2} exists, V_{j-1}'s only after P_{j-3}·V
+        int32_t page[2] = {0, 0}, prev[2] = {0, 0};
+        for (int j = 0; j <= n_kvt; ++j) {
+#pragma unroll
+            for (int pg = 0; pg < 2; ++pg) {
+                prev[pg] = page[pg];
+                const int pi = 2 * j + pg;
+                if (j < n_kvt) page[pg] = bt[pi < p.max_pages_per_seq ? pi : 2 * j];      // a missing second page is fully masked anyway
             }
-            const int32_t* bt = p.block_tables + (size_t)tile.seq * p.max_pages_per_seq;
-            uint64_t* full = is_v ? v_full : k_full;
-            uint64_t* empty = is_v ? v_empty : k_empty;
-            for (int j = 0; j < n_kvt; ++j) {
-                const int st = j & 1;
-                mbar_wait(&empty[st], (((uint32_t)j >> 1) & 1) ^ 1);
-                uint8_t* dst = kv_s + st * Cfg::STAGE_BYTES + (is_v ? Cfg::KV_BYTES : 0);
-                mbar_expect_tx(&full[st], Cfg::KV_BYTES);
 #pragma unroll
-                for (int pg = 0; pg < 2; ++pg) {
-                    const int pi = 2 * j + pg;
-                    const int page = bt[pi < p.max_pages_per_seq ? pi : 2 * j];      // a missing second page is fully masked anyway
-                    const int64_t row = layer_row0 + ((int64_t)page * p.n_kv + kvh) * 64 + (is_v ? kv_stride_rows : 0);
+            for (int v = 0; v < 2; ++v) {
+                const int jt = j - v;                                     // tile loaded: K of j, V of j - 1
+                if (jt < 0 || jt >= n_kvt) continue;
+                const int st = jt & 1;
+                uint64_t* full = (v ? v_full : k_full) + st;
+                mbar_wait((v ? v_empty : k_empty) + st, (((uint32_t)jt >> 1) & 1) ^ 1);
+                if (elect_one()) {
+                    uint8_t* dst = kv_s + st * Cfg::STAGE_BYTES + (v ? Cfg::KV_BYTES : 0);
+                    mbar_expect_tx(full, Cfg::KV_BYTES);
 #pragma unroll
-                    for (int h = 0; h < HALVES; ++h)
-                        tma_load_2d(dst + h * Cfg::HALF_BYTES + pg * 8192, &tm_kv, &full[st], h * 64, (int32_t)row, kEvictLast);
+                    for (int pg = 0; pg < 2; ++pg) {
+                        const int64_t row = layer_row0 + ((int64_t)(v ? prev[pg] : page[pg]) * p.n_kv + kvh) * 64 + (v ? kv_stride_rows : 0);
+#pragma unroll
+                        for (int h = 0; h < HALVES; ++h)
+                            tma_load_2d(dst + h * Cfg::HALF_BYTES + pg * 8192, &tm_kv, full, h * 64, (int32_t)row, kEvictLast);
+                    }
                 }
+                __syncwarp();
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc_s = umma_idesc_bf16(128, KV_TILE);
-            constexpr uint32_t idesc_t = umma_idesc_bf16_bmn(128, D);
-            const uint32_t q_addr = smem_u32(q_s);
-            auto issue_s = [&](int j) {
-                const int st = j & 1, sb = j & 1;
-                mbar_wait(&k_full[st], ((uint32_t)j >> 1) & 1);
-                mbar_wait(&s_empty[sb], (((uint32_t)j >> 1) & 1) ^ 1);
-                tcgen05_fence_after();
-                const uint32_t k_addr = smem_u32(kv_s + st * Cfg::STAGE_BYTES);
+        // The whole warp walks the loop, an elected lane issues: descriptors stay in uniform registers
+        constexpr uint32_t idesc_s = umma_idesc_bf16(128, KV_TILE);
+        constexpr uint32_t idesc_t = umma_idesc_bf16_bmn(128, D);
+        const uint64_t q_desc = umma_desc_sw128(smem_u32(q_s)), k_desc = umma_desc_sw128(smem_u32(kv_s)), p_desc = umma_desc_sw128(smem_u32(p_s));
+        const uint64_t v_desc = umma_desc_sw128_mn(smem_u32(kv_s + Cfg::KV_BYTES), (uint32_t)Cfg::HALF_BYTES, 1024u);
+        auto issue_s = [&](int j) {
+            const int st = j & 1;
+            mbar_wait(&k_full[st], ((uint32_t)j >> 1) & 1);
+            mbar_wait(&s_empty[st], (((uint32_t)j >> 1) & 1) ^ 1);
+            tcgen05_fence_after();
+            if (elect_one()) {
+                const uint64_t b = k_desc + (uint64_t)(st * (Cfg::STAGE_BYTES >> 4));
 #pragma unroll
                 for (int ks = 0; ks < D / 16; ++ks) {
-                    const uint32_t off = (uint32_t)((ks >> 2) * Cfg::HALF_BYTES + (ks & 3) * 32);
-                    umma_bf16(tmem_base + (uint32_t)(sb * 128), umma_desc_sw128(q_addr + off), umma_desc_sw128(k_addr + off), idesc_s, ks > 0 ? 1u : 0u);
+                    const uint64_t off = (uint64_t)(((ks >> 2) * Cfg::HALF_BYTES + (ks & 3) * 32) >> 4);
+                    umma_bf16(tmem_base + (uint32_t)(st * 128), q_desc + off, b + off, idesc_s, ks > 0 ? 1u : 0u);
                 }
-                umma_commit(&s_full[sb]);
+                umma_commit(&s_full[st]);
                 umma_commit(&k_empty[st]);                                 // K_j is free once S_j exists
-            };
-            mbar_wait(q_full, 0);
-            issue_s(0);
-            for (int j = 0; j < n_kvt; ++j) {
-                if (j + 1 < n_kvt) issue_s(j + 1);                         // keep the tensor pipe ahead of the softmax warps
-                const int st = j & 1, pb = j & 1;
-                mbar_wait(&p_full[pb], ((uint32_t)j >> 1) & 1);            // P_j is in shared memory
-                mbar_wait(&v_full[st], ((uint32_t)j >> 1) & 1);
-                tcgen05_fence_after();
-                const uint32_t p_addr = smem_u32(p_s + pb * Cfg::P_BYTES);
-                const uint32_t v_addr = smem_u32(kv_s + st * Cfg::STAGE_BYTES + Cfg::KV_BYTES);
+            }
+            __syncwarp();
+        };
+        mbar_wait(q_full, 0);
+        issue_s(0);
+        for (int j = 0; j < n_kvt; ++j) {
+            if (j + 1 < n_kvt) issue_s(j + 1);                         // keep the tensor pipe ahead of the softmax warps
+            const int st = j & 1;
+            mbar_wait(&p_full[st], ((uint32_t)j >> 1) & 1);            // P_j is in shared memory
+            mbar_wait(&v_full[st], ((uint32_t)j >> 1) & 1);
+            tcgen05_fence_after();
+            if (elect_one()) {
+                const uint64_t a = p_desc + (uint64_t)(st * (Cfg::P_BYTES >> 4)), b = v_desc + (uint64_t)(st * (Cfg::STAGE_BYTES >> 4));
 #pragma unroll
-                for (int ks = 0; ks < KV_TILE / 16; ++ks) {
-                    const uint64_t a_desc = umma_desc_sw128(p_addr + (uint32_t)((ks >> 2) * Cfg::HALF_BYTES + (ks & 3) * 32));
-                    const uint64_t b_desc = umma_desc_sw128_mn(v_addr + (uint32_t)(ks * 2048), (uint32_t)Cfg::HALF_BYTES, 1024u);
-                    umma_bf16(tmem_base + Cfg::T_COL, a_desc, b_desc, idesc_t, (j > 0 || ks > 0) ? 1u : 0u);      // O accumulates over all KV tiles
-                }
+                for (int ks = 0; ks < KV_TILE / 16; ++ks)              // O accumulates over all KV tiles
+                    umma_bf16(tmem_base + Cfg::T_COL, a + (uint64_t)(((ks >> 2) * Cfg::HALF_BYTES + (ks & 3) * 32) >> 4), b + (uint64_t)(ks * (2048 >> 4)), idesc_t, (j > 0 || ks > 0) ? 1u : 0u);
                 umma_commit(t_full);
                 umma_commit(&v_empty[st]);
             }
+            __syncwarp();
         }
     } else {
         const int q = warp & 3, wg = (warp - 2) >> 2;               // warps w and w + 4 own the same rows (TMEM lanes 32 * (w % 4) ...)
@@ -247,24 +311,10 @@ __global__ void __launch_bounds__(64 + 128 * NWG, 1) prefill_attention_tc_kernel
             l_run = xch[(xb * 2 + 0) * 128 + row] + xch[(xb * 2 + 1) * 128 + row];
         }
         const float inv = 1.0f / l_run;
-        uint16_t* orow = reinterpret_cast<uint16_t*>(p.out) + (size_t)(tile.q_row0 + row) * p.n_heads * D + (size_t)head * D;
-#pragma unroll 1
-        for (int c = 0; c < OC; c += 32) {
-            uint32_t o[32];
-            tmem_ld_32x32b_x32(tmem_base + lane_addr + Cfg::T_COL + (uint32_t)(o_base + c), o);
-            tmem_ld_wait();
-            if (row < tile.n_rows) {
-#pragma unroll
-                for (int i = 0; i < 32; i += 8) {
-                    uint4 w;
-                    w.x = pack_bf16x2(__uint_as_float(o[i]) * inv, __uint_as_float(o[i + 1]) * inv);
-                    w.y = pack_bf16x2(__uint_as_float(o[i + 2]) * inv, __uint_as_float(o[i + 3]) * inv);
-                    w.z = pack_bf16x2(__uint_as_float(o[i + 4]) * inv, __uint_as_float(o[i + 5]) * inv);
-                    w.w = pack_bf16x2(__uint_as_float(o[i + 6]) * inv, __uint_as_float(o[i + 7]) * inv);
-                    *reinterpret_cast<uint4*>(orow + o_base + c + i) = w;
-                }
-            }
-        }
+        uint16_t* orow = reinterpret_cast<uint16_t*>(p.out) + (size_t)(tile.q_row0 + q * 32) * p.n_heads * D + (size_t)head * D;
+        const uint32_t o_addr = tmem_base + lane_addr + Cfg::T_COL + (uint32_t)o_base;
+        if (OC == 64 && tile.n_rows >= q * 32 + 32) store_o_64(p_s + (warp - 2) * 4096, o_addr, inv, orow + o_base, (size_t)p.n_heads * D, lane);      // P has been read by the last product
+        else store_o_direct<OC>(o_addr, inv, orow + (size_t)lane * p.n_heads * D + o_base, row < tile.n_rows);
     }
     tcgen05_fence_before();
     __syncthreads();
@@ -287,10 +337,14 @@ __global__ void __launch_bounds__(64 + 128 * NWG, 1) prefill_attention_tc_kernel
 // A group with an odd number of heads leaves its last one alone in an item (warpgroup B idles).
 // A row's scores, reference maxima, probabilities and sums are those of the kernel above, in its order: which of the two a batch takes moves no bit.
 // (Four sums per row instead of two are 3 % faster, and moved the last one.)
-// Measured against the kernel above: 4096 rows behind 12288 cached ones, 64 / 8 heads of 128: 1963 -> 1590 us in a burst (the tensor and the
-// special-function pipe are each busy 60 % of the time and the clock is down to 1.63 GHz under the 1000 W cap); five prompts of 1.4 thousand rows,
-// 32 / 8 heads: 184 -> 122 us.  Handing P over in two or three parts, taking exponentials from a reference that may still rise, moving an eighth
-// or a quarter of them to the FMA pipe and two threads per row were each 3 to 12 % slower.
+// Measured against the kernel above: 4096 rows behind 12288 cached ones, 64 / 8 heads of 128: 1963 -> 1416 us in a burst; five prompts of 1.4 thousand rows,
+// 32 / 8 heads: 184 -> 102 us.  Of that: the issuing warp stays converged (behind one lane its 32 products a tile pair took longer than the tensor core
+// has for them): 1548 -> 1489 and 120 -> 114 us; P is handed over in two parts, so that the first 64 keys are multiplied under the other exponentials:
+// -> 1417 and 108 us (three or four parts, or loading S in two halves under the maxima: no difference); O leaves in whole lines and the next item
+// is read under the last product: -> 1416 and 102 us.  What bounds it now is a head's chain in a tile, 2900 cycles: 125 to fetch S, 275 for the
+// maximum, 1500 for 128 exponentials a row (1024 alone on the special-function units, which the other head's overlap in part), 970 for the rest of P·V
+// and the next S.  Tensor and special-function pipes are busy 65 to 70 % of it, and a long loop runs into the 1000 W cap.  Taking exponentials from a reference
+// that may still rise, moving an eighth or a quarter of them to the FMA pipe and two threads per row were each 3 to 12 % slower.
 // ---------------------------------------------------------------------------------------------
 template <int D>
 struct PtpCfg {
@@ -298,7 +352,9 @@ struct PtpCfg {
     static constexpr int HALF_BYTES = 128 * 128;
     static constexpr int TILE_BYTES = HALVES * HALF_BYTES;       // Q of one head, K or V of one 128-token tile
     static constexpr int STAGES = 2;
-    static constexpr int SMEM_BYTES = (2 + 2 * STAGES) * TILE_BYTES + 256;
+    static constexpr int OUT_BYTES = D == 128 ? 8 * 4096 : 0;    // what a softmax warp writes its rows of O through
+    static constexpr int SMEM_BYTES = (2 + 2 * STAGES) * TILE_BYTES + OUT_BYTES + 256;
+    static_assert(SMEM_BYTES <= 232448, "shared memory budget of one CTA");
     static constexpr uint32_t TMEM_COLS = 512;
     static constexpr uint32_t S_COL = 0, O_COL = 256;            // S_A, S_B (P over them), then O_A, O_B: 128 columns each
     static constexpr int THREADS = 3 * 128;
@@ -330,7 +386,8 @@ __global__ void __launch_bounds__(PtpCfg<D>::THREADS, 1) prefill_attention_pair_
     uint8_t* q_s = smem_raw;                                     // [2 heads]
     uint8_t* k_s = q_s + 2 * Cfg::TILE_BYTES;                    // [STAGES]
     uint8_t* v_s = k_s + STAGES * Cfg::TILE_BYTES;               // [STAGES]
-    uint64_t* bars = reinterpret_cast<uint64_t*>(v_s + STAGES * Cfg::TILE_BYTES);
+    uint8_t* out_s = v_s + STAGES * Cfg::TILE_BYTES;             // [8 warps]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(out_s + Cfg::OUT_BYTES);
     uint64_t* q_full = bars;                  // 1
     uint64_t* q_empty = bars + 1;             // 1
     uint64_t* k_full = bars + 2;              // [STAGES]
@@ -338,11 +395,11 @@ __global__ void __launch_bounds__(PtpCfg<D>::THREADS, 1) prefill_attention_pair_
     uint64_t* v_full = k_empty + STAGES;
     uint64_t* v_empty = v_full + STAGES;
     uint64_t* s_full = v_empty + STAGES;      // [2 heads]
-    uint64_t* p_full = s_full + 2;
-    uint64_t* o_full = p_full + 2;
+    uint64_t* p_full = s_full + 2;            // [2 heads][lower, upper 64 keys]
+    uint64_t* o_full = p_full + 4;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 2);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // warp: uniform, and known to be
     const int grp = p.n_heads / p.n_kv, ppg = (grp + 1) / 2;
     PtpItem it;
 
@@ -350,23 +407,26 @@ __global__ void __launch_bounds__(PtpCfg<D>::THREADS, 1) prefill_attention_pair_
         tma_prefetch_desc(&tm_q); tma_prefetch_desc(&tm_kv);
         mbar_init(q_full, 1); mbar_init(q_empty, 1);
         for (int i = 0; i < STAGES; ++i) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
-        for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 4); mbar_init(&o_full[i], 1); }
+        for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&p_full[2 * i], 4); mbar_init(&p_full[2 * i + 1], 4); mbar_init(&o_full[i], 1); }
         fence_barrier_init();
     }
     if (warp == 1) tmem_alloc<Cfg::TMEM_COLS>(tmem_slot);
     tcgen05_fence_before();
     __syncthreads();
     tcgen05_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     griddep_launch();
 
     // registers: 384 x 168 at launch = 128 x (88 + 208 + 208)
     if (warp < 4) {
         reg_dec<88>();
-        if (warp == 0 && lane == 0) {
+        if (warp == 0) {
             griddep_wait();
             uint32_t kc = 0;
-            for (int r = 0; ptp_item(p, ppg, r, it); ++r) {
+            PtpItem next;
+            bool more = ptp_item(p, ppg, 0, it);
+            for (int r = 0; more; ++r, it = next) {
+                const int n_kvt = __shfl_sync(0xffffffffu, it.n_kvt, 0);
                 const int32_t* bt = p.block_tables + (size_t)it.tile.seq * p.max_pages_per_seq;
                 const int kvh = it.head / grp;
                 auto page_row = [&](int pi, int fallback) { return layer_row0 + ((int64_t)bt[pi < p.max_pages_per_seq ? pi : fallback] * p.n_kv + kvh) * 64; };   // a missing second page is fully masked anyway
@@ -379,67 +439,99 @@ __global__ void __launch_bounds__(PtpCfg<D>::THREADS, 1) prefill_attention_pair_
                     }
                 };
                 int64_t r0 = page_row(0, 0), r1 = page_row(1, 0);
-                for (int j = 0; j < it.n_kvt; ++j, ++kc) {
+                for (int j = 0; j < n_kvt; ++j, ++kc) {
                     const uint32_t st = kc % STAGES, ph = (kc / STAGES) & 1;
                     mbar_wait(&k_empty[st], ph ^ 1);
-                    load(k_s + st * Cfg::TILE_BYTES, &k_full[st], r0, r1);
+                    if (elect_one()) load(k_s + st * Cfg::TILE_BYTES, &k_full[st], r0, r1);
+                    __syncwarp();
                     if (j == 0) {
                         mbar_wait(q_empty, ((uint32_t)r & 1) ^ 1);
-                        mbar_expect_tx(q_full, (it.two ? 2 : 1) * Cfg::TILE_BYTES);
-                        for (int x = 0; x <= it.two; ++x)
+                        if (elect_one()) {
+                            mbar_expect_tx(q_full, (it.two ? 2 : 1) * Cfg::TILE_BYTES);
+                            for (int x = 0; x <= it.two; ++x)
 #pragma unroll
-                            for (int h = 0; h < HALVES; ++h)
-                                tma_load_2d(q_s + x * Cfg::TILE_BYTES + h * Cfg::HALF_BYTES, &tm_q, q_full, (it.head + x) * D + h * 64, it.tile.q_row0, kEvictFirst);
+                                for (int h = 0; h < HALVES; ++h)
+                                    tma_load_2d(q_s + x * Cfg::TILE_BYTES + h * Cfg::HALF_BYTES, &tm_q, q_full, (it.head + x) * D + h * 64, it.tile.q_row0, kEvictFirst);
+                        }
+                        __syncwarp();
+                        more = ptp_item(p, ppg, r + 1, next);                  // read now, needed an item later
                     }
                     int64_t n0 = r0, n1 = r1;                                  // the next tile's pages are looked up while this one's slot is waited for
-                    if (j + 1 < it.n_kvt) { n0 = page_row(2 * j + 2, 0); n1 = page_row(2 * j + 3, 2 * j + 2); }
+                    if (j + 1 < n_kvt) { n0 = page_row(2 * j + 2, 0); n1 = page_row(2 * j + 3, 2 * j + 2); }
                     mbar_wait(&v_empty[st], ph ^ 1);
-                    load(v_s + st * Cfg::TILE_BYTES, &v_full[st], r0 + kv_stride_rows, r1 + kv_stride_rows);
+                    if (elect_one()) load(v_s + st * Cfg::TILE_BYTES, &v_full[st], r0 + kv_stride_rows, r1 + kv_stride_rows);
+                    __syncwarp();
                     r0 = n0; r1 = n1;
                 }
             }
-        } else if (warp == 1 && lane == 0) {
+        } else if (warp == 1) {
+            // The whole warp walks the loop, an elected lane issues: descriptors stay in uniform registers
             constexpr uint32_t idesc_s = umma_idesc_bf16(128, KV_TILE), idesc_o = umma_idesc_bf16_bmn(128, D);
-            const uint32_t q_addr = smem_u32(q_s), k_addr0 = smem_u32(k_s), v_addr0 = smem_u32(v_s);
+            const uint64_t q_desc = umma_desc_sw128(smem_u32(q_s)), k_desc = umma_desc_sw128(smem_u32(k_s)), v_desc = umma_desc_sw128_mn(smem_u32(v_s), (uint32_t)Cfg::HALF_BYTES, 1024u);
+            constexpr uint64_t TILE = Cfg::TILE_BYTES >> 4;                    // in a descriptor's address units
             uint32_t kc = 0, vc = 0, pc[2] = {0, 0};                           // K / V tiles taken, P tiles taken per head
             auto issue_s = [&](int x) {                                        // S_x = Q_x K^T with K tile kc
-                const uint32_t a = q_addr + x * Cfg::TILE_BYTES, b = k_addr0 + (kc % STAGES) * Cfg::TILE_BYTES;
+                const uint64_t a = q_desc + x * TILE, b = k_desc + (kc % STAGES) * TILE;
 #pragma unroll
                 for (int ks = 0; ks < D / 16; ++ks) {
-                    const uint32_t off = (uint32_t)((ks >> 2) * Cfg::HALF_BYTES + (ks & 3) * 32);
-                    umma_bf16(tmem_base + Cfg::S_COL + x * 128, umma_desc_sw128(a + off), umma_desc_sw128(b + off), idesc_s, ks > 0 ? 1u : 0u);
+                    const uint64_t off = (uint64_t)(((ks >> 2) * Cfg::HALF_BYTES + (ks & 3) * 32) >> 4);
+                    umma_bf16(tmem_base + Cfg::S_COL + x * 128, a + off, b + off, idesc_s, ks > 0 ? 1u : 0u);
                 }
                 umma_commit(&s_full[x]);
             };
-            auto issue_o = [&](int x, bool first) {                            // O_x (+)= P_x V with V tile vc
-                mbar_wait(&p_full[x], pc[x] & 1); ++pc[x];
-                tcgen05_fence_after();
-                const uint32_t b = v_addr0 + (vc % STAGES) * Cfg::TILE_BYTES;
+            auto issue_o = [&](int x, int half, bool first) {                  // O_x (+)= P_x V with 64 keys of V tile vc
+                const uint64_t b = v_desc + (vc % STAGES) * TILE;
 #pragma unroll
-                for (int ks = 0; ks < KV_TILE / 16; ++ks)
-                    umma_bf16_ta(tmem_base + Cfg::O_COL + x * 128, tmem_base + Cfg::S_COL + x * 128 + ks * 8, umma_desc_sw128_mn(b + (uint32_t)(ks * 2048), (uint32_t)Cfg::HALF_BYTES, 1024u),
-                                 idesc_o, (!first || ks > 0) ? 1u : 0u);
+                for (int k4 = 0; k4 < KV_TILE / 32; ++k4) {
+                    const int ks = half * (KV_TILE / 32) + k4;
+                    umma_bf16_ta(tmem_base + Cfg::O_COL + x * 128, tmem_base + Cfg::S_COL + x * 128 + ks * 8, b + (uint64_t)(ks * (2048 >> 4)), idesc_o, (!first || ks > 0) ? 1u : 0u);
+                }
             };
-            for (int r = 0; ptp_item(p, ppg, r, it); ++r) {
+            PtpItem next;
+            bool more = ptp_item(p, ppg, 0, it);
+            for (int r = 0; more; ++r, it = next) {
+                const int n_kvt = __shfl_sync(0xffffffffu, it.n_kvt, 0);
                 mbar_wait(q_full, (uint32_t)r & 1);
                 mbar_wait(&k_full[kc % STAGES], (kc / STAGES) & 1);
                 tcgen05_fence_after();
-                for (int x = 0; x <= it.two; ++x) issue_s(x);
-                umma_commit(&k_empty[kc % STAGES]); ++kc;
-                if (it.n_kvt == 1) umma_commit(q_empty);
-                for (int j = 0; j < it.n_kvt; ++j) {
-                    const bool last = j + 1 == it.n_kvt;
+                if (elect_one()) {
+                    issue_s(0);
+                    if (it.two) issue_s(1);
+                    umma_commit(&k_empty[kc % STAGES]);
+                    if (n_kvt == 1) umma_commit(q_empty);
+                }
+                __syncwarp();
+                ++kc;
+                more = ptp_item(p, ppg, r + 1, next);                          // read now, needed an item later
+                for (int j = 0; j < n_kvt; ++j) {
+                    const bool last = j + 1 == n_kvt;
                     mbar_wait(&v_full[vc % STAGES], (vc / STAGES) & 1);
                     if (!last) mbar_wait(&k_full[kc % STAGES], (kc / STAGES) & 1);
-                    for (int x = 0; x <= it.two; ++x) {
-                        issue_o(x, j == 0);
-                        if (last) umma_commit(&o_full[x]); else issue_s(x);
+#pragma unroll
+                    for (int x = 0; x < 2; ++x) {
+                        if (x > it.two) break;
+                        mbar_wait(&p_full[2 * x], pc[x] & 1);
+                        tcgen05_fence_after();
+                        if (elect_one()) issue_o(x, 0, j == 0);
+                        __syncwarp();
+                        mbar_wait(&p_full[2 * x + 1], pc[x] & 1); ++pc[x];
+                        tcgen05_fence_after();
+                        if (elect_one()) {
+                            issue_o(x, 1, j == 0);
+                            if (last) umma_commit(&o_full[x]); else issue_s(x);
+                        }
+                        __syncwarp();
                     }
-                    umma_commit(&v_empty[vc % STAGES]); ++vc;
-                    if (!last) {
-                        umma_commit(&k_empty[kc % STAGES]); ++kc;
-                        if (j + 2 == it.n_kvt) umma_commit(q_empty);           // the item's last S: the next item's Q may come
+                    if (elect_one()) {
+                        umma_commit(&v_empty[vc % STAGES]);
+                        if (!last) {
+                            umma_commit(&k_empty[kc % STAGES]);
+                            if (j + 2 == n_kvt) umma_commit(q_empty);          // the item's last S: the next item's Q may come
+                        }
                     }
+                    __syncwarp();
+                    ++vc;
+                    if (!last) ++kc;
                 }
             }
         }
@@ -453,8 +545,9 @@ __global__ void __launch_bounds__(PtpCfg<D>::THREADS, 1) prefill_attention_pair_
         const uint64_t scale2 = pack_f32x2(p.scale_log2e, p.scale_log2e);
         griddep_wait();                                             // the output may still be read by a predecessor
         uint32_t sc = 0, oc = 0;                                    // S tiles and items this warpgroup has taken
-        for (int r = 0; ptp_item(p, ppg, r, it); ++r) {
-            if (x > it.two) continue;
+        bool more = ptp_item(p, ppg, 0, it);
+        for (int r = 0; more; ++r) {
+            if (x > it.two) { more = ptp_item(p, ppg, r + 1, it); continue; }
             const int qpos = it.tile.pos0 + row;
             float m_ref = -INFINITY, l_lo = 0.f, l_hi = 0.f;        // row sums of the tiles' lower and upper 64 keys: the order of the kernel above
             for (int j = 0; j < it.n_kvt; ++j, ++sc) {
@@ -499,54 +592,42 @@ __global__ void __launch_bounds__(PtpCfg<D>::THREADS, 1) prefill_attention_pair_
                     if (raise) m_ref = mx;
                 }
                 const uint64_t nref2 = pack_f32x2(-m_ref, -m_ref);
-                uint64_t sum2 = 0ull;                               // the two halves' sums, each in ascending keys
+                float sum[2] = {0.f, 0.f};                          // the two halves' sums, each in ascending keys
 #pragma unroll
-                for (int c = 0; c < 2; ++c) {                       // 32 scores of either half -> 16 columns of P each: p = 2^(s * scale - m_ref)
-                    uint32_t pw[2][16];
+                for (int hf = 0; hf < 2; ++hf) {                    // 64 scores -> 32 columns of P: p = 2^(s * scale - m_ref); handed over as soon as they stand
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        float p0[2], p1[2];
+                    for (int c = 0; c < 2; ++c) {
+                        uint32_t pw[16];
 #pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(v[c + 2 * h][2 * i]), __uint_as_float(v[c + 2 * h][2 * i + 1])), scale2, nref2), p0[h], p1[h]);
-                            p0[h] = ex2_approx(p0[h]); p1[h] = ex2_approx(p1[h]);
-                            pw[h][i] = pack_bf16x2(p0[h], p1[h]);
+                        for (int i = 0; i < 16; ++i) {
+                            float p0, p1;
+                            unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(v[2 * hf + c][2 * i]), __uint_as_float(v[2 * hf + c][2 * i + 1])), scale2, nref2), p0, p1);
+                            p0 = ex2_approx(p0); p1 = ex2_approx(p1);
+                            pw[i] = pack_bf16x2(p0, p1);
+                            sum[hf] += p0; sum[hf] += p1;
                         }
-                        sum2 = add_f32x2(sum2, pack_f32x2(p0[0], p0[1]));
-                        sum2 = add_f32x2(sum2, pack_f32x2(p1[0], p1[1]));
+                        tmem_st_32x32b_x16(s_addr + (uint32_t)((2 * hf + c) * 16), pw);
                     }
-                    tmem_st_32x32b_x16(s_addr + (uint32_t)(c * 16), pw[0]);
-                    tmem_st_32x32b_x16(s_addr + (uint32_t)((c + 2) * 16), pw[1]);
+                    tmem_st_wait();
+                    tcgen05_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&p_full[2 * x + hf]);
                 }
-                tmem_st_wait();
-                tcgen05_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&p_full[x]);
-                float a, b;
-                unpack_f32x2(sum2, a, b);
-                l_lo += a; l_hi += b;
+                l_lo += sum[0]; l_hi += sum[1];
             }
+            PtpItem next;
+            more = ptp_item(p, ppg, r + 1, next);                   // read under the item's last product, needed after its output
             mbar_wait(&o_full[x], oc & 1); ++oc;
             tcgen05_fence_after();
             const float inv = 1.0f / (l_lo + l_hi);
-            uint16_t* orow = reinterpret_cast<uint16_t*>(p.out) + (size_t)(it.tile.q_row0 + row) * p.n_heads * D + (size_t)(it.head + x) * D;
+            uint16_t* orow = reinterpret_cast<uint16_t*>(p.out) + (size_t)(it.tile.q_row0 + q * 32) * p.n_heads * D + (size_t)(it.head + x) * D;
+            // a warp with rows missing: their pieces are few (sixteen prompts of 30 rows: 11.1 us against 12.7 through shared memory)
+            if (D == 64 || it.tile.n_rows < q * 32 + 32) store_o_direct<D>(o_addr, inv, orow + (size_t)lane * p.n_heads * D, row < it.tile.n_rows);
+            else {
 #pragma unroll 1
-            for (int c = 0; c < D; c += 32) {
-                uint32_t o[32];
-                tmem_ld_32x32b_x32(o_addr + (uint32_t)c, o);
-                tmem_ld_wait();
-                if (row < it.tile.n_rows) {
-#pragma unroll
-                    for (int i = 0; i < 32; i += 8) {
-                        uint4 w4;
-                        w4.x = pack_bf16x2(__uint_as_float(o[i]) * inv, __uint_as_float(o[i + 1]) * inv);
-                        w4.y = pack_bf16x2(__uint_as_float(o[i + 2]) * inv, __uint_as_float(o[i + 3]) * inv);
-                        w4.z = pack_bf16x2(__uint_as_float(o[i + 4]) * inv, __uint_as_float(o[i + 5]) * inv);
-                        w4.w = pack_bf16x2(__uint_as_float(o[i + 6]) * inv, __uint_as_float(o[i + 7]) * inv);
-                        *reinterpret_cast<uint4*>(orow + c + i) = w4;
-                    }
-                }
+                for (int c = 0; c < D; c += 64) store_o_64(out_s + (warp - 4) * 4096, o_addr + (uint32_t)c, inv, orow + c, (size_t)p.n_heads * D, lane);
             }
+            it = next;
             tcgen05_fence_before();                                 // O has been read before this warp's next p_full lets P·V overwrite it
         }
     }
@@ -584,8 +665,8 @@ cudaError_t launch_prefill_attention_tc(const CUtensorMap* tm_q, const CUtensorM
     const int grp = p.n_heads / p.n_kv, items = p.n_tiles * p.n_kv * ((grp + 1) / 2);
     const int sms = prefill_sm_count();
     // Up to half as many items as SMs, twice as many single-head CTAs are all resident at once and each is done sooner (32 / 8 heads, 400 rows
-    // behind 6000, 64 items: 97 us against 130 in pairs); above that the pairs win (700 rows behind 4000, 96 items: 125 -> 107 us; 614 rows,
-    // 80 items: 47 -> 46; 1536 rows, 192 items: 76 -> 62).
+    // behind 6000, 64 items: 58 us against 91 in pairs); above that the pairs win (700 rows behind 4000, 96 items: 82 -> 73; 614 rows, 80 items: 14.8
+    // and 14.9; 640 behind 3000, 80 items: 64 -> 59; 850 behind 2000, 112 items: 54 -> 48).
     if (grp > 1 && items > sms / 2) {
         if (kv.head_dim == 128) return launch_ptp<128>(tm_q, tm_kv, kv, p, items, sms, s);
         if (kv.head_dim == 64) return launch_ptp<64>(tm_q, tm_kv, kv, p, items, sms, s);
