@@ -6,6 +6,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <initializer_list>
 #include <string>
 #include <vector>
 
@@ -58,16 +59,47 @@ struct DevBuf {
     DevBuf(const DevBuf&) = delete;
     ~DevBuf() { if (p) cudaFreeAsync(p, s); }
 };
+// Pinned host memory for the arrays of one call: a copy from pageable memory is pushed or staged by the calling thread (6 to 10 us for 8 to 16 KB, against 2
+// to 3 from pinned memory in a loop of its own; six conversations of 1750 tokens: 40.3 -> 38.3 us a call).  A buffer belongs to one call at a time and goes
+// back once the call's stream has passed its copy; a handful of up to 1 MB stay for later calls, everything else is freed at once.  (A kernel that reads
+// the pinned buffer instead of a copy was slower than either for such sizes: it and the attention behind it run one after the other, 41.8 us.)
+struct PinnedPool {
+    static constexpr size_t KEEP_BYTES = 1 << 20, KEEP_BUFFERS = 8;
+    struct Buf { uint8_t* p; size_t cap; };
+    std::mutex mu; Buf kept[KEEP_BUFFERS]; size_t n = 0;
+    Buf take(size_t bytes) {
+        {
+            std::lock_guard<std::mutex> lk(mu);
+            for (size_t i = 0; i < n; ++i) if (kept[i].cap >= bytes) { const Buf b = kept[i]; kept[i] = kept[--n]; return b; }
+        }
+        size_t cap = 64 << 10;
+        while (cap < bytes) cap *= 2;
+        void* p = nullptr;
+        return cudaHostAlloc(&p, cap, cudaHostAllocPortable) == cudaSuccess ? Buf{(uint8_t*)p, cap} : Buf{nullptr, 0};
+    }
+    void give(const Buf& b) {
+        if (b.cap <= KEEP_BYTES) {
+            std::lock_guard<std::mutex> lk(mu);
+            if (n < KEEP_BUFFERS) { kept[n++] = b; return; }
+        }
+        cudaFreeHost(b.p);
+    }
+};
+PinnedPool& pinned_pool() { static PinnedPool* pool = new PinnedPool(); return *pool; }      // never destroyed: the driver may be gone by then
 // Host arrays of one call, packed so that ONE copy brings them to the device (each on a 16-byte boundary)
 struct Packed {
-    std::vector<uint8_t> bytes;
+    PinnedPool::Buf buf; size_t used = 0;
+    explicit Packed(size_t bytes) : buf(pinned_pool().take(bytes)) {}
+    Packed(const Packed&) = delete;
+    ~Packed() { if (buf.p) pinned_pool().give(buf); }
+    size_t reserve(size_t bytes) { const size_t at = (used + 15) & ~size_t(15); used = at + bytes; return at; }
     size_t add(const void* src, size_t n) {
-        const size_t at = (bytes.size() + 15) & ~size_t(15);
-        bytes.resize(at + n);
-        if (n) std::memcpy(bytes.data() + at, src, n);
+        const size_t at = reserve(n);
+        if (n) std::memcpy(buf.p + at, src, n);
         return at;
     }
 };
+size_t packed_bytes(std::initializer_list<size_t> parts) { size_t n = 0; for (size_t p : parts) n += (p + 15) & ~size_t(15); return n; }
 int rc_of(cudaError_t e) { return e == cudaSuccess ? OA_OK : OA_ERR_INTERNAL; }
 }  // namespace
 
@@ -122,19 +154,20 @@ int oa_k_gemm(const void* A, const void* B, int32_t M, int32_t N, int32_t K, int
     p.bias = bias; p.resid = resid; p.ldr = N; p.logits = logits; p.ldl = N;
     if (epilogue == EPI_LOGITS) block_n = gemm_logits_bn(M, N, block_n);
     p.few_rows_ok = 1;
-    if (make_tmap_bf16_2d(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)K, (uint32_t)gemm_a_box(p, epilogue, block_n), 64) != 0) return OA_ERR_INTERNAL;
-    if (make_tmap_bf16_2d(&tmB, B, (uint64_t)N, (uint64_t)K, (uint64_t)K, (uint32_t)gemm_b_box(p, epilogue, block_n), 64) != 0) return OA_ERR_INTERNAL;
+    const GemmChoice choice = gemm_choice(p, epilogue, block_n);
+    if (make_tmap_bf16_2d(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)K, (uint32_t)choice.a_box, 64) != 0) return OA_ERR_INTERNAL;
+    if (make_tmap_bf16_2d(&tmB, B, (uint64_t)N, (uint64_t)K, (uint64_t)K, (uint32_t)choice.b_box, 64) != 0) return OA_ERR_INTERNAL;
     if (epilogue == EPI_LOGITS) {
         const int nt = gemm_n_tiles(N, block_n);
         DevBuf av((size_t)M * nt * 4, s), ai((size_t)M * nt * 4, s);
         if (!av.p || !ai.p) return OA_ERR_INTERNAL;
         p.amax_val = (float*)av.p; p.amax_idx = (int*)ai.p;
-        cudaError_t e = launch_gemm(&tmA, &tmB, p, epilogue, block_n, s);
+        cudaError_t e = launch_gemm(&tmA, &tmB, p, epilogue, block_n, s, &choice);
         if (e == cudaSuccess) e = launch_argmax_reduce(p.amax_val, p.amax_idx, M, nt, argmax_out, nullptr, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         return rc_of(e);
     }
-    return rc_of(launch_gemm(&tmA, &tmB, p, epilogue, block_n, s));
+    return rc_of(launch_gemm(&tmA, &tmB, p, epilogue, block_n, s, &choice));
 }
 
 int oa_k_hybrid_gemm(int32_t mode, const void* A, int32_t lda, const void* B, int32_t ldb, void* C, int32_t ldc, int32_t M, int32_t N, int32_t K, float alpha,
@@ -152,21 +185,23 @@ int oa_k_gemm_ext(const void* A, const void* B, int32_t M, int32_t N, int32_t K,
     if (epilogue == EPI_F32) { p.f32_out = (float*)out; p.ldf = N; p.bias_f32 = (const float*)bias; p.alpha = alpha; p.f32_accumulate = accumulate; }
     else { p.out = out; p.ldo = epilogue == EPI_SWIGLU ? N / 2 : N; p.bias = epilogue == EPI_STORE ? bias : nullptr; }
     if (epilogue == EPI_STORE) { p.store_act = act; p.act_col0 = act_col0; p.act_col1 = act_col1; } else p.glu_gelu = act == 2;
-    if (make_tmap_bf16_2d(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)K, (uint32_t)gemm_a_box(p, epilogue, block_n), 64) != 0) return OA_ERR_INTERNAL;
-    if (make_tmap_bf16_2d(&tmB, B, (uint64_t)N, (uint64_t)K, (uint64_t)K, (uint32_t)gemm_b_box(p, epilogue, block_n), 64) != 0) return OA_ERR_INTERNAL;
-    return rc_of(launch_gemm(&tmA, &tmB, p, epilogue, block_n, (cudaStream_t)stream));
+    const GemmChoice choice = gemm_choice(p, epilogue, block_n);
+    if (make_tmap_bf16_2d(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)K, (uint32_t)choice.a_box, 64) != 0) return OA_ERR_INTERNAL;
+    if (make_tmap_bf16_2d(&tmB, B, (uint64_t)N, (uint64_t)K, (uint64_t)K, (uint32_t)choice.b_box, 64) != 0) return OA_ERR_INTERNAL;
+    return rc_of(launch_gemm(&tmA, &tmB, p, epilogue, block_n, (cudaStream_t)stream, &choice));
 }
 
 int oa_host_gemm_kernel(int32_t M, int32_t N, int32_t K, int32_t epilogue, int32_t block_n, int32_t few_rows, int32_t grouped) {
     GemmParams p{}; p.M = M; p.N = N; p.K = K; p.few_rows_ok = few_rows;
     static const int32_t group = 0;
     if (grouped) p.m_tile_group = &group;
-    return (int)gemm_kernel_of(p, epilogue, block_n);
+    return (int)gemm_choice(p, epilogue, block_n).kernel;
 }
 
 int oa_host_gemm_pair_width(int32_t M, int32_t N, int32_t K, int32_t epilogue, int32_t block_n) {
     GemmParams p{}; p.M = M; p.N = N; p.K = K;
-    return gemm_kernel_of(p, epilogue, block_n) == GEMM_PAIR ? 2 * gemm_b_box(p, epilogue, block_n) : 0;
+    const GemmChoice c = gemm_choice(p, epilogue, block_n);
+    return c.kernel == GEMM_PAIR ? c.width : 0;
 }
 
 static int paged_attention(const void* q, void* out, const void* kv_cache, int32_t num_pages, const int32_t* block_tables,
@@ -181,30 +216,36 @@ static int paged_attention(const void* q, void* out, const void* kv_cache, int32
     const int grp = n_heads / n_kv;
     bool decode = true; int total_q = 0;
     for (int i = 0; i < n_seqs; ++i) { if (q_lens && q_lens[i] != 1) decode = false; total_q += q_lens ? q_lens[i] : 1; }
-    Packed host;
-    const size_t o_bt = host.add(block_tables, (size_t)n_seqs * max_pages_per_seq * 4), o_ctx = host.add(ctx_lens, (size_t)n_seqs * 4);
+    const size_t table_bytes = (size_t)n_seqs * max_pages_per_seq * 4, ctx_bytes = (size_t)n_seqs * 4;
     cudaError_t e;
+    // every path below that has started the copy waits for the stream before the pinned buffer goes back
     if (decode) {
-        DecodePlan plan;
+        static thread_local DecodePlan plan;         // its vectors keep their room from call to call
         build_decode_plan(ctx_lens, n_seqs, n_kv, 2 * 148, force_splits, plan);
-        const size_t o_segs = host.add(plan.segs.data(), plan.segs.size() * sizeof(DecodeSeg)), o_ptr = host.add(plan.cta_ptr.data(), plan.cta_ptr.size() * 4);
-        const std::vector<int32_t> zeros(plan.n_cut + 1, 0);
-        const size_t o_count = host.add(zeros.data(), zeros.size() * 4);         // merge counters: the CTA with an item's last piece merges it
-        const size_t o_po = (host.bytes.size() + 255) & ~size_t(255), o_pml = o_po + (size_t)(plan.n_slots + 1) * grp * head_dim * 4;
+        const size_t seg_bytes = plan.segs.size() * sizeof(DecodeSeg), ptr_bytes = plan.cta_ptr.size() * 4, count_bytes = (size_t)(plan.n_cut + 1) * 4;
+        Packed host(packed_bytes({table_bytes, ctx_bytes, seg_bytes, ptr_bytes, count_bytes}));
+        if (!host.buf.p) return OA_ERR_INTERNAL;
+        const size_t o_bt = host.add(block_tables, table_bytes), o_ctx = host.add(ctx_lens, ctx_bytes);
+        const size_t o_segs = host.add(plan.segs.data(), seg_bytes), o_ptr = host.add(plan.cta_ptr.data(), ptr_bytes);
+        const size_t o_count = host.reserve(count_bytes);                        // merge counters: the CTA with an item's last piece merges it
+        std::memset(host.buf.p + o_count, 0, count_bytes);
+        const size_t o_po = (host.used + 255) & ~size_t(255), o_pml = o_po + (size_t)(plan.n_slots + 1) * grp * head_dim * 4;
         DevBuf d_meta(o_pml + (size_t)(plan.n_slots + 1) * grp * 2 * 4, s);       // [tables, plan, counters | partial outputs | partial maxima and sums]
         if (!d_meta.p) return OA_ERR_INTERNAL;
-        cudaMemcpyAsync(d_meta.p, host.bytes.data(), host.bytes.size(), cudaMemcpyHostToDevice, s);
+        e = cudaMemcpyAsync(d_meta.p, host.buf.p, host.used, cudaMemcpyHostToDevice, s);
         const char* meta = (const char*)d_meta.p;
         DecodeAttnParams a{}; a.q = q; a.out = out; a.block_tables = (const int32_t*)(meta + o_bt); a.ctx_lens = (const int32_t*)(meta + o_ctx);
         a.max_pages_per_seq = max_pages_per_seq; a.segs = (const DecodeSeg*)(meta + o_segs); a.cta_seg_ptr = (const int32_t*)(meta + o_ptr);
         a.n_ctas = (int)plan.cta_ptr.size() - 1; a.part_o = (float*)(meta + o_po); a.part_ml = (float*)(meta + o_pml); a.layer = 0;
         a.n_heads = n_heads; a.n_kv = n_kv; a.scale_log2e = scale_log2e;
         a.merge_counters = (int32_t*)((char*)d_meta.p + o_count);
-        e = launch_decode_attention(&tm, kv, a, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        return rc_of(e);
+        if (e == cudaSuccess) e = launch_decode_attention(&tm, kv, a, s);
+        const cudaError_t done = cudaStreamSynchronize(s);
+        return rc_of(e == cudaSuccess ? done : e);
     }
-    std::vector<PrefillTile> tiles; int row = 0;
+    static thread_local std::vector<PrefillTile> tiles;
+    tiles.clear();
+    int row = 0;
     for (int i = 0; i < n_seqs; ++i) {
         const int ql = q_lens[i], p0 = ctx_lens[i] - ql;
         for (int r = 0; r < ql; r += PREFILL_TILE_ROWS) tiles.push_back(PrefillTile{i, row + r, p0 + r, std::min(PREFILL_TILE_ROWS, ql - r)});
@@ -212,22 +253,22 @@ static int paged_attention(const void* q, void* out, const void* kv_cache, int32
     }
     // the tiles with most keys first, as the engine has them: the causal triangle otherwise ends in a tail of heavy tiles
     std::stable_sort(tiles.begin(), tiles.end(), [](const PrefillTile& x, const PrefillTile& y) { return x.pos0 + x.n_rows > y.pos0 + y.n_rows; });
-    const size_t o_tiles = host.add(tiles.data(), tiles.size() * sizeof(PrefillTile));
-    DevBuf d_meta(host.bytes.size(), s);
+    const size_t tile_bytes = tiles.size() * sizeof(PrefillTile);
+    Packed host(packed_bytes({table_bytes, tile_bytes}));
+    if (!host.buf.p) return OA_ERR_INTERNAL;
+    const size_t o_bt = host.add(block_tables, table_bytes), o_tiles = host.add(tiles.data(), tile_bytes);
+    DevBuf d_meta(host.used, s);
     if (!d_meta.p) return OA_ERR_INTERNAL;
-    cudaMemcpyAsync(d_meta.p, host.bytes.data(), host.bytes.size(), cudaMemcpyHostToDevice, s);
-    const char* meta = (const char*)d_meta.p;
-    PrefillAttnParams a{}; a.q = q; a.out = out; a.block_tables = (const int32_t*)(meta + o_bt); a.max_pages_per_seq = max_pages_per_seq;
-    a.tiles = (const PrefillTile*)(meta + o_tiles); a.n_tiles = (int)tiles.size(); a.layer = 0; a.n_heads = n_heads; a.n_kv = n_kv; a.scale_log2e = scale_log2e;
+    PrefillAttnParams a{}; a.q = q; a.out = out; a.block_tables = (const int32_t*)((const char*)d_meta.p + o_bt); a.max_pages_per_seq = max_pages_per_seq;
+    a.tiles = (const PrefillTile*)((const char*)d_meta.p + o_tiles); a.n_tiles = (int)tiles.size(); a.layer = 0; a.n_heads = n_heads; a.n_kv = n_kv; a.scale_log2e = scale_log2e;
     const char* leg = std::getenv("OA_PREFILL_ATTN");
-    if (leg && std::string(leg) == "legacy") e = launch_prefill_attention(&tm, kv, a, s);
-    else {
-        CUtensorMap tmq;
-        if (make_tmap_bf16_2d(&tmq, q, (uint64_t)total_q, (uint64_t)n_heads * head_dim, (uint64_t)n_heads * head_dim, 128, 64) != 0) return OA_ERR_INTERNAL;
-        e = launch_prefill_attention_tc(&tmq, &tm, kv, a, s);
-    }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    return rc_of(e);
+    const bool legacy = leg && std::string(leg) == "legacy";
+    CUtensorMap tmq;
+    if (!legacy && make_tmap_bf16_2d(&tmq, q, (uint64_t)total_q, (uint64_t)n_heads * head_dim, (uint64_t)n_heads * head_dim, 128, 64) != 0) return OA_ERR_INTERNAL;
+    e = cudaMemcpyAsync(d_meta.p, host.buf.p, host.used, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = legacy ? launch_prefill_attention(&tm, kv, a, s) : launch_prefill_attention_tc(&tmq, &tm, kv, a, s);
+    const cudaError_t done = cudaStreamSynchronize(s);
+    return rc_of(e == cudaSuccess ? done : e);
 }
 int oa_k_paged_attention(const void* q, void* out, const void* kv_cache, int32_t num_pages, const int32_t* block_tables,
                          int32_t max_pages_per_seq, const int32_t* ctx_lens, const int32_t* q_lens, int32_t n_seqs,

@@ -379,7 +379,7 @@ static cudaError_t launch_bn(const CUtensorMap* tmA, const CUtensorMap* tmB, con
 
 static bool persistent_disabled();
 static bool head_persistent(int M, int N);
-static cudaError_t launch_head(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, cudaStream_t stream);
+static cudaError_t launch_head(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int a_rows, cudaStream_t stream);
 static constexpr int HEAD_BN = 128;
 static int sm_count_cached();
 template <int EPI>
@@ -404,7 +404,7 @@ static PairWidth gemm_pair_width(const GemmParams& p, int sms) {
     }
     return best;
 }
-GemmKernel gemm_kernel_of(const GemmParams& p, int epilogue, int block_n) {
+static GemmKernel kernel_of(const GemmParams& p, int epilogue, int block_n, PairWidth& pair) {
     if (block_n != 32 && block_n != 64 && block_n != 128 && block_n != 256) return GEMM_NONE;
     if (p.M <= 0 || p.N <= 0 || p.K <= 0 || (p.N % 8) != 0 || (p.K % 8) != 0) return GEMM_NONE;
     if (epilogue == EPI_SWIGLU && (p.N % 32) != 0) return GEMM_NONE;
@@ -418,7 +418,8 @@ GemmKernel gemm_kernel_of(const GemmParams& p, int epilogue, int block_n) {
         const long long tiles = ceil_div(p.N, block_n) * ceil_div(p.M, BLOCK_M), rounds = ceil_div(tiles, sms);
         const double busy = (double)tiles / (double)(rounds * sms);
         const double per_kb = block_n >= 256 ? 0.22 + 0.27 * busy : block_n == 128 ? 0.17 + 0.13 * busy : 0.15 + 0.07 * busy;
-        if (gemm_pair_width(p, sms).us < (double)(rounds * ceil_div(p.K, BLOCK_K)) * per_kb + (block_n >= 256 ? 10.0 : 7.0)) return GEMM_PAIR;
+        pair = gemm_pair_width(p, sms);
+        if (pair.us < (double)(rounds * ceil_div(p.K, BLOCK_K)) * per_kb + (block_n >= 256 ? 10.0 : 7.0)) return GEMM_PAIR;
     }
     return block_n == 256 && ceil_div(p.N, 256) * ceil_div(p.M, BLOCK_M) >= (forced ? std::atoll(forced) : 2LL * sms) ? GEMM_PERSISTENT : GEMM_TILE;
 }
@@ -428,26 +429,23 @@ static int few_width(int N, int sms) {
     for (int bn : {32, 64}) if (ceil_div(N, bn) <= 2 * sms) return bn;
     return 128;
 }
-int gemm_b_box(const GemmParams& p, int epilogue, int block_n) {
-    switch (gemm_kernel_of(p, epilogue, block_n)) {
-        case GEMM_PAIR: return gemm_pair_width(p, sm_count_cached()).bn / 2;
-        case GEMM_FEW: return few_width(p.N, sm_count_cached());
-        default: return block_n;
-    }
-}
-int gemm_a_box(const GemmParams& p, int epilogue, int block_n) {
-    const GemmKernel k = gemm_kernel_of(p, epilogue, block_n);
-    return k == GEMM_FEW || (k == GEMM_HEAD && p.few_rows_ok && p.M <= FEW_MAX_ROWS) ? few_box(p.M) : 128;
+GemmChoice gemm_choice(const GemmParams& p, int epilogue, int block_n) {
+    PairWidth pair{256, 0.0};
+    GemmChoice c{kernel_of(p, epilogue, block_n, pair), 128, block_n, block_n};
+    if (c.kernel == GEMM_PAIR) { c.width = pair.bn; c.b_box = pair.bn / 2; }
+    if (c.kernel == GEMM_FEW) { c.a_box = few_box(p.M); c.width = c.b_box = few_width(p.N, sm_count_cached()); }
+    if (c.kernel == GEMM_HEAD && p.few_rows_ok && p.M <= FEW_MAX_ROWS) c.a_box = few_box(p.M);
+    return c;
 }
 
 cudaError_t launch_gemm(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epilogue, int block_n,
-                        cudaStream_t stream) {
+                        cudaStream_t stream, const GemmChoice* choice) {
     if (epilogue == EPI_F32 && ((p.ldf % 4) != 0 || !p.f32_out)) return cudaErrorInvalidValue;
-    const GemmKernel kernel = gemm_kernel_of(p, epilogue, block_n);
-    switch (kernel) {
+    const GemmChoice c = choice ? *choice : gemm_choice(p, epilogue, block_n);
+    switch (c.kernel) {
         case GEMM_NONE: return cudaErrorInvalidValue;
-        case GEMM_HEAD: return launch_head(tmA, tmB, p, stream);
-        case GEMM_PAIR: return launch_gemm_pair(tmA, tmB, p, epilogue, gemm_pair_width(p, sm_count_cached()).bn, sm_count_cached(), stream);
+        case GEMM_HEAD: return launch_head(tmA, tmB, p, c.a_box, stream);
+        case GEMM_PAIR: return launch_gemm_pair(tmA, tmB, p, epilogue, c.width, sm_count_cached(), stream);
         case GEMM_PERSISTENT:      // the widest tile over many rows: the epilogue overlaps the next tile
             switch (epilogue) {
                 case EPI_STORE: return launch_persistent<EPI_STORE>(tmA, tmB, p, stream);
@@ -457,7 +455,7 @@ cudaError_t launch_gemm(const CUtensorMap* tmA, const CUtensorMap* tmB, const Ge
             }
             return cudaErrorInvalidValue;
         case GEMM_FEW:
-            switch (few_width(p.N, sm_count_cached())) {
+            switch (c.width) {
                 case 32: return launch_few_bn<32>(tmA, tmB, p, epilogue, stream);
                 case 64: return launch_few_bn<64>(tmA, tmB, p, epilogue, stream);
                 default: return launch_few_bn<128>(tmA, tmB, p, epilogue, stream);
@@ -474,7 +472,7 @@ cudaError_t launch_gemm(const CUtensorMap* tmA, const CUtensorMap* tmB, const Ge
 }
 
 // =============================================================================================
-// persistent tile GEMM (grouped products, and prefill shapes that gemm_kernel_of leaves here): one CTA per SM loops over 128 x 256 tiles in grouped raster order; TMEM holds
+// persistent tile GEMM (grouped products, and prefill shapes that gemm_choice leaves here): one CTA per SM loops over 128 x 256 tiles in grouped raster order; TMEM holds
 // TWO accumulators so the epilogue of tile i (tcgen05.ld -> smem transpose -> coalesced bf16 stores, fused bias /
 // residual / SwiGLU) overlaps the tcgen05.mma main loop of tile i+1.
 // =============================================================================================
@@ -735,11 +733,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_head_kernel(const __grid
     __syncthreads();
     if (warp == 1) { tcgen05_fence_after(); tmem_dealloc<Cfg::TMEM_COLS>(tmem_base); }
 }
-static cudaError_t launch_head(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, cudaStream_t stream) {
+static cudaError_t launch_head(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int a_rows, cudaStream_t stream) {
     static bool attr_done[16] = {};
     { cudaError_t e = ensure_dynamic_smem(gemm_head_kernel, HeadCfg::SMEM_BYTES, attr_done); if (e != cudaSuccess) return e; }
     const int tiles = gemm_n_tiles(p.N, HeadCfg::BN) * ((p.M + BLOCK_M - 1) / BLOCK_M);
-    return launch_k(gemm_head_kernel, dim3(std::min(tiles, sm_count_cached())), dim3(GEMM_THREADS), HeadCfg::SMEM_BYTES, stream, *tmA, *tmB, p, gemm_a_box(p, EPI_LOGITS, HEAD_BN));
+    return launch_k(gemm_head_kernel, dim3(std::min(tiles, sm_count_cached())), dim3(GEMM_THREADS), HeadCfg::SMEM_BYTES, stream, *tmA, *tmB, p, a_rows);
 }
 // the persistent kernel from two rounds of its tiles on; the narrow tiles of a small vocabulary fill the SMs better one CTA each
 static bool head_persistent(int M, int N) { return (long long)gemm_n_tiles(N, HeadCfg::BN) * ((M + BLOCK_M - 1) / BLOCK_M) >= 2LL * sm_count_cached(); }

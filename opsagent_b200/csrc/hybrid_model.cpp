@@ -597,14 +597,14 @@ void HybridModel::gemm(int mode, const void* A, int lda, const Mat& B, void* C, 
     else tc = tc && B.N % 8 == 0 && ldc % 4 == 0 && aligned16(C) && (!bias || aligned16(bias)) && act.kind == 0;
     GemmParams g{}; g.M = M; g.N = up8(B.N); g.K = B.ld; g.few_rows_ok = 1;
     const int bn = pick_tile_n(M, g.N, sm_count), epi = mode == HY_STORE ? EPI_STORE : EPI_F32;
+    const GemmChoice choice = gemm_choice(g, epi, bn);
     CUtensorMap tmA;
-    if (tc && make_tmap_bf16_2d(&tmA, A, (uint64_t)M, (uint64_t)B.ld, (uint64_t)lda, (uint32_t)gemm_a_box(g, epi, bn), 64) != 0) tc = false;
+    if (tc && make_tmap_bf16_2d(&tmA, A, (uint64_t)M, (uint64_t)B.ld, (uint64_t)lda, (uint32_t)choice.a_box, 64) != 0) tc = false;
     if (!tc) { cuda_check(hy_gemm(f32_, mode, A, lda, B.p, B.ld, C, ldc, M, B.N, B.K, bias, alpha, 1, 0, 0, 0, stream, act), "gemm"); return; }
-    const int box = gemm_b_box(g, epi, bn);
-    const CUtensorMap* tmB = &B.tm[gemm_b_box_index(box)];
-    if (mode == HY_STORE) { g.out = C; g.ldo = ldc; g.bias = bias ? bias_act : nullptr; g.store_act = act.kind; g.act_col0 = act.col0; g.act_col1 = act.col1; cuda_check(launch_gemm(&tmA, tmB, g, EPI_STORE, bn, stream), "gemm (tcgen05)"); return; }
+    const CUtensorMap* tmB = &B.tm[gemm_b_box_index(choice.b_box)];
+    if (mode == HY_STORE) { g.out = C; g.ldo = ldc; g.bias = bias ? bias_act : nullptr; g.store_act = act.kind; g.act_col0 = act.col0; g.act_col1 = act.col1; cuda_check(launch_gemm(&tmA, tmB, g, EPI_STORE, bn, stream, &choice), "gemm (tcgen05)"); return; }
     g.f32_out = reinterpret_cast<float*>(C); g.ldf = ldc; g.f32_accumulate = mode == HY_ACC_F32; g.alpha = alpha; g.bias_f32 = bias;
-    cuda_check(launch_gemm(&tmA, tmB, g, EPI_F32, bn, stream), "gemm (tcgen05, fp32 out)");
+    cuda_check(launch_gemm(&tmA, tmB, g, EPI_F32, bn, stream, &choice), "gemm (tcgen05, fp32 out)");
 }
 
 bool HybridModel::moe(const LayerW& w, const HyLayer& l, const void* h_in, const HyRows& r, const std::function<void(int)>& MARK, const int32_t* tokens, float beta) {
@@ -614,10 +614,11 @@ bool HybridModel::moe(const LayerW& w, const HyLayer& l, const void* h_in, const
     const bool relu2 = m.act == HY_EXPERT_RELU2; const int rows1 = relu2 ? w.ffp : 2 * w.ffp;
     if (m.dense && m.act == HY_EXPERT_GELU_GLU) {        // gated: both halves in one product, gelu(gate) * up in its epilogue
         GemmParams g{}; g.M = T; g.N = w.up.N; g.K = w.up.ld; g.out = act_; g.ldo = w.ffp; g.glu_gelu = 1; g.few_rows_ok = 1;
-        const int bn = pick_tile_n(T, g.N, sm_count), box = gemm_b_box(g, EPI_SWIGLU, bn);
+        const int bn = pick_tile_n(T, g.N, sm_count);
+        const GemmChoice choice = gemm_choice(g, EPI_SWIGLU, bn);
         CUtensorMap tmA;
-        if (w.up.tc && make_tmap_bf16_2d(&tmA, h_in, (uint64_t)T, (uint64_t)w.up.ld, (uint64_t)Wld_, (uint32_t)gemm_a_box(g, EPI_SWIGLU, bn), 64) == 0) {
-            cuda_check(launch_gemm(&tmA, &w.up.tm[gemm_b_box_index(box)], g, EPI_SWIGLU, bn, stream), "gated feed-forward (tcgen05)");
+        if (w.up.tc && make_tmap_bf16_2d(&tmA, h_in, (uint64_t)T, (uint64_t)w.up.ld, (uint64_t)Wld_, (uint32_t)choice.a_box, 64) == 0) {
+            cuda_check(launch_gemm(&tmA, &w.up.tm[gemm_b_box_index(choice.b_box)], g, EPI_SWIGLU, bn, stream, &choice), "gated feed-forward (tcgen05)");
         } else {
             if (!glu_) throw std::runtime_error("tensor map for the feed-forward's input failed");
             gemm(HY_STORE, h_in, Wld_, w.up, glu_, ld_glu_, T, nullptr, 1.f);

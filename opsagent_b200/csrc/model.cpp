@@ -356,29 +356,25 @@ void build_decode_plan(const int32_t* ctx_lens, int n_seqs, int n_kv, int n_ctas
     const long long per = (total + n_ctas - 1) / n_ctas;
     n_ctas = (total + per - 1) / per;
     out.cta_ptr.assign((size_t)n_ctas + 1, 0);
-    long long gpos = 0;   // global chunk cursor
-    std::vector<int> cta_of_seg;
-    for (int s = 0; s < n_seqs; ++s) for (int h = 0; h < n_kv; ++h) {
+    // walked along, without a division an item: 128 conversations of 8 key/value heads are a thousand of them, 12.9 us a plan with two each
+    out.segs.reserve((size_t)n_seqs * n_kv + (size_t)n_ctas);      // an item is cut at most once a CTA border
+    long long c = 0, left = per;                                   // CTA at hand and the chunks it still takes
+    for (int s = 0; s < n_seqs; ++s) {
         const int nch = (ctx_lens[s] + 63) / 64; if (nch == 0) continue;
-        const long long g0 = gpos, g1 = gpos + nch;
-        const long long c_first = g0 / per, c_last = (g1 - 1) / per;
-        const int pieces = (int)(c_last - c_first + 1);
-        const int slot0 = out.n_slots, item = out.n_cut;
-        for (long long c = c_first; c <= c_last; ++c) {
-            const long long a = std::max(g0, c * per), b = std::min(g1, (c + 1) * per);
-            DecodeSeg sg{s, h, (int32_t)(a - g0), (int32_t)(b - g0), pieces > 1 ? out.n_slots++ : -1, slot0, pieces, item};
-            out.segs.push_back(sg); cta_of_seg.push_back((int)c);
+        for (int h = 0; h < n_kv; ++h) {
+            int pieces = 1;
+            if (nch > left) pieces += (int)((nch - left + per - 1) / per);
+            const int slot0 = out.n_slots, item = out.n_cut;
+            for (int at = 0; at < nch;) {
+                const int take = (int)std::min<long long>(left, nch - at);
+                out.segs.push_back(DecodeSeg{s, h, at, at + take, pieces > 1 ? out.n_slots++ : -1, slot0, pieces, item});
+                at += take; left -= take;
+                if (left == 0) { out.cta_ptr[(size_t)++c] = (int32_t)out.segs.size(); left = per; }
+            }
+            out.n_cut += pieces > 1;
         }
-        out.n_cut += pieces > 1;
-        gpos = g1;
     }
-    // segs are already ordered by CTA; build the CSR pointer
-    size_t k = 0;
-    for (long long c = 0; c < n_ctas; ++c) {
-        out.cta_ptr[(size_t)c] = (int32_t)k;
-        while (k < cta_of_seg.size() && cta_of_seg[k] == c) ++k;
-    }
-    out.cta_ptr[(size_t)n_ctas] = (int32_t)k;
+    if (left < per) out.cta_ptr[(size_t)++c] = (int32_t)out.segs.size();      // the last CTA, if it takes fewer
 }
 
 void DeviceModel::forward(const StepInput& in, float* logits_out) {
@@ -580,37 +576,41 @@ void DeviceModel::forward(const StepInput& in, float* logits_out) {
                 cuda_check(launch_ar_resid_bf16(comm->d_peer_sym(b), tp, x_, T, H, stream), "allreduce+resid");
             }
         };
+        auto product = [&](const CUtensorMap* a, const WeightMat& w, const GemmParams& g, int epilogue, int bn) {
+            const GemmChoice c = gemm_choice(g, epilogue, bn);
+            return launch_gemm(a, w.map(c.b_box), g, epilogue, bn, stream, &c);
+        };
         const int bn_qkv = pick_bn(T, qkvd, opt.bn_qkv, false), bn_o = pick_bn(T, H, opt.bn_o, false);
         const int bn_gu = pick_bn(T, 2 * F, opt.bn_gu, true), bn_down = pick_bn(T, H, opt.bn_down, false);
         for (int l = 0; l < L; ++l) {
             const Layer& ly = layers[l];
             cuda_check(launch_rmsnorm(x_, ly.ln1, xn_, T, H, cfg.rms_eps, stream), "rmsnorm1"); MARK(1);
             GemmParams g{}; g.M = T; g.N = qkvd; g.K = H; g.out = qkv_; g.ldo = qkvd; g.bias = ly.bqkv;
-            cuda_check(launch_gemm(&tm_xn_, ly.qkv.map(gemm_b_box(g, EPI_STORE, bn_qkv)), g, EPI_STORE, bn_qkv, stream), "qkv gemm"); MARK(2);
+            cuda_check(product(&tm_xn_, ly.qkv, g, EPI_STORE, bn_qkv), "qkv gemm"); MARK(2);
             cuda_check(launch_rope_kv_write(qkv_, d_pos, d_slot, rope_cos, rope_sin, q_, kv, l, T, nh, stream), "rope"); MARK(3);
             attention(l);
             if (use_tp) {      // bf16 partial -> symmetric buffer, barrier, x += sum over ranks (rank order)
                 const int b = comm->next_buffer();
                 GemmParams go{}; go.M = T; go.N = H; go.K = qd; go.out = comm->sym(b); go.ldo = H;
-                cuda_check(launch_gemm(&tm_attn_, ly.o.map(gemm_b_box(go, EPI_STORE, bn_o)), go, EPI_STORE, bn_o, stream), "o gemm"); MARK(6);
+                cuda_check(product(&tm_attn_, ly.o, go, EPI_STORE, bn_o), "o gemm"); MARK(6);
                 cuda_check(comm->barrier(stream), "xgpu barrier");
                 allreduce_resid_bf16(b);
             } else {
                 GemmParams go{}; go.M = T; go.N = H; go.K = qd; go.out = x_; go.ldo = H; go.resid = x_; go.ldr = H;
-                cuda_check(launch_gemm(&tm_attn_, ly.o.map(gemm_b_box(go, EPI_RESID, bn_o)), go, EPI_RESID, bn_o, stream), "o gemm"); MARK(6);
+                cuda_check(product(&tm_attn_, ly.o, go, EPI_RESID, bn_o), "o gemm"); MARK(6);
             }
             cuda_check(launch_rmsnorm(x_, ly.ln2, xn_, T, H, cfg.rms_eps, stream), "rmsnorm2"); MARK(1);
             GemmParams gg{}; gg.M = T; gg.N = 2 * F; gg.K = H; gg.out = act_; gg.ldo = F;
-            cuda_check(launch_gemm(&tm_xn_, ly.gu.map(gemm_b_box(gg, EPI_SWIGLU, bn_gu)), gg, EPI_SWIGLU, bn_gu, stream), "gate_up gemm"); MARK(8);
+            cuda_check(product(&tm_xn_, ly.gu, gg, EPI_SWIGLU, bn_gu), "gate_up gemm"); MARK(8);
             if (use_tp) {
                 const int b = comm->next_buffer();
                 GemmParams gd{}; gd.M = T; gd.N = H; gd.K = F; gd.out = comm->sym(b); gd.ldo = H;
-                cuda_check(launch_gemm(&tm_act_, ly.down.map(gemm_b_box(gd, EPI_STORE, bn_down)), gd, EPI_STORE, bn_down, stream), "down gemm"); MARK(10);
+                cuda_check(product(&tm_act_, ly.down, gd, EPI_STORE, bn_down), "down gemm"); MARK(10);
                 cuda_check(comm->barrier(stream), "xgpu barrier");
                 allreduce_resid_bf16(b);
             } else {
                 GemmParams gd{}; gd.M = T; gd.N = H; gd.K = F; gd.out = x_; gd.ldo = H; gd.resid = x_; gd.ldr = H;
-                cuda_check(launch_gemm(&tm_act_, ly.down.map(gemm_b_box(gd, EPI_RESID, bn_down)), gd, EPI_RESID, bn_down, stream), "down gemm"); MARK(10);
+                cuda_check(product(&tm_act_, ly.down, gd, EPI_RESID, bn_down), "down gemm"); MARK(10);
             }
         }
     }
@@ -636,8 +636,8 @@ void DeviceModel::forward(const StepInput& in, float* logits_out) {
                 lb = comm->next_buffer(); gl.logits = reinterpret_cast<float*>(comm->sym(lb)); gl.ldl = V;
             }
         }
-        const int lm_rows = gemm_a_box(gl, EPI_LOGITS, bn_lm);
-        cuda_check(launch_gemm(lm_rows == 128 ? &tm_xsn_ : &tm_few_xsn_[lm_rows >> 5], lm_head.map(bn_lm), gl, EPI_LOGITS, bn_lm, stream), "lm_head gemm"); MARK(12);
+        const GemmChoice lm = gemm_choice(gl, EPI_LOGITS, bn_lm);
+        cuda_check(launch_gemm(lm.a_box == 128 ? &tm_xsn_ : &tm_few_xsn_[lm.a_box >> 5], lm_head.map(bn_lm), gl, EPI_LOGITS, bn_lm, stream, &lm), "lm_head gemm"); MARK(12);
         if (use_tp) {
             const int b = comm->next_buffer();
             cuda_check(launch_argmax_reduce_pair(amax_val_, amax_idx_, S, n_tiles, tp_rank * V, comm->arg(b), stream), "argmax (local shard)");

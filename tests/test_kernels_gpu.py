@@ -332,6 +332,47 @@ def test_paged_decode_attention_merges_many_pieces(L, ctx, nh, nkv, D):
     assert (out.float() - ref).abs().max().item() < 2 * 3 * 2.0 ** -8
 
 
+def test_attention_calls_of_several_threads(L):
+    """calls of different sizes at once, each on a stream of its own: none sees another's tables (one of the tables is larger than what is kept between calls)"""
+    import threading
+    nh, nkv, D = 32, 8, 128
+    jobs = []
+    for k, (ctx, qlens, maxp) in enumerate([([70, 300, 5], None, 8), ([1000] * 40, None, 20), ([130, 64], [130, 10], 4), ([400, 90, 33], [33, 90, 1], 150000)]):
+        n, pages = len(ctx), sum((c + 63) // 64 for c in ctx)
+        kv = _mk_cache(pages, nkv, D, 30 + k)
+        bt = np.zeros((n, maxp), np.int32); at = 0
+        for i, c in enumerate(ctx):
+            npg = (c + 63) // 64; bt[i, :npg] = np.arange(at, at + npg)[::-1]; at += npg
+        q = torch.randn(sum(qlens or [1] * n), nh, D, generator=torch.Generator(device="cpu").manual_seed(k)).to(torch.bfloat16).to(dev())
+        jobs.append((q, kv, pages, bt, maxp, np.array(ctx, np.int32), np.array(qlens, np.int32) if qlens else None, n))
+
+    def attend(job, out, stream):
+        q, kv, pages, bt, maxp, ctx, ql, n = job
+        return L.oa_k_paged_attention(ptr(q), ptr(out), ptr(kv), pages, bt.ctypes.data, maxp, ctx.ctypes.data, ql.ctypes.data if ql is not None else None, n, nh, nkv, D, 0, stream)
+
+    want = []
+    for job in jobs:
+        out = torch.empty_like(job[0]); assert attend(job, out, None) == 0; want.append(out)
+    bad = []
+
+    def work(t):
+        stream = torch.cuda.Stream()
+        for r in range(20):
+            k = (t + r) % len(jobs)
+            out = torch.full_like(jobs[k][0], float("nan"))
+            stream.wait_stream(torch.cuda.current_stream())
+            rc = attend(jobs[k], out, C.c_void_p(stream.cuda_stream))
+            if rc != 0 or not torch.equal(out, want[k]):
+                bad.append((t, r, k, rc))
+
+    threads = [threading.Thread(target=work, args=(t,)) for t in range(6)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad, bad[:5]
+
+
 def test_streamk_result_on_any_float_boundary(L):
     M, N, K = 37, 1000, 320
     g = torch.Generator(device="cpu").manual_seed(1)
