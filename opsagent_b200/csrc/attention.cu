@@ -89,10 +89,11 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) decode_attention_kernel(const 
                 const DecodeSeg sg = p.segs[si];
                 const int32_t* bt = p.block_tables + (size_t)sg.seq * p.max_pages_per_seq;
                 const int mutable_chunk = (p.ctx_lens[sg.seq] - 1) / PAGE;
+                int page = bt[sg.chunk_begin];
                 for (int c = sg.chunk_begin; c < sg.chunk_end; ++c) {
+                    const int next_page = c + 1 < sg.chunk_end ? bt[c + 1] : 0;      // looked up while this one's slot is waited for
                     if (!waited && (issued >= STAGES || c >= mutable_chunk)) { griddep_wait(); waited = true; }
                     ++issued;
-                    const int page = bt[c];
                     mbar_wait(&empty_bar[s], ph ^ 1);
                     uint8_t* kdst = smem + s * Cfg::STAGE_BYTES;
                     uint8_t* vdst = kdst + Cfg::KV_BYTES;
@@ -104,6 +105,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) decode_attention_kernel(const 
                         tma_load_2d(kdst + h * Cfg::TILE_BYTES, &tm_kv, &full_bar[s], h * 64, (int32_t)krow, kEvictFirst);
                         tma_load_2d(vdst + h * Cfg::TILE_BYTES, &tm_kv, &full_bar[s], h * 64, (int32_t)vrow, kEvictFirst);
                     }
+                    page = next_page;
                     if (++s == STAGES) { s = 0; ph ^= 1; }
                 }
             }
@@ -239,42 +241,61 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) decode_attention_kernel(const 
             }
             if (sg.partial_slot >= 0) {
                 // flash-decoding merge without a second kernel: the CTA that finishes an item's LAST piece combines all pieces.
-                // Counters advance by n_pieces per layer and start each step at zero, so "last" is a multiple of n_pieces.
-                __threadfence();
+                // Counters advance by n_pieces per layer and start each step at zero, so "last" is a multiple of n_pieces.  What is written before has
+                // to be seen by whoever counts later, no more: an acquire-release fence, of one lane for its warp.
                 __syncwarp();
-                if (lane == 0 && ((atomicAdd(p.merge_counters + sg.item, 1) + 1) % sg.n_pieces) == 0) { __threadfence(); const int n = merge_s[0]; merge_s[1 + n] = si; merge_s[0] = n + 1; }
+                if (lane == 0) fence_acq_rel_gpu();
+                if (lane == 0 && ((atomicAdd(p.merge_counters + sg.item, 1) + 1) % sg.n_pieces) == 0) { fence_acq_rel_gpu(); const int n = merge_s[0]; merge_s[1 + n] = si; merge_s[0] = n + 1; }
             }
         }
         named_bar_sync(1, 128);   // scratch free for the next segment
     }
     // Merges this CTA came last for: at most its first and its last segment belong to cut items.  The four warps take a quarter of the columns each
-    // (lane: head g, NC consecutive columns from t * NC of the quarter), pieces in slot order (deterministic), four pieces' loads in flight: a context
-    // cut over the whole chip has up to 37 pieces per item, and one warp reading them one after the other was as long as the attention itself
-    // (one sequence of 3000 tokens, 32 / 8 heads: 22.5 -> 17.5 us a layer).
-    constexpr int NC = D / 16;                               // columns per lane: 8 (D = 128) or 4
+    // (lane: head g, NC consecutive columns from t * NC of the quarter), pieces in slot order (deterministic), eight pieces' loads in flight: a context
+    // cut over the whole chip has up to 37 pieces per item, and one warp reading them one after the other was as long as the attention itself.  The
+    // maximum over the pieces comes from the head's four lanes, a quarter of them each, under the first pieces' loads.  us a layer, before the lighter
+    // fences and this order of the merge -> now: 6 x 1750 tokens (heads of 64) 12.5 -> 11.5, 32 x 100 10.9 -> 10.4, 16 x 900 (40 heads) 17.7 -> 16.6, 32 x 1500
+    // 36.8 -> 36.2, 1 x 17000 21.7 -> 21.1, 128 x 1664 135 and 135.  (One record of 48 bytes a CTA instead of offsets, segment, length and page read one
+    // after the other starts 0.3 us sooner and costs a call's copy more than that.)
+    constexpr int NC = D / 16, MP = 8;       // columns per lane: 8 (D = 128) or 4; pieces read at a time
     const int n_merge = merge_s[0];
-    if (n_merge > 0) __threadfence();
+    if (n_merge > 0) fence_acq_rel_gpu();
     for (int k = 0; k < n_merge; ++k) {
         const DecodeSeg sg = p.segs[merge_s[1 + k]];
-        if (g >= grp) continue;
-        const float* ml = p.part_ml + ((size_t)sg.slot_begin * grp + g) * 2;
-        const float* po = p.part_o + ((size_t)sg.slot_begin * grp + g) * D + warp * (D / 4) + t * NC;
+        const int gg = g < grp ? g : 0;                      // lanes beyond the group's heads go along for the shuffles
+        const float* ml = p.part_ml + ((size_t)sg.slot_begin * grp + gg) * 2;
+        const float* po = p.part_o + ((size_t)sg.slot_begin * grp + gg) * D + warp * (D / 4) + t * NC;
+        float2 st[MP]; float4 u[MP][NC / 4];
+        auto load = [&](int i0) {
+#pragma unroll
+            for (int i = 0; i < MP; ++i) {
+                if (i0 + i >= sg.n_pieces) break;
+                st[i] = __ldcg(reinterpret_cast<const float2*>(ml + (size_t)(i0 + i) * grp * 2));
+#pragma unroll
+                for (int c = 0; c < NC / 4; ++c) u[i][c] = __ldcg(reinterpret_cast<const float4*>(po + (size_t)(i0 + i) * grp * D) + c);
+            }
+        };
+        load(0);
         float m_all = -INFINITY;
-        for (int i = 0; i < sg.n_pieces; ++i) m_all = fmaxf(m_all, __ldcg(ml + (size_t)i * grp * 2));
+#pragma unroll 4
+        for (int i = t; i < sg.n_pieces; i += 4) m_all = fmaxf(m_all, __ldcg(ml + (size_t)i * grp * 2));
+        m_all = fmaxf(m_all, __shfl_xor_sync(0xffffffffu, m_all, 1));
+        m_all = fmaxf(m_all, __shfl_xor_sync(0xffffffffu, m_all, 2));
         float l_all = 0.f, o[NC];
 #pragma unroll
         for (int c = 0; c < NC; ++c) o[c] = 0.f;
-#pragma unroll 4
-        for (int i = 0; i < sg.n_pieces; ++i) {
-            const float2 st = __ldcg(reinterpret_cast<const float2*>(ml + (size_t)i * grp * 2));
-            float4 u[NC / 4];
+        for (int i0 = 0; i0 < sg.n_pieces; i0 += MP) {
+            if (i0 > 0) load(i0);
 #pragma unroll
-            for (int c = 0; c < NC / 4; ++c) u[c] = __ldcg(reinterpret_cast<const float4*>(po + (size_t)i * grp * D) + c);
-            const float f = exp2f(st.x - m_all);
-            l_all += f * st.y;
+            for (int i = 0; i < MP; ++i) {
+                if (i0 + i >= sg.n_pieces) break;
+                const float f = exp2f(st[i].x - m_all);
+                l_all += f * st[i].y;
 #pragma unroll
-            for (int c = 0; c < NC / 4; ++c) { o[4 * c] += f * u[c].x; o[4 * c + 1] += f * u[c].y; o[4 * c + 2] += f * u[c].z; o[4 * c + 3] += f * u[c].w; }
+                for (int c = 0; c < NC / 4; ++c) { o[4 * c] += f * u[i][c].x; o[4 * c + 1] += f * u[i][c].y; o[4 * c + 2] += f * u[i][c].z; o[4 * c + 3] += f * u[i][c].w; }
+            }
         }
+        if (g >= grp) continue;
         const float inv = 1.0f / l_all;
         uint32_t* orow = reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(p.out) + (size_t)sg.seq * p.n_heads * D + (size_t)(sg.kvh * grp + g) * D + warp * (D / 4) + t * NC);
 #pragma unroll

@@ -63,6 +63,7 @@ OA_DEVINL void mbar_init(uint64_t* bar, uint32_t count) {
 OA_DEVINL void fence_barrier_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 OA_DEVINL void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 OA_DEVINL void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }    // generic-proxy global writes -> later TMA (async proxy) reads
+OA_DEVINL void fence_acq_rel_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }      // lighter than __threadfence(), which is sequentially consistent
 // grid-wide counter barrier for persistent kernels whose CTAs are all co-resident (grid <= SM count, one CTA per SM)
 OA_DEVINL unsigned long long ld_acquire_gpu_u64(const unsigned long long* p) {
     unsigned long long v;
