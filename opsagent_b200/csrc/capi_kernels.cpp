@@ -221,7 +221,7 @@ static int paged_attention(const void* q, void* out, const void* kv_cache, int32
     // every path below that has started the copy waits for the stream before the pinned buffer goes back
     if (decode) {
         static thread_local DecodePlan plan;         // its vectors keep their room from call to call
-        build_decode_plan(ctx_lens, n_seqs, n_kv, 2 * 148, force_splits, plan);
+        plan_decode_attention(ctx_lens, n_seqs, n_kv, 2 * 148, force_splits, plan);
         const size_t seg_bytes = plan.segs.size() * sizeof(DecodeSeg), ptr_bytes = plan.cta_ptr.size() * 4, count_bytes = (size_t)(plan.n_cut + 1) * 4;
         Packed host(packed_bytes({table_bytes, ctx_bytes, seg_bytes, ptr_bytes, count_bytes}));
         if (!host.buf.p) return OA_ERR_INTERNAL;

@@ -377,6 +377,29 @@ void build_decode_plan(const int32_t* ctx_lens, int n_seqs, int n_kv, int n_ctas
     if (left < per) out.cta_ptr[(size_t)++c] = (int32_t)out.segs.size();      // the last CTA, if it takes fewer
 }
 
+// A CTA that shares an item waits for its partials to be written, counted and read back, 3 to 5 us; a chunk of 64 tokens more takes 0.3 to 0.5 us as long as
+// memory is not the bound.  So where every item can have a CTA of its own and the longest is at most 8 chunks (16 from 64 items on, whose merges hold each
+// other up) above an equal share, none is cut.  us a layer, cut -> whole, 32 / 8 heads of 128: 1 x 500 tokens 6.8 -> 5.8, 32 x 40 .. 156 10.7 -> 6.5,
+// 16 x 500 12.0 -> 8.2, 32 x 700 19.0 -> 14.8, 8 x 1000 12.3 -> 11.2, 37 x 1500 31.2 -> 29.0; beyond the line 1 x 1000 7.2 -> 8.4, 1 x 1500 8.0 -> 11.1.
+void plan_decode_attention(const int32_t* ctx_lens, int n_seqs, int n_kv, int n_ctas_target, int force_splits, DecodePlan& out) {
+    long long live = 0, total = 0, longest = 0;
+    for (int i = 0; i < n_seqs; ++i) {
+        const long long nch = (ctx_lens[i] + 63) / 64;
+        if (nch > 0) { ++live; total += nch * n_kv; longest = std::max(longest, nch); }
+    }
+    const long long items = live * n_kv, share_ctas = std::min<long long>(n_ctas_target, std::max<long long>(1, total / 2));
+    if (force_splits > 0 || items == 0 || items > n_ctas_target || longest > (total + share_ctas - 1) / share_ctas + (items >= 64 ? 16 : 8)) {
+        build_decode_plan(ctx_lens, n_seqs, n_kv, n_ctas_target, force_splits, out);
+        return;
+    }
+    out.segs.clear(); out.cta_ptr.clear(); out.n_slots = 0; out.n_cut = 0;
+    for (int s = 0; s < n_seqs; ++s) {
+        const int nch = (ctx_lens[s] + 63) / 64; if (nch <= 0) continue;
+        for (int h = 0; h < n_kv; ++h) { out.cta_ptr.push_back((int32_t)out.segs.size()); out.segs.push_back(DecodeSeg{s, h, 0, nch, -1, 0, 1, 0}); }
+    }
+    out.cta_ptr.push_back((int32_t)out.segs.size());
+}
+
 void DeviceModel::forward(const StepInput& in, float* logits_out) {
     const int T = (int)in.tokens.size(), S = (int)in.sample_rows.size();
     // all projection sizes below are this rank's shard (== the global sizes when tp == 1)
@@ -410,7 +433,7 @@ void DeviceModel::forward(const StepInput& in, float* logits_out) {
     if (n_dec < 0 || n_dec > in.n_seqs || n_dec > T) throw std::runtime_error("forward: bad n_decode");
     if (n_dec > 0) {
         const int n_ctas = opt.attn_ctas > 0 ? opt.attn_ctas : 2 * sm_count;
-        build_decode_plan(in.ctx_lens.data(), n_dec, nkv, n_ctas, 0, plan_);
+        plan_decode_attention(in.ctx_lens.data(), n_dec, nkv, n_ctas, 0, plan_);
         if (plan_.n_slots > max_part_slots_) throw std::runtime_error("forward: partial workspace overflow");
         o_segs = put(plan_.segs.data(), plan_.segs.size() * 8);
         o_ptr = put(plan_.cta_ptr.data(), plan_.cta_ptr.size());

@@ -332,6 +332,28 @@ def test_paged_decode_attention_merges_many_pieces(L, ctx, nh, nkv, D):
     assert (out.float() - ref).abs().max().item() < 2 * 3 * 2.0 ** -8
 
 
+# one CTA an item or items cut over CTAs: batches on both sides of the line (an equal share of 2 chunks + 8, + 16 from 64 items on; one item more than CTAs)
+@pytest.mark.parametrize("D", [128, 64])
+@pytest.mark.parametrize("nh,nkv,ctx", [(8, 1, [640]), (8, 1, [641]), (32, 8, [640] * 2 + [1]), (32, 8, [1] * 7 + [1152]), (32, 8, [1] * 7 + [1153]), (32, 8, [640] + [3] * 6), (32, 8, [641] + [3] * 6),
+                                        (32, 8, [70, 300, 5, 129] * 9 + [64]), (32, 8, [70, 300, 5, 129] * 9 + [64, 65]), (12, 4, list(range(1, 741, 10)))])
+def test_decode_attention_whole_items_and_cut_ones(L, nh, nkv, D, ctx):
+    n = len(ctx); maxp = (max(ctx) + 63) // 64; num_pages = sum((c + 63) // 64 for c in ctx)
+    kv = _mk_cache(num_pages, nkv, D, 19)
+    g = torch.Generator(device="cpu").manual_seed(8)
+    perm = torch.randperm(num_pages, generator=g)
+    bt = torch.zeros(n, maxp, dtype=torch.int32); k = 0
+    for i, c in enumerate(ctx):
+        npg = (c + 63) // 64; bt[i, :npg] = perm[k:k + npg].to(torch.int32); k += npg
+    q = (torch.randn(n, nh, D, generator=g) * 2).to(torch.bfloat16).to(dev())
+    out = torch.full((n, nh, D), float("nan"), dtype=torch.bfloat16, device=dev())
+    ctx_a = np.array(ctx, np.int32); bt_np = np.ascontiguousarray(bt.numpy())
+    for _ in range(2):
+        assert L.oa_k_paged_attention(ptr(q), ptr(out), ptr(kv), num_pages, bt_np.ctypes.data, maxp, ctx_a.ctypes.data, None, n, nh, nkv, D, 0, None) == 0, _lib.last_error()
+    ref = _attn_ref(q, kv[0], kv[1], bt.to(dev()).long(), ctx, [1] * n, nh, nkv, D)
+    # probabilities and result are rounded to bf16 (2^-9 relative each); a mean of unit normals weighted by them stays below 4.5, alone (one token) or not
+    assert (out.float() - ref).abs().max().item() < 2 * 4.5 * 2.0 ** -8
+
+
 def test_attention_calls_of_several_threads(L):
     """calls of different sizes at once, each on a stream of its own: none sees another's tables (one of the tables is larger than what is kept between calls)"""
     import threading
