@@ -404,13 +404,15 @@ struct FewArgs {
 constexpr int FEW_RPT = 16;      // state rows per thread: dim <= 8 * 16
 template <bool DELTA>
 __global__ void __launch_bounds__(256) hy_few_memory_kernel(FewArgs f, HyRows r) {
-    HY_PDL();
+    // The state was written in an earlier step and the rows' metadata copied in ahead of this one: both are read before the wait, under the projection that
+    // makes the rows' operands.
+    griddep_launch();
     const BlockArgs& p = f.p;
     __shared__ __align__(16) float qs[BM_FEW][128], ks[BM_FEW][128], vs[BM_FEW][128], part[8][128], po[2][8][128];
     __shared__ float gb[BM_FEW][2];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, seq = blockIdx.x, h = blockIdx.y, D = p.D, VD = p.VD;
     const long long row0 = r.seq_row0[seq]; const int len = r.seq_row0[seq + 1] - (int)row0, pos0 = r.seq_pos0[seq], slot = r.seq_state[seq];
-    if (len > BM_FEW) return;                            // the block form takes this sequence
+    if (len > BM_FEW) { griddep_wait(); return; }        // the block form takes this sequence
     const int qh = h / (p.H / p.QH), c4 = lane * 4; const bool ok = c4 < VD;
     float* st = p.state + (((long long)slot * p.H + h) * D) * VD;
     float4 S[FEW_RPT];
@@ -419,6 +421,7 @@ __global__ void __launch_bounds__(256) hy_few_memory_kernel(FewArgs f, HyRows r)
         const int d = warp + 8 * i;
         S[i] = (pos0 > 0 && ok && d < D) ? *reinterpret_cast<const float4*>(st + (long long)d * VD + c4) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
+    griddep_wait();
     const int n = 2 * D + VD;
     for (int i = tid; i < len * n; i += 256) {
         const int t = i / n, c = i - t * n;

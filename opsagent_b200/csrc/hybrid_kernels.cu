@@ -207,8 +207,8 @@ __global__ void __launch_bounds__(256) hy_layernorm_kernel(const float* x, const
 // latent attention
 // ---------------------------------------------------------------------------------------------------------------------------------
 template <typename TA>
-__global__ void __launch_bounds__(128) hy_mla_prep_kernel(HyLatentAttn a, const TA* q, int ldq, const TA* ckv, int ldc, const float* norm_w, float eps,
-                                                           const float* rope_cos, const float* rope_sin, TA* cache, float* q_abs, HyRows r) {
+__global__ void __launch_bounds__(128) hy_mla_prep_kernel(HyLatentAttn a, const TA* __restrict__ q, int ldq, const TA* __restrict__ ckv, int ldc, const float* __restrict__ norm_w, float eps,
+                                                           const float* __restrict__ rope_cos, const float* __restrict__ rope_sin, TA* __restrict__ cache, float* __restrict__ q_abs, HyRows r) {
     HY_PDL();
     __shared__ float red[32];
     const int t = blockIdx.x, R = a.kv_rank, rot = a.rot_dim, half = a.rot_dims / 2, E = R + rot;
@@ -229,7 +229,8 @@ __global__ void __launch_bounds__(128) hy_mla_prep_kernel(HyLatentAttn a, const 
         } else v = ldf(c + R + i);
         stf(dst + R + i, v);
     }
-    for (int i = threadIdx.x; i < a.heads * rot; i += blockDim.x) {   // rotated query parts
+#pragma unroll 4
+    for (int i = threadIdx.x; i < a.heads * rot; i += blockDim.x) {   // rotated query parts (no array here overlaps another: several of these in flight)
         const int h = i / rot, d = i - h * rot; const TA* qh = q + (long long)t * ldq + (long long)h * (a.dim + rot) + a.dim;
         float v;
         if (d < 2 * half) {
@@ -451,7 +452,8 @@ static size_t mla_decode_smem(int E, int nvb, int stages) {
 template <int NVB, int STAGES>
 __global__ void __launch_bounds__(128) hy_mla_decode_mma_kernel(HyLatentAttn a, const float* __restrict__ q_abs, const __nv_bfloat16* __restrict__ cache,
                                                                 __nv_bfloat16* __restrict__ lat_out, HyRows r, const int32_t* __restrict__ tile_seq, HyMlaSplit sp) {
-    HY_PDL();
+    // lookups and cache rows of earlier steps before the wait, under the kernels that make this step's query and cache row
+    griddep_launch();
     extern __shared__ __align__(16) uint8_t mla_smem[];
     const int R = a.kv_rank, E = R + a.rot_dim, EP = E + 8, H = a.heads;
     __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(mla_smem);      // [16][EP]
@@ -482,7 +484,10 @@ __global__ void __launch_bounds__(128) hy_mla_decode_mma_kernel(HyLatentAttn a, 
         for (int j = n; j < 16; ++j) for (int c = lane; c < E / 8; c += 32) *reinterpret_cast<uint4*>(dst + j * EP + c * 8) = make_uint4(0, 0, 0, 0);
         __syncwarp();
     };
-    for (int s = 0; s < STAGES; ++s) if (g_begin + 4 * s < g_end) issue(g_begin + 4 * s, s);
+    auto older = [&](int g) { return min(last, g * 16 + 15) < pos; };      // not one row of the group is of this step (a decoding row: its own)
+    for (int s = 0; s < STAGES; ++s) if (g_begin + 4 * s < g_end && older(g_begin + 4 * s)) issue(g_begin + 4 * s, s);
+    griddep_wait();
+    for (int s = 0; s < STAGES; ++s) if (g_begin + 4 * s < g_end && !older(g_begin + 4 * s)) issue(g_begin + 4 * s, s);
     const float qscale = a.scale * 1.4426950408889634f;
     const int e4 = E / 4;
 #pragma unroll 6
@@ -1163,10 +1168,17 @@ __global__ void __launch_bounds__(128) hy_gated_norm_warp_kernel(const float* __
 template <typename TA, int NV>      // NV x 4 channels per thread: group <= 1024 NV
 __global__ void __launch_bounds__(256) hy_gated_norm_wide_kernel(const float* __restrict__ o, int C, int group, const float* __restrict__ w, int wlen, const TA* __restrict__ gate, int ld_gate, int act,
                                                                  TA* __restrict__ out, int ld_out, float eps) {
-    HY_PDL();
+    griddep_launch();
     __shared__ float red[32];
     const long long t = blockIdx.x; const int c0 = blockIdx.y * group;
-    float v[NV][4], g[NV][4], ss = 0.f;
+    float v[NV][4], g[NV][4], wv[NV][4], ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {                       // weights ahead of the wait
+        const int i = (threadIdx.x + k * 256) * 4;
+        wv[k][0] = wv[k][1] = wv[k][2] = wv[k][3] = 1.f;
+        if (w && i < group) ld4(w + (wlen == group ? i : c0 + i), wv[k]);
+    }
+    griddep_wait();
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
         const int i = (threadIdx.x + k * 256) * 4;
@@ -1181,11 +1193,9 @@ __global__ void __launch_bounds__(256) hy_gated_norm_wide_kernel(const float* __
     for (int k = 0; k < NV; ++k) {
         const int i = (threadIdx.x + k * 256) * 4;
         if (i >= group) continue;
-        float wv[4] = {1.f, 1.f, 1.f, 1.f};
-        if (w) ld4(w + (wlen == group ? i : c0 + i), wv);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            v[k][e] *= rr * wv[e];
+            v[k][e] *= rr * wv[k][e];
             if (gate) v[k][e] *= act ? silu_for(g[k][e], out) : sigmoid_for(g[k][e], out);
         }
         st4(out + t * ld_out + c0 + i, v[k]);

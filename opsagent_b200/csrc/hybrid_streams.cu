@@ -211,9 +211,13 @@ __device__ __forceinline__ FVec<V> branch_add(const HyBranch& b, long long src, 
 template <typename TA, int NV>      // NV float4 per thread: W <= 1024 NV
 __global__ void __launch_bounds__(256) hy_branch_norm_reg_kernel(float* __restrict__ x, HyBranch b, const int32_t* __restrict__ rows, const float* __restrict__ w, float eps,
                                                                  TA* __restrict__ h, int ldh, int W) {
-    HY_PDL();
+    griddep_launch();
     __shared__ float red[32];
     const long long t = blockIdx.x, src = rows ? rows[t] : t;
+    FVec<4> gb[NV], gw[NV];                              // weights ahead of the wait: both sums' latencies follow one another as it is
+#pragma unroll
+    for (int k = 0; k < NV; ++k) { const int c = (threadIdx.x + k * 256) * 4; if (c < W) { if (b.y && b.w) gb[k].load(b.w + c); if (w) gw[k].load(w + c); } }
+    griddep_wait();
     float* xr = x + src * W;
     FVec<4> v[NV];
 #pragma unroll
@@ -230,10 +234,8 @@ __global__ void __launch_bounds__(256) hy_branch_norm_reg_kernel(float* __restri
         for (int k = 0; k < NV; ++k) {
             const int c = (threadIdx.x + k * 256) * 4;
             if (c < W) {
-                FVec<4> g;
-                if (b.w) g.load(b.w + c);
 #pragma unroll
-                for (int e = 0; e < 4; ++e) v[k].v[e] = fmaf(y[k].v[e] * ry, b.w ? g.v[e] : 1.f, v[k].v[e]);
+                for (int e = 0; e < 4; ++e) v[k].v[e] = fmaf(y[k].v[e] * ry, b.w ? gb[k].v[e] : 1.f, v[k].v[e]);
             }
         }
     }
@@ -255,9 +257,9 @@ __global__ void __launch_bounds__(256) hy_branch_norm_reg_kernel(float* __restri
     for (int k = 0; k < NV; ++k) {
         const int c = (threadIdx.x + k * 256) * 4;
         if (c < W) {
-            FVec<4> g; g.load(w + c); float o[4];
+            float o[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) o[e] = v[k].v[e] * rr * g.v[e];
+            for (int e = 0; e < 4; ++e) o[e] = v[k].v[e] * rr * gw[k].v[e];
             store_act<4>(h + t * ldh + c, o);
         }
     }

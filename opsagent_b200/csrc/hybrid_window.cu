@@ -745,7 +745,9 @@ __global__ void __launch_bounds__(256) hy_win_decode_mma_kernel(HyWinAttn a, con
                                                                 const float* __restrict__ sink, const __nv_bfloat16* __restrict__ gate, int ldg,
                                                                 __nv_bfloat16* __restrict__ out, int ldo, float eps, HyRows r, const int32_t* __restrict__ tile_seq,
                                                                 const int32_t* __restrict__ tile_q0) {
-    HY_PDL();
+    // Tables and keys of earlier steps are read before the wait: the chain of lookups (tile, rows, positions, page) and a warp's first tile run under the
+    // kernel that prepares this step's queries and keys.
+    griddep_launch();
     extern __shared__ __align__(16) uint8_t win_smem[];
     __shared__ float pm[WIN_DEC_WARPS][MAPS][16], pl[WIN_DEC_WARPS][MAPS][16];
     __shared__ int qpos[16];
@@ -760,6 +762,30 @@ __global__ void __launch_bounds__(256) hy_win_decode_mma_kernel(HyWinAttn a, con
     const int seq = tile_seq[blockIdx.x], q0 = tile_q0[blockIdx.x];
     const int row0 = r.seq_row0[seq], len = r.seq_row0[seq + 1] - row0;
     const int nq = min(16, len * HG - q0);
+    const int pos_min = r.positions[row0 + q0 / HG], pos_max = r.positions[row0 + (q0 + nq - 1) / HG];
+    const int lo_min = max(0, pos_min - a.window + 1);
+    const int win_t0 = lo_min / WIN_KT, n_kt = pos_max / WIN_KT + 1;
+    const int n_keep = min((min(a.keep_first, lo_min) + WIN_KT - 1) / WIN_KT, win_t0);
+    const int n_it = n_keep + (n_kt - win_t0);
+    const int32_t* bt = r.block_tables + (long long)seq * r.max_pages_per_seq;
+    const int kc = QD / 8, nc = kc + VD / 8, step_j = 32 / nc, step_c = 32 % nc, j0 = lane / nc, c0 = lane % nc;      // a lane walks its warp's tile chunks in steps of 32
+    auto tile_of = [&](int it) { return it < n_keep ? it : win_t0 + (it - n_keep); };
+    auto load_tile = [&](int kt) {
+        const int key0 = kt * WIN_KT;              // the tile's 32 keys lie in one page
+        const __nv_bfloat16* page = cache + ((long long)bt[key0 >> 6] * 64 + (key0 & 63)) * CW;
+        int j = j0, c = c0;
+        while (j < WIN_KT) {
+            __nv_bfloat16* dst = c < kc ? Kw + j * QP + c * 8 : Vw + j * VP + (c - kc) * 8;
+            if (key0 + j <= pos_max) cp_async16(dst, page + (long long)j * CW + (c < kc ? g * QD + c * 8 : KW + g * VD + (c - kc) * 8));
+            else *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
+            j += step_j; c += step_c;
+            if (c >= nc) { c -= nc; ++j; }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const bool early = warp < n_it && tile_of(warp) * WIN_KT + WIN_KT <= r.seq_pos0[seq];      // all of the warp's first tile is older than this step
+    if (early) load_tile(tile_of(warp));
+    griddep_wait();
     for (int idx = tid; idx < 16 * (QD / 8); idx += 256) {
         const int qi = idx / (QD / 8), c = idx - qi * (QD / 8);
         uint4 v = make_uint4(0, 0, 0, 0);
@@ -768,12 +794,6 @@ __global__ void __launch_bounds__(256) hy_win_decode_mma_kernel(HyWinAttn a, con
     }
     if (tid < 16) qpos[tid] = tid < nq ? r.positions[row0 + (q0 + tid) / HG] : -1;
     __syncthreads();
-    const int pos_min = r.positions[row0 + q0 / HG], pos_max = r.positions[row0 + (q0 + nq - 1) / HG];
-    const int lo_min = max(0, pos_min - a.window + 1);
-    const int win_t0 = lo_min / WIN_KT, n_kt = pos_max / WIN_KT + 1;
-    const int n_keep = min((min(a.keep_first, lo_min) + WIN_KT - 1) / WIN_KT, win_t0);
-    const int n_it = n_keep + (n_kt - win_t0);
-    const int32_t* bt = r.block_tables + (long long)seq * r.max_pages_per_seq;
     float o[MAPS][NVB][4];
     float m_lo[MAPS], m_hi[MAPS], l_lo[MAPS], l_hi[MAPS];
 #pragma unroll
@@ -792,24 +812,11 @@ __global__ void __launch_bounds__(256) hy_win_decode_mma_kernel(HyWinAttn a, con
         rel_lo = a.rel + (long long)h_lo * a.rel_len; rel_hi = a.rel + (long long)h_hi * a.rel_len;
     }
     const int p_lo = qpos[lane >> 2], p_hi = qpos[(lane >> 2) + 8];
-    const int kc = QD / 8, nc = kc + VD / 8, step_j = 32 / nc, step_c = 32 % nc, j0 = lane / nc, c0 = lane % nc;      // a lane walks its warp's tile chunks in steps of 32
     for (int it = warp; it < n_it; it += WIN_DEC_WARPS) {
-        const int kt = it < n_keep ? it : win_t0 + (it - n_keep);
+        const int kt = tile_of(it);
         __syncwarp();                                  // the previous tile has been read by every lane
-        {
-            const int key0 = kt * WIN_KT;              // the tile's 32 keys lie in one page
-            const __nv_bfloat16* page = cache + ((long long)bt[key0 >> 6] * 64 + (key0 & 63)) * CW;
-            int j = j0, c = c0;
-            while (j < WIN_KT) {
-                __nv_bfloat16* dst = c < kc ? Kw + j * QP + c * 8 : Vw + j * VP + (c - kc) * 8;
-                if (key0 + j <= pos_max) cp_async16(dst, page + (long long)j * CW + (c < kc ? g * QD + c * 8 : KW + g * VD + (c - kc) * 8));
-                else *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
-                j += step_j; c += step_c;
-                if (c >= nc) { c -= nc; ++j; }
-            }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
+        if (it != warp || !early) load_tile(kt);
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncwarp();
         uint32_t pa[MAPS][2][4];
 #pragma unroll
