@@ -54,7 +54,9 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? 2 : 1) hy_block_memo
     HY_PDL();
     constexpr int NW = THREADS / 32, TPR = THREADS / BM_TB, NT = DP / 8, PP = BM_PP;
     extern __shared__ __align__(16) uint8_t bm_smem[];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, seq = blockIdx.x, h = blockIdx.y, D = p.D, VD = p.VD, VP = (VD + 15) / 16 * 16;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, D = p.D, VD = p.VD, VP = (VD + 15) / 16 * 16;
+    // every head of the longest sequence first: CTAs come in the order of their index, and a long one that starts in the second round would be the tail
+    const int rank = blockIdx.x + gridDim.x * blockIdx.y, seq = r.seq_by_len[rank / p.H], h = rank - rank / p.H * p.H;
     const long long row0 = r.seq_row0[seq]; const int len = r.seq_row0[seq + 1] - (int)row0, pos0 = r.seq_pos0[seq];
     if (len <= BM_FEW) return;                           // the token form takes this sequence
     const BlockSmem L(DELTA, DP, VP);

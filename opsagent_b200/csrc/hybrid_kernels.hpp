@@ -30,6 +30,7 @@ struct HyRows {
     const int32_t* seq_pos0;      // [S] position of a sequence's first row in this step (0: the sequence starts here, its state is taken as zero)
     const int32_t* seq_state;     // [S] recurrent-state slot
     const int32_t* block_tables;  // [S, max_pages_per_seq]
+    const int32_t* seq_by_len;    // [S] sequences, those with most rows in this step first
     int max_pages_per_seq, T, S;
 };
 

@@ -554,7 +554,7 @@ HybridModel::HybridModel(const ModelConfig& c, const EngineOptions& o) : ModelBa
             tails_[r.state_idx] = dmalloc((size_t)state_slots * std::max(1, l.conv - 1) * lw_[r.layer].conv_ch * es_);
         }
     }
-    meta_cap_words_ = 4 * MR + (size_t)MS_ + (size_t)opt.max_batch * (max_pages_per_seq + 8) + 64;
+    meta_cap_words_ = 4 * MR + (size_t)MS_ + (size_t)opt.max_batch * (max_pages_per_seq + 9) + 72;
     ctx_cap_ = 2 * MR_;
     if (max_kv > 0) { ld_kv_ = max_kv; lat_ctx_ = dmalloc((size_t)ctx_cap_ * max_Eattn * 2); kv_ctx_ = dmalloc((size_t)ctx_cap_ * ld_kv_ * 2); }
     for (const HyLayer& l : hc_.layers) if (l.type == HY_LATENT_ATTENTION) meta_cap_words_ += 3 * ((MR / 64 + (size_t)opt.max_batch) * l.heads + 8) + (size_t)opt.max_batch + 8;
@@ -930,6 +930,18 @@ void HybridModel::forward_sequential(const HyRows& r, const std::vector<TileList
     pending_ = pending; pend_mix_ = pend_mix; pend_out_ = pend_out;      // the final norm folds the last y_ into the rows it reads; the streams themselves are not needed again
 }
 
+// attention tiles with most keys first (their index is the order they start in; the long ones of a causal triangle otherwise make the tail): a counting sort,
+// equal tiles in the order they had.  With the longest sequences' recurrences first too: 2454 rows of 16 prompts of 30 to 300, four layers, 1400 -> 1314 us.
+static void heaviest_first(const std::vector<int32_t>& keys, std::initializer_list<std::vector<int32_t>*> lists) {
+    const int top = keys.empty() ? 0 : *std::max_element(keys.begin(), keys.end());
+    std::vector<int32_t> at((size_t)top + 2, 0), old;
+    for (int32_t k : keys) ++at[(size_t)(top - k) + 1];
+    for (size_t i = 1; i < at.size(); ++i) at[i] += at[i - 1];
+    std::vector<int32_t> place(keys.size());
+    for (size_t i = 0; i < keys.size(); ++i) place[i] = at[(size_t)(top - keys[i])]++;
+    for (std::vector<int32_t>* v : lists) { old = *v; for (size_t i = 0; i < old.size(); ++i) (*v)[(size_t)place[i]] = old[i]; }
+}
+
 void HybridModel::forward(const StepInput& in, float* logits_out) {
     const int T = (int)in.tokens.size(), S = in.n_seqs, NS = (int)in.sample_rows.size(), W = hc_.width, V = hc_.vocab;
     if (T <= 0 || T > MR_ || NS > MS_ || S <= 0 || S > opt.max_batch) throw std::runtime_error("forward: bad batch size");
@@ -954,6 +966,10 @@ void HybridModel::forward(const StepInput& in, float* logits_out) {
     const size_t o_tok = put(in.tokens.data(), T), o_pos = put(in.positions.data(), T), o_slot = put(in.slots.data(), T), o_samp = put(in.sample_rows.data(), NS);
     const size_t o_bt = put(in.block_tables.data(), in.block_tables.size()), o_rs = put(row_seq_.data(), T), o_r0 = put(in.seq_row0.data(), S + 1);
     const size_t o_p0 = put(seq_pos0_.data(), S), o_st = put(in.state_slots.data(), S);
+    seq_by_len_.resize(S);
+    for (int s = 0; s < S; ++s) seq_by_len_[s] = s;
+    if (many_rows_) std::stable_sort(seq_by_len_.begin(), seq_by_len_.end(), [&](int a, int b) { return in.seq_row0[a + 1] - in.seq_row0[a] > in.seq_row0[b + 1] - in.seq_row0[b]; });
+    const size_t o_len = put(seq_by_len_.data(), S);
     // attention plans, one per attention layer.  Sequences that bring at least hy_unabsorbed_rows rows take the prefill form (keys / values of
     // their context up-projected by a GEMM, ordinary multi-head attention); the others — decoding rows, short portions — the absorbed form:
     // tiles of 64 consecutive (row, head) pairs of one sequence, a decoding row with a long context cut into parts.
@@ -964,13 +980,17 @@ void HybridModel::forward(const StepInput& in, float* logits_out) {
             // windowed attention on the tensor cores: tiles of 64 consecutive (row, head-of-the-group) pairs of one sequence; a decoding row is one tile per key/value head
             tl.mma = !f32_ && opt.hy_tensor_core && ld_proj_ % 8 == 0 && (l.type == HY_WINDOW_ATTENTION || l.scaled_sum ? ld_mix_ : ld_mix2_) % 8 == 0 && hy_win_mma_supported(window_params(l, lw_[li]));
             if (!tl.mma) continue;
-            tile_seq_.clear(); tile_q0_.clear(); ptile_seq_.clear(); ptile_row0_.clear();
+            tile_seq_.clear(); tile_q0_.clear(); ptile_seq_.clear(); ptile_row0_.clear(); tile_keys_.clear();
             const int group = l.heads / l.kv_heads;
             for (int sq = 0; sq < S; ++sq) {
                 const int nq = (in.seq_row0[sq + 1] - in.seq_row0[sq]) * group;
                 if (nq <= HY_WIN_DECODE_QUERIES) { ptile_seq_.push_back(sq); ptile_row0_.push_back(0); continue; }       // decoding rows: the form whose warps split the keys
-                for (int q0 = 0; q0 < nq; q0 += HY_WIN_TILE_QUERIES) { tile_seq_.push_back(sq); tile_q0_.push_back(q0); }
+                for (int q0 = 0; q0 < nq; q0 += HY_WIN_TILE_QUERIES) {
+                    tile_seq_.push_back(sq); tile_q0_.push_back(q0);
+                    tile_keys_.push_back(std::min(seq_pos0_[sq] + (std::min(nq, q0 + HY_WIN_TILE_QUERIES) - 1) / group, l.window) / 32);
+                }
             }
+            heaviest_first(tile_keys_, {&tile_seq_, &tile_q0_});
             tl.n_w = (int)tile_seq_.size(); tl.o_wseq = put(tile_seq_.data(), tile_seq_.size()); tl.o_wq0 = put(tile_q0_.data(), tile_q0_.size());
             tl.n_d = (int)ptile_seq_.size(); tl.o_dseq = put(ptile_seq_.data(), ptile_seq_.size()); tl.o_dq0 = put(ptile_row0_.data(), ptile_row0_.size());
             continue;
@@ -979,14 +999,14 @@ void HybridModel::forward(const StepInput& in, float* logits_out) {
         const bool prefill_form = lw_[li].kv_up.tc && kv_ctx_;
         tl.mma = !f32_ && opt.hy_tensor_core && hy_mla_mma_supported(latent_params(l, lw_[li]));
         tile_seq_.clear(); tile_q0_.clear(); tile_k0_.clear(); tile_k1_.clear(); tile_slot_.clear(); merge_row_.clear(); merge_slot_.clear(); merge_parts_.clear();
-        ptile_seq_.clear(); ptile_head_.clear(); ptile_row0_.clear(); seq_base_.assign(S, -1);
+        ptile_seq_.clear(); ptile_head_.clear(); ptile_row0_.clear(); tile_keys_.clear(); seq_base_.assign(S, -1);
         int next_slot = 0;
         for (int sq = 0; sq < S; ++sq) {
             const int len = in.seq_row0[sq + 1] - in.seq_row0[sq], nq = len * l.heads, ctx_end = seq_pos0_[sq] + len;
             // many rows, or a short portion that is a good part of its own context (the start of a prompt cut by the step's token budget)
             if (prefill_form && (len >= opt.hy_unabsorbed_rows || (len >= 2 && ctx_end <= 8 * len)) && tl.ctx_rows + ctx_end <= ctx_cap_) {
                 seq_base_[sq] = tl.ctx_rows; tl.ctx_rows += ctx_end; tl.max_ctx = std::max(tl.max_ctx, ctx_end);
-                for (int hd = 0; hd < l.heads; ++hd) for (int q0 = 0; q0 < len; q0 += 64) { ptile_seq_.push_back(sq); ptile_head_.push_back(hd); ptile_row0_.push_back(q0); }
+                for (int hd = 0; hd < l.heads; ++hd) for (int q0 = 0; q0 < len; q0 += 64) { ptile_seq_.push_back(sq); ptile_head_.push_back(hd); ptile_row0_.push_back(q0); tile_keys_.push_back((seq_pos0_[sq] + std::min(len, q0 + 64)) / 32); }
                 continue;
             }
             tl.any_small = true;
@@ -1019,6 +1039,7 @@ void HybridModel::forward(const StepInput& in, float* logits_out) {
                     for (size_t i = 0; i < n; ++i) (*v)[i] = old[order[i]];
                 }
         }
+        heaviest_first(tile_keys_, {&ptile_seq_, &ptile_head_, &ptile_row0_});
         tl.n = (int)tile_seq_.size(); tl.n_merge = (int)merge_row_.size(); tl.n_ptiles = (int)ptile_seq_.size();
         tl.o_seq = put(tile_seq_.data(), tile_seq_.size()); tl.o_q0 = put(tile_q0_.data(), tile_q0_.size());
         tl.o_k0 = put(tile_k0_.data(), tile_k0_.size()); tl.o_k1 = put(tile_k1_.data(), tile_k1_.size()); tl.o_slot = put(tile_slot_.data(), tile_slot_.size());
@@ -1029,7 +1050,7 @@ void HybridModel::forward(const StepInput& in, float* logits_out) {
     cuda_check(cudaMemcpyAsync(d_meta_, hm, wd * 4, cudaMemcpyHostToDevice, stream), "meta H2D");
     cuda_check(cudaEventRecord(meta_ev_[meta_idx_], stream), "meta event");
     h2d_bytes += wd * 4;
-    HyRows r{d_meta_ + o_pos, d_meta_ + o_slot, d_meta_ + o_rs, d_meta_ + o_r0, d_meta_ + o_p0, d_meta_ + o_st, d_meta_ + o_bt, max_pages_per_seq, T, S};
+    HyRows r{d_meta_ + o_pos, d_meta_ + o_slot, d_meta_ + o_rs, d_meta_ + o_r0, d_meta_ + o_p0, d_meta_ + o_st, d_meta_ + o_bt, d_meta_ + o_len, max_pages_per_seq, T, S};
     static const char* dbg_layers = std::getenv("OA_DEBUG_LAYERS");      // debug: file that receives the residual stream after every layer execution of each forward
     std::vector<float> dbg_buf;
     if (dbg_layers && !capture_layers) capture_layers = &dbg_buf;
