@@ -162,9 +162,13 @@ OA_API int oa_k_paged_attention(const void* q, void* out, const void* kv_cache, 
 /* ---- host-only logic, callable without a GPU (CPU tests) ---- */
 /* chat template + tokenizer of the model described by config_json */
 OA_API int oa_host_apply_chat_template(const char* config_json, const oa_msg* msgs, int32_t n_msgs, int32_t* out_ids, int32_t cap, int32_t* n_out);
-/* decode-attention work plan: segs_out[cap_segs*5] = {seq, kvh, chunk_begin, chunk_end, partial_slot}, cta_ptr_out[n_ctas+1];
- * returns the number of CTAs in *n_ctas_out and of segments in *n_segs_out */
+/* balanced partition of a decoding batch's (sequence, kv head) contexts, the pieces decode attention cuts them into: segs_out[cap_segs*5] = {seq, kvh,
+ * chunk_begin, chunk_end, partial_slot}, cta_ptr_out[n_ctas+1]; returns the number of CTAs in *n_ctas_out and of segments in *n_segs_out */
 OA_API int oa_host_decode_plan(const int32_t* ctx_lens, int32_t n_seqs, int32_t n_kv, int32_t n_ctas_target, int32_t force_splits,
+                        int32_t* segs_out, int32_t cap_segs, int32_t* cta_ptr_out, int32_t cap_ctas, int32_t* n_ctas_out,
+                        int32_t* n_segs_out, int32_t* n_slots_out);
+/* the plan decode attention runs: the same pieces, on that partition's CTAs or with all pieces of a (sequence, kv head) on one CTA */
+OA_API int oa_host_decode_attention_plan(const int32_t* ctx_lens, int32_t n_seqs, int32_t n_kv, int32_t n_ctas_target, int32_t force_splits,
                         int32_t* segs_out, int32_t cap_segs, int32_t* cta_ptr_out, int32_t cap_ctas, int32_t* n_ctas_out,
                         int32_t* n_segs_out, int32_t* n_slots_out);
 /* stream-K unit plan of the decode projections (host only, no GPU): CTA c owns k-block units [cta_unit0[c], cta_unit0[c+1]) of

@@ -242,15 +242,23 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) decode_attention_kernel(const 
             if (sg.partial_slot >= 0) {
                 // flash-decoding merge without a second kernel: the CTA that finishes an item's LAST piece combines all pieces.
                 // Counters advance by n_pieces per layer and start each step at zero, so "last" is a multiple of n_pieces.  What is written before has
-                // to be seen by whoever counts later, no more: an acquire-release fence, of one lane for its warp.
+                // to be seen by whoever counts later, no more: an acquire-release fence, of one lane for its warp.  A CTA that has all pieces of an item
+                // counts nothing: its last is the last, and the barrier below is all that its own reads need.
                 __syncwarp();
-                if (lane == 0) fence_acq_rel_gpu();
-                if (lane == 0 && ((atomicAdd(p.merge_counters + sg.item, 1) + 1) % sg.n_pieces) == 0) { fence_acq_rel_gpu(); const int n = merge_s[0]; merge_s[1 + n] = si; merge_s[0] = n + 1; }
+                if (lane == 0) {
+                    bool last = sg.partial_slot + 1 == sg.slot_begin + sg.n_pieces;
+                    if (sg.item >= 0) {
+                        fence_acq_rel_gpu();
+                        last = (atomicAdd(p.merge_counters + sg.item, 1) + 1) % sg.n_pieces == 0;
+                        if (last) fence_acq_rel_gpu();
+                    }
+                    if (last) { const int n = merge_s[0]; merge_s[1 + n] = si; merge_s[0] = n + 1; }
+                }
             }
         }
         named_bar_sync(1, 128);   // scratch free for the next segment
     }
-    // Merges this CTA came last for: at most its first and its last segment belong to cut items.  The four warps take a quarter of the columns each
+    // Merges this CTA came last for: at most its first and its last segment belong to items shared with others, or all of them to one item of its own.  The four warps take a quarter of the columns each
     // (lane: head g, NC consecutive columns from t * NC of the quarter), pieces in slot order (deterministic), eight pieces' loads in flight: a context
     // cut over the whole chip has up to 37 pieces per item, and one warp reading them one after the other was as long as the attention itself.  The
     // maximum over the pieces comes from the head's four lanes, a quarter of them each, under the first pieces' loads.  us a layer, before the lighter

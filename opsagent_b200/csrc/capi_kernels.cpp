@@ -292,11 +292,8 @@ int oa_host_apply_chat_template(const char* config_json, const oa_msg* msgs, int
     return OA_OK;
 }
 
-int oa_host_decode_plan(const int32_t* ctx_lens, int32_t n_seqs, int32_t n_kv, int32_t n_ctas_target, int32_t force_splits,
-                        int32_t* segs_out, int32_t cap_segs, int32_t* cta_ptr_out, int32_t cap_ctas, int32_t* n_ctas_out,
-                        int32_t* n_segs_out, int32_t* n_slots_out) {
-    DecodePlan plan;
-    build_decode_plan(ctx_lens, n_seqs, n_kv, n_ctas_target, force_splits, plan);
+static int export_decode_plan(const DecodePlan& plan, int32_t* segs_out, int32_t cap_segs, int32_t* cta_ptr_out, int32_t cap_ctas, int32_t* n_ctas_out,
+                              int32_t* n_segs_out, int32_t* n_slots_out) {
     if ((int)plan.segs.size() > cap_segs || (int)plan.cta_ptr.size() > cap_ctas + 1) return OA_ERR_BAD_REQUEST;
     for (size_t i = 0; i < plan.segs.size(); ++i) {
         const DecodeSeg& g = plan.segs[i];
@@ -305,6 +302,20 @@ int oa_host_decode_plan(const int32_t* ctx_lens, int32_t n_seqs, int32_t n_kv, i
     std::memcpy(cta_ptr_out, plan.cta_ptr.data(), plan.cta_ptr.size() * 4);
     *n_ctas_out = (int32_t)plan.cta_ptr.size() - 1; *n_segs_out = (int32_t)plan.segs.size(); *n_slots_out = plan.n_slots;
     return OA_OK;
+}
+int oa_host_decode_plan(const int32_t* ctx_lens, int32_t n_seqs, int32_t n_kv, int32_t n_ctas_target, int32_t force_splits,
+                        int32_t* segs_out, int32_t cap_segs, int32_t* cta_ptr_out, int32_t cap_ctas, int32_t* n_ctas_out,
+                        int32_t* n_segs_out, int32_t* n_slots_out) {
+    DecodePlan plan;
+    build_decode_plan(ctx_lens, n_seqs, n_kv, n_ctas_target, force_splits, plan);
+    return export_decode_plan(plan, segs_out, cap_segs, cta_ptr_out, cap_ctas, n_ctas_out, n_segs_out, n_slots_out);
+}
+int oa_host_decode_attention_plan(const int32_t* ctx_lens, int32_t n_seqs, int32_t n_kv, int32_t n_ctas_target, int32_t force_splits,
+                                  int32_t* segs_out, int32_t cap_segs, int32_t* cta_ptr_out, int32_t cap_ctas, int32_t* n_ctas_out,
+                                  int32_t* n_segs_out, int32_t* n_slots_out) {
+    DecodePlan plan;
+    plan_decode_attention(ctx_lens, n_seqs, n_kv, n_ctas_target, force_splits, plan);
+    return export_decode_plan(plan, segs_out, cap_segs, cta_ptr_out, cap_ctas, n_ctas_out, n_segs_out, n_slots_out);
 }
 
 int oa_host_streamk_plan(int32_t N, int32_t K, int32_t block_n, int32_t n_ctas, int64_t* cta_unit0_out, int32_t cap_ctas,

@@ -158,7 +158,7 @@ cudaError_t launch_init_weight(void* dst, uint64_t seed, uint64_t tensor_id, int
 struct DecodeSeg {        // one contiguous piece of one (sequence, kv head) handled by one CTA
     int32_t seq, kvh, chunk_begin, chunk_end;   // chunks of 64 tokens
     int32_t partial_slot;                        // index into the partial workspace, or -1: single-piece, write final
-    int32_t slot_begin, n_pieces, item;          // cut items: first slot, piece count and merge-counter index of the (seq, kv head) item
+    int32_t slot_begin, n_pieces, item;          // cut items: first slot, piece count and merge-counter index of the (seq, kv head) item (-1: its pieces are all this CTA's)
 };
 struct DecodeAttnParams {
     const void* q;                 // bf16 [B, nh*D] (already rotated)

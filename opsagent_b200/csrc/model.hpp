@@ -41,7 +41,7 @@ struct DecodePlan {
 };
 // contiguous, balanced partition of all (sequence, kv head) page lists over n_ctas CTAs
 void build_decode_plan(const int32_t* ctx_lens, int n_seqs, int n_kv, int n_ctas_target, int force_splits, DecodePlan& out);
-// what decode attention runs: that partition, or one CTA an item where cutting costs more than it evens out
+// what decode attention runs: that partition's pieces on its CTAs, or all pieces of an item on a CTA of its own where sharing one costs more than it evens out
 void plan_decode_attention(const int32_t* ctx_lens, int n_seqs, int n_kv, int n_ctas_target, int force_splits, DecodePlan& out);
 
 // What the scheduler (engine.cpp) sees of a model: its step function, the geometry of its paged cache and of its per-sequence state slots,

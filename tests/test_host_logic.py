@@ -79,13 +79,13 @@ def test_bad_configs_are_rejected():
     assert L.oa_host_model_info(b'not json', buf, 512) == 400
 
 
-def plan(ctx, n_kv, n_ctas, force=0):
+def plan(ctx, n_kv, n_ctas, force=0, entry="oa_host_decode_plan"):
     L = _lib.load()
     ctx = np.ascontiguousarray(ctx, np.int32)
     cap = len(ctx) * n_kv * 64 + n_ctas + 64
     segs = np.zeros((cap, 5), np.int32); ptr = np.zeros(cap + 1, np.int32)
     nc, ns, nsl = C.c_int32(), C.c_int32(), C.c_int32()
-    assert L.oa_host_decode_plan(ctx.ctypes.data, len(ctx), n_kv, n_ctas, force, segs.ctypes.data, cap, ptr.ctypes.data, cap,
+    assert getattr(L, entry)(ctx.ctypes.data, len(ctx), n_kv, n_ctas, force, segs.ctypes.data, cap, ptr.ctypes.data, cap,
                                  C.byref(nc), C.byref(ns), C.byref(nsl)) == 0
     return segs[:ns.value], ptr[:nc.value + 1], nsl.value
 
@@ -123,6 +123,34 @@ def test_decode_plan_covers_every_page_exactly_once_and_is_balanced(ctx, n_kv, n
 def test_empty_and_zero_length_plans():
     segs, ptr, n_slots = plan([0, 0], 4, 296)
     assert len(segs) == 0 and n_slots == 0
+
+
+# batches on both sides of the line of one CTA an item (3 chunks above an equal share; as many items as CTAs), with zero-length sequences, one head and eight
+RUN_PLANS = [([64 * 5], 1, 1), ([64 * 6], 1, 0), ([320] * 2 + [1], 8, 1), ([321] * 2 + [1], 8, 0), ([70, 300, 5, 129] * 9, 8, 1), ([70, 300, 5, 129] * 9 + [64, 65], 8, 0),
+             ([40 + 3 * i for i in range(32)], 8, 1), ([700] * 32, 8, 1), ([700] * 31 + [1500], 8, 0), ([0, 130, 0, 64], 4, 1), ([3000], 1, 0), ([1] * 37, 8, 1), ([1664] * 128, 8, 0)]
+
+
+@pytest.mark.parametrize("ctx,n_kv,whole", RUN_PLANS)
+def test_decode_attention_runs_the_pieces_of_the_balanced_partition(ctx, n_kv, whole):
+    """A row's bits follow from its pieces: the plan that runs has those of the partition over 296 CTAs, in one order and with the same slots, whichever CTAs
+    run them; every page is covered once, and an item's pieces are together exactly where the rule says so."""
+    segs, ptr, n_slots = plan(ctx, n_kv, 296, entry="oa_host_decode_attention_plan")
+    chunks = [(c + 63) // 64 for c in ctx]
+    total = sum(chunks) * n_kv
+    per = -(-total // min(296, max(1, total // 2)))
+    pieces, at, slot = [], 0, 0
+    for s, n in enumerate(chunks):
+        for h in range(n_kv):
+            cuts = [at] + [x for x in range((at // per + 1) * per, at + n, per)] + [at + n]
+            for a, b in zip(cuts, cuts[1:]):
+                if b > a:
+                    pieces.append((s, h, a - at, b - at, slot if len(cuts) > 2 else -1)); slot += len(cuts) > 2
+            at += n
+    assert [tuple(x) for x in segs.tolist()] == pieces and n_slots == slot
+    assert ptr[0] == 0 and ptr[-1] == len(segs) and (np.diff(ptr) > 0).all()
+    items = [tuple(x[:2]) for x in segs.tolist()]
+    own = len(ptr) - 1 == len(set(items)) and all(len(set(items[a:b])) == 1 for a, b in zip(ptr, ptr[1:]))
+    assert own == bool(whole) == (len(set(items)) <= 296 and max(chunks) <= per + 3)
 
 
 # ---- Chat() retry semantics of the Python mirror (reference pkg/llms/openai.go:77-103) ----

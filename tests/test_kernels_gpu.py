@@ -312,6 +312,15 @@ def test_paged_prefill_attention_two_heads_per_cta(L, nh, nkv, D):
     assert err < 2 * 5 * 2.0 ** -8, err
 
 
+def _decode_route(L, ctx, nkv):
+    """segments, CTAs and partial slots of the plan that a decoding batch runs on 148 SMs"""
+    ctx = np.ascontiguousarray(ctx, np.int32); cap = int(((ctx + 63) // 64).sum()) * nkv + 512
+    segs, cta_ptr = np.zeros((cap, 5), np.int32), np.zeros(cap + 1, np.int32)
+    n = [C.c_int32() for _ in range(3)]
+    assert L.oa_host_decode_attention_plan(ctx.ctypes.data, len(ctx), nkv, 296, 0, segs.ctypes.data, cap, cta_ptr.ctypes.data, cap, *[C.byref(x) for x in n]) == 0
+    return n[1].value, n[0].value, n[2].value
+
+
 # few long contexts: an item is cut over up to 37 CTAs and the last of them merges the pieces (one, two, several, more than four at a time)
 @pytest.mark.parametrize("ctx,nh,nkv,D", [([9000], 32, 8, 128), ([9001, 5, 70], 16, 2, 128), ([5000, 64], 32, 8, 64), ([700], 5, 1, 64), ([3333, 3334, 129], 40, 8, 128)])
 def test_paged_decode_attention_merges_many_pieces(L, ctx, nh, nkv, D):
@@ -330,6 +339,31 @@ def test_paged_decode_attention_merges_many_pieces(L, ctx, nh, nkv, D):
     ref = _attn_ref(q, kv[0], kv[1], bt.to(dev()).long(), ctx, [1] * n, nh, nkv, D)
     # probabilities and result are rounded to bf16 (2^-9 relative each); |values| stay below 3
     assert (out.float() - ref).abs().max().item() < 2 * 3 * 2.0 ** -8
+
+
+# a sequence more that is one chunk above the line takes the batch from one CTA an item to shared items, and leaves the pieces of the others where they are
+@pytest.mark.parametrize("n,nh,nkv,D,ctx", [(10, 5, 1, 64, 320), (12, 8, 1, 128, 257), (6, 32, 8, 128, 319), (16, 32, 8, 64, 320), (28, 40, 8, 128, 257)])
+def test_decode_rows_keep_their_bits_whoever_runs_their_pieces(L, n, nh, nkv, D, ctx):
+    per = -(-5 * n * nkv // min(296, 5 * n * nkv // 2))
+    last = 64 * (per + 4)
+    assert per == -(-(5 * n + per + 4) * nkv // min(296, (5 * n + per + 4) * nkv // 2))
+    lens = [ctx] * n + [last]
+    num_pages = 5 * n + per + 4
+    kv = _mk_cache(num_pages, nkv, D, 23)
+    g = torch.Generator(device="cpu").manual_seed(9)
+    bt = np.zeros((n + 1, per + 4), np.int32); perm = torch.randperm(num_pages, generator=g).numpy(); k = 0
+    for i, c in enumerate(lens):
+        npg = (c + 63) // 64; bt[i, :npg] = perm[k:k + npg]; k += npg
+    q = (torch.randn(n + 1, nh, D, generator=g) * 2).to(torch.bfloat16).to(dev())
+    outs = []
+    for m, together in ((n, True), (n + 1, False)):
+        segs, ctas, slots = _decode_route(L, lens[:m], nkv)
+        assert (ctas == m * nkv) == together and slots > 0
+        out = torch.full((m, nh, D), float("nan"), dtype=torch.bfloat16, device=dev())
+        a = np.array(lens[:m], np.int32)
+        assert L.oa_k_paged_attention(ptr(q), ptr(out), ptr(kv), num_pages, bt.ctypes.data, per + 4, a.ctypes.data, None, m, nh, nkv, D, 0, None) == 0, _lib.last_error()
+        outs.append(out)
+    assert not torch.isnan(outs[1]).any() and torch.equal(outs[0], outs[1][:n])
 
 
 # one CTA an item or items cut over CTAs: batches on both sides of the line (an equal share of 2 chunks + 8, + 16 from 64 items on; one item more than CTAs)
