@@ -112,7 +112,8 @@ __global__ void __launch_bounds__(64 + 128 * NWG, 1) prefill_attention_tc_kernel
     uint64_t* s_full = bars + 9;              // [2]
     uint64_t* s_empty = bars + 11;            // [2]
     uint64_t* p_full = bars + 13;             // [2]
-    uint64_t* t_full = bars + 15;             // 1 (one completion per P·V)
+    uint64_t* t_full = bars + 15;             // 1 (one completion per P·V but the last)
+    uint64_t* o_full = bars + 16;             // 1 (the last P·V)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
     float* xch = reinterpret_cast<float*>(p_s + 2 * Cfg::P_BYTES + 256);       // [2][2][128]
 
@@ -127,7 +128,7 @@ __global__ void __launch_bounds__(64 + 128 * NWG, 1) prefill_attention_tc_kernel
         mbar_init(q_full, 1);
         for (int i = 0; i < 2; ++i) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1);
                                       mbar_init(&s_full[i], 1); mbar_init(&s_empty[i], 4 * NWG); mbar_init(&p_full[i], 4 * NWG); }
-        mbar_init(t_full, 1);
+        mbar_init(t_full, 1); mbar_init(o_full, 1);
         fence_barrier_init();
     }
     if (warp == 1) tmem_alloc<Cfg::TMEM_COLS>(tmem_slot);
@@ -212,7 +213,7 @@ __global__ void __launch_bounds__(64 + 128 * NWG, 1) prefill_attention_tc_kernel
 #pragma unroll
                 for (int ks = 0; ks < KV_TILE / 16; ++ks)              // O accumulates over all KV tiles
                     umma_bf16(tmem_base + Cfg::T_COL, a + (uint64_t)(((ks >> 2) * Cfg::HALF_BYTES + (ks & 3) * 32) >> 4), b + (uint64_t)(ks * (2048 >> 4)), idesc_t, (j > 0 || ks > 0) ? 1u : 0u);
-                umma_commit(t_full);
+                umma_commit(j + 1 < n_kvt ? t_full : o_full);
                 umma_commit(&v_empty[st]);
             }
             __syncwarp();
@@ -302,7 +303,10 @@ __global__ void __launch_bounds__(64 + 128 * NWG, 1) prefill_attention_tc_kernel
             __syncwarp();
             if (lane == 0) mbar_arrive(&p_full[sb]);
         }
-        mbar_wait(t_full, (uint32_t)(n_kvt - 1) & 1);
+        // A barrier of its own: S of the last tile says that all products up to the third last P·V have landed, no more, and with the second last one still
+        // under way a wait for the last one's parity on t_full would find the third last one's phase and pass.  (In the loop S_j says that P_{j-2}·V has
+        // landed, so the wait for P_{j-1}·V cannot be taken for an earlier one.)
+        mbar_wait(o_full, 0);
         tcgen05_fence_after();
         {                                                           // row sum = the two key halves' sums (fixed order: half 0 + half 1)
             const int xb = n_kvt & 1;                               // the buffer the last tile did not use

@@ -282,6 +282,36 @@ def test_paged_prefill_attention(L, nh, nkv, D):
     assert err < 2e-2, err
 
 
+# few rows take the kernel of one head a CTA, whose output may only be read once its last products have landed however late their values come: one to six
+# key tiles, keys in L2 and values not, full and ragged last tiles; the bits of the two-head kernel, which the same prompt takes among copies of itself
+@pytest.mark.parametrize("nh,nkv,D", [(8, 2, 128), (16, 4, 64)])
+@pytest.mark.parametrize("ctx,rows", [(128, 128), (256, 128), (256, 100), (257, 129), (512, 32), (700, 33), (700, 200)])
+def test_prefill_output_waits_for_the_last_values(L, nh, nkv, D, ctx, rows):
+    pages, maxp = (ctx + 63) // 64, (ctx + 63) // 64
+    kv = _mk_cache(pages, nkv, D, 41)
+    g = torch.Generator(device="cpu").manual_seed(12)
+    q1 = torch.randn(rows, nh, D, generator=g).to(torch.bfloat16).to(dev())
+    flush = torch.empty(256 << 20, dtype=torch.uint8, device=dev())
+
+    def attend(copies):
+        assert ((rows + 127) // 128 * copies * nkv * (nh // nkv + 1) // 2 > 74) == (copies > 1)
+        q = q1.repeat(copies, 1, 1).contiguous()
+        out = torch.full_like(q, float("nan"))
+        bt = np.tile(np.arange(pages, dtype=np.int32)[::-1], (copies, 1)).copy()
+        c, n = np.full(copies, ctx, np.int32), np.full(copies, rows, np.int32)
+        flush.zero_(); kv[0].float().sum().item()
+        assert L.oa_k_paged_attention(ptr(q), ptr(out), ptr(kv), pages, bt.ctypes.data, maxp, c.ctypes.data, n.ctypes.data, copies, nh, nkv, D, 0, None) == 0, _lib.last_error()
+        return out
+
+    want = attend(40)
+    ref = _attn_ref(q1, kv[0], kv[1], torch.arange(pages - 1, -1, -1, device=dev())[None], [ctx], [rows], nh, nkv, D)
+    # probabilities and result are rounded to bf16 (2^-9 relative each); |values| stay below 5
+    assert (want[:rows].float() - ref).abs().max().item() < 2 * 5 * 2.0 ** -8
+    for _ in range(10):
+        assert torch.equal(attend(1), want[:rows])
+    assert torch.equal(want, want[:rows].repeat(40, 1, 1))
+
+
 # batches that fill the chip take the two-heads-per-CTA kernel: an even and an odd number of heads per group (the last head of an odd group is
 # alone), portions behind a cached prefix, tiles of one row, key tiles whose second page is missing, and more items than CTAs
 @pytest.mark.parametrize("nh,nkv,D", [(32, 8, 128), (20, 4, 128), (32, 8, 64), (15, 3, 64), (16, 2, 128)])
