@@ -19,6 +19,7 @@
 #include "tokenizer.hpp"
 #include "model.hpp"
 #include "hybrid_kernels.hpp"
+#include "pinned_pool.hpp"
 #include "sk_consumers.cuh"
 #include "tokenizer.hpp"
 
@@ -61,41 +62,26 @@ struct DevBuf {
 };
 // Pinned host memory for the arrays of one call: a copy from pageable memory is pushed or staged by the calling thread (6 to 10 us for 8 to 16 KB, against 2
 // to 3 from pinned memory in a loop of its own; six conversations of 1750 tokens: 40.3 -> 38.3 us a call).  A buffer belongs to one call at a time and goes
-// back once the call's stream has passed its copy; a handful of up to 1 MB stay for later calls, everything else is freed at once.  (A kernel that reads
-// the pinned buffer instead of a copy was slower than either for such sizes: it and the attention behind it run one after the other, 41.8 us.)
-struct PinnedPool {
-    static constexpr size_t KEEP_BYTES = 1 << 20, KEEP_BUFFERS = 8;
-    struct Buf { uint8_t* p; size_t cap; };
-    std::mutex mu; Buf kept[KEEP_BUFFERS]; size_t n = 0;
-    Buf take(size_t bytes) {
-        {
-            std::lock_guard<std::mutex> lk(mu);
-            for (size_t i = 0; i < n; ++i) if (kept[i].cap >= bytes) { const Buf b = kept[i]; kept[i] = kept[--n]; return b; }
-        }
-        size_t cap = 64 << 10;
-        while (cap < bytes) cap *= 2;
-        void* p = nullptr;
-        return cudaHostAlloc(&p, cap, cudaHostAllocPortable) == cudaSuccess ? Buf{(uint8_t*)p, cap} : Buf{nullptr, 0};
-    }
-    void give(const Buf& b) {
-        if (b.cap <= KEEP_BYTES) {
-            std::lock_guard<std::mutex> lk(mu);
-            if (n < KEEP_BUFFERS) { kept[n++] = b; return; }
-        }
-        cudaFreeHost(b.p);
-    }
-};
-PinnedPool& pinned_pool() { static PinnedPool* pool = new PinnedPool(); return *pool; }      // never destroyed: the driver may be gone by then
+// back once the call's stream has passed its copy.  (A kernel that reads the pinned buffer instead of a copy was slower than either for such sizes: it and
+// the attention behind it run one after the other, 41.8 us.)
+uint8_t* pin_host(size_t bytes) {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;          // pinning touches no stream: another thread's capture goes on
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, bytes, cudaHostAllocPortable) != cudaSuccess) { p = nullptr; cudaGetLastError(); }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return (uint8_t*)p;
+}
+PinnedPool& pinned_pool() { static PinnedPool* pool = new PinnedPool(pin_host); return *pool; }      // never destroyed: the driver may be gone by then
 // Host arrays of one call, packed so that ONE copy brings them to the device (each on a 16-byte boundary)
 struct Packed {
-    PinnedPool::Buf buf; size_t used = 0;
-    explicit Packed(size_t bytes) : buf(pinned_pool().take(bytes)) {}
-    Packed(const Packed&) = delete;
-    ~Packed() { if (buf.p) pinned_pool().give(buf); }
+    CallMemory mem; size_t used = 0;
+    explicit Packed(size_t bytes) : mem(pinned_pool(), bytes) {}
     size_t reserve(size_t bytes) { const size_t at = (used + 15) & ~size_t(15); used = at + bytes; return at; }
+    uint8_t* data() const { return mem.get(); }
     size_t add(const void* src, size_t n) {
         const size_t at = reserve(n);
-        if (n) std::memcpy(buf.p + at, src, n);
+        if (n) std::memcpy(data() + at, src, n);
         return at;
     }
 };
@@ -218,21 +204,20 @@ static int paged_attention(const void* q, void* out, const void* kv_cache, int32
     for (int i = 0; i < n_seqs; ++i) { if (q_lens && q_lens[i] != 1) decode = false; total_q += q_lens ? q_lens[i] : 1; }
     const size_t table_bytes = (size_t)n_seqs * max_pages_per_seq * 4, ctx_bytes = (size_t)n_seqs * 4;
     cudaError_t e;
-    // every path below that has started the copy waits for the stream before the pinned buffer goes back
+    // every path below that has started the copy waits for the stream before the host memory goes back
     if (decode) {
         static thread_local DecodePlan plan;         // its vectors keep their room from call to call
         plan_decode_attention(ctx_lens, n_seqs, n_kv, 2 * 148, force_splits, plan);
         const size_t seg_bytes = plan.segs.size() * sizeof(DecodeSeg), ptr_bytes = plan.cta_ptr.size() * 4, count_bytes = (size_t)(plan.n_cut + 1) * 4;
         Packed host(packed_bytes({table_bytes, ctx_bytes, seg_bytes, ptr_bytes, count_bytes}));
-        if (!host.buf.p) return OA_ERR_INTERNAL;
         const size_t o_bt = host.add(block_tables, table_bytes), o_ctx = host.add(ctx_lens, ctx_bytes);
         const size_t o_segs = host.add(plan.segs.data(), seg_bytes), o_ptr = host.add(plan.cta_ptr.data(), ptr_bytes);
         const size_t o_count = host.reserve(count_bytes);                        // merge counters: the CTA with an item's last piece merges it
-        std::memset(host.buf.p + o_count, 0, count_bytes);
+        std::memset(host.data() + o_count, 0, count_bytes);
         const size_t o_po = (host.used + 255) & ~size_t(255), o_pml = o_po + (size_t)(plan.n_slots + 1) * grp * head_dim * 4;
         DevBuf d_meta(o_pml + (size_t)(plan.n_slots + 1) * grp * 2 * 4, s);       // [tables, plan, counters | partial outputs | partial maxima and sums]
         if (!d_meta.p) return OA_ERR_INTERNAL;
-        e = cudaMemcpyAsync(d_meta.p, host.buf.p, host.used, cudaMemcpyHostToDevice, s);
+        e = cudaMemcpyAsync(d_meta.p, host.data(), host.used, cudaMemcpyHostToDevice, s);
         const char* meta = (const char*)d_meta.p;
         DecodeAttnParams a{}; a.q = q; a.out = out; a.block_tables = (const int32_t*)(meta + o_bt); a.ctx_lens = (const int32_t*)(meta + o_ctx);
         a.max_pages_per_seq = max_pages_per_seq; a.segs = (const DecodeSeg*)(meta + o_segs); a.cta_seg_ptr = (const int32_t*)(meta + o_ptr);
@@ -255,7 +240,6 @@ static int paged_attention(const void* q, void* out, const void* kv_cache, int32
     std::stable_sort(tiles.begin(), tiles.end(), [](const PrefillTile& x, const PrefillTile& y) { return x.pos0 + x.n_rows > y.pos0 + y.n_rows; });
     const size_t tile_bytes = tiles.size() * sizeof(PrefillTile);
     Packed host(packed_bytes({table_bytes, tile_bytes}));
-    if (!host.buf.p) return OA_ERR_INTERNAL;
     const size_t o_bt = host.add(block_tables, table_bytes), o_tiles = host.add(tiles.data(), tile_bytes);
     DevBuf d_meta(host.used, s);
     if (!d_meta.p) return OA_ERR_INTERNAL;
@@ -265,7 +249,7 @@ static int paged_attention(const void* q, void* out, const void* kv_cache, int32
     const bool legacy = leg && std::string(leg) == "legacy";
     CUtensorMap tmq;
     if (!legacy && make_tmap_bf16_2d(&tmq, q, (uint64_t)total_q, (uint64_t)n_heads * head_dim, (uint64_t)n_heads * head_dim, 128, 64) != 0) return OA_ERR_INTERNAL;
-    e = cudaMemcpyAsync(d_meta.p, host.buf.p, host.used, cudaMemcpyHostToDevice, s);
+    e = cudaMemcpyAsync(d_meta.p, host.data(), host.used, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = legacy ? launch_prefill_attention(&tm, kv, a, s) : launch_prefill_attention_tc(&tmq, &tm, kv, a, s);
     const cudaError_t done = cudaStreamSynchronize(s);
     return rc_of(e == cudaSuccess ? done : e);

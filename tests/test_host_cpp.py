@@ -341,3 +341,59 @@ def test_cpp_toolprompt_unmarshal_equals_the_python_mirror_on_random_json(tmp_pa
             want = None
         assert g == want, (text, g, want)
     assert 300 < n_ok < 2900          # both outcomes are well represented
+
+
+SRC_PINNED = r'''
+#include <atomic>
+#include <cstdio>
+#include <cstring>
+#include <memory>
+#include <thread>
+#include <vector>
+#include "opsagent_b200/csrc/pinned_pool.hpp"
+using namespace oa;
+static std::atomic<int> pins{0}; static bool refuse = false;
+static uint8_t* pin(size_t n) { if (refuse) return nullptr; ++pins; return new uint8_t[n]; }
+#define CHECK(x) do { if (!(x)) { std::printf("line %d: %s\\n", __LINE__, #x); return 1; } } while (0)
+int main() {
+    PinnedPool pool(pin);
+    refuse = true;                                       // no page-locked memory: the call goes on with pageable memory, and later ones ask again
+    { CallMemory m(pool, 100); CHECK(m.get() && !m.pinned()); }
+    refuse = false;
+    for (int i = 0; i < 50; ++i) { CallMemory m(pool, 100 + 20000 * i); CHECK(m.pinned()); std::memset(m.get(), i, 100 + 20000 * i); }
+    CHECK(pins == 1);
+    for (int i = 0; i < 50; ++i) {                       // more than a buffer holds: nothing is pinned for it
+        CallMemory m(pool, PinnedPool::BUF_BYTES + 1), whole(pool, PinnedPool::BUF_BYTES);
+        CHECK(!m.pinned() && m.get() && whole.pinned());
+    }
+    CHECK(pins == 1);
+    for (int round = 0; round < 3; ++round) {            // bursts of small calls, then large ones: never more buffers, never one pinned in a call's way
+        std::vector<std::unique_ptr<CallMemory>> held;
+        for (int i = 0; i < 3 * PinnedPool::BUFFERS; ++i) held.emplace_back(new CallMemory(pool, round ? PinnedPool::BUF_BYTES : 64));
+        for (int i = 0; i < (int)held.size(); ++i) {
+            CHECK(held[i]->pinned() == (i < PinnedPool::BUFFERS));
+            for (int j = 0; j < i; ++j) CHECK(held[i]->get() != held[j]->get());
+        }
+        CHECK(pins == PinnedPool::BUFFERS);
+    }
+    std::atomic<int> bad{0};
+    std::vector<std::thread> ts;
+    for (int t = 0; t < 16; ++t) ts.emplace_back([&, t] {
+        for (int i = 0; i < 2000; ++i) {
+            CallMemory m(pool, 512); std::memset(m.get(), t, 512); std::this_thread::yield();
+            for (int k = 0; k < 512; ++k) if (m.get()[k] != t) { ++bad; break; }
+        }
+    });
+    for (auto& t : ts) t.join();
+    CHECK(bad == 0 && pins == PinnedPool::BUFFERS);
+    return 0;
+}
+'''
+
+
+def test_pinned_buffers_are_few_and_calls_go_on_without_one(tmp_path):
+    src = tmp_path / "pool.cpp"; src.write_text(SRC_PINNED)
+    exe = tmp_path / "pool"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-Werror", f"-I{ROOT}", str(src), "-o", str(exe), "-lpthread"], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout
