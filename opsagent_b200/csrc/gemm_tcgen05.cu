@@ -340,9 +340,10 @@ static cudaError_t launch_few_kq(const CUtensorMap* tmA, const CUtensorMap* tmB,
 template <int BN, int EPI>
 static cudaError_t launch_few(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, cudaStream_t stream) {
     const FewRing few = few_ring(p.M, p.N, BN, sm_count_cached());
-    if constexpr (BN <= 32) if (few.kq == 4) return launch_few_kq<BN, EPI, 4>(tmA, tmB, p, few, stream);
-    if constexpr (BN <= 64) if (few.kq == 2) return launch_few_kq<BN, EPI, 2>(tmA, tmB, p, few, stream);
-    return few.kq == 1 ? launch_few_kq<BN, EPI, 1>(tmA, tmB, p, few, stream) : cudaErrorInvalidValue;
+    // what few_ring gives: 32 columns four k blocks a stage, of 64 rows two; 64 columns two; 128 one
+    if constexpr (BN == 32) if (few.kq == 4) return launch_few_kq<BN, EPI, 4>(tmA, tmB, p, few, stream);
+    constexpr int KQ = BN <= 64 ? 2 : 1;
+    return few.kq == KQ ? launch_few_kq<BN, EPI, KQ>(tmA, tmB, p, few, stream) : cudaErrorInvalidValue;
 }
 template <int BN>
 static cudaError_t launch_few_bn(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epi, cudaStream_t s) {
