@@ -354,6 +354,8 @@ def _decode_route(L, ctx, nkv):
 # few long contexts: an item is cut over up to 37 CTAs and the last of them merges the pieces (one, two, several, more than four at a time)
 @pytest.mark.parametrize("ctx,nh,nkv,D", [([9000], 32, 8, 128), ([9001, 5, 70], 16, 2, 128), ([5000, 64], 32, 8, 64), ([700], 5, 1, 64), ([3333, 3334, 129], 40, 8, 128)])
 def test_paged_decode_attention_merges_many_pieces(L, ctx, nh, nkv, D):
+    segs, ctas, slots = _decode_route(L, ctx, nkv)
+    assert slots > 0 and ctas != len(ctx) * nkv          # items shared by CTAs
     n = len(ctx); maxp = (max(ctx) + 63) // 64; num_pages = sum((c + 63) // 64 for c in ctx)
     kv = _mk_cache(num_pages, nkv, D, 17)
     g = torch.Generator(device="cpu").manual_seed(6)
@@ -396,11 +398,16 @@ def test_decode_rows_keep_their_bits_whoever_runs_their_pieces(L, n, nh, nkv, D,
     assert not torch.isnan(outs[1]).any() and torch.equal(outs[0], outs[1][:n])
 
 
-# one CTA an item or items cut over CTAs: batches on both sides of the line (an equal share of 2 chunks + 8, + 16 from 64 items on; one item more than CTAs)
+# all pieces of an item on one CTA or shared items: batches on both sides of the line (3 chunks above an equal share; one item more than CTAs)
 @pytest.mark.parametrize("D", [128, 64])
-@pytest.mark.parametrize("nh,nkv,ctx", [(8, 1, [640]), (8, 1, [641]), (32, 8, [640] * 2 + [1]), (32, 8, [1] * 7 + [1152]), (32, 8, [1] * 7 + [1153]), (32, 8, [640] + [3] * 6), (32, 8, [641] + [3] * 6),
-                                        (32, 8, [70, 300, 5, 129] * 9 + [64]), (32, 8, [70, 300, 5, 129] * 9 + [64, 65]), (12, 4, list(range(1, 741, 10)))])
-def test_decode_attention_whole_items_and_cut_ones(L, nh, nkv, D, ctx):
+@pytest.mark.parametrize("nh,nkv,ctx,together", [(8, 1, [320], True), (8, 1, [321], False), (8, 1, [640], False), (8, 1, [641], False), (32, 8, [320] * 2 + [1], True),
+                                                 (32, 8, [321] * 2 + [1], False), (32, 8, [640] * 2 + [1], False),
+                                                 (32, 8, [1] * 7 + [1152], False), (32, 8, [1] * 7 + [1153], False), (32, 8, [3] * 6 + [320], True),
+                                                 (32, 8, [3] * 6 + [321], False), (32, 8, [640] + [3] * 6, False), (32, 8, [641] + [3] * 6, False),
+                                                 (32, 8, [70, 300, 5, 129] * 9 + [64], True), (32, 8, [70, 300, 5, 129] * 9 + [64, 65], False), (12, 4, list(range(1, 741, 10)), False),
+                                                 (12, 4, list(range(1, 449, 7)), True)])
+def test_decode_attention_whole_items_and_cut_ones(L, nh, nkv, D, ctx, together):
+    assert (_decode_route(L, ctx, nkv)[1] == len(ctx) * nkv) == together
     n = len(ctx); maxp = (max(ctx) + 63) // 64; num_pages = sum((c + 63) // 64 for c in ctx)
     kv = _mk_cache(num_pages, nkv, D, 19)
     g = torch.Generator(device="cpu").manual_seed(8)
