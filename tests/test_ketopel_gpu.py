@@ -158,6 +158,39 @@ def test_unequal_requests_in_one_batch_and_reused_pages_and_slots(tmp_path, dtyp
         check(got[r], K.forward(cfg, W, toks[r]), dtype)
 
 
+MIXED = {1: [5] + [1] * 40, 2: [130] + [1] * 12, 3: [33] + [2] * 10, 4: [15] + [2] * 12 + [1] * 3, 5: [31, 2, 1] * 3, 6: [64] + [1, 2, 1, 1] * 3,      # request -> its portions
+         7: [90, 2, 1, 2, 40, 1, 1], 8: [20] + [3, 1] * 5, 9: [250, 1, 2, 1, 2, 1, 1]}
+MIXED_START = {7: 1, 8: 2, 9: 4}
+
+
+def test_mixed_steps_read_only_older_rows_early(tmp_path):
+    """Kernels of decoding rows read states and cache rows ahead of the kernels that make this step's; long recurrences and heavy attention tiles start first.
+    Steps of decoding rows, two- and three-row portions whose own rows share a 16- or 32-row group with older ones (positions 15 to 17, 31 to 34, 63 to
+    65, ..) and prompts of unequal length, in pages and slots that hold another run's rows: a row read before it was written, or a tile that took another's
+    place, shows against the same run on fresh memory (equal bits), each request alone, and the float64 oracle."""
+    cfg = K.make_config([D(heads=4, kv_heads=2, dim=32, vdim=32, conv=3, mlp=F(64)), P(A(heads=4, kv_heads=2, dim=32, vdim=32, dims=8), R(heads=2, dim=32, vdim=32)),
+                         L(heads=4, dim=16, rot_dim=16, vdim=16, kv_rank=64), D(heads=2, kv_heads=1, dim=64, vdim=64, conv=4), P(A(heads=2, kv_heads=1, dim=16, vdim=16, dims=16), R(heads=4, dim=16, vdim=64)),
+                         L(heads=2, dim=32, rot_dim=16, vdim=32, kv_rank=128)], width=64)
+    W = checkpoint(tmp_path, cfg, seed=13)
+    plan = [[(r, sizes[k - MIXED_START.get(r, 0)]) for r, sizes in MIXED.items() if 0 <= k - MIXED_START.get(r, 0) < len(sizes)] for k in range(41)]
+    toks, other = ({r: tokens_of(cfg, sum(sizes), base + r) for r, sizes in MIXED.items()} for base in (50, 70))
+    options = dict(pages=32, slots=len(MIXED))
+    with engine(tmp_path, "bfloat16", **options) as eng:
+        fresh = run_crowd(eng, toks, plan)
+    with engine(tmp_path, "bfloat16", **options) as eng:
+        run_crowd(eng, other, plan)
+        for _ in range(3):
+            got = run_crowd(eng, toks, plan)
+            for r in toks:
+                assert np.array_equal(got[r], fresh[r]), r
+        assert eng.stats()["pages_free"] == 32
+        for r in toks:
+            alone = replay(eng, 20 + r, toks[r], MIXED[r])
+            assert K.rel_err(got[r].astype(np.float64), alone.astype(np.float64)).max() < 5e-2, r
+    for r in toks:
+        check(got[r], K.forward(cfg, W, toks[r]), "bfloat16")
+
+
 @pytest.mark.parametrize("loop", [(0, 1, 4), (1, 3, 2), (3, 6, 2), (0, 6, 1), (5, 6, 3)])
 def test_looped_block_adds_embedding_and_step(tmp_path, loop):
     """Where the block starts and ends, one pass or several.  Oracles that leave out the embedding, or take no or another pass's vector, differ by far
