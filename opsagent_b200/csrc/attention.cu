@@ -261,9 +261,9 @@ __global__ void __launch_bounds__(ATT_THREADS, 2) decode_attention_kernel(const 
     // Merges this CTA came last for: at most its first and its last segment belong to items shared with others, or all of them to one item of its own.  The four warps take a quarter of the columns each
     // (lane: head g, NC consecutive columns from t * NC of the quarter), pieces in slot order (deterministic), eight pieces' loads in flight: a context
     // cut over the whole chip has up to 37 pieces per item, and one warp reading them one after the other was as long as the attention itself.  The
-    // maximum over the pieces comes from the head's four lanes, a quarter of them each, under the first pieces' loads.  us a layer, before the lighter
-    // fences and this order of the merge -> now: 6 x 1750 tokens (heads of 64) 12.5 -> 11.5, 32 x 100 10.9 -> 10.4, 16 x 900 (40 heads) 17.7 -> 16.6, 32 x 1500
-    // 36.8 -> 36.2, 1 x 17000 21.7 -> 21.1, 128 x 1664 135 and 135.  (One record of 48 bytes a CTA instead of offsets, segment, length and page read one
+    // maximum over the pieces comes from the head's four lanes, a quarter of them each, under the first pieces' loads.  us a layer of shared items, before
+    // the lighter fences and this order of the merge -> with them: 6 x 1750 tokens (heads of 64) 12.5 -> 11.5, 16 x 900 (40 heads) 17.7 -> 16.6, 1 x 17000
+    // 21.7 -> 21.1, 128 x 1664 135 and 135.  A CTA that merges pieces of its own takes 1.5 us for it.  (One record of 48 bytes a CTA instead of offsets, segment, length and page read one
     // after the other starts 0.3 us sooner and costs a call's copy more than that.)
     constexpr int NC = D / 16, MP = 8;       // columns per lane: 8 (D = 128) or 4; pieces read at a time
     const int n_merge = merge_s[0];

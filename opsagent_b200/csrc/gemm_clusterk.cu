@@ -1,7 +1,7 @@
 // gemm_clusterk.cu — decode projections with FEW output tiles (o, down, qkv: 32-48 tiles of 128 columns on 148 SMs) as a
 // cluster split-K GEMM: the S CTAs of one thread-block cluster own ONE 128 x 128 output tile and a 1/S slice of K each, reduce their
 // TMEM accumulators through distributed shared memory and finish the epilogue together — no fp32 partial round trip through L2, no
-// consumer launch, no serial tail of a few finishing CTAs (what made the stream-K finisher fusion slower, profiles/r02a).
+// consumer launch, no serial tail of a few finishing CTAs (what made the stream-K finisher fusion slower).
 //
 //   grid = n_tiles x S CTAs, cluster (S,1,1); CTA (tile, r) streams k-blocks [r*kb/S, (r+1)*kb/S) of the tile's weights
 //   warp 0   : TMA producer (weights issued BEFORE griddepcontrol.wait: they depend on no predecessor)

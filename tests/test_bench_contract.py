@@ -1,5 +1,5 @@
-"""The one-line JSON contract of bench.py, checked on the committed outputs of the last GPU run (profiles/): every key the driver
-reads is present with the right type, for both arms.  (bench.py itself needs a B200; this guards the schema on CPU.)"""
+"""The one-line JSON contract of bench.py, checked on committed outputs of earlier GPU runs: every key its readers use is
+present with the right type, for both arms.  (bench.py itself needs a B200; this guards the schema on CPU.)"""
 import json
 import os
 

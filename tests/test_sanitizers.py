@@ -1,6 +1,6 @@
 """Host-side race / memory-error detection: the native HTTP front under TSAN and ASAN+UBSAN with a stub engine, and the parsers of
 untrusted bytes (BPE, tokenizer.json, config JSON, safetensors headers, the ToolPrompt automaton + token masks) under ASAN+UBSAN.  The device side is
-covered by compute-sanitizer runs; results in profiles/r02j_sanitizers.md."""
+covered by earlier compute-sanitizer runs."""
 import pytest
 
 # ---- race / memory-error detection on the host side -----------------------------------------------------------------------

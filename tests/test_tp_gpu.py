@@ -1,7 +1,6 @@
 """Tensor parallelism on >= 2 GPUs: column/row-parallel shards, NVLink peer-memory all-reduce
 written in this repo (no NCCL), vocab-parallel arg-max — against the CPU oracle.  t=4 runs the per-rank head layout of Qwen2.5-32B TP=4,
-t=8 that of Llama-3-70B TP=8 (tests/tp_worker.py).  Skipped on a box with fewer GPUs — `bench.py --gpus N` runs the same check at t=N
-so that the driver's scaling runs carry the verdict."""
+t=8 that of Llama-3-70B TP=8 (tests/tp_worker.py).  Skipped on a box with fewer GPUs — `bench.py --gpus N` runs the same check at t=N."""
 import os
 import subprocess
 import sys

@@ -1,8 +1,8 @@
 """Tensor-parallel parity worker — run as `python -m torch.distributed.run --nproc-per-node T tests/tp_worker.py [case ...]`.
 Rank 0 drives the engine and checks it against the CPU oracle; ranks > 0 serve.  Prints TP_OK on success.
 
-`run_cases()` is also what `bench.py --gpus N` calls after its data-parallel headline (N >= 2), so that the driver's own scaling runs
-carry a tensor-parallel parity verdict at t = N (the GPU test tier runs on a 1-GPU box, where tests/test_tp_gpu.py skips).
+`run_cases()` is also what `bench.py --gpus N` calls after its data-parallel headline (N >= 2), so that scaling runs carry a
+tensor-parallel parity verdict at t = N (on one GPU tests/test_tp_gpu.py skips).
 Default cases per degree: t=2 tiny-llama-tp + tiny-qwen-tp; t=4 tiny-llama-tp + tiny-qwen-tp4 (Qwen2.5-32B TP=4's per-rank layout:
 10 query heads on 2 kv heads, qkv bias); t=8 tiny-llama-tp8 (Llama-3-70B TP=8's per-rank layout: 8 query heads on ONE kv head)."""
 import os

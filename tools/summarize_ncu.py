@@ -1,6 +1,6 @@
-"""Summarise ncu outputs into profiles/ (tracked):
-   python tools/summarize_ncu.py launches gpurun_out/launches_X.csv profiles/rNN_launches.md [n_steps]
-   python tools/summarize_ncu.py report   gpurun_out/prof_X.ncu-rep profiles/rNN_kernels.md
+"""Summarise ncu outputs as markdown:
+   python tools/summarize_ncu.py launches launches.csv launches.md [n_steps]
+   python tools/summarize_ncu.py report   prof.ncu-rep kernels.md
 """
 import collections
 import csv
