@@ -3,6 +3,7 @@ from __future__ import annotations
 
 import ctypes as C
 import json
+from array import array
 from typing import Sequence
 
 from . import _lib
@@ -28,6 +29,15 @@ def _msgs(messages) -> tuple:
         keep += [r, c]
         arr[i].role, arr[i].content = r, c
     return arr, keep
+
+
+def _ints(code: str, values: list) -> array:
+    """Whole numbers as a C array ('i' 32 bits, 'q' 64); other numbers are cut to whole ones."""
+    try:
+        return array(code, values)
+    except TypeError:
+        import numpy as np
+        return array(code, np.array(values, dtype=np.int32 if code == "i" else np.int64).tobytes())
 
 
 class Completion:
@@ -148,15 +158,13 @@ class Engine:
         """One step of a token-level replay: entries = [(request id: int, next tokens, wanted places among them)], all run as one batch
         from the cache and state earlier steps left; `end` lists request ids that are finished after it.  Returns fp32 logits [wanted, vocab]."""
         import numpy as np
-        ids = np.array([e[0] for e in entries], dtype=np.int64)
-        ntok = np.array([len(e[1]) for e in entries], dtype=np.int32)
-        toks = np.array([t for e in entries for t in e[1]], dtype=np.int32)
-        nwant = np.array([len(e[2]) for e in entries], dtype=np.int32)
-        want = np.array([w for e in entries for w in e[2]], dtype=np.int32)
-        ends = np.array(list(end), dtype=np.int64)
-        out = np.empty((int(nwant.sum()), self.info["vocab"]), dtype=np.float32)
-        _check(self._L.oa_trace_step(self._h, len(entries), ids.ctypes.data, ntok.ctypes.data, toks.ctypes.data, nwant.ctypes.data, want.ctypes.data,
-                                     len(ends), ends.ctypes.data, out.ctypes.data, out.shape[0]))
+        # plain arrays: a step of 32 single tokens is described in 12 us, as numpy arrays and their ctypes views in 23, while the GPU waits
+        ids, ends = _ints("q", [e[0] for e in entries]), _ints("q", list(end))
+        ntok, toks = _ints("i", [len(e[1]) for e in entries]), _ints("i", [t for e in entries for t in e[1]])
+        nwant, want = _ints("i", [len(e[2]) for e in entries]), _ints("i", [w for e in entries for w in e[2]])
+        out = np.empty((sum(nwant), self.info["vocab"]), dtype=np.float32)
+        ids_at, ntok_at, toks_at, nwant_at, want_at, ends_at = (a.buffer_info()[0] for a in (ids, ntok, toks, nwant, want, ends))
+        _check(self._L.oa_trace_step(self._h, len(entries), ids_at, ntok_at, toks_at, nwant_at, want_at, len(ends), ends_at, out.ctypes.data, out.shape[0]))
         return out
 
     def kernel_times(self, reset: bool = True) -> dict:

@@ -779,3 +779,17 @@ def test_trace_step_mixes_single_tokens_and_portions(preset):
             g = np.concatenate(got[i])
             assert g.shape == ref[i].shape
             assert np.abs(g - ref[i]).max() < 2.5e-2          # two kernels' roundings, as between the engine and the oracle
+
+
+# the logits of a step come back through four page-locked pieces of 512 KB (32 rows here): fewer rows than a piece, whole pieces, more than there are pieces
+@pytest.mark.parametrize("rows", [1, 31, 32, 33, 128, 129, 290])
+def test_trace_step_brings_all_logits_back(rows):
+    cfg = dict(model="custom", hidden=256, n_layers=1, n_heads=4, n_kv_heads=2, head_dim=64, ffn=512, vocab=4096, seed=5, num_pages=16, max_batch=8, max_seq_len=512,
+               max_step_tokens=512, prefix_cache=0)
+    toks = np.random.default_rng(rows).integers(0, 4096, 300).tolist()
+    with Engine(cfg) as eng:
+        ref = eng.debug_prefill_logits(toks)
+        places = sorted(np.random.default_rng(1).permutation(300)[:rows].tolist())
+        for step in range(2):                              # the second step finds the pieces used
+            out = eng.trace_step([(step, np.array(toks, np.int64), places)], [step])
+            assert np.array_equal(out, ref[places])
