@@ -13,7 +13,10 @@
 //               overlaps the tensor-core work of its neighbours (S and P are double-buffered).
 // Row sums use the unrounded p, P·V the bf16-rounded p — the rounding points the oracle mirrors.  TMEM: 2x128 (S) + D (O).
 
+#include <algorithm>
+
 #include "common.cuh"
+#include "cta_pair.cuh"
 #include "kernels.hpp"
 
 namespace oa {
@@ -70,6 +73,11 @@ OA_DEVINL void store_o_direct(uint32_t addr, float inv, uint16_t* row, bool live
         }
     }
 }
+
+// A row's sum, in one order in all three kernels: of each half (64 keys) of a tile the probabilities of even and of odd keys, those two added, and the tiles'
+// half sums added up over an item's even and over its odd tiles; each of the four is relative to 2^m of its own last tile until the item ends.
+OA_DEVINL float sum_rescale(float m, float m_new) { return m == m_new ? 1.0f : exp2f(m - m_new); }
+OA_DEVINL float sum_add(float l, float f, uint64_t pair) { float a, b; unpack_f32x2(pair, a, b); return __fadd_rn(__fmul_rn(l, f), __fadd_rn(a, b)); }
 
 template <int D>
 struct PtcCfg {
@@ -228,7 +236,7 @@ __global__ void __launch_bounds__(64 + 128 * NWG, 1) prefill_attention_tc_kernel
         constexpr int OC = D / NWG;                                 // O columns this thread rescales / writes
         const int o_base = wg * OC;
         constexpr float kRescaleThreshold = 8.0f;                   // log2 units: p may reach 2^8 before O is rescaled
-        float m_ref = -INFINITY, l_run = 0.f;
+        float m_ref = -INFINITY, l_run = 0.f, l_other = 0.f, m_run = -INFINITY, m_other = -INFINITY;      // row sums of this tile's parity and of the other, and what they are relative to
         for (int j = 0; j < n_kvt; ++j) {
             const int sb = j & 1;
             mbar_wait(&s_full[sb], ((uint32_t)j >> 1) & 1);
@@ -277,18 +285,19 @@ __global__ void __launch_bounds__(64 + 128 * NWG, 1) prefill_attention_tc_kernel
                     }
                     tmem_st_wait();
                     tcgen05_fence_before();
-                    l_run *= alpha;
                 }
                 if (raise) m_ref = mx;
             }
             uint8_t* prow = p_s + sb * Cfg::P_BYTES + row * 128;
-            float psum = 0.f;
+            uint64_t psum = 0;
             const float neg_ref = -m_ref;                                       // p = 2^(s*scale - m_ref): one FFMA + one SFU op per score
 #pragma unroll
             for (int c = 0; c < CH; ++c) {
                 float pr[32];
 #pragma unroll
-                for (int i = 0; i < 32; ++i) { pr[i] = ex2_approx(fmaf(__uint_as_float(v[c][i]), p.scale_log2e, neg_ref)); psum += pr[i]; }
+                for (int i = 0; i < 32; ++i) pr[i] = ex2_approx(fmaf(__uint_as_float(v[c][i]), p.scale_log2e, neg_ref));
+#pragma unroll
+                for (int i = 0; i < 32; i += 2) psum = add_f32x2(psum, pack_f32x2(pr[i], pr[i + 1]));
 #pragma unroll
                 for (int g8 = 0; g8 < 4; ++g8) {                    // four 16-byte chunks (8 keys each)
                     const int key0 = key_base + c * 32 + g8 * 8, hh = key0 >> 6, chunk = (key0 & 63) >> 3;
@@ -298,23 +307,25 @@ __global__ void __launch_bounds__(64 + 128 * NWG, 1) prefill_attention_tc_kernel
                     *reinterpret_cast<uint4*>(prow + hh * Cfg::HALF_BYTES + ((chunk ^ (row & 7)) << 4)) = w;
                 }
             }
-            l_run += psum;
             fence_proxy_async();                                    // P stores must be visible to the tensor-core (async) proxy
             __syncwarp();
             if (lane == 0) mbar_arrive(&p_full[sb]);
+            const float l_new = sum_add(l_run, sum_rescale(m_run, m_ref), psum);
+            l_run = l_other; m_run = m_other; l_other = l_new; m_other = m_ref;
         }
         // A barrier of its own: S of the last tile says that all products up to the third last P·V have landed, no more, and with the second last one still
         // under way a wait for the last one's parity on t_full would find the third last one's phase and pass.  (In the loop S_j says that P_{j-2}·V has
         // landed, so the wait for P_{j-1}·V cannot be taken for an earlier one.)
         mbar_wait(o_full, 0);
         tcgen05_fence_after();
-        {                                                           // row sum = the two key halves' sums (fixed order: half 0 + half 1)
-            const int xb = n_kvt & 1;                               // the buffer the last tile did not use
-            xch[(xb * 2 + wg) * 128 + row] = l_run;
+        float l_row;
+        {                                                           // the two key halves' sums meet, of either parity (every maximum there has been read: P of the last tile stands)
+            xch[wg * 128 + row] = __fmul_rn(l_run, sum_rescale(m_run, m_ref));
+            xch[(2 + wg) * 128 + row] = l_other;
             asm volatile("bar.sync 2, 256;" ::: "memory");
-            l_run = xch[(xb * 2 + 0) * 128 + row] + xch[(xb * 2 + 1) * 128 + row];
+            l_row = (xch[row] + xch[128 + row]) + (xch[256 + row] + xch[384 + row]);
         }
-        const float inv = 1.0f / l_run;
+        const float inv = 1.0f / l_row;
         uint16_t* orow = reinterpret_cast<uint16_t*>(p.out) + (size_t)(tile.q_row0 + q * 32) * p.n_heads * D + (size_t)head * D;
         const uint32_t o_addr = tmem_base + lane_addr + Cfg::T_COL + (uint32_t)o_base;
         if (OC == 64 && tile.n_rows >= q * 32 + 32) store_o_64(p_s + (warp - 2) * 4096, o_addr, inv, orow + o_base, (size_t)p.n_heads * D, lane);      // P has been read by the last product
@@ -340,7 +351,6 @@ __global__ void __launch_bounds__(64 + 128 * NWG, 1) prefill_attention_tc_kernel
 //   warp 0    : TMA (K, Q, V)        warp 1 : tcgen05.mma        warps 4-7 / 8-11 : softmax and output of head A / B, one query row per thread
 // A group with an odd number of heads leaves its last one alone in an item (warpgroup B idles).
 // A row's scores, reference maxima, probabilities and sums are those of the kernel above, in its order: which of the two a batch takes moves no bit.
-// (Four sums per row instead of two are 3 % faster, and moved the last one.)
 // Measured against the kernel above: 4096 rows behind 12288 cached ones, 64 / 8 heads of 128: 1963 -> 1416 us in a burst; five prompts of 1.4 thousand rows,
 // 32 / 8 heads: 184 -> 102 us.  Of that: the issuing warp stays converged (behind one lane its 32 products a tile pair took longer than the tensor core
 // has for them): 1548 -> 1489 and 120 -> 114 us; P is handed over in two parts, so that the first 64 keys are multiplied under the other exponentials:
@@ -553,7 +563,8 @@ __global__ void __launch_bounds__(PtpCfg<D>::THREADS, 1) prefill_attention_pair_
         for (int r = 0; more; ++r) {
             if (x > it.two) { more = ptp_item(p, ppg, r + 1, it); continue; }
             const int qpos = it.tile.pos0 + row;
-            float m_ref = -INFINITY, l_lo = 0.f, l_hi = 0.f;        // row sums of the tiles' lower and upper 64 keys: the order of the kernel above
+            float m_ref = -INFINITY, l_lo = 0.f, l_hi = 0.f, m_run = -INFINITY;                   // row sums of the lower and upper 64 keys, tiles of this one's parity
+            float o_lo = 0.f, o_hi = 0.f, m_other = -INFINITY;                                    // and of the other
             for (int j = 0; j < it.n_kvt; ++j, ++sc) {
                 mbar_wait(&s_full[x], sc & 1);
                 tcgen05_fence_after();
@@ -591,12 +602,11 @@ __global__ void __launch_bounds__(PtpCfg<D>::THREADS, 1) prefill_attention_pair_
                             for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
                             tmem_st_32x32b_x16(o_addr + (uint32_t)c, o);
                         }
-                        l_lo *= alpha; l_hi *= alpha;
                     }
                     if (raise) m_ref = mx;
                 }
                 const uint64_t nref2 = pack_f32x2(-m_ref, -m_ref);
-                float sum[2] = {0.f, 0.f};                          // the two halves' sums, each in ascending keys
+                uint64_t sum[2] = {0, 0};                           // the two halves' sums of even and odd keys
 #pragma unroll
                 for (int hf = 0; hf < 2; ++hf) {                    // 64 scores -> 32 columns of P: p = 2^(s * scale - m_ref); handed over as soon as they stand
 #pragma unroll
@@ -608,7 +618,7 @@ __global__ void __launch_bounds__(PtpCfg<D>::THREADS, 1) prefill_attention_pair_
                             unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(v[2 * hf + c][2 * i]), __uint_as_float(v[2 * hf + c][2 * i + 1])), scale2, nref2), p0, p1);
                             p0 = ex2_approx(p0); p1 = ex2_approx(p1);
                             pw[i] = pack_bf16x2(p0, p1);
-                            sum[hf] += p0; sum[hf] += p1;
+                            sum[hf] = add_f32x2(sum[hf], pack_f32x2(p0, p1));
                         }
                         tmem_st_32x32b_x16(s_addr + (uint32_t)((2 * hf + c) * 16), pw);
                     }
@@ -617,13 +627,15 @@ __global__ void __launch_bounds__(PtpCfg<D>::THREADS, 1) prefill_attention_pair_
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&p_full[2 * x + hf]);
                 }
-                l_lo += sum[0]; l_hi += sum[1];
+                const float f = sum_rescale(m_run, m_ref), n_lo = sum_add(l_lo, f, sum[0]), n_hi = sum_add(l_hi, f, sum[1]);
+                l_lo = o_lo; l_hi = o_hi; m_run = m_other; o_lo = n_lo; o_hi = n_hi; m_other = m_ref;
             }
             PtpItem next;
             more = ptp_item(p, ppg, r + 1, next);                   // read under the item's last product, needed after its output
             mbar_wait(&o_full[x], oc & 1); ++oc;
             tcgen05_fence_after();
-            const float inv = 1.0f / (l_lo + l_hi);
+            const float f = sum_rescale(m_run, m_ref);
+            const float inv = 1.0f / ((__fmul_rn(l_lo, f) + __fmul_rn(l_hi, f)) + (o_lo + o_hi));
             uint16_t* orow = reinterpret_cast<uint16_t*>(p.out) + (size_t)(it.tile.q_row0 + q * 32) * p.n_heads * D + (size_t)(it.head + x) * D;
             // a warp with rows missing: their pieces are few (sixteen prompts of 30 rows: 11.1 us against 12.7 through shared memory)
             if (D == 64 || it.tile.n_rows < q * 32 + 32) store_o_direct<D>(o_addr, inv, orow + (size_t)lane * p.n_heads * D, row < it.tile.n_rows);
@@ -638,6 +650,384 @@ __global__ void __launch_bounds__(PtpCfg<D>::THREADS, 1) prefill_attention_pair_
     tcgen05_fence_before();
     __syncthreads();
     if (warp == 1) { tcgen05_fence_after(); tmem_dealloc<Cfg::TMEM_COLS>(tmem_base); }
+}
+
+// ---------------------------------------------------------------------------------------------
+// Two heads of one key/value group on a CTA PAIR, heads of 128.
+//
+// The kernel above is bound by a head's chain in a tile: its S may only be computed once the P that stands over the last one has been multiplied, and TMEM has
+// no room for a second S of both heads.  Here each CTA of a pair carries ONE head's 128 rows, so TMEM holds three S tiles and O, and the two softmax
+// warpgroups take the tiles in turn: while one takes the exponentials of tile t, the other fetches S and finds the maxima of t + 1, and the tensor core
+// runs P V of t - 1 and S of t + 2.  What a head still does in order is one value a row: a tile's reference maximum follows from the last one's, so it goes from
+// warpgroup to warpgroup as soon as the maxima stand.  Keys and values are shared by the pair: a product is 256 x 128 x 16 (cta_group::2) with half of B in
+// each CTA, so each loads one of a tile's two K pages and 64 of V's 128 columns, half of what a CTA alone would have to fetch for its head (which would be the
+// L2's limit: 64 KB a tile in 1100 cycles).
+//   warp 0     : TMA: this CTA's Q (two items ahead), K page and V half           warp 1 (even CTA): tcgen05.mma for both
+//   warps 4-11 : softmax of even and odd tiles, one query row per thread         warps 12-15: output, while the next item's tiles run
+// A row's sums are kept per warpgroup (even and odd tiles of the item) and joined at its end, as in the kernels above: the same bits.
+// us, two heads a CTA -> here: 4096 rows behind 12288, 64 / 8 heads 1410 -> 1302; five prompts of 1.4 thousand rows, 32 / 8 heads 97 -> 84; 1000 rows behind 6000
+// 104 -> 88; 600 rows 14.7 -> 11.2 (one head a CTA: 14.7); 300 rows behind 6000 57 -> 46 (one head a CTA).  A launch costs 2 us more.
+// What bounds it now: a warpgroup takes 2600 cycles a tile, 1650 of them exponentials (1024 alone), 550 fetching S, the maxima and the reference, 120 waiting
+// for S; tensor and special-function pipes are busy 79 %, and the clock is down to 1.6 GHz in the long case (1.76 in the short ones).
+// Waits and arrivals are of CTA scope: what crosses the pair stands in TMEM (ordered by tcgen05.fence) or comes by TMA; with acquire and release of cluster
+// scope a tile took 2100 cycles instead of 1300.  Slower: S of two tiles and P of two in places of their own, S issued as soon as it is fetched (84 -> 90 us),
+// P handed over in two halves (85.5); no faster: the first item and its pages looked up ahead of the set-up.
+// ---------------------------------------------------------------------------------------------
+struct PcpCfg {
+    static constexpr int D = 128, STAGES = 4, S_BUFS = 3;
+    static constexpr int Q_BYTES = 128 * D * 2, Q_HALF = 128 * 128;
+    static constexpr int KV_BYTES = 64 * D * 2, K_HALF = 64 * 128;       // a CTA's share of a K or V tile of 128 keys: 64 keys x 128, 128 keys x 64 columns
+    static constexpr int OUT_WARP_BYTES = 32 * D * 2;
+    static constexpr int ROWS_BYTES = 2 * 128 * 4;                       // one value per row and softmax warpgroup
+    static constexpr int SMEM_BYTES = 2 * Q_BYTES + 2 * STAGES * KV_BYTES + 4 * OUT_WARP_BYTES + 2 * ROWS_BYTES + 512;
+    static_assert(SMEM_BYTES <= 232448, "shared memory budget of one CTA");
+    static constexpr uint32_t O_COL = S_BUFS * 128;
+    static constexpr int THREADS = 4 * 128;
+    static constexpr int REGS_CONTROL = 64, REGS_OUT = 64, REGS_SOFTMAX = 192;
+    static_assert(REGS_CONTROL + REGS_OUT + 2 * REGS_SOFTMAX <= 4 * 128, "an increase draws on what the launch gave: 512 threads x 128 registers");
+};
+
+// item of this pair of CTAs in round r (as above: heaviest first, every second round in reverse)
+struct PcpItem { PrefillTile tile; int kvh, head0, n_kvt; };
+OA_DEVINL bool pcp_item(const PrefillAttnParams& p, int ppg, int round, PcpItem& it) {
+    const int G = (int)gridDim.x >> 1, pair = (int)blockIdx.x >> 1, per_tile = p.n_kv * ppg;
+    const int idx = round * G + ((round & 1) ? G - 1 - pair : pair);
+    if (idx >= p.n_tiles * per_tile) return false;
+    const int ti = idx / per_tile, hp = idx - ti * per_tile;
+    it.kvh = hp / ppg;
+    it.head0 = it.kvh * 2 * ppg + 2 * (hp - it.kvh * ppg);
+    it.tile = p.tiles[ti];
+    it.n_kvt = (it.tile.pos0 + it.tile.n_rows + KV_TILE - 1) / KV_TILE;
+    return true;
+}
+
+__global__ void __launch_bounds__(PcpCfg::THREADS, 1) prefill_attention_cluster_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_kv,
+                                                                                       const PrefillAttnParams p, const int64_t layer_row0, const int64_t kv_stride_rows) {
+    using Cfg = PcpCfg;
+    constexpr int D = Cfg::D, STAGES = Cfg::STAGES;
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t* q_s = smem_raw;                                     // [item & 1]
+    uint8_t* k_s = q_s + 2 * Cfg::Q_BYTES;                       // [STAGES]
+    uint8_t* v_s = k_s + STAGES * Cfg::KV_BYTES;                 // [STAGES]
+    uint8_t* out_s = v_s + STAGES * Cfg::KV_BYTES;               // [4 warps]
+    float* sum_s = reinterpret_cast<float*>(out_s + 4 * Cfg::OUT_WARP_BYTES);      // [warpgroup][row]: row sums of the item at hand
+    float* ref_s = sum_s + 2 * 128;                              // [warpgroup][row]: reference maximum after the warpgroup's last tile
+    uint64_t* bars = reinterpret_cast<uint64_t*>(ref_s + 2 * 128);
+    uint64_t* q_full = bars;                  // [2]  even CTA
+    uint64_t* q_empty = q_full + 2;           // [2]
+    uint64_t* k_full = q_empty + 2;           // [STAGES]  even CTA
+    uint64_t* k_empty = k_full + STAGES;
+    uint64_t* v_full = k_empty + STAGES;      // [STAGES]  even CTA
+    uint64_t* v_empty = v_full + STAGES;      // [STAGES]  also: P V of this tile has landed
+    uint64_t* s_full = v_empty + STAGES;      // [6]  two per buffer: every one is waited for by one warpgroup alone, phase by phase
+    uint64_t* p_full = s_full + 6;            // [S_BUFS]  even CTA
+    uint64_t* r_full = p_full + Cfg::S_BUFS;  // [2 warpgroups][4 warps]  a warp's reference maxima stand
+    uint64_t* l_full = r_full + 8;            // the item's row sums stand
+    uint64_t* l_empty = l_full + 1;           // ... and have been read
+    uint64_t* o_full = l_empty + 1;           // the item's last P V has landed
+    uint64_t* o_empty = o_full + 1;           // even CTA: O has been read in both
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_empty + 1);
+
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // warp: uniform, and known to be
+    const uint32_t rank = gp_rank();
+    const int ppg = p.n_heads / p.n_kv / 2;
+    PcpItem it;
+
+    if (warp == 0 && lane == 0) {
+        tma_prefetch_desc(&tm_q); tma_prefetch_desc(&tm_kv);
+        for (int i = 0; i < 2; ++i) { mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1); }
+        for (int i = 0; i < STAGES; ++i) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
+        for (int i = 0; i < 6; ++i) mbar_init(&s_full[i], 1);
+        for (int i = 0; i < Cfg::S_BUFS; ++i) mbar_init(&p_full[i], 8);
+        for (int i = 0; i < 8; ++i) mbar_init(&r_full[i], 1);
+        mbar_init(l_full, 8); mbar_init(l_empty, 4); mbar_init(o_full, 1); mbar_init(o_empty, 8);
+        fence_barrier_init();
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_slot)) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+    gp_cluster_sync();                               // the other CTA's barriers are initialised before anything arrives on them
+    tcgen05_fence_after();
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    griddep_launch();
+
+    if (warp < 4) {
+        reg_dec<Cfg::REGS_CONTROL>();
+        if (warp == 0) {
+            griddep_wait();
+            uint32_t kc = 0;
+            int r = 0;
+            PcpItem next;
+            bool more = pcp_item(p, ppg, 0, it);
+            for (; more; ++r, it = next) {
+                const int n_kvt = __shfl_sync(0xffffffffu, it.n_kvt, 0);
+                const int32_t* bt = p.block_tables + (size_t)it.tile.seq * p.max_pages_per_seq;
+                auto page_row = [&](int pi, int fallback) { return layer_row0 + ((int64_t)bt[pi < p.max_pages_per_seq ? pi : fallback] * p.n_kv + it.kvh) * 64; };   // a missing second page is fully masked anyway
+                int64_t r0 = page_row(0, 0), r1 = page_row(1, 0);
+                for (int j = 0; j < n_kvt; ++j, ++kc) {
+                    const uint32_t st = kc % STAGES, ph = (kc / STAGES) & 1;
+                    mbar_wait(&k_empty[st], ph ^ 1);
+                    if (elect_one()) {
+                        uint8_t* dst = k_s + st * Cfg::KV_BYTES;
+                        if (rank == 0) mbar_expect_tx(&k_full[st], 2 * Cfg::KV_BYTES);              // both CTAs' shares
+                        const uint32_t bar = gp_mapa(&k_full[st], 0);
+                        const int32_t row = (int32_t)(rank ? r1 : r0);
+                        gp_tma_load(dst, &tm_kv, bar, 0, row, kEvictLast);
+                        gp_tma_load(dst + Cfg::K_HALF, &tm_kv, bar, 64, row, kEvictLast);
+                    }
+                    __syncwarp();
+                    if (j == 0) {
+                        const int qb = r & 1;
+                        mbar_wait(&q_empty[qb], (((uint32_t)r >> 1) & 1) ^ 1);
+                        if (elect_one()) {
+                            uint8_t* dst = q_s + qb * Cfg::Q_BYTES;
+                            if (rank == 0) mbar_expect_tx(&q_full[qb], 2 * Cfg::Q_BYTES);
+                            const uint32_t bar = gp_mapa(&q_full[qb], 0);
+                            const int32_t col = (it.head0 + (int)rank) * D;
+                            gp_tma_load(dst, &tm_q, bar, col, it.tile.q_row0, kEvictFirst);
+                            gp_tma_load(dst + Cfg::Q_HALF, &tm_q, bar, col + 64, it.tile.q_row0, kEvictFirst);
+                        }
+                        __syncwarp();
+                        more = pcp_item(p, ppg, r + 1, next);                  // read now, needed an item later
+                    }
+                    int64_t n0 = r0, n1 = r1;                                  // the next tile's pages are looked up while this one's slot is waited for
+                    if (j + 1 < n_kvt) { n0 = page_row(2 * j + 2, 0); n1 = page_row(2 * j + 3, 2 * j + 2); }
+                    mbar_wait(&v_empty[st], ph ^ 1);
+                    if (elect_one()) {
+                        uint8_t* dst = v_s + st * Cfg::KV_BYTES;
+                        if (rank == 0) mbar_expect_tx(&v_full[st], 2 * Cfg::KV_BYTES);
+                        const uint32_t bar = gp_mapa(&v_full[st], 0);
+                        gp_tma_load(dst, &tm_kv, bar, (int)rank * 64, (int32_t)(r0 + kv_stride_rows), kEvictLast);
+                        gp_tma_load(dst + 8192, &tm_kv, bar, (int)rank * 64, (int32_t)(r1 + kv_stride_rows), kEvictLast);
+                    }
+                    __syncwarp();
+                    r0 = n0; r1 = n1;
+                }
+            }
+            for (int i = 0; i < STAGES; ++i, ++kc) { mbar_wait(&k_empty[kc % STAGES], ((kc / STAGES) & 1) ^ 1); mbar_wait(&v_empty[kc % STAGES], ((kc / STAGES) & 1) ^ 1); }   // the last
+            for (int i = 0; i < 2; ++i, ++r) mbar_wait(&q_empty[r & 1], (((uint32_t)r >> 1) & 1) ^ 1);                  // releases have arrived here before the CTA may go
+        } else if (warp == 1 && rank == 0) {
+            // The whole warp walks the loop, an elected lane issues: descriptors stay in uniform registers.  S runs two tiles ahead of P V, across items.
+            constexpr uint32_t idesc_s = umma_idesc_bf16(256, KV_TILE), idesc_o = umma_idesc_bf16_bmn(256, D);
+            const uint64_t q_desc = umma_desc_sw128(smem_u32(q_s)), k_desc = umma_desc_sw128(smem_u32(k_s)), v_desc = umma_desc_sw128_mn(smem_u32(v_s), (uint32_t)Cfg::KV_BYTES, 1024u);
+            PcpItem s_it, nxt;
+            uint32_t sc = 0;                                                   // tiles whose S has been issued
+            int s_r = 0, s_j = 0;
+            bool s_more = pcp_item(p, ppg, 0, s_it);
+            int s_n = s_more ? __shfl_sync(0xffffffffu, s_it.n_kvt, 0) : 0;
+            auto issue_s = [&] {
+                if (!s_more) return;
+                if (s_j == 0) mbar_wait(&q_full[s_r & 1], ((uint32_t)s_r >> 1) & 1);
+                const uint32_t st = sc % STAGES;
+                mbar_wait(&k_full[st], (sc / STAGES) & 1);
+                tcgen05_fence_after();
+                if (elect_one()) {
+                    const uint64_t a = q_desc + (uint64_t)((s_r & 1) * (Cfg::Q_BYTES >> 4)), b = k_desc + (uint64_t)(st * (Cfg::KV_BYTES >> 4));
+                    const uint32_t d = tmem_base + (sc % Cfg::S_BUFS) * 128;
+#pragma unroll
+                    for (int ks = 0; ks < D / 16; ++ks)
+                        gp_umma(d, a + (uint64_t)(((ks >> 2) * Cfg::Q_HALF + (ks & 3) * 32) >> 4), b + (uint64_t)(((ks >> 2) * Cfg::K_HALF + (ks & 3) * 32) >> 4), idesc_s, ks > 0 ? 1u : 0u);
+                    gp_commit(&s_full[sc % 6]);
+                    gp_commit(&k_empty[st]);
+                    if (s_j + 1 == s_n) gp_commit(&q_empty[s_r & 1]);
+                }
+                __syncwarp();
+                ++sc;
+                if (++s_j == s_n) {
+                    s_j = 0; ++s_r;
+                    s_more = pcp_item(p, ppg, s_r, s_it);
+                    s_n = s_more ? __shfl_sync(0xffffffffu, s_it.n_kvt, 0) : 0;
+                }
+            };
+            issue_s(); issue_s();
+            uint32_t t = 0;
+            bool more = pcp_item(p, ppg, 0, it);
+            for (int r = 0; more; ++r, it = nxt) {
+                const int n_kvt = __shfl_sync(0xffffffffu, it.n_kvt, 0);
+                more = pcp_item(p, ppg, r + 1, nxt);                           // read now, needed an item later
+                for (int j = 0; j < n_kvt; ++j, ++t) {
+                    issue_s();                                                 // over the P of tile t - 1, whose product is ahead of it
+                    const uint32_t st = t % STAGES;
+                    if (j == 0) mbar_wait(o_empty, ((uint32_t)r & 1) ^ 1);       // O of the last item has been read
+                    mbar_wait(&v_full[st], (t / STAGES) & 1);
+                    mbar_wait(&p_full[t % Cfg::S_BUFS], (t / Cfg::S_BUFS) & 1);
+                    tcgen05_fence_after();
+                    if (elect_one()) {
+                        const uint64_t b = v_desc + (uint64_t)(st * (Cfg::KV_BYTES >> 4));
+                        const uint32_t a = tmem_base + (t % Cfg::S_BUFS) * 128;
+#pragma unroll
+                        for (int ks = 0; ks < KV_TILE / 16; ++ks) gp_umma_ta(tmem_base + Cfg::O_COL, a + ks * 8, b + (uint64_t)(ks * (2048 >> 4)), idesc_o, (j | ks) != 0 ? 1u : 0u);
+                        gp_commit(&v_empty[st]);
+                        if (j + 1 == n_kvt) gp_commit(o_full);
+                    }
+                    __syncwarp();
+                }
+            }
+        }
+    } else if (warp < 12) {
+        reg_inc<Cfg::REGS_SOFTMAX>();
+        const int q = warp & 3, w = (warp - 4) >> 2;                // TMEM lanes 32 q ..; this warpgroup takes tiles w, w + 2, .. of all there are
+        const int row = q * 32 + lane;
+        const uint32_t lane_base = tmem_base + ((uint32_t)(q * 32) << 16), o_addr = lane_base + Cfg::O_COL;
+        constexpr float kRescaleThreshold = 8.0f;                   // log2 units: p may reach 2^8 before O is rescaled
+        const uint64_t scale2 = pack_f32x2(p.scale_log2e, p.scale_log2e);
+        uint32_t t = 0;                                             // tiles so far, of both warpgroups
+        auto other_ref = [&] {                                      // the reference maximum after tile t - 1
+            mbar_wait(&r_full[(w ^ 1) * 4 + q], ((t - 1) >> 1) & 1);
+            return ref_s[(w ^ 1) * 128 + row];
+        };
+        bool more = pcp_item(p, ppg, 0, it);
+        for (int r = 0; more; ++r) {
+            const int n_kvt = it.n_kvt, pos0 = it.tile.pos0, qpos = pos0 + row;
+            more = pcp_item(p, ppg, r + 1, it);                     // read now, needed an item later
+            float m_own = -INFINITY, l_lo = 0.f, l_hi = 0.f;        // this warpgroup's row sums, relative to 2^m_own
+            for (int j = 0; j < n_kvt; ++j, ++t) {
+                if ((int)(t & 1) != w) continue;
+                const uint32_t s_addr = lane_base + (t % Cfg::S_BUFS) * 128;
+                mbar_wait(&s_full[t % 6], (t / 6) & 1);
+                tcgen05_fence_after();
+                uint32_t v[4][32];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) tmem_ld_32x32b_x32(s_addr + (uint32_t)(c * 32), v[c]);
+                const float m_last = j > 0 ? other_ref() : -INFINITY;               // under the loads: it has stood for half a tile's time
+#pragma unroll
+                for (int c = 0; c < 4; ++c) tmem_ld_wait_for(v[c]);
+                if (j * KV_TILE + KV_TILE - 1 > pos0 + q * 32) {                    // some (row, key) pairs of this warp are masked
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        if (j * KV_TILE + c * 32 + 31 > pos0 + q * 32) {
+#pragma unroll
+                            for (int i = 0; i < 32; ++i) if (j * KV_TILE + c * 32 + i > qpos) v[c][i] = 0xff800000u;
+                        }
+                }
+                float m[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    m[k] = __uint_as_float(v[0][k]);
+#pragma unroll
+                    for (int i = 4; i < 124; i += 8) m[k] = fmax3_nan(m[k], __uint_as_float(v[(i + k) / 32][(i + k) % 32]), __uint_as_float(v[(i + k + 4) / 32][(i + k + 4) % 32]));
+                    m[k] = fmax_nan(m[k], __uint_as_float(v[3][28 + k]));
+                }
+                const float mx = fmax_nan(fmax3_nan(m[0], m[1], m[2]), m[3]) * p.scale_log2e;       // the scale is positive
+                // always true on tile 0 (key 0 is visible to every row); also where a score is NaN: then the reference, every p and the row's result are
+                const bool raise = !(mx <= m_last + kRescaleThreshold);
+                const float m_ref = raise ? mx : m_last;
+                ref_s[w * 128 + row] = m_ref;                       // the other warpgroup has read the last one: it has published since
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&r_full[w * 4 + q]);
+                if (j > 0 && __any_sync(0xffffffffu, raise)) {
+                    mbar_wait(&v_empty[(t - 1) % STAGES], ((t - 1) / STAGES) & 1);    // O holds every tile before this one (S_t says that P V of t - 3 has landed: no earlier phase is taken for this)
+                    tcgen05_fence_after();
+                    const float alpha = raise ? exp2f(m_last - mx) : 1.0f;
+#pragma unroll 1
+                    for (int c = 0; c < D; c += 16) {
+                        uint32_t o[16];
+                        tmem_ld_32x32b_x16(o_addr + (uint32_t)c, o);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                        tmem_st_32x32b_x16(o_addr + (uint32_t)c, o);
+                    }
+                }
+                const uint64_t nref2 = pack_f32x2(-m_ref, -m_ref);
+                uint64_t sum[2] = {0, 0};                           // the two halves' sums of even and odd keys
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {                       // 128 scores -> 64 columns of P: p = 2^(s * scale - m_ref)
+                    uint32_t pw[16];
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        float p0, p1;
+                        unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(v[c][2 * i]), __uint_as_float(v[c][2 * i + 1])), scale2, nref2), p0, p1);
+                        p0 = ex2_approx(p0); p1 = ex2_approx(p1);
+                        pw[i] = pack_bf16x2(p0, p1);
+                        sum[c >> 1] = add_f32x2(sum[c >> 1], pack_f32x2(p0, p1));
+                    }
+                    tmem_st_32x32b_x16(s_addr + (uint32_t)(c * 16), pw);
+                }
+                tmem_st_wait();
+                tcgen05_fence_before();
+                __syncwarp();
+                if (lane == 0) gp_arrive_tmem(gp_mapa(&p_full[t % Cfg::S_BUFS], 0));
+                const float f = sum_rescale(m_own, m_ref);
+                l_lo = sum_add(l_lo, f, sum[0]); l_hi = sum_add(l_hi, f, sum[1]); m_own = m_ref;
+            }
+            // the item is over and ended at the reference of its last tile, which either warpgroup may have had
+            const float f = sum_rescale(m_own, (int)(t & 1) == w ? other_ref() : m_own);
+            mbar_wait(l_empty, ((uint32_t)r & 1) ^ 1);
+            sum_s[w * 128 + row] = __fmul_rn(l_lo, f) + __fmul_rn(l_hi, f);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(l_full);
+        }
+    } else {
+        // Output: O scaled, rounded and written in whole lines while the next item's tiles run.  O is free as soon as it stands in shared memory.
+        reg_dec<Cfg::REGS_OUT>();
+        constexpr int ROW_BYTES = D * 2, CH = ROW_BYTES / 16, ROWS_AT_ONCE = 32 / CH;      // 16-byte pieces of a row; rows a store instruction covers
+        const int q = warp & 3, row = q * 32 + lane;
+        uint8_t* stage = out_s + q * Cfg::OUT_WARP_BYTES;
+        const uint32_t o_addr = tmem_base + ((uint32_t)(q * 32) << 16) + Cfg::O_COL;
+        griddep_wait();                                             // the output may still be read by a predecessor
+        bool more = pcp_item(p, ppg, 0, it);
+        for (int r = 0; more; ++r) {
+            const int rows_here = it.tile.n_rows - q * 32;          // of this warp's 32
+            uint16_t* orow = reinterpret_cast<uint16_t*>(p.out) + (size_t)(it.tile.q_row0 + q * 32) * p.n_heads * D + (size_t)(it.head0 + (int)rank) * D;
+            more = pcp_item(p, ppg, r + 1, it);
+            mbar_wait(l_full, (uint32_t)r & 1);
+            const float inv = 1.0f / (sum_s[row] + sum_s[128 + row]);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(l_empty);
+            mbar_wait(o_full, (uint32_t)r & 1);
+            tcgen05_fence_after();
+#pragma unroll
+            for (int c = 0; c < D; c += 32) {
+                uint32_t o[32];
+                tmem_ld_32x32b_x32(o_addr + (uint32_t)c, o);
+                tmem_ld_wait_for(o);
+#pragma unroll
+                for (int i = 0; i < 32; i += 8) {
+                    uint4 u;
+                    u.x = pack_bf16x2(__uint_as_float(o[i]) * inv, __uint_as_float(o[i + 1]) * inv);
+                    u.y = pack_bf16x2(__uint_as_float(o[i + 2]) * inv, __uint_as_float(o[i + 3]) * inv);
+                    u.z = pack_bf16x2(__uint_as_float(o[i + 4]) * inv, __uint_as_float(o[i + 5]) * inv);
+                    u.w = pack_bf16x2(__uint_as_float(o[i + 6]) * inv, __uint_as_float(o[i + 7]) * inv);
+                    *reinterpret_cast<uint4*>(stage + lane * ROW_BYTES + ((((c + i) >> 3) ^ (lane & 7)) << 4)) = u;
+                }
+            }
+            tcgen05_fence_before();
+            __syncwarp();
+            if (lane == 0) gp_arrive_tmem(gp_mapa(o_empty, 0));
+#pragma unroll 4
+            for (int i = 0; i < 32; i += ROWS_AT_ONCE) {
+                const int rr = i + lane / CH, ch = lane % CH;
+                if (rr < rows_here)
+                    *reinterpret_cast<uint4*>(orow + (size_t)rr * p.n_heads * D + ch * 8) = *reinterpret_cast<const uint4*>(stage + rr * ROW_BYTES + ((ch ^ (rr & 7)) << 4));
+            }
+            __syncwarp();
+        }
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+    gp_cluster_sync();                               // nothing of the pair may still arrive on, read from or allocate in a CTA that has gone
+    if (warp == 1) {
+        tcgen05_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");
+    }
+}
+
+static cudaError_t launch_pcp(const CUtensorMap* tm_q, const CUtensorMap* tm_kv, const KvLayout& kv, const PrefillAttnParams& p, int items, int sms, cudaStream_t s) {
+    auto kern = prefill_attention_cluster_kernel;
+    static bool attr_done[16] = {};
+    { cudaError_t e = ensure_dynamic_smem(kern, PcpCfg::SMEM_BYTES, attr_done); if (e != cudaSuccess) return e; }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * std::min(items, sms / 2)); cfg.blockDim = dim3(PcpCfg::THREADS); cfg.dynamicSmemBytes = PcpCfg::SMEM_BYTES; cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension; attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    count_launch();
+    return cudaLaunchKernelEx(&cfg, kern, *tm_q, *tm_kv, p, (int64_t)p.layer * kv.layer_stride_rows, kv.kv_stride_rows);
 }
 
 template <int D>
@@ -663,17 +1053,37 @@ static int prefill_sm_count() {
     return n;
 }
 
+// Which of the three.  us, kernels alone, 32 and 64 heads over 8, 145 batches of 1 to 32 prompts of 100 to 1400 rows behind 0 to 3000 cached ones: with n tiles of
+// 128 keys for the longest item, one head a CTA takes 4.9 + 1.0 n while all its CTAs are resident (up to half as many items of two heads as SMs; one query tile
+// of 100 rows: n = 1 5.8, 4 8.9, 11 15.9, 25 29.9); two heads a CTA 6.3 + 2.6 for each further round over the SMs + 1.72 a tile on the longest CTA (96 items of
+// 1, 4, 11 and 25 tiles: 8.0, 13.3, 25.6, 49.2; 1024 of 1: 32.1); a CTA pair 7.1 + 1.25 for each further round over the pairs + 0.77 a tile (7.5, 9.9, 14.6, 24.7 for
+// the first, 10.0, 15.0, 25.6, 47.2 and 33.8 for the second).  Ragged items: the longest CTA has the longest item at least, else the mean one a round.  The least
+// estimate was within 2 % of the fastest kernel for all but 3 batches (5 %).  A pair's two CTAs take the two heads of an item, so groups with an odd head stay on
+// the other two, and so do heads of 64 (a product of 64 columns would leave each CTA 32 of V's).
+PrefillKernel prefill_attention_kernel_of(int n_tiles, int key_tiles, int max_key_tiles, int n_heads, int n_kv, int head_dim) {
+    const int sms = prefill_sm_count(), grp = n_heads / n_kv, items = n_tiles * n_kv * ((grp + 1) / 2);
+    const bool few = items <= sms / 2, pairs_ok = head_dim == 128 && grp % 2 == 0 && sms >= 2 && key_tiles > 0;
+    // (few items of any kind and ungrouped heads: 400 rows behind 6000, 32 / 8 heads, 64 items: one head a CTA 58 us, two 91)
+    const PrefillKernel plain = grp > 1 && !few ? PREFILL_TWO_HEADS : PREFILL_ONE_HEAD;
+    if (!pairs_ok) return plain;
+    const double mean = (double)key_tiles / n_tiles, longest = max_key_tiles;
+    auto rounds = [&](int ctas) { return (items + ctas - 1) / ctas; };
+    const int r_sm = rounds(sms), r_pair = rounds(sms / 2);
+    const double us_plain = few ? 4.9 + 1.0 * longest : 6.3 + 2.6 * (r_sm - 1) + 1.72 * std::max(longest, mean * r_sm);
+    const double us_pair = 7.1 + 1.25 * (r_pair - 1) + 0.77 * std::max(longest, mean * r_pair);
+    return us_pair < us_plain ? PREFILL_CTA_PAIR : plain;
+}
+
 cudaError_t launch_prefill_attention_tc(const CUtensorMap* tm_q, const CUtensorMap* tm_kv, const KvLayout& kv, const PrefillAttnParams& p, cudaStream_t s) {
     if (p.n_tiles <= 0) return cudaSuccess;
     if (kv.page_size != 64 || p.n_heads % p.n_kv != 0) return cudaErrorInvalidValue;
-    const int grp = p.n_heads / p.n_kv, items = p.n_tiles * p.n_kv * ((grp + 1) / 2);
-    const int sms = prefill_sm_count();
-    // Up to half as many items as SMs, twice as many single-head CTAs are all resident at once and each is done sooner (32 / 8 heads, 400 rows
-    // behind 6000, 64 items: 58 us against 91 in pairs); above that the pairs win (700 rows behind 4000, 96 items: 82 -> 73; 614 rows, 80 items: 14.8
-    // and 14.9; 640 behind 3000, 80 items: 64 -> 59; 850 behind 2000, 112 items: 54 -> 48).
-    if (grp > 1 && items > sms / 2) {
+    const int grp = p.n_heads / p.n_kv, items = p.n_tiles * p.n_kv * ((grp + 1) / 2), sms = prefill_sm_count();
+    const PrefillKernel k = prefill_attention_kernel_of(p.n_tiles, p.key_tiles, p.max_key_tiles, p.n_heads, p.n_kv, kv.head_dim);
+    if (k == PREFILL_CTA_PAIR) return launch_pcp(tm_q, tm_kv, kv, p, items, sms, s);
+    if (k == PREFILL_TWO_HEADS) {
         if (kv.head_dim == 128) return launch_ptp<128>(tm_q, tm_kv, kv, p, items, sms, s);
         if (kv.head_dim == 64) return launch_ptp<64>(tm_q, tm_kv, kv, p, items, sms, s);
+        return cudaErrorInvalidValue;
     }
     if (kv.head_dim == 128) return launch_ptc<128>(tm_q, tm_kv, kv, p, s);
     if (kv.head_dim == 64) return launch_ptc<64>(tm_q, tm_kv, kv, p, s);

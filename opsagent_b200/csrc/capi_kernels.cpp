@@ -190,6 +190,17 @@ int oa_host_gemm_pair_width(int32_t M, int32_t N, int32_t K, int32_t epilogue, i
     return c.kernel == GEMM_PAIR ? c.width : 0;
 }
 
+int oa_host_prefill_attention_kernel(const int32_t* ctx_lens, const int32_t* q_lens, int32_t n_seqs, int32_t n_heads, int32_t n_kv, int32_t head_dim) {
+    if (n_seqs < 0 || n_kv <= 0 || n_heads <= 0 || n_heads % n_kv != 0) return OA_ERR_BAD_REQUEST;
+    int n_tiles = 0, sum = 0, longest = 0;
+    for (int i = 0; i < n_seqs; ++i)
+        for (int r = 0; r < q_lens[i]; r += PREFILL_TILE_ROWS) {
+            const int k = (ctx_lens[i] - q_lens[i] + std::min(r + PREFILL_TILE_ROWS, q_lens[i]) + 127) / 128;
+            ++n_tiles; sum += k; longest = std::max(longest, k);
+        }
+    return (int)prefill_attention_kernel_of(n_tiles, sum, longest, n_heads, n_kv, head_dim);
+}
+
 static int paged_attention(const void* q, void* out, const void* kv_cache, int32_t num_pages, const int32_t* block_tables,
                            int32_t max_pages_per_seq, const int32_t* ctx_lens, const int32_t* q_lens, int32_t n_seqs,
                            int32_t n_heads, int32_t n_kv, int32_t head_dim, int32_t force_splits, void* stream) {
@@ -245,6 +256,7 @@ static int paged_attention(const void* q, void* out, const void* kv_cache, int32
     if (!d_meta.p) return OA_ERR_INTERNAL;
     PrefillAttnParams a{}; a.q = q; a.out = out; a.block_tables = (const int32_t*)((const char*)d_meta.p + o_bt); a.max_pages_per_seq = max_pages_per_seq;
     a.tiles = (const PrefillTile*)((const char*)d_meta.p + o_tiles); a.n_tiles = (int)tiles.size(); a.layer = 0; a.n_heads = n_heads; a.n_kv = n_kv; a.scale_log2e = scale_log2e;
+    set_key_tiles(a, tiles.data(), tiles.size());
     const char* leg = std::getenv("OA_PREFILL_ATTN");
     const bool legacy = leg && std::string(leg) == "legacy";
     CUtensorMap tmq;

@@ -442,11 +442,13 @@ void DeviceModel::forward(const StepInput& in, float* logits_out) {
         zero_counters_.assign(plan_.n_cut + 1, 0);
         o_cnt = put(zero_counters_.data(), zero_counters_.size());     // merge counters start every step at zero
     }
+    PrefillAttnParams key_tiles{};
     if (!in.decode) {
         // heaviest query tiles (most visible keys) first: the causal triangle otherwise leaves a long tail of big CTAs
         sorted_tiles_ = in.tiles;
         std::stable_sort(sorted_tiles_.begin(), sorted_tiles_.end(), [](const PrefillTile& a, const PrefillTile& b) { return a.pos0 + a.n_rows > b.pos0 + b.n_rows; });
         o_tiles = put(sorted_tiles_.data(), sorted_tiles_.size() * 4);
+        set_key_tiles(key_tiles, sorted_tiles_.data(), sorted_tiles_.size());
     }
     cuda_check(cudaMemcpyAsync(d_meta_, h_meta_, w * 4, cudaMemcpyHostToDevice, stream), "meta H2D");
     for (size_t u = 0; u < n_upd; ++u) {           // new automaton states: bitset rows of the device table (read by the LM-head epilogue below)
@@ -482,7 +484,7 @@ void DeviceModel::forward(const StepInput& in, float* logits_out) {
         if (!in.decode && !in.tiles.empty()) {     // mixed step: both kernels, disjoint rows of q_/attn_
             PrefillAttnParams a{}; a.q = q_; a.out = attn_; a.block_tables = d_bt; a.max_pages_per_seq = max_pages_per_seq;
             a.tiles = reinterpret_cast<const PrefillTile*>(d_meta_ + o_tiles); a.n_tiles = (int)in.tiles.size();
-            a.layer = l; a.n_heads = nh; a.n_kv = nkv; a.scale_log2e = scale_log2e;
+            a.layer = l; a.n_heads = nh; a.n_kv = nkv; a.scale_log2e = scale_log2e; a.key_tiles = key_tiles.key_tiles; a.max_key_tiles = key_tiles.max_key_tiles;
             static const bool legacy = [] { const char* e = std::getenv("OA_PREFILL_ATTN"); return e && std::string(e) == "legacy"; }();
             if (legacy) cuda_check(launch_prefill_attention(&tm_kv, kv, a, stream), "prefill attention (mma.sync)");
             else cuda_check(launch_prefill_attention_tc(&tm_q_, &tm_kv, kv, a, stream), "prefill attention (tcgen05)");

@@ -342,6 +342,45 @@ def test_paged_prefill_attention_two_heads_per_cta(L, nh, nkv, D):
     assert err < 2 * 5 * 2.0 ** -8, err
 
 
+# one head a CTA, two heads a CTA, two heads a CTA pair: a batch takes the kernel that the estimate of its time names, and a row's bits are the same in all.
+# Items of one, two, three and many key tiles (the pair's warpgroups take them in turn: odd and even ends, items shorter than what is on its way), a last tile
+# without its second page, more items than CTAs, references raised in later tiles
+@pytest.mark.parametrize("nh,nkv", [(8, 4), (16, 2)])
+@pytest.mark.parametrize("ctx,rows", [(2, 2), (64, 64), (128, 128), (129, 129), (256, 255), (384, 130), (449, 33), (1000, 130), (1280, 65)])
+def test_prefill_attention_kernels_agree(L, nh, nkv, ctx, rows):
+    D, pages = 128, (ctx + 63) // 64
+    kv = _mk_cache(pages, nkv, D, 5)
+    g = torch.Generator(device="cpu").manual_seed(ctx)
+    q1 = torch.randn(rows, nh, D, generator=g)
+    q1[::5] *= 9
+    q1 = q1.to(torch.bfloat16).to(dev())
+
+    def arrays(copies):
+        return np.full(copies, ctx, np.int32), np.full(copies, rows, np.int32), np.tile(np.arange(pages, dtype=np.int32)[::-1], (copies, 1)).copy()
+
+    def kernel(copies):
+        c, n, _ = arrays(copies)
+        return L.oa_host_prefill_attention_kernel(c.ctypes.data, n.ctypes.data, copies, nh, nkv, D)
+
+    first = {}
+    for copies in [1, 3, 5, 9, 17, 33, 50, 75, 101, 160, 300]:
+        first.setdefault(kernel(copies), copies)
+    assert 3 in first and len(first) >= 2
+    outs = []
+    for copies in first.values():
+        q = q1.repeat(copies, 1, 1).contiguous()
+        out = torch.full_like(q, float("nan"))
+        c, n, bt = arrays(copies)
+        assert L.oa_k_paged_attention(ptr(q), ptr(out), ptr(kv), pages, bt.ctypes.data, pages, c.ctypes.data, n.ctypes.data, copies, nh, nkv, D, 0, None) == 0, _lib.last_error()
+        assert torch.equal(out, out[:rows].repeat(copies, 1, 1))
+        outs.append(out[:rows])
+    for o in outs[1:]:
+        assert torch.equal(o, outs[0])
+    ref = _attn_ref(q1, kv[0], kv[1], torch.arange(pages - 1, -1, -1, device=dev())[None], [ctx], [rows], nh, nkv, D)
+    # probabilities and result are rounded to bf16 (2^-9 relative each); |values| stay below 5
+    assert (outs[0].float() - ref).abs().max().item() < 2 * 5 * 2.0 ** -8
+
+
 def _decode_route(L, ctx, nkv):
     """segments, CTAs and partial slots of the plan that a decoding batch runs on 148 SMs"""
     ctx = np.ascontiguousarray(ctx, np.int32); cap = int(((ctx + 63) // 64).sum()) * nkv + 512
