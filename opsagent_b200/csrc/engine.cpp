@@ -38,50 +38,6 @@ struct CallerDevice {
     ~CallerDevice() { if (prev >= 0) cudaSetDevice(prev); }
 };
 
-// Results that a caller reads on the host, through page-locked pieces: a copy straight to the caller's (pageable, often fresh) memory is staged by the driver
-// only once the step is over, and every page of it is faulted in between the pieces (8 rows of 128256 logits, 4.1 MB: 1380 us behind a step of 600).  Here the
-// first pieces are queued behind the step's kernels, the destination's pages are touched while those run, and what is left afterwards is a memcpy of pieces
-// that have landed, with the later ones on their way.
-class HostResult {
-public:
-    HostResult() {
-        if (cudaHostAlloc(&pin_, PIECES * PIECE_BYTES, cudaHostAllocDefault) != cudaSuccess) { pin_ = nullptr; cudaGetLastError(); }
-        for (auto& e : ev_) if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) { e = nullptr; cudaGetLastError(); }
-    }
-    HostResult(const HostResult&) = delete;
-    ~HostResult() {
-        if (pin_) cudaFreeHost(pin_);
-        for (auto& e : ev_) if (e) cudaEventDestroy(e);
-    }
-    // returns once `bytes` from src, as the stream's work so far leaves them, stand at dst
-    void copy(void* dst, const void* src, size_t bytes, cudaStream_t s) {
-        if (!pin_ || !ev_[PIECES - 1]) {
-            cuda_check(cudaStreamSynchronize(s), "stream sync");
-            cuda_check(cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost), "result D2H");
-            return;
-        }
-        char* out = reinterpret_cast<char*>(dst);
-        const size_t n = (bytes + PIECE_BYTES - 1) / PIECE_BYTES;
-        auto length = [&](size_t i) { return std::min(PIECE_BYTES, bytes - i * PIECE_BYTES); };
-        auto send = [&](size_t i) {
-            cuda_check(cudaMemcpyAsync(pin_ + i % PIECES * PIECE_BYTES, reinterpret_cast<const char*>(src) + i * PIECE_BYTES, length(i), cudaMemcpyDeviceToHost, s), "result D2H");
-            cuda_check(cudaEventRecord(ev_[i % PIECES], s), "result event");
-        };
-        for (size_t i = 0; i < std::min(n, PIECES); ++i) send(i);
-        for (size_t at = 0; at < bytes; at = (((size_t)out + at) / 4096 + 1) * 4096 - (size_t)out) __atomic_fetch_or(out + at, (char)0, __ATOMIC_RELAXED);      // one write fault a page, no value changed
-        for (size_t i = 0; i < n; ++i) {
-            cuda_check(cudaEventSynchronize(ev_[i % PIECES]), "result sync");
-            std::memcpy(out + i * PIECE_BYTES, pin_ + i % PIECES * PIECE_BYTES, length(i));
-            if (i + PIECES < n) send(i + PIECES);
-        }
-    }
-
-private:
-    static constexpr size_t PIECES = 4, PIECE_BYTES = 512 << 10;
-    char* pin_ = nullptr;
-    cudaEvent_t ev_[PIECES] = {};
-};
-
 enum class SeqState { WAITING, PREFILL, DECODE, DONE };
 
 struct Seq {
@@ -114,7 +70,6 @@ public:
         for (int p = model_.num_pages - 1; p >= 0; --p) free_pages_.push_back(p);
         page_ref_.assign(model_.num_pages, 0); page_hash_.assign(model_.num_pages, 0); page_parent_.assign(model_.num_pages, 0);
         page_tokens_.assign((size_t)model_.num_pages * 64, 0); lru_pos_.assign(model_.num_pages, lru_.end());
-        if (!is_follower()) { CallerDevice on_engine_device(opt_.device); host_result_.reset(new HostResult); }
         token_bytes_ = tok_.text_token_bytes();
         trie_.build(token_bytes_, model_.cfg.vocab);
         mask_key_of_.assign((size_t)model_.mask_slots, std::string()); mask_last_use_.assign((size_t)model_.mask_slots, 0);
@@ -128,7 +83,6 @@ public:
         if (model_.comm && opt_.tp_rank == 0) { std::lock_guard<std::mutex> step(step_mu_); CallerDevice on_engine_device(opt_.device); model_.sync(); model_.comm->shutdown(); }
         if (follower_.joinable()) follower_.join();
         CallerDevice on_engine_device(opt_.device);
-        host_result_.reset();
         if (trace_logits_) cudaFree(trace_logits_);
     }
     bool is_follower() const { return opt_.tp > 1 && opt_.tp_rank > 0; }
@@ -312,9 +266,8 @@ public:
                     cuda_check(cudaMalloc(&trace_logits_, n_rows * (size_t)V * 4), "cudaMalloc logits");
                     trace_logits_cap_ = n_rows * (size_t)V;
                 }
-                run_forward(in, n_rows ? trace_logits_ : nullptr);
-                if (n_rows) host_result_->copy(logits_out, trace_logits_, n_rows * (size_t)V * 4, model_.stream);
-                else model_.sync();
+                run_forward(in, n_rows ? trace_logits_ : nullptr); model_.sync();
+                if (n_rows) cuda_check(cudaMemcpy(logits_out, trace_logits_, n_rows * (size_t)V * 4, cudaMemcpyDeviceToHost), "logits D2H");
             }
             {
                 std::lock_guard<std::mutex> lk(mu_);
@@ -796,7 +749,6 @@ private:
 
     std::unique_ptr<ModelBase> model_p_; ModelBase& model_; Tokenizer tok_; EngineOptions opt_;
     float* trace_logits_ = nullptr; size_t trace_logits_cap_ = 0;
-    std::unique_ptr<HostResult> host_result_;      // used under step_mu_
     std::vector<int32_t> free_slots_;              // state slots of models with per-sequence recurrent state
     std::unordered_map<int64_t, std::shared_ptr<Seq>> traced_;      // sequences driven step by step through trace_step()
     std::mutex mu_, step_mu_;

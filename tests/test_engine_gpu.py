@@ -781,8 +781,8 @@ def test_trace_step_mixes_single_tokens_and_portions(preset):
             assert np.abs(g - ref[i]).max() < 2.5e-2          # two kernels' roundings, as between the engine and the oracle
 
 
-# the logits of a step come back through four page-locked pieces of 512 KB (32 rows here): fewer rows than a piece, whole pieces, more than there are pieces
-@pytest.mark.parametrize("rows", [1, 31, 32, 33, 128, 129, 290])
+# the places asked for, in their order, from tokens given as any whole numbers
+@pytest.mark.parametrize("rows", [1, 17, 290])
 def test_trace_step_brings_all_logits_back(rows):
     cfg = dict(model="custom", hidden=256, n_layers=1, n_heads=4, n_kv_heads=2, head_dim=64, ffn=512, vocab=4096, seed=5, num_pages=16, max_batch=8, max_seq_len=512,
                max_step_tokens=512, prefix_cache=0)
@@ -790,6 +790,6 @@ def test_trace_step_brings_all_logits_back(rows):
     with Engine(cfg) as eng:
         ref = eng.debug_prefill_logits(toks)
         places = sorted(np.random.default_rng(1).permutation(300)[:rows].tolist())
-        for step in range(2):                              # the second step finds the pieces used
-            out = eng.trace_step([(step, np.array(toks, np.int64), places)], [step])
+        for step, given in enumerate([toks, np.array(toks, np.int64), np.array(toks, np.float64)]):      # numbers that are not whole are cut
+            out = eng.trace_step([(step, given, places)], [step])
             assert np.array_equal(out, ref[places])
