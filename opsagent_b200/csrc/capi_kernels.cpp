@@ -92,11 +92,13 @@ int rc_of(cudaError_t e) { return e == cudaSuccess ? OA_OK : OA_ERR_INTERNAL; }
 // materialise the deterministic fixed-order sum of stream-K partials as fp32 [M,N]: 8 columns of a row per thread, every partial's loads in
 // flight together (a row per CTA with one column and one load at a time was latency-bound: 23 us for 32 x 6144, more than the product itself)
 __global__ void sk_reduce_f32_kernel(const StreamK sk, float* __restrict__ out, int N, int aligned) {
-    griddep_launch(); griddep_wait();
+    griddep_launch();
     const int row = blockIdx.y, col = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
+    const SkCols at = sk_locate(sk, row, col < N ? col : 0);
+    griddep_wait();
     if (col >= N) return;
     float acc[8];
-    sk_sum8(sk, row, col, acc);
+    sk_sum8(sk, at, acc);
     float* o = out + (size_t)row * N + col;
     if (aligned) {
         reinterpret_cast<float4*>(o)[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);

@@ -146,12 +146,12 @@ cudaError_t launch_rope_kv_write(const void* qkv, const int32_t* positions, cons
 
 
 // =============================================================================================
-// stream-K consumers (stand-alone kernels; the bodies live in sk_consumers.cuh)
+// stream-K consumers (stand-alone kernels; the bodies live in sk_consumers.cuh, the wait for the product too: what it does not write is read ahead of it)
 // =============================================================================================
 template <int VPT>
 __global__ void __launch_bounds__(SK_RESID_THREADS) sk_resid_rmsnorm_kernel(const StreamK sk, uint4* __restrict__ x, const uint4* __restrict__ g,
                                                                             uint4* __restrict__ y, int H8, float inv_h, float eps) {
-    griddep_launch(); griddep_wait();
+    griddep_launch();
     __shared__ float red[SK_RESID_THREADS / 32];
     sk_resid_rmsnorm_row<VPT>(sk, blockIdx.x, threadIdx.x, red, 0, x, g, y, H8, inv_h, eps);
 }
@@ -166,7 +166,7 @@ cudaError_t launch_sk_resid_rmsnorm(const StreamK& sk, void* x, const void* gain
 
 template <int VPT>
 __global__ void __launch_bounds__(SK_RESID_THREADS) rmsnorm_wide_kernel(uint4* __restrict__ x, const uint4* __restrict__ g, uint4* __restrict__ y, int H8, float inv_h, float eps) {
-    griddep_launch(); griddep_wait();
+    griddep_launch();
     __shared__ float red[SK_RESID_THREADS / 32];
     sk_resid_rmsnorm_row<VPT, false>(StreamK{}, blockIdx.x, threadIdx.x, red, 0, x, g, y, H8, inv_h, eps);
 }
@@ -191,9 +191,9 @@ cudaError_t launch_sk_swiglu(const StreamK& sk, void* act, int T, int F, cudaStr
 }
 
 __global__ void sk_rope_kv_write_kernel(const StreamK sk, const SkRopeArgs a) {
-    griddep_launch(); griddep_wait();
-    const int t = blockIdx.y, items = sk_rope_items_per_row(a);
-    for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < items; w += gridDim.x * blockDim.x) sk_rope_item(sk, a, t, w);
+    griddep_launch();
+    const int w = blockIdx.x * blockDim.x + threadIdx.x;      // the grid has a thread for every item
+    sk_rope_item(sk, a, blockIdx.y, w, w < sk_rope_items_per_row(a));
 }
 SkRopeArgs make_sk_rope_args(const void* bias, const int32_t* positions, const int32_t* slots, const float* rope_cos, const float* rope_sin,
                              void* q_out, const KvLayout& kv, int layer, int nh) {
