@@ -401,9 +401,12 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? 2 : 1) hy_block_memo
 // ---- token form ----
 struct FewArgs {
     BlockArgs p;
-    const bf* in; const float* conv_w; int taps, C; const bf* tails;      // delta rule: the short convolution's input rows [T, ld_in] of C channels, taps [C, taps], carried tails
+    const bf* in; const float* conv_w; int taps, C; bf* tails;            // delta rule: the short convolution's input rows [T, ld_in] of C channels, taps [C, taps], carried tails
+    bool keep;                                                            // taps of FEW_TAPS, in aligned groups
+    int tail_group;                                                       // > 0: this kernel leaves the new tails, the heads that share a query head being a cluster of so many CTAs
 };
 constexpr int FEW_RPT = 16;      // state rows per thread: dim <= 8 * 16
+constexpr int FEW_TAPS = 4;      // taps of which a thread keeps its channels' carried inputs and weights
 template <bool DELTA>
 __global__ void __launch_bounds__(256) hy_few_memory_kernel(FewArgs f, HyRows r) {
     // The state was written in an earlier step and the rows' metadata copied in ahead of this one: both are read before the wait, under the projection that
@@ -423,14 +426,54 @@ __global__ void __launch_bounds__(256) hy_few_memory_kernel(FewArgs f, HyRows r)
         const int d = warp + 8 * i;
         S[i] = (pos0 > 0 && ok && d < D) ? *reinterpret_cast<const float4*>(st + (long long)d * VD + c4) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    griddep_wait();
     const int n = 2 * D + VD;
-    for (int i = tid; i < len * n; i += 256) {
+    // channel of the convolution: [q heads | k heads | v heads]
+    auto channel = [&](int c) { return c < D ? qh * D + c : c < 2 * D ? p.QH * D + qh * D + (c - D) : 2 * p.QH * D + h * VD + (c - 2 * D); };
+    bf* tail = DELTA ? f.tails + (long long)slot * (f.taps - 1) * f.C : nullptr;
+    // Delta rule: what the earlier steps carried and the weights of this thread's channels (its items of the first token: at most two), the norm's weights and
+    // the decay's, all ahead of the wait
+    const bool keep = DELTA && f.keep;
+    bf old[2][FEW_TAPS - 1]; float cw[2][FEW_TAPS], A_log = 0.f, dt_bias = 0.f;
+    float4 nw = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (DELTA) {
+        if (keep)
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const int c = tid + k * 256;
+                if (c >= n) continue;
+                const int ch = channel(c);
+#pragma unroll
+                for (int j = 0; j < FEW_TAPS - 1; ++j) old[k][j] = pos0 > 0 ? tail[(long long)j * f.C + ch] : __float2bfloat16_rn(0.f);
+                const float4 w = *reinterpret_cast<const float4*>(f.conv_w + ch * FEW_TAPS);
+                cw[k][0] = w.x; cw[k][1] = w.y; cw[k][2] = w.z; cw[k][3] = w.w;
+            }
+        if (ok) nw = *reinterpret_cast<const float4*>(p.norm_w + c4);
+        if (tid < len) { A_log = p.A_log[h]; dt_bias = p.dt_bias[h]; }
+    }
+    griddep_wait();
+    bf fresh[2][FEW_TAPS - 1];                           // the carried inputs that this step leaves, of this thread's channels
+    for (int i = tid, k = 0; i < len * n; i += 256, ++k) {
         const int t = i / n, c = i - t * n;
         float* dst = c < D ? &qs[t][c] : c < 2 * D ? &ks[t][c - D] : &vs[t][c - 2 * D];
-        if (DELTA) {                                     // channel of the convolution: [q heads | k heads | v heads]
-            const int ch = c < D ? qh * D + c : c < 2 * D ? p.QH * D + qh * D + (c - D) : 2 * p.QH * D + h * VD + (c - 2 * D);
-            const bf* tail = f.tails + (long long)slot * (f.taps - 1) * f.C;
+        if (DELTA && keep && t == 0) {
+            const int ch = channel(c), kk = k & 1;       // n <= 384: the first token's items are the first two rounds
+            float acc = 0.f;
+#pragma unroll
+            for (int j = 0; j < FEW_TAPS - 1; ++j) acc = fmaf(kk ? cw[1][j] : cw[0][j], __bfloat162float(kk ? old[1][j] : old[0][j]), acc);
+            const bf now = f.in[row0 * p.ld_in + ch];
+            acc = fmaf(kk ? cw[1][FEW_TAPS - 1] : cw[0][FEW_TAPS - 1], __bfloat162float(now), acc);
+            *dst = __bfloat162float(__float2bfloat16_rn(silu_fast_f32(acc)));
+            if (f.tail_group > 0)
+#pragma unroll
+                for (int j = 0; j < FEW_TAPS - 1; ++j) {
+                    const int src = len - (FEW_TAPS - 1) + j;      // of this step's rows, or (negative) of what was carried
+                    bf v = src == 0 ? now : src > 0 ? f.in[(row0 + src) * p.ld_in + ch] : now;
+#pragma unroll
+                    for (int o = 0; o < FEW_TAPS - 1; ++o) if (src == o - (FEW_TAPS - 1)) v = kk ? old[1][o] : old[0][o];
+                    if (kk) fresh[1][j] = v; else fresh[0][j] = v;
+                }
+        } else if (DELTA) {
+            const int ch = channel(c);
             float acc = 0.f;
             for (int j = 0; j < f.taps; ++j) {
                 const int src = t - (f.taps - 1) + j;
@@ -443,7 +486,7 @@ __global__ void __launch_bounds__(256) hy_few_memory_kernel(FewArgs f, HyRows r)
     if (tid < len) {
         if (DELTA) {
             const long long at = (row0 + tid) * p.ld_in + h;
-            gb[tid][0] = expf(log_decay(p.A_log[h], ldf(p.a + at) + p.dt_bias[h])); gb[tid][1] = sigmoidf_(ldf(p.b + at));
+            gb[tid][0] = expf(log_decay(A_log, ldf(p.a + at) + dt_bias)); gb[tid][1] = sigmoidf_(ldf(p.b + at));
         } else gb[tid][0] = p.decay[h];
     }
     __syncthreads();
@@ -457,8 +500,25 @@ __global__ void __launch_bounds__(256) hy_few_memory_kernel(FewArgs f, HyRows r)
         }
         __syncthreads();
     }
+    // New tails: every CTA that reads a channel has read it (a cluster shares its query and key channels, values are a CTA's own); the cluster's first head leaves
+    // the shared ones.  (A kernel of their own behind this one took 4 us a layer.)
+    if (DELTA && f.tail_group > 0) {
+        if (f.tail_group > 1) {
+            asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        } else __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int c = tid + k * 256;
+            if (c < n && (c >= 2 * D || h % f.tail_group == 0))
+#pragma unroll
+                for (int j = 0; j < FEW_TAPS - 1; ++j) tail[(long long)j * f.C + channel(c)] = fresh[k][j];
+        }
+    }
     for (int t = 0; t < len; ++t) {
         const float g = gb[t][0];
+        uint2 gr = make_uint2(0, 0);
+        if (DELTA && ok && warp == (t & 7)) gr = *reinterpret_cast<const uint2*>(p.gate + (row0 + t) * p.ld_in + (long long)h * VD + c4);      // of the warp that joins this token's read-out
         float4 u = ok ? *reinterpret_cast<const float4*>(&vs[t][c4]) : make_float4(0.f, 0.f, 0.f, 0.f), o = make_float4(0.f, 0.f, 0.f, 0.f);
         if (DELTA) {
             float4 dot = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -498,7 +558,7 @@ __global__ void __launch_bounds__(256) hy_few_memory_kernel(FewArgs f, HyRows r)
             if (DELTA) {
                 const float ss = warp_sum(ok ? (o.x * o.x + o.y * o.y) + (o.z * o.z + o.w * o.w) : 0.f), rr = 1.0f / sqrtf(ss / (float)VD + p.eps);
                 if (ok) {
-                    const uint2 gr = *reinterpret_cast<const uint2*>(p.gate + (row0 + t) * p.ld_in + (long long)h * VD + c4); const float4 w = *reinterpret_cast<const float4*>(p.norm_w + c4);
+                    const float4 w = nw;
                     *reinterpret_cast<uint2*>(reinterpret_cast<bf*>(p.out) + (row0 + t) * p.ldo + (long long)h * VD + c4) =
                         make_uint2(pack_bf16x2(o.x * rr * w.x * siluf_(bf16lo(gr.x)), o.y * rr * w.y * siluf_(bf16hi(gr.x))), pack_bf16x2(o.z * rr * w.z * siluf_(bf16lo(gr.y)), o.w * rr * w.w * siluf_(bf16hi(gr.y))));
                 }
@@ -539,6 +599,11 @@ cudaError_t hy_lightning_mix(const HyBlockHead& m, const void* q, const void* k,
     return many ? block_launch<false>(p, r, s) : cudaSuccess;
 }
 
+// four taps, at most eight heads a query head (a portable cluster), heads whose operands are two items a thread
+bool hy_delta_leaves_tails(const HyBlockHead& m, const HyDeltaMix& d) {
+    return d.taps == FEW_TAPS && al16(d.conv_w) && m.qk_heads > 0 && m.heads % m.qk_heads == 0 && m.heads / m.qk_heads <= 8;
+}
+
 cudaError_t hy_delta_mix(const HyBlockHead& m, const HyDeltaMix& d, float* state, void* out, int ldo, bool few, bool many, const HyRows& r, cudaStream_t s) {
     if (r.T <= 0) return cudaSuccess;
     if (!hy_block_memory_supported(m.dim, m.vdim) || m.qk_heads <= 0 || m.heads % m.qk_heads || d.ld_conv % 8 || d.ld_in % 8 || ldo % 8 || !al16(d.conv) || !al16(d.in) || !al16(d.gate) ||
@@ -547,8 +612,17 @@ cudaError_t hy_delta_mix(const HyBlockHead& m, const HyDeltaMix& d, float* state
     p.q = (const bf*)d.conv; p.k = p.q + qk; p.v = p.k + qk; p.ld = d.ld_conv; p.gate = (const bf*)d.gate; p.a = (const bf*)d.a; p.b = (const bf*)d.b; p.ld_in = d.ld_in;
     p.A_log = d.A_log; p.dt_bias = d.dt_bias; p.norm_w = d.norm_w; p.eps = d.eps; p.state = state; p.out = out; p.ldo = ldo; p.H = m.heads; p.QH = m.qk_heads; p.D = m.dim; p.VD = m.vdim;
     if (few) {
-        FewArgs f{}; f.p = p; f.in = (const bf*)d.in; f.conv_w = d.conv_w; f.taps = d.taps; f.C = 2 * qk + m.heads * m.vdim; f.tails = (const bf*)d.tails;
-        if (cudaError_t e = launch_plain(hy_few_memory_kernel<true>, dim3(r.S, m.heads), dim3(256), 0, s, f, r); e != cudaSuccess) return e;
+        FewArgs f{}; f.p = p; f.in = (const bf*)d.in; f.conv_w = d.conv_w; f.taps = d.taps; f.C = 2 * qk + m.heads * m.vdim; f.tails = (bf*)d.tails;
+        f.keep = d.taps == FEW_TAPS && al16(d.conv_w);
+        f.tail_group = hy_delta_leaves_tails(m, d) ? m.heads / m.qk_heads : 0;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(r.S, m.heads); cfg.blockDim = dim3(256); cfg.stream = s;
+        cudaLaunchAttribute attr[2]; int n_attr = 0;
+        if (f.tail_group > 1) { attr[n_attr].id = cudaLaunchAttributeClusterDimension; attr[n_attr].val.clusterDim.x = 1; attr[n_attr].val.clusterDim.y = f.tail_group; attr[n_attr++].val.clusterDim.z = 1; }
+        if (pdl_enabled()) { attr[n_attr].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[n_attr++].val.programmaticStreamSerializationAllowed = 1; }
+        cfg.attrs = attr; cfg.numAttrs = n_attr;
+        count_launch();
+        if (cudaError_t e = cudaLaunchKernelEx(&cfg, hy_few_memory_kernel<true>, f, r); e != cudaSuccess) return e;
     }
     return many ? block_launch<true>(p, r, s) : cudaSuccess;
 }

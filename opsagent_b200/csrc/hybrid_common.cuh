@@ -33,6 +33,17 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
     return t;
 }
 
+// two sums at once, each as block_sum adds it
+__device__ __forceinline__ void block_sum2(float& u, float& v, float* red_u, float* red_v) {
+    u = warp_sum(u); v = warp_sum(v);
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
+    __syncthreads();
+    if (l == 0) { red_u[w] = u; red_v[w] = v; }
+    __syncthreads();
+    u = v = 0.f;
+    for (int i = 0; i < nw; ++i) { u += red_u[i]; v += red_v[i]; }
+}
+
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem)), "l"(gmem) : "memory");
 }

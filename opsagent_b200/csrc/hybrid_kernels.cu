@@ -79,21 +79,27 @@ __global__ void __launch_bounds__(256) hy_gemm_kernel(const TA* __restrict__ A, 
 // us, 16 heads at 16 rows: 512 x 128 with fp32 results 4.5, 128 x 512 5.1 (a warp per column that walks the rows: 27).  mma.sync takes 2.6 and 2.9, but
 // its sums are 1.2e-7 off the 64-bit result where these are 4.8e-8, and hy_tensor_core = 0 promises plain FMA.
 template <int MODE, int G>
-__global__ void __launch_bounds__(128) hy_gemm_fewrows_kernel(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bfloat16* __restrict__ B, int ldb, void* Cv, int ldc, int M, int N,
-                                                              int K, const float* __restrict__ bias, float alpha, long long sA, long long sB, long long sC, HyGemmAct act) {
-    HY_PDL();
+__device__ __forceinline__ void few_rows_body(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bfloat16* __restrict__ B, int ldb, void* Cv, int ldc, int M, int N,
+                                              int K, const float* __restrict__ bias, float alpha, long long sA, long long sB, long long sC, HyGemmAct act, int bx, int by, int bz, bool b_early) {
     constexpr int ROWS = 8, COLS = 2;
-    const int l = threadIdx.x & (G - 1), n0 = (blockIdx.x * (128 / G) + threadIdx.x / G) * COLS, m0 = blockIdx.z * ROWS;
-    A += (long long)blockIdx.y * sA + (long long)m0 * lda; B += (long long)blockIdx.y * sB;
+    const int l = threadIdx.x & (G - 1), n0 = (bx * (128 / G) + threadIdx.x / G) * COLS, m0 = bz * ROWS;
+    A += (long long)by * sA + (long long)m0 * lda; B += (long long)by * sB;
+    if (!b_early) griddep_wait();                            // else B is weights that no kernel of the step writes: the first of them are read ahead of the wait
+    uint4 b[COLS];
+    auto load_b = [&](int k) {
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) b[c] = n0 + c < N && k < K ? *reinterpret_cast<const uint4*>(B + (long long)(n0 + c) * ldb + k) : make_uint4(0, 0, 0, 0);
+    };
+    load_b(l * 8);
+    if (b_early) griddep_wait();
     float acc[COLS][ROWS];
 #pragma unroll
     for (int c = 0; c < COLS; ++c)
 #pragma unroll
         for (int r = 0; r < ROWS; ++r) acc[c][r] = 0.f;
     for (int k = l * 8; k < K; k += G * 8) {
-        uint4 a[ROWS], b[COLS];
-#pragma unroll
-        for (int c = 0; c < COLS; ++c) b[c] = n0 + c < N ? *reinterpret_cast<const uint4*>(B + (long long)(n0 + c) * ldb + k) : make_uint4(0, 0, 0, 0);
+        uint4 a[ROWS];
+        if (k > l * 8) load_b(k);
 #pragma unroll
         for (int r = 0; r < ROWS; ++r) a[r] = m0 + r < M ? *reinterpret_cast<const uint4*>(A + (long long)r * lda + k) : make_uint4(0, 0, 0, 0);
         float bf[COLS][8];
@@ -142,11 +148,18 @@ __global__ void __launch_bounds__(128) hy_gemm_fewrows_kernel(const __nv_bfloat1
         if (rest != c || m >= M || n >= N) continue;
         float v = acc[c][0] * alpha + (bias ? bias[n] : 0.f);
         v = gemm_act(act, v, n);
-        const long long at = (long long)blockIdx.y * sC + (long long)m * ldc + n;
+        const long long at = (long long)by * sC + (long long)m * ldc + n;
         if (MODE == HY_STORE) reinterpret_cast<__nv_bfloat16*>(Cv)[at] = __float2bfloat16_rn(v);
         else if (MODE == HY_STORE_F32) reinterpret_cast<float*>(Cv)[at] = v;
         else reinterpret_cast<float*>(Cv)[at] += v;
     }
+}
+
+template <int MODE, int G>
+__global__ void __launch_bounds__(128) hy_gemm_fewrows_kernel(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bfloat16* __restrict__ B, int ldb, void* Cv, int ldc, int M, int N,
+                                                              int K, const float* __restrict__ bias, float alpha, long long sA, long long sB, long long sC, HyGemmAct act, bool b_early) {
+    griddep_launch();
+    few_rows_body<MODE, G>(A, lda, B, ldb, Cv, ldc, M, N, K, bias, alpha, sA, sB, sC, act, blockIdx.x, blockIdx.y, blockIdx.z, b_early);
 }
 
 template <typename TA>
@@ -206,40 +219,70 @@ __global__ void __launch_bounds__(256) hy_layernorm_kernel(const float* x, const
 // ---------------------------------------------------------------------------------------------------------------------------------
 // latent attention
 // ---------------------------------------------------------------------------------------------------------------------------------
+// One row: the latent's norm and the shared rotated key go to the cache, the rotated query parts behind the heads' absorbed ones.  A decoding step waits for every
+// load here one after the other, so slot, position, the rotation's factors and the norm's weights (host data and weights) are read ahead of the wait, the
+// latent once, and the queries turn ahead of the sum that the norm waits for.
+template <typename TA>
+__device__ __forceinline__ void mla_prep_row(const HyLatentAttn& a, const TA* __restrict__ q, int ldq, const TA* __restrict__ ckv, int ldc, const float* __restrict__ norm_w, float eps,
+                                             const float* __restrict__ rope_cos, const float* __restrict__ rope_sin, TA* __restrict__ cache, float* __restrict__ q_abs, const HyRows& r, int t, float* red) {
+    constexpr int KEEP = 4;                                       // channels a thread keeps: kv_rank up to 512 is read once
+    const int R = a.kv_rank, rot = a.rot_dim, half = a.rot_dims / 2, E = R + rot;
+    const TA* c = ckv + (long long)t * ldc;
+    TA* dst = cache + (long long)r.slots[t] * E;
+    const int pos = r.positions[t];
+    const float* cs = rope_cos + (long long)pos * half; const float* sn = rope_sin + (long long)pos * half;
+    // channel d of a rotated part turns with pair p_of(d); a thread's queries all have its own d where 128 is a multiple of rot, and so one pair
+    auto second_of = [&](int d) { return a.rot_layout ? d >= half : (d & 1) != 0; };
+    auto pair_of = [&](int d) { return a.rot_layout ? (d >= half ? d - half : d) : d >> 1; };
+    const bool one_pair = rot > 0 && 128 % rot == 0;
+    const int d0 = rot > 0 ? threadIdx.x % rot : 0;
+    float co = 1.f, si = 0.f, w[KEEP], v[KEEP];
+    if (one_pair && d0 < 2 * half) { co = cs[pair_of(d0)]; si = sn[pair_of(d0)]; }
+#pragma unroll
+    for (int k = 0; k < KEEP; ++k) { const int i = threadIdx.x + k * 128; w[k] = i < R ? norm_w[i] : 0.f; }
+    griddep_wait();
+#pragma unroll
+    for (int k = 0; k < KEEP; ++k) { const int i = threadIdx.x + k * 128; v[k] = i < R ? ldf(c + i) : 0.f; }
+    auto turn = [&](const TA* x, int d) {
+        if (d >= 2 * half) return ldf(x + d);
+        const int p = pair_of(d);
+        const float u0 = ldf(x + (a.rot_layout ? p : 2 * p)), u1 = ldf(x + (a.rot_layout ? p + half : 2 * p + 1)), f = one_pair ? co : cs[p], g = one_pair ? si : sn[p];
+        return second_of(d) ? (u1 * f + u0 * g) : (u0 * f - u1 * g);
+    };
+#pragma unroll 8
+    for (int i = threadIdx.x; i < a.heads * rot; i += 128) {      // rotated query parts (no array here overlaps another: several of these in flight)
+        const int h = i / rot, d = i - h * rot;
+        q_abs[((long long)t * a.heads + h) * E + R + d] = turn(q + (long long)t * ldq + (long long)h * (a.dim + rot) + a.dim, d);
+    }
+    for (int i = threadIdx.x; i < rot; i += 128) stf(dst + R + i, turn(c + R, i));         // shared rotated key
+    float ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < KEEP; ++k) if (threadIdx.x + k * 128 < R) ss += v[k] * v[k];
+    for (int i = threadIdx.x + KEEP * 128; i < R; i += 128) { const float u = ldf(c + i); ss += u * u; }
+    const float rr = 1.0f / sqrtf(block_sum(ss, red) / (float)R + eps);
+#pragma unroll
+    for (int k = 0; k < KEEP; ++k) { const int i = threadIdx.x + k * 128; if (i < R) stf(dst + i, v[k] * rr * w[k]); }
+    for (int i = threadIdx.x + KEEP * 128; i < R; i += 128) stf(dst + i, ldf(c + i) * rr * norm_w[i]);
+}
 template <typename TA>
 __global__ void __launch_bounds__(128) hy_mla_prep_kernel(HyLatentAttn a, const TA* __restrict__ q, int ldq, const TA* __restrict__ ckv, int ldc, const float* __restrict__ norm_w, float eps,
                                                            const float* __restrict__ rope_cos, const float* __restrict__ rope_sin, TA* __restrict__ cache, float* __restrict__ q_abs, HyRows r) {
-    HY_PDL();
+    griddep_launch();
     __shared__ float red[32];
-    const int t = blockIdx.x, R = a.kv_rank, rot = a.rot_dim, half = a.rot_dims / 2, E = R + rot;
-    const TA* c = ckv + (long long)t * ldc;
-    float ss = 0.f;
-    for (int i = threadIdx.x; i < R; i += blockDim.x) { const float v = ldf(c + i); ss += v * v; }
-    const float rr = 1.0f / sqrtf(block_sum(ss, red) / (float)R + eps);
-    TA* dst = cache + (long long)r.slots[t] * E;
-    for (int i = threadIdx.x; i < R; i += blockDim.x) stf(dst + i, ldf(c + i) * rr * norm_w[i]);
-    const int pos = r.positions[t];
-    const float* cs = rope_cos + (long long)pos * half; const float* sn = rope_sin + (long long)pos * half;
-    for (int i = threadIdx.x; i < rot; i += blockDim.x) {          // shared rotated key
-        float v;
-        if (i < 2 * half) {
-            const bool second = a.rot_layout ? i >= half : (i & 1); const int p = a.rot_layout ? (second ? i - half : i) : i >> 1;
-            const float u0 = ldf(c + R + (a.rot_layout ? p : 2 * p)), u1 = ldf(c + R + (a.rot_layout ? p + half : 2 * p + 1));
-            v = second ? (u1 * cs[p] + u0 * sn[p]) : (u0 * cs[p] - u1 * sn[p]);
-        } else v = ldf(c + R + i);
-        stf(dst + R + i, v);
-    }
-#pragma unroll 4
-    for (int i = threadIdx.x; i < a.heads * rot; i += blockDim.x) {   // rotated query parts (no array here overlaps another: several of these in flight)
-        const int h = i / rot, d = i - h * rot; const TA* qh = q + (long long)t * ldq + (long long)h * (a.dim + rot) + a.dim;
-        float v;
-        if (d < 2 * half) {
-            const bool second = a.rot_layout ? d >= half : (d & 1); const int p = a.rot_layout ? (second ? d - half : d) : d >> 1;
-            const float u0 = ldf(qh + (a.rot_layout ? p : 2 * p)), u1 = ldf(qh + (a.rot_layout ? p + half : 2 * p + 1));
-            v = second ? (u1 * cs[p] + u0 * sn[p]) : (u0 * cs[p] - u1 * sn[p]);
-        } else v = ldf(qh + d);
-        q_abs[((long long)t * a.heads + h) * E + R + d] = v;
-    }
+    mla_prep_row(a, q, ldq, ckv, ldc, norm_w, eps, rope_cos, rope_sin, cache, q_abs, r, blockIdx.x, red);
+}
+// The rows' preparation and the absorbed products of a few rows (q_abs[t, h, :rank] = W_uk[h]^T q_unrotated[t, h], hy_gemm_fewrows_kernel's) in one launch:
+// neither reads what the other writes, and one behind the other they took 8.1 and 5.2 us of a step of 16 rows.
+template <int G>
+__global__ void __launch_bounds__(128) hy_mla_prep_absorb_kernel(HyLatentAttn a, const __nv_bfloat16* __restrict__ q, int ldq, const __nv_bfloat16* __restrict__ ckv, int ldc,
+                                                                 const float* __restrict__ norm_w, float eps, const float* __restrict__ rope_cos, const float* __restrict__ rope_sin,
+                                                                 __nv_bfloat16* __restrict__ cache, float* __restrict__ q_abs, HyRows r, const __nv_bfloat16* __restrict__ uk_t, int nx) {
+    griddep_launch();
+    __shared__ float red[32];
+    const int E = a.kv_rank + a.rot_dim, b = (int)blockIdx.x - r.T;
+    if (b < 0) mla_prep_row(a, q, ldq, ckv, ldc, norm_w, eps, rope_cos, rope_sin, cache, q_abs, r, blockIdx.x, red);
+    else few_rows_body<HY_STORE_F32, G>(q, ldq, uk_t, a.dim, q_abs, a.heads * E, r.T, a.kv_rank, a.dim, nullptr, 1.f, a.dim + a.rot_dim, (long long)a.kv_rank * a.dim, E, HyGemmAct{},
+                                        b % nx, b / nx % a.heads, b / nx / a.heads, true);
 }
 
 constexpr int MLA_ACC = 32;     // latent channels per lane: kv_rank <= 32 * MLA_ACC
@@ -490,7 +533,7 @@ __global__ void __launch_bounds__(128) hy_mla_decode_mma_kernel(HyLatentAttn a, 
     for (int s = 0; s < STAGES; ++s) if (g_begin + 4 * s < g_end && !older(g_begin + 4 * s)) issue(g_begin + 4 * s, s);
     const float qscale = a.scale * 1.4426950408889634f;
     const int e4 = E / 4;
-#pragma unroll 6
+#pragma unroll 9
     for (int idx = tid; idx < MLA_DQ * e4; idx += 128) {
         const int qi = idx / e4, e = (idx - qi * e4) * 4;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -604,21 +647,33 @@ __global__ void __launch_bounds__(128) hy_mla_decode_mma_kernel(HyLatentAttn a, 
 }
 
 // joins the parts of a decoding row: out = sum_p 2^(m_p - M) O_p / sum_p 2^(m_p - M) l_p, parts in order
-__global__ void __launch_bounds__(128) hy_mla_merge_kernel(const int32_t* item_row, const int32_t* item_slot0, const int32_t* item_parts, const float* ws_o,
-                                                           const float* ws_ml, __nv_bfloat16* lat_out, int H, int R, const float* sink,
-                                                           const __nv_bfloat16* head_gate, int ldg) {
-    HY_PDL();
+// Four channels a thread, all parts' loads in flight: a row's items come from the host and are read ahead of the wait.  (A channel a thread and its parts one
+// behind the other: 4.6 us for 16 rows of two parts, 16 heads of 512 channels, against 3.4.)
+__global__ void __launch_bounds__(128) hy_mla_merge_kernel(const int32_t* __restrict__ item_row, const int32_t* __restrict__ item_slot0, const int32_t* __restrict__ item_parts,
+                                                           const float* __restrict__ ws_o, const float* __restrict__ ws_ml, __nv_bfloat16* __restrict__ lat_out, int H, int R,
+                                                           const float* __restrict__ sink, const __nv_bfloat16* __restrict__ head_gate, int ldg) {
+    griddep_launch();
     const int row = item_row[blockIdx.x], slot0 = item_slot0[blockIdx.x], P = item_parts[blockIdx.x], h = blockIdx.y;
     const float s2 = sink ? sink[h] * 1.4426950408889634f : -INFINITY;       // the sink, in the partials' base-2 units
+    griddep_wait();
+    const float2* ml = reinterpret_cast<const float2*>(ws_ml) + (long long)slot0 * H + h;
+    const float* po = ws_o + ((long long)slot0 * H + h) * R;
     float M = s2;
-    for (int p = 0; p < P; ++p) M = fmaxf(M, ws_ml[((long long)(slot0 + p) * H + h) * 2]);
+#pragma unroll 8
+    for (int p = 0; p < P; ++p) M = fmaxf(M, ml[(long long)p * H].x);
     float L = sink ? exp2f(s2 - M) : 0.f;
-    for (int p = 0; p < P; ++p) { const float* ml = ws_ml + ((long long)(slot0 + p) * H + h) * 2; L += exp2f(ml[0] - M) * ml[1]; }
+#pragma unroll 8
+    for (int p = 0; p < P; ++p) { const float2 v = ml[(long long)p * H]; L += exp2f(v.x - M) * v.y; }
     const float inv = (head_gate ? sigmoidf_(ldf(head_gate + (long long)row * ldg + h)) : 1.0f) / L;
-    for (int c = threadIdx.x; c < R; c += blockDim.x) {
-        float acc = 0.f;
-        for (int p = 0; p < P; ++p) acc += exp2f(ws_ml[((long long)(slot0 + p) * H + h) * 2] - M) * ws_o[((long long)(slot0 + p) * H + h) * R + c];
-        lat_out[((long long)row * H + h) * R + c] = __float2bfloat16_rn(acc * inv);
+    for (int c = threadIdx.x * 4; c < R; c += 128 * 4) {                      // the latent's channels come in groups of 64
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+        for (int p = 0; p < P; ++p) {
+            const float f = exp2f(ml[(long long)p * H].x - M);
+            const float4 u = *reinterpret_cast<const float4*>(po + (long long)p * H * R + c);
+            acc.x += f * u.x; acc.y += f * u.y; acc.z += f * u.z; acc.w += f * u.w;
+        }
+        *reinterpret_cast<uint2*>(lat_out + ((long long)row * H + h) * R + c) = make_uint2(pack_bf16x2(acc.x * inv, acc.y * inv), pack_bf16x2(acc.z * inv, acc.w * inv));
     }
 }
 
@@ -793,6 +848,28 @@ __device__ __forceinline__ void st4(__nv_bfloat16* p, const float* f) {
     const __nv_bfloat162 a = __floats2bfloat162_rn(f[0], f[1]), b = __floats2bfloat162_rn(f[2], f[3]);
     *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
 }
+// hy_embed_kernel in groups of eight channels.  A thread of that one loads a channel, stores it and only then loads the next (they may overlap, for all the
+// compiler knows): 16 trips to HBM one behind the other for a row of 2048, 10 us of every step.  Here a row is one load a thread.  (A step's first kernel
+// of 16 rows 10 -> 3 us, of 2640 rows 17 -> 9.)
+template <typename TA>
+__global__ void __launch_bounds__(256) hy_embed_vec8_kernel(const int32_t* __restrict__ ids, const TA* __restrict__ table, float* __restrict__ x, float* __restrict__ x0, int W, int vocab,
+                                                            float scale, TA* __restrict__ h, int ldh) {
+    HY_PDL();
+    const long long t = blockIdx.x; int id = ids[t]; id = id < 0 ? 0 : (id >= vocab ? vocab - 1 : id);
+    for (int c = threadIdx.x * 8; c < W; c += 256 * 8) {
+        float v[8];
+        ld4(table + (long long)id * W + c, v); ld4(table + (long long)id * W + c + 4, v + 4);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] *= scale;
+#pragma unroll
+        for (int e = 0; e < 8; e += 4) {
+            const float4 u = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+            *reinterpret_cast<float4*>(x + t * W + c + e) = u;
+            if (x0) *reinterpret_cast<float4*>(x0 + t * W + c + e) = u;
+            if (h) st4(h + t * ldh + c + e, v + e);
+        }
+    }
+}
 // SiLU / sigmoid of a value that is stored as the pointer's type: the fast exponential and divide where bf16 rounding follows
 __device__ __forceinline__ float silu_for(float z, const float*) { return siluf_(z); }
 __device__ __forceinline__ float silu_for(float z, const __nv_bfloat16*) { return silu_fast_f32(z); }
@@ -878,11 +955,12 @@ __global__ void __launch_bounds__(128) hy_conv_silu_vec8_kernel(const __nv_bfloa
     }
 }
 template <typename TA>
-__global__ void hy_conv_tails_kernel(const TA* in, int ld_in, int C, int taps, TA* tails, HyRows r) {
+__global__ void hy_conv_tails_kernel(const TA* in, int ld_in, int C, int taps, TA* tails, HyRows r, int skip_len) {
     HY_PDL();
     const int c = blockIdx.x * blockDim.x + threadIdx.x, seq = blockIdx.y;
     if (c >= C) return;
     const int row0 = r.seq_row0[seq], len = r.seq_row0[seq + 1] - row0, pos0 = r.seq_pos0[seq];
+    if (len <= skip_len) return;
     TA* tail = tails + (long long)r.seq_state[seq] * (taps - 1) * C;
     float v[16];
     for (int j = 0; j < taps - 1; ++j) v[j] = conv_input(in, ld_in, C, tail, taps, row0, pos0, len - (taps - 1) + j, c);
@@ -1504,15 +1582,18 @@ static cudaError_t gemm_t(int mode, const void* A, int lda, const void* B, int l
     }
     return cudaErrorInvalidValue;
 }
-cudaError_t hy_gemm(bool f32, int mode, const void* A, int lda, const void* B, int ldb, void* C, int ldc, int M, int N, int K, const float* bias, float alpha, int batch,
-                    long long sA, long long sB, long long sC, cudaStream_t s, HyGemmAct act) {
-    if (M <= 0 || N <= 0 || K <= 0 || batch <= 0) return cudaSuccess;
+static bool few_rows_ok(const void* A, int lda, const void* B, int ldb, int M, int K, long long sA, long long sB) {
     auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
-    if (!f32 && M <= HY_GEMM_FEW_ROWS && K % 8 == 0 && K <= 1024 && lda % 8 == 0 && ldb % 8 == 0 && sA % 8 == 0 && sB % 8 == 0 && al16(A) && al16(B)) {
+    return M <= HY_GEMM_FEW_ROWS && K % 8 == 0 && K <= 1024 && lda % 8 == 0 && ldb % 8 == 0 && sA % 8 == 0 && sB % 8 == 0 && al16(A) && al16(B);
+}
+cudaError_t hy_gemm(bool f32, int mode, const void* A, int lda, const void* B, int ldb, void* C, int ldc, int M, int N, int K, const float* bias, float alpha, int batch,
+                    long long sA, long long sB, long long sC, cudaStream_t s, HyGemmAct act, bool b_weights) {
+    if (M <= 0 || N <= 0 || K <= 0 || batch <= 0) return cudaSuccess;
+    if (!f32 && few_rows_ok(A, lda, B, ldb, M, K, sA, sB)) {
         const bool half = K <= 128;
         const dim3 grid(half ? (N + 15) / 16 : (N + 7) / 8, batch, (M + 7) / 8);
-#define HY_FEW(MODE) (half ? launch_plain(hy_gemm_fewrows_kernel<MODE, 16>, grid, dim3(128), 0, s, (const bf*)A, lda, (const bf*)B, ldb, C, ldc, M, N, K, bias, alpha, sA, sB, sC, act) \
-                           : launch_plain(hy_gemm_fewrows_kernel<MODE, 32>, grid, dim3(128), 0, s, (const bf*)A, lda, (const bf*)B, ldb, C, ldc, M, N, K, bias, alpha, sA, sB, sC, act))
+#define HY_FEW(MODE) (half ? launch_plain(hy_gemm_fewrows_kernel<MODE, 16>, grid, dim3(128), 0, s, (const bf*)A, lda, (const bf*)B, ldb, C, ldc, M, N, K, bias, alpha, sA, sB, sC, act, b_weights) \
+                           : launch_plain(hy_gemm_fewrows_kernel<MODE, 32>, grid, dim3(128), 0, s, (const bf*)A, lda, (const bf*)B, ldb, C, ldc, M, N, K, bias, alpha, sA, sB, sC, act, b_weights))
         return mode == HY_STORE ? HY_FEW(HY_STORE) : mode == HY_STORE_F32 ? HY_FEW(HY_STORE_F32) : HY_FEW(HY_ACC_F32);
 #undef HY_FEW
     }
@@ -1520,6 +1601,10 @@ cudaError_t hy_gemm(bool f32, int mode, const void* A, int lda, const void* B, i
                : gemm_t<bf>(mode, A, lda, B, ldb, C, ldc, M, N, K, bias, alpha, batch, sA, sB, sC, s, act);
 }
 cudaError_t hy_embed(bool f32, const int32_t* ids, const void* table, float* x, float* x0, int T, int W, int vocab, float scale, cudaStream_t s, void* h, int ldh) {
+    auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+    if (W % 8 == 0 && ldh % 8 == 0 && al16(table) && al16(x) && al16(x0) && al16(h))
+        return f32 ? launch_plain(hy_embed_vec8_kernel<float>, dim3(T), dim3(256), 0, s, ids, (const float*)table, x, x0, W, vocab, scale, (float*)h, ldh)
+                   : launch_plain(hy_embed_vec8_kernel<bf>, dim3(T), dim3(256), 0, s, ids, (const bf*)table, x, x0, W, vocab, scale, (bf*)h, ldh);
     return f32 ? launch_plain(hy_embed_kernel<float>, dim3(T), dim3(128), 0, s, ids, (const float*)table, x, x0, T, W, vocab, scale, (float*)h, ldh)
                : launch_plain(hy_embed_kernel<bf>, dim3(T), dim3(128), 0, s, ids, (const bf*)table, x, x0, T, W, vocab, scale, (bf*)h, ldh);
 }
@@ -1539,6 +1624,15 @@ cudaError_t hy_mla_prep(bool f32, const HyLatentAttn& a, const void* q, int ldq,
                         const float* rope_sin, void* cache, float* q_abs, const HyRows& r, cudaStream_t s) {
     return f32 ? launch_plain(hy_mla_prep_kernel<float>, dim3(r.T), dim3(128), 0, s, a, (const float*)q, ldq, (const float*)ckv, ldc, norm_w, eps, rope_cos, rope_sin, (float*)cache, q_abs, r)
                : launch_plain(hy_mla_prep_kernel<bf>, dim3(r.T), dim3(128), 0, s, a, (const bf*)q, ldq, (const bf*)ckv, ldc, norm_w, eps, rope_cos, rope_sin, (bf*)cache, q_abs, r);
+}
+// both in one launch where the products' kernel of a few rows takes them; else cudaErrorNotSupported and nothing is launched
+cudaError_t hy_mla_prep_absorb(const HyLatentAttn& a, const void* q, int ldq, const void* ckv, int ldc, const float* norm_w, float eps, const float* rope_cos, const float* rope_sin,
+                               void* cache, float* q_abs, const void* uk_t, const HyRows& r, cudaStream_t s) {
+    if (r.T <= 0 || a.dim <= 0 || !few_rows_ok(q, ldq, uk_t, a.dim, r.T, a.dim, a.dim + a.rot_dim, (long long)a.kv_rank * a.dim)) return cudaErrorNotSupported;
+    const bool half = a.dim <= 128;
+    const int nx = half ? (a.kv_rank + 15) / 16 : (a.kv_rank + 7) / 8, grid = r.T + nx * a.heads * ((r.T + 7) / 8);
+    return half ? launch_plain(hy_mla_prep_absorb_kernel<16>, dim3(grid), dim3(128), 0, s, a, (const bf*)q, ldq, (const bf*)ckv, ldc, norm_w, eps, rope_cos, rope_sin, (bf*)cache, q_abs, r, (const bf*)uk_t, nx)
+                : launch_plain(hy_mla_prep_absorb_kernel<32>, dim3(grid), dim3(128), 0, s, a, (const bf*)q, ldq, (const bf*)ckv, ldc, norm_w, eps, rope_cos, rope_sin, (bf*)cache, q_abs, r, (const bf*)uk_t, nx);
 }
 cudaError_t hy_mla_attention(bool f32, const HyLatentAttn& a, const float* q_abs, const void* cache, void* lat_out, const HyRows& r, cudaStream_t s) {
     if (a.kv_rank > 32 * MLA_ACC) return cudaErrorInvalidValue;
@@ -1657,11 +1751,11 @@ cudaError_t hy_conv_silu(bool f32, const void* in, int ld_in, int C, const float
     return f32 ? launch_plain(hy_conv_silu_kernel<float>, grid, dim3(128), 0, s, (const float*)in, ld_in, C, w, bias, taps, (float*)out, ld_out, (const float*)tails, r, act)
                : launch_plain(hy_conv_silu_kernel<bf>, grid, dim3(128), 0, s, (const bf*)in, ld_in, C, w, bias, taps, (bf*)out, ld_out, (const bf*)tails, r, act);
 }
-cudaError_t hy_conv_tails(bool f32, const void* in, int ld_in, int C, int taps, void* tails, const HyRows& r, cudaStream_t s) {
+cudaError_t hy_conv_tails(bool f32, const void* in, int ld_in, int C, int taps, void* tails, const HyRows& r, cudaStream_t s, int skip_len) {
     if (taps <= 1) return cudaSuccess;
     dim3 grid((C + 127) / 128, r.S);
-    return f32 ? launch_plain(hy_conv_tails_kernel<float>, grid, dim3(128), 0, s, (const float*)in, ld_in, C, taps, (float*)tails, r)
-               : launch_plain(hy_conv_tails_kernel<bf>, grid, dim3(128), 0, s, (const bf*)in, ld_in, C, taps, (bf*)tails, r);
+    return f32 ? launch_plain(hy_conv_tails_kernel<float>, grid, dim3(128), 0, s, (const float*)in, ld_in, C, taps, (float*)tails, r, skip_len)
+               : launch_plain(hy_conv_tails_kernel<bf>, grid, dim3(128), 0, s, (const bf*)in, ld_in, C, taps, (bf*)tails, r, skip_len);
 }
 cudaError_t hy_delta_prep(bool f32, const HyDelta& d, const void* conv, int ld_conv, const void* b, int ld_b, const void* a, int ld_a, const float* A_log,
                           const float* dt_bias, float* qq, float* kk, float* vv, float* dec, float* beta, int T, cudaStream_t s) {

@@ -42,7 +42,7 @@ struct HyGemmAct { int kind = 0, col0 = 0, col1 = 0; };
 // bf16 steps of at most HY_GEMM_FEW_ROWS rows with K <= 1024 in aligned groups of 8 take a kernel of a few rows on fp32 FMA instead of the tile kernel
 constexpr int HY_GEMM_FEW_ROWS = 32;
 cudaError_t hy_gemm(bool f32, int mode, const void* A, int lda, const void* B, int ldb, void* C, int ldc, int M, int N, int K, const float* bias,
-                    float alpha, int batch, long long sA, long long sB, long long sC, cudaStream_t s, HyGemmAct act = HyGemmAct());
+                    float alpha, int batch, long long sA, long long sB, long long sC, cudaStream_t s, HyGemmAct act = HyGemmAct(), bool b_weights = false);      // b_weights: no kernel of the stream writes B
 
 // x[t] = table[ids[t]] * scale (fp32); x0 (optional) keeps a copy for a looped block's re-injection
 // h (optional, [T, ldh] in the activation type): the same rows as the input of sublayers that read the residual itself
@@ -134,6 +134,8 @@ struct HyLatentAttn {             // sizes of one latent-attention layer
 // parts go to q_abs[t, h, rank:] (fp32, [T, heads, rank + rot_dim]).
 cudaError_t hy_mla_prep(bool f32, const HyLatentAttn& a, const void* q, int ldq, const void* ckv, int ldc, const float* norm_w, float eps,
                         const float* rope_cos, const float* rope_sin, void* cache, float* q_abs, const HyRows& r, cudaStream_t s);
+cudaError_t hy_mla_prep_absorb(const HyLatentAttn& a, const void* q, int ldq, const void* ckv, int ldc, const float* norm_w, float eps, const float* rope_cos, const float* rope_sin,
+                               void* cache, float* q_abs, const void* uk_t, const HyRows& r, cudaStream_t s);      // bf16 steps of a few rows: prepared and absorbed in one launch, else cudaErrorNotSupported
 // causal softmax attention of every row over its sequence's cached rows 0..position, with absorbed queries q_abs = [W_uk^T q_unrotated | q_rotated]:
 // lat_out[t, h, :rank] = sum_j softmax_j(scale * q_abs[t,h] . cache[j]) cache[j][:rank]
 cudaError_t hy_mla_attention(bool f32, const HyLatentAttn& a, const float* q_abs, const void* cache, void* lat_out, const HyRows& r, cudaStream_t s);
@@ -170,7 +172,7 @@ cudaError_t hy_mha_prefill(const HyLatentAttn& a, const void* q, int ldq, const 
 // act = 0: no activation (y is the convolution itself)
 cudaError_t hy_conv_silu(bool f32, const void* in, int ld_in, int C, const float* w, const float* bias, int taps, void* out, int ld_out,
                          const void* tails, const HyRows& r, cudaStream_t s, int act = 1);
-cudaError_t hy_conv_tails(bool f32, const void* in, int ld_in, int C, int taps, void* tails, const HyRows& r, cudaStream_t s);
+cudaError_t hy_conv_tails(bool f32, const void* in, int ld_in, int C, int taps, void* tails, const HyRows& r, cudaStream_t s, int skip_len = 0);      // sequences of at most skip_len rows keep theirs
 
 struct HyDelta { int heads, kv_heads, dim, vdim, head_decay = 0; };
 // unit-norm q (times dim^-1/2) and k, v, beta = sigmoid(b), decay exp(-exp(A_log_h) softplus(a + dt_bias)) per key channel (a, dt_bias, dec: [heads, dim])
@@ -221,9 +223,10 @@ cudaError_t hy_lightning_mix(const HyBlockHead& m, const void* q, const void* k,
 // weight norm_w [vdim], times silu(gate).  conv [T, ld_conv] = the activated short convolutions' rows [q heads | k heads | v heads] (read for `many` sequences); the rows of
 // `few` sequences go through the convolution here, from its inputs in [T, ld_in] (same columns), taps conv_w [channels, taps] and the carried tails.
 // a, b, gate: projections [T, ld_in]; out [T, ldo] bf16
-struct HyDeltaMix { const void* conv; int ld_conv; const void* in; int ld_in; const float* conv_w; int taps; const void* tails; const void* a; const void* b; const void* gate;
+struct HyDeltaMix { const void* conv; int ld_conv; const void* in; int ld_in; const float* conv_w; int taps; void* tails; const void* a; const void* b; const void* gate;
                     const float* A_log; const float* dt_bias; const float* norm_w; float eps; };
 cudaError_t hy_delta_mix(const HyBlockHead& m, const HyDeltaMix& d, float* state, void* out, int ldo, bool few, bool many, const HyRows& r, cudaStream_t s);
+bool hy_delta_leaves_tails(const HyBlockHead& m, const HyDeltaMix& d);      // hy_delta_mix stores the new tails of `few` sequences; those of `many` are hy_conv_tails' (skip_len) then
 // Matrix memory.  gates [T, ldg] fp32 = [W_i h + b_i | W_f h + b_f] (heads each).  hy_mlstm_gates: log gates i = cap tanh(. / cap),
 // f = logsigmoid(cap tanh(. / cap)); the running maximum m_t = max(f_t + m_(t-1), i_t) per (sequence, head), carried in mstate [slots, heads]
 // (a sequence whose step starts at position 0 starts from m = 0); out: dec[t, h] = exp(f + m_(t-1) - m_t), gin[t, h] = exp(i - m_t), floor_[t, h] = exp(-m_t)

@@ -600,7 +600,7 @@ void HybridModel::gemm(int mode, const void* A, int lda, const Mat& B, void* C, 
     const GemmChoice choice = gemm_choice(g, epi, bn);
     CUtensorMap tmA;
     if (tc && make_tmap_bf16_2d(&tmA, A, (uint64_t)M, (uint64_t)B.ld, (uint64_t)lda, (uint32_t)choice.a_box, 64) != 0) tc = false;
-    if (!tc) { cuda_check(hy_gemm(f32_, mode, A, lda, B.p, B.ld, C, ldc, M, B.N, B.K, bias, alpha, 1, 0, 0, 0, stream, act), "gemm"); return; }
+    if (!tc) { cuda_check(hy_gemm(f32_, mode, A, lda, B.p, B.ld, C, ldc, M, B.N, B.K, bias, alpha, 1, 0, 0, 0, stream, act, true), "gemm"); return; }
     const CUtensorMap* tmB = &B.tm[gemm_b_box_index(choice.b_box)];
     if (mode == HY_STORE) { g.out = C; g.ldo = ldc; g.bias = bias ? bias_act : nullptr; g.store_act = act.kind; g.act_col0 = act.col0; g.act_col1 = act.col1; cuda_check(launch_gemm(&tmA, tmB, g, EPI_STORE, bn, stream, &choice), "gemm (tcgen05)"); return; }
     g.f32_out = reinterpret_cast<float*>(C); g.ldf = ldc; g.f32_accumulate = mode == HY_ACC_F32; g.alpha = alpha; g.bias_f32 = bias;
@@ -751,8 +751,11 @@ void HybridModel::delta_mixer(const HyRun& run, const HyLayer& l, const LayerW& 
         const void* in = at(proj_, w.off_a);
         if (many_rows_) { cuda_check(hy_conv_silu(f32_, in, ld_proj_, w.conv_ch, w.conv_w, nullptr, l.conv, conv_, ld_conv_, tails_[run.state_idx], r, stream), "conv"); MARK(6); }
         const HyDeltaMix dm{conv_, ld_conv_, in, ld_proj_, w.conv_w, l.conv, tails_[run.state_idx], at(proj_, w.off_c), at(proj_, w.off_b), at(proj_, w.off_d), w.A_log, w.dt_bias, w.norm_w, hc_.eps};
-        cuda_check(hy_delta_mix(HyBlockHead{l.heads, l.kv_heads, l.dim, l.vdim}, dm, states_[run.state_idx], mix_, ld_mix_, few_rows_, many_rows_, r, stream), "delta rule"); MARK(8);
-        cuda_check(hy_conv_tails(f32_, in, ld_proj_, w.conv_ch, l.conv, tails_[run.state_idx], r, stream), "conv tails"); MARK(6);
+        const HyBlockHead head{l.heads, l.kv_heads, l.dim, l.vdim};
+        const bool left = hy_delta_leaves_tails(head, dm);
+        cuda_check(hy_delta_mix(head, dm, states_[run.state_idx], mix_, ld_mix_, few_rows_, many_rows_, r, stream), "delta rule"); MARK(8);
+        if (many_rows_ || !left) cuda_check(hy_conv_tails(f32_, in, ld_proj_, w.conv_ch, l.conv, tails_[run.state_idx], r, stream, left ? HY_FORGET_FEW_ROWS : 0), "conv tails");
+        MARK(6);
         return;
     }
     cuda_check(hy_conv_silu(f32_, at(proj_, w.off_a), ld_proj_, w.conv_ch, w.conv_w, nullptr, l.conv, conv_, ld_conv_, tails_[run.state_idx], r, stream), "conv");
@@ -806,13 +809,18 @@ void HybridModel::latent_mixer(const HyRun& run, const HyLayer& l, const LayerW&
     HyLatentAttn a = latent_params(l, w);
     if (l.gate == HY_GATE_HEAD) { a.head_gate = gate; a.ldg = ldg; gate = nullptr; }        // a factor per head rides in the attention kernels' epilogues
     const int E = l.kv_rank + l.rot_dim;
-    cuda_check(hy_mla_prep(f32_, a, q, ldq, ckv, ldc, w.dkv_norm, hc_.eps, ropes_[w.rope].cos, ropes_[w.rope].sin, caches_[run.cache_idx], q_abs_, r, stream), "latent cache write"); MARK(4);
+    const bool head_tc = tl.any_small && !w.uk_heads.empty() && T >= 256 && ldq % 8 == 0;      // prefill-sized steps: one tcgen05 GEMM per head; smaller ones: one batched launch
+    cudaError_t absorbed = cudaErrorNotSupported;
+    if (tl.any_small && !head_tc && !f32_)
+        absorbed = hy_mla_prep_absorb(a, q, ldq, ckv, ldc, w.dkv_norm, hc_.eps, ropes_[w.rope].cos, ropes_[w.rope].sin, caches_[run.cache_idx], q_abs_, w.uk_t, r, stream);
+    if (absorbed != cudaErrorNotSupported) cuda_check(absorbed, "latent cache write and query absorption");
+    else cuda_check(hy_mla_prep(f32_, a, q, ldq, ckv, ldc, w.dkv_norm, hc_.eps, ropes_[w.rope].cos, ropes_[w.rope].sin, caches_[run.cache_idx], q_abs_, r, stream), "latent cache write");
+    MARK(4);
     if (tl.any_small) {
         // absorbed queries: q_abs[t, h, :rank] = W_uk[h]^T q_unrotated[t, h]
-        const bool head_tc = !w.uk_heads.empty() && T >= 256 && ldq % 8 == 0;      // prefill-sized steps: one tcgen05 GEMM per head; smaller ones: one batched launch
         if (head_tc) for (int hd = 0; hd < l.heads; ++hd) gemm(HY_STORE_F32, at(q, (size_t)hd * (l.dim + l.rot_dim)), ldq, w.uk_heads[hd], q_abs_ + (size_t)hd * E, l.heads * E, T, nullptr, 1.f);
-        else cuda_check(hy_gemm(f32_, HY_STORE_F32, q, ldq, w.uk_t, l.dim, q_abs_, l.heads * E, T, l.kv_rank, l.dim, nullptr, 1.f, l.heads,
-                                l.dim + l.rot_dim, (long long)l.kv_rank * l.dim, E, stream), "query absorption");
+        else if (absorbed != cudaSuccess) cuda_check(hy_gemm(f32_, HY_STORE_F32, q, ldq, w.uk_t, l.dim, q_abs_, l.heads * E, T, l.kv_rank, l.dim, nullptr, 1.f, l.heads,
+                                l.dim + l.rot_dim, (long long)l.kv_rank * l.dim, E, stream, HyGemmAct(), true), "query absorption");
         MARK(3);
         if (tl.mma) {
             HyMlaSplit sp{nullptr, nullptr, nullptr, split_o_, split_ml_};
@@ -826,7 +834,7 @@ void HybridModel::latent_mixer(const HyRun& run, const HyLayer& l, const LayerW&
         MARK(5);
         if (head_tc) for (int hd = 0; hd < l.heads; ++hd) gemm(HY_STORE, at(lat_, (size_t)hd * l.kv_rank), l.heads * l.kv_rank, w.uv_heads[hd], at(mix_, (size_t)hd * l.vdim), ld_mix_, T, nullptr, 1.f);
         else cuda_check(hy_gemm(f32_, HY_STORE, lat_, l.heads * l.kv_rank, w.uv, l.kv_rank, mix_, ld_mix_, T, l.vdim, l.kv_rank, nullptr, 1.f, l.heads, l.kv_rank,
-                                (long long)l.vdim * l.kv_rank, l.vdim, stream), "value up-projection");
+                                (long long)l.vdim * l.kv_rank, l.vdim, stream, HyGemmAct(), true), "value up-projection");
         MARK(3);
         if (gate) { cuda_check(hy_sigmoid_gate(f32_, mix_, ld_mix_, gate, ldg, l.heads * l.vdim, T, stream), "output gate"); MARK(9); }
     }

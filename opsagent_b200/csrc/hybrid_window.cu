@@ -137,11 +137,20 @@ __global__ void __launch_bounds__(128) hy_win_prep_whole_kernel(HyWinAttn a, TA*
 __global__ void __launch_bounds__(128) hy_win_prep_whole_vec8_kernel(HyWinAttn a, __nv_bfloat16* __restrict__ q, int ldq, const __nv_bfloat16* __restrict__ k,
                                                                      const __nv_bfloat16* __restrict__ v, int ldkv, const float* __restrict__ qw, const float* __restrict__ kw, float eps,
                                                                      __nv_bfloat16* __restrict__ cache, HyRows r, HyRotary rot) {
-    HY_PDL();
-    __shared__ float red[32];
+    griddep_launch();
+    __shared__ float red[32], red2[32];
     const long long t = blockIdx.x;
     const int QW = a.heads * a.maps * a.dim, KW = a.kv_heads * a.maps * a.dim, VW = a.kv_heads * a.vdim, CW = KW + VW;
     __nv_bfloat16* qr = q + t * ldq; __nv_bfloat16* crow = cache + (long long)r.slots[t] * CW;
+    // Slot, position, norm weights and rotation factors come from the host or are weights: on their way ahead of the wait (what a decoding step reads behind it,
+    // it waits for one load after the other).
+    const int pos = r.positions[t], half = rot.dims / 2;
+    const float temp = win_q_temp(a, pos);
+    const float* cs = rot.cos + (long long)pos * half; const float* sn = rot.sin + (long long)pos * half;
+    for (int c = threadIdx.x * 32; c < QW; c += blockDim.x * 32) asm volatile("prefetch.global.L1 [%0];" ::"l"(qw + c));
+    if (k) for (int c = threadIdx.x * 32; c < KW; c += blockDim.x * 32) asm volatile("prefetch.global.L1 [%0];" ::"l"(kw + c));
+    for (int c = threadIdx.x * 32; c < half; c += blockDim.x * 32) { asm volatile("prefetch.global.L1 [%0];" ::"l"(cs + c)); asm volatile("prefetch.global.L1 [%0];" ::"l"(sn + c)); }
+    griddep_wait();
     auto sq8 = [](const uint4& u) {
         const float x[8] = {bf16lo(u.x), bf16hi(u.x), bf16lo(u.y), bf16hi(u.y), bf16lo(u.z), bf16hi(u.z), bf16lo(u.w), bf16hi(u.w)};
         float s = 0.f;
@@ -157,11 +166,11 @@ __global__ void __launch_bounds__(128) hy_win_prep_whole_vec8_kernel(HyWinAttn a
     float sq = 0.f, sk = 0.f;
     for (int c = threadIdx.x * 8; c < QW; c += blockDim.x * 8) sq += sq8(*reinterpret_cast<const uint4*>(qr + c));
     if (k) for (int c = threadIdx.x * 8; c < KW; c += blockDim.x * 8) sk += sq8(*reinterpret_cast<const uint4*>(k + t * ldkv + c));
-    const float rq = 1.0f / sqrtf(block_sum(sq, red) / (float)QW + eps) * win_q_temp(a, r.positions[t]);
-    const float rk = k ? 1.0f / sqrtf(block_sum(sk, red) / (float)KW + eps) : 0.f;
+    if (v) for (int c = threadIdx.x * 8; c < VW; c += blockDim.x * 8) *reinterpret_cast<uint4*>(crow + KW + c) = *reinterpret_cast<const uint4*>(v + t * ldkv + c);
+    block_sum2(sq, sk, red, red2);
+    const float rq = 1.0f / sqrtf(sq / (float)QW + eps) * temp;
+    const float rk = k ? 1.0f / sqrtf(sk / (float)KW + eps) : 0.f;
     // rotated channels: the thread of a group of 8 in a head's first half turns its partner group too (rotate-half pairs, rot.dims / 2 a multiple of 8)
-    const int half = rot.dims / 2;
-    const float* cs = rot.cos + (long long)r.positions[t] * half; const float* sn = rot.sin + (long long)r.positions[t] * half;
     auto norm8 = [](const uint4& u, float rr, const float* w, float* f) {
         const float4 w0 = *reinterpret_cast<const float4*>(w), w1 = *reinterpret_cast<const float4*>(w + 4);
         f[0] = bf16lo(u.x) * rr * w0.x; f[1] = bf16hi(u.x) * rr * w0.y; f[2] = bf16lo(u.y) * rr * w0.z; f[3] = bf16hi(u.y) * rr * w0.w;
@@ -180,7 +189,6 @@ __global__ void __launch_bounds__(128) hy_win_prep_whole_vec8_kernel(HyWinAttn a
     };
     for (int c = threadIdx.x * 8; c < QW; c += blockDim.x * 8) finish(qr, qr, qw, rq, c);
     if (k) for (int c = threadIdx.x * 8; c < KW; c += blockDim.x * 8) finish(k + t * ldkv, crow, kw, rk, c);
-    if (v) for (int c = threadIdx.x * 8; c < VW; c += blockDim.x * 8) *reinterpret_cast<uint4*>(crow + KW + c) = *reinterpret_cast<const uint4*>(v + t * ldkv + c);
 }
 
 // score modifiers shared by every form: s is the scaled score of the query at position p (head h) with the key at position j
