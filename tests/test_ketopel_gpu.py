@@ -419,3 +419,20 @@ def test_greedy_generation_through_the_scheduler(tmp_path, dtype):
                 assert lg.max() - lg[tok] < (1e-3 if dtype == "float32" else 0.2), "greedy token differs from the oracle's outside a near tie"
                 break
             seq.append(tok)
+
+
+# the token form of the delta rule leaves the carried convolution inputs itself (four taps; heads that share a query head are a cluster, more than eight are not), beside
+# the block form of portions above four rows; rows of a few tokens prepare and absorb a latent layer's queries in one launch (up to 128 channels, and above)
+@pytest.mark.parametrize("delta,latent", [(dict(heads=3, kv_heads=3, dim=128, vdim=128, conv=4), dict(heads=2, dim=128, rot_dim=64, vdim=32, kv_rank=512)),
+                                          (dict(heads=4, kv_heads=2, dim=128, vdim=128, conv=4), dict(heads=3, dim=136, rot_dim=16, vdim=32, kv_rank=64)),
+                                          (dict(heads=8, kv_heads=1, dim=16, vdim=24, conv=4), dict(heads=16, dim=8, rot_dim=8, vdim=16, kv_rank=640)),
+                                          (dict(heads=9, kv_heads=1, dim=16, vdim=16, conv=4), dict(heads=5, dim=24, rot_dim=0, vdim=16, kv_rank=64))])
+def test_short_portions_leave_what_the_next_ones_carry(tmp_path, delta, latent):
+    cfg = K.make_config([D(**delta), L(**latent), D(**delta)], width=64, vocab=96)
+    W = checkpoint(tmp_path, cfg, seed=19)
+    toks = tokens_of(cfg, 60, 3)
+    want = K.forward(cfg, W, toks)
+    with engine(tmp_path, "bfloat16") as eng:
+        for cuts in ([1, 2, 3, 4, 5, 1, 4, 1, 6, 2, 1, 1, 3], [5, 1, 1, 20, 2, 4], [4, 4, 4]):
+            e = K.rel_err(replay(eng, 1, toks, cuts).astype(np.float64), want)
+            assert np.quantile(e, 0.95) < 0.05 and e.max() < 0.1, f"cuts {cuts}: 95% {np.quantile(e, 0.95):.3e}, worst {e.max():.3e}"
