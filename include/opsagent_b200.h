@@ -184,7 +184,7 @@ OA_API int oa_host_streamk_plan(int32_t N, int32_t K, int32_t block_n, int32_t n
  * come from a table */
 OA_API int oa_host_gemm_kernel(int32_t M, int32_t N, int32_t K, int32_t epilogue, int32_t block_n, int32_t few_rows, int32_t grouped);
 /* columns of the tiles the CTA-pair kernel takes for that product (128, 160, .. 256), 0 where another kernel runs it */
-/* the kernel that oa_k_paged_attention takes for a batch of prompts: 1 one head per CTA, 2 two heads per CTA, 3 two heads per CTA pair (the same bits) */
+/* the kernel that oa_k_paged_attention takes for a batch of prompts: 1 one head per CTA, 2 two heads per CTA, 3 and 4 key tiles in turns on a CTA pair or a CTA (the same bits) */
 OA_API int oa_host_prefill_attention_kernel(const int32_t* ctx_lens, const int32_t* q_lens, int32_t n_seqs, int32_t n_heads, int32_t n_kv, int32_t head_dim);
 OA_API int oa_host_gemm_pair_width(int32_t M, int32_t N, int32_t K, int32_t epilogue, int32_t block_n);
 /* byte-level BPE tokenizer read from a Hugging Face tokenizer.json (Llama-3 / Qwen2.5 format), host only: what the engine uses

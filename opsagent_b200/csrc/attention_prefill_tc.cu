@@ -653,30 +653,34 @@ __global__ void __launch_bounds__(PtpCfg<D>::THREADS, 1) prefill_attention_pair_
 }
 
 // ---------------------------------------------------------------------------------------------
-// Two heads of one key/value group on a CTA PAIR, heads of 128.
+// Softmax warpgroups that take a head's key tiles in turn: heads of 128 on a CTA PAIR (two heads of one key/value group), heads of 64 on a CTA.
 //
 // The kernel above is bound by a head's chain in a tile: its S may only be computed once the P that stands over the last one has been multiplied, and TMEM has
-// no room for a second S of both heads.  Here each CTA of a pair carries ONE head's 128 rows, so TMEM holds three S tiles and O, and the two softmax
+// no room for a second S of two heads.  Here a CTA carries ONE head's 128 rows, so TMEM holds three S tiles and O, and the two softmax
 // warpgroups take the tiles in turn: while one takes the exponentials of tile t, the other fetches S and finds the maxima of t + 1, and the tensor core
 // runs P V of t - 1 and S of t + 2.  What a head still does in order is one value a row: a tile's reference maximum follows from the last one's, so it goes from
-// warpgroup to warpgroup as soon as the maxima stand.  Keys and values are shared by the pair: a product is 256 x 128 x 16 (cta_group::2) with half of B in
-// each CTA, so each loads one of a tile's two K pages and 64 of V's 128 columns, half of what a CTA alone would have to fetch for its head (which would be the
-// L2's limit: 64 KB a tile in 1100 cycles).
-//   warp 0     : TMA: this CTA's Q (two items ahead), K page and V half           warp 1 (even CTA): tcgen05.mma for both
+// warpgroup to warpgroup as soon as the maxima stand.  With heads of 128 a CTA alone would fetch 64 KB of keys and values a tile, in 1300 cycles: what the L2 gives
+// (five prompts of 1.4 thousand rows 139 us, 1000 rows behind 6000 worse than above).  So two heads' CTAs share them: a product is 256 x 128 x 16
+// (cta_group::2) with half of B in each CTA, and each loads one of a tile's two K pages and 64 of V's 128 columns.  Heads of 64 need half the bytes and no pair.
+//   warp 0     : TMA: this CTA's Q (two items ahead), its share of K and V       warp 1 (of a pair: the even CTA's): tcgen05.mma
 //   warps 4-11 : softmax of even and odd tiles, one query row per thread         warps 12-15: output, while the next item's tiles run
 // A row's sums are kept per warpgroup (even and odd tiles of the item) and joined at its end, as in the kernels above: the same bits.
-// us, two heads a CTA -> here: 4096 rows behind 12288, 64 / 8 heads 1410 -> 1302; five prompts of 1.4 thousand rows, 32 / 8 heads 97 -> 84; 1000 rows behind 6000
-// 104 -> 88; 600 rows 14.7 -> 11.2 (one head a CTA: 14.7); 300 rows behind 6000 57 -> 46 (one head a CTA).  A launch costs 2 us more.
-// What bounds it now: a warpgroup takes 2600 cycles a tile, 1650 of them exponentials (1024 alone), 550 fetching S, the maxima and the reference, 120 waiting
+// us, two heads a CTA -> here: 4096 rows behind 12288, 64 / 8 heads of 128 1410 -> 1302; five prompts of 1.4 thousand rows, 32 / 8 heads of 128 97 -> 84; 1000 rows
+// behind 6000 104 -> 88; 600 rows 14.7 -> 11.2 (one head a CTA: 14.7); 300 rows behind 6000 57 -> 46 (one head a CTA).  A pair's launch costs 2 us more.  Heads of 64:
+// the five prompts 85.6 -> 76.5, 1400 rows behind 3000 93 -> 72, 600 rows 13.0 -> 8.9, 100 rows behind 3000 29.9 (one head a CTA) -> 22.7.
+// What bounds it now (128): a warpgroup takes 2600 cycles a tile, 1650 of them exponentials (1024 alone), 550 fetching S, the maxima and the reference, 120 waiting
 // for S; tensor and special-function pipes are busy 79 %, and the clock is down to 1.6 GHz in the long case (1.76 in the short ones).
 // Waits and arrivals are of CTA scope: what crosses the pair stands in TMEM (ordered by tcgen05.fence) or comes by TMA; with acquire and release of cluster
 // scope a tile took 2100 cycles instead of 1300.  Slower: S of two tiles and P of two in places of their own, S issued as soon as it is fetched (84 -> 90 us),
 // P handed over in two halves (85.5); no faster: the first item and its pages looked up ahead of the set-up.
 // ---------------------------------------------------------------------------------------------
+template <int D, int CTAS>
 struct PcpCfg {
-    static constexpr int D = 128, STAGES = 4, S_BUFS = 3;
+    static_assert(CTAS == 1 || D == 128, "a pair's V halves are 64 columns each");
+    static constexpr int S_BUFS = 3;
     static constexpr int Q_BYTES = 128 * D * 2, Q_HALF = 128 * 128;
-    static constexpr int KV_BYTES = 64 * D * 2, K_HALF = 64 * 128;       // a CTA's share of a K or V tile of 128 keys: 64 keys x 128, 128 keys x 64 columns
+    static constexpr int KV_BYTES = 128 / CTAS * D * 2, K_HALF = 128 / CTAS * 128;      // a CTA's share of a K or V tile of 128 keys (of a pair: 64 keys x 128, 128 keys x 64 columns)
+    static constexpr int STAGES = KV_BYTES > 16384 ? 2 : 4;
     static constexpr int OUT_WARP_BYTES = 32 * D * 2;
     static constexpr int ROWS_BYTES = 2 * 128 * 4;                       // one value per row and softmax warpgroup
     static constexpr int SMEM_BYTES = 2 * Q_BYTES + 2 * STAGES * KV_BYTES + 4 * OUT_WARP_BYTES + 2 * ROWS_BYTES + 512;
@@ -687,24 +691,27 @@ struct PcpCfg {
     static_assert(REGS_CONTROL + REGS_OUT + 2 * REGS_SOFTMAX <= 4 * 128, "an increase draws on what the launch gave: 512 threads x 128 registers");
 };
 
-// item of this pair of CTAs in round r (as above: heaviest first, every second round in reverse)
+// item of this CTA or pair in round r (as above: heaviest first, every second round in reverse)
 struct PcpItem { PrefillTile tile; int kvh, head0, n_kvt; };
-OA_DEVINL bool pcp_item(const PrefillAttnParams& p, int ppg, int round, PcpItem& it) {
-    const int G = (int)gridDim.x >> 1, pair = (int)blockIdx.x >> 1, per_tile = p.n_kv * ppg;
-    const int idx = round * G + ((round & 1) ? G - 1 - pair : pair);
+template <int CTAS>
+OA_DEVINL bool pcp_item(const PrefillAttnParams& p, int grp, int round, PcpItem& it) {
+    const int G = (int)gridDim.x / CTAS, me = (int)blockIdx.x / CTAS, per_tile = p.n_heads / CTAS;
+    const int idx = round * G + ((round & 1) ? G - 1 - me : me);
     if (idx >= p.n_tiles * per_tile) return false;
-    const int ti = idx / per_tile, hp = idx - ti * per_tile;
-    it.kvh = hp / ppg;
-    it.head0 = it.kvh * 2 * ppg + 2 * (hp - it.kvh * ppg);
+    const int ti = idx / per_tile;
+    it.head0 = (idx - ti * per_tile) * CTAS;
+    it.kvh = it.head0 / grp;
     it.tile = p.tiles[ti];
     it.n_kvt = (it.tile.pos0 + it.tile.n_rows + KV_TILE - 1) / KV_TILE;
     return true;
 }
 
-__global__ void __launch_bounds__(PcpCfg::THREADS, 1) prefill_attention_cluster_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_kv,
-                                                                                       const PrefillAttnParams p, const int64_t layer_row0, const int64_t kv_stride_rows) {
-    using Cfg = PcpCfg;
-    constexpr int D = Cfg::D, STAGES = Cfg::STAGES;
+template <int D, int CTAS>
+__global__ void __launch_bounds__(PcpCfg<D, CTAS>::THREADS, 1) prefill_attention_turns_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_kv,
+                                                                                              const PrefillAttnParams p, const int64_t layer_row0, const int64_t kv_stride_rows) {
+    using Cfg = PcpCfg<D, CTAS>;
+    constexpr int STAGES = Cfg::STAGES, HALVES = D / 64;
+    constexpr bool PAIR = CTAS == 2;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* q_s = smem_raw;                                     // [item & 1]
     uint8_t* k_s = q_s + 2 * Cfg::Q_BYTES;                       // [STAGES]
@@ -729,8 +736,9 @@ __global__ void __launch_bounds__(PcpCfg::THREADS, 1) prefill_attention_cluster_
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_empty + 1);
 
     const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // warp: uniform, and known to be
-    const uint32_t rank = gp_rank();
-    const int ppg = p.n_heads / p.n_kv / 2;
+    const uint32_t rank = PAIR ? gp_rank() : 0;
+    const int grp = p.n_heads / p.n_kv;
+    auto arrive_even = [&](uint64_t* bar) { if (PAIR) gp_arrive_tmem(gp_mapa(bar, 0)); else mbar_arrive(bar); };
     PcpItem it;
 
     if (warp == 0 && lane == 0) {
@@ -738,18 +746,20 @@ __global__ void __launch_bounds__(PcpCfg::THREADS, 1) prefill_attention_cluster_
         for (int i = 0; i < 2; ++i) { mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1); }
         for (int i = 0; i < STAGES; ++i) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
         for (int i = 0; i < 6; ++i) mbar_init(&s_full[i], 1);
-        for (int i = 0; i < Cfg::S_BUFS; ++i) mbar_init(&p_full[i], 8);
+        for (int i = 0; i < Cfg::S_BUFS; ++i) mbar_init(&p_full[i], 4 * CTAS);
         for (int i = 0; i < 8; ++i) mbar_init(&r_full[i], 1);
-        mbar_init(l_full, 8); mbar_init(l_empty, 4); mbar_init(o_full, 1); mbar_init(o_empty, 8);
+        mbar_init(l_full, 8); mbar_init(l_empty, 4); mbar_init(o_full, 1); mbar_init(o_empty, 4 * CTAS);
         fence_barrier_init();
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_slot)) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        if (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_slot)) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else tmem_alloc<512>(tmem_slot);
     }
     tcgen05_fence_before();
     __syncthreads();
-    gp_cluster_sync();                               // the other CTA's barriers are initialised before anything arrives on them
+    if (PAIR) gp_cluster_sync();                     // the other CTA's barriers are initialised before anything arrives on them
     tcgen05_fence_after();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     griddep_launch();
@@ -761,7 +771,7 @@ __global__ void __launch_bounds__(PcpCfg::THREADS, 1) prefill_attention_cluster_
             uint32_t kc = 0;
             int r = 0;
             PcpItem next;
-            bool more = pcp_item(p, ppg, 0, it);
+            bool more = pcp_item<CTAS>(p, grp, 0, it);
             for (; more; ++r, it = next) {
                 const int n_kvt = __shfl_sync(0xffffffffu, it.n_kvt, 0);
                 const int32_t* bt = p.block_tables + (size_t)it.tile.seq * p.max_pages_per_seq;
@@ -772,11 +782,18 @@ __global__ void __launch_bounds__(PcpCfg::THREADS, 1) prefill_attention_cluster_
                     mbar_wait(&k_empty[st], ph ^ 1);
                     if (elect_one()) {
                         uint8_t* dst = k_s + st * Cfg::KV_BYTES;
-                        if (rank == 0) mbar_expect_tx(&k_full[st], 2 * Cfg::KV_BYTES);              // both CTAs' shares
-                        const uint32_t bar = gp_mapa(&k_full[st], 0);
-                        const int32_t row = (int32_t)(rank ? r1 : r0);
-                        gp_tma_load(dst, &tm_kv, bar, 0, row, kEvictLast);
-                        gp_tma_load(dst + Cfg::K_HALF, &tm_kv, bar, 64, row, kEvictLast);
+                        if (rank == 0) mbar_expect_tx(&k_full[st], CTAS * Cfg::KV_BYTES);           // both CTAs' shares
+                        if (PAIR) {
+                            const uint32_t bar = gp_mapa(&k_full[st], 0);
+                            const int32_t row = (int32_t)(rank ? r1 : r0);
+                            gp_tma_load(dst, &tm_kv, bar, 0, row, kEvictLast);
+                            gp_tma_load(dst + Cfg::K_HALF, &tm_kv, bar, 64, row, kEvictLast);
+                        } else
+#pragma unroll
+                            for (int h = 0; h < HALVES; ++h) {
+                                tma_load_2d(dst + h * Cfg::K_HALF, &tm_kv, &k_full[st], h * 64, (int32_t)r0, kEvictLast);
+                                tma_load_2d(dst + h * Cfg::K_HALF + 8192, &tm_kv, &k_full[st], h * 64, (int32_t)r1, kEvictLast);
+                            }
                     }
                     __syncwarp();
                     if (j == 0) {
@@ -784,24 +801,33 @@ __global__ void __launch_bounds__(PcpCfg::THREADS, 1) prefill_attention_cluster_
                         mbar_wait(&q_empty[qb], (((uint32_t)r >> 1) & 1) ^ 1);
                         if (elect_one()) {
                             uint8_t* dst = q_s + qb * Cfg::Q_BYTES;
-                            if (rank == 0) mbar_expect_tx(&q_full[qb], 2 * Cfg::Q_BYTES);
-                            const uint32_t bar = gp_mapa(&q_full[qb], 0);
+                            if (rank == 0) mbar_expect_tx(&q_full[qb], CTAS * Cfg::Q_BYTES);
                             const int32_t col = (it.head0 + (int)rank) * D;
-                            gp_tma_load(dst, &tm_q, bar, col, it.tile.q_row0, kEvictFirst);
-                            gp_tma_load(dst + Cfg::Q_HALF, &tm_q, bar, col + 64, it.tile.q_row0, kEvictFirst);
+#pragma unroll
+                            for (int h = 0; h < HALVES; ++h) {
+                                if (PAIR) gp_tma_load(dst + h * Cfg::Q_HALF, &tm_q, gp_mapa(&q_full[qb], 0), col + h * 64, it.tile.q_row0, kEvictFirst);
+                                else tma_load_2d(dst + h * Cfg::Q_HALF, &tm_q, &q_full[qb], col + h * 64, it.tile.q_row0, kEvictFirst);
+                            }
                         }
                         __syncwarp();
-                        more = pcp_item(p, ppg, r + 1, next);                  // read now, needed an item later
+                        more = pcp_item<CTAS>(p, grp, r + 1, next);                  // read now, needed an item later
                     }
                     int64_t n0 = r0, n1 = r1;                                  // the next tile's pages are looked up while this one's slot is waited for
                     if (j + 1 < n_kvt) { n0 = page_row(2 * j + 2, 0); n1 = page_row(2 * j + 3, 2 * j + 2); }
                     mbar_wait(&v_empty[st], ph ^ 1);
                     if (elect_one()) {
                         uint8_t* dst = v_s + st * Cfg::KV_BYTES;
-                        if (rank == 0) mbar_expect_tx(&v_full[st], 2 * Cfg::KV_BYTES);
-                        const uint32_t bar = gp_mapa(&v_full[st], 0);
-                        gp_tma_load(dst, &tm_kv, bar, (int)rank * 64, (int32_t)(r0 + kv_stride_rows), kEvictLast);
-                        gp_tma_load(dst + 8192, &tm_kv, bar, (int)rank * 64, (int32_t)(r1 + kv_stride_rows), kEvictLast);
+                        if (rank == 0) mbar_expect_tx(&v_full[st], CTAS * Cfg::KV_BYTES);
+                        if (PAIR) {
+                            const uint32_t bar = gp_mapa(&v_full[st], 0);
+                            gp_tma_load(dst, &tm_kv, bar, (int)rank * 64, (int32_t)(r0 + kv_stride_rows), kEvictLast);
+                            gp_tma_load(dst + 8192, &tm_kv, bar, (int)rank * 64, (int32_t)(r1 + kv_stride_rows), kEvictLast);
+                        } else
+#pragma unroll
+                            for (int h = 0; h < HALVES; ++h) {
+                                tma_load_2d(dst + h * 16384, &tm_kv, &v_full[st], h * 64, (int32_t)(r0 + kv_stride_rows), kEvictLast);
+                                tma_load_2d(dst + h * 16384 + 8192, &tm_kv, &v_full[st], h * 64, (int32_t)(r1 + kv_stride_rows), kEvictLast);
+                            }
                     }
                     __syncwarp();
                     r0 = n0; r1 = n1;
@@ -811,12 +837,13 @@ __global__ void __launch_bounds__(PcpCfg::THREADS, 1) prefill_attention_cluster_
             for (int i = 0; i < 2; ++i, ++r) mbar_wait(&q_empty[r & 1], (((uint32_t)r >> 1) & 1) ^ 1);                  // releases have arrived here before the CTA may go
         } else if (warp == 1 && rank == 0) {
             // The whole warp walks the loop, an elected lane issues: descriptors stay in uniform registers.  S runs two tiles ahead of P V, across items.
-            constexpr uint32_t idesc_s = umma_idesc_bf16(256, KV_TILE), idesc_o = umma_idesc_bf16_bmn(256, D);
-            const uint64_t q_desc = umma_desc_sw128(smem_u32(q_s)), k_desc = umma_desc_sw128(smem_u32(k_s)), v_desc = umma_desc_sw128_mn(smem_u32(v_s), (uint32_t)Cfg::KV_BYTES, 1024u);
+            constexpr uint32_t idesc_s = umma_idesc_bf16(128 * CTAS, KV_TILE), idesc_o = umma_idesc_bf16_bmn(128 * CTAS, D);
+            auto commit = [&](uint64_t* bar) { if (PAIR) gp_commit(bar); else umma_commit(bar); };
+            const uint64_t q_desc = umma_desc_sw128(smem_u32(q_s)), k_desc = umma_desc_sw128(smem_u32(k_s)), v_desc = umma_desc_sw128_mn(smem_u32(v_s), 16384u, 1024u);
             PcpItem s_it, nxt;
             uint32_t sc = 0;                                                   // tiles whose S has been issued
             int s_r = 0, s_j = 0;
-            bool s_more = pcp_item(p, ppg, 0, s_it);
+            bool s_more = pcp_item<CTAS>(p, grp, 0, s_it);
             int s_n = s_more ? __shfl_sync(0xffffffffu, s_it.n_kvt, 0) : 0;
             auto issue_s = [&] {
                 if (!s_more) return;
@@ -828,26 +855,28 @@ __global__ void __launch_bounds__(PcpCfg::THREADS, 1) prefill_attention_cluster_
                     const uint64_t a = q_desc + (uint64_t)((s_r & 1) * (Cfg::Q_BYTES >> 4)), b = k_desc + (uint64_t)(st * (Cfg::KV_BYTES >> 4));
                     const uint32_t d = tmem_base + (sc % Cfg::S_BUFS) * 128;
 #pragma unroll
-                    for (int ks = 0; ks < D / 16; ++ks)
-                        gp_umma(d, a + (uint64_t)(((ks >> 2) * Cfg::Q_HALF + (ks & 3) * 32) >> 4), b + (uint64_t)(((ks >> 2) * Cfg::K_HALF + (ks & 3) * 32) >> 4), idesc_s, ks > 0 ? 1u : 0u);
-                    gp_commit(&s_full[sc % 6]);
-                    gp_commit(&k_empty[st]);
-                    if (s_j + 1 == s_n) gp_commit(&q_empty[s_r & 1]);
+                    for (int ks = 0; ks < D / 16; ++ks) {
+                        const uint64_t ak = a + (uint64_t)(((ks >> 2) * Cfg::Q_HALF + (ks & 3) * 32) >> 4), bk = b + (uint64_t)(((ks >> 2) * Cfg::K_HALF + (ks & 3) * 32) >> 4);
+                        if (PAIR) gp_umma(d, ak, bk, idesc_s, ks > 0 ? 1u : 0u); else umma_bf16(d, ak, bk, idesc_s, ks > 0 ? 1u : 0u);
+                    }
+                    commit(&s_full[sc % 6]);
+                    commit(&k_empty[st]);
+                    if (s_j + 1 == s_n) commit(&q_empty[s_r & 1]);
                 }
                 __syncwarp();
                 ++sc;
                 if (++s_j == s_n) {
                     s_j = 0; ++s_r;
-                    s_more = pcp_item(p, ppg, s_r, s_it);
+                    s_more = pcp_item<CTAS>(p, grp, s_r, s_it);
                     s_n = s_more ? __shfl_sync(0xffffffffu, s_it.n_kvt, 0) : 0;
                 }
             };
             issue_s(); issue_s();
             uint32_t t = 0;
-            bool more = pcp_item(p, ppg, 0, it);
+            bool more = pcp_item<CTAS>(p, grp, 0, it);
             for (int r = 0; more; ++r, it = nxt) {
                 const int n_kvt = __shfl_sync(0xffffffffu, it.n_kvt, 0);
-                more = pcp_item(p, ppg, r + 1, nxt);                           // read now, needed an item later
+                more = pcp_item<CTAS>(p, grp, r + 1, nxt);                           // read now, needed an item later
                 for (int j = 0; j < n_kvt; ++j, ++t) {
                     issue_s();                                                 // over the P of tile t - 1, whose product is ahead of it
                     const uint32_t st = t % STAGES;
@@ -859,9 +888,12 @@ __global__ void __launch_bounds__(PcpCfg::THREADS, 1) prefill_attention_cluster_
                         const uint64_t b = v_desc + (uint64_t)(st * (Cfg::KV_BYTES >> 4));
                         const uint32_t a = tmem_base + (t % Cfg::S_BUFS) * 128;
 #pragma unroll
-                        for (int ks = 0; ks < KV_TILE / 16; ++ks) gp_umma_ta(tmem_base + Cfg::O_COL, a + ks * 8, b + (uint64_t)(ks * (2048 >> 4)), idesc_o, (j | ks) != 0 ? 1u : 0u);
-                        gp_commit(&v_empty[st]);
-                        if (j + 1 == n_kvt) gp_commit(o_full);
+                        for (int ks = 0; ks < KV_TILE / 16; ++ks) {
+                            if (PAIR) gp_umma_ta(tmem_base + Cfg::O_COL, a + ks * 8, b + (uint64_t)(ks * (2048 >> 4)), idesc_o, (j | ks) != 0 ? 1u : 0u);
+                            else umma_bf16_ta(tmem_base + Cfg::O_COL, a + ks * 8, b + (uint64_t)(ks * (2048 >> 4)), idesc_o, (j | ks) != 0 ? 1u : 0u);
+                        }
+                        commit(&v_empty[st]);
+                        if (j + 1 == n_kvt) commit(o_full);
                     }
                     __syncwarp();
                 }
@@ -879,10 +911,10 @@ __global__ void __launch_bounds__(PcpCfg::THREADS, 1) prefill_attention_cluster_
             mbar_wait(&r_full[(w ^ 1) * 4 + q], ((t - 1) >> 1) & 1);
             return ref_s[(w ^ 1) * 128 + row];
         };
-        bool more = pcp_item(p, ppg, 0, it);
+        bool more = pcp_item<CTAS>(p, grp, 0, it);
         for (int r = 0; more; ++r) {
             const int n_kvt = it.n_kvt, pos0 = it.tile.pos0, qpos = pos0 + row;
-            more = pcp_item(p, ppg, r + 1, it);                     // read now, needed an item later
+            more = pcp_item<CTAS>(p, grp, r + 1, it);                     // read now, needed an item later
             float m_own = -INFINITY, l_lo = 0.f, l_hi = 0.f;        // this warpgroup's row sums, relative to 2^m_own
             for (int j = 0; j < n_kvt; ++j, ++t) {
                 if ((int)(t & 1) != w) continue;
@@ -950,7 +982,7 @@ __global__ void __launch_bounds__(PcpCfg::THREADS, 1) prefill_attention_cluster_
                 tmem_st_wait();
                 tcgen05_fence_before();
                 __syncwarp();
-                if (lane == 0) gp_arrive_tmem(gp_mapa(&p_full[t % Cfg::S_BUFS], 0));
+                if (lane == 0) arrive_even(&p_full[t % Cfg::S_BUFS]);
                 const float f = sum_rescale(m_own, m_ref);
                 l_lo = sum_add(l_lo, f, sum[0]); l_hi = sum_add(l_hi, f, sum[1]); m_own = m_ref;
             }
@@ -969,11 +1001,11 @@ __global__ void __launch_bounds__(PcpCfg::THREADS, 1) prefill_attention_cluster_
         uint8_t* stage = out_s + q * Cfg::OUT_WARP_BYTES;
         const uint32_t o_addr = tmem_base + ((uint32_t)(q * 32) << 16) + Cfg::O_COL;
         griddep_wait();                                             // the output may still be read by a predecessor
-        bool more = pcp_item(p, ppg, 0, it);
+        bool more = pcp_item<CTAS>(p, grp, 0, it);
         for (int r = 0; more; ++r) {
             const int rows_here = it.tile.n_rows - q * 32;          // of this warp's 32
             uint16_t* orow = reinterpret_cast<uint16_t*>(p.out) + (size_t)(it.tile.q_row0 + q * 32) * p.n_heads * D + (size_t)(it.head0 + (int)rank) * D;
-            more = pcp_item(p, ppg, r + 1, it);
+            more = pcp_item<CTAS>(p, grp, r + 1, it);
             mbar_wait(l_full, (uint32_t)r & 1);
             const float inv = 1.0f / (sum_s[row] + sum_s[128 + row]);
             __syncwarp();
@@ -997,7 +1029,7 @@ __global__ void __launch_bounds__(PcpCfg::THREADS, 1) prefill_attention_cluster_
             }
             tcgen05_fence_before();
             __syncwarp();
-            if (lane == 0) gp_arrive_tmem(gp_mapa(o_empty, 0));
+            if (lane == 0) arrive_even(o_empty);
 #pragma unroll 4
             for (int i = 0; i < 32; i += ROWS_AT_ONCE) {
                 const int rr = i + lane / CH, ch = lane % CH;
@@ -1009,23 +1041,27 @@ __global__ void __launch_bounds__(PcpCfg::THREADS, 1) prefill_attention_cluster_
     }
     tcgen05_fence_before();
     __syncthreads();
-    gp_cluster_sync();                               // nothing of the pair may still arrive on, read from or allocate in a CTA that has gone
+    if (PAIR) gp_cluster_sync();                     // nothing of the pair may still arrive on, read from or allocate in a CTA that has gone
     if (warp == 1) {
         tcgen05_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");
+        if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");
+        else tmem_dealloc<512>(tmem_base);
     }
 }
 
-static cudaError_t launch_pcp(const CUtensorMap* tm_q, const CUtensorMap* tm_kv, const KvLayout& kv, const PrefillAttnParams& p, int items, int sms, cudaStream_t s) {
-    auto kern = prefill_attention_cluster_kernel;
+template <int D, int CTAS>
+static cudaError_t launch_pcp(const CUtensorMap* tm_q, const CUtensorMap* tm_kv, const KvLayout& kv, const PrefillAttnParams& p, int sms, cudaStream_t s) {
+    using Cfg = PcpCfg<D, CTAS>;
+    auto kern = prefill_attention_turns_kernel<D, CTAS>;
     static bool attr_done[16] = {};
-    { cudaError_t e = ensure_dynamic_smem(kern, PcpCfg::SMEM_BYTES, attr_done); if (e != cudaSuccess) return e; }
+    { cudaError_t e = ensure_dynamic_smem(kern, Cfg::SMEM_BYTES, attr_done); if (e != cudaSuccess) return e; }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * std::min(items, sms / 2)); cfg.blockDim = dim3(PcpCfg::THREADS); cfg.dynamicSmemBytes = PcpCfg::SMEM_BYTES; cfg.stream = s;
+    cfg.gridDim = dim3(CTAS * std::min(p.n_tiles * (p.n_heads / CTAS), sms / CTAS)); cfg.blockDim = dim3(Cfg::THREADS); cfg.dynamicSmemBytes = Cfg::SMEM_BYTES; cfg.stream = s;
     cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension; attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr; cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    int n_attr = 0;
+    if (CTAS > 1) { attr[n_attr].id = cudaLaunchAttributeClusterDimension; attr[n_attr].val.clusterDim.x = CTAS; attr[n_attr].val.clusterDim.y = 1; attr[n_attr++].val.clusterDim.z = 1; }
+    if (pdl_enabled()) { attr[n_attr].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[n_attr++].val.programmaticStreamSerializationAllowed = 1; }
+    cfg.attrs = attr; cfg.numAttrs = n_attr;
     count_launch();
     return cudaLaunchKernelEx(&cfg, kern, *tm_q, *tm_kv, p, (int64_t)p.layer * kv.layer_stride_rows, kv.kv_stride_rows);
 }
@@ -1053,25 +1089,27 @@ static int prefill_sm_count() {
     return n;
 }
 
-// Which of the three.  us, kernels alone, 32 and 64 heads over 8, 145 batches of 1 to 32 prompts of 100 to 1400 rows behind 0 to 3000 cached ones: with n tiles of
-// 128 keys for the longest item, one head a CTA takes 4.9 + 1.0 n while all its CTAs are resident (up to half as many items of two heads as SMs; one query tile
-// of 100 rows: n = 1 5.8, 4 8.9, 11 15.9, 25 29.9); two heads a CTA 6.3 + 2.6 for each further round over the SMs + 1.72 a tile on the longest CTA (96 items of
-// 1, 4, 11 and 25 tiles: 8.0, 13.3, 25.6, 49.2; 1024 of 1: 32.1); a CTA pair 7.1 + 1.25 for each further round over the pairs + 0.77 a tile (7.5, 9.9, 14.6, 24.7 for
-// the first, 10.0, 15.0, 25.6, 47.2 and 33.8 for the second).  Ragged items: the longest CTA has the longest item at least, else the mean one a round.  The least
-// estimate was within 2 % of the fastest kernel for all but 3 batches (5 %).  A pair's two CTAs take the two heads of an item, so groups with an odd head stay on
-// the other two, and so do heads of 64 (a product of 64 columns would leave each CTA 32 of V's).
+// Which of them.  us, kernels alone, 32 to 64 heads over 8, 211 batches of 1 to 32 prompts of 30 to 4000 rows behind 0 to 3000 cached ones, fitted with n tiles of
+// 128 keys for the longest item and r rounds over the SMs or pairs: one head a CTA 4.9 + 1.0 n (heads of 64: 4.2 + 1.0 n) while all its CTAs are resident, up to half
+// as many items of two heads as SMs; two heads a CTA 6.3 + 2.6 (r - 1) + 1.72 a tile on the longest CTA (5.4 + 1.9 (r - 1) + 1.72); in turns on a pair
+// 7.1 + 1.25 (r - 1) + 0.77 a tile, on a CTA 4.9 + 0.7 (r - 1) + 0.77.  Heads of 128, n = 1, 4, 11, 25: one query tile of 100 rows 5.8, 8.9, 15.9, 29.9 one head a CTA,
+// 7.5, 9.9, 14.6, 24.7 in turns; nine of them 8.6, 14.3, 26.8, 52.1 two heads a CTA, 10.4, 15.6, 26.5, 49.6.  Heads of 64, n = 1, 6, 25: one tile 5.2, 10.2, 29.9 against
+// 5.4, 9.1, 22.7, nine 7.1, 16.0, 48.2 against 7.6, 15.4, 44.5.  Ragged items: the longest CTA has the longest item at least, else the mean one a round.  The least
+// estimate was within 2 % of the fastest kernel for all but a few batches of single tiles (5 %).  A pair takes two heads of a group, so groups of 128 with an odd
+// head stay on the first two (in turns on a CTA alone they meet the L2's limit: five prompts of 1.4 thousand rows, 40 / 8 heads 126 -> 171).
 PrefillKernel prefill_attention_kernel_of(int n_tiles, int key_tiles, int max_key_tiles, int n_heads, int n_kv, int head_dim) {
     const int sms = prefill_sm_count(), grp = n_heads / n_kv, items = n_tiles * n_kv * ((grp + 1) / 2);
-    const bool few = items <= sms / 2, pairs_ok = head_dim == 128 && grp % 2 == 0 && sms >= 2 && key_tiles > 0;
-    // (few items of any kind and ungrouped heads: 400 rows behind 6000, 32 / 8 heads, 64 items: one head a CTA 58 us, two 91)
-    const PrefillKernel plain = grp > 1 && !few ? PREFILL_TWO_HEADS : PREFILL_ONE_HEAD;
-    if (!pairs_ok) return plain;
+    const bool few = items <= sms / 2, small = head_dim == 64, turns_ok = key_tiles > 0 && (small || (head_dim == 128 && grp % 2 == 0 && sms >= 2));
+    // (few items of any kind: 400 rows behind 6000, 32 / 8 heads, 64 items: one head a CTA 58 us, two 91)
+    const PrefillKernel plain = grp > 1 && !few ? PREFILL_TWO_HEADS : PREFILL_ONE_HEAD, turns = small ? PREFILL_TURNS : PREFILL_TURNS_PAIR;
+    if (!turns_ok) return plain;
+    if (grp == 1 && !few) return turns;                     // one head a CTA is for items that are all resident
     const double mean = (double)key_tiles / n_tiles, longest = max_key_tiles;
-    auto rounds = [&](int ctas) { return (items + ctas - 1) / ctas; };
-    const int r_sm = rounds(sms), r_pair = rounds(sms / 2);
-    const double us_plain = few ? 4.9 + 1.0 * longest : 6.3 + 2.6 * (r_sm - 1) + 1.72 * std::max(longest, mean * r_sm);
-    const double us_pair = 7.1 + 1.25 * (r_pair - 1) + 0.77 * std::max(longest, mean * r_pair);
-    return us_pair < us_plain ? PREFILL_CTA_PAIR : plain;
+    const int turn_items = small ? n_tiles * n_heads : items, turn_ctas = small ? sms : sms / 2;
+    const int r_plain = (items + sms - 1) / sms, r_turns = (turn_items + turn_ctas - 1) / turn_ctas;
+    const double us_plain = few ? (small ? 4.2 : 4.9) + 1.0 * longest : (small ? 5.4 + 1.9 * (r_plain - 1) : 6.3 + 2.6 * (r_plain - 1)) + 1.72 * std::max(longest, mean * r_plain);
+    const double us_turns = (small ? 4.9 + 0.7 * (r_turns - 1) : 7.1 + 1.25 * (r_turns - 1)) + 0.77 * std::max(longest, mean * r_turns);
+    return us_turns < us_plain ? turns : plain;
 }
 
 cudaError_t launch_prefill_attention_tc(const CUtensorMap* tm_q, const CUtensorMap* tm_kv, const KvLayout& kv, const PrefillAttnParams& p, cudaStream_t s) {
@@ -1079,7 +1117,8 @@ cudaError_t launch_prefill_attention_tc(const CUtensorMap* tm_q, const CUtensorM
     if (kv.page_size != 64 || p.n_heads % p.n_kv != 0) return cudaErrorInvalidValue;
     const int grp = p.n_heads / p.n_kv, items = p.n_tiles * p.n_kv * ((grp + 1) / 2), sms = prefill_sm_count();
     const PrefillKernel k = prefill_attention_kernel_of(p.n_tiles, p.key_tiles, p.max_key_tiles, p.n_heads, p.n_kv, kv.head_dim);
-    if (k == PREFILL_CTA_PAIR) return launch_pcp(tm_q, tm_kv, kv, p, items, sms, s);
+    if (k == PREFILL_TURNS_PAIR) return launch_pcp<128, 2>(tm_q, tm_kv, kv, p, sms, s);
+    if (k == PREFILL_TURNS) return launch_pcp<64, 1>(tm_q, tm_kv, kv, p, sms, s);
     if (k == PREFILL_TWO_HEADS) {
         if (kv.head_dim == 128) return launch_ptp<128>(tm_q, tm_kv, kv, p, items, sms, s);
         if (kv.head_dim == 64) return launch_ptp<64>(tm_q, tm_kv, kv, p, items, sms, s);

@@ -191,7 +191,7 @@ inline void set_key_tiles(PrefillAttnParams& p, const PrefillTile* host_tiles, s
         p.key_tiles += k; if (k > p.max_key_tiles) p.max_key_tiles = k;
     }
 }
-enum PrefillKernel : int { PREFILL_ONE_HEAD = 1, PREFILL_TWO_HEADS = 2, PREFILL_CTA_PAIR = 3 };      // the same bits in all three
+enum PrefillKernel : int { PREFILL_ONE_HEAD = 1, PREFILL_TWO_HEADS = 2, PREFILL_TURNS_PAIR = 3, PREFILL_TURNS = 4 };      // the same bits in all of them
 PrefillKernel prefill_attention_kernel_of(int n_tiles, int key_tiles, int max_key_tiles, int n_heads, int n_kv, int head_dim);
 cudaError_t launch_prefill_attention(const CUtensorMap* tm_kv, const KvLayout& kv, const PrefillAttnParams& p, cudaStream_t s);   // legacy mma.sync path
 // tcgen05 path (attention_prefill_tc.cu): tm_q = box {64 cols, 128 rows} over q[T, nh*D]

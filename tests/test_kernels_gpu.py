@@ -342,13 +342,13 @@ def test_paged_prefill_attention_two_heads_per_cta(L, nh, nkv, D):
     assert err < 2 * 5 * 2.0 ** -8, err
 
 
-# one head a CTA, two heads a CTA, two heads a CTA pair: a batch takes the kernel that the estimate of its time names, and a row's bits are the same in all.
+# one head a CTA, two heads a CTA, key tiles in turns on a CTA pair (heads of 128) or a CTA (heads of 64): a batch takes the kernel that the estimate of its time names, and a row's bits are the same in all.
 # Items of one, two, three and many key tiles (the pair's warpgroups take them in turn: odd and even ends, items shorter than what is on its way), a last tile
 # without its second page, more items than CTAs, references raised in later tiles
-@pytest.mark.parametrize("nh,nkv", [(8, 4), (16, 2)])
+@pytest.mark.parametrize("nh,nkv,D", [(8, 4, 128), (16, 2, 128), (12, 4, 64), (16, 2, 64)])
 @pytest.mark.parametrize("ctx,rows", [(2, 2), (64, 64), (128, 128), (129, 129), (256, 255), (384, 130), (449, 33), (1000, 130), (1280, 65)])
-def test_prefill_attention_kernels_agree(L, nh, nkv, ctx, rows):
-    D, pages = 128, (ctx + 63) // 64
+def test_prefill_attention_kernels_agree(L, nh, nkv, D, ctx, rows):
+    pages = (ctx + 63) // 64
     kv = _mk_cache(pages, nkv, D, 5)
     g = torch.Generator(device="cpu").manual_seed(ctx)
     q1 = torch.randn(rows, nh, D, generator=g)
@@ -365,7 +365,7 @@ def test_prefill_attention_kernels_agree(L, nh, nkv, ctx, rows):
     first = {}
     for copies in [1, 3, 5, 9, 17, 33, 50, 75, 101, 160, 300]:
         first.setdefault(kernel(copies), copies)
-    assert 3 in first and len(first) >= 2
+    assert (3 if D == 128 else 4) in first and len(first) >= (2 if D == 128 else 1)
     outs = []
     for copies in first.values():
         q = q1.repeat(copies, 1, 1).contiguous()
