@@ -34,7 +34,7 @@ SYMBOLS = [
     "oa_tokens_submit", "oa_count_tokens", "oa_apply_chat_template", "oa_last_error", "oa_engine_stats", "oa_model_info",
     "oa_debug_prefill_logits", "oa_bench_decode", "oa_k_rmsnorm", "oa_k_gemm", "oa_k_init_weight", "oa_k_paged_attention",
     "oa_kernel_launches", "oa_version", "oa_host_apply_chat_template", "oa_host_decode_plan", "oa_host_decode_attention_plan", "oa_host_streamk_plan", "oa_host_bpe_encode", "oa_host_bpe_decode", "oa_host_model_info",
-    "oa_k_gemm_streamk", "oa_k_hybrid_gemm", "oa_k_gemm_ext", "oa_host_gemm_kernel", "oa_host_gemm_pair_width", "oa_host_prefill_attention_kernel", "oa_debug_kernel_times", "oa_engine_serve", "oa_host_grammar_step", "oa_host_grammar_step_ex", "oa_host_grammar_token_mask", "oa_http_start", "oa_http_port", "oa_http_stats", "oa_http_stop", "oa_http_last_error", "oa_host_json_roundtrip", "oa_chat_cancel", "oa_chat_submit_ex", "oa_chat_wait_ex", "oa_trace_step",
+    "oa_k_gemm_streamk", "oa_k_hybrid_gemm", "oa_k_gemm_ext", "oa_host_gemm_kernel", "oa_host_gemm_pair_width", "oa_host_gemm_pair_swapped", "oa_host_prefill_attention_kernel", "oa_debug_kernel_times", "oa_engine_serve", "oa_host_grammar_step", "oa_host_grammar_step_ex", "oa_host_grammar_token_mask", "oa_http_start", "oa_http_port", "oa_http_stats", "oa_http_stop", "oa_http_last_error", "oa_host_json_roundtrip", "oa_chat_cancel", "oa_chat_submit_ex", "oa_chat_wait_ex", "oa_trace_step",
 ]
 
 _lib = None
@@ -73,6 +73,7 @@ def load() -> C.CDLL:
     L.oa_k_gemm_ext.argtypes = [vp, vp, i32, i32, i32, i32, i32, vp, vp, i32, i32, i32, f32, i32, vp]; L.oa_k_gemm_ext.restype = C.c_int
     L.oa_host_gemm_kernel.argtypes = [i32] * 7; L.oa_host_gemm_kernel.restype = C.c_int
     L.oa_host_prefill_attention_kernel.argtypes = [vp, vp, i32, i32, i32, i32]; L.oa_host_prefill_attention_kernel.restype = C.c_int
+    L.oa_host_gemm_pair_swapped.argtypes = [i32] * 5; L.oa_host_gemm_pair_swapped.restype = C.c_int
     L.oa_host_gemm_pair_width.argtypes = [i32] * 5; L.oa_host_gemm_pair_width.restype = C.c_int
     L.oa_k_hybrid_gemm.argtypes = [i32, vp, i32, vp, i32, vp, i32, i32, i32, i32, f32, i32, C.c_int64, C.c_int64, C.c_int64, vp]; L.oa_k_hybrid_gemm.restype = C.c_int
     L.oa_k_gemm_streamk.argtypes = [vp, vp, i32, i32, i32, i32, i32, vp, vp]; L.oa_k_gemm_streamk.restype = C.c_int

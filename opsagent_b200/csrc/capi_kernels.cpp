@@ -141,7 +141,7 @@ int oa_k_gemm(const void* A, const void* B, int32_t M, int32_t N, int32_t K, int
     GemmParams p{}; p.M = M; p.N = N; p.K = K; p.out = out; p.ldo = epilogue == EPI_SWIGLU ? N / 2 : N;
     p.bias = bias; p.resid = resid; p.ldr = N; p.logits = logits; p.ldl = N;
     if (epilogue == EPI_LOGITS) block_n = gemm_logits_bn(M, N, block_n);
-    p.few_rows_ok = 1;
+    p.few_rows_ok = p.swap_ok = 1;
     const GemmChoice choice = gemm_choice(p, epilogue, block_n);
     if (make_tmap_bf16_2d(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)K, (uint32_t)choice.a_box, 64) != 0) return OA_ERR_INTERNAL;
     if (make_tmap_bf16_2d(&tmB, B, (uint64_t)N, (uint64_t)K, (uint64_t)K, (uint32_t)choice.b_box, 64) != 0) return OA_ERR_INTERNAL;
@@ -169,7 +169,7 @@ int oa_k_gemm_ext(const void* A, const void* B, int32_t M, int32_t N, int32_t K,
     if (epilogue != EPI_STORE && epilogue != EPI_SWIGLU && epilogue != EPI_F32) return OA_ERR_BAD_REQUEST;
     if (act < 0 || act > 3 || (epilogue == EPI_F32 && act != 0) || (epilogue == EPI_SWIGLU && act != 0 && act != 2)) return OA_ERR_BAD_REQUEST;
     CUtensorMap tmA, tmB;
-    GemmParams p{}; p.M = M; p.N = N; p.K = K; p.few_rows_ok = 1;
+    GemmParams p{}; p.M = M; p.N = N; p.K = K; p.few_rows_ok = p.swap_ok = 1;
     if (epilogue == EPI_F32) { p.f32_out = (float*)out; p.ldf = N; p.bias_f32 = (const float*)bias; p.alpha = alpha; p.f32_accumulate = accumulate; }
     else { p.out = out; p.ldo = epilogue == EPI_SWIGLU ? N / 2 : N; p.bias = epilogue == EPI_STORE ? bias : nullptr; }
     if (epilogue == EPI_STORE) { p.store_act = act; p.act_col0 = act_col0; p.act_col1 = act_col1; } else p.glu_gelu = act == 2;
@@ -201,6 +201,12 @@ int oa_host_prefill_attention_kernel(const int32_t* ctx_lens, const int32_t* q_l
             ++n_tiles; sum += k; longest = std::max(longest, k);
         }
     return (int)prefill_attention_kernel_of(n_tiles, sum, longest, n_heads, n_kv, head_dim);
+}
+
+int oa_host_gemm_pair_swapped(int32_t M, int32_t N, int32_t K, int32_t epilogue, int32_t block_n) {
+    GemmParams p{}; p.M = M; p.N = N; p.K = K; p.few_rows_ok = p.swap_ok = 1;
+    const GemmChoice c = gemm_choice(p, epilogue, block_n);
+    return c.kernel == GEMM_PAIR && c.swapped ? c.width : 0;
 }
 
 static int paged_attention(const void* q, void* out, const void* kv_cache, int32_t num_pages, const int32_t* block_tables,

@@ -24,34 +24,41 @@ OA_DEVINL void raster_tile(int idx, int m_tiles, int n_tiles, int& m_blk, int& n
 }
 
 // One warp: rows row_base .. row_base + 31 (TMEM lanes of `acc`), columns n0 .. n0 + bn - 1 of the product.  glu_sc: scales of the two rows this
-// lane stores in a clamped gated activation.
-template <int EPI, bool CLAMPED = true>      // CLAMPED: the product may ask for the clamped gated activation (only grouped ones do)
-OA_DEVINL void persist_epilogue(const GemmParams& p, float* stage, uint32_t acc, int row_base, int n0, int bn, int lane, const float (&glu_sc)[2]) {
+// lane stores in a clamped gated activation.  SWAPPED: the lanes are columns n0 .. n0 + 31 and the accumulator's columns rows row_base .. row_base + bn - 1: a
+// chunk is turned on its way through shared memory and goes on as the other form's.
+template <int EPI, bool CLAMPED = true, bool SWAPPED = false>      // CLAMPED: the product may ask for the clamped gated activation (only grouped ones do)
+OA_DEVINL void persist_epilogue(const GemmParams& p, float* stage, uint32_t acc, int row_start, int n0, int bn, int lane, const float (&glu_sc)[2]) {
     // residual of the columns at hand and, on their way meanwhile, of the next ones (each lane reads and writes its own places: out may be resid)
     uint4 res[4], res_next[4];
     auto load_res = [&](int cc, uint4 (&rr)[4]) {
 #pragma unroll
         for (int i4 = 0; i4 < 4; ++i4) {
-            const int row = row_base + i4 * 8 + (lane >> 2), col = n0 + cc + (lane & 3) * 8;
+            const int row = row_start + (SWAPPED ? cc : 0) + i4 * 8 + (lane >> 2), col = n0 + (SWAPPED ? 0 : cc) + (lane & 3) * 8;
             if (row < p.M && col < p.N) rr[i4] = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.resid) + (size_t)row * p.ldr + col);
         }
     };
     if (EPI == EPI_RESID) load_res(0, res_next);
 #pragma unroll 1
     for (int cc = 0; cc < bn; cc += 32) {
+        const int col0 = n0 + (SWAPPED ? 0 : cc), row_base = row_start + (SWAPPED ? cc : 0);
+        if (SWAPPED && row_base >= p.M) break;
         uint32_t v[32];
         tmem_ld_32x32b_x32(acc + (uint32_t)cc, v);
         tmem_ld_wait();
-        const int col0 = n0 + cc;
         if (EPI == EPI_RESID) {
 #pragma unroll
             for (int i4 = 0; i4 < 4; ++i4) res[i4] = res_next[i4];
             if (cc + 32 < bn) load_res(cc + 32, res_next);
         }
+        if (SWAPPED) {
 #pragma unroll
-        for (int j = 0; j < 32; j += 4)
-            *reinterpret_cast<float4*>(stage + lane * EPI_ROW_FLOATS + j) =
-                make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
+            for (int j = 0; j < 32; ++j) stage[j * EPI_ROW_FLOATS + lane] = __uint_as_float(v[j]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 32; j += 4)
+                *reinterpret_cast<float4*>(stage + lane * EPI_ROW_FLOATS + j) =
+                    make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
+        }
         __syncwarp();
         if (EPI == EPI_SWIGLU) {
             // chunk = 16 gate + 16 up columns -> 16 output features; lane = (row, 8-feature half)

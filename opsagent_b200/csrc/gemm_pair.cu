@@ -30,8 +30,9 @@ static int gp_smem_bytes(const PairRing& r) { return r.stages * gp_stage_bytes(r
 static PairRing gp_ring(int bn) { return PairRing{bn, std::min(GP_MAX_STAGES, (232448 - 4 * EPI_WARP_BYTES - GP_BAR_BYTES) / gp_stage_bytes(bn))}; }
 static constexpr int GP_GROUP_M = RASTER_GROUP_M / 2;           // a band of row tiles whose A rows stay in L2
 
-template <int EPI>
-__global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+// SWAPPED: the weights' rows are the 256 of a tile (operand U) and the tokens its bn (operand V); else the other way round
+template <int EPI, bool SWAPPED>
+__global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_constant__ CUtensorMap tmU, const __grid_constant__ CUtensorMap tmV,
                                                                   const GemmParams p, const PairRing ring) {
     const int BN = ring.bn, STAGES = ring.stages, STAGE_BYTES = GP_A_BYTES + BN * GP_BK;
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -44,11 +45,11 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
 
     const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // warp: uniform, and known to be
     const uint32_t rank = gp_rank();
-    const int n_tiles = (p.N + BN - 1) / BN, m_tiles = (p.M + 255) / 256, tiles = n_tiles * m_tiles;
+    const int v_tiles = ((SWAPPED ? p.M : p.N) + BN - 1) / BN, u_tiles = ((SWAPPED ? p.N : p.M) + 255) / 256, tiles = v_tiles * u_tiles;
     const int num_kb = (p.K + GP_BK - 1) / GP_BK, pair = (int)blockIdx.x >> 1, pairs = (int)gridDim.x >> 1;
 
     if (warp == 0 && lane == 0) {
-        tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmB);
+        tma_prefetch_desc(&tmU); tma_prefetch_desc(&tmV);
         for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
         for (int s = 0; s < 2; ++s) { mbar_init(&acc_full[s], 1); mbar_init(&acc_empty[s], 8); }
         fence_barrier_init();
@@ -68,16 +69,16 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
         griddep_wait();
         int s = 0; uint32_t ph = 0;
         for (int t = pair; t < tiles; t += pairs) {
-            int m_blk, n_blk; raster_tile(t, m_tiles, n_tiles, m_blk, n_blk, GP_GROUP_M);
-            const int a_row = m_blk * 256 + (int)rank * 128, b_row = n_blk * BN + (int)rank * (BN / 2);
+            int u_blk, v_blk; raster_tile(t, u_tiles, v_tiles, u_blk, v_blk, GP_GROUP_M);
+            const int u_row = u_blk * 256 + (int)rank * 128, v_row = v_blk * BN + (int)rank * (BN / 2);
             for (int kb = 0; kb < num_kb; ++kb) {
                 gp_wait(&empty_bar[s], ph ^ 1);
                 if (elect_one()) {
                     uint8_t* dst = smem + s * STAGE_BYTES;
-                    if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * STAGE_BYTES);      // both CTAs' A rows and B halves
+                    if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * STAGE_BYTES);      // both CTAs' rows of U and halves of V
                     const uint32_t bar = gp_mapa(&full_bar[s], 0);
-                    gp_tma_load(dst, &tmA, bar, kb * GP_BK, a_row, kEvictNormal);
-                    gp_tma_load(dst + GP_A_BYTES, &tmB, bar, kb * GP_BK, b_row, kEvictNormal);
+                    gp_tma_load(dst, &tmU, bar, kb * GP_BK, u_row, kEvictNormal);
+                    gp_tma_load(dst + GP_A_BYTES, &tmV, bar, kb * GP_BK, v_row, kEvictNormal);
                 }
                 __syncwarp();
                 if (++s == STAGES) { s = 0; ph ^= 1; }
@@ -120,12 +121,13 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
         griddep_wait();
         int it = 0;
         for (int t = pair; t < tiles; t += pairs, ++it) {
-            int m_blk, n_blk; raster_tile(t, m_tiles, n_tiles, m_blk, n_blk, GP_GROUP_M);
-            const int as = it & 1, row_base = m_blk * 256 + (int)rank * 128 + q * 32;
+            int u_blk, v_blk; raster_tile(t, u_tiles, v_tiles, u_blk, v_blk, GP_GROUP_M);
+            const int as = it & 1, u_base = u_blk * 256 + (int)rank * 128 + q * 32;
             const uint32_t acc = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * GP_ACC_COLS);
             gp_wait(&acc_full[as], ((uint32_t)it >> 1) & 1);
             tcgen05_fence_after();
-            if (row_base < p.M) persist_epilogue<EPI, false>(p, stage, acc, row_base, n_blk * BN, BN, lane, no_scale);
+            if (SWAPPED) { if (u_base < p.N) persist_epilogue<EPI, false, true>(p, stage, acc, v_blk * BN, u_base, BN, lane, no_scale); }
+            else if (u_base < p.M) persist_epilogue<EPI, false, false>(p, stage, acc, u_base, v_blk * BN, BN, lane, no_scale);
             tcgen05_fence_before();
             __syncwarp();
             if (lane == 0) gp_arrive_remote(gp_mapa(&acc_empty[as], 0));
@@ -140,12 +142,12 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
     }
 }
 
-template <int EPI>
-static cudaError_t launch_gp(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, const PairRing& ring, int sms, cudaStream_t stream) {
-    auto kern = gemm_pair_kernel<EPI>;
+template <int EPI, bool SWAPPED>
+static cudaError_t launch_gp(const CUtensorMap* tmU, const CUtensorMap* tmV, const GemmParams& p, const PairRing& ring, int sms, cudaStream_t stream) {
+    auto kern = gemm_pair_kernel<EPI, SWAPPED>;
     static bool attr_done[16] = {};
     { cudaError_t e = ensure_dynamic_smem(kern, 227 * 1024, attr_done); if (e != cudaSuccess) return e; }
-    const int tiles = ((p.N + ring.bn - 1) / ring.bn) * ((p.M + 255) / 256);
+    const int tiles = SWAPPED ? ((p.M + ring.bn - 1) / ring.bn) * ((p.N + 255) / 256) : ((p.N + ring.bn - 1) / ring.bn) * ((p.M + 255) / 256);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * std::min(tiles, sms / 2)); cfg.blockDim = dim3(GP_THREADS); cfg.dynamicSmemBytes = gp_smem_bytes(ring); cfg.stream = stream;
     cudaLaunchAttribute attr[2];
@@ -153,17 +155,17 @@ static cudaError_t launch_gp(const CUtensorMap* tmA, const CUtensorMap* tmB, con
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr; cfg.numAttrs = pdl_enabled() ? 2 : 1;
     count_launch();
-    return cudaLaunchKernelEx(&cfg, kern, *tmA, *tmB, p, ring);
+    return cudaLaunchKernelEx(&cfg, kern, *tmU, *tmV, p, ring);
 }
 
-cudaError_t launch_gemm_pair(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epilogue, int bn, int sms, cudaStream_t stream) {
+cudaError_t launch_gemm_pair(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epilogue, int bn, bool swapped, int sms, cudaStream_t stream) {
     if (p.m_tile_group || p.glu_limit > 0.f || sms < 2 || bn < 128 || bn > 256 || bn % 32 != 0) return cudaErrorInvalidValue;
     const PairRing ring = gp_ring(bn);
     switch (epilogue) {
-        case EPI_STORE: return launch_gp<EPI_STORE>(tmA, tmB, p, ring, sms, stream);
-        case EPI_RESID: return launch_gp<EPI_RESID>(tmA, tmB, p, ring, sms, stream);
-        case EPI_SWIGLU: return launch_gp<EPI_SWIGLU>(tmA, tmB, p, ring, sms, stream);
-        case EPI_F32: return launch_gp<EPI_F32>(tmA, tmB, p, ring, sms, stream);
+        case EPI_STORE: return swapped ? launch_gp<EPI_STORE, true>(tmB, tmA, p, ring, sms, stream) : launch_gp<EPI_STORE, false>(tmA, tmB, p, ring, sms, stream);
+        case EPI_RESID: return swapped ? launch_gp<EPI_RESID, true>(tmB, tmA, p, ring, sms, stream) : launch_gp<EPI_RESID, false>(tmA, tmB, p, ring, sms, stream);
+        case EPI_SWIGLU: return swapped ? launch_gp<EPI_SWIGLU, true>(tmB, tmA, p, ring, sms, stream) : launch_gp<EPI_SWIGLU, false>(tmA, tmB, p, ring, sms, stream);
+        case EPI_F32: return swapped ? launch_gp<EPI_F32, true>(tmB, tmA, p, ring, sms, stream) : launch_gp<EPI_F32, false>(tmA, tmB, p, ring, sms, stream);
     }
     return cudaErrorInvalidValue;
 }

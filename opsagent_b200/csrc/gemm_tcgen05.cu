@@ -393,17 +393,33 @@ static cudaError_t launch_persistent(const CUtensorMap* tmA, const CUtensorMap* 
 // 76 71 67 62 57, 1334 x 5120 x 27648 363 347 401 372 412, 2029 x 7168 x 5120 132 126 128 123 132, 5968 x 28672 x 4096 1070 1077 1094 1110 1161.  A tile of one CTA:
 // 128 x 256 0.22 + 0.27 x busy (354 x 57344 x 8192: 353 us, three row tiles instead of two of 256 rows: 384 on pairs), 128 x 128 0.17 + 0.13 x busy, narrower
 // 0.15 + 0.07 x busy.  Up to 128 rows half of a pair's rows would be padding.  Every kernel sums k in the same order: the choice moves no bit.
-struct PairWidth { int bn; double us; };
+// Either operand's rows may be the 256 of a tile.  With the weights' there, tokens come in steps of 32 instead of 256: 1337 rows are 1344 or 1440, not 1536, 300 are
+// 320, not 512, and there are more ways to fill the last round.  The same estimate serves both; us in loops, tokens' rows the 256 -> weights': 1337 x 4096 x 14336
+// 126 -> 115, 300 x 28672 x 4096 83 -> 68, 300 x 7168 x 5120 36 -> 25, 1337 x 55296 x 5120 521 -> 480, 4000 x 4096 x 14336 337 -> 304; where it is the wrong way
+// 1024 x 28672 x 4096 155 -> 177, 1621 x 55296 x 5120 609 -> 646 (128 tokens instead of 256 columns: narrow tiles fetch more from L2 a product, which the estimate
+// leaves out).  So the weights' have to be 2.5 % better, 6 % where their tiles are the narrower ones, 7 % against tiles of one CTA; up to 512 rows and 100 MB of
+// weights equal estimates go to them (200 x 7168 x 5120 24.8 -> 23.6, 512 x 2048 x 2048 12.3 -> 10.6).  Over 162 products of 130 to 8192 rows of the four models 5.5 %
+// faster than without, 4 of them 3 to 10 % slower within what their neighbours of a few rows differ by.
+struct PairWidth { int bn; double us; bool swapped; };
 static long long ceil_div(long long a, long long b) { return (a + b - 1) / b; }
 static PairWidth gemm_pair_width(const GemmParams& p, int sms) {
     const long long pairs = sms / 2, kb = ceil_div(p.K, BLOCK_K);
-    PairWidth best{0, 0.0};
-    for (int bn = 256; bn >= 128; bn -= 32) {
-        const long long tiles = ceil_div(p.N, bn) * ceil_div(p.M, 256), rounds = ceil_div(tiles, pairs);
-        const double us = (double)(rounds * kb) * (bn / 256.0 * (0.28 + 0.14 * (double)tiles / (double)(rounds * pairs)) + 0.02) + 8.5;
-        if (!best.bn || us < best.us) best = PairWidth{bn, us};
-    }
-    return best;
+    auto least = [&](long long rows256, long long rows, bool swapped) {
+        PairWidth best{0, 0.0, swapped};
+        for (int bn = 256; bn >= 128; bn -= 32) {
+            const long long tiles = ceil_div(rows, bn) * ceil_div(rows256, 256), rounds = ceil_div(tiles, pairs);
+            const double us = (double)(rounds * kb) * (bn / 256.0 * (0.28 + 0.14 * (double)tiles / (double)(rounds * pairs)) + 0.02) + 8.5;
+            if (!best.bn || us < best.us) { best.bn = bn; best.us = us; }
+        }
+        return best;
+    };
+    const PairWidth plain = least(p.M, p.N, false);
+    if (!p.swap_ok) return plain;
+    PairWidth swapped = least(p.N, p.M, true);
+    const double line = p.M <= 512 && 2LL * p.N * p.K <= 100000000LL ? 1.0001 : swapped.bn < plain.bn ? 0.94 : 0.975;
+    if (swapped.us >= plain.us * line) return plain;
+    swapped.us = std::min(swapped.us * 1.07, plain.us);          // what one-CTA tiles have to beat
+    return swapped;
 }
 static GemmKernel kernel_of(const GemmParams& p, int epilogue, int block_n, PairWidth& pair) {
     if (block_n != 32 && block_n != 64 && block_n != 128 && block_n != 256) return GEMM_NONE;
@@ -431,9 +447,9 @@ static int few_width(int N, int sms) {
     return 128;
 }
 GemmChoice gemm_choice(const GemmParams& p, int epilogue, int block_n) {
-    PairWidth pair{256, 0.0};
+    PairWidth pair{256, 0.0, false};
     GemmChoice c{kernel_of(p, epilogue, block_n, pair), 128, block_n, block_n};
-    if (c.kernel == GEMM_PAIR) { c.width = pair.bn; c.b_box = pair.bn / 2; }
+    if (c.kernel == GEMM_PAIR) { c.width = pair.bn; c.swapped = pair.swapped; (c.swapped ? c.a_box : c.b_box) = pair.bn / 2; if (c.swapped) c.b_box = 128; }
     if (c.kernel == GEMM_FEW) { c.a_box = few_box(p.M); c.width = c.b_box = few_width(p.N, sm_count_cached()); }
     if (c.kernel == GEMM_HEAD && p.few_rows_ok && p.M <= FEW_MAX_ROWS) c.a_box = few_box(p.M);
     return c;
@@ -446,7 +462,7 @@ cudaError_t launch_gemm(const CUtensorMap* tmA, const CUtensorMap* tmB, const Ge
     switch (c.kernel) {
         case GEMM_NONE: return cudaErrorInvalidValue;
         case GEMM_HEAD: return launch_head(tmA, tmB, p, c.a_box, stream);
-        case GEMM_PAIR: return launch_gemm_pair(tmA, tmB, p, epilogue, c.width, sm_count_cached(), stream);
+        case GEMM_PAIR: return launch_gemm_pair(tmA, tmB, p, epilogue, c.width, c.swapped, sm_count_cached(), stream);
         case GEMM_PERSISTENT:      // the widest tile over many rows: the epilogue overlaps the next tile
             switch (epilogue) {
                 case EPI_STORE: return launch_persistent<EPI_STORE>(tmA, tmB, p, stream);

@@ -595,7 +595,7 @@ void HybridModel::gemm(int mode, const void* A, int lda, const Mat& B, void* C, 
     bool tc = B.tc && !f32_ && lda % 8 == 0 && aligned16(A) && lda >= B.ld;
     if (mode == HY_STORE) tc = tc && ldc % 8 == 0 && aligned16(C) && (!bias || (bias_act && aligned16(bias_act))) && alpha == 1.f;     // a bias in the activation type, padded to N rounded up to 8
     else tc = tc && B.N % 8 == 0 && ldc % 4 == 0 && aligned16(C) && (!bias || aligned16(bias)) && act.kind == 0;
-    GemmParams g{}; g.M = M; g.N = up8(B.N); g.K = B.ld; g.few_rows_ok = 1;
+    GemmParams g{}; g.M = M; g.N = up8(B.N); g.K = B.ld; g.few_rows_ok = g.swap_ok = 1;
     const int bn = pick_tile_n(M, g.N, sm_count), epi = mode == HY_STORE ? EPI_STORE : EPI_F32;
     const GemmChoice choice = gemm_choice(g, epi, bn);
     CUtensorMap tmA;
@@ -613,7 +613,7 @@ bool HybridModel::moe(const LayerW& w, const HyLayer& l, const void* h_in, const
     if (hc_.sequential) { out = y_; beta = 0.f; }        // the residual is closed by whoever opens the next sublayer
     const bool relu2 = m.act == HY_EXPERT_RELU2; const int rows1 = relu2 ? w.ffp : 2 * w.ffp;
     if (m.dense && m.act == HY_EXPERT_GELU_GLU) {        // gated: both halves in one product, gelu(gate) * up in its epilogue
-        GemmParams g{}; g.M = T; g.N = w.up.N; g.K = w.up.ld; g.out = act_; g.ldo = w.ffp; g.glu_gelu = 1; g.few_rows_ok = 1;
+        GemmParams g{}; g.M = T; g.N = w.up.N; g.K = w.up.ld; g.out = act_; g.ldo = w.ffp; g.glu_gelu = 1; g.few_rows_ok = g.swap_ok = 1;
         const int bn = pick_tile_n(T, g.N, sm_count);
         const GemmChoice choice = gemm_choice(g, EPI_SWIGLU, bn);
         CUtensorMap tmA;

@@ -41,23 +41,25 @@ struct GemmParams {
     // EPI_SWIGLU with glu_limit > 0: out = g sigmoid(glu_slope g) (u + 1), g = min(s gate, limit), u = clamp(s up, -limit, limit), where row r's s is
     // row_scale[row_scale_idx[r]] (0 for a negative index: a padding row of a grouped product) — the router's weight on an expert's input, exact in fp32
     float glu_limit, glu_slope; const float* row_scale; const int32_t* row_scale_idx;
-    int few_rows_ok;                // the caller's A map has the box gemm_choice() asks for (else 128 rows)
+    int few_rows_ok;                // the caller's A map has the box gemm_choice() asks for (else 128 rows): products of up to 64 rows
+    int swap_ok;                    // the same: tiles on CTA pairs with the operands' roles swapped (boxes of half their width)
     int glu_gelu;                   // EPI_SWIGLU: the gate passes the tanh form of GELU instead of SiLU
 };
 // which kernel launch_gemm runs for a product: a 128 x block_n tile per CTA (FEW: of up to 64 loaded rows), the persistent 128 x 256 tiles, CTA pairs, the
 // persistent vocabulary head; NONE: refused.  All sum k in ascending order in one accumulator: the choice moves no bit.
 enum GemmKernel : int { GEMM_NONE = -1, GEMM_TILE = 0, GEMM_FEW = 1, GEMM_PERSISTENT = 2, GEMM_PAIR = 3, GEMM_HEAD = 4 };
 // a_box, b_box: rows of the boxes of the tensor maps over A[M,K] and B[N,K] that the kernel reads ({64, a_box} and {64, b_box}); width: columns of its tiles
-struct GemmChoice { GemmKernel kernel; int a_box, b_box, width; };
+// swapped (PAIR): the weights' rows are the 256 of a tile and width counts its tokens
+struct GemmChoice { GemmKernel kernel; int a_box, b_box, width; bool swapped = false; };
 GemmChoice gemm_choice(const GemmParams& p, int epilogue, int block_n);
-// tmA: box {64, 128} over A[M,K] (few_rows_ok: {64, a_box}); tmB: box {64, b_box} over B[N,K].  block_n in {32,64,128,256}.  choice: gemm_choice of the very
+// tmA: box {64, 128} over A[M,K] (few_rows_ok, swap_ok: {64, a_box}); tmB: box {64, b_box} over B[N,K].  block_n in {32,64,128,256}.  choice: gemm_choice of the very
 // same arguments, where the caller has it
 cudaError_t launch_gemm(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epilogue, int block_n,
                         cudaStream_t stream, const GemmChoice* choice = nullptr);
 int gemm_n_tiles(int N, int block_n);
 int gemm_logits_bn(int M, int N, int block_n);      // EPI_LOGITS: the tile width to ask launch_gemm for (and to count the arg-max partials by) where block_n would do
-// CTA-pair kernel (gemm_pair.cu): tiles of 256 x bn, bn = 128, 160, .. 256; tmB: box {64, bn / 2}
-cudaError_t launch_gemm_pair(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epilogue, int bn, int sms, cudaStream_t stream);
+// CTA-pair kernel (gemm_pair.cu): tiles of 256 x bn, bn = 128, 160, .. 256; tmB: box {64, bn / 2}.  swapped: tiles of 256 columns x bn rows; tmA: box {64, bn / 2}, tmB: {64, 128}
+cudaError_t launch_gemm_pair(const CUtensorMap* tmA, const CUtensorMap* tmB, const GemmParams& p, int epilogue, int bn, bool swapped, int sms, cudaStream_t stream);
 // the box heights gemm_choice can ask for of B: a weight matrix keeps one map of each
 constexpr int GEMM_B_BOXES[] = {32, 64, 80, 96, 112, 128, 256}, GEMM_N_B_BOXES = 7;
 constexpr int gemm_b_box_index(int box) { int i = 0; while (i + 1 < GEMM_N_B_BOXES && GEMM_B_BOXES[i] != box) ++i; return i; }

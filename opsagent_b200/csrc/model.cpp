@@ -143,6 +143,7 @@ DeviceModel::DeviceModel(const ModelConfig& c, const EngineOptions& o) : ModelBa
     };
     amap(&tm_xn_, xn_, MR, H); amap(&tm_attn_, attn_, MR, qd); amap(&tm_act_, act_, MR, F); amap(&tm_q_, q_, MR, qd);
     for (int i = 0; i < 3; ++i) { amap(&tm_few_xn_[i], xn_, MR, H, 16 << i); amap(&tm_few_attn_[i], attn_, MR, qd, 16 << i); amap(&tm_few_act_[i], act_, MR, F, 16 << i); }
+    for (int i = 0; i < 3; ++i) { const int box = 80 + 16 * i; amap(&tm_swap_xn_[i], xn_, MR, H, box); amap(&tm_swap_attn_[i], attn_, MR, qd, box); amap(&tm_swap_act_[i], act_, MR, F, box); }
     cuda_check(cudaMemsetAsync(q_, 0, (size_t)MR * qd * 2, stream), "memset");
     // sampled rows (debug logits sample every row of a short prefill: up to 2048)
     const int MS = max_sample_;
@@ -603,9 +604,12 @@ void DeviceModel::forward(const StepInput& in, float* logits_out) {
                 cuda_check(launch_ar_resid_bf16(comm->d_peer_sym(b), tp, x_, T, H, stream), "allreduce+resid");
             }
         };
-        auto product = [&](const CUtensorMap* a, const WeightMat& w, const GemmParams& g, int epilogue, int bn) {
+        struct Maps { const CUtensorMap &full, (&few)[3], (&swap)[3]; };
+        const Maps xn{tm_xn_, tm_few_xn_, tm_swap_xn_}, attn{tm_attn_, tm_few_attn_, tm_swap_attn_}, actv{tm_act_, tm_few_act_, tm_swap_act_};
+        auto product = [&](const Maps& a, const WeightMat& w, GemmParams g, int epilogue, int bn) {
+            g.swap_ok = 1;
             const GemmChoice c = gemm_choice(g, epilogue, bn);
-            return launch_gemm(a, w.map(c.b_box), g, epilogue, bn, stream, &c);
+            return launch_gemm(c.a_box == 128 ? &a.full : c.a_box == 64 ? &a.few[2] : &a.swap[(c.a_box - 80) / 16], w.map(c.b_box), g, epilogue, bn, stream, &c);
         };
         const int bn_qkv = pick_bn(T, qkvd, opt.bn_qkv, false), bn_o = pick_bn(T, H, opt.bn_o, false);
         const int bn_gu = pick_bn(T, 2 * F, opt.bn_gu, true), bn_down = pick_bn(T, H, opt.bn_down, false);
@@ -613,31 +617,31 @@ void DeviceModel::forward(const StepInput& in, float* logits_out) {
             const Layer& ly = layers[l];
             cuda_check(launch_rmsnorm(x_, ly.ln1, xn_, T, H, cfg.rms_eps, stream), "rmsnorm1"); MARK(1);
             GemmParams g{}; g.M = T; g.N = qkvd; g.K = H; g.out = qkv_; g.ldo = qkvd; g.bias = ly.bqkv;
-            cuda_check(product(&tm_xn_, ly.qkv, g, EPI_STORE, bn_qkv), "qkv gemm"); MARK(2);
+            cuda_check(product(xn, ly.qkv, g, EPI_STORE, bn_qkv), "qkv gemm"); MARK(2);
             cuda_check(launch_rope_kv_write(qkv_, d_pos, d_slot, rope_cos, rope_sin, q_, kv, l, T, nh, stream), "rope"); MARK(3);
             attention(l);
             if (use_tp) {      // bf16 partial -> symmetric buffer, barrier, x += sum over ranks (rank order)
                 const int b = comm->next_buffer();
                 GemmParams go{}; go.M = T; go.N = H; go.K = qd; go.out = comm->sym(b); go.ldo = H;
-                cuda_check(product(&tm_attn_, ly.o, go, EPI_STORE, bn_o), "o gemm"); MARK(6);
+                cuda_check(product(attn, ly.o, go, EPI_STORE, bn_o), "o gemm"); MARK(6);
                 cuda_check(comm->barrier(stream), "xgpu barrier");
                 allreduce_resid_bf16(b);
             } else {
                 GemmParams go{}; go.M = T; go.N = H; go.K = qd; go.out = x_; go.ldo = H; go.resid = x_; go.ldr = H;
-                cuda_check(product(&tm_attn_, ly.o, go, EPI_RESID, bn_o), "o gemm"); MARK(6);
+                cuda_check(product(attn, ly.o, go, EPI_RESID, bn_o), "o gemm"); MARK(6);
             }
             cuda_check(launch_rmsnorm(x_, ly.ln2, xn_, T, H, cfg.rms_eps, stream), "rmsnorm2"); MARK(1);
             GemmParams gg{}; gg.M = T; gg.N = 2 * F; gg.K = H; gg.out = act_; gg.ldo = F;
-            cuda_check(product(&tm_xn_, ly.gu, gg, EPI_SWIGLU, bn_gu), "gate_up gemm"); MARK(8);
+            cuda_check(product(xn, ly.gu, gg, EPI_SWIGLU, bn_gu), "gate_up gemm"); MARK(8);
             if (use_tp) {
                 const int b = comm->next_buffer();
                 GemmParams gd{}; gd.M = T; gd.N = H; gd.K = F; gd.out = comm->sym(b); gd.ldo = H;
-                cuda_check(product(&tm_act_, ly.down, gd, EPI_STORE, bn_down), "down gemm"); MARK(10);
+                cuda_check(product(actv, ly.down, gd, EPI_STORE, bn_down), "down gemm"); MARK(10);
                 cuda_check(comm->barrier(stream), "xgpu barrier");
                 allreduce_resid_bf16(b);
             } else {
                 GemmParams gd{}; gd.M = T; gd.N = H; gd.K = F; gd.out = x_; gd.ldo = H; gd.resid = x_; gd.ldr = H;
-                cuda_check(product(&tm_act_, ly.down, gd, EPI_RESID, bn_down), "down gemm"); MARK(10);
+                cuda_check(product(actv, ly.down, gd, EPI_RESID, bn_down), "down gemm"); MARK(10);
             }
         }
     }

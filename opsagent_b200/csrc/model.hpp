@@ -98,6 +98,7 @@ private:
     void *x_ = nullptr, *xn_ = nullptr, *qkv_ = nullptr, *q_ = nullptr, *attn_ = nullptr, *act_ = nullptr, *xs_ = nullptr, *xsn_ = nullptr;
     CUtensorMap tm_xn_, tm_attn_, tm_act_, tm_xsn_, tm_q_;
     CUtensorMap tm_few_xn_[3], tm_few_attn_[3], tm_few_act_[3], tm_few_xsn_[3];      // the same rows in boxes of 16, 32 and 64, for steps of that few
+    CUtensorMap tm_swap_xn_[3], tm_swap_attn_[3], tm_swap_act_[3];                   // in boxes of 80, 96 and 112, for tiles of twice that many tokens
     float* amax_val_ = nullptr; int* amax_idx_ = nullptr; int32_t* d_out_ids_ = nullptr;
     uint32_t* mask_table_ = nullptr;               // [mask_slots][mask_words] allowed-token bitsets of grammar states (filled on demand by the scheduler)
     float *part_o_ = nullptr, *part_ml_ = nullptr; int max_part_slots_ = 0;

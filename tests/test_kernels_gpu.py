@@ -747,6 +747,56 @@ def test_decoding_rows_keep_their_bits_beside_others(L, N, K):
     _bits_follow_the_row(L, N, K, 300, [(0, 300), (0, 1), (17, 18), (0, 16), (3, 20), (0, 32), (7, 40), (0, 64), (30, 95), (0, 128), (50, 179), (299, 300)], (32, 64, 128, 256))
 
 
+# Tiles on CTA pairs with the weights' rows as their 256: every width in tokens, one round and several, rows and columns that end inside a tile (and inside a warp's
+# 32), a k range shorter than the ring, every epilogue; the bits of one-CTA tiles.  The width a case is for is asserted.
+@pytest.mark.parametrize("M,N,K,width", [(129, 4096, 320, 128), (257, 264, 2056, 128), (321, 6152, 1032, 192), (300, 8192, 320, 160), (1337, 3080, 1032, 128), (800, 3080, 2056, 160),
+                                         (2100, 5120, 320, 192), (2000, 4096, 1032, 224), (200, 16384, 320, 224)])
+def test_pair_tiles_with_the_operands_swapped(L, monkeypatch, M, N, K, width):
+    assert L.oa_host_gemm_pair_swapped(M, N, K, EPI_STORE, 256) == width
+    g = torch.Generator(device=dev()).manual_seed(M + N + K)
+    A = torch.randn(M, K, generator=g, device=dev()).to(torch.bfloat16)
+    B = (torch.randn(N, K, generator=g, device=dev()) * 0.05).to(torch.bfloat16)
+    bias, resid = torch.randn(N, generator=g, device=dev()).to(torch.bfloat16), torch.randn(M, N, generator=g, device=dev()).to(torch.bfloat16)
+    bias32 = torch.randn(N, generator=g, device=dev())
+    ref = A.double() @ B.double().T
+    room = 0.05 * K ** 1.5 * 2.0 ** -24              # fp32 sums of K products; the rounding to bf16 besides
+
+    def products(bn):
+        bf = lambda cols: torch.full((M, cols), float("nan"), dtype=torch.bfloat16, device=dev())
+        outs = [bf(N), bf(N), bf(N), torch.full((M, N), 1.0, device=dev()), bf(N // 2)]
+        assert L.oa_k_gemm(ptr(A), ptr(B), M, N, K, EPI_STORE, bn, ptr(outs[0]), ptr(bias), None, None, None, None) == 0
+        assert L.oa_k_gemm(ptr(A), ptr(B), M, N, K, EPI_RESID, bn, ptr(outs[1]), None, ptr(resid), None, None, None) == 0
+        assert L.oa_k_gemm_ext(ptr(A), ptr(B), M, N, K, EPI_STORE, bn, ptr(outs[2]), None, 3, 64, 200, 1.0, 0, None) == 0
+        assert L.oa_k_gemm_ext(ptr(A), ptr(B), M, N, K, 4, bn, ptr(outs[3]), ptr(bias32), 0, 0, 0, 0.5, 1, None) == 0
+        if N % 32 == 0:
+            assert L.oa_k_gemm(ptr(A), ptr(B), M, N, K, EPI_SWIGLU, bn, ptr(outs[4]), None, None, None, None, None) == 0
+        torch.cuda.synchronize()
+        return outs
+
+    got = products(256)
+    with monkeypatch.context() as m:                 # with that threshold set, one-CTA tiles are all there is
+        m.setenv("OA_GEMM_PERSISTENT_MIN_TILES", "1000000000")
+        assert L.oa_host_gemm_kernel(M, N, K, EPI_STORE, 64, 0, 0) == 0
+        plain = products(64)
+    want = [ref + bias.double(), ref + resid.double(), ref.clone(), 1.0 + 0.5 * ref + bias32.double()]
+    want[2][:, 64:200] = torch.nn.functional.silu(want[2][:, 64:200])
+    if N % 32 == 0:
+        y = ref.view(M, -1, 2, 16)
+        want.append((torch.nn.functional.silu(y[:, :, 0]) * y[:, :, 1]).reshape(M, -1))
+    for i, w in enumerate(want):
+        o = got[i].double()
+        assert torch.isfinite(o).all()
+        # bf16 outputs round to 2^-9 relative; the fast exponential and divide of the activations another 2^-9; sums as above, through a gate's slope (below 1.1) and factor
+        assert ((o - w).abs() <= 2.0 ** -8 * w.abs() + 8 * room * (1 + w.abs())).all(), i
+        assert torch.equal(got[i], plain[i]), i
+    # rows alone or among others: the bits do not move
+    part = slice(37, 37 + 130) if M > 170 else slice(0, M)
+    a = A[part].contiguous(); alone = torch.full((a.shape[0], N), float("nan"), dtype=torch.bfloat16, device=dev())
+    assert L.oa_k_gemm(ptr(a), ptr(B), a.shape[0], N, K, EPI_STORE, 64, ptr(alone), ptr(bias), None, None, None, None) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(alone, got[0][part])
+
+
 # A prompt's attention has the same bits alone (few items: one head per CTA) and beside others (the two-heads-per-CTA kernel): both take the same keys per
 # tile, raise a row's reference maximum at the same scores and sum its exponentials in the same order.
 @pytest.mark.parametrize("nh,nkv,D", [(32, 8, 128), (20, 4, 128), (32, 8, 64), (15, 3, 64), (16, 2, 128)])
