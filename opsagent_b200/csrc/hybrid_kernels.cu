@@ -849,8 +849,8 @@ __device__ __forceinline__ void st4(__nv_bfloat16* p, const float* f) {
     *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
 }
 // hy_embed_kernel in groups of eight channels.  A thread of that one loads a channel, stores it and only then loads the next (they may overlap, for all the
-// compiler knows): 16 trips to HBM one behind the other for a row of 2048, 10 us of every step.  Here a row is one load a thread.  (A step's first kernel
-// of 16 rows 10 -> 3 us, of 2640 rows 17 -> 9.)
+// compiler knows): 16 trips to HBM one behind the other for a row of 2048, 10 us of every step.  Here a row is one load a thread.  (What it
+// adds to the time line, mean of a prefill of 2640 rows and eight steps of 16: 11.4 -> 2.9 us.)
 template <typename TA>
 __global__ void __launch_bounds__(256) hy_embed_vec8_kernel(const int32_t* __restrict__ ids, const TA* __restrict__ table, float* __restrict__ x, float* __restrict__ x0, int W, int vocab,
                                                             float scale, TA* __restrict__ h, int ldh) {
@@ -892,66 +892,74 @@ __global__ void hy_conv_silu_kernel(const TA* in, int ld_in, int C, const float*
     for (int j = 0; j < taps; ++j) acc = fmaf(w[c * taps + j], conv_input(in, ld_in, C, tail, taps, row0, pos0, i - (taps - 1) + j, c), acc);
     stf(out + (long long)t * ld_out + c, act ? silu_for(acc, out) : acc);
 }
-// bf16 rows of prefill-sized steps whose channels come in aligned groups of 8: a thread computes 8 channels of CONV_ROWS consecutive rows
-// from 16-byte loads, with its taps' weights and the last inputs in registers, so that every input row is read once.  The sum runs over
-// the taps in the same order as in the kernel above: both give the same bits.
+// bf16 rows of prefill-sized steps whose channels come in aligned groups of 8: a thread computes 4 channels of CONV_ROWS consecutive rows, with its taps' weights
+// and the last inputs in registers, so that every input row is read once.  The sum runs over the taps in the same order as in the kernel above: both
+// give the same bits.  Eight channels a thread took 122 registers, 16 warps an SM, and all sixteen rows unrolled more code than stays in the instruction cache:
+// 2640 rows of 4096 channels, behind the projection, 21.5 us a launch (15.5 with four rows unrolled, 14.0 so; four channels of 32, 24 and 8 rows 15.2, 14.6, 13.4;
+// 64 registers spill: 17).  The 43 MB it moves would take 6.6 from HBM; a block's chain is its metadata, its first rows and then four rows in flight a thread.
 constexpr int CONV_ROWS = 16;
-__device__ __forceinline__ void bf8_to_f32(const uint4& u, float* f) {
-    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+__device__ __forceinline__ void bf4_to_f32(const uint2& u, float* f) {
+    const uint32_t w[2] = {u.x, u.y};
 #pragma unroll
-    for (int i = 0; i < 4; ++i) { f[2 * i] = __uint_as_float(w[i] << 16); f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
+    for (int i = 0; i < 2; ++i) { f[2 * i] = __uint_as_float(w[i] << 16); f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
 }
 template <int TAPS>
-__global__ void __launch_bounds__(128) hy_conv_silu_vec8_kernel(const __nv_bfloat16* __restrict__ in, int ld_in, int C, const float* __restrict__ w, const float* __restrict__ bias,
-                                                                 __nv_bfloat16* __restrict__ out, int ld_out, const __nv_bfloat16* __restrict__ tails, HyRows r, int act) {
-    HY_PDL();
+__global__ void __launch_bounds__(128) hy_conv_silu_rows_kernel(const __nv_bfloat16* __restrict__ in, int ld_in, int C, const float* __restrict__ w, const float* __restrict__ bias,
+                                                                __nv_bfloat16* __restrict__ out, int ld_out, const __nv_bfloat16* __restrict__ tails, HyRows r, int act) {
+    constexpr int VEC = 4, AHEAD = 4;
+    griddep_launch();
     // the block's row metadata once, in shared memory, and input rows requested ahead: a thread's chain per row is arithmetic only
     __shared__ int s_row0[CONV_ROWS], s_pos0[CONV_ROWS], s_state[CONV_ROWS];
-    const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 8, t0 = blockIdx.y * CONV_ROWS, n = min(CONV_ROWS, r.T - t0);
+    const int c = (blockIdx.x * blockDim.x + threadIdx.x) * VEC, t0 = blockIdx.y * CONV_ROWS, n = min(CONV_ROWS, r.T - t0);
     if (threadIdx.x < n) { const int seq = r.row_seq[t0 + threadIdx.x]; s_row0[threadIdx.x] = r.seq_row0[seq]; s_pos0[threadIdx.x] = r.seq_pos0[seq]; s_state[threadIdx.x] = r.seq_state[seq]; }
+    float wf[VEC * TAPS], win[TAPS][VEC], b8[VEC];             // taps of the thread's channels, [channel][tap] as they lie
+    if (c < C) {
+#pragma unroll
+        for (int i = 0; i < TAPS; ++i) ld4(w + (long long)c * TAPS + i * 4, wf + i * 4);
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) b8[e] = bias ? bias[c + e] : 0.f;
+    }
+    griddep_wait();
     __syncthreads();
     if (c >= C) return;
-    constexpr int AHEAD = 4;
-    uint4 ring[AHEAD];
+    uint2 ring[AHEAD];
 #pragma unroll
-    for (int k = 0; k < AHEAD; ++k) if (k < n) ring[k] = *reinterpret_cast<const uint4*>(in + (long long)(t0 + k) * ld_in + c);
-    float wf[8 * TAPS], win[TAPS][8], b8[8];             // taps of the thread's channels, [channel][tap] as they lie
+    for (int k = 0; k < AHEAD; ++k) if (k < n) ring[k] = *reinterpret_cast<const uint2*>(in + (long long)(t0 + k) * ld_in + c);
+#pragma unroll 1
+    for (int tb = 0; tb < n; tb += AHEAD)
 #pragma unroll
-    for (int i = 0; i < 2 * TAPS; ++i) ld4(w + (long long)c * TAPS + i * 4, wf + i * 4);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) b8[e] = bias ? bias[c + e] : 0.f;
-#pragma unroll
-    for (int tt = 0; tt < CONV_ROWS; ++tt) {
+    for (int tk = 0; tk < AHEAD; ++tk) {
+        const int tt = tb + tk;
         if (tt >= n) break;
         const int t = t0 + tt, row0 = s_row0[tt], i = t - row0;
-        const uint4 cur = ring[tt % AHEAD];
-        if (tt + AHEAD < n) ring[tt % AHEAD] = *reinterpret_cast<const uint4*>(in + (long long)(t + AHEAD) * ld_in + c);
+        const uint2 cur = ring[tk];
+        if (tt + AHEAD < n) ring[tk] = *reinterpret_cast<const uint2*>(in + (long long)(t + AHEAD) * ld_in + c);
         if (tt == 0 || i == 0) {                        // the inputs before this row: earlier rows of the step, the carried tail, or zeros
             const int pos0 = s_pos0[tt];
             const __nv_bfloat16* tail = tails + (long long)s_state[tt] * (TAPS - 1) * C;
 #pragma unroll
             for (int j = 0; j < TAPS - 1; ++j) {
                 const int src = i - (TAPS - 1) + j;
-                uint4 u = make_uint4(0u, 0u, 0u, 0u);
-                if (src >= 0) u = *reinterpret_cast<const uint4*>(in + (long long)(row0 + src) * ld_in + c);
-                else if (pos0 > 0) u = *reinterpret_cast<const uint4*>(tail + (long long)(TAPS - 1 + src) * C + c);
-                bf8_to_f32(u, win[j]);
+                uint2 u = make_uint2(0u, 0u);
+                if (src >= 0) u = *reinterpret_cast<const uint2*>(in + (long long)(row0 + src) * ld_in + c);
+                else if (pos0 > 0) u = *reinterpret_cast<const uint2*>(tail + (long long)(TAPS - 1 + src) * C + c);
+                bf4_to_f32(u, win[j]);
             }
         }
-        bf8_to_f32(cur, win[TAPS - 1]);
-        float o[8];
+        bf4_to_f32(cur, win[TAPS - 1]);
+        float o[VEC];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
+        for (int e = 0; e < VEC; ++e) {
             float a = b8[e];
 #pragma unroll
             for (int j = 0; j < TAPS; ++j) a = fmaf(wf[e * TAPS + j], win[j][e], a);
             o[e] = act ? silu_for(a, out) : a;
         }
-        *reinterpret_cast<uint4*>(out + (long long)t * ld_out + c) = make_uint4(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]), pack_bf16x2(o[4], o[5]), pack_bf16x2(o[6], o[7]));
+        *reinterpret_cast<uint2*>(out + (long long)t * ld_out + c) = make_uint2(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]));
 #pragma unroll
         for (int j = 0; j < TAPS - 1; ++j)
 #pragma unroll
-            for (int e = 0; e < 8; ++e) win[j][e] = win[j + 1][e];
+            for (int e = 0; e < VEC; ++e) win[j][e] = win[j + 1][e];
     }
 }
 template <typename TA>
@@ -1740,11 +1748,11 @@ cudaError_t hy_conv_silu(bool f32, const void* in, int ld_in, int C, const float
                          cudaStream_t s, int act) {
     auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
     if (!f32 && r.T >= 512 && taps >= 2 && taps <= 4 && C % 8 == 0 && ld_in % 8 == 0 && ld_out % 8 == 0 && al16(in) && al16(out) && al16(tails) && al16(w)) {
-        const dim3 g((C / 8 + 127) / 128, (r.T + CONV_ROWS - 1) / CONV_ROWS);
+        const dim3 g((C / 4 + 127) / 128, (r.T + CONV_ROWS - 1) / CONV_ROWS);
         switch (taps) {
-            case 2: return launch_plain(hy_conv_silu_vec8_kernel<2>, g, dim3(128), 0, s, (const bf*)in, ld_in, C, w, bias, (bf*)out, ld_out, (const bf*)tails, r, act);
-            case 3: return launch_plain(hy_conv_silu_vec8_kernel<3>, g, dim3(128), 0, s, (const bf*)in, ld_in, C, w, bias, (bf*)out, ld_out, (const bf*)tails, r, act);
-            default: return launch_plain(hy_conv_silu_vec8_kernel<4>, g, dim3(128), 0, s, (const bf*)in, ld_in, C, w, bias, (bf*)out, ld_out, (const bf*)tails, r, act);
+            case 2: return launch_plain(hy_conv_silu_rows_kernel<2>, g, dim3(128), 0, s, (const bf*)in, ld_in, C, w, bias, (bf*)out, ld_out, (const bf*)tails, r, act);
+            case 3: return launch_plain(hy_conv_silu_rows_kernel<3>, g, dim3(128), 0, s, (const bf*)in, ld_in, C, w, bias, (bf*)out, ld_out, (const bf*)tails, r, act);
+            default: return launch_plain(hy_conv_silu_rows_kernel<4>, g, dim3(128), 0, s, (const bf*)in, ld_in, C, w, bias, (bf*)out, ld_out, (const bf*)tails, r, act);
         }
     }
     dim3 grid((C + 127) / 128, r.T);

@@ -436,3 +436,25 @@ def test_short_portions_leave_what_the_next_ones_carry(tmp_path, delta, latent):
         for cuts in ([1, 2, 3, 4, 5, 1, 4, 1, 6, 2, 1, 1, 3], [5, 1, 1, 20, 2, 4], [4, 4, 4]):
             e = K.rel_err(replay(eng, 1, toks, cuts).astype(np.float64), want)
             assert np.quantile(e, 0.95) < 0.05 and e.max() < 0.1, f"cuts {cuts}: 95% {np.quantile(e, 0.95):.3e}, worst {e.max():.3e}"
+
+
+# steps of 512 rows and more take the convolution in blocks of 16 rows and four channels a thread: sequences that begin inside a block, in its last row and at its edge, one of
+# fewer rows than taps, tails carried between two such steps, and channels (16 x 2 + 24 a head, in eights) that end inside a CTA's 512
+@pytest.mark.parametrize("taps", [2, 3, 4])
+@pytest.mark.parametrize("heads,dim,vdim", [(2, 16, 24), (5, 64, 24)])
+def test_convolutions_of_many_rows(tmp_path, taps, heads, dim, vdim):
+    cfg = K.make_config([D(heads=heads, kv_heads=heads, dim=dim, vdim=vdim, conv=taps)], width=64, vocab=96)
+    W = checkpoint(tmp_path, cfg, seed=23)
+    cuts = [(1, 270, 3), (15, 241, 2), (240, 2, 270), (257, 47, 256)]           # rows of a sequence in each step: 513, 560, 531
+    seqs = [tokens_of(cfg, sum(c), 40 + i) for i, c in enumerate(cuts)]
+    got = [[] for _ in cuts]
+    with engine(tmp_path, "bfloat16", pages=48) as eng:
+        for s in range(3):
+            at = [sum(c[:s]) for c in cuts]
+            lg = eng.trace_step([(i + 1, seqs[i][at[i]:at[i] + c[s]], list(range(c[s]))) for i, c in enumerate(cuts)], [])
+            row = 0
+            for i, c in enumerate(cuts):
+                got[i].append(lg[row:row + c[s]]); row += c[s]
+    for i, toks in enumerate(seqs):
+        e = K.rel_err(np.concatenate(got[i]).astype(np.float64), K.forward(cfg, W, toks))
+        assert np.quantile(e, 0.95) < 0.05 and e.max() < 0.1, f"sequence {i}: 95% {np.quantile(e, 0.95):.3e}, worst {e.max():.3e}"
