@@ -660,7 +660,7 @@ __global__ void __launch_bounds__(PtpCfg<D>::THREADS, 1) prefill_attention_pair_
 // warpgroups take the tiles in turn: while one takes the exponentials of tile t, the other fetches S and finds the maxima of t + 1, and the tensor core
 // runs P V of t - 1 and S of t + 2.  What a head still does in order is one value a row: a tile's reference maximum follows from the last one's, so it goes from
 // warpgroup to warpgroup as soon as the maxima stand.  With heads of 128 a CTA alone would fetch 64 KB of keys and values a tile, in 1300 cycles: what the L2 gives
-// (five prompts of 1.4 thousand rows 139 us, 1000 rows behind 6000 worse than above).  So two heads' CTAs share them: a product is 256 x 128 x 16
+// (32 / 8 heads: five prompts of 1.4 thousand rows 139 us against 97 above, 1400 rows behind 3000 123 against 96).  So two heads' CTAs share them: a product is 256 x 128 x 16
 // (cta_group::2) with half of B in each CTA, and each loads one of a tile's two K pages and 64 of V's 128 columns.  Heads of 64 need half the bytes and no pair.
 //   warp 0     : TMA: this CTA's Q (two items ahead), its share of K and V       warp 1 (of a pair: the even CTA's): tcgen05.mma
 //   warps 4-11 : softmax of even and odd tiles, one query row per thread         warps 12-15: output, while the next item's tiles run

@@ -1,13 +1,14 @@
 // gemm_pair.cu — prefill projections on CTA pairs: C[M,N] = A[M,K] · B[N,K]^T with tcgen05.mma.cta_group::2.
 //
-// The two CTAs of a cluster (two SMs of one TPC) share one 256 x bn output tile, bn = 128, 160, .. 256: each holds its own 128 rows of A and HALF of the B
-// tile in shared memory, and one thread of the even CTA issues 256 x bn x 16 products that read both halves.  Against a 128 x 256 tile per SM that is 2/3
+// The two CTAs of a cluster (two SMs of one TPC) share one 256 x bn output tile: each holds its own 128 rows of one operand (U) and HALF of the bn rows of the
+// other (V) in shared memory, and one thread of the even CTA issues 256 x bn x 16 products that read both halves.  U is A (the tokens) and bn 128, 160, .. 256, or
+// U is B (the weights) and bn 160, 192, .. 256 tokens, whichever fills the last round better.  Against a 128 x 256 tile per SM that is 2/3
 // of the shared-memory reads and of the L2 traffic per product.  Large products run against the 1000 W cap here (85 % of the tensor peak at a clock that is
 // down to 1.25 GHz), so what counts there is the energy per product: 8192 x 28672 x 4096 gated 1505 us a call in a loop on 128 x 256 tiles, 1445 on pairs.
 // The width is what fills the last round: 1337 x 4096 x 14336 (residual) is 96 tiles of 256 columns, two rounds of 74 pairs of which the second is a third
 // full, and 132 tiles of 192: 149 -> 127 us; 1000 x 5120 x 27648 80 tiles of 256, 128 of 160: 288 -> 205; 400 x 2048 x 2048 19.8 -> 12.0 at 128.  Narrow tiles
 // take warps that stay converged and issue under elect.sync: behind `if (lane == 0)` a k block cost 0.26 us whatever its width.
-//   warp 0   : TMA producer of this CTA's A rows and B half; both CTAs' bytes are counted on the EVEN CTA's `full` barrier
+//   warp 0   : TMA producer of this CTA's U rows and half of V; both CTAs' bytes are counted on the EVEN CTA's `full` barrier
 //   warp 1   : allocates TMEM (both CTAs); in the even CTA it issues the products; commits release the ring slot in both CTAs
 //   warps 2-5: epilogue of this CTA's 128 rows while the next tile is multiplied (two accumulators)
 // Persistent over tiles in grouped raster order.  Every tile sums its k blocks in ascending order in one accumulator, as the single-CTA kernels do: a

@@ -486,7 +486,7 @@ __global__ void __launch_bounds__(128) hy_mla_attention_mma_kernel(HyLatentAttn 
 // turns at groups of 16 cache rows instead, each with an online softmax and accumulators of its own, joined once at the end.  Cache rows come
 // by one bulk copy each into a ring per warp: no warp waits for another before the join.  What bounds it is the chain of a warp's groups.
 // 16 rows of 170 cached tokens, 16 heads of a 512 + 64 wide latent: 60 -> 20 us against the 64-query tile, of which three warps idled.
-// In a decoding step 15.0 -> 13.5 us with all loads of a warp's queries in flight at once and the warps' sums written without bank conflicts (eight rows a store).
+// In a decoding step 15.0 -> 13.6 us with all loads of a warp's queries in flight at once and the warps' sums written without bank conflicts (eight rows a store).
 // ---------------------------------------------------------------------------------------------------------------------------------
 constexpr int MLA_DQ = 16;
 static size_t mla_decode_smem(int E, int nvb, int stages) {
