@@ -556,7 +556,8 @@ __global__ void __launch_bounds__(256) hy_few_memory_kernel(FewArgs f, HyRows r)
 #pragma unroll
             for (int w = 0; w < 8; ++w) { const float4 x = *reinterpret_cast<const float4*>(&po[t & 1][w][c4]); o.x += x.x; o.y += x.y; o.z += x.z; o.w += x.w; }
             if (DELTA) {
-                const float ss = warp_sum(ok ? (o.x * o.x + o.y * o.y) + (o.z * o.z + o.w * o.w) : 0.f), rr = 1.0f / sqrtf(ss / (float)VD + p.eps);
+                // in this rounding whatever stands around it: left to the compiler, which product of each pair was rounded first depended on the surrounding code
+                const float ss = warp_sum(ok ? __fadd_rn(fmaf(o.x, o.x, __fmul_rn(o.y, o.y)), fmaf(o.z, o.z, __fmul_rn(o.w, o.w))) : 0.f), rr = 1.0f / sqrtf(ss / (float)VD + p.eps);
                 if (ok) {
                     const float4 w = nw;
                     *reinterpret_cast<uint2*>(reinterpret_cast<bf*>(p.out) + (row0 + t) * p.ldo + (long long)h * VD + c4) =

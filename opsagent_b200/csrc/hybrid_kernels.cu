@@ -247,7 +247,7 @@ __device__ __forceinline__ void mla_prep_row(const HyLatentAttn& a, const TA* __
         if (d >= 2 * half) return ldf(x + d);
         const int p = pair_of(d);
         const float u0 = ldf(x + (a.rot_layout ? p : 2 * p)), u1 = ldf(x + (a.rot_layout ? p + half : 2 * p + 1)), f = one_pair ? co : cs[p], g = one_pair ? si : sn[p];
-        return second_of(d) ? (u1 * f + u0 * g) : (u0 * f - u1 * g);
+        return second_of(d) ? fmaf(u1, f, __fmul_rn(u0, g)) : fmaf(u0, f, -__fmul_rn(u1, g));      // which product is rounded first is written down: nothing around this moves a bit
     };
 #pragma unroll 8
     for (int i = threadIdx.x; i < a.heads * rot; i += 128) {      // rotated query parts (no array here overlaps another: several of these in flight)

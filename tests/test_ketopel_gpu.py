@@ -3,6 +3,10 @@ through Engine.trace_step, which drives the scheduler's own batch builder, pages
 decoding, mixed batches, pages and slots that are used again, far keys, what a looped block adds ahead of its passes, the soft cap, decays near
 one and near zero, the first tokens of a sequence, long decoding, the tensor-core kernels against the plain ones, and greedy generation through
 the scheduler.  Small random checkpoints are written per test."""
+import hashlib
+import json
+import os
+
 import numpy as np
 import pytest
 
@@ -458,3 +462,35 @@ def test_convolutions_of_many_rows(tmp_path, taps, heads, dim, vdim):
     for i, toks in enumerate(seqs):
         e = K.rel_err(np.concatenate(got[i]).astype(np.float64), K.forward(cfg, W, toks))
         assert np.quantile(e, 0.95) < 0.05 and e.max() < 0.1, f"sequence {i}: 95% {np.quantile(e, 0.95):.3e}, worst {e.max():.3e}"
+
+
+def step_digests(folder, seed, passes=2):
+    """the four layers of the large sizes (16 heads, a latent of 512 + 64 channels) once each, weights the engine seeds itself: 16 prompts in one step, then
+    eight steps of a token each; -> sha256 (16 digits) of every step's logits, for each of `passes` passes through one engine"""
+    from opsagent_b200 import hybrid_bench
+    sizes = hybrid_bench.ketopel_sizes("large")
+    del sizes["loop"]
+    with open(os.path.join(str(folder), "config.json"), "w") as f:
+        json.dump(sizes, f)
+    rng = np.random.default_rng(seed)
+    prompts = [rng.integers(0, sizes["vocab"], n).tolist() for n in rng.integers(30, 301, 16)]
+    steps = rng.integers(0, sizes["vocab"], (8, 16)).tolist()
+    out = []
+    with engine(folder, "bfloat16", pages=96, slots=16, max_seq_len=384, max_step_tokens=8192) as eng:
+        for _ in range(passes):
+            logits = [eng.trace_step([(i, p, [len(p) - 1]) for i, p in enumerate(prompts)])]
+            for k, tokens in enumerate(steps):
+                logits.append(eng.trace_step([(i, [t], [0]) for i, t in enumerate(tokens)], list(range(16)) if k == 7 else []))
+            out.append([hashlib.sha256(x.tobytes()).hexdigest()[:16] for x in logits])
+    return out
+
+
+# The bits of a hybrid prefill and its decoding steps: the same in every pass, and those recorded in golden/ketopel_steps.json when every multiply-add whose
+# rounding the source leaves open (a x b + c x d) stood in kernels of another shape.  A step whose sums run in another order on purpose records them again.
+@pytest.mark.parametrize("seed", [8, 13])
+def test_steps_keep_their_bits(tmp_path, seed):
+    with open(os.path.join(os.path.dirname(os.path.abspath(__file__)), "golden", "ketopel_steps.json")) as f:
+        want = json.load(f)[str(seed)]
+    first, second = step_digests(tmp_path, seed)
+    assert first == second
+    assert first == want, [i for i, (a, b) in enumerate(zip(first, want)) if a != b]
