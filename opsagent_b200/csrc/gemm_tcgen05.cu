@@ -394,30 +394,30 @@ static cudaError_t launch_persistent(const CUtensorMap* tmA, const CUtensorMap* 
 // 128 x 256 0.22 + 0.27 x busy (354 x 57344 x 8192: 353 us, three row tiles instead of two of 256 rows: 384 on pairs), 128 x 128 0.17 + 0.13 x busy, narrower
 // 0.15 + 0.07 x busy.  Up to 128 rows half of a pair's rows would be padding.  Every kernel sums k in the same order: the choice moves no bit.
 // Either operand's rows may be the 256 of a tile.  With the weights' there, tokens come in steps of 32 instead of 256: 1337 rows are 1344 or 1440, not 1536, 300 are
-// 320, not 512, and there are more ways to fill the last round.  The same estimate serves both; us in loops, tokens' rows the 256 -> weights': 1337 x 4096 x 14336
-// 126 -> 115, 300 x 28672 x 4096 83 -> 68, 300 x 7168 x 5120 36 -> 25, 1337 x 55296 x 5120 521 -> 480, 4000 x 4096 x 14336 337 -> 304; where it is the wrong way
-// 1024 x 28672 x 4096 155 -> 177, 1621 x 55296 x 5120 609 -> 646 (128 tokens instead of 256 columns: narrow tiles fetch more from L2 a product, which the estimate
-// leaves out).  So the weights' have to be 2.5 % better, 6 % where their tiles are the narrower ones, 7 % against tiles of one CTA; up to 512 rows and 100 MB of
-// weights equal estimates go to them (200 x 7168 x 5120 24.8 -> 23.6, 512 x 2048 x 2048 12.3 -> 10.6).  Over 162 products of 130 to 8192 rows of the four models 5.5 %
-// faster than without, 4 of them 3 to 10 % slower within what their neighbours of a few rows differ by.
-struct PairWidth { int bn; double us; bool swapped; };
+// 320, not 512, and there are more ways to fill the last round.  The same estimate serves both.  us in loops, on operands that no call before has touched, and alone
+// behind a flush of L2, tokens' rows the 256 -> weights': 1337 x 4096 x 14336 127 -> 117, 150 -> 126, 173 -> 153; 300 x 28672 x 4096 83 -> 68, 98 -> 77, 118 -> 96;
+// 300 x 7168 x 5120 29 -> 22, 30 -> 24, 48 -> 41; 2366 x 6144 x 4096 91 -> 82, 104 -> 94, 123 -> 114.  It pays where a pair then multiplies fewer columns one after the
+// other (chain).  Where only padding goes, the estimate's credit for idle pairs is not there, and an epilogue that turns its chunks is 1 to 2 us longer in a call alone:
+// 433 x 4096 x 4096 29.6 -> 31.2, 834 x 8192 x 8192 94 -> 104 in loops, 138 x 10240 x 8192 50 -> 53.  So the chain has to be shorter and the estimate 6 % lower
+// (of 50 products short of that, 29 were more than 2 % slower in one of the three kinds of call and one faster in all), 7 % against tiles of one CTA.  Over 70
+// products of the four models that take it: 13, 14 and 11 % faster.
+struct PairWidth { int bn; double us; bool swapped; long long chain; };      // chain: columns (tokens) a pair multiplies one after the other
 static long long ceil_div(long long a, long long b) { return (a + b - 1) / b; }
 static PairWidth gemm_pair_width(const GemmParams& p, int sms) {
     const long long pairs = sms / 2, kb = ceil_div(p.K, BLOCK_K);
     auto least = [&](long long rows256, long long rows, bool swapped) {
-        PairWidth best{0, 0.0, swapped};
+        PairWidth best{0, 0.0, swapped, 0};
         for (int bn = 256; bn >= 128; bn -= 32) {
             const long long tiles = ceil_div(rows, bn) * ceil_div(rows256, 256), rounds = ceil_div(tiles, pairs);
             const double us = (double)(rounds * kb) * (bn / 256.0 * (0.28 + 0.14 * (double)tiles / (double)(rounds * pairs)) + 0.02) + 8.5;
-            if (!best.bn || us < best.us) { best.bn = bn; best.us = us; }
+            if (!best.bn || us < best.us) { best.bn = bn; best.us = us; best.chain = rounds * bn; }
         }
         return best;
     };
     const PairWidth plain = least(p.M, p.N, false);
     if (!p.swap_ok) return plain;
     PairWidth swapped = least(p.N, p.M, true);
-    const double line = p.M <= 512 && 2LL * p.N * p.K <= 100000000LL ? 1.0001 : swapped.bn < plain.bn ? 0.94 : 0.975;
-    if (swapped.us >= plain.us * line) return plain;
+    if (swapped.us >= plain.us * 0.94 || swapped.chain >= plain.chain) return plain;
     swapped.us = std::min(swapped.us * 1.07, plain.us);          // what one-CTA tiles have to beat
     return swapped;
 }
@@ -447,7 +447,7 @@ static int few_width(int N, int sms) {
     return 128;
 }
 GemmChoice gemm_choice(const GemmParams& p, int epilogue, int block_n) {
-    PairWidth pair{256, 0.0, false};
+    PairWidth pair{256, 0.0, false, 0};
     GemmChoice c{kernel_of(p, epilogue, block_n, pair), 128, block_n, block_n};
     if (c.kernel == GEMM_PAIR) { c.width = pair.bn; c.swapped = pair.swapped; (c.swapped ? c.a_box : c.b_box) = pair.bn / 2; if (c.swapped) c.b_box = 128; }
     if (c.kernel == GEMM_FEW) { c.a_box = few_box(p.M); c.width = c.b_box = few_width(p.N, sm_count_cached()); }

@@ -756,6 +756,18 @@ def test_which_kernel_a_product_takes(monkeypatch):
     assert k(64, 4096, 4096, 0, 256, 1, 0) == PERSISTENT and k(8192, 28672, 4096, 0, 256, 1, 0) == PERSISTENT and k(300, 1024, 512, 0, 128, 1, 0) == TILE
 
 
+# Tiles with the weights' rows as their 256 are for products whose pairs then multiply fewer columns one after the other, by an estimate clearly below the other form's.  The
+# first group took them for a smaller padding alone and lost up to 9 % (each measured in loops, on operands met for the first time and in single calls).
+def test_operands_are_swapped_only_where_that_shortens_a_pairs_work():
+    swapped = _lib.load().oa_host_gemm_pair_swapped
+    for m, n, k, epi, bn in [(168, 5120, 5120, 1, 64), (218, 5120, 5120, 1, 64), (433, 4096, 4096, 1, 64), (296, 2048, 2048, 1, 32), (473, 5120, 5120, 1, 128), (834, 8192, 8192, 1, 256),
+                             (620, 5120, 5120, 1, 128), (211, 28672, 4096, 2, 256), (408, 7168, 5120, 0, 128), (138, 10240, 8192, 0, 128), (889, 8192, 28672, 1, 256)]:
+        assert swapped(m, n, k, epi, bn) == 0, (m, n, k)
+    for m, n, k, epi, bn, width in [(1337, 4096, 14336, 1, 256, 160), (300, 28672, 4096, 2, 256, 160), (300, 7168, 5120, 0, 128, 160), (374, 6144, 4096, 0, 128, 128), (551, 5120, 5120, 1, 128, 192),
+                                    (1556, 5120, 5120, 1, 256, 224), (304, 55296, 5120, 2, 256, 160), (775, 5120, 27648, 1, 128, 128)]:
+        assert swapped(m, n, k, epi, bn) == width, (m, n, k)
+
+
 @pytest.mark.parametrize("value,kernel", [("0", 0), ("1", 3)])
 def test_the_switch_that_turns_persistent_products_off(value, kernel):
     """OA_GEMM_PERSISTENT=0: one CTA per tile for every product, also for those that CTA pairs would take"""

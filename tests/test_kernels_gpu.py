@@ -747,10 +747,10 @@ def test_decoding_rows_keep_their_bits_beside_others(L, N, K):
     _bits_follow_the_row(L, N, K, 300, [(0, 300), (0, 1), (17, 18), (0, 16), (3, 20), (0, 32), (7, 40), (0, 64), (30, 95), (0, 128), (50, 179), (299, 300)], (32, 64, 128, 256))
 
 
-# Tiles on CTA pairs with the weights' rows as their 256: every width in tokens, one round and several, rows and columns that end inside a tile (and inside a warp's
-# 32), a k range shorter than the ring, every epilogue; the bits of one-CTA tiles.  The width a case is for is asserted.
-@pytest.mark.parametrize("M,N,K,width", [(129, 4096, 320, 128), (257, 264, 2056, 128), (321, 6152, 1032, 192), (300, 8192, 320, 160), (1337, 3080, 1032, 128), (800, 3080, 2056, 160),
-                                         (2100, 5120, 320, 192), (2000, 4096, 1032, 224), (200, 16384, 320, 224)])
+# Tiles on CTA pairs with the weights' rows as their 256: every width in tokens that the rule takes, one round and several, rows and columns that end inside a tile
+# (and inside a warp's 32), a k range shorter than the ring, every epilogue; the bits of one-CTA tiles.  The width a case is for is asserted.
+@pytest.mark.parametrize("M,N,K,width", [(257, 5120, 1032, 128), (1337, 3080, 1032, 128), (321, 28672, 192, 128), (258, 9000, 320, 160), (800, 3080, 2056, 160), (130, 28672, 192, 160),
+                                         (322, 9000, 1032, 192), (513, 16384, 320, 192), (385, 9000, 2056, 224), (1537, 10240, 320, 224)])
 def test_pair_tiles_with_the_operands_swapped(L, monkeypatch, M, N, K, width):
     assert L.oa_host_gemm_pair_swapped(M, N, K, EPI_STORE, 256) == width
     g = torch.Generator(device=dev()).manual_seed(M + N + K)
