@@ -183,10 +183,10 @@ OA_API int oa_host_streamk_plan(int32_t N, int32_t K, int32_t block_n, int32_t n
  * vocabulary head.  few_rows: the caller's A map may have the narrower box (the entry points above and the hybrid models); grouped: a row tile's weights
  * come from a table */
 OA_API int oa_host_gemm_kernel(int32_t M, int32_t N, int32_t K, int32_t epilogue, int32_t block_n, int32_t few_rows, int32_t grouped);
-/* columns of the tiles the CTA-pair kernel takes for that product (128, 160, .. 256), 0 where another kernel runs it */
 /* the kernel that oa_k_paged_attention takes for a batch of prompts: 1 one head per CTA, 2 two heads per CTA, 3 and 4 key tiles in turns on a CTA pair or a CTA (the same bits) */
 OA_API int oa_host_prefill_attention_kernel(const int32_t* ctx_lens, const int32_t* q_lens, int32_t n_seqs, int32_t n_heads, int32_t n_kv, int32_t head_dim);
-/* tokens of a tile where oa_k_gemm multiplies on CTA pairs with the weights' rows as a tile's 256, else 0 (oa_host_gemm_pair_width: columns of a tile of 256 tokens) */
+/* where oa_k_gemm multiplies on CTA pairs, the other side of its tiles (128, 160, .. 256): pair_width the columns of a tile of 256 tokens, pair_swapped the tokens of a
+ * tile of 256 of the weights' rows; each 0 where the product runs in the other form or in another kernel */
 OA_API int oa_host_gemm_pair_swapped(int32_t M, int32_t N, int32_t K, int32_t epilogue, int32_t block_n);
 OA_API int oa_host_gemm_pair_width(int32_t M, int32_t N, int32_t K, int32_t epilogue, int32_t block_n);
 /* byte-level BPE tokenizer read from a Hugging Face tokenizer.json (Llama-3 / Qwen2.5 format), host only: what the engine uses

@@ -180,16 +180,16 @@ int oa_k_gemm_ext(const void* A, const void* B, int32_t M, int32_t N, int32_t K,
 }
 
 int oa_host_gemm_kernel(int32_t M, int32_t N, int32_t K, int32_t epilogue, int32_t block_n, int32_t few_rows, int32_t grouped) {
-    GemmParams p{}; p.M = M; p.N = N; p.K = K; p.few_rows_ok = few_rows;
+    GemmParams p{}; p.M = M; p.N = N; p.K = K; p.few_rows_ok = few_rows; p.swap_ok = !grouped;
     static const int32_t group = 0;
     if (grouped) p.m_tile_group = &group;
     return (int)gemm_choice(p, epilogue, block_n).kernel;
 }
 
 int oa_host_gemm_pair_width(int32_t M, int32_t N, int32_t K, int32_t epilogue, int32_t block_n) {
-    GemmParams p{}; p.M = M; p.N = N; p.K = K;
+    GemmParams p{}; p.M = M; p.N = N; p.K = K; p.few_rows_ok = p.swap_ok = 1;
     const GemmChoice c = gemm_choice(p, epilogue, block_n);
-    return c.kernel == GEMM_PAIR ? c.width : 0;
+    return c.kernel == GEMM_PAIR && !c.swapped ? c.width : 0;
 }
 
 int oa_host_prefill_attention_kernel(const int32_t* ctx_lens, const int32_t* q_lens, int32_t n_seqs, int32_t n_heads, int32_t n_kv, int32_t head_dim) {

@@ -763,9 +763,13 @@ def test_operands_are_swapped_only_where_that_shortens_a_pairs_work():
     for m, n, k, epi, bn in [(168, 5120, 5120, 1, 64), (218, 5120, 5120, 1, 64), (433, 4096, 4096, 1, 64), (296, 2048, 2048, 1, 32), (473, 5120, 5120, 1, 128), (834, 8192, 8192, 1, 256),
                              (620, 5120, 5120, 1, 128), (211, 28672, 4096, 2, 256), (408, 7168, 5120, 0, 128), (138, 10240, 8192, 0, 128), (889, 8192, 28672, 1, 256)]:
         assert swapped(m, n, k, epi, bn) == 0, (m, n, k)
+    lib = _lib.load()
     for m, n, k, epi, bn, width in [(1337, 4096, 14336, 1, 256, 160), (300, 28672, 4096, 2, 256, 160), (300, 7168, 5120, 0, 128, 160), (374, 6144, 4096, 0, 128, 128), (551, 5120, 5120, 1, 128, 192),
                                     (1556, 5120, 5120, 1, 256, 224), (304, 55296, 5120, 2, 256, 160), (775, 5120, 27648, 1, 128, 128)]:
         assert swapped(m, n, k, epi, bn) == width, (m, n, k)
+        # what the other questions about the same call answer
+        assert lib.oa_host_gemm_kernel(m, n, k, epi, bn, 1, 0) == lib.oa_host_gemm_kernel(m, n, k, epi, bn, 0, 0) == 3 and lib.oa_host_gemm_pair_width(m, n, k, epi, bn) == 0
+    assert lib.oa_host_gemm_kernel(300, 28672, 4096, 2, 256, 0, 1) == 2                              # grouped products keep tiles of one CTA
 
 
 @pytest.mark.parametrize("value,kernel", [("0", 0), ("1", 3)])

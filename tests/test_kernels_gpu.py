@@ -520,15 +520,17 @@ TILE, FEW, PERSISTENT, PAIR, HEAD = 0, 1, 2, 3, 4                  # oa_host_gem
 
 
 # CTA-pair kernel: one round of tiles and several, ragged last rows and columns, one CTA's rows all beyond the last, and k ranges shorter than the ring
-# over many tiles (ring phases run across tiles, accumulators change hands every block or two); store, residual and gated.  Which kernel a product takes is
-# asserted: a rule that moves must not empty a case.
-PAIR_CASES = [(614, 6144, 4096), (257, 6152, 4096), (700, 6152, 2056), (400, 2048, 8192), (614, 4096, 14336), (1337, 4096, 14336), (1000, 5120, 4160), (384, 296, 27648), (2000, 1000, 8192),
-              (7900, 14336, 320), (8192, 24576, 192)]
+# over many tiles (ring phases run across tiles, accumulators change hands every block or two); store, residual and gated.  Which kernel a product takes, and
+# whose rows are the 256 of its tiles, is asserted: a rule that moves must not empty a case.
+PAIR_TOKENS = [(257, 6144, 320), (257, 6152, 192), (700, 6152, 2056), (400, 2048, 8192), (449, 8192, 1032), (1000, 4096, 4096), (1000, 5120, 4160), (384, 296, 27648), (2000, 1000, 8192),
+               (7900, 14336, 320), (8192, 24576, 192)]
+PAIR_WEIGHTS = [(614, 6144, 4096), (257, 6152, 4096), (614, 4096, 14336), (1337, 4096, 14336)]
 
 
-@pytest.mark.parametrize("M,N,K", PAIR_CASES)
-def test_gemm_cta_pairs(L, M, N, K):
+@pytest.mark.parametrize("M,N,K,swapped", [(*c, 0) for c in PAIR_TOKENS] + [(*c, 1) for c in PAIR_WEIGHTS])
+def test_gemm_cta_pairs(L, M, N, K, swapped):
     assert L.oa_host_gemm_kernel(M, N, K, EPI_STORE, 256, 1, 0) == PAIR
+    assert (L.oa_host_gemm_pair_width(M, N, K, EPI_STORE, 256) > 0) == (not swapped) and (L.oa_host_gemm_pair_swapped(M, N, K, EPI_STORE, 256) > 0) == bool(swapped)
     g = torch.Generator(device=dev()).manual_seed(M + N + K)
     A = torch.randn(M, K, generator=g, device=dev()).to(torch.bfloat16)
     B = (torch.randn(N, K, generator=g, device=dev()) * 0.05).to(torch.bfloat16)
@@ -712,8 +714,9 @@ def test_prefill_rows_keep_their_bits_beside_others(L, N, K):
 
 # Every width of a pair's tile: one round and several, ragged last rows and columns (N no multiple of the width, and where the gated form runs, of 64), a k
 # range shorter than the ring; the bits of one-CTA tiles.  The width a case is for is asserted.
-@pytest.mark.parametrize("M,N,K,width", [(257, 264, 2056, 128), (129, 9000, 1032, 128), (300, 5120, 4096, 160), (700, 3080, 1032, 160), (1000, 6152, 2056, 192), (513, 8192, 1032, 192),
-                                         (640, 5120, 4096, 224), (2000, 8192, 320, 224), (1000, 9000, 2056, 256), (2000, 2048, 4096, 256)])
+@pytest.mark.parametrize("M,N,K,width", [(257, 264, 2056, 128), (129, 9000, 1032, 128), (700, 3080, 1032, 160), (1100, 4096, 320, 160), (385, 10240, 4096, 160), (1000, 6152, 2056, 192),
+                                         (513, 4096, 320, 192), (321, 6152, 4096, 192), (640, 5120, 4096, 224), (2000, 8192, 320, 224), (1000, 9000, 2056, 256),
+                                         (2000, 2048, 320, 256), (900, 4096, 4096, 256)])
 def test_pair_tiles_of_every_width(L, M, N, K, width):
     assert L.oa_host_gemm_pair_width(M, N, K, EPI_STORE, 256) == width
     g = torch.Generator(device=dev()).manual_seed(M + N + K)
@@ -750,7 +753,8 @@ def test_decoding_rows_keep_their_bits_beside_others(L, N, K):
 # Tiles on CTA pairs with the weights' rows as their 256: every width in tokens that the rule takes, one round and several, rows and columns that end inside a tile
 # (and inside a warp's 32), a k range shorter than the ring, every epilogue; the bits of one-CTA tiles.  The width a case is for is asserted.
 @pytest.mark.parametrize("M,N,K,width", [(257, 5120, 1032, 128), (1337, 3080, 1032, 128), (321, 28672, 192, 128), (258, 9000, 320, 160), (800, 3080, 2056, 160), (130, 28672, 192, 160),
-                                         (322, 9000, 1032, 192), (513, 16384, 320, 192), (385, 9000, 2056, 224), (1537, 10240, 320, 224)])
+                                         (322, 9000, 1032, 192), (513, 16384, 320, 192), (385, 9000, 2056, 224), (1537, 10240, 320, 224),
+                                         (300, 5120, 4096, 128), (513, 8192, 1032, 160), (2000, 2048, 4096, 224)])
 def test_pair_tiles_with_the_operands_swapped(L, monkeypatch, M, N, K, width):
     assert L.oa_host_gemm_pair_swapped(M, N, K, EPI_STORE, 256) == width
     g = torch.Generator(device=dev()).manual_seed(M + N + K)
