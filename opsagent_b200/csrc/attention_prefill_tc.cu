@@ -1116,9 +1116,9 @@ cudaError_t launch_prefill_attention_tc(const CUtensorMap* tm_q, const CUtensorM
     if (p.n_tiles <= 0) return cudaSuccess;
     if (kv.page_size != 64 || p.n_heads % p.n_kv != 0) return cudaErrorInvalidValue;
     const int grp = p.n_heads / p.n_kv, items = p.n_tiles * p.n_kv * ((grp + 1) / 2), sms = prefill_sm_count();
-    const PrefillKernel k = prefill_attention_kernel_of(p.n_tiles, p.key_tiles, p.max_key_tiles, p.n_heads, p.n_kv, kv.head_dim);
-    if (k == PREFILL_TURNS_PAIR) return launch_pcp<128, 2>(tm_q, tm_kv, kv, p, sms, s);
-    if (k == PREFILL_TURNS) return launch_pcp<64, 1>(tm_q, tm_kv, kv, p, sms, s);
+    const PrefillKernel k = p.forced ? (PrefillKernel)p.forced : prefill_attention_kernel_of(p.n_tiles, p.key_tiles, p.max_key_tiles, p.n_heads, p.n_kv, kv.head_dim);
+    if (k == PREFILL_TURNS_PAIR) return kv.head_dim == 128 && grp % 2 == 0 && sms >= 2 ? launch_pcp<128, 2>(tm_q, tm_kv, kv, p, sms, s) : cudaErrorInvalidValue;
+    if (k == PREFILL_TURNS) return kv.head_dim == 64 ? launch_pcp<64, 1>(tm_q, tm_kv, kv, p, sms, s) : cudaErrorInvalidValue;
     if (k == PREFILL_TWO_HEADS) {
         if (kv.head_dim == 128) return launch_ptp<128>(tm_q, tm_kv, kv, p, items, sms, s);
         if (kv.head_dim == 64) return launch_ptp<64>(tm_q, tm_kv, kv, p, items, sms, s);

@@ -265,8 +265,10 @@ static int paged_attention(const void* q, void* out, const void* kv_cache, int32
     PrefillAttnParams a{}; a.q = q; a.out = out; a.block_tables = (const int32_t*)((const char*)d_meta.p + o_bt); a.max_pages_per_seq = max_pages_per_seq;
     a.tiles = (const PrefillTile*)((const char*)d_meta.p + o_tiles); a.n_tiles = (int)tiles.size(); a.layer = 0; a.n_heads = n_heads; a.n_kv = n_kv; a.scale_log2e = scale_log2e;
     set_key_tiles(a, tiles.data(), tiles.size());
-    const char* leg = std::getenv("OA_PREFILL_ATTN");
-    const bool legacy = leg && std::string(leg) == "legacy";
+    const char* env = std::getenv("OA_PREFILL_ATTN");            // for tests: the kernel that runs, where it takes these heads (else the call is refused)
+    const std::string which = env ? env : "";
+    const bool legacy = which == "legacy";
+    a.forced = which == "one_head" ? PREFILL_ONE_HEAD : which == "two_heads" ? PREFILL_TWO_HEADS : which == "turns" ? (head_dim == 64 ? PREFILL_TURNS : PREFILL_TURNS_PAIR) : 0;
     CUtensorMap tmq;
     if (!legacy && make_tmap_bf16_2d(&tmq, q, (uint64_t)total_q, (uint64_t)n_heads * head_dim, (uint64_t)n_heads * head_dim, 128, 64) != 0) return OA_ERR_INTERNAL;
     e = cudaMemcpyAsync(d_meta.p, host.data(), host.used, cudaMemcpyHostToDevice, s);

@@ -185,6 +185,7 @@ struct PrefillAttnParams {
     int32_t layer, n_heads, n_kv;
     float scale_log2e;
     int32_t key_tiles, max_key_tiles;      // 128-key tiles that the query tiles see, in all and at most (set_key_tiles): they choose the tcgen05 path's kernel
+    int32_t forced;                        // a PrefillKernel that runs whatever the estimate says (tests; refused where it does not take these heads), else 0
 };
 inline void set_key_tiles(PrefillAttnParams& p, const PrefillTile* host_tiles, size_t n) {
     p.key_tiles = p.max_key_tiles = 0;

@@ -282,19 +282,24 @@ def test_paged_prefill_attention(L, nh, nkv, D):
     assert err < 2e-2, err
 
 
-# few rows take the kernel of one head a CTA, whose output may only be read once its last products have landed however late their values come: one to six
-# key tiles, keys in L2 and values not, full and ragged last tiles; the bits of the two-head kernel, which the same prompt takes among copies of itself
-@pytest.mark.parametrize("nh,nkv,D", [(8, 2, 128), (16, 4, 64)])
+# prefill attention's kernels that take such heads, by the names that OA_PREFILL_ATTN asks for
+def _prefill_kernels(nh, nkv, D):
+    return ["one_head", "two_heads"] + (["turns"] if D == 64 or nh // nkv % 2 == 0 else [])
+
+
+# An output may only be read once its last products have landed, however late their values come: one to six key tiles, keys in L2 and values not, full and ragged last
+# tiles; in every kernel, a prompt alone and among copies of itself, with the same bits
+@pytest.mark.parametrize("nh,nkv,D", [(8, 2, 128), (16, 4, 64), (10, 2, 128), (15, 3, 64)])
 @pytest.mark.parametrize("ctx,rows", [(128, 128), (256, 128), (256, 100), (257, 129), (512, 32), (700, 33), (700, 200)])
-def test_prefill_output_waits_for_the_last_values(L, nh, nkv, D, ctx, rows):
+def test_prefill_output_waits_for_the_last_values(L, monkeypatch, nh, nkv, D, ctx, rows):
     pages, maxp = (ctx + 63) // 64, (ctx + 63) // 64
     kv = _mk_cache(pages, nkv, D, 41)
     g = torch.Generator(device="cpu").manual_seed(12)
     q1 = torch.randn(rows, nh, D, generator=g).to(torch.bfloat16).to(dev())
     flush = torch.empty(256 << 20, dtype=torch.uint8, device=dev())
 
-    def attend(copies):
-        assert ((rows + 127) // 128 * copies * nkv * (nh // nkv + 1) // 2 > 74) == (copies > 1)
+    def attend(copies, kernel):
+        monkeypatch.setenv("OA_PREFILL_ATTN", kernel)
         q = q1.repeat(copies, 1, 1).contiguous()
         out = torch.full_like(q, float("nan"))
         bt = np.tile(np.arange(pages, dtype=np.int32)[::-1], (copies, 1)).copy()
@@ -303,19 +308,22 @@ def test_prefill_output_waits_for_the_last_values(L, nh, nkv, D, ctx, rows):
         assert L.oa_k_paged_attention(ptr(q), ptr(out), ptr(kv), pages, bt.ctypes.data, maxp, c.ctypes.data, n.ctypes.data, copies, nh, nkv, D, 0, None) == 0, _lib.last_error()
         return out
 
-    want = attend(40)
+    want = attend(40, "two_heads")
     ref = _attn_ref(q1, kv[0], kv[1], torch.arange(pages - 1, -1, -1, device=dev())[None], [ctx], [rows], nh, nkv, D)
     # probabilities and result are rounded to bf16 (2^-9 relative each); |values| stay below 5
     assert (want[:rows].float() - ref).abs().max().item() < 2 * 5 * 2.0 ** -8
-    for _ in range(10):
-        assert torch.equal(attend(1), want[:rows])
     assert torch.equal(want, want[:rows].repeat(40, 1, 1))
+    for kernel in _prefill_kernels(nh, nkv, D):
+        for _ in range(5):
+            assert torch.equal(attend(1, kernel), want[:rows]), kernel
+        assert torch.equal(attend(40, kernel), want), kernel
 
 
-# batches that fill the chip take the two-heads-per-CTA kernel: an even and an odd number of heads per group (the last head of an odd group is
-# alone), portions behind a cached prefix, tiles of one row, key tiles whose second page is missing, and more items than CTAs
-@pytest.mark.parametrize("nh,nkv,D", [(32, 8, 128), (20, 4, 128), (32, 8, 64), (15, 3, 64), (16, 2, 128)])
-def test_paged_prefill_attention_two_heads_per_cta(L, nh, nkv, D):
+# Batches that fill the chip, in every kernel: an even and an odd number of heads per group (two heads a CTA leave the last head of an odd group alone), portions behind a
+# cached prefix, tiles of one row, key tiles whose second page is missing, and more items than CTAs
+@pytest.mark.parametrize("nh,nkv,D,kernel", [(*h, k) for h in [(32, 8, 128), (20, 4, 128), (32, 8, 64), (15, 3, 64), (16, 2, 128)] for k in _prefill_kernels(*h)])
+def test_paged_prefill_attention_of_full_batches(L, monkeypatch, nh, nkv, D, kernel):
+    monkeypatch.setenv("OA_PREFILL_ATTN", kernel)
     cases = [(64, 64), (130, 130), (200, 37), (1, 1), (700, 513), (128, 128), (65, 65), (449, 1), (333, 300), (1000, 129)] * 2
     ctx = [c for c, _ in cases]; qlens = [q for _, q in cases]
     n = len(ctx); maxp = 16; num_pages = 140
@@ -342,12 +350,12 @@ def test_paged_prefill_attention_two_heads_per_cta(L, nh, nkv, D):
     assert err < 2 * 5 * 2.0 ** -8, err
 
 
-# one head a CTA, two heads a CTA, key tiles in turns on a CTA pair (heads of 128) or a CTA (heads of 64): a batch takes the kernel that the estimate of its time names, and a row's bits are the same in all.
-# Items of one, two, three and many key tiles (the pair's warpgroups take them in turn: odd and even ends, items shorter than what is on its way), a last tile
-# without its second page, more items than CTAs, references raised in later tiles
-@pytest.mark.parametrize("nh,nkv,D", [(8, 4, 128), (16, 2, 128), (12, 4, 64), (16, 2, 64)])
+# One head a CTA, two heads a CTA, key tiles in turns on a CTA pair (heads of 128, even groups) or a CTA (heads of 64): a batch takes the kernel that the estimate of its time
+# names, and a row's bits are the same in all.  Items of one, two, three and many key tiles (in turns two warpgroups take them: odd and even ends, items shorter than what is
+# on its way), a last tile without its second page, fewer and more items than CTAs, references raised in later tiles
+@pytest.mark.parametrize("nh,nkv,D", [(8, 4, 128), (16, 2, 128), (10, 2, 128), (12, 4, 64), (16, 2, 64), (4, 4, 64)])
 @pytest.mark.parametrize("ctx,rows", [(2, 2), (64, 64), (128, 128), (129, 129), (256, 255), (384, 130), (449, 33), (1000, 130), (1280, 65)])
-def test_prefill_attention_kernels_agree(L, nh, nkv, D, ctx, rows):
+def test_prefill_attention_kernels_agree(L, monkeypatch, nh, nkv, D, ctx, rows):
     pages = (ctx + 63) // 64
     kv = _mk_cache(pages, nkv, D, 5)
     g = torch.Generator(device="cpu").manual_seed(ctx)
@@ -355,30 +363,27 @@ def test_prefill_attention_kernels_agree(L, nh, nkv, D, ctx, rows):
     q1[::5] *= 9
     q1 = q1.to(torch.bfloat16).to(dev())
 
-    def arrays(copies):
-        return np.full(copies, ctx, np.int32), np.full(copies, rows, np.int32), np.tile(np.arange(pages, dtype=np.int32)[::-1], (copies, 1)).copy()
-
-    def kernel(copies):
-        c, n, _ = arrays(copies)
-        return L.oa_host_prefill_attention_kernel(c.ctypes.data, n.ctypes.data, copies, nh, nkv, D)
-
-    first = {}
-    for copies in [1, 3, 5, 9, 17, 33, 50, 75, 101, 160, 300]:
-        first.setdefault(kernel(copies), copies)
-    assert (3 if D == 128 else 4) in first and len(first) >= (2 if D == 128 else 1)
-    outs = []
-    for copies in first.values():
+    def attend(copies, kernel):
+        if kernel:
+            monkeypatch.setenv("OA_PREFILL_ATTN", kernel)
+        else:
+            monkeypatch.delenv("OA_PREFILL_ATTN")
         q = q1.repeat(copies, 1, 1).contiguous()
         out = torch.full_like(q, float("nan"))
-        c, n, bt = arrays(copies)
-        assert L.oa_k_paged_attention(ptr(q), ptr(out), ptr(kv), pages, bt.ctypes.data, pages, c.ctypes.data, n.ctypes.data, copies, nh, nkv, D, 0, None) == 0, _lib.last_error()
-        assert torch.equal(out, out[:rows].repeat(copies, 1, 1))
-        outs.append(out[:rows])
-    for o in outs[1:]:
-        assert torch.equal(o, outs[0])
+        c, n, bt = np.full(copies, ctx, np.int32), np.full(copies, rows, np.int32), np.tile(np.arange(pages, dtype=np.int32)[::-1], (copies, 1)).copy()
+        rc = L.oa_k_paged_attention(ptr(q), ptr(out), ptr(kv), pages, bt.ctypes.data, pages, c.ctypes.data, n.ctypes.data, copies, nh, nkv, D, 0, None)
+        return out if rc == 0 else None
+
+    first = attend(1, "one_head")
     ref = _attn_ref(q1, kv[0], kv[1], torch.arange(pages - 1, -1, -1, device=dev())[None], [ctx], [rows], nh, nkv, D)
     # probabilities and result are rounded to bf16 (2^-9 relative each); |values| stay below 5
-    assert (outs[0].float() - ref).abs().max().item() < 2 * 5 * 2.0 ** -8
+    assert (first.float() - ref).abs().max().item() < 2 * 5 * 2.0 ** -8
+    kernels = _prefill_kernels(nh, nkv, D)
+    for copies in (1, 7, 75):
+        for kernel in [*kernels, None]:
+            assert torch.equal(attend(copies, kernel), first.repeat(copies, 1, 1)), (copies, kernel)
+    if "turns" not in kernels:                       # heads that a kernel does not take are refused, not given to another
+        assert attend(1, "turns") is None
 
 
 def _decode_route(L, ctx, nkv):
@@ -801,13 +806,13 @@ def test_pair_tiles_with_the_operands_swapped(L, monkeypatch, M, N, K, width):
     assert torch.equal(alone, got[0][part])
 
 
-# A prompt's attention has the same bits alone (few items: one head per CTA) and beside others (the two-heads-per-CTA kernel): both take the same keys per
-# tile, raise a row's reference maximum at the same scores and sum its exponentials in the same order.
+# A prompt's attention has the same bits alone (in the one-head kernel) and beside others (in any): all take the same keys per tile, raise a row's reference maximum at the
+# same scores and sum its exponentials in the same order.
 @pytest.mark.parametrize("nh,nkv,D", [(32, 8, 128), (20, 4, 128), (32, 8, 64), (15, 3, 64), (16, 2, 128)])
-def test_prefill_attention_keeps_its_bits_beside_others(L, nh, nkv, D):
+def test_prefill_attention_keeps_its_bits_beside_others(L, monkeypatch, nh, nkv, D):
     pairs = nkv * ((nh // nkv + 1) // 2)
     half = torch.cuda.get_device_properties(0).multi_processor_count // 2
-    few = half // pairs                                  # row tiles of a lone prompt that stay on the one-head kernel
+    few = half // pairs                                  # row tiles of a lone prompt that are all resident in the one-head kernel
     cases = [(c, min(q, 128 * few)) for c, q in [(64, 64), (130, 130), (700, 200), (513, 513), (1, 1), (999, 385), (2000, 129)]] * 2
     ctx = [c for c, _ in cases]; qlens = [q for _, q in cases]
     assert sum((q + 127) // 128 for q in qlens) * pairs > half and all((q + 127) // 128 * pairs <= half for q in qlens)
@@ -831,6 +836,10 @@ def test_prefill_attention_keeps_its_bits_beside_others(L, nh, nkv, D):
         return out
 
     whole = attend(list(range(n)), list(range(T)))
+    for kernel in _prefill_kernels(nh, nkv, D):
+        monkeypatch.setenv("OA_PREFILL_ATTN", kernel)
+        assert torch.equal(attend(list(range(n)), list(range(T))), whole), kernel
+    monkeypatch.setenv("OA_PREFILL_ATTN", "one_head")
     row0 = 0
     for i in range(n):
         if qlens[i] > 1:                                 # (a lone row is a decoding row: another kernel)
