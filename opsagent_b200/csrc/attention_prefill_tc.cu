@@ -1094,21 +1094,24 @@ static int prefill_sm_count() {
 // as many items of two heads as SMs; two heads a CTA 6.3 + 2.6 (r - 1) + 1.72 a tile on the longest CTA (5.4 + 1.9 (r - 1) + 1.72); in turns on a pair
 // 7.1 + 1.25 (r - 1) + 0.77 a tile, on a CTA 4.9 + 0.7 (r - 1) + 0.77.  Heads of 128, n = 1, 4, 11, 25: one query tile of 100 rows 5.8, 8.9, 15.9, 29.9 one head a CTA,
 // 7.5, 9.9, 14.6, 24.7 in turns; nine of them 8.6, 14.3, 26.8, 52.1 two heads a CTA, 10.4, 15.6, 26.5, 49.6.  Heads of 64, n = 1, 6, 25: one tile 5.2, 10.2, 29.9 against
-// 5.4, 9.1, 22.7, nine 7.1, 16.0, 48.2 against 7.6, 15.4, 44.5.  Ragged items: the longest CTA has the longest item at least, else the mean one a round.  The least
-// estimate was within 2 % of the fastest kernel for all but a few batches of single tiles (5 %).  A pair takes two heads of a group, so groups of 128 with an odd
-// head stay on the first two (in turns on a CTA alone they meet the L2's limit: five prompts of 1.4 thousand rows, 40 / 8 heads 126 -> 171).
-PrefillKernel prefill_attention_kernel_of(int n_tiles, int key_tiles, int max_key_tiles, int n_heads, int n_kv, int head_dim) {
+// 5.4, 9.1, 22.7, nine 7.1, 16.0, 48.2 against 7.6, 15.4, 44.5.  Ragged items: the longest CTA has the longest item at least, else the mean one a round.  Rows of a query
+// tile that are not there cost nothing where a warp has none, and that is more of an item where its output is not written under the next one: 28 prompts of 23 rows, 64 / 8
+// heads of 128, 25.5 two heads a CTA and 27.9 in turns, 20 of 128 rows 26.2 and 23.8; 40 of 20 rows, 32 / 8 heads of 64, 18.5 and 16.8, of 128 rows 22.6 and 17.5.  Over 703
+// batches of 1 to 6 key tiles the least estimate's kernel was 0.3 % above the fastest in the mean, and 2 batches (77 without that term) were more than 1.5 % slower
+// than they are without the kernels in turns.  A pair takes two heads of a group, so groups of 128 with an odd head stay on the first two (in turns on a CTA alone they meet the L2's limit: five prompts of 1.4 thousand rows, 40 / 8 heads 126 -> 171).
+PrefillKernel prefill_attention_kernel_of(int n_tiles, int key_tiles, int max_key_tiles, int rows, int n_heads, int n_kv, int head_dim) {
     const int sms = prefill_sm_count(), grp = n_heads / n_kv, items = n_tiles * n_kv * ((grp + 1) / 2);
     const bool few = items <= sms / 2, small = head_dim == 64, turns_ok = key_tiles > 0 && (small || (head_dim == 128 && grp % 2 == 0 && sms >= 2));
     // (few items of any kind: 400 rows behind 6000, 32 / 8 heads, 64 items: one head a CTA 58 us, two 91)
     const PrefillKernel plain = grp > 1 && !few ? PREFILL_TWO_HEADS : PREFILL_ONE_HEAD, turns = small ? PREFILL_TURNS : PREFILL_TURNS_PAIR;
     if (!turns_ok) return plain;
     if (grp == 1 && !few) return turns;                     // one head a CTA is for items that are all resident
-    const double mean = (double)key_tiles / n_tiles, longest = max_key_tiles;
+    const double mean = (double)key_tiles / n_tiles, longest = max_key_tiles, empty = 1.0 - rows / (128.0 * n_tiles);      // empty: rows of a query tile that are not there
     const int turn_items = small ? n_tiles * n_heads : items, turn_ctas = small ? sms : sms / 2;
     const int r_plain = (items + sms - 1) / sms, r_turns = (turn_items + turn_ctas - 1) / turn_ctas;
-    const double us_plain = few ? (small ? 4.2 : 4.9) + 1.0 * longest : (small ? 5.4 + 1.9 * (r_plain - 1) : 6.3 + 2.6 * (r_plain - 1)) + 1.72 * std::max(longest, mean * r_plain);
-    const double us_turns = (small ? 4.9 + 0.7 * (r_turns - 1) : 7.1 + 1.25 * (r_turns - 1)) + 0.77 * std::max(longest, mean * r_turns);
+    const double us_plain = few ? (small ? 4.2 : 4.9) + 1.0 * longest - 0.4 * empty
+                                : (small ? 5.4 + 1.9 * (r_plain - 1) : 6.3 + 2.6 * (r_plain - 1)) + 1.72 * std::max(longest, mean * r_plain) - (small ? 0.6 : 1.2) * r_plain * empty;
+    const double us_turns = (small ? 4.9 + 0.7 * (r_turns - 1) : 7.1 + 1.25 * (r_turns - 1)) + 0.77 * std::max(longest, mean * r_turns) - (small ? 0.05 : 0.4) * r_turns * empty;
     return us_turns < us_plain ? turns : plain;
 }
 
@@ -1116,7 +1119,7 @@ cudaError_t launch_prefill_attention_tc(const CUtensorMap* tm_q, const CUtensorM
     if (p.n_tiles <= 0) return cudaSuccess;
     if (kv.page_size != 64 || p.n_heads % p.n_kv != 0) return cudaErrorInvalidValue;
     const int grp = p.n_heads / p.n_kv, items = p.n_tiles * p.n_kv * ((grp + 1) / 2), sms = prefill_sm_count();
-    const PrefillKernel k = p.forced ? (PrefillKernel)p.forced : prefill_attention_kernel_of(p.n_tiles, p.key_tiles, p.max_key_tiles, p.n_heads, p.n_kv, kv.head_dim);
+    const PrefillKernel k = p.forced ? (PrefillKernel)p.forced : prefill_attention_kernel_of(p.n_tiles, p.key_tiles, p.max_key_tiles, p.rows, p.n_heads, p.n_kv, kv.head_dim);
     if (k == PREFILL_TURNS_PAIR) return kv.head_dim == 128 && grp % 2 == 0 && sms >= 2 ? launch_pcp<128, 2>(tm_q, tm_kv, kv, p, sms, s) : cudaErrorInvalidValue;
     if (k == PREFILL_TURNS) return kv.head_dim == 64 ? launch_pcp<64, 1>(tm_q, tm_kv, kv, p, sms, s) : cudaErrorInvalidValue;
     if (k == PREFILL_TWO_HEADS) {

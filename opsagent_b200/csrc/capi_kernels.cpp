@@ -194,13 +194,13 @@ int oa_host_gemm_pair_width(int32_t M, int32_t N, int32_t K, int32_t epilogue, i
 
 int oa_host_prefill_attention_kernel(const int32_t* ctx_lens, const int32_t* q_lens, int32_t n_seqs, int32_t n_heads, int32_t n_kv, int32_t head_dim) {
     if (n_seqs < 0 || n_kv <= 0 || n_heads <= 0 || n_heads % n_kv != 0) return OA_ERR_BAD_REQUEST;
-    int n_tiles = 0, sum = 0, longest = 0;
+    int n_tiles = 0, sum = 0, longest = 0, rows = 0;
     for (int i = 0; i < n_seqs; ++i)
         for (int r = 0; r < q_lens[i]; r += PREFILL_TILE_ROWS) {
             const int k = (ctx_lens[i] - q_lens[i] + std::min(r + PREFILL_TILE_ROWS, q_lens[i]) + 127) / 128;
-            ++n_tiles; sum += k; longest = std::max(longest, k);
+            ++n_tiles; sum += k; longest = std::max(longest, k); rows += std::min(PREFILL_TILE_ROWS, q_lens[i] - r);
         }
-    return (int)prefill_attention_kernel_of(n_tiles, sum, longest, n_heads, n_kv, head_dim);
+    return (int)prefill_attention_kernel_of(n_tiles, sum, longest, rows, n_heads, n_kv, head_dim);
 }
 
 int oa_host_gemm_pair_swapped(int32_t M, int32_t N, int32_t K, int32_t epilogue, int32_t block_n) {

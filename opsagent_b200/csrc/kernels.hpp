@@ -184,18 +184,18 @@ struct PrefillAttnParams {
     const PrefillTile* tiles; int32_t n_tiles;
     int32_t layer, n_heads, n_kv;
     float scale_log2e;
-    int32_t key_tiles, max_key_tiles;      // 128-key tiles that the query tiles see, in all and at most (set_key_tiles): they choose the tcgen05 path's kernel
+    int32_t key_tiles, max_key_tiles, rows;      // 128-key tiles that the query tiles see, in all and at most, and query rows (set_key_tiles): they choose the tcgen05 path's kernel
     int32_t forced;                        // a PrefillKernel that runs whatever the estimate says (tests; refused where it does not take these heads), else 0
 };
 inline void set_key_tiles(PrefillAttnParams& p, const PrefillTile* host_tiles, size_t n) {
-    p.key_tiles = p.max_key_tiles = 0;
+    p.key_tiles = p.max_key_tiles = p.rows = 0;
     for (size_t i = 0; i < n; ++i) {
         const int k = (host_tiles[i].pos0 + host_tiles[i].n_rows + 127) / 128;
-        p.key_tiles += k; if (k > p.max_key_tiles) p.max_key_tiles = k;
+        p.key_tiles += k; p.rows += host_tiles[i].n_rows; if (k > p.max_key_tiles) p.max_key_tiles = k;
     }
 }
 enum PrefillKernel : int { PREFILL_ONE_HEAD = 1, PREFILL_TWO_HEADS = 2, PREFILL_TURNS_PAIR = 3, PREFILL_TURNS = 4 };      // the same bits in all of them
-PrefillKernel prefill_attention_kernel_of(int n_tiles, int key_tiles, int max_key_tiles, int n_heads, int n_kv, int head_dim);
+PrefillKernel prefill_attention_kernel_of(int n_tiles, int key_tiles, int max_key_tiles, int rows, int n_heads, int n_kv, int head_dim);
 cudaError_t launch_prefill_attention(const CUtensorMap* tm_kv, const KvLayout& kv, const PrefillAttnParams& p, cudaStream_t s);   // legacy mma.sync path
 // tcgen05 path (attention_prefill_tc.cu): tm_q = box {64 cols, 128 rows} over q[T, nh*D]
 cudaError_t launch_prefill_attention_tc(const CUtensorMap* tm_q, const CUtensorMap* tm_kv, const KvLayout& kv, const PrefillAttnParams& p, cudaStream_t s);

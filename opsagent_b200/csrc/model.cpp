@@ -485,7 +485,7 @@ void DeviceModel::forward(const StepInput& in, float* logits_out) {
         if (!in.decode && !in.tiles.empty()) {     // mixed step: both kernels, disjoint rows of q_/attn_
             PrefillAttnParams a{}; a.q = q_; a.out = attn_; a.block_tables = d_bt; a.max_pages_per_seq = max_pages_per_seq;
             a.tiles = reinterpret_cast<const PrefillTile*>(d_meta_ + o_tiles); a.n_tiles = (int)in.tiles.size();
-            a.layer = l; a.n_heads = nh; a.n_kv = nkv; a.scale_log2e = scale_log2e; a.key_tiles = key_tiles.key_tiles; a.max_key_tiles = key_tiles.max_key_tiles;
+            a.layer = l; a.n_heads = nh; a.n_kv = nkv; a.scale_log2e = scale_log2e; a.key_tiles = key_tiles.key_tiles; a.max_key_tiles = key_tiles.max_key_tiles; a.rows = key_tiles.rows;
             static const bool legacy = [] { const char* e = std::getenv("OA_PREFILL_ATTN"); return e && std::string(e) == "legacy"; }();
             if (legacy) cuda_check(launch_prefill_attention(&tm_kv, kv, a, stream), "prefill attention (mma.sync)");
             else cuda_check(launch_prefill_attention_tc(&tm_q_, &tm_kv, kv, a, stream), "prefill attention (tcgen05)");

@@ -772,6 +772,21 @@ def test_operands_are_swapped_only_where_that_shortens_a_pairs_work():
     assert lib.oa_host_gemm_kernel(300, 28672, 4096, 2, 256, 0, 1) == 2                              # grouped products keep tiles of one CTA
 
 
+# Prefill attention (1 one head a CTA, 2 two heads, 3 and 4 key tiles in turns): query tiles of few rows in batches of single key tiles are sooner done two heads a
+# CTA (3 to 9 % of the kernel's time), full ones in turns; heads of 128 and of 64, an odd group
+def test_which_attention_kernel_a_batch_of_prompts_takes():
+    lib = _lib.load()
+
+    def kernel(n, rows, past, heads):
+        q = np.full(n, rows, np.int32); ctx = q + np.int32(past)
+        return lib.oa_host_prefill_attention_kernel(ctx.ctypes.data, q.ctypes.data, n, *heads)
+
+    for n, rows, past, heads, want in [(28, 23, 0, (64, 8, 128), 2), (45, 20, 0, (16, 2, 128), 2), (13, 18, 60, (32, 8, 128), 2), (36, 5, 100, (64, 8, 128), 2), (20, 128, 0, (64, 8, 128), 3),
+                                       (40, 128, 0, (32, 8, 128), 3), (5, 1400, 0, (32, 8, 128), 3), (1, 4096, 12288, (64, 8, 128), 3), (5, 1400, 0, (40, 8, 128), 2), (2, 100, 0, (40, 8, 128), 1),
+                                       (7, 20, 0, (32, 8, 64), 2), (7, 128, 128, (32, 8, 64), 4), (40, 20, 0, (32, 8, 64), 4), (2, 100, 0, (32, 8, 64), 1), (2, 100, 500, (32, 8, 64), 4)]:
+        assert kernel(n, rows, past, heads) == want, (n, rows, past, heads)
+
+
 @pytest.mark.parametrize("value,kernel", [("0", 0), ("1", 3)])
 def test_the_switch_that_turns_persistent_products_off(value, kernel):
     """OA_GEMM_PERSISTENT=0: one CTA per tile for every product, also for those that CTA pairs would take"""
