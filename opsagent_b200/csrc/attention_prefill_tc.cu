@@ -670,8 +670,8 @@ __global__ void __launch_bounds__(PtpCfg<D>::THREADS, 1) prefill_attention_pair_
 // the five prompts 85.6 -> 76.5, 1400 rows behind 3000 93 -> 72, 600 rows 13.0 -> 8.9, 100 rows behind 3000 29.9 (one head a CTA) -> 22.7.
 // What bounds it now (128): a warpgroup takes 2600 cycles a tile, 1650 of them exponentials (1024 alone), 550 fetching S, the maxima and the reference, 120 waiting
 // for S; tensor and special-function pipes are busy 79 %, and the clock is down to 1.6 GHz in the long case (1.76 in the short ones).
-// Waits and arrivals are of CTA scope: what crosses the pair stands in TMEM (ordered by tcgen05.fence) or comes by TMA; with acquire and release of cluster
-// scope a tile took 2100 cycles instead of 1300.  Slower: S of two tiles and P of two in places of their own, S issued as soon as it is fetched (84 -> 90 us),
+// What crosses the pair stands in TMEM, ordered by tcgen05.fence, or comes by TMA: arrivals and waits for TMEM are relaxed, of cluster scope; only the loading and the issuing
+// warp acquire.  With the softmax warps' arrivals as releases a tile took 2100 cycles instead of 1300: each waits for its thread's stores.  Slower: S of two tiles and P of two in places of their own, S issued as soon as it is fetched (84 -> 90 us),
 // P handed over in two halves (85.5); no faster: the first item and its pages looked up ahead of the set-up.
 // ---------------------------------------------------------------------------------------------
 template <int D, int CTAS>
@@ -738,6 +738,9 @@ __global__ void __launch_bounds__(PcpCfg<D, CTAS>::THREADS, 1) prefill_attention
     const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // warp: uniform, and known to be
     const uint32_t rank = PAIR ? gp_rank() : 0;
     const int grp = p.n_heads / p.n_kv;
+    // barriers that the pair shares: of loads and freed shared memory, and of what stands in TMEM
+    auto wait_smem = [&](uint64_t* bar, uint32_t parity) { if (PAIR) gp_wait(bar, parity); else mbar_wait(bar, parity); };
+    auto wait_tmem = [&](uint64_t* bar, uint32_t parity) { if (PAIR) gp_wait_tmem(bar, parity); else mbar_wait(bar, parity); };
     auto arrive_even = [&](uint64_t* bar) { if (PAIR) gp_arrive_tmem(gp_mapa(bar, 0)); else mbar_arrive(bar); };
     PcpItem it;
 
@@ -779,7 +782,7 @@ __global__ void __launch_bounds__(PcpCfg<D, CTAS>::THREADS, 1) prefill_attention
                 int64_t r0 = page_row(0, 0), r1 = page_row(1, 0);
                 for (int j = 0; j < n_kvt; ++j, ++kc) {
                     const uint32_t st = kc % STAGES, ph = (kc / STAGES) & 1;
-                    mbar_wait(&k_empty[st], ph ^ 1);
+                    wait_smem(&k_empty[st], ph ^ 1);
                     if (elect_one()) {
                         uint8_t* dst = k_s + st * Cfg::KV_BYTES;
                         if (rank == 0) mbar_expect_tx(&k_full[st], CTAS * Cfg::KV_BYTES);           // both CTAs' shares
@@ -798,7 +801,7 @@ __global__ void __launch_bounds__(PcpCfg<D, CTAS>::THREADS, 1) prefill_attention
                     __syncwarp();
                     if (j == 0) {
                         const int qb = r & 1;
-                        mbar_wait(&q_empty[qb], (((uint32_t)r >> 1) & 1) ^ 1);
+                        wait_smem(&q_empty[qb], (((uint32_t)r >> 1) & 1) ^ 1);
                         if (elect_one()) {
                             uint8_t* dst = q_s + qb * Cfg::Q_BYTES;
                             if (rank == 0) mbar_expect_tx(&q_full[qb], CTAS * Cfg::Q_BYTES);
@@ -814,7 +817,7 @@ __global__ void __launch_bounds__(PcpCfg<D, CTAS>::THREADS, 1) prefill_attention
                     }
                     int64_t n0 = r0, n1 = r1;                                  // the next tile's pages are looked up while this one's slot is waited for
                     if (j + 1 < n_kvt) { n0 = page_row(2 * j + 2, 0); n1 = page_row(2 * j + 3, 2 * j + 2); }
-                    mbar_wait(&v_empty[st], ph ^ 1);
+                    wait_smem(&v_empty[st], ph ^ 1);
                     if (elect_one()) {
                         uint8_t* dst = v_s + st * Cfg::KV_BYTES;
                         if (rank == 0) mbar_expect_tx(&v_full[st], CTAS * Cfg::KV_BYTES);
@@ -833,8 +836,8 @@ __global__ void __launch_bounds__(PcpCfg<D, CTAS>::THREADS, 1) prefill_attention
                     r0 = n0; r1 = n1;
                 }
             }
-            for (int i = 0; i < STAGES; ++i, ++kc) { mbar_wait(&k_empty[kc % STAGES], ((kc / STAGES) & 1) ^ 1); mbar_wait(&v_empty[kc % STAGES], ((kc / STAGES) & 1) ^ 1); }   // the last
-            for (int i = 0; i < 2; ++i, ++r) mbar_wait(&q_empty[r & 1], (((uint32_t)r >> 1) & 1) ^ 1);                  // releases have arrived here before the CTA may go
+            for (int i = 0; i < STAGES; ++i, ++kc) { wait_smem(&k_empty[kc % STAGES], ((kc / STAGES) & 1) ^ 1); wait_smem(&v_empty[kc % STAGES], ((kc / STAGES) & 1) ^ 1); }   // the last
+            for (int i = 0; i < 2; ++i, ++r) wait_smem(&q_empty[r & 1], (((uint32_t)r >> 1) & 1) ^ 1);                  // releases have arrived here before the CTA may go
         } else if (warp == 1 && rank == 0) {
             // The whole warp walks the loop, an elected lane issues: descriptors stay in uniform registers.  S runs two tiles ahead of P V, across items.
             constexpr uint32_t idesc_s = umma_idesc_bf16(128 * CTAS, KV_TILE), idesc_o = umma_idesc_bf16_bmn(128 * CTAS, D);
@@ -847,9 +850,9 @@ __global__ void __launch_bounds__(PcpCfg<D, CTAS>::THREADS, 1) prefill_attention
             int s_n = s_more ? __shfl_sync(0xffffffffu, s_it.n_kvt, 0) : 0;
             auto issue_s = [&] {
                 if (!s_more) return;
-                if (s_j == 0) mbar_wait(&q_full[s_r & 1], ((uint32_t)s_r >> 1) & 1);
+                if (s_j == 0) wait_smem(&q_full[s_r & 1], ((uint32_t)s_r >> 1) & 1);
                 const uint32_t st = sc % STAGES;
-                mbar_wait(&k_full[st], (sc / STAGES) & 1);
+                wait_smem(&k_full[st], (sc / STAGES) & 1);
                 tcgen05_fence_after();
                 if (elect_one()) {
                     const uint64_t a = q_desc + (uint64_t)((s_r & 1) * (Cfg::Q_BYTES >> 4)), b = k_desc + (uint64_t)(st * (Cfg::KV_BYTES >> 4));
@@ -880,9 +883,9 @@ __global__ void __launch_bounds__(PcpCfg<D, CTAS>::THREADS, 1) prefill_attention
                 for (int j = 0; j < n_kvt; ++j, ++t) {
                     issue_s();                                                 // over the P of tile t - 1, whose product is ahead of it
                     const uint32_t st = t % STAGES;
-                    if (j == 0) mbar_wait(o_empty, ((uint32_t)r & 1) ^ 1);       // O of the last item has been read
-                    mbar_wait(&v_full[st], (t / STAGES) & 1);
-                    mbar_wait(&p_full[t % Cfg::S_BUFS], (t / Cfg::S_BUFS) & 1);
+                    if (j == 0) wait_tmem(o_empty, ((uint32_t)r & 1) ^ 1);       // O of the last item has been read
+                    wait_smem(&v_full[st], (t / STAGES) & 1);
+                    wait_tmem(&p_full[t % Cfg::S_BUFS], (t / Cfg::S_BUFS) & 1);
                     tcgen05_fence_after();
                     if (elect_one()) {
                         const uint64_t b = v_desc + (uint64_t)(st * (Cfg::KV_BYTES >> 4));
@@ -919,7 +922,7 @@ __global__ void __launch_bounds__(PcpCfg<D, CTAS>::THREADS, 1) prefill_attention
             for (int j = 0; j < n_kvt; ++j, ++t) {
                 if ((int)(t & 1) != w) continue;
                 const uint32_t s_addr = lane_base + (t % Cfg::S_BUFS) * 128;
-                mbar_wait(&s_full[t % 6], (t / 6) & 1);
+                wait_tmem(&s_full[t % 6], (t / 6) & 1);
                 tcgen05_fence_after();
                 uint32_t v[4][32];
 #pragma unroll
@@ -951,7 +954,7 @@ __global__ void __launch_bounds__(PcpCfg<D, CTAS>::THREADS, 1) prefill_attention
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&r_full[w * 4 + q]);
                 if (j > 0 && __any_sync(0xffffffffu, raise)) {
-                    mbar_wait(&v_empty[(t - 1) % STAGES], ((t - 1) / STAGES) & 1);    // O holds every tile before this one (S_t says that P V of t - 3 has landed: no earlier phase is taken for this)
+                    wait_tmem(&v_empty[(t - 1) % STAGES], ((t - 1) / STAGES) & 1);    // O holds every tile before this one (S_t says that P V of t - 3 has landed: no earlier phase is taken for this)
                     tcgen05_fence_after();
                     const float alpha = raise ? exp2f(m_last - mx) : 1.0f;
 #pragma unroll 1
@@ -1010,7 +1013,7 @@ __global__ void __launch_bounds__(PcpCfg<D, CTAS>::THREADS, 1) prefill_attention
             const float inv = 1.0f / (sum_s[row] + sum_s[128 + row]);
             __syncwarp();
             if (lane == 0) mbar_arrive(l_empty);
-            mbar_wait(o_full, (uint32_t)r & 1);
+            wait_tmem(o_full, (uint32_t)r & 1);
             tcgen05_fence_after();
 #pragma unroll
             for (int c = 0; c < D; c += 32) {

@@ -38,8 +38,20 @@ OA_DEVINL void gp_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
 }
 OA_DEVINL void gp_arrive_remote(uint32_t bar) { asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory"); }
-// the same where what is handed over stands in TMEM alone: tcgen05.fence orders that, and nothing else has to be made visible to the cluster
-OA_DEVINL void gp_arrive_tmem(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory"); }
+// The same where what is handed over stands in TMEM alone: tcgen05.fence ahead of the arrival and behind the wait orders it, so arrival and wait order execution, in
+// the cluster's scope, and make no other memory visible (a release there waits for all of the thread's stores)
+OA_DEVINL void gp_arrive_tmem(uint32_t bar) { asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory"); }
+OA_DEVINL void gp_wait_tmem(uint64_t* bar, uint32_t parity) {
+    uint32_t spins = 0, ok;
+    do {
+        asm volatile(
+            "{\n\t.reg .pred P;\n\t"
+            "mbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 P, [%1], %2;\n\t"
+            "selp.b32 %0, 1, 0, P;\n\t}"
+            : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+        if (!ok && ++spins > OA_MBAR_SPIN_LIMIT) { __trap(); }
+    } while (!ok);
+}
 // as mbar_wait, for barriers the other CTA arrives on
 OA_DEVINL void gp_wait(uint64_t* bar, uint32_t parity) {
     uint32_t spins = 0, ok;
