@@ -680,7 +680,7 @@ struct PcpCfg {
     static constexpr int S_BUFS = 3;
     static constexpr int Q_BYTES = 128 * D * 2, Q_HALF = 128 * 128;
     static constexpr int KV_BYTES = 128 / CTAS * D * 2, K_HALF = 128 / CTAS * 128;      // a CTA's share of a K or V tile of 128 keys (of a pair: 64 keys x 128, 128 keys x 64 columns)
-    static constexpr int STAGES = KV_BYTES > 16384 ? 2 : 4;
+    static constexpr int STAGES = 4;                                     // of 16 KB each
     static constexpr int OUT_WARP_BYTES = 32 * D * 2;
     static constexpr int ROWS_BYTES = 2 * 128 * 4;                       // one value per row and softmax warpgroup
     static constexpr int SMEM_BYTES = 2 * Q_BYTES + 2 * STAGES * KV_BYTES + 4 * OUT_WARP_BYTES + 2 * ROWS_BYTES + 512;

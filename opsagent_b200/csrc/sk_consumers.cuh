@@ -156,9 +156,6 @@ OA_DEVINL void sk_finish8_bf16(bool biased, const uint4& bb, float (&v)[8]) {
 #pragma unroll
     for (int k = 0; k < 8; ++k) v[k] = bf16_bits_to_f32(f32_to_bf16_bits(v[k]));
 }
-OA_DEVINL void sk_finish8_bf16(const uint16_t* bias, int col, float (&v)[8]) {
-    sk_finish8_bf16(bias != nullptr, bias ? *reinterpret_cast<const uint4*>(bias + col) : make_uint4(0, 0, 0, 0), v);
-}
 
 OA_DEVINL int sk_rope_items_per_row(const SkRopeArgs& a) { return (a.nh + a.nkv) * (a.D >> 4) + a.nkv * (a.D >> 3); }
 // item w of token row t: w < (nh+nkv)*D/16 rotates 8 (lo, hi) pairs of one q or k head; the rest copy 8 elements of v.  Slot, position, the rotation's factors and the
