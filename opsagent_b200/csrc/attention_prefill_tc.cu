@@ -1,6 +1,10 @@
 // attention_prefill_tc.cu — causal prefill attention over the paged KV cache on the 5th-generation tensor cores.
 //
-// One CTA = 128 query rows of one (sequence, head); KV is consumed in tiles of 128 tokens (two 64-token pages):
+// Three kernels with one order of a row's sums, so one result; prefill_attention_kernel_of() at the end of the file chooses by the batch: one head a CTA (few short items),
+// two heads a CTA (short query tiles, odd groups of heads of 128) and, for most batches, one head a CTA whose softmax warpgroups take the key tiles in turn, on
+// pairs of CTAs for heads of 128.
+//
+// The first.  One CTA = 128 query rows of one (sequence, head); KV is consumed in tiles of 128 tokens (two 64-token pages):
 //   warp 0    : TMA producer — Q tile once, then the K pages of a KV tile and the V pages of the one before it.  K and V have SEPARATE
 //               2-stage rings: K_j is released as soon as S_j has been computed, V_j only after P_j·V_j, so the K load of tile
 //               j+2 gets a full tile period of slack instead of being exposed behind the second MMA
@@ -337,7 +341,7 @@ __global__ void __launch_bounds__(64 + 128 * NWG, 1) prefill_attention_tc_kernel
 }
 
 // ---------------------------------------------------------------------------------------------
-// Two heads of one key/value group per CTA, for batches that fill the chip.
+// Two heads of one key/value group per CTA, for batches of short query tiles that fill the chip and for odd groups of heads of 128.
 //
 // One query tile's chain per KV tile — S, maximum, 128 exponentials a row, P, P·V — keeps either the tensor pipe or the softmax warps waiting
 // (30 % of the tensor pipe at prompts of 1.5 thousand tokens).  Here a CTA carries the SAME 128 query rows of TWO heads that read the same keys
@@ -351,11 +355,11 @@ __global__ void __launch_bounds__(64 + 128 * NWG, 1) prefill_attention_tc_kernel
 //   warp 0    : TMA (K, Q, V)        warp 1 : tcgen05.mma        warps 4-7 / 8-11 : softmax and output of head A / B, one query row per thread
 // A group with an odd number of heads leaves its last one alone in an item (warpgroup B idles).
 // A row's scores, reference maxima, probabilities and sums are those of the kernel above, in its order: which of the two a batch takes moves no bit.
-// Measured against the kernel above: 4096 rows behind 12288 cached ones, 64 / 8 heads of 128: 1963 -> 1416 us in a burst; five prompts of 1.4 thousand rows,
-// 32 / 8 heads: 184 -> 102 us.  Of that: the issuing warp stays converged (behind one lane its 32 products a tile pair took longer than the tensor core
+// Measured against the kernel above: 4096 rows behind 12288 cached ones, 64 / 8 heads of 128: 1664 -> 1348 us in a burst; five prompts of 1.4 thousand rows,
+// 32 / 8 heads: 147 -> 95 us (40 / 8: 180 -> 129).  Before two probabilities an addition, 1963 -> 1416 and 184 -> 102; of that: the issuing warp stays converged (behind one lane its 32 products a tile pair took longer than the tensor core
 // has for them): 1548 -> 1489 and 120 -> 114 us; P is handed over in two parts, so that the first 64 keys are multiplied under the other exponentials:
 // -> 1417 and 108 us (three or four parts, or loading S in two halves under the maxima: no difference); O leaves in whole lines and the next item
-// is read under the last product: -> 1416 and 102 us.  What bounds it now is a head's chain in a tile, 2900 cycles: 125 to fetch S, 275 for the
+// is read under the last product: -> 1416 and 102 us.  What bounds it is a head's chain in a tile, 2900 cycles then: 125 to fetch S, 275 for the
 // maximum, 1500 for 128 exponentials a row (1024 alone on the special-function units, which the other head's overlap in part), 970 for the rest of P·V
 // and the next S.  Tensor and special-function pipes are busy 65 to 70 % of it, and a long loop runs into the 1000 W cap.  Taking exponentials from a reference
 // that may still rise, moving an eighth or a quarter of them to the FMA pipe and two threads per row were each 3 to 12 % slower.
@@ -665,9 +669,9 @@ __global__ void __launch_bounds__(PtpCfg<D>::THREADS, 1) prefill_attention_pair_
 //   warp 0     : TMA: this CTA's Q (two items ahead), its share of K and V       warp 1 (of a pair: the even CTA's): tcgen05.mma
 //   warps 4-11 : softmax of even and odd tiles, one query row per thread         warps 12-15: output, while the next item's tiles run
 // A row's sums are kept per warpgroup (even and odd tiles of the item) and joined at its end, as in the kernels above: the same bits.
-// us, two heads a CTA -> here: 4096 rows behind 12288, 64 / 8 heads of 128 1410 -> 1302; five prompts of 1.4 thousand rows, 32 / 8 heads of 128 97 -> 84; 1000 rows
-// behind 6000 104 -> 88; 600 rows 14.7 -> 11.2 (one head a CTA: 14.7); 300 rows behind 6000 57 -> 46 (one head a CTA).  A pair's launch costs 2 us more.  Heads of 64:
-// the five prompts 85.6 -> 76.5, 1400 rows behind 3000 93 -> 72, 600 rows 13.0 -> 8.9, 100 rows behind 3000 29.9 (one head a CTA) -> 22.7.
+// us, kernels alone, two heads a CTA -> here: 4096 rows behind 12288, 64 / 8 heads of 128 1348 -> 1291; five prompts of 1.4 thousand rows, 32 / 8 heads of 128 95 -> 87;
+// 1000 rows behind 6000 100 -> 89; 600 rows 14.7 -> 11.2 (one head a CTA: 14.7); 300 rows behind 6000 57 -> 46 (one head a CTA).  A pair's launch costs 2 us more.
+// Heads of 64: the five prompts 87 -> 78, 1400 rows behind 3000 94 -> 73, 600 rows 13.0 -> 8.9, 100 rows behind 3000 29.9 (one head a CTA) -> 22.7.
 // What bounds it now (128): a warpgroup takes 2600 cycles a tile, 1650 of them exponentials (1024 alone), 550 fetching S, the maxima and the reference, 120 waiting
 // for S; tensor and special-function pipes are busy 79 %, and the clock is down to 1.6 GHz in the long case (1.76 in the short ones).
 // What crosses the pair stands in TMEM, ordered by tcgen05.fence, or comes by TMA: arrivals and waits for TMEM are relaxed, of cluster scope; only the loading and the issuing

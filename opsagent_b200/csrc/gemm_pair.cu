@@ -2,7 +2,7 @@
 //
 // The two CTAs of a cluster (two SMs of one TPC) share one 256 x bn output tile: each holds its own 128 rows of one operand (U) and HALF of the bn rows of the
 // other (V) in shared memory, and one thread of the even CTA issues 256 x bn x 16 products that read both halves.  U is A (the tokens) and bn 128, 160, .. 256, or
-// U is B (the weights) and bn 160, 192, .. 256 tokens, whichever fills the last round better.  Against a 128 x 256 tile per SM that is 2/3
+// U is B (the weights) and bn as many tokens, whichever leaves a pair less to multiply (gemm_pair_width).  Against a 128 x 256 tile per SM that is 2/3
 // of the shared-memory reads and of the L2 traffic per product.  Large products run against the 1000 W cap here (85 % of the tensor peak at a clock that is
 // down to 1.25 GHz), so what counts there is the energy per product: 8192 x 28672 x 4096 gated 1505 us a call in a loop on 128 x 256 tiles, 1445 on pairs.
 // The width is what fills the last round: 1337 x 4096 x 14336 (residual) is 96 tiles of 256 columns, two rounds of 74 pairs of which the second is a third
@@ -24,12 +24,12 @@ namespace oa {
 
 static constexpr int GP_BK = 64, GP_THREADS = 192, GP_MAX_STAGES = 8, GP_ACC_COLS = 256, GP_BAR_BYTES = 256;
 static constexpr int GP_A_BYTES = 128 * GP_BK * 2;
-// a stage: this CTA's 128 rows of A and half of the tile's bn rows of B; as many stages as fit
+// a stage: this CTA's 128 rows of U and half of the tile's bn rows of V; as many stages as fit
 struct PairRing { int bn, stages; };
 static int gp_stage_bytes(int bn) { return GP_A_BYTES + bn / 2 * GP_BK * 2; }
 static int gp_smem_bytes(const PairRing& r) { return r.stages * gp_stage_bytes(r.bn) + 4 * EPI_WARP_BYTES + GP_BAR_BYTES; }
 static PairRing gp_ring(int bn) { return PairRing{bn, std::min(GP_MAX_STAGES, (232448 - 4 * EPI_WARP_BYTES - GP_BAR_BYTES) / gp_stage_bytes(bn))}; }
-static constexpr int GP_GROUP_M = RASTER_GROUP_M / 2;           // a band of row tiles whose A rows stay in L2
+static constexpr int GP_GROUP_M = RASTER_GROUP_M / 2;           // a band of tiles whose rows of U stay in L2
 
 // SWAPPED: the weights' rows are the 256 of a tile (operand U) and the tokens its bn (operand V); else the other way round
 template <int EPI, bool SWAPPED>
