@@ -539,10 +539,10 @@ def test_prompt_fixtures_are_the_reference_constants_verbatim():
         assert len(raw) == meta["bytes"] and hashlib.sha256(raw).hexdigest() == meta["sha256"], name
         if name in want:
             assert len(raw) == want[name]
-    if os.path.isdir("/root/reference/pkg"):
-        sys.path.insert(0, PROMPTS_DIR)
-        import extract_prompts
-        for name, (text, _where, _use) in extract_prompts.extract("/root/reference").items():
+    sys.path.insert(0, PROMPTS_DIR)
+    import extract_prompts
+    if os.path.isdir(os.path.join(extract_prompts.REF, "pkg")):
+        for name, (text, _where, _use) in extract_prompts.extract(extract_prompts.REF).items():
             assert open(os.path.join(PROMPTS_DIR, name + ".txt"), "rb").read() == text.encode("utf-8"), name
 
 
