@@ -75,21 +75,19 @@ OA_DEVINL void sk_sum8_pair(const StreamK& sk, const SkCols& at_a, const SkCols&
 // x[t,:] += sum of partials (bf16 residual stream), y[t,:] = rmsnorm(x[t,:]) * g.  SK_RESID_THREADS threads (tid) per row, so that
 // at H <= 4096 every thread owns ONE 16-byte item and all its partial loads are in flight together; `red` = 16 floats of
 // shared memory, `bar_id` = a hardware barrier those threads own.  Waits for the kernel ahead (griddep_wait) once the gains are on their way.
+// us a decoding step of four layers, 1 and 32 requests: without that 282.6 and 286.1 (1B sizes, ten partials a column), 480 and 520 (8B, five); with it 280.6 and 284.0,
+// 478 and 515; with the partials' places found ahead of the wait, too, 289.1 and 295.7, 478 and 513.
 constexpr int SK_RESID_THREADS = 512;
 template <int VPT, bool SUM = true>     // SUM == false: the residual stream already holds x + projection (fused GEMM epilogue); only normalise
 OA_DEVINL void sk_resid_rmsnorm_row(const StreamK& sk, int t, int tid, float* red, int bar_id, uint4* __restrict__ x,
                                     const uint4* __restrict__ g, uint4* __restrict__ y, int H8, float inv_h, float eps) {
     uint4* xr = x + (size_t)t * H8;
     uint4 v[VPT], gg[VPT];
-    SkCols at[VPT];
     float ss = 0.f;
 #pragma unroll
     for (int k = 0; k < VPT; ++k) {
         const int i = tid + k * SK_RESID_THREADS;
-        if (i < H8) {
-            gg[k] = g[i];
-            if constexpr (SUM) at[k] = sk_locate(sk, t, i * 8);
-        }
+        if (i < H8) gg[k] = g[i];
     }
     griddep_wait();
 #pragma unroll
@@ -100,7 +98,7 @@ OA_DEVINL void sk_resid_rmsnorm_row(const StreamK& sk, int t, int tid, float* re
             uint4 xn = xo;
             if constexpr (SUM) {
                 float acc[8];
-                sk_sum8(sk, at[k], acc);
+                sk_sum8(sk, t, i * 8, acc);            // (its places found here: kept across the wait they cost 38 of 78 registers, and so the loads in flight)
                 xn.x = pack_bf16x2(bf16lo(xo.x) + acc[0], bf16hi(xo.x) + acc[1]); xn.y = pack_bf16x2(bf16lo(xo.y) + acc[2], bf16hi(xo.y) + acc[3]);
                 xn.z = pack_bf16x2(bf16lo(xo.z) + acc[4], bf16hi(xo.z) + acc[5]); xn.w = pack_bf16x2(bf16lo(xo.w) + acc[6], bf16hi(xo.w) + acc[7]);
                 xr[i] = xn;
