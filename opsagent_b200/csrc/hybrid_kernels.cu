@@ -658,8 +658,9 @@ __global__ void __launch_bounds__(128) hy_mla_decode_mma_kernel(HyLatentAttn a, 
 }
 
 // joins the parts of a decoding row: out = sum_p 2^(m_p - M) O_p / sum_p 2^(m_p - M) l_p, parts in order
-// Four channels a thread, all parts' loads in flight: a row's items come from the host and are read ahead of the wait.  (A channel a thread and its parts one
-// behind the other: 4.6 us for 16 rows of two parts, 16 heads of 512 channels, against 3.4.)
+// Four channels a thread, four parts' loads in flight: a row's items come from the host and are read ahead of the wait.  us, a channel a thread and its parts one behind the
+// other / eight parts at once / four: 64 rows of 700 tokens, 16 heads of 256 and of 512 channels, 4.6 / 7.3 / 4.2 and 6.0 / 8.2 / 5.1 (eight take 80 registers, so six CTAs
+// an SM, and a thousand CTAs come twice; four take 48); 16 rows of 300 3.9 / 3.7 / 3.5; four rows 4.7 / 3.8 / 3.8; one of 900 4.3 / 4.6 / 3.3.
 __global__ void __launch_bounds__(128) hy_mla_merge_kernel(const int32_t* __restrict__ item_row, const int32_t* __restrict__ item_slot0, const int32_t* __restrict__ item_parts,
                                                            const float* __restrict__ ws_o, const float* __restrict__ ws_ml, __nv_bfloat16* __restrict__ lat_out, int H, int R,
                                                            const float* __restrict__ sink, const __nv_bfloat16* __restrict__ head_gate, int ldg) {
@@ -670,15 +671,15 @@ __global__ void __launch_bounds__(128) hy_mla_merge_kernel(const int32_t* __rest
     const float2* ml = reinterpret_cast<const float2*>(ws_ml) + (long long)slot0 * H + h;
     const float* po = ws_o + ((long long)slot0 * H + h) * R;
     float M = s2;
-#pragma unroll 8
+#pragma unroll 4
     for (int p = 0; p < P; ++p) M = fmaxf(M, ml[(long long)p * H].x);
     float L = sink ? exp2f(s2 - M) : 0.f;
-#pragma unroll 8
+#pragma unroll 4
     for (int p = 0; p < P; ++p) { const float2 v = ml[(long long)p * H]; L += exp2f(v.x - M) * v.y; }
     const float inv = (head_gate ? sigmoidf_(ldf(head_gate + (long long)row * ldg + h)) : 1.0f) / L;
     for (int c = threadIdx.x * 4; c < R; c += 128 * 4) {                      // the latent's channels come in groups of 64
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
+#pragma unroll 4
         for (int p = 0; p < P; ++p) {
             const float f = exp2f(ml[(long long)p * H].x - M);
             const float4 u = *reinterpret_cast<const float4*>(po + (long long)p * H * R + c);
